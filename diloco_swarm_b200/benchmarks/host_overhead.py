@@ -90,7 +90,6 @@ def measure(iters: int = 2000, M: int = 16384, d: int = 768) -> Dict[str, float]
             "gemm weight gradient (split-K)": _time_us(
                 lambda: K.gemm(dy, x, a_t=True, b_t=False, mode=K.EPI_ATOMIC_F32, out=dw,
                                split_k=K.wgrad_split(3 * d, d, M)), iters),
-            "tile and split choice": _time_us(lambda: (K._pick_bn(M, 3 * d, 1), K.wgrad_split(3 * d, d, M)), iters),
             "layernorm forward (allocates 3 outputs)": _time_us(lambda: K.layernorm_fwd(x, gamma, beta), max(1, iters // 10)),
             "adamw step": _time_us(lambda: K.adamw_step(p, p, p, p, p16, 1e-3, (0.9, 0.95), 1e-8, 0.1, 1, stats), max(1, iters // 10)),
         }

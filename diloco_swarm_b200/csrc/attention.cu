@@ -27,16 +27,10 @@
 // right halves, and the epilogues write the first 32 columns only.
 #include <cuda.h>
 #include "ptx.cuh"
+#include "tmap.h"
 #include "dswarm.h"
 
 namespace dsw {
-
-int make_tmap_bf16_2d(CUtensorMap* tm, const void* ptr, long long inner, long long outer, long long ld,
-                      int box_inner, int box_outer);
-int make_tmap_f32_2d(CUtensorMap* tm, const void* ptr, long long inner, long long outer, long long ld, int box_inner,
-                     int box_outer);
-int make_tmap_3d(CUtensorMap* tm, int is_f32, const void* ptr, long long inner, long long ncol, long long rows,
-                 long long ld, int box_inner, int box_rows);
 
 // [128 x 64] operand tile of column block `cb` (= part * heads + head) at `row`.
 __device__ __forceinline__ void att_load_tile(void* dst, const CUtensorMap* tm, uint64_t* bar, int hs, int cb, int row) {
@@ -130,7 +124,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, __nv_bfloat16
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nq = T / ATT_BQ;
+  const int nq = (T + ATT_BQ - 1) / ATT_BQ;
   const int total = nq * n_bh;
   const int G = gridDim.x, cta = blockIdx.x;
   const int rounds = (total + G - 1) / G;
@@ -374,6 +368,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, __nv_bfloat16
       tc_fence_after();
       const float inv = 1.f / l;
       const int row0 = b * T + qi * ATT_BQ;                // first global row of this query tile
+      const bool in_seq = qi * ATT_BQ + r < T;             // a last tile may reach into the next sequence
       __nv_bfloat16* dst = out + (long long)(row0 + r) * d + h * hs;
       uint32_t ov[2][32];
       tmem_ld_32x32(tmem_o + lane_addr, ov[0]);
@@ -384,7 +379,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, __nv_bfloat16
       if (lane == 0) mbar_arrive(o_free);          // the next item's first product may overwrite the rows
 #pragma unroll
       for (int i = 0; i < ATT_HS; i += 8)
-        if (i < hs) {
+        if (i < hs && in_seq) {
           const uint32_t* o = ov[i >> 5] + (i & 31);
           *reinterpret_cast<uint4*>(dst + i) =
               make_uint4(pack_bf16(__uint_as_float(o[0]) * inv, __uint_as_float(o[1]) * inv),
@@ -393,7 +388,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, __nv_bfloat16
                          pack_bf16(__uint_as_float(o[6]) * inv, __uint_as_float(o[7]) * inv));
         }
       // natural-log LSE of the scaled scores
-      lse_out[(long long)bh * T + qi * ATT_BQ + r] = (m + log2f(l)) * 0.6931471805599453f;
+      if (in_seq) lse_out[(long long)bh * T + qi * ATT_BQ + r] = (m + log2f(l)) * 0.6931471805599453f;
     }
   }
 
@@ -551,7 +546,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nq = T / ATT_BQ;
+  const int nq = (T + ATT_BQ - 1) / ATT_BQ;
   const int total = nq * n_bh;                   // items, heaviest first: kv tile 0 meets every query tile
   const int G = gridDim.x, cta = blockIdx.x;
   const int rounds = (total + G - 1) / G;
@@ -747,14 +742,16 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
           // dK and dV of the item: two [128 x 64] bf16 tiles staged in the P buffer, one bulk store each
           if (!mbar_wait(dkv_staged, w & 1, abort_flag, status)) break;
           const int kvrow = b * T + j * ATT_BK;
+          if ((j + 1) * ATT_BK <= T) {
 #pragma unroll
-          for (int which = 0; which < 2; ++which)
-            asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];"
-                         ::"l"(&tmap_dkv), "r"(((which + 1) * nh + h) * ATT_HS), "r"(kvrow),
-                           "r"(smem_u32(smem + L::P_OFF + which * ATT_TILE_BYTES))
-                         : "memory");
-          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-          asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+            for (int which = 0; which < 2; ++which)
+              asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];"
+                           ::"l"(&tmap_dkv), "r"(((which + 1) * nh + h) * ATT_HS), "r"(kvrow),
+                             "r"(smem_u32(smem + L::P_OFF + which * ATT_TILE_BYTES))
+                           : "memory");
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+          }
           mbar_arrive(dkv_stored);
         }
         ++w;
@@ -808,7 +805,8 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
       for (int r2 = rr + 1; r2 < rounds; ++r2) {
         int idx2;
         if (att_item(r2, cta, G, total, idx2)) {
-          stat_after = (idx2 % n_bh) * T + (idx2 / n_bh) * ATT_BQ + r;
+          // a row past the end of the sequence: its statistics are never used
+          stat_after = (idx2 / n_bh) * ATT_BQ + r < T ? (idx2 % n_bh) * T + (idx2 / n_bh) * ATT_BQ + r : -1;
           break;
         }
       }
@@ -816,13 +814,17 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
         const int i = j + it;
         const int stat = bh * T + i * ATT_BQ + r;       // < 2^31: the launcher checks B * nh * T
         // row statistics: loaded for the CTA's first step, fetched one step ahead (across items too) after that
-        const float lse2 = (g == 0 ? lse[stat] : lse_next) * 1.4426950408889634f;
-        const float Dr = g == 0 ? Dvec[stat] : D_next;
+        // Rows past the end of the sequence (last tile of a length that is no multiple of 128) have an infinite
+        // log-sum-exp: their P and dS come out as zeros, so whatever the tile holds there adds nothing.
+        const bool in_seq = i * ATT_BQ + r < T;
+        if (g == 0 && in_seq) { lse_next = lse[stat]; D_next = Dvec[stat]; }
+        const float lse2 = in_seq ? lse_next * 1.4426950408889634f : INFINITY;
+        const float Dr = in_seq ? D_next : 0.f;
         ATT_TRACE(tr, 0, tslot);              // step start
         if (!mbar_wait(sdp_full, g & 1, abort_flag, status)) { ok = false; break; }
         tc_fence_after();
         {
-          const int sn = it + 1 < steps ? stat + ATT_BQ : stat_after;
+          const int sn = it + 1 < steps ? ((i + 1) * ATT_BQ + r < T ? stat + ATT_BQ : -1) : stat_after;
           if (sn >= 0) { lse_next = lse[sn]; D_next = Dvec[sn]; }
         }
         ATT_TRACE(tr, 0, tslot);              // S, dP arrived
@@ -886,7 +888,9 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
       }
       // the last step's dQ; its barrier also says that every dV / dK product of the item is done
       if (!ok || !drain_dq(g - 1)) { ok = false; break; }
-      // dV and dK rows of this kv tile (TMEM lane = kv row)
+      // dV and dK rows of this kv tile (TMEM lane = kv row).  A tile that ends behind its sequence cannot leave as
+      // a whole (the rows there belong to the next sequence): its rows are stored one by one.
+      const bool whole = (j + 1) * ATT_BK <= T;
       __nv_bfloat16* row = dqkv + (long long)(b * T + j * ATT_BK + r) * 3 * d + h * hs;
       uint32_t vk[32], vv[32];
       tmem_ld_32x32(tm_dk + lane_addr + half * 32, vk);
@@ -895,7 +899,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(dkv_free);          // the next item's first products may overwrite the sums
-      if (hs == 64) {
+      if (hs == 64 && whole) {
         // staged as two 128-byte-swizzled [128 x 64] bf16 tiles (dK, dV) in the P buffer, which nothing reads
         // any more; the reducer warp stores them with one bulk copy each
 #pragma unroll
@@ -912,7 +916,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
         fence_proxy_async();
         __syncwarp();
         if (lane == 0) mbar_arrive(dkv_staged);
-      } else if (half * 32 < hs) {
+      } else if (half * 32 < hs && j * ATT_BK + r < T) {
 #pragma unroll
         for (int which = 0; which < 2; ++which) {
           __nv_bfloat16* dst = row + (which == 0 ? d : 2 * d) + half * 32;
@@ -926,6 +930,10 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
                 pack_bf16(__uint_as_float(v[c + 6]), __uint_as_float(v[c + 7])));
           }
         }
+      }
+      if (hs == 64 && !whole) {                        // nothing staged: the reducer only passes the buffer on
+        __syncwarp();
+        if (lane == 0) mbar_arrive(dkv_staged);
       }
       ++w;
     }
@@ -959,14 +967,14 @@ static int att_num_sms() {
 extern "C" int dsw_attention_set_trace(long long* buf) { g_att_trace = buf; return 0; }
 
 // qkv: bf16 [B*T, 3*nh*hs]; out: bf16 [B*T, nh*hs]; lse: fp32 [B*nh*T].
-// Requires hs == 64 or 32 and T a multiple of 128.
+// Requires hs == 64 or 32.
 extern "C" int dsw_attention_fwd(const void* qkv, void* out, float* lse, int B, int T, int nh, int hs, float scale,
                                  int* status, cudaStream_t st) {
-  if ((hs != 64 && hs != 32) || T % ATT_BQ != 0) return -10;
+  if ((hs != 64 && hs != 32) || T <= 0) return -10;
   const int d = nh * hs;
   CUtensorMap tm;
-  int rc = hs == 64 ? make_tmap_bf16_2d(&tm, qkv, 3LL * d, (long long)B * T, 3LL * d, 64, 128)
-                    : make_tmap_3d(&tm, 0, qkv, hs, 3LL * nh, (long long)B * T, 3LL * d, 64, 128);
+  int rc = hs == 64 ? cached_tmap(&tm, TMAP_BF16_2D, qkv, 3LL * d, 1, (long long)B * T, 3LL * d, 64, 128)
+                    : cached_tmap(&tm, TMAP_BF16_3D, qkv, hs, 3LL * nh, (long long)B * T, 3LL * d, 64, 128);
   if (rc) return rc;
   static bool attr_set = false;
   if (!attr_set) {
@@ -976,7 +984,7 @@ extern "C" int dsw_attention_fwd(const void* qkv, void* out, float* lse, int B, 
     attr_set = true;
   }
   // persistent: two CTAs per SM walk the work items
-  const int total = (T / ATT_BQ) * B * nh;
+  const int total = ((T + ATT_BQ - 1) / ATT_BQ) * B * nh;
   const int G = total < 2 * att_num_sms() ? total : 2 * att_num_sms();
   attention_fwd_kernel<<<G, ATT_THREADS, AttSmem::TOTAL, st>>>(tm, (__nv_bfloat16*)out, lse, T, nh, B * nh, hs,
                                                                scale * 1.4426950408889634f, status, g_att_trace);
@@ -988,21 +996,21 @@ extern "C" int dsw_attention_fwd(const void* qkv, void* out, float* lse, int B, 
 extern "C" int dsw_attention_bwd(const void* qkv, const void* out, const void* dout, const float* lse, void* dqkv,
                                  float* dq_acc, float* Dvec, int B, int T, int nh, int hs, float scale, int* status,
                                  cudaStream_t st) {
-  if ((hs != 64 && hs != 32) || T % ATT_BQ != 0 || (long long)B * nh * T >= (1LL << 31)) return -10;
+  if ((hs != 64 && hs != 32) || T <= 0 || (long long)B * nh * T >= (1LL << 31)) return -10;
   const int d = nh * hs;
   const long long rows = (long long)B * T;
   CUtensorMap tq, tdo, tdq, tdkv;
   int rc;
   if (hs == 64) {
-    rc = make_tmap_bf16_2d(&tq, qkv, 3LL * d, rows, 3LL * d, 64, 128);
-    if (!rc) rc = make_tmap_bf16_2d(&tdkv, dqkv, 3LL * d, rows, 3LL * d, 64, 128);
-    if (!rc) rc = make_tmap_bf16_2d(&tdo, dout, d, rows, d, 64, 128);
-    if (!rc) rc = make_tmap_f32_2d(&tdq, dq_acc, d, rows, d, 32, 128);
+    rc = cached_tmap(&tq, TMAP_BF16_2D, qkv, 3LL * d, 1, rows, 3LL * d, 64, 128);
+    if (!rc) rc = cached_tmap(&tdkv, TMAP_BF16_2D, dqkv, 3LL * d, 1, rows, 3LL * d, 64, 128);
+    if (!rc) rc = cached_tmap(&tdo, TMAP_BF16_2D, dout, d, 1, rows, d, 64, 128);
+    if (!rc) rc = cached_tmap(&tdq, TMAP_F32_2D, dq_acc, d, 1, rows, d, 32, 128);
   } else {
-    rc = make_tmap_3d(&tq, 0, qkv, hs, 3LL * nh, rows, 3LL * d, 64, 128);
+    rc = cached_tmap(&tq, TMAP_BF16_3D, qkv, hs, 3LL * nh, rows, 3LL * d, 64, 128);
     tdkv = tq;            // not used with 32 columns per head: dK and dV are stored by the row threads
-    if (!rc) rc = make_tmap_3d(&tdo, 0, dout, hs, nh, rows, d, 64, 128);
-    if (!rc) rc = make_tmap_3d(&tdq, 1, dq_acc, hs, nh, rows, d, 32, 128);
+    if (!rc) rc = cached_tmap(&tdo, TMAP_BF16_3D, dout, hs, nh, rows, d, 64, 128);
+    if (!rc) rc = cached_tmap(&tdq, TMAP_F32_3D, dq_acc, hs, nh, rows, d, 32, 128);
   }
   if (rc) return rc;
   static bool attr_set = false;
@@ -1020,7 +1028,7 @@ extern "C" int dsw_attention_bwd(const void* qkv, const void* out, const void* d
         (const __nv_bfloat16*)out, (const __nv_bfloat16*)dout, Dvec, dq_acc, B, T, nh, hs);
   }
   // persistent: one CTA per SM walks the work items
-  const int total = (T / ATT_BK) * B * nh;
+  const int total = ((T + ATT_BK - 1) / ATT_BK) * B * nh;
   const int G = total < att_num_sms() ? total : att_num_sms();
   attention_bwd_kernel<<<G, ATT_BWD_THREADS, AttBwdSmem::TOTAL, st>>>(tq, tdo, tdq, tdkv, lse, Dvec, (__nv_bfloat16*)dqkv, T, nh,
                                                                        B * nh, hs, scale, status, g_att_trace);

@@ -37,7 +37,8 @@ extern "C" {
 // out[M,N] = A * B^T-or-B with fp32 accumulation on the tcgen05 tensor cores.
 // A: [M,K] row-major (a_mn_major = 0) or [K,M] row-major (1); B: [N,K] (b_mn_major = 0) or [K,N] (1);
 // lda/ldb/ldo/ldr/ldaux are row pitches in elements.  bn = 128 or 256 picks the one-CTA tile width,
-// 512 the CTA-pair kernel (256 x 256 per pair).  split_k > 1 only with DSW_EPI_ATOMIC_F32.
+// 512 the CTA-pair kernel (256 x 256 per pair), 0 leaves the choice to the library.  split_k > 1 only with
+// DSW_EPI_ATOMIC_F32 (0: chosen by the library).
 // max_ctas > 0 caps the grid.
 int dsw_gemm_bf16(const void* A, long long lda, int a_mn_major, const void* B, long long ldb, int b_mn_major,
                   int M, int N, int K, int mode, int split_k, void* out, long long ldo, const float* bias,
@@ -49,7 +50,7 @@ int dsw_gemm_set_trace(long long* buf);
 
 // ---------------------------------------------------------------- attention (attention.cu)
 // Causal flash attention over a packed activation qkv: bf16 [B*T, 3*nh*hs] (Q | K | V, head h at columns
-// h*hs of each).  out: bf16 [B*T, nh*hs]; lse: fp32 [B*nh*T].  hs is 64 or 32, T a multiple of 128.
+// h*hs of each).  out: bf16 [B*T, nh*hs]; lse: fp32 [B*nh*T].  hs is 64 or 32.
 int dsw_attention_fwd(const void* qkv, void* out, float* lse, int B, int T, int nh, int hs, float scale,
                       int* status, cudaStream_t st);
 // dqkv: bf16 like qkv.  dq_acc: fp32 [B*T, nh*hs] and Dvec: fp32 [B*nh*T] are work arrays, contents irrelevant.

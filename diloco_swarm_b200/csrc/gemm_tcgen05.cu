@@ -17,10 +17,13 @@
 // Two accumulators (2 x BN columns of TMEM) let the epilogue of tile i overlap
 // the main loop of tile i+1.  No thread-block clusters and no multicast loads.
 #include <cuda.h>
+#include <cmath>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <mutex>
 #include "gemm_kernels.cuh"
+#include "tmap.h"
 #include "dswarm.h"
 
 namespace dsw {
@@ -90,33 +93,86 @@ int make_tmap_3d(CUtensorMap* tm, int is_f32, const void* ptr, long long inner, 
 }
 
 
-// Encoded tensor maps of recent launches.  A training step calls the GEMMs thousands of times on a few
-// dozen distinct (pointer, shape, pitch, box) combinations, because the caching allocator hands the same
-// blocks back microbatch after microbatch; encoding a map costs more host time than the rest of a launch.
-// One small direct-mapped table per host thread, so no lock is taken.
+// Encoded tensor maps of recent launches.  A training step calls the GEMMs and the attention kernels thousands of
+// times on a few dozen distinct (pointer, shape, pitch, box) combinations, because work areas and the caching
+// allocator's blocks come back microbatch after microbatch; encoding a map costs more host time than the rest of a
+// launch.  One small direct-mapped table per host thread, so no lock is taken.
 struct TmapKey {
-  const void* ptr; long long inner, outer, ld; int box_inner, box_outer;
+  const void* ptr; long long inner, ncol, outer, ld; int box_inner, box_outer, kind;
   bool operator==(const TmapKey& o) const {
-    return ptr == o.ptr && inner == o.inner && outer == o.outer && ld == o.ld && box_inner == o.box_inner &&
-           box_outer == o.box_outer;
+    return ptr == o.ptr && inner == o.inner && ncol == o.ncol && outer == o.outer && ld == o.ld &&
+           box_inner == o.box_inner && box_outer == o.box_outer && kind == o.kind;
   }
 };
 struct TmapSlot { TmapKey key; CUtensorMap map; bool used; };
-constexpr int TMAP_SLOTS = 1024;
+constexpr int TMAP_SLOTS = 2048;
 
-static int cached_tmap_bf16_2d(CUtensorMap* tm, const void* ptr, long long inner, long long outer, long long ld,
-                               int box_inner, int box_outer) {
+int cached_tmap(CUtensorMap* tm, int kind, const void* ptr, long long inner, long long ncol, long long outer, long long ld,
+                int box_inner, int box_outer) {
   static thread_local TmapSlot table[TMAP_SLOTS];
-  const TmapKey key{ptr, inner, outer, ld, box_inner, box_outer};
+  const TmapKey key{ptr, inner, ncol, outer, ld, box_inner, box_outer, kind};
   unsigned long long h = reinterpret_cast<unsigned long long>(ptr) >> 8;
   h ^= (unsigned long long)inner * 0x9E3779B97F4A7C15ull;
-  h ^= ((unsigned long long)outer << 21) ^ ((unsigned long long)ld << 7) ^ (unsigned long long)(box_inner * 131 + box_outer);
+  h ^= ((unsigned long long)outer << 21) ^ ((unsigned long long)ld << 7) ^
+       (unsigned long long)(box_inner * 131 + box_outer + kind * 8191 + ncol * 524287);
   h ^= h >> 29;
   TmapSlot& s = table[h % TMAP_SLOTS];
   if (s.used && s.key == key) { *tm = s.map; return 0; }
-  const int rc = make_tmap_bf16_2d(tm, ptr, inner, outer, ld, box_inner, box_outer);
+  int rc;
+  if (kind == TMAP_BF16_2D)     rc = make_tmap_bf16_2d(tm, ptr, inner, outer, ld, box_inner, box_outer);
+  else if (kind == TMAP_F32_2D) rc = make_tmap_f32_2d(tm, ptr, inner, outer, ld, box_inner, box_outer);
+  else                          rc = make_tmap_3d(tm, kind == TMAP_F32_3D, ptr, inner, ncol, outer, ld, box_inner, box_outer);
   if (rc == 0) { s.key = key; s.map = *tm; s.used = true; }
   return rc;
+}
+
+// ------------------------------------------------------------------ tile choice
+static double tile_efficiency(long long M, long long N, int splits, int bm, int bn, int units) {
+  const long long tm = (M + bm - 1) / bm, tn = (N + bn - 1) / bn, tiles = tm * tn * splits;
+  const long long waves = (tiles + units - 1) / units;
+  return double(M) * N / (double(tm) * bm * tn * bn) * tiles / (double(waves) * units);
+}
+
+// Cap on the CTAs of every GEMM launch (0 = all SMs): leaves SMs to kernels that sit on the device while the GEMMs run,
+// such as a pipeline transfer waiting for its peer.
+static int default_max_ctas() {
+  static const int n = [] { const char* e = getenv("DSWARM_GEMM_MAX_CTAS"); return e ? atoi(e) : 0; }();
+  return n;
+}
+
+static bool use_pair() {
+  static const bool on = [] { const char* e = getenv("DSWARM_GEMM_PAIR"); return !(e && e[0] == '0' && e[1] == 0); }();
+  return on;
+}
+
+// 512 = 256 x 256 on a CTA pair (least operand traffic per FLOP), 256 = 128 x 256 on one CTA, 128 = 128 x 128.  A wider
+// tile wins unless a narrower one fills the SMs clearly better.
+static int pick_bn(int M, int N, int splits, int sms) {
+  if (N <= 128) return 128;
+  const double e128 = tile_efficiency(M, N, splits, 128, 128, sms), e256 = tile_efficiency(M, N, splits, 128, 256, sms);
+  if (use_pair() && M >= 256) {
+    const double pair = tile_efficiency(M, N, splits, 256, 256, sms / 2);
+    if (pair >= fmax(e128 * 0.8, e256 * 0.9)) return 512;
+  }
+  return e256 >= e128 * 0.93 ? 256 : 128;
+}
+
+// Split of K (tokens) for a weight gradient dW[M,N]: few output tiles, so K is split until the SMs are full.
+static int pick_wgrad_split(int M, int N, int K, int sms) {
+  const bool pair = use_pair() && M >= 256;
+  const int bm = pair ? 256 : 128, units = pair ? sms / 2 : sms;
+  const long long tiles = (long long)((M + bm - 1) / bm) * ((N + 255) / 256);
+  if (tiles >= 4 * units) return 1;
+  const int kb = (K + 63) / 64;
+  int best = 1;
+  double best_eff = 0.0;
+  for (int s = 1; s <= 16 && kb / s >= 4; ++s) {
+    const long long waves = (tiles * s + units - 1) / units;
+    const double eff = double(tiles * s) / double(waves * units) - 0.01 * (s - 1);      // small price per split (atomics)
+    if (eff > best_eff + 1e-9) { best = s; best_eff = eff; }
+  }
+  const int per = (kb + best - 1) / best;
+  return (kb + per - 1) / per;                   // no empty split
 }
 
 }  // namespace dsw
@@ -130,7 +186,7 @@ extern "C" int dsw_gemm_set_trace(long long* buf) { g_gemm_trace = buf; return 0
 // A: [M,K] row-major (a_mn_major = 0) or [K,M] row-major (1); lda = row pitch in
 // elements.  B: [N,K] (b_mn_major = 0) or [K,N] (1).  All pitches and the
 // contiguous extents must be multiples of 8 elements; pointers 16-byte aligned.
-// bn = 128 or 256 selects the one-CTA tile width, 512 the CTA-pair kernel; max_ctas > 0 caps the
+// bn = 128 or 256 selects the one-CTA tile width, 512 the CTA-pair kernel, 0 leaves it to the shape; max_ctas > 0 caps the
 // grid (to leave SMs to a concurrent kernel).  Returns 0 or a negative error code.
 extern "C" int dsw_gemm_bf16(const void* A, long long lda, int a_mn_major, const void* B, long long ldb,
                              int b_mn_major, int M, int N, int K, int mode, int split_k, void* out, long long ldo,
@@ -140,7 +196,7 @@ extern "C" int dsw_gemm_bf16(const void* A, long long lda, int a_mn_major, const
   if ((lda | ldb | ldo) % 8 || N % 8 || (a_mn_major ? M % 8 : K % 8) || (b_mn_major ? N % 8 : K % 8)) return -10;
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(out)) & 15)
     return -11;
-  if (bn != 128 && bn != 256 && bn != 512) return -12;   // 512 = CTA-pair kernel (256 x 256 per cluster)
+  if (bn != 0 && bn != 128 && bn != 256 && bn != 512) return -12;   // 512 = CTA-pair kernel (256 x 256 per cluster)
   if (mode < EPI_STORE || mode > EPI_STORE_F32) return -13;
   if ((mode == EPI_RESID && (resid == nullptr || ldr % 8)) || (mode == EPI_MUL && (aux_in == nullptr || ldaux % 8)) ||
       (mode == EPI_GELU && aux_out != nullptr && ldaux % 8))
@@ -149,13 +205,16 @@ extern "C" int dsw_gemm_bf16(const void* A, long long lda, int a_mn_major, const
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -2;
   if (num_sms[dev] == 0) cudaDeviceGetAttribute(&num_sms[dev], cudaDevAttrMultiProcessorCount, dev);
+  if (split_k == 0) split_k = mode == EPI_ATOMIC_F32 ? pick_wgrad_split(M, N, K, num_sms[dev]) : 1;
+  if (bn == 0) bn = pick_bn(M, N, split_k, num_sms[dev]);
+  if (max_ctas == 0) max_ctas = default_max_ctas();
   CUtensorMap ta, tb;
   int rc;
-  if (!a_mn_major) rc = cached_tmap_bf16_2d(&ta, A, K, M, lda, BK, BM);
-  else             rc = cached_tmap_bf16_2d(&ta, A, M, K, lda, 64, BK);
+  if (!a_mn_major) rc = cached_tmap(&ta, TMAP_BF16_2D, A, K, 1, M, lda, BK, BM);
+  else             rc = cached_tmap(&ta, TMAP_BF16_2D, A, M, 1, K, lda, 64, BK);
   if (rc) return rc;
-  if (!b_mn_major) rc = cached_tmap_bf16_2d(&tb, B, K, N, ldb, BK, bn == 512 ? 128 : bn);
-  else             rc = cached_tmap_bf16_2d(&tb, B, N, K, ldb, 64, BK);
+  if (!b_mn_major) rc = cached_tmap(&tb, TMAP_BF16_2D, B, K, 1, N, ldb, BK, bn == 512 ? 128 : bn);
+  else             rc = cached_tmap(&tb, TMAP_BF16_2D, B, N, 1, K, ldb, 64, BK);
   if (rc) return rc;
   GemmArgs g;
   g.M = M; g.N = N; g.K = K;

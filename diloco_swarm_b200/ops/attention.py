@@ -25,14 +25,14 @@ from ._lib import Status, check, cuda_lib, stream_ptr
 BF16 = torch.bfloat16
 
 
-def _native_available(hs: int, T: int) -> bool:
+def native_available(hs: int) -> bool:
     """The sm_100a kernels cover head size 64 (GPT-2 small to xl) and 32 (the
-    4-head, 128-wide test model) at sequence lengths that are multiples of 128;
-    other shapes use the library kernel."""
+    4-head, 128-wide test model) at any sequence length; other head sizes use
+    the library kernel."""
     if os.environ.get("DSWARM_ATTENTION", "native") == "sdpa":
         return False
     lib = cuda_lib()
-    return hs in (32, 64) and T % 128 == 0 and hasattr(lib, "dsw_attention_fwd") and hasattr(lib, "dsw_attention_bwd")
+    return hs in (32, 64) and hasattr(lib, "dsw_attention_fwd") and hasattr(lib, "dsw_attention_bwd")
 
 
 class AttnCtx:
@@ -47,7 +47,7 @@ def attention_fwd(qkv: torch.Tensor, B: int, T: int, nh: int, need_ctx: bool = T
     d = d3 // 3
     hs = d // nh
     ctx = AttnCtx() if need_ctx else None
-    if _native_available(hs, T):
+    if native_available(hs):
         out = torch.empty(M, d, dtype=BF16, device=qkv.device)
         lse = torch.empty(B * nh * T, dtype=torch.float32, device=qkv.device)
         check(cuda_lib().dsw_attention_fwd(qkv.data_ptr(), out.data_ptr(), lse.data_ptr(), B, T, nh, hs,

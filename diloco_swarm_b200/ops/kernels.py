@@ -6,9 +6,7 @@ its outputs.  The docstrings name the reference call site each one replaces.
 """
 from __future__ import annotations
 
-import functools
 import math
-import os
 from typing import Optional, Tuple
 
 import torch
@@ -18,40 +16,6 @@ from ._lib import Status, check, cuda_lib, ptr, stream_ptr
 BF16, F32 = torch.bfloat16, torch.float32
 
 EPI_STORE, EPI_GELU, EPI_RESID, EPI_MUL, EPI_ATOMIC_F32, EPI_STORE_F32 = range(6)
-
-_NUM_SMS = 148
-
-
-_USE_PAIR = os.environ.get("DSWARM_GEMM_PAIR", "1") != "0"
-# Cap on the CTAs of every GEMM launch (0 = all SMs): leaves SMs to kernels that sit on the device while
-# the GEMMs run, such as a pipeline transfer waiting for its peer.
-_MAX_CTAS = int(os.environ.get("DSWARM_GEMM_MAX_CTAS", "0"))
-
-
-def _efficiency(M: int, N: int, splits: int, bm: int, bn: int, units: int) -> float:
-    """Fraction of the machine busy with real tiles when the grid runs in whole waves."""
-    tiles = math.ceil(M / bm) * math.ceil(N / bn) * splits
-    waves = math.ceil(tiles / units)
-    useful = (M * N) / (math.ceil(M / bm) * bm * math.ceil(N / bn) * bn)
-    return useful * tiles / (waves * units)
-
-
-@functools.lru_cache(maxsize=None)          # a training run asks for a handful of shapes, thousands of times a step
-def _pick_bn(M: int, N: int, splits: int = 1) -> int:
-    """Tile choice: 512 = 256x256 on a CTA pair (least operand traffic per FLOP),
-    256 = 128x256 on one CTA, 128 = 128x128.  A wider tile wins unless a
-    narrower one fills the SMs clearly better."""
-    if N <= 128:
-        return 128
-    e128 = _efficiency(M, N, splits, 128, 128, _NUM_SMS)
-    e256 = _efficiency(M, N, splits, 128, 256, _NUM_SMS)
-    best = 256 if e256 >= e128 * 0.93 else 128
-    if _USE_PAIR and M >= 256:
-        epair = _efficiency(M, N, splits, 256, 256, _NUM_SMS // 2)
-        if epair >= max(e128 * 0.8, e256 * 0.9):
-            best = 512
-    return best
-
 
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool = True, mode: int = EPI_STORE,
          out: Optional[torch.Tensor] = None, bias: Optional[torch.Tensor] = None,
@@ -66,6 +30,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool = Tru
     Epilogues: EPI_GELU returns gelu(acc + bias) (exact erf form) and, when
     ``aux_out`` is given, also stores gelu'(acc + bias) there; EPI_MUL returns
     acc * ``aux_in``, which with that saved derivative is the GELU backward.
+    ``bn`` (tile) and ``split_k`` (with EPI_ATOMIC_F32) are chosen by the library when 0.
     """
     assert a.dtype == BF16 and b.dtype == BF16 and a.dim() == 2 and b.dim() == 2
     assert a.stride(1) == 1 and b.stride(1) == 1
@@ -91,16 +56,11 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool = Tru
         assert resid is not None and resid.shape == (M, N) and resid.dtype == BF16
     if bias is not None:
         assert bias.dtype == F32 and bias.numel() == N
-    kb_total = math.ceil(K / 64)
-    split_k = max(1, min(split_k, kb_total))
     if split_k > 1:
         assert mode == EPI_ATOMIC_F32, "split-K needs the accumulating epilogue"
-        per = math.ceil(kb_total / split_k)
+        kb_total = math.ceil(K / 64)
+        per = math.ceil(kb_total / min(split_k, kb_total))
         split_k = math.ceil(kb_total / per)       # no empty split
-    if bn == 0:
-        bn = _pick_bn(M, N, split_k)
-    if max_ctas == 0:
-        max_ctas = _MAX_CTAS
     aux = aux_out if aux_out is not None else aux_in
     rc = cuda_lib().dsw_gemm_bf16(
         a.data_ptr(), a.stride(0), 1 if a_t else 0, b.data_ptr(), b.stride(0), 0 if b_t else 1, M, N, K, mode,
@@ -124,28 +84,14 @@ def set_deterministic(on: bool) -> None:
     _DETERMINISTIC = bool(on)
 
 
+def deterministic() -> bool:
+    return _DETERMINISTIC
+
+
 def wgrad_split(M: int, N: int, K: int) -> int:
-    """Split-K factor for dW[M,N] = dy^T x with K = tokens: the weight gradients
-    of a block have few output tiles, so K is split until the SMs are full."""
-    return 1 if _DETERMINISTIC else _wgrad_split(M, N, K)
-
-
-@functools.lru_cache(maxsize=None)
-def _wgrad_split(M: int, N: int, K: int) -> int:
-    bm, units = (256, _NUM_SMS // 2) if (_USE_PAIR and M >= 256) else (128, _NUM_SMS)
-    tiles = math.ceil(M / bm) * math.ceil(N / 256)
-    if tiles >= 4 * units:
-        return 1
-    kb = math.ceil(K / 64)
-    best, best_eff = 1, 0.0
-    for s in range(1, 17):
-        if kb // s < 4:
-            break
-        waves = math.ceil(tiles * s / units)
-        eff = tiles * s / (waves * units) - 0.01 * (s - 1)      # small price per extra split (atomics)
-        if eff > best_eff + 1e-9:
-            best, best_eff = s, eff
-    return best
+    """``split_k`` for dW[M,N] = dy^T x with K = tokens: 0 (the library's choice for the shape), or 1 with
+    deterministic gradients."""
+    return 1 if _DETERMINISTIC else 0
 
 
 def layernorm_fwd(x: torch.Tensor, gamma: torch.Tensor, beta: Optional[torch.Tensor], eps: float = 1e-5
