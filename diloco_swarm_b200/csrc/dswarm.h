@@ -84,6 +84,8 @@ int dsw_embedding_bwd_sorted(const long long* sorted, const long long* perm, con
                              float* dwpe, int B, int T, int d, int V, cudaStream_t st);
 // count[0] += number of non-zero mask entries; the caller clears count first.
 int dsw_mask_count(const long long* mask, int M, float* count, cudaStream_t st);
+// loss[0] = 0; count[0] = number of non-zero mask entries, or M when mask is null.
+int dsw_loss_begin(const long long* mask, int M, float* count, float* loss, cudaStream_t st);
 // Masked mean cross-entropy over bf16 logits [M, V] (row pitch ld): loss_acc += scale * mean loss; with
 // write_grad the logits are overwritten by d(loss)/d(logits).  mask may be null (count must then hold M).
 int dsw_cross_entropy(void* logits, long long ld, const long long* targets, const long long* mask,
@@ -145,6 +147,22 @@ int dsw_outer_sync_nvls(void* const* bufs, void* mc, void* const* flags, float* 
 int dsw_grad_allreduce_nvls(void* const* bufs, void* mc, void* const* flags, float* grad, long long offset,
                             long long count, long long shard, int rank, int R, int wire_bf16, unsigned seq,
                             long long wait_limit, int blocks, int* status, cudaStream_t st);
+
+// ---------------------------------------------------------------- stage executor (stage.cu)
+// A pipeline stage's forward and backward as sequences of the launches above, one call each.  desc: int64 array of
+// sizes and device pointers (layout at dsw_stage_create); saved / scratch: work areas of the sizes that
+// dsw_stage_sizes gives for the same B, T, keep, grad and chunks.  Several threads may call; a pass is queued whole.
+int dsw_stage_create(const long long* desc, int len, void** out);
+int dsw_stage_destroy(void* stage);
+int dsw_stage_launches();
+int dsw_stage_sizes(void* stage, int B, int T, int keep, int grad, int chunks, size_t* saved, size_t* scratch);
+int dsw_stage_forward(void* stage, const long long* ids, const void* x, void* saved, void* y, float* infer_logits,
+                      int B, int T, int keep, cudaStream_t st);
+int dsw_stage_head(void* stage, void* saved, void* scratch, const long long* targets, const long long* mask,
+                   float scale, float* loss, int B, int T, int keep, int grad, int chunks, int deterministic,
+                   cudaStream_t st);
+int dsw_stage_backward(void* stage, int hi, int lo, const void* dy, const void* x, const long long* ids, void* saved,
+                       void* scratch, void* dx0, int B, int T, int chunks, int deterministic, cudaStream_t st);
 
 // ---------------------------------------------------------------- bounds-checking build (-DDSWARM_BOUNDS)
 // First failed bounds check since the last call: 0 = none, else 100000 * unit + source line (units: 1

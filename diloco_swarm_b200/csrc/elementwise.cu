@@ -490,6 +490,35 @@ __global__ void mask_count_kernel(const long long* __restrict__ mask, int M, flo
   }
 }
 
+// Start of a microbatch's loss: loss[0] = 0 and count[0] = number of rows the mean is over (mask != 0, all M without a
+// mask), in one launch of one block: the count decides nothing until the cross-entropy, and two memsets and a
+// reduction over blocks cost three launches.  Eight independent loads per thread and round keep it at some 6 us for
+// 65536 rows.
+__global__ void __launch_bounds__(1024)
+loss_begin_kernel(const long long* __restrict__ mask, int M, float* __restrict__ count, float* __restrict__ loss) {
+  __shared__ int sh[32];
+  int c = 0;
+  if (mask) {
+    for (int i0 = threadIdx.x; i0 < M; i0 += 8 * 1024) {
+      long long v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = i0 + u * 1024 < M ? mask[i0 + u * 1024] : 0;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) c += v[u] != 0;
+    }
+  }
+  c = __reduce_add_sync(0xffffffffu, c);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = c;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    c = __reduce_add_sync(0xffffffffu, sh[threadIdx.x]);
+    if (threadIdx.x == 0) {
+      count[0] = mask ? float(c) : float(M);
+      loss[0] = 0.f;
+    }
+  }
+}
+
 // One block per row.  loss_acc += scale/count * (lse - logit[target]) for kept
 // rows; with write_grad the row is overwritten by scale/count * (softmax - onehot)
 // (zeros for masked rows).  Two passes over the row; the second hits L2.
@@ -705,6 +734,11 @@ extern "C" int dsw_mask_count(const long long* mask, int M, float* count, cudaSt
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
+extern "C" int dsw_loss_begin(const long long* mask, int M, float* count, float* loss, cudaStream_t st) {
+  loss_begin_kernel<<<1, 1024, 0, st>>>(mask, M, count, loss);
+  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+}
+
 extern "C" int dsw_cross_entropy(void* logits, long long ld, const long long* targets, const long long* mask,
                                  const float* count, float scale, float* loss_acc, int M, int V, int write_grad,
                                  int* status, cudaStream_t st) {
@@ -770,7 +804,7 @@ extern "C" int dsw_load_elementwise() {
   L(layernorm_bwd_kernel<5>); L(layernorm_bwd_kernel<6>); L(layernorm_bwd_kernel<7>); L(layernorm_bwd_kernel<8>);
   L(layernorm_bwd_finish_kernel); L(colsum_kernel); L(embedding_fwd_kernel); L(embedding_bwd_kernel);
   L(embedding_bwd_sorted_kernel); L(embedding_bwd_pos_kernel);
-  L(mask_count_kernel); L(cross_entropy_kernel); L(cast_f32_bf16_kernel); L(cast_bf16_f32_kernel);
+  L(mask_count_kernel); L(loss_begin_kernel); L(cross_entropy_kernel); L(cast_f32_bf16_kernel); L(cast_bf16_f32_kernel);
 #undef L
   return bad ? -1 : 0;
 }

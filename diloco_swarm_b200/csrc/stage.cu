@@ -1,0 +1,393 @@
+// Native executor of a GPT-2 pipeline stage: the forward and the backward of its blocks, embedding and LM head as
+// sequences of launches of this library's kernels, queued by one call each.
+//
+// What it is for.  A microbatch is some twenty launches per block.  Queued one by one from Python (argument checks,
+// an allocation, a ctypes call, stream bookkeeping) a launch costs about 20 us of host time, which is what bounded
+// every pass of fewer than some eight thousand tokens: one position of the sampling loop on GPT-2 small spent
+// 730 us on the device and 2050 us on the host.  From here a launch costs the driver's own 2 us.
+//
+// Memory.  The caller hands in two work areas per call: `saved` holds what the backward of a microbatch needs (one
+// per microbatch in flight), `scratch` what lives within a call.  Their sizes come from dsw_stage_sizes.  Nothing is
+// allocated here, so no pass waits for the allocator, and memory that the side stream reads needs no bookkeeping
+// beyond the events below.
+//
+// Streams.  Weight-gradient GEMMs and bias column sums feed nothing in the backward, so they go to the stage's side
+// stream (when it has one) and fill the SMs that the dgrad chain leaves idle.  The buffers they read (dh, dx1, dqkv)
+// are doubled by block parity: before a block overwrites a set the main stream waits for the side work of the block
+// two up, which is long done.  A block's outgoing gradient is read by the side work of the block below it, so those
+// buffers form a ring of three.
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+#include <atomic>
+#include <cmath>
+#include <cstdlib>
+#include <mutex>
+#include <new>
+#include <vector>
+#include "dswarm.h"
+
+namespace {
+
+typedef __nv_bfloat16 bf16;
+
+std::atomic<int> g_launches{0};      // launcher calls made from here (each launches at least one kernel)
+
+enum { W_QKV = 0, W_O = 1, W_FC = 2, W_PR = 3 };
+
+struct Block {
+  const float *ln1_w, *ln1_b, *ln2_w, *ln2_b;
+  float *dln1_w, *dln1_b, *dln2_w, *dln2_b;
+  const bf16* w[4];
+  const float* b[4];
+  float *dw[4], *db[4];
+};
+
+struct Stage {
+  int n, d, nh, V;
+  int* status;
+  cudaStream_t side;
+  const float *wte, *wpe;
+  float *dwte, *dwpe;
+  const float *lnf_w, *lnf_b;
+  float *dlnf_w, *dlnf_b;
+  const bf16* head_w;
+  float *dhead_w, *count;
+  std::vector<Block> blocks;
+  cudaEvent_t fork;              // main -> side
+  cudaEvent_t side_done[2];      // side work of the last block of each parity
+  cudaEvent_t head_done;         // side work on the logits
+  bool side_used[2], head_used;
+  std::mutex mu;                 // one pass is queued at a time: passes of one stage share its scratch
+};
+
+// Layout of a work area: pieces are handed out 256 bytes apart.
+struct Area {
+  char* base;
+  size_t used = 0;
+  explicit Area(void* p) : base(static_cast<char*>(p)) {}
+  template <class T>
+  T* take(size_t count) {
+    T* p = reinterpret_cast<T*>(base + used);
+    used += (count * sizeof(T) + 255) / 256 * 256;
+    return p;
+  }
+};
+
+// What a block leaves for its backward.
+struct Saved {
+  bf16 *ln1, *qkv, *att, *x1, *ln2, *h, *g, *out;
+  float *mu1, *rs1, *mu2, *rs2, *lse;
+};
+
+Saved take_block(Area& a, const Stage& s, size_t M, bool keep) {
+  const size_t d = s.d;
+  Saved v;
+  v.ln1 = a.take<bf16>(M * d);
+  v.qkv = a.take<bf16>(M * 3 * d);
+  v.att = a.take<bf16>(M * d);
+  v.x1 = a.take<bf16>(M * d);
+  v.ln2 = a.take<bf16>(M * d);
+  v.h = keep ? a.take<bf16>(M * 4 * d) : nullptr;
+  v.g = a.take<bf16>(M * 4 * d);
+  v.out = a.take<bf16>(M * d);
+  v.mu1 = a.take<float>(M);
+  v.rs1 = a.take<float>(M);
+  v.mu2 = a.take<float>(M);
+  v.rs2 = a.take<float>(M);
+  v.lse = a.take<float>(M * s.nh);
+  return v;
+}
+
+// saved area of a microbatch: input embedding (first stage), blocks, final LayerNorm
+struct SavedAll {
+  bf16* x0;
+  std::vector<Saved> blk;
+  bf16* lnf;
+  float *muf, *rsf;
+};
+
+SavedAll take_saved(Area& a, const Stage& s, size_t M, bool keep) {
+  SavedAll v;
+  v.x0 = s.wte ? a.take<bf16>(M * s.d) : nullptr;
+  v.blk.resize(s.n);
+  if (keep) {
+    for (int l = 0; l < s.n; ++l) v.blk[l] = take_block(a, s, M, true);
+  } else {
+    // without a backward two sets of block buffers take turns (a block reads the one before's output)
+    Saved two[2] = {take_block(a, s, M, false), take_block(a, s, M, false)};
+    for (int l = 0; l < s.n; ++l) v.blk[l] = two[l & 1];
+  }
+  v.lnf = s.head_w ? a.take<bf16>(M * s.d) : nullptr;
+  v.muf = s.head_w ? a.take<float>(M) : nullptr;
+  v.rsf = s.head_w ? a.take<float>(M) : nullptr;
+  return v;
+}
+
+struct Scratch {
+  bf16 *dh[2], *dx[3], *dx1[2], *dqkv[2], *dln, *datt, *logits;
+  float *dq_acc, *dvec, *ln;
+};
+
+// logit_rows: rows of the logits that exist at a time (0: the caller keeps them elsewhere)
+Scratch take_scratch(Area& a, const Stage& s, size_t M, bool grad, size_t logit_rows) {
+  const size_t d = s.d;
+  Scratch v = {};
+  v.logits = s.head_w && logit_rows ? a.take<bf16>(logit_rows * s.V) : nullptr;
+  if (!grad) return v;
+  for (int p = 0; p < 2; ++p) {
+    v.dh[p] = a.take<bf16>(M * 4 * d);
+    v.dx1[p] = a.take<bf16>(M * d);
+    v.dqkv[p] = a.take<bf16>(M * 3 * d);
+  }
+  for (int r = 0; r < 3; ++r) v.dx[r] = a.take<bf16>(M * d);
+  v.dln = a.take<bf16>(M * d);
+  v.datt = a.take<bf16>(M * d);
+  v.dq_acc = a.take<float>(M * d);
+  v.dvec = a.take<float>(M * s.nh);
+  v.ln = a.take<float>(size_t(dsw_layernorm_bwd_blocks(int(M))) * 3 * d);
+  return v;
+}
+
+size_t head_rows(size_t M, int chunks) {
+  if (chunks <= 1) return M;
+  size_t rows = (M + chunks - 1) / chunks;
+  rows = (rows + 255) / 256 * 256;          // whole GEMM tiles per slice
+  return rows < M ? rows : M;
+}
+
+// Return codes of a sequence of launches: the first failure is kept, nothing more is queued after it.
+#define TRY(call) do { const int rc_ = (call); if (rc_) return rc_; } while (0)
+#define LAUNCH(call) do { const int rc_ = (call); if (rc_) return rc_; g_launches.fetch_add(1, std::memory_order_relaxed); } while (0)
+#define TRY_CUDA(call) do { if ((call) != cudaSuccess) return -3; } while (0)
+
+struct Run {
+  Stage& s;
+  int B, T, M, deterministic;
+  cudaStream_t st;
+
+  int gemm(const void* A, const void* W, bool w_t, int N, int K, void* out, int mode, const float* bias, const void* resid,
+           void* aux_out, const void* aux_in, int rows) const {
+    // activations [rows, K] times W: [N, K] (w_t) or [K, N]
+    return dsw_gemm_bf16(A, K, 0, W, w_t ? K : N, w_t ? 0 : 1, rows, N, K, mode, 1, out, N, bias, resid, N, aux_out, aux_in, N,
+                         0, 0, s.status, st);
+  }
+  // dW[n_out, n_in] += dy[rows, n_out]^T x[rows, n_in] on the given stream
+  int wgrad(const void* dy, const void* x, int n_out, int n_in, float* dw, int rows, cudaStream_t on) const {
+    return dsw_gemm_bf16(dy, n_out, 1, x, n_in, 1, n_out, n_in, rows, DSW_EPI_ATOMIC_F32, deterministic ? 1 : 0 /* chosen by shape */, dw, n_in,
+                         nullptr, nullptr, 0, nullptr, nullptr, 0, 0, 0, s.status, on);
+  }
+  cudaStream_t side() const { return s.side ? s.side : st; }
+  // the side stream may use everything queued on the main stream so far
+  int fork() const {
+    if (!s.side) return 0;
+    TRY_CUDA(cudaEventRecord(s.fork, st));
+    TRY_CUDA(cudaStreamWaitEvent(s.side, s.fork, 0));
+    return 0;
+  }
+
+  // everything queued on the side stream by earlier calls is done before what follows on the main stream
+  int join() const {
+    for (int p = 0; p < 2; ++p)
+      if (s.side_used[p]) TRY_CUDA(cudaStreamWaitEvent(st, s.side_done[p], 0));
+    return 0;
+  }
+
+  int block_fwd(const Block& b, const bf16* x, const Saved& v, bf16* out) const {
+    const int d = s.d;
+    LAUNCH(dsw_layernorm_fwd(x, b.ln1_w, b.ln1_b, v.ln1, v.mu1, v.rs1, M, d, 1e-5f, st));
+    LAUNCH(gemm(v.ln1, b.w[W_QKV], true, 3 * d, d, v.qkv, DSW_EPI_STORE, b.b[W_QKV], nullptr, nullptr, nullptr, M));
+    LAUNCH(dsw_attention_fwd(v.qkv, v.att, v.lse, B, T, s.nh, d / s.nh, scale(), s.status, st));
+    LAUNCH(gemm(v.att, b.w[W_O], true, d, d, v.x1, DSW_EPI_RESID, b.b[W_O], x, nullptr, nullptr, M));
+    LAUNCH(dsw_layernorm_fwd(v.x1, b.ln2_w, b.ln2_b, v.ln2, v.mu2, v.rs2, M, d, 1e-5f, st));
+    // the GELU epilogue also emits gelu'(pre-activation) when there is a backward, which then only multiplies by it
+    LAUNCH(gemm(v.ln2, b.w[W_FC], true, 4 * d, d, v.g, DSW_EPI_GELU, b.b[W_FC], nullptr, v.h, nullptr, M));
+    LAUNCH(gemm(v.g, b.w[W_PR], true, d, 4 * d, out, DSW_EPI_RESID, b.b[W_PR], v.x1, nullptr, nullptr, M));
+    return 0;
+  }
+
+  int block_bwd(int l, const Block& b, const bf16* x, const Saved& v, const Scratch& c, const bf16* dx2, bf16* dx0) const {
+    const int d = s.d, p = l & 1;
+    if (s.side_used[p]) TRY_CUDA(cudaStreamWaitEvent(st, s.side_done[p], 0));
+    LAUNCH(gemm(dx2, b.w[W_PR], false, 4 * d, d, c.dh[p], DSW_EPI_MUL, nullptr, nullptr, nullptr, v.h, M));
+    TRY(fork());
+    LAUNCH(wgrad(dx2, v.g, d, 4 * d, b.dw[W_PR], M, side()));
+    LAUNCH(dsw_colsum_accum(c.dh[p], 4 * d, b.db[W_FC], M, 4 * d, side()));
+    LAUNCH(wgrad(c.dh[p], v.ln2, 4 * d, d, b.dw[W_FC], M, side()));
+    LAUNCH(gemm(c.dh[p], b.w[W_FC], false, d, 4 * d, c.dln, DSW_EPI_STORE, nullptr, nullptr, nullptr, nullptr, M));
+    // the column sum of dx2 (bias gradient of the MLP's second projection) rides along with the LayerNorm backward
+    LAUNCH(dsw_layernorm_bwd(c.dln, v.x1, b.ln2_w, v.mu2, v.rs2, dx2, c.dx1[p], b.dln2_w, b.dln2_b, b.db[W_PR], c.ln, M, d, st));
+    LAUNCH(gemm(c.dx1[p], b.w[W_O], false, d, d, c.datt, DSW_EPI_STORE, nullptr, nullptr, nullptr, nullptr, M));
+    TRY(fork());
+    LAUNCH(wgrad(c.dx1[p], v.att, d, d, b.dw[W_O], M, side()));
+    LAUNCH(dsw_attention_bwd(v.qkv, v.att, c.datt, v.lse, c.dqkv[p], c.dq_acc, c.dvec, B, T, s.nh, d / s.nh, scale(), s.status, st));
+    TRY(fork());
+    LAUNCH(dsw_colsum_accum(c.dqkv[p], 3 * d, b.db[W_QKV], M, 3 * d, side()));
+    LAUNCH(wgrad(c.dqkv[p], v.ln1, 3 * d, d, b.dw[W_QKV], M, side()));
+    if (s.side) {
+      TRY_CUDA(cudaEventRecord(s.side_done[p], s.side));
+      s.side_used[p] = true;
+    }
+    LAUNCH(gemm(c.dqkv[p], b.w[W_QKV], false, d, 3 * d, c.dln, DSW_EPI_STORE, nullptr, nullptr, nullptr, nullptr, M));
+    LAUNCH(dsw_layernorm_bwd(c.dln, x, b.ln1_w, v.mu1, v.rs1, c.dx1[p], dx0, b.dln1_w, b.dln1_b, b.db[W_O], c.ln, M, d, st));
+    return 0;
+  }
+
+  float scale() const { return 1.f / sqrtf(float(s.d / s.nh)); }
+};
+
+}  // namespace
+
+// desc: n, d, heads, V, status, side stream, wte, wpe, dwte, dwpe, lnf_w, lnf_b, dlnf_w, dlnf_b, head_w, dhead_w,
+// count, then per block ln1_w, ln1_b, dln1_w, dln1_b, ln2_w, ln2_b, dln2_w, dln2_b and for each of qkv, out, fc,
+// proj: w (bf16), b, dw, db.  Device pointers as integers; those of a part that the stage does not have are 0.
+extern "C" int dsw_stage_create(const long long* desc, int len, void** out) {
+  constexpr int HEAD = 17, PER_BLOCK = 24;
+  if (len < HEAD || desc[0] < 0 || len != HEAD + PER_BLOCK * desc[0] || desc[1] % 8 || desc[1] > 2048 || desc[3] % 8) return -10;
+  Stage* s = new (std::nothrow) Stage();
+  if (!s) return -1;
+  const long long* p = desc;
+  s->n = int(*p++); s->d = int(*p++); s->nh = int(*p++); s->V = int(*p++);
+  s->status = reinterpret_cast<int*>(*p++);
+  s->side = reinterpret_cast<cudaStream_t>(*p++);
+  auto f = [&p] { return reinterpret_cast<float*>(*p++); };
+  s->wte = f(); s->wpe = f(); s->dwte = f(); s->dwpe = f();
+  s->lnf_w = f(); s->lnf_b = f(); s->dlnf_w = f(); s->dlnf_b = f();
+  s->head_w = reinterpret_cast<const bf16*>(*p++);
+  s->dhead_w = f(); s->count = f();
+  for (int l = 0; l < s->n; ++l) {
+    Block b;
+    b.ln1_w = f(); b.ln1_b = f(); b.dln1_w = f(); b.dln1_b = f();
+    b.ln2_w = f(); b.ln2_b = f(); b.dln2_w = f(); b.dln2_b = f();
+    for (int k = 0; k < 4; ++k) {
+      b.w[k] = reinterpret_cast<const bf16*>(*p++);
+      b.b[k] = f(); b.dw[k] = f(); b.db[k] = f();
+    }
+    s->blocks.push_back(b);
+  }
+  bool ok = cudaEventCreateWithFlags(&s->fork, cudaEventDisableTiming) == cudaSuccess &&
+            cudaEventCreateWithFlags(&s->head_done, cudaEventDisableTiming) == cudaSuccess;
+  for (int i = 0; i < 2; ++i) ok = ok && cudaEventCreateWithFlags(&s->side_done[i], cudaEventDisableTiming) == cudaSuccess;
+  if (!ok) { delete s; return -2; }
+  *out = s;
+  return 0;
+}
+
+extern "C" int dsw_stage_destroy(void* stage) {
+  Stage* s = static_cast<Stage*>(stage);
+  if (!s) return 0;
+  cudaEventDestroy(s->fork);
+  cudaEventDestroy(s->head_done);
+  for (int i = 0; i < 2; ++i) cudaEventDestroy(s->side_done[i]);
+  delete s;
+  return 0;
+}
+
+// Launcher calls made by the executor since the library was loaded.
+extern "C" int dsw_stage_launches() { return g_launches.load(std::memory_order_relaxed); }
+
+// Bytes of the two work areas of a microbatch of B sequences of T tokens.  keep: a backward will follow; grad: the
+// scratch serves a backward too; chunks: slices of the LM head (0: no logits in the scratch).
+extern "C" int dsw_stage_sizes(void* stage, int B, int T, int keep, int grad, int chunks, size_t* saved, size_t* scratch) {
+  const Stage& s = *static_cast<Stage*>(stage);
+  if (B <= 0 || T <= 0) return -10;
+  const size_t M = size_t(B) * T;
+  Area a(nullptr), c(nullptr);
+  take_saved(a, s, M, keep != 0);
+  take_scratch(c, s, M, grad != 0, chunks > 0 ? head_rows(M, chunks) : 0);
+  *saved = a.used;
+  *scratch = c.used;
+  return 0;
+}
+
+// Embedding (ids) or a hidden state (x) through the stage's blocks; y (bf16 [B*T, d]) is the last block's output, by
+// default a place in `saved`.  infer_logits (fp32 [B*T, V]): also the final LayerNorm and the LM head.
+extern "C" int dsw_stage_forward(void* stage, const long long* ids, const void* x, void* saved, void* y,
+                                 float* infer_logits, int B, int T, int keep, cudaStream_t st) {
+  Stage& s = *static_cast<Stage*>(stage);
+  if (B <= 0 || T <= 0 || (s.wte ? ids == nullptr : x == nullptr)) return -10;
+  std::lock_guard<std::mutex> lock(s.mu);
+  const Run r{s, B, T, B * T, 0, st};
+  Area a(saved);
+  const SavedAll v = take_saved(a, s, size_t(B) * T, keep != 0);
+  const bf16* in = static_cast<const bf16*>(x);
+  if (s.wte) {
+    LAUNCH(dsw_embedding_fwd(ids, s.wte, s.wpe, v.x0, B, T, s.d, s.V, s.status, st));
+    in = v.x0;
+  }
+  for (int l = 0; l < s.n; ++l) {
+    bf16* out = l + 1 == s.n && y ? static_cast<bf16*>(y) : v.blk[l].out;
+    TRY(r.block_fwd(s.blocks[l], in, v.blk[l], out));
+    in = out;
+  }
+  if (infer_logits) {
+    LAUNCH(dsw_layernorm_fwd(in, s.lnf_w, s.lnf_b, v.lnf, v.muf, v.rsf, r.M, s.d, 1e-5f, st));
+    LAUNCH(dsw_gemm_bf16(v.lnf, s.d, 0, s.head_w, s.d, 0, r.M, s.V, s.d, DSW_EPI_STORE_F32, 1, infer_logits, s.V, nullptr,
+                      nullptr, 0, nullptr, nullptr, 0, 0, 0, s.status, st));
+  }
+  return 0;
+}
+
+// Final LayerNorm, LM head and masked mean cross-entropy of what dsw_stage_forward left in `saved` (loss[0] is
+// overwritten); with grad also the head's gradients, the gradient of the last block's output staying in the scratch
+// for dsw_stage_backward.  The logits exist one slice of rows at a time.
+extern "C" int dsw_stage_head(void* stage, void* saved, void* scratch, const long long* targets, const long long* mask,
+                              float scale, float* loss, int B, int T, int keep, int grad, int chunks, int deterministic,
+                              cudaStream_t st) {
+  Stage& s = *static_cast<Stage*>(stage);
+  if (B <= 0 || T <= 0 || !s.head_w || s.n < 1) return -10;
+  std::lock_guard<std::mutex> lock(s.mu);
+  const int M = B * T, d = s.d, V = s.V;
+  const Run r{s, B, T, M, deterministic, st};
+  Area a(saved), ca(scratch);
+  const SavedAll v = take_saved(a, s, M, keep != 0);
+  const int rows = int(head_rows(M, chunks));
+  const Scratch c = take_scratch(ca, s, M, grad != 0, rows);
+  const bf16* x = v.blk[s.n - 1].out;
+  TRY(r.join());           // an earlier call may have laid the scratch out differently
+  LAUNCH(dsw_loss_begin(mask, M, s.count, loss, st));
+  LAUNCH(dsw_layernorm_fwd(x, s.lnf_w, s.lnf_b, v.lnf, v.muf, v.rsf, M, d, 1e-5f, st));
+  for (int r0 = 0; r0 < M; r0 += rows) {
+    const int m = M - r0 < rows ? M - r0 : rows;
+    const bf16* ln = v.lnf + size_t(r0) * d;
+    if (s.head_used) TRY_CUDA(cudaStreamWaitEvent(st, s.head_done, 0));      // the slice before is still read
+    LAUNCH(r.gemm(ln, s.head_w, true, V, d, c.logits, DSW_EPI_STORE, nullptr, nullptr, nullptr, nullptr, m));
+    LAUNCH(dsw_cross_entropy(c.logits, V, targets + r0, mask ? mask + r0 : nullptr, s.count, scale, loss, m, V, grad, s.status, st));
+    if (!grad) continue;
+    TRY(r.fork());
+    LAUNCH(r.wgrad(c.logits, ln, V, d, s.dhead_w, m, r.side()));
+    if (s.side) {
+      TRY_CUDA(cudaEventRecord(s.head_done, s.side));
+      s.head_used = true;
+    }
+    LAUNCH(r.gemm(c.logits, s.head_w, false, d, V, c.dln + size_t(r0) * d, DSW_EPI_STORE, nullptr, nullptr, nullptr, nullptr, m));
+  }
+  if (grad)
+    LAUNCH(dsw_layernorm_bwd(c.dln, x, s.lnf_w, v.muf, v.rsf, nullptr, c.dx[s.n % 3], s.dlnf_w, s.dlnf_b, nullptr, c.ln, M, d, st));
+  return 0;
+}
+
+// Backward of the blocks hi-1 .. lo.  dy: gradient of block hi-1's output, or null for the one that dsw_stage_head or
+// the call for the blocks above left in the scratch.  x: the stage's input hidden state (null on the first stage).
+// dx0: where block 0 puts the input's gradient (bf16 [B*T, d]), null for a place in the scratch.  With ids, block 0 is
+// followed by the embedding's gradient.
+extern "C" int dsw_stage_backward(void* stage, int hi, int lo, const void* dy, const void* x, const long long* ids,
+                                  void* saved, void* scratch, void* dx0, int B, int T, int chunks, int deterministic,
+                                  cudaStream_t st) {
+  Stage& s = *static_cast<Stage*>(stage);
+  if (B <= 0 || T <= 0 || hi > s.n || lo < 0) return -10;
+  std::lock_guard<std::mutex> lock(s.mu);
+  const Run r{s, B, T, B * T, deterministic, st};
+  Area a(saved), ca(scratch);
+  const SavedAll v = take_saved(a, s, size_t(r.M), true);
+  const Scratch c = take_scratch(ca, s, size_t(r.M), true, chunks > 0 ? head_rows(size_t(r.M), chunks) : 0);
+  if (hi == s.n && dy) TRY(r.join());
+  const bf16* g = dy ? static_cast<const bf16*>(dy) : c.dx[hi % 3];
+  for (int l = hi - 1; l >= lo; --l) {
+    const bf16* in = l > 0 ? v.blk[l - 1].out : (s.wte ? v.x0 : static_cast<const bf16*>(x));
+    bf16* out = l == 0 && dx0 ? static_cast<bf16*>(dx0) : c.dx[l % 3];
+    TRY(r.block_bwd(l, s.blocks[l], in, v.blk[l], c, g, out));
+    g = out;
+  }
+  if (lo == 0 && ids) LAUNCH(dsw_embedding_bwd(ids, g, s.dwte, s.dwpe, B, T, s.d, s.V, st));
+  return 0;
+}

@@ -26,9 +26,10 @@ import torch
 import torch.distributed as dist
 
 from .gpt2 import GPT2Config, init_tensor, split_layers, stage_param_specs
+from .stage_exec import SavedArea, StageExec
 from ..ops import kernels as K
 from ..ops._lib import Status, load_all_kernels
-from ..ops.attention import attention_bwd, attention_fwd
+from ..ops.attention import attention_bwd, attention_fwd, native_available
 from ..parallel.collectives import GradSync, OuterSync, StageRendezvous, wait_cycles_for
 from ..parallel.symm import SymmetricBuffer
 
@@ -122,6 +123,7 @@ class B200Engine:
         self.buckets = self._make_buckets()
         self._buckets_sent = 0
         self._overlap = os.environ.get("DSWARM_GRAD_OVERLAP", "1") != "0"
+        self.exec = self._make_exec()
         self._canary_every_step = os.environ.get("DSWARM_CANARY_CHECK", "0") == "1"
 
     # ------------------------------------------------------------------ views
@@ -162,6 +164,25 @@ class B200Engine:
             self.dlnf_w, self.dlnf_b = self.g32("transformer.ln_f.weight"), self.g32("transformer.ln_f.bias")
             hk = "lm_head.weight" if "lm_head.weight" in self.offsets else "transformer.wte.weight"
             self.head_w, self.dhead_w = self.p16(hk), self.g32(hk)
+
+    def _make_exec(self) -> Optional[StageExec]:
+        """The native executor of this stage's passes, for the shapes its kernels cover (a head size that the
+        attention kernels have, a width of at most 2048); other stages run launch by launch from here."""
+        c = self.cfg
+        if not native_available(c.n_embd // c.n_head) or c.n_embd > 2048 or c.n_embd % c.n_head or not self.blocks:
+            return None
+        g = lambda name: getattr(self, name, None)
+        ends = [g("wte"), g("wpe"), g("dwte"), g("dwpe"), g("lnf_w"), g("lnf_b"), g("dlnf_w"), g("dlnf_b"),
+                g("head_w"), g("dhead_w"), self.count_buf]
+        blocks = []
+        for b in self.blocks:
+            t = [getattr(b, p + ln + s) for ln in ("ln1", "ln2") for p in ("", "d") for s in ("_w", "_b")]
+            t += [getattr(b, f"{p}{m}{s}") for m in ("qkv", "o", "fc", "pr") for p in ("", "d") for s in ("_w", "_b")]
+            blocks.append(t)
+        return StageExec(len(blocks), c.n_embd, c.n_head, c.vocab_size, self.status, self.side, ends, blocks, self.device)
+
+    def _native(self) -> bool:
+        return self.exec is not None and native_available(self.cfg.n_embd // self.cfg.n_head)
 
     # ------------------------------------------------------------------ small API
     def train(self):
@@ -370,8 +391,63 @@ class B200Engine:
             return None
         return dx.view(B, T, -1)
 
+    # ------------------------------------------------------------------ the same passes through the native executor
+    def _input(self, input_ids, hidden):
+        """(ids, hidden state, B, T) as the kernels read them."""
+        if self.is_first:
+            B, T = input_ids.shape
+            return input_ids.contiguous(), None, B, T
+        B, T = hidden.shape[0], hidden.shape[1]
+        x = hidden if hidden.dtype == BF16 else hidden.to(BF16)
+        return None, x.contiguous(), B, T
+
+    def _exec_head(self, saved, scratch, targets, mask, scale: float, loss, B: int, T: int, grad: bool, st) -> None:
+        tg = targets.reshape(-1).contiguous()
+        mk = mask.reshape(-1).contiguous() if mask is not None else None
+        assert tg.dtype == torch.long and tg.numel() == B * T
+        assert mk is None or (mk.dtype == torch.long and mk.numel() == B * T)
+        self.exec.head(saved, scratch, tg, mk, scale, loss, B, T, grad, grad, self.head_chunks, st)
+
+    def _exec_backward(self, area: SavedArea, dy, ids, x, B: int, T: int, sync: bool, chunks: int, st
+                       ) -> Optional[torch.Tensor]:
+        """Backward of the blocks (and the embedding) behind ``dy``, or behind what the head left in the scratch;
+        gradient buckets are sent as they are completed when ``sync``."""
+        ex, n = self.exec, len(self.blocks)
+        scratch = ex.area("scratch", ex.sizes(B, T, True, True, chunks)[1], st)
+        dx0 = None if self.is_first and not K.deterministic() else torch.empty(B, T, ex.d, dtype=BF16, device=self.device)
+        emb = ids if dx0 is None else None
+        if sync and self.is_last:
+            self._side_dirty = True
+            self._send_bucket()                       # final LayerNorm + LM head
+        for hi, lo in [(l + 1, l) for l in reversed(range(n))] if sync else [(n, 0)]:
+            last = lo == 0
+            ex.backward(hi, lo, dy if hi == n else None, x, emb if last and not sync else None, area.buf, scratch,
+                        dx0 if last else None, B, T, chunks, st)
+            self._side_dirty = self.side is not None
+            if sync:
+                self._send_bucket()
+        if sync and emb is not None:
+            ex.backward(0, 0, None, x, emb, area.buf, scratch, None, B, T, chunks, st)
+        elif self.is_first and emb is None:
+            K.embedding_bwd(ids, dx0.view(B * T, -1), self.dwte, self.dwpe)
+            dx0 = None
+        if sync and self.is_first:
+            self._send_bucket()
+        ex.give(area, st)
+        return dx0
+
     # ------------------------------------------------------------------ engine API
     def forward(self, key: int, input_ids, hidden, keep: bool = True) -> torch.Tensor:
+        if self._native():
+            ex, st = self.exec, torch.cuda.current_stream()
+            ids, x, B, T = self._input(input_ids, hidden)
+            nbytes = ex.sizes(B, T, keep, False, 0)[0]
+            area = ex.take(nbytes, st) if keep else None
+            y = torch.empty(B, T, ex.d, dtype=BF16, device=self.device)
+            ex.forward(ids, x, area.buf if keep else ex.area("saved", nbytes, st), y, None, B, T, keep, st)
+            if keep:
+                self.stash[key] = {"area": area, "ids": ids, "x": x, "B": B, "T": T}
+            return y
         x, saved, B, T = self._body_fwd(input_ids, hidden, keep)
         if keep:
             self.stash[key] = {"saved": saved, "ids": input_ids, "B": B, "T": T}
@@ -383,6 +459,12 @@ class B200Engine:
         dx = grad_out.reshape(B * T, -1)
         if dx.dtype != BF16:
             dx = dx.to(BF16)
+        if "area" in s:
+            dx = dx.contiguous()
+            if self.side is not None:
+                dx.record_stream(self.side)           # the last block's weight gradient reads it there
+            return self._exec_backward(s["area"], dx, s["ids"], s["x"], B, T, self._want_overlap(sync), 0,
+                                       torch.cuda.current_stream())
         return self._body_bwd(s["saved"], dx.contiguous(), s["ids"], B, T, sync=self._want_overlap(sync))
 
     def _want_overlap(self, sync: bool) -> bool:
@@ -425,6 +507,15 @@ class B200Engine:
         return loss, lnf, mu, rs, dlnf
 
     def forward_backward(self, key: int, input_ids, hidden, targets, mask, scale: float, sync: bool = False):
+        if self._native():
+            ex, st, chunks = self.exec, torch.cuda.current_stream(), self.head_chunks
+            ids, x, B, T = self._input(input_ids, hidden)
+            saved_bytes, scratch_bytes = ex.sizes(B, T, True, True, chunks)
+            area = ex.take(saved_bytes, st)
+            loss = torch.empty((), dtype=F32, device=self.device)
+            ex.forward(ids, x, area.buf, None, None, B, T, True, st)
+            self._exec_head(area.buf, ex.area("scratch", scratch_bytes, st), targets, mask, scale, loss, B, T, True, st)
+            return loss, self._exec_backward(area, None, ids, x, B, T, self._want_overlap(sync), chunks, st)
         x, saved, B, T = self._body_fwd(input_ids, hidden, True)
         if self.head_chunks > 1:
             loss, lnf, mu, rs, dlnf = self._head_chunked(x, targets, mask, scale, grad=True)
@@ -441,6 +532,15 @@ class B200Engine:
 
     @torch.no_grad()
     def forward_loss(self, input_ids, hidden, targets, mask, scale: float) -> torch.Tensor:
+        if self._native():
+            ex, st = self.exec, torch.cuda.current_stream()
+            ids, x, B, T = self._input(input_ids, hidden)
+            saved_bytes, scratch_bytes = ex.sizes(B, T, False, False, self.head_chunks)
+            saved = ex.area("saved", saved_bytes, st)
+            loss = torch.empty((), dtype=F32, device=self.device)
+            ex.forward(ids, x, saved, None, None, B, T, False, st)
+            self._exec_head(saved, ex.area("scratch", scratch_bytes, st), targets, mask, scale, loss, B, T, False, st)
+            return loss
         x, _, _, _ = self._body_fwd(input_ids, hidden, False)
         if self.head_chunks > 1:
             return self._head_chunked(x, targets, mask, scale, grad=False)[0]
@@ -449,6 +549,17 @@ class B200Engine:
 
     @torch.no_grad()
     def forward_infer(self, input_ids, hidden) -> torch.Tensor:
+        if self._native():
+            ex, st = self.exec, torch.cuda.current_stream()
+            ids, x, B, T = self._input(input_ids, hidden)
+            saved = ex.area("saved", ex.sizes(B, T, False, False, 0)[0], st)
+            if self.is_last:          # the LM head's fp32 accumulators are the result
+                logits = torch.empty(B, T, self.cfg.vocab_size, dtype=F32, device=self.device)
+                ex.forward(ids, x, saved, None, logits, B, T, False, st)
+                return logits
+            y = torch.empty(B, T, ex.d, dtype=BF16, device=self.device)
+            ex.forward(ids, x, saved, y, None, B, T, False, st)
+            return y.float()
         x, _, B, T = self._body_fwd(input_ids, hidden, False)
         if self.is_last:
             lnf, _, _ = K.layernorm_fwd(x, self.lnf_w, self.lnf_b)

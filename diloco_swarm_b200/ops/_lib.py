@@ -31,6 +31,7 @@ _SIGS = {
     "dsw_embedding_bwd": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
     "dsw_embedding_bwd_sorted": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
     "dsw_mask_count": [c_void_p, c_int, c_void_p, c_void_p],
+    "dsw_loss_begin": [c_void_p, c_int, c_void_p, c_void_p, c_void_p],
     "dsw_cross_entropy": [c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_int, c_int, c_int,
                           c_void_p, c_void_p],
     "dsw_cast_f32_bf16": [c_void_p, c_void_p, c_ll, c_void_p],
@@ -40,6 +41,15 @@ _SIGS = {
     "dsw_adamw": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_ll, c_float, c_float, c_float, c_float, c_float,
                   c_int, c_void_p, c_int, c_void_p],
     "dsw_sgd": [c_void_p, c_void_p, c_void_p, c_void_p, c_ll, c_float, c_float, c_int, c_void_p, c_int, c_void_p],
+    "dsw_stage_create": [c_void_p, c_int, ctypes.POINTER(c_void_p)],
+    "dsw_stage_destroy": [c_void_p],
+    "dsw_stage_launches": [],
+    "dsw_stage_sizes": [c_void_p, c_int, c_int, c_int, c_int, c_int, ctypes.POINTER(c_size_t), ctypes.POINTER(c_size_t)],
+    "dsw_stage_forward": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
+    "dsw_stage_head": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_int, c_int, c_int, c_int,
+                       c_int, c_int, c_void_p],
+    "dsw_stage_backward": [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
+                           c_int, c_int, c_int, c_void_p],
     "dsw_symm_alloc": [c_size_t, ctypes.POINTER(c_void_p)],
     "dsw_symm_free": [c_void_p],
     "dsw_symm_export": [c_void_p, c_void_p],
@@ -123,7 +133,8 @@ def check(rc: int, what: str) -> None:
 
 
 def launch_count() -> int:
-    return LAUNCHES
+    """Launcher calls from Python and those that the stage executor made itself."""
+    return LAUNCHES + cuda_lib().dsw_stage_launches()
 
 
 _STATUS_TEXT = {1: "an mbarrier wait ran out inside a kernel",
