@@ -27,6 +27,7 @@
 // right halves, and the epilogues write the first 32 columns only.
 #include <cuda.h>
 #include "ptx.cuh"
+#include "launch.h"
 #include "tmap.h"
 #include "dswarm.h"
 
@@ -165,6 +166,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, __nv_bfloat16
     // ------------------------------------------------------------ TMA producer
     if (lane == 0) {
       tma_prefetch_desc(&tmap_qkv);
+      pdl_wait();
       uint32_t g = 0, w = 0;
       bool ok = true;
       for (int r = 0; r < rounds && ok; ++r) {
@@ -185,6 +187,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, __nv_bfloat16
         }
         ++w;
       }
+      pdl_launch();
     }
   } else if (warp == 4) {
     // ------------------------------------------------------------ MMA issuer
@@ -447,6 +450,8 @@ attention_bwd_prep_kernel(const __nv_bfloat16* __restrict__ out, const __nv_bflo
   const int lane = threadIdx.x & 31;
   const int d = nh * hs, chunks = d >> 3, lanes_per_head = hs >> 3;
   const long long rows = (long long)B * T;
+  pdl_wait();
+  pdl_launch();
   const long long warps = ((long long)gridDim.x * blockDim.x) >> 5;
   for (long long row = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < rows; row += warps) {
     const int b = int(row / T), t = int(row - (long long)b * T);
@@ -476,6 +481,8 @@ attention_bwd_prep_kernel(const __nv_bfloat16* __restrict__ out, const __nv_bflo
 // dqkv[:, 0:d] = bf16(dq_acc)
 __global__ void __launch_bounds__(256)
 attention_dq_convert_kernel(const float* __restrict__ dq_acc, __nv_bfloat16* __restrict__ dqkv, long long rows, int d) {
+  pdl_wait();
+  pdl_launch();
   const int per_row = d / 8;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < rows * per_row;
        i += (long long)gridDim.x * blockDim.x) {
@@ -584,6 +591,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
     if (lane == 0) {
       tma_prefetch_desc(&tmap_qkv);
       tma_prefetch_desc(&tmap_do);
+      pdl_wait();
       uint32_t g = 0, w = 0;
       bool ok = true;
       for (int r = 0; r < rounds && ok; ++r) {
@@ -616,6 +624,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
         }
         ++w;
       }
+      pdl_launch();
     }
   } else if (warp == MMA_WARP) {
     // ------------------------------------------------------------ MMA issuer
@@ -770,6 +779,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
     uint8_t* sdq = smem + L::DQ_OFF + half * ATT_TILE_BYTES;     // this thread's half: [128 rows][32 fp32]
     uint32_t g = 0, w = 0;
     float lse_next = 0.f, D_next = 0.f;
+    pdl_wait();
     // dQ of global step gs: TMEM -> registers -> swizzled shared tile, which the reducer warp adds into the
     // fp32 dQ scratch.
     auto drain_dq = [&](uint32_t gs) -> bool {
@@ -986,9 +996,8 @@ extern "C" int dsw_attention_fwd(const void* qkv, void* out, float* lse, int B, 
   // persistent: two CTAs per SM walk the work items
   const int total = ((T + ATT_BQ - 1) / ATT_BQ) * B * nh;
   const int G = total < 2 * att_num_sms() ? total : 2 * att_num_sms();
-  attention_fwd_kernel<<<G, ATT_THREADS, AttSmem::TOTAL, st>>>(tm, (__nv_bfloat16*)out, lse, T, nh, B * nh, hs,
-                                                               scale * 1.4426950408889634f, status, g_att_trace);
-  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+  return launch(attention_fwd_kernel, G, ATT_THREADS, AttSmem::TOTAL, st, 1, tm, (__nv_bfloat16*)out, lse, T, nh, B * nh, hs,
+                scale * 1.4426950408889634f, status, g_att_trace) == cudaSuccess ? 0 : -3;
 }
 
 // qkv, out, dout as in the forward; lse from the forward.  dqkv: bf16 [B*T, 3*d] (all of it is written).
@@ -1024,16 +1033,20 @@ extern "C" int dsw_attention_bwd(const void* qkv, const void* out, const void* d
   {
     const long long want = (rows * 32 + 255) / 256;
     const int cap = att_num_sms() * 16;
-    attention_bwd_prep_kernel<<<(unsigned)(want < cap ? want : cap), 256, 0, st>>>(
-        (const __nv_bfloat16*)out, (const __nv_bfloat16*)dout, Dvec, dq_acc, B, T, nh, hs);
+    if (launch(attention_bwd_prep_kernel, (unsigned)(want < cap ? want : cap), 256, 0, st, 1, (const __nv_bfloat16*)out,
+               (const __nv_bfloat16*)dout, Dvec, dq_acc, B, T, nh, hs) != cudaSuccess)
+      return -3;
   }
   // persistent: one CTA per SM walks the work items
   const int total = ((T + ATT_BK - 1) / ATT_BK) * B * nh;
   const int G = total < att_num_sms() ? total : att_num_sms();
-  attention_bwd_kernel<<<G, ATT_BWD_THREADS, AttBwdSmem::TOTAL, st>>>(tq, tdo, tdq, tdkv, lse, Dvec, (__nv_bfloat16*)dqkv, T, nh,
-                                                                       B * nh, hs, scale, status, g_att_trace);
-  attention_dq_convert_kernel<<<148 * 4, 256, 0, st>>>(dq_acc, (__nv_bfloat16*)dqkv, (long long)B * T, d);
-  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+  if (launch(attention_bwd_kernel, G, ATT_BWD_THREADS, AttBwdSmem::TOTAL, st, 1, tq, tdo, tdq, tdkv, lse, Dvec,
+             (__nv_bfloat16*)dqkv, T, nh, B * nh, hs, scale, status, g_att_trace) != cudaSuccess)
+    return -3;
+  return launch(attention_dq_convert_kernel, 148 * 4, 256, 0, st, 1, dq_acc, (__nv_bfloat16*)dqkv, (long long)B * T, d) ==
+                 cudaSuccess
+             ? 0
+             : -3;
 }
 
 extern "C" int dsw_load_attention() {

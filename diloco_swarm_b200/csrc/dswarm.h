@@ -24,7 +24,7 @@
 // Epilogue modes of dsw_gemm_bf16.
 #define DSW_EPI_STORE 0       // out(bf16) = acc (+ bias)
 #define DSW_EPI_GELU 1        // out(bf16) = gelu(acc + bias), exact erf form; aux_out (bf16, optional) = gelu'(acc + bias)
-#define DSW_EPI_RESID 2       // out(bf16) = acc + bias + resid
+#define DSW_EPI_RESID 2       // out(bf16) = acc + bias + resid (+ aux_in); aux_out (bf16, optional) = the sum minus out
 #define DSW_EPI_MUL 3         // out(bf16) = acc * aux_in (with the aux_out of DSW_EPI_GELU: the GELU backward)
 #define DSW_EPI_ATOMIC_F32 4  // out(fp32) += acc, safe under split-K
 #define DSW_EPI_STORE_F32 5   // out(fp32) = acc
@@ -63,6 +63,9 @@ int dsw_attention_set_trace(long long* buf);
 // x, y: bf16 [M, d]; gamma, beta: fp32 [d]; mean, rstd: fp32 [M] (written).  d <= 2048.
 int dsw_layernorm_fwd(const void* x, const float* gamma, const float* beta, void* y, float* mean, float* rstd,
                       int M, int d, float eps, cudaStream_t st);
+// The same of x + x_lo (x_lo: bf16 like x, or null).
+int dsw_layernorm_fwd_lo(const void* x, const void* x_lo, const float* gamma, const float* beta, void* y, float* mean,
+                         float* rstd, int M, int d, float eps, cudaStream_t st);
 // Number of blocks dsw_layernorm_bwd launches for M rows = rows of scratch it needs.
 int dsw_layernorm_bwd_blocks(int M);
 // dx = LayerNorm backward of dy (+ dres when given: the residual branch's gradient).  dgamma, dbeta and the

@@ -9,6 +9,7 @@
 // accesses and keeps statistics in fp32.
 #include "ptx.cuh"
 #include "dswarm.h"
+#include "launch.h"
 
 namespace dsw {
 
@@ -70,15 +71,15 @@ __device__ __forceinline__ void ln_load_row(uint4 (&o)[NCH], const __nv_bfloat16
   }
 }
 
-template <int NCH>
+// LO: the row is the sum of two bf16 arrays (a residual stream kept with the bits that rounding to bf16 leaves over).
+template <int NCH, bool LO>
 __global__ void __launch_bounds__(256)
-layernorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ gamma,
+layernorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ x_lo, const float* __restrict__ gamma,
                      const float* __restrict__ beta, __nv_bfloat16* __restrict__ y, float* __restrict__ mean_out,
                      float* __restrict__ rstd_out, int M, int d, float eps) {
   const int lane = threadIdx.x & 31;
   const int stride = gridDim.x * (blockDim.x >> 5);
   int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (row >= M) return;
   float g[NCH][8], b[NCH][8];
 #pragma unroll
   for (int c = 0; c < NCH; ++c) {
@@ -91,16 +92,30 @@ layernorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const float* __restric
     }
   }
   const float inv_d = 1.f / d;
+  if (row >= M) return;
+  pdl_wait();          // gamma and beta above are older than the kernel before
+  pdl_launch();
   uint4 cur[NCH], nxt[NCH];
   ln_load_row<NCH>(cur, x, row, d, lane, M);
   for (; row < M; row += stride) {
     const bool more = row + stride < M;
     if (more) ln_load_row<NCH>(nxt, x, row + stride, d, lane, M);
+    uint4 low[LO ? NCH : 1];
+    if constexpr (LO) ln_load_row<NCH>(low, x_lo, row, d, lane, M);
+    const auto value = [&](int c, float (&v)[8]) {       // a chunk of the row in fp32
+      unpack8(cur[c], v);                          // columns past d were loaded as zeros
+      if constexpr (LO) {
+        float t[8];
+        unpack8(low[c], t);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] += t[j];
+      }
+    };
     float s = 0.f;
 #pragma unroll
     for (int c = 0; c < NCH; ++c) {
       float v[8];
-      unpack8(cur[c], v);                          // columns past d were loaded as zeros
+      value(c, v);
 #pragma unroll
       for (int j = 0; j < 8; ++j) s += v[j];
     }
@@ -110,7 +125,7 @@ layernorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const float* __restric
     for (int c = 0; c < NCH; ++c) {
       if (c * 256 + lane * 8 < d) {
         float v[8];
-        unpack8(cur[c], v);
+        value(c, v);
 #pragma unroll
         for (int j = 0; j < 8; ++j) { const float t = v[j] - mean; q += t * t; }
       }
@@ -123,7 +138,7 @@ layernorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const float* __restric
       const int col = c * 256 + lane * 8;
       if (col < d && DSW_OK(row < M && col + 8 <= d)) {
         float v[8], o[8];
-        unpack8(cur[c], v);
+        value(c, v);
 #pragma unroll
         for (int j = 0; j < 8; ++j) o[j] = fmaf((v[j] - mean) * rstd, g[c][j], b[c][j]);
         store8(yr + col, o);
@@ -204,6 +219,8 @@ layernorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
     // gamma lives in registers next to the sums (read per row it was 12 of a 768-wide row's 24 memory instructions)
     if (REG_ACC && c * 256 + lane * 8 < d) load8f(gamma + c * 256 + lane * 8, gm[c]);
   }
+  pdl_wait();
+  pdl_launch();
   const int stride = gridDim.x * LN_BWD_WARPS;
   int row = blockIdx.x * LN_BWD_WARPS + warp;
   LnBwdRow<LN_MAX_CHUNKS> cur, nxt;
@@ -320,6 +337,8 @@ __global__ void __launch_bounds__(1024)
 layernorm_bwd_finish_kernel(const float* __restrict__ partial, int nblocks, int d, float* __restrict__ dgamma,
                             float* __restrict__ dbeta, float* __restrict__ dres_sum) {
   __shared__ float sh[32][33];
+  pdl_wait();
+  pdl_launch();
   const int i = blockIdx.x * 32 + threadIdx.x;          // index into [3][d]
   float s = 0.f;
   if (i < 3 * d)
@@ -341,6 +360,8 @@ layernorm_bwd_finish_kernel(const float* __restrict__ partial, int nblocks, int 
 __global__ void __launch_bounds__(256)
 colsum_kernel(const __nv_bfloat16* __restrict__ x, long long ld, float* __restrict__ out, int M, int N) {
   __shared__ float sh[8][256];
+  pdl_wait();
+  pdl_launch();
   const int cg = threadIdx.x & 31, rl = threadIdx.x >> 5;
   const int col = blockIdx.x * 256 + cg * 8;
   float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -385,6 +406,8 @@ __global__ void __launch_bounds__(256)
 embedding_fwd_kernel(const long long* __restrict__ ids, const float* __restrict__ wte,
                      const float* __restrict__ wpe, __nv_bfloat16* __restrict__ y, int BT, int T, int d, int V,
                      int* status) {
+  pdl_wait();
+  pdl_launch();
   const int per_row = d / 8;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (long long)BT * per_row;
        i += (long long)gridDim.x * blockDim.x) {
@@ -404,6 +427,8 @@ embedding_fwd_kernel(const long long* __restrict__ ids, const float* __restrict_
 __global__ void __launch_bounds__(256)
 embedding_bwd_kernel(const long long* __restrict__ ids, const __nv_bfloat16* __restrict__ dx,
                      float* __restrict__ dwte, float* __restrict__ dwpe, int B, int T, int d, int V) {
+  pdl_wait();
+  pdl_launch();
   const int per_row = d / 8;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (long long)T * per_row;
        i += (long long)gridDim.x * blockDim.x) {
@@ -497,6 +522,8 @@ __global__ void mask_count_kernel(const long long* __restrict__ mask, int M, flo
 __global__ void __launch_bounds__(1024)
 loss_begin_kernel(const long long* __restrict__ mask, int M, float* __restrict__ count, float* __restrict__ loss) {
   __shared__ int sh[32];
+  pdl_wait();
+  pdl_launch();
   int c = 0;
   if (mask) {
     for (int i0 = threadIdx.x; i0 < M; i0 += 8 * 1024) {
@@ -527,6 +554,8 @@ cross_entropy_kernel(__nv_bfloat16* __restrict__ logits, long long ld, const lon
                      const long long* __restrict__ mask, const float* __restrict__ count, float scale,
                      float* __restrict__ loss_acc, int M, int V, int write_grad, int* status) {
   __shared__ float shm[16], shs[16];
+  pdl_wait();
+  pdl_launch();
   const int row = blockIdx.x;
   if (row >= M) return;
   __nv_bfloat16* lr = logits + (long long)row * ld;
@@ -639,16 +668,26 @@ typedef __nv_bfloat16 bf16;
 
 extern "C" int dsw_layernorm_fwd(const void* x, const float* gamma, const float* beta, void* y, float* mean,
                                  float* rstd, int M, int d, float eps, cudaStream_t st) {
+  return dsw_layernorm_fwd_lo(x, nullptr, gamma, beta, y, mean, rstd, M, d, eps, st);
+}
+
+extern "C" int dsw_layernorm_fwd_lo(const void* x, const void* x_lo, const float* gamma, const float* beta, void* y, float* mean,
+                                 float* rstd, int M, int d, float eps, cudaStream_t st) {
   if (d % 8 || d > 256 * LN_MAX_CHUNKS_ALL) return -10;
   // two blocks per SM, several rows per warp when there are enough rows: gamma and beta are paid once per warp
   const int grid = grid_for(M, 16, 148 * 2);
-#define LN_FWD(NCH) layernorm_fwd_kernel<NCH><<<grid, 256, 0, st>>>((const bf16*)x, gamma, beta, (bf16*)y, mean, rstd, M, d, eps)
+  cudaError_t rc;
+#define LN_FWD(NCH)                                                                                                  \
+  rc = x_lo ? launch(layernorm_fwd_kernel<NCH, true>, grid, 256, 0, st, 1, (const bf16*)x, (const bf16*)x_lo, gamma, beta, \
+                     (bf16*)y, mean, rstd, M, d, eps)                                                                \
+            : launch(layernorm_fwd_kernel<NCH, false>, grid, 256, 0, st, 1, (const bf16*)x, (const bf16*)x_lo, gamma, beta, \
+                     (bf16*)y, mean, rstd, M, d, eps)
   switch ((d + 255) / 256) {
     case 1: LN_FWD(1); break; case 2: LN_FWD(2); break; case 3: LN_FWD(3); break; case 4: LN_FWD(4); break;
     case 5: LN_FWD(5); break; case 6: LN_FWD(6); break; case 7: LN_FWD(7); break; default: LN_FWD(8); break;
   }
 #undef LN_FWD
-  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+  return rc == cudaSuccess ? 0 : -3;
 }
 
 // Number of blocks dsw_layernorm_bwd launches for M rows = rows of scratch it needs.
@@ -669,6 +708,7 @@ extern "C" int dsw_layernorm_bwd(const void* dy, const void* x, const float* gam
   const size_t shmem = sizeof(float) * LN_BWD_WARPS * 3 * d;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -2;
+  cudaError_t rc;
 #define LN_BWD(NCH)                                                                                              \
   do {                                                                                                           \
     static bool attr[64] = {false};          /* the attribute is per device */                                 \
@@ -678,41 +718,39 @@ extern "C" int dsw_layernorm_bwd(const void* dy, const void* x, const float* gam
         return -2;                                                                                               \
       attr[dev] = true;                                                                                          \
     }                                                                                                            \
-    layernorm_bwd_kernel<NCH><<<grid, 32 * LN_BWD_WARPS, shmem, st>>>((const bf16*)dy, (const bf16*)x, gamma, mean, rstd, \
-                                                                     (const bf16*)dres, (bf16*)dx, scratch, M, d); \
+    rc = launch(layernorm_bwd_kernel<NCH>, grid, 32 * LN_BWD_WARPS, shmem, st, 1, (const bf16*)dy, (const bf16*)x, gamma, \
+                mean, rstd, (const bf16*)dres, (bf16*)dx, scratch, M, d);                                        \
   } while (0)
   switch ((d + 255) / 256) {
     case 1: LN_BWD(1); break; case 2: LN_BWD(2); break; case 3: LN_BWD(3); break; case 4: LN_BWD(4); break;
     case 5: LN_BWD(5); break; case 6: LN_BWD(6); break; case 7: LN_BWD(7); break; default: LN_BWD(8); break;
   }
 #undef LN_BWD
-  if (cudaGetLastError() != cudaSuccess) return -3;
-  layernorm_bwd_finish_kernel<<<(3 * d + 31) / 32, dim3(32, 32), 0, st>>>(scratch, grid, d, dgamma, dbeta,
-                                                                         want ? dres_sum : nullptr);
-  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+  if (rc != cudaSuccess) return -3;
+  return launch(layernorm_bwd_finish_kernel, (3 * d + 31) / 32, dim3(32, 32), 0, st, 1, scratch, grid, d, dgamma, dbeta,
+                want ? dres_sum : nullptr) == cudaSuccess
+             ? 0
+             : -3;
 }
 
 extern "C" int dsw_colsum_accum(const void* x, long long ld, float* out, int M, int N, cudaStream_t st) {
   if (N % 8 || ld % 8) return -10;
   dim3 grid((N + 255) / 256, M >= 4096 ? 128 : (M >= 256 ? 16 : 1));
-  colsum_kernel<<<grid, 256, 0, st>>>((const bf16*)x, ld, out, M, N);
-  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+  return launch(colsum_kernel, grid, 256, 0, st, 1, (const bf16*)x, ld, out, M, N) == cudaSuccess ? 0 : -3;
 }
 
 extern "C" int dsw_embedding_fwd(const long long* ids, const float* wte, const float* wpe, void* y, int B, int T,
                                  int d, int V, int* status, cudaStream_t st) {
   if (d % 8) return -10;
-  embedding_fwd_kernel<<<grid_for((long long)B * T * (d / 8), 256), 256, 0, st>>>(ids, wte, wpe, (bf16*)y, B * T, T, d,
-                                                                                V, status);
-  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+  return launch(embedding_fwd_kernel, grid_for((long long)B * T * (d / 8), 256), 256, 0, st, 1, ids, wte, wpe, (bf16*)y, B * T,
+                T, d, V, status) == cudaSuccess ? 0 : -3;
 }
 
 extern "C" int dsw_embedding_bwd(const long long* ids, const void* dx, float* dwte, float* dwpe, int B, int T, int d,
                                  int V, cudaStream_t st) {
   if (d % 8) return -10;
-  embedding_bwd_kernel<<<grid_for((long long)T * (d / 8), 256), 256, 0, st>>>(ids, (const bf16*)dx, dwte, dwpe, B, T, d,
-                                                                             V);
-  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+  return launch(embedding_bwd_kernel, grid_for((long long)T * (d / 8), 256), 256, 0, st, 1, ids, (const bf16*)dx, dwte, dwpe, B,
+                T, d, V) == cudaSuccess ? 0 : -3;
 }
 
 // Same result as dsw_embedding_bwd with a fixed order of additions: sorted / perm = stable ascending sort of the
@@ -735,17 +773,15 @@ extern "C" int dsw_mask_count(const long long* mask, int M, float* count, cudaSt
 }
 
 extern "C" int dsw_loss_begin(const long long* mask, int M, float* count, float* loss, cudaStream_t st) {
-  loss_begin_kernel<<<1, 1024, 0, st>>>(mask, M, count, loss);
-  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+  return launch(loss_begin_kernel, 1, 1024, 0, st, 1, mask, M, count, loss) == cudaSuccess ? 0 : -3;
 }
 
 extern "C" int dsw_cross_entropy(void* logits, long long ld, const long long* targets, const long long* mask,
                                  const float* count, float scale, float* loss_acc, int M, int V, int write_grad,
                                  int* status, cudaStream_t st) {
   if (V % 8 || ld % 8) return -10;
-  cross_entropy_kernel<<<M, 512, 0, st>>>((bf16*)logits, ld, targets, mask, count, scale, loss_acc, M, V, write_grad,
-                                          status);
-  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+  return launch(cross_entropy_kernel, M, 512, 0, st, 1, (bf16*)logits, ld, targets, mask, count, scale, loss_acc, M, V,
+                write_grad, status) == cudaSuccess ? 0 : -3;
 }
 
 extern "C" int dsw_cast_f32_bf16(const float* src, void* dst, long long n, cudaStream_t st) {
@@ -798,8 +834,8 @@ extern "C" int dsw_load_elementwise() {
   cudaFuncAttributes a;
   int bad = 0;
 #define L(f) bad |= cudaFuncGetAttributes(&a, f) != cudaSuccess
-  L(layernorm_fwd_kernel<1>); L(layernorm_fwd_kernel<2>); L(layernorm_fwd_kernel<3>); L(layernorm_fwd_kernel<4>);
-  L(layernorm_fwd_kernel<5>); L(layernorm_fwd_kernel<6>); L(layernorm_fwd_kernel<7>); L(layernorm_fwd_kernel<8>);
+  L((layernorm_fwd_kernel<1, false>)); L((layernorm_fwd_kernel<1, true>)); L((layernorm_fwd_kernel<2, false>)); L((layernorm_fwd_kernel<2, true>)); L((layernorm_fwd_kernel<3, false>)); L((layernorm_fwd_kernel<3, true>)); L((layernorm_fwd_kernel<4, false>)); L((layernorm_fwd_kernel<4, true>));
+  L((layernorm_fwd_kernel<5, false>)); L((layernorm_fwd_kernel<5, true>)); L((layernorm_fwd_kernel<6, false>)); L((layernorm_fwd_kernel<6, true>)); L((layernorm_fwd_kernel<7, false>)); L((layernorm_fwd_kernel<7, true>)); L((layernorm_fwd_kernel<8, false>)); L((layernorm_fwd_kernel<8, true>));
   L(layernorm_bwd_kernel<1>); L(layernorm_bwd_kernel<2>); L(layernorm_bwd_kernel<3>); L(layernorm_bwd_kernel<4>);
   L(layernorm_bwd_kernel<5>); L(layernorm_bwd_kernel<6>); L(layernorm_bwd_kernel<7>); L(layernorm_bwd_kernel<8>);
   L(layernorm_bwd_finish_kernel); L(colsum_kernel); L(embedding_fwd_kernel); L(embedding_bwd_kernel);

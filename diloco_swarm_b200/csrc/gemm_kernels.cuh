@@ -33,7 +33,7 @@ constexpr int GEMM_THREADS = 32 * (EPI_WARP0 + EPI_WARPS);
 enum EpiMode : int {
   EPI_STORE = 0,        // out = acc (+ bias)
   EPI_GELU = 1,         // out = gelu(acc + bias) ; aux_out (optional) = gelu'(acc + bias), what the backward multiplies by
-  EPI_RESID = 2,        // out = acc + bias + resid
+  EPI_RESID = 2,        // out = acc + bias + resid (+ aux_in); aux_out (optional) = what rounding out to bf16 left over
   EPI_MUL = 3,          // out = acc * aux_in  (aux_in = the gelu' saved by EPI_GELU: the GELU backward)
   EPI_ATOMIC_F32 = 4,   // out_f32 += acc   (split-K safe)
   EPI_STORE_F32 = 5,    // out_f32 = acc
@@ -49,6 +49,7 @@ struct GemmArgs {
   const __nv_bfloat16* resid; long long ldr;
   __nv_bfloat16* aux_out; const __nv_bfloat16* aux_in; long long ldaux;
   int* status;
+  int b_static;         // B is older than the kernel before in the stream (weights): it may be loaded before pdl_wait()
   long long* trace;     // optional: CTA 0's MMA thread stores %globaltimer stamps per k-block (tuning aid)
 };
 
@@ -189,10 +190,29 @@ __device__ __forceinline__ void epilogue_warp(const GemmArgs& g, uint32_t t_addr
         if constexpr (EXTRA) {
           uint32_t du[4] = {d.x, d.y, d.z, d.w};
           const uint32_t xu[4] = {x[i].x, x[i].y, x[i].z, x[i].w};
+          uint32_t lo[4] = {0, 0, 0, 0};
+          if constexpr (MODE == EPI_RESID) {
+            if (g.aux_in != nullptr) {
+              const uint4 t = *reinterpret_cast<const uint4*>(g.aux_in + (long long)row * g.ldaux + col);
+              lo[0] = t.x; lo[1] = t.y; lo[2] = t.z; lo[3] = t.w;
+            }
+          }
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
             const float2 a = unpack_bf16(du[q]), e = unpack_bf16(xu[q]);
-            du[q] = MODE == EPI_RESID ? pack_bf16(a.x + e.x, a.y + e.y) : pack_bf16(a.x * e.x, a.y * e.y);
+            if constexpr (MODE == EPI_RESID) {
+              const float2 t = unpack_bf16(lo[q]);
+              const float s0 = a.x + (e.x + t.x), s1 = a.y + (e.y + t.y);
+              du[q] = pack_bf16(s0, s1);
+              const float2 h = unpack_bf16(du[q]);
+              lo[q] = pack_bf16(s0 - h.x, s1 - h.y);
+            } else {
+              du[q] = pack_bf16(a.x * e.x, a.y * e.y);
+            }
+          }
+          if constexpr (MODE == EPI_RESID) {
+            if (g.aux_out != nullptr)
+              *reinterpret_cast<uint4*>(g.aux_out + (long long)row * g.ldaux + col) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
           }
           d = make_uint4(du[0], du[1], du[2], du[3]);
         }
@@ -298,6 +318,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     if (lane == 0) {
       tma_prefetch_desc(&tmap_a);
       tma_prefetch_desc(&tmap_b);
+      pdl_wait();
       uint32_t it = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
@@ -329,6 +350,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
           }
         }
       }
+      pdl_launch();
       if (!ok) {
         // give loads that are still in flight a bounded chance to land before the CTA exits
         for (int s = 0; s < NSTAGE; ++s) {
@@ -396,6 +418,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       const int rem = tile % (tiles_m * tiles_n);
       prefetch_extra<MODE, BN / 4>(g, (rem % tiles_m) * BM + q * 32, lane, (rem / tiles_m) * BN + part * (BN / 4));
     };
+    pdl_wait();
     prefetch_tile(blockIdx.x);
     for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++tcount) {
       const int ks = tile / (tiles_m * tiles_n);
@@ -506,6 +529,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     if (lane == 0) {
       tma_prefetch_desc(&tmap_a);
       tma_prefetch_desc(&tmap_b);
+      pdl_wait();
       uint32_t it = 0;
       bool ok = true;
       for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
@@ -541,6 +565,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           }
         }
       }
+      pdl_launch();
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader CTA only)
@@ -613,6 +638,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       prefetch_extra<MODE, BN / 4>(g, (rem % tiles_m) * 256 + int(rank) * 128 + q * 32, lane,
                                    (rem / tiles_m) * BN + part * (BN / 4));
     };
+    pdl_wait();
     prefetch_tile(pair);
     for (int tile = pair; tile < num_tiles && ok; tile += num_pairs, ++tcount) {
       const int ks = tile / (tiles_m * tiles_n);

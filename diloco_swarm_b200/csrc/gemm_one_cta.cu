@@ -2,6 +2,7 @@
 // 128 x 256 tiles, one instantiation per epilogue class.
 #include "gemm_kernels.cuh"
 #include "dswarm.h"
+#include "launch.h"
 
 namespace dsw {
 
@@ -24,8 +25,7 @@ int launch_one(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& g, 
   const int tiles = ((g.M + BM - 1) / BM) * ((g.N + BN - 1) / BN) * (g.split_k > 1 ? g.split_k : 1);
   int grid = tiles < num_sms ? tiles : num_sms;
   if (max_ctas > 0 && grid > max_ctas) grid = max_ctas;
-  gemm_kernel<BN, NSTAGE, MODE><<<grid, GEMM_THREADS, L::TOTAL, st>>>(ta, tb, g);
-  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+  return launch(gemm_kernel<BN, NSTAGE, MODE>, grid, GEMM_THREADS, L::TOTAL, st, 1, ta, tb, g) == cudaSuccess ? 0 : -3;
 }
 
 template <int BN, int NSTAGE>

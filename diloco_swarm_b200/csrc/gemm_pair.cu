@@ -2,6 +2,7 @@
 // two CTAs of a cluster (cta_group::2), one instantiation per epilogue class.
 #include "gemm_kernels.cuh"
 #include "dswarm.h"
+#include "launch.h"
 
 namespace dsw {
 
@@ -24,8 +25,7 @@ int launch_pair_mode(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArg
   int pairs = num_sms / 2;
   if (max_ctas > 0 && pairs > max_ctas / 2) pairs = max_ctas / 2 > 0 ? max_ctas / 2 : 1;
   if (pairs > tiles) pairs = tiles;
-  gemm_pair_kernel<MODE><<<2 * pairs, GEMM_THREADS, PairSmem::TOTAL, st>>>(ta, tb, g);
-  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+  return launch(gemm_pair_kernel<MODE>, 2 * pairs, GEMM_THREADS, PairSmem::TOTAL, st, 1, ta, tb, g) == cudaSuccess ? 0 : -3;
 }
 }  // namespace
 

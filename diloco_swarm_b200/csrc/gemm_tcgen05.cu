@@ -22,11 +22,14 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
-#include "gemm_kernels.cuh"
+#include "gemm_split.cuh"
+#include "launch.h"
 #include "tmap.h"
 #include "dswarm.h"
 
 namespace dsw {
+
+thread_local LaunchMode tl_launch;
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -157,6 +160,26 @@ static int pick_bn(int M, int N, int splits, int sms) {
   return e256 >= e128 * 0.93 ? 256 : 128;
 }
 
+// Few rows: tile width and split of K for the cluster kernel (gemm_split.cuh), or 0 where the kernels for many rows are
+// the better ones.  The cluster kernel has one tile per CTA and no overlap of epilogue and main loop, so it only comes
+// into question while all its CTAs fit on the SMs at once.  Times in ns, fitted to launches of 24 to 2128 rows (N and K
+// of GPT-2 small, weights cold in L2): a k-block takes its share of the load latency, which falls with the stages in
+// flight; partial sums leave a CTA at 18 bytes per ns; a thread stores one row of the CTA's columns.
+static int pick_few_rows(int M, int N, int K, bool b_mn, int sms, int* split) {
+  const int tm = (M + BM - 1) / BM, kb = (K + BK - 1) / BK;
+  const int waves = (tm * ((N + 127) / 128) + sms - 1) / sms;          // of the 128 x 128 kernel
+  double best = 1500.0 + 280.0 * waves * kb;
+  int bn = 0;
+  for (int w = b_mn ? 64 : 32; w <= 128; w *= 2)
+    for (int s = 1; s <= 8 && s <= kb && w / s >= 8; s *= 2) {
+      if ((long long)tm * ((N + w - 1) / w) * s > sms) continue;
+      const double per_kb = w == 32 ? 220.0 : w == 64 ? 280.0 : 300.0;
+      const double t = ((kb + s - 1) / s) * per_kb + (s > 1 ? 300.0 + 512.0 * w * (s - 1) / s / 18.0 : 0.0) + 25.0 * w / s;
+      if (t < best) { best = t; bn = w; *split = s; }
+    }
+  return bn;
+}
+
 // Split of K (tokens) for a weight gradient dW[M,N]: few output tiles, so K is split until the SMs are full.
 static int pick_wgrad_split(int M, int N, int K, int sms) {
   const bool pair = use_pair() && M >= 256;
@@ -196,16 +219,21 @@ extern "C" int dsw_gemm_bf16(const void* A, long long lda, int a_mn_major, const
   if ((lda | ldb | ldo) % 8 || N % 8 || (a_mn_major ? M % 8 : K % 8) || (b_mn_major ? N % 8 : K % 8)) return -10;
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(out)) & 15)
     return -11;
-  if (bn != 0 && bn != 128 && bn != 256 && bn != 512) return -12;   // 512 = CTA-pair kernel (256 x 256 per cluster)
+  bool few_rows = bn == 1032 || bn == 1064 || bn == 1128;      // the split-K cluster kernel, tile 32 / 64 / 128 wide
+  if (bn != 0 && bn != 128 && bn != 256 && bn != 512 && !few_rows) return -12;   // 512 = CTA-pair kernel (256 x 256 per cluster)
   if (mode < EPI_STORE || mode > EPI_STORE_F32) return -13;
   if ((mode == EPI_RESID && (resid == nullptr || ldr % 8)) || (mode == EPI_MUL && (aux_in == nullptr || ldaux % 8)) ||
-      (mode == EPI_GELU && aux_out != nullptr && ldaux % 8))
+      ((mode == EPI_GELU || mode == EPI_RESID) && (aux_out != nullptr || aux_in != nullptr) && ldaux % 8))
     return -10;
   static int num_sms[64] = {0};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -2;
   if (num_sms[dev] == 0) cudaDeviceGetAttribute(&num_sms[dev], cudaDevAttrMultiProcessorCount, dev);
   if (split_k == 0) split_k = mode == EPI_ATOMIC_F32 ? pick_wgrad_split(M, N, K, num_sms[dev]) : 1;
+  if (bn == 0 && split_k == 1 && mode <= EPI_MUL && !a_mn_major && max_ctas == 0 && default_max_ctas() == 0) {
+    bn = pick_few_rows(M, N, K, b_mn_major != 0, num_sms[dev], &split_k);
+    if (bn) { bn += 1000; few_rows = true; }
+  }
   if (bn == 0) bn = pick_bn(M, N, split_k, num_sms[dev]);
   if (max_ctas == 0) max_ctas = default_max_ctas();
   CUtensorMap ta, tb;
@@ -213,7 +241,7 @@ extern "C" int dsw_gemm_bf16(const void* A, long long lda, int a_mn_major, const
   if (!a_mn_major) rc = cached_tmap(&ta, TMAP_BF16_2D, A, K, 1, M, lda, BK, BM);
   else             rc = cached_tmap(&ta, TMAP_BF16_2D, A, M, 1, K, lda, 64, BK);
   if (rc) return rc;
-  if (!b_mn_major) rc = cached_tmap(&tb, TMAP_BF16_2D, B, K, 1, N, ldb, BK, bn == 512 ? 128 : bn);
+  if (!b_mn_major) rc = cached_tmap(&tb, TMAP_BF16_2D, B, K, 1, N, ldb, BK, bn == 512 ? 128 : bn % 1000);
   else             rc = cached_tmap(&tb, TMAP_BF16_2D, B, N, 1, K, ldb, 64, BK);
   if (rc) return rc;
   GemmArgs g;
@@ -225,10 +253,12 @@ extern "C" int dsw_gemm_bf16(const void* A, long long lda, int a_mn_major, const
   g.aux_out = reinterpret_cast<__nv_bfloat16*>(aux_out);
   g.aux_in = reinterpret_cast<const __nv_bfloat16*>(aux_in); g.ldaux = ldaux;
   g.status = status;
+  g.b_static = tl_launch.static_b;
   g.trace = g_gemm_trace;
+  if (few_rows) return launch_split(bn - 1000, ta, tb, g, stream);
   if (bn == 512) return launch_pair(ta, tb, g, num_sms[dev], max_ctas, stream);
   return launch_one_cta(bn, ta, tb, g, num_sms[dev], max_ctas, stream);
 }
 
 // Force the modules that hold the GEMM kernels to load now (see dsw_load_all).
-extern "C" int dsw_load_gemm() { return (load_one_cta_kernels() | load_pair_kernels()) ? -1 : 0; }
+extern "C" int dsw_load_gemm() { return (load_one_cta_kernels() | load_pair_kernels() | load_split_kernels()) ? -1 : 0; }

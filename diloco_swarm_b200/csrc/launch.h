@@ -1,0 +1,47 @@
+// Launch helper: clusters and programmatic dependent launch.
+//
+// A kernel that is launched with `pdl` may start while its predecessor in the stream is still running, once every CTA
+// of the predecessor has called pdl_launch() or has ended; it sets itself up (barriers, tensor memory, parameters) and
+// touches nothing that the predecessor writes before pdl_wait(), which returns when the predecessor has completed and
+// its writes are visible.  Two rules keep that safe along a whole chain of launches.  Every kernel of the library calls
+// pdl_wait() before its first access to activations, so completion is transitive.  No kernel calls pdl_launch() before
+// its own pdl_wait(), so when a kernel starts, everything before its predecessor has completed: what was written two
+// launches back (weights, by an optimiser step of an earlier pass) may be read before pdl_wait().
+#pragma once
+#include <cuda_runtime.h>
+
+namespace dsw {
+
+// How the calling thread wants its next launches: set by the stage executor, all off for calls from elsewhere.
+struct LaunchMode {
+  bool pdl = false;           // the predecessor in the stream is a kernel of this library and nothing lies in between
+  bool static_b = false;      // a GEMM's B operand (the weights) is older than the predecessor
+};
+extern thread_local LaunchMode tl_launch;
+
+template <class... P, class... A>
+inline cudaError_t launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, int cluster, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  int n = 0;
+  if (cluster > 1) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = cluster;
+    attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+    ++n;
+  }
+  if (tl_launch.pdl) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n].val.programmaticStreamSerializationAllowed = 1;
+    ++n;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = n;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+}  // namespace dsw

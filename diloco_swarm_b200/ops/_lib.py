@@ -23,6 +23,8 @@ _SIGS = {
     "dsw_gemm_bf16": [c_void_p, c_ll, c_int, c_void_p, c_ll, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_ll,
                       c_void_p, c_void_p, c_ll, c_void_p, c_void_p, c_ll, c_int, c_int, c_void_p, c_void_p],
     "dsw_layernorm_fwd": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float, c_void_p],
+    "dsw_layernorm_fwd_lo": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float,
+                             c_void_p],
     "dsw_layernorm_bwd": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                           c_void_p, c_void_p, c_int, c_int, c_void_p],
     "dsw_layernorm_bwd_blocks": [c_int],

@@ -56,7 +56,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool = Tru
         assert resid is not None and resid.shape == (M, N) and resid.dtype == BF16
     if bias is not None:
         assert bias.dtype == F32 and bias.numel() == N
-    if split_k > 1:
+    if split_k > 1 and bn < 1000:
         assert mode == EPI_ATOMIC_F32, "split-K needs the accumulating epilogue"
         kb_total = math.ceil(K / 64)
         per = math.ceil(kb_total / min(split_k, kb_total))
