@@ -60,3 +60,28 @@ def test_inference_logits_match_the_loss_path():
     ref = et.model(input_ids=ids).float()
     assert out.dtype == torch.float32 and out.shape == ref.shape
     assert (out - ref).abs().max() < 3e-2 * ref.abs().max()
+
+
+def test_replayed_passes_equal_the_queued_ones():
+    """The same microbatch three times (queued, captured, replayed), with other inputs in between and from another
+    stream: loss, logits and gradients stay the same."""
+    cfg, eng, _ = _engines()
+    a, b = _batch(cfg, B=3, T=50, seed=1), _batch(cfg, B=3, T=50, seed=2)
+    seen = []
+    side = torch.cuda.Stream()
+    for i in range(5):
+        if i == 3:
+            side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side if i >= 3 else torch.cuda.current_stream()):
+            ids, tg, mask = (t.clone() for t in a)              # the caller's tensors lie elsewhere every time
+            eng.grad.zero_()
+            loss, _ = eng.forward_backward(0, ids, None, tg, mask, 0.5)
+            eng._join()
+            out = eng.forward_infer(ids, None)
+            seen.append((loss, out, eng.grad.clone()))
+            eng.forward_backward(0, b[0], None, b[1], b[2], 0.5)
+    torch.cuda.synchronize()
+    eng.check_status()
+    for loss, out, grad in seen[1:]:
+        assert abs(loss.item() - seen[0][0].item()) < 1e-5 and torch.equal(out, seen[0][1])
+        assert torch.allclose(grad, seen[0][2], rtol=1e-3, atol=1e-5 * seen[0][2].abs().max().item())
