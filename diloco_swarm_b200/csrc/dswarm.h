@@ -37,8 +37,9 @@ extern "C" {
 // out[M,N] = A * B^T-or-B with fp32 accumulation on the tcgen05 tensor cores.
 // A: [M,K] row-major (a_mn_major = 0) or [K,M] row-major (1); B: [N,K] (b_mn_major = 0) or [K,N] (1);
 // lda/ldb/ldo/ldr/ldaux are row pitches in elements.  bn = 128 or 256 picks the one-CTA tile width,
-// 512 the CTA-pair kernel (256 x 256 per pair), 0 leaves the choice to the library.  split_k > 1 only with
-// DSW_EPI_ATOMIC_F32 (0: chosen by the library).
+// 384 / 512 the CTA-pair kernel (256 x 128 / 256 x 256 per pair), 1032 / 1064 / 1128 the kernel for few rows (tiles 32 /
+// 64 / 128 wide, split_k = CTAs that share a tile's K), 0 leaves the choice to the library.  Elsewhere split_k > 1 only
+// with DSW_EPI_ATOMIC_F32 (0: chosen by the library).
 // max_ctas > 0 caps the grid.
 int dsw_gemm_bf16(const void* A, long long lda, int a_mn_major, const void* B, long long ldb, int b_mn_major,
                   int M, int N, int K, int mode, int split_k, void* out, long long ldo, const float* bias,

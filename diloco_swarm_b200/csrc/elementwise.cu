@@ -642,6 +642,8 @@ cross_entropy_kernel(__nv_bfloat16* __restrict__ logits, long long ld, const lon
 
 // ------------------------------------------------------------------ casts
 __global__ void cast_f32_bf16_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, long long n) {
+  pdl_wait();
+  pdl_launch();
   const long long n8 = n / 8;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n8; i += (long long)gridDim.x * blockDim.x) {
     if (!DSW_OK(i * 8 + 8 <= n)) continue;
@@ -785,8 +787,7 @@ extern "C" int dsw_cross_entropy(void* logits, long long ld, const long long* ta
 }
 
 extern "C" int dsw_cast_f32_bf16(const float* src, void* dst, long long n, cudaStream_t st) {
-  cast_f32_bf16_kernel<<<grid_for(n / 8 + 1, 256), 256, 0, st>>>(src, (bf16*)dst, n);
-  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+  return launch(cast_f32_bf16_kernel, grid_for(n / 8 + 1, 256), 256, 0, st, 1, src, (bf16*)dst, n) == cudaSuccess ? 0 : -3;
 }
 extern "C" int dsw_cast_bf16_f32(const void* src, float* dst, long long n, cudaStream_t st) {
   cast_bf16_f32_kernel<<<grid_for(n, 256), 256, 0, st>>>((const bf16*)src, dst, n);

@@ -314,28 +314,30 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   const uint32_t tmem_base = *tmem_holder;
 
   if (warp == 0) {
-    // ------------------------------------------------------------ producer
-    if (lane == 0) {
+    // ------------------------------------------------------------ producer (the whole warp, one lane issues)
+    if (elect_one()) {
       tma_prefetch_desc(&tmap_a);
       tma_prefetch_desc(&tmap_b);
-      pdl_wait();
-      uint32_t it = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-        const int ks = tile / (tiles_m * tiles_n);
-        const int rem = tile - ks * tiles_m * tiles_n;
-        const int m0 = (rem % tiles_m) * BM;
-        const int n0 = (rem / tiles_m) * BN;
-        const int kb0 = ks * kb_per_split;
-        const int kb1 = min(kb_total, kb0 + kb_per_split);
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          const int s = it % NSTAGE;
-          const uint32_t ph = (it / NSTAGE) & 1;
-          if (!mbar_wait(&empty_bar[s], ph ^ 1, abort_flag, g.status)) { ok = false; break; }
-          uint8_t* sa = smem + s * L::STAGE_BYTES;
-          uint8_t* sb = sa + L::A_BYTES;
+    }
+    pdl_wait();
+    uint32_t it = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+      const int ks = tile / (tiles_m * tiles_n);
+      const int rem = tile - ks * tiles_m * tiles_n;
+      const int m0 = (rem % tiles_m) * BM;
+      const int n0 = (rem / tiles_m) * BN;
+      const int kb0 = ks * kb_per_split;
+      const int kb1 = min(kb_total, kb0 + kb_per_split);
+      for (int kb = kb0; kb < kb1; ++kb, ++it) {
+        const int s = it % NSTAGE;
+        const uint32_t ph = (it / NSTAGE) & 1;
+        if (!mbar_wait_warp(&empty_bar[s], ph ^ 1, abort_flag, g.status)) { ok = false; break; }
+        uint8_t* sa = smem + s * L::STAGE_BYTES;
+        uint8_t* sb = sa + L::A_BYTES;
+        const int k0 = kb * BK;
+        if (elect_one()) {
           mbar_expect_tx(&full_bar[s], L::STAGE_BYTES);
-          const int k0 = kb * BK;
           if (!g.a_mn_major) {
             tma_load_2d(sa, &tmap_a, &full_bar[s], k0, m0);
           } else {
@@ -349,63 +351,63 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
             for (int c = 0; c < BN / 64; ++c) tma_load_2d(sb + c * 8192, &tmap_b, &full_bar[s], n0 + 64 * c, k0);
           }
         }
+        __syncwarp();
       }
-      pdl_launch();
-      if (!ok) {
-        // give loads that are still in flight a bounded chance to land before the CTA exits
-        for (int s = 0; s < NSTAGE; ++s) {
-          for (int spin = 0; spin < 100000; ++spin)
-            if (mbar_try_wait(&full_bar[s], 0) || mbar_try_wait(&full_bar[s], 1)) break;
-        }
+    }
+    pdl_launch();
+    if (!ok) {
+      // give loads that are still in flight a bounded chance to land before the CTA exits
+      for (int s = 0; s < NSTAGE; ++s) {
+        for (int spin = 0; spin < 100000; ++spin)
+          if (mbar_try_wait(&full_bar[s], 0) || mbar_try_wait(&full_bar[s], 1)) break;
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      const uint32_t idesc = make_idesc_bf16(BM, BN, g.a_mn_major, g.b_mn_major);
-      const uint32_t desc_hi = smem_desc_hi(1024);
-      const uint32_t a_lbo = g.a_mn_major ? 8192 : 16, b_lbo = g.b_mn_major ? 8192 : 16;
-      const uint32_t a_step = g.a_mn_major ? (2048 >> 4) : (32 >> 4), b_step = g.b_mn_major ? (2048 >> 4) : (32 >> 4);
-      uint32_t it = 0;
-      uint32_t tcount = 0;
-      bool ok = true;
-      long long* tr = blockIdx.x == 0 ? g.trace : nullptr;
-      int tslot = 0;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++tcount) {
-        const int ks = tile / (tiles_m * tiles_n);
-        const int kb0 = ks * kb_per_split;
-        const int kb1 = min(kb_total, kb0 + kb_per_split);
-        const int ab = tcount & 1;
-        const uint32_t aph = (tcount >> 1) & 1;
-        if (!mbar_wait(&acc_empty[ab], aph ^ 1, abort_flag, g.status)) { ok = false; break; }
-        tc_fence_after();
-        const uint32_t d_tmem = tmem_base + ab * BN;
-        uint32_t accumulate = 0;
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          const int s = it % NSTAGE;
-          const uint32_t ph = (it / NSTAGE) & 1;
-          GEMM_TRACE(tr, tslot);
-          if (!mbar_wait(&full_bar[s], ph, abort_flag, g.status)) { ok = false; break; }
-          GEMM_TRACE(tr, tslot);
-          // no tcgen05 fence here: the operands were written by TMA (async proxy) and the mbarrier
-          // wait orders them; a fence per k-block only delays the next MMAs behind the previous ones
-          const uint32_t sa = smem_u32(smem + s * L::STAGE_BYTES);
-          const uint32_t sb = sa + L::A_BYTES;
-          // K-major: 16 elements = 32 bytes further along the swizzled row per MMA.
-          // MN-major: 16 k-rows of 128 bytes further down.  Only the low descriptor word moves.
-          uint32_t a_lo = smem_desc_lo(sa, a_lbo), b_lo = smem_desc_lo(sb, b_lbo);
+    // ------------------------------------------------------------ MMA issuer (the whole warp, one lane issues)
+    const uint32_t idesc = make_idesc_bf16(BM, BN, g.a_mn_major, g.b_mn_major);
+    const uint32_t desc_hi = smem_desc_hi(1024);
+    const uint32_t a_lbo = g.a_mn_major ? 8192 : 16, b_lbo = g.b_mn_major ? 8192 : 16;
+    const uint32_t a_step = g.a_mn_major ? (2048 >> 4) : (32 >> 4), b_step = g.b_mn_major ? (2048 >> 4) : (32 >> 4);
+    uint32_t it = 0;
+    uint32_t tcount = 0;
+    bool ok = true;
+    long long* tr = blockIdx.x == 0 && lane == 0 ? g.trace : nullptr;
+    int tslot = 0;
+    (void)tr; (void)tslot;
+    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++tcount) {
+      const int ks = tile / (tiles_m * tiles_n);
+      const int kb0 = ks * kb_per_split;
+      const int kb1 = min(kb_total, kb0 + kb_per_split);
+      const int ab = tcount & 1;
+      const uint32_t aph = (tcount >> 1) & 1;
+      if (!mbar_wait_warp(&acc_empty[ab], aph ^ 1, abort_flag, g.status)) { ok = false; break; }
+      tc_fence_after();
+      const uint32_t d_tmem = tmem_base + ab * BN;
+      for (int kb = kb0; kb < kb1; ++kb, ++it) {
+        const int s = it % NSTAGE;
+        const uint32_t ph = (it / NSTAGE) & 1;
+        GEMM_TRACE(tr, tslot);
+        if (!mbar_wait_warp(&full_bar[s], ph, abort_flag, g.status)) { ok = false; break; }
+        GEMM_TRACE(tr, tslot);
+        // no tcgen05 fence here: the operands were written by TMA (async proxy) and the mbarrier
+        // wait orders them; a fence per k-block only delays the next MMAs behind the previous ones
+        const uint32_t sa = smem_u32(smem + s * L::STAGE_BYTES);
+        const uint32_t sb = sa + L::A_BYTES;
+        // K-major: 16 elements = 32 bytes further along the swizzled row per MMA.
+        // MN-major: 16 k-rows of 128 bytes further down.  Only the low descriptor word moves.
+        const uint32_t a_lo = smem_desc_lo(sa, a_lbo), b_lo = smem_desc_lo(sb, b_lbo);
+        if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k) {
-            umma_bf16_lohi(d_tmem, a_lo, b_lo, desc_hi, idesc, accumulate);
-            a_lo += a_step; b_lo += b_step;
-            accumulate = 1;
-          }
-          GEMM_TRACE(tr, tslot);
+          for (int k = 0; k < BK / UMMA_K; ++k)
+            umma_bf16_lohi(d_tmem, a_lo + k * a_step, b_lo + k * b_step, desc_hi, idesc, kb > kb0 || k > 0);
           umma_commit(&empty_bar[s]);      // frees the smem stage when these MMAs retire
-          GEMM_TRACE(tr, tslot);
         }
-        if (ok) umma_commit(&acc_full[ab]);  // accumulator complete
+        __syncwarp();
+        GEMM_TRACE(tr, tslot);
+        GEMM_TRACE(tr, tslot);
       }
+      if (ok && elect_one()) umma_commit(&acc_full[ab]);  // accumulator complete
+      __syncwarp();
     }
   } else if (warp >= EPI_WARP0) {
     // ------------------------------------------------------------ epilogue
@@ -452,7 +454,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
 }
 
 // ------------------------------------------------------------------ CTA-pair variant
-// 256 x 256 output tile per cluster of two CTAs (tcgen05 cta_group::2).  Each CTA
+// 256 x BN output tile per cluster of two CTAs (tcgen05 cta_group::2).  Each CTA
 // loads only its half of A (128 rows) and its half of B (128 columns) per k-block,
 // 32 KB instead of the 48 KB a lone 128 x 256 CTA needs for the same FLOPs, which is
 // what matters once the main loop is bound by L2-to-shared-memory traffic.  The
@@ -464,27 +466,29 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
 //   acc_empty[b] in the leader, one arrival per epilogue warp of both CTAs
 // KSUB k-blocks share one full/empty barrier pair (KSUB = 2: a stage is two 64-wide k-blocks, so the issuing
 // thread pays one barrier wait and one commit per eight MMAs instead of per four).
-constexpr int PAIR_BN = 256;
-constexpr int PAIR_STAGES = 6;          // k-blocks resident in shared memory
+// BN = 128 (64 columns of B per CTA) serves outputs too narrow, or with too few tiles, for 256: an SM takes in 24 KB per
+// 128 x 128 x 64 products instead of the 32 KB of a lone 128 x 128 CTA, and that intake (some 120 bytes per ns) is what
+// bounds a tile this small.
+template <int BN>
 struct PairSmem {
+  static constexpr int STAGES = BN == 256 ? 6 : 8;      // k-blocks resident in shared memory
   static constexpr int A_BYTES = 128 * BK * 2;
-  static constexpr int B_BYTES = 128 * BK * 2;
+  static constexpr int B_BYTES = BN / 2 * BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int EPI_OFFSET = PAIR_STAGES * STAGE_BYTES;
+  static constexpr int EPI_OFFSET = STAGES * STAGE_BYTES;
   static constexpr int BAR_OFFSET = EPI_OFFSET + EPI_WARPS * EPI_STAGE_BYTES;
   static constexpr int TOTAL = BAR_OFFSET + 256 + 1024;
 };
 
 constexpr int PAIR_KSUB = 2;           // k-blocks per barrier pair
 
-template <int MODE>
+template <int BN, int MODE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, GemmArgs g) {
-  using L = PairSmem;
+  using L = PairSmem<BN>;
   constexpr int KSUB = PAIR_KSUB;
-  constexpr int NSTAGE = PAIR_STAGES / KSUB;          // barrier pairs; each covers KSUB k-blocks
-  static_assert(PAIR_STAGES % KSUB == 0, "stages must divide into groups");
-  constexpr int BN = PAIR_BN;
+  constexpr int NSTAGE = L::STAGES / KSUB;            // barrier pairs; each covers KSUB k-blocks
+  static_assert(L::STAGES % KSUB == 0, "stages must divide into groups");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + L::BAR_OFFSET);
@@ -525,28 +529,32 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   const uint32_t tmem_base = *tmem_holder;
 
   if (warp == 0) {
-    // ------------------------------------------------------------ producer (one per CTA)
-    if (lane == 0) {
+    // ------------------------------------------------------------ producer (one warp per CTA, one lane issues)
+    if (elect_one()) {
       tma_prefetch_desc(&tmap_a);
       tma_prefetch_desc(&tmap_b);
-      pdl_wait();
-      uint32_t it = 0;
-      bool ok = true;
-      for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
-        const int ks = tile / (tiles_m * tiles_n);
-        const int rem = tile - ks * tiles_m * tiles_n;
-        const int m0 = (rem % tiles_m) * 256 + int(rank) * 128;     // this CTA's rows of A
-        const int n0 = (rem / tiles_m) * BN + int(rank) * 128;      // this CTA's columns of B
-        const int kb0 = ks * kb_per_split;
-        const int kb1 = min(kb_total, kb0 + kb_per_split);
-        for (int kb = kb0; kb < kb1; kb += KSUB, ++it) {
-          const int s = it % NSTAGE;
-          const uint32_t ph = (it / NSTAGE) & 1;
-          const int nsub = min(KSUB, kb1 - kb);
-          if (!mbar_wait(&empty_bar[s], ph ^ 1, abort_flag, g.status)) { ok = false; break; }
-          const uint32_t full_leader = map_to_cta(smem_u32(&full_bar[s]), 0);
+    }
+    pdl_wait();
+    uint32_t it = 0;
+    bool ok = true;
+    for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
+      const int ks = tile / (tiles_m * tiles_n);
+      const int rem = tile - ks * tiles_m * tiles_n;
+      const int m0 = (rem % tiles_m) * 256 + int(rank) * 128;     // this CTA's rows of A
+      const int n0 = (rem / tiles_m) * BN + int(rank) * (BN / 2);      // this CTA's columns of B
+      const int kb0 = ks * kb_per_split;
+      const int kb1 = min(kb_total, kb0 + kb_per_split);
+      for (int kb = kb0; kb < kb1; kb += KSUB, ++it) {
+        const int s = it % NSTAGE;
+        const uint32_t ph = (it / NSTAGE) & 1;
+        const int nsub = min(KSUB, kb1 - kb);
+        if (!mbar_wait_warp(&empty_bar[s], ph ^ 1, abort_flag, g.status)) { ok = false; break; }
+        const uint32_t full_leader = map_to_cta(smem_u32(&full_bar[s]), 0);
+        if (elect_one()) {
           mbar_expect_tx_cluster(full_leader, nsub * L::STAGE_BYTES);
-          for (int sub = 0; sub < nsub; ++sub) {
+#pragma unroll
+          for (int sub = 0; sub < KSUB; ++sub) {
+            if (sub >= nsub) break;
             uint8_t* sa = smem + (s * KSUB + sub) * L::STAGE_BYTES;
             uint8_t* sb = sa + L::A_BYTES;
             const int k0 = (kb + sub) * BK;
@@ -560,16 +568,17 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
               tma_load_2d_pair(sb, &tmap_b, full_leader, k0, n0);
             } else {
               tma_load_2d_pair(sb, &tmap_b, full_leader, n0, k0);
-              tma_load_2d_pair(sb + 8192, &tmap_b, full_leader, n0 + 64, k0);
+              if constexpr (BN == 256) tma_load_2d_pair(sb + 8192, &tmap_b, full_leader, n0 + 64, k0);
             }
           }
         }
+        __syncwarp();
       }
-      pdl_launch();
     }
+    pdl_launch();
   } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer (leader CTA only)
-    if (lane == 0 && rank == 0) {
+    // ------------------------------------------------------------ MMA issuer (leader CTA only; the whole warp, one lane issues)
+    if (rank == 0) {
       const uint32_t idesc = make_idesc_bf16(256, BN, g.a_mn_major, g.b_mn_major);
       const uint32_t desc_hi = smem_desc_hi(1024);
       const uint32_t a_lbo = g.a_mn_major ? 8192 : 16, b_lbo = g.b_mn_major ? 8192 : 16;
@@ -577,48 +586,47 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       uint32_t it = 0;
       uint32_t tcount = 0;
       bool ok = true;
-      long long* tr = blockIdx.x == 0 ? g.trace : nullptr;
+      long long* tr = blockIdx.x == 0 && lane == 0 ? g.trace : nullptr;
       int tslot = 0;
+      (void)tr; (void)tslot;
       for (int tile = pair; tile < num_tiles && ok; tile += num_pairs, ++tcount) {
         const int ks = tile / (tiles_m * tiles_n);
         const int kb0 = ks * kb_per_split;
         const int kb1 = min(kb_total, kb0 + kb_per_split);
         const int ab = tcount & 1;
         const uint32_t aph = (tcount >> 1) & 1;
-        if (!mbar_wait(&acc_empty[ab], aph ^ 1, abort_flag, g.status)) { ok = false; break; }
+        if (!mbar_wait_warp(&acc_empty[ab], aph ^ 1, abort_flag, g.status)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + ab * BN;
-        uint32_t accumulate = 0;
         for (int kb = kb0; kb < kb1; kb += KSUB, ++it) {
           const int s = it % NSTAGE;
           const uint32_t ph = (it / NSTAGE) & 1;
           const int nsub = min(KSUB, kb1 - kb);
           GEMM_TRACE(tr, tslot);
-          if (!mbar_wait(&full_bar[s], ph, abort_flag, g.status)) { ok = false; break; }
+          if (!mbar_wait_warp(&full_bar[s], ph, abort_flag, g.status)) { ok = false; break; }
           GEMM_TRACE(tr, tslot);
           // no tcgen05 fence here: the operands were written by TMA (async proxy) and the mbarrier
           // wait orders them; a fence per k-block only delays the next MMAs behind the previous ones
+          const uint32_t sa = smem_u32(smem + s * KSUB * L::STAGE_BYTES);
+          const uint32_t a_lo = smem_desc_lo(sa, a_lbo), b_lo = smem_desc_lo(sa + L::A_BYTES, b_lbo);
+          if (elect_one()) {
 #pragma unroll
-          for (int sub = 0; sub < KSUB; ++sub) {
-            if (sub < nsub) {
-              const uint32_t sa = smem_u32(smem + (s * KSUB + sub) * L::STAGE_BYTES);
-              const uint32_t sb = sa + L::A_BYTES;
-              uint32_t a_lo = smem_desc_lo(sa, a_lbo), b_lo = smem_desc_lo(sb, b_lbo);
+            for (int sub = 0; sub < KSUB; ++sub) {
+              if (sub >= nsub) break;
+              constexpr uint32_t SUB16 = L::STAGE_BYTES >> 4;
 #pragma unroll
-              for (int k = 0; k < BK / UMMA_K; ++k) {
-                umma_bf16_pair_lohi(d_tmem, a_lo, b_lo, desc_hi, idesc, accumulate);
-                a_lo += a_step; b_lo += b_step;
-                accumulate = 1;
-              }
+              for (int k = 0; k < BK / UMMA_K; ++k)
+                umma_bf16_pair_lohi(d_tmem, a_lo + sub * SUB16 + k * a_step, b_lo + sub * SUB16 + k * b_step, desc_hi, idesc,
+                                    kb > kb0 || sub > 0 || k > 0);
             }
+            umma_commit_pair_all(smem_u32(&empty_bar[s]), 0x3);     // frees the stage in both CTAs
           }
+          __syncwarp();
           GEMM_TRACE(tr, tslot);
-          umma_commit_pair_all(smem_u32(&empty_bar[s]), 0x3);     // frees the stage in both CTAs
           GEMM_TRACE(tr, tslot);
         }
-        if (ok) {
-          umma_commit_pair_all(smem_u32(&acc_full[ab]), 0x3);
-        }
+        if (ok && elect_one()) umma_commit_pair_all(smem_u32(&acc_full[ab]), 0x3);
+        __syncwarp();
       }
     }
   } else if (warp >= EPI_WARP0) {
@@ -682,7 +690,8 @@ __host__ __device__ constexpr int epi_class(int mode) { return mode == EPI_STORE
 // Defined in gemm_one_cta.cu / gemm_pair.cu.  bn = 128 or 256 for the one-CTA kernel.
 int launch_one_cta(int bn, const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& g, int num_sms, int max_ctas,
                    cudaStream_t st);
-int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& g, int num_sms, int max_ctas,
+// bn = 256 or 128
+int launch_pair(int bn, const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& g, int num_sms, int max_ctas,
                 cudaStream_t st);
 int load_one_cta_kernels();
 int load_pair_kernels();

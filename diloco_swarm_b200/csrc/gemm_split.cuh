@@ -83,25 +83,23 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   bool ok = true;
 
   if (warp == 4) {
-    // ------------------------------------------------------------ producer
-    if (lane == 0) {
-      tma_prefetch_desc(&tmap_a);
-      tma_prefetch_desc(&tmap_b);
-      const auto load_b = [&](int i) {
-        uint8_t* sb = smem + (i % NSTAGE) * L::STAGE_BYTES + L::A_BYTES;
-        uint64_t* bar = &full_bar[i % NSTAGE];
-        const int k0 = (kb0 + i) * BK;
-        if (!g.b_mn_major) {
-          tma_load_2d(sb, &tmap_b, bar, k0, n0);
-        } else {
+    // ------------------------------------------------------------ producer (the whole warp, one lane issues)
+    const auto load_b = [&](int i) {
+      uint8_t* sb = smem + (i % NSTAGE) * L::STAGE_BYTES + L::A_BYTES;
+      uint64_t* bar = &full_bar[i % NSTAGE];
+      const int k0 = (kb0 + i) * BK;
+      if (!g.b_mn_major) {
+        tma_load_2d(sb, &tmap_b, bar, k0, n0);
+      } else {
 #pragma unroll
-          for (int c = 0; c < (BN + 63) / 64; ++c) tma_load_2d(sb + c * 8192, &tmap_b, bar, n0 + 64 * c, k0);
-        }
-      };
-      const int nkb = kb1 - kb0;
-      int early = 0;                      // stages whose B operand is already on its way
-      if (g.b_static) {
-        early = nkb < NSTAGE ? nkb : NSTAGE;
+        for (int c = 0; c < (BN + 63) / 64; ++c) tma_load_2d(sb + c * 8192, &tmap_b, bar, n0 + 64 * c, k0);
+      }
+    };
+    const int nkb = kb1 - kb0;
+    int early = 0;                      // stages whose B operand is already on its way
+    if (g.b_static) {
+      early = nkb < NSTAGE ? nkb : NSTAGE;
+      if (elect_one()) {
         for (int i = 0; i < early; ++i) { mbar_expect_tx(&full_bar[i], L::STAGE_BYTES); load_b(i); }
         for (int i = early; i < nkb; ++i) {                       // the rest is asked into L2
           const int k0 = (kb0 + i) * BK;
@@ -113,38 +111,38 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           }
         }
       }
-      pdl_wait();
-      pdl_launch();
-      for (int i = 0; i < nkb; ++i) {
-        const int s = i % NSTAGE;
-        if (i >= NSTAGE && !mbar_wait(&empty_bar[s], ((i / NSTAGE) & 1) ^ 1, abort_flag, g.status)) break;
+      __syncwarp();
+    }
+    pdl_wait();
+    pdl_launch();
+    for (int i = 0; i < nkb; ++i) {
+      const int s = i % NSTAGE;
+      if (i >= NSTAGE && !mbar_wait_warp(&empty_bar[s], ((i / NSTAGE) & 1) ^ 1, abort_flag, g.status)) break;
+      if (elect_one()) {
         if (i >= early) { mbar_expect_tx(&full_bar[s], L::STAGE_BYTES); load_b(i); }
         tma_load_2d(smem + s * L::STAGE_BYTES, &tmap_a, &full_bar[s], (kb0 + i) * BK, m0);
       }
+      __syncwarp();
     }
-    __syncwarp();
   } else if (warp == 5) {
-    // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      const uint32_t idesc = make_idesc_bf16(BM, BN, 0, g.b_mn_major);
-      const uint32_t desc_hi = smem_desc_hi(1024);
-      const uint32_t b_lbo = g.b_mn_major ? 8192 : 16, b_step = g.b_mn_major ? (2048 >> 4) : (32 >> 4);
-      uint32_t accumulate = 0;
-      for (int i = 0; i < kb1 - kb0; ++i) {
-        const int s = i % NSTAGE;
-        if (!mbar_wait(&full_bar[s], (i / NSTAGE) & 1, abort_flag, g.status)) { ok = false; break; }
-        const uint32_t sa = smem_u32(smem + s * L::STAGE_BYTES);
-        uint32_t a_lo = smem_desc_lo(sa, 16), b_lo = smem_desc_lo(sa + L::A_BYTES, b_lbo);
+    // ------------------------------------------------------------ MMA issuer (the whole warp, one lane issues)
+    const uint32_t idesc = make_idesc_bf16(BM, BN, 0, g.b_mn_major);
+    const uint32_t desc_hi = smem_desc_hi(1024);
+    const uint32_t b_lbo = g.b_mn_major ? 8192 : 16, b_step = g.b_mn_major ? (2048 >> 4) : (32 >> 4);
+    for (int i = 0; i < kb1 - kb0; ++i) {
+      const int s = i % NSTAGE;
+      if (!mbar_wait_warp(&full_bar[s], (i / NSTAGE) & 1, abort_flag, g.status)) { ok = false; break; }
+      const uint32_t sa = smem_u32(smem + s * L::STAGE_BYTES);
+      const uint32_t a_lo = smem_desc_lo(sa, 16), b_lo = smem_desc_lo(sa + L::A_BYTES, b_lbo);
+      if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < BK / UMMA_K; ++k) {
-          umma_bf16_lohi(tmem_base, a_lo, b_lo, desc_hi, idesc, accumulate);
-          a_lo += 32 >> 4; b_lo += b_step;
-          accumulate = 1;
-        }
+        for (int k = 0; k < BK / UMMA_K; ++k)
+          umma_bf16_lohi(tmem_base, a_lo + k * (32 >> 4), b_lo + k * b_step, desc_hi, idesc, i > 0 || k > 0);
         umma_commit(&empty_bar[s]);
       }
-      if (ok) umma_commit(acc_full);
+      __syncwarp();
     }
+    if (ok && elect_one()) umma_commit(acc_full);
     __syncwarp();
   }
 

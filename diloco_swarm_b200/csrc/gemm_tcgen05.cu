@@ -130,12 +130,6 @@ int cached_tmap(CUtensorMap* tm, int kind, const void* ptr, long long inner, lon
 }
 
 // ------------------------------------------------------------------ tile choice
-static double tile_efficiency(long long M, long long N, int splits, int bm, int bn, int units) {
-  const long long tm = (M + bm - 1) / bm, tn = (N + bn - 1) / bn, tiles = tm * tn * splits;
-  const long long waves = (tiles + units - 1) / units;
-  return double(M) * N / (double(tm) * bm * tn * bn) * tiles / (double(waves) * units);
-}
-
 // Cap on the CTAs of every GEMM launch (0 = all SMs): leaves SMs to kernels that sit on the device while the GEMMs run,
 // such as a pipeline transfer waiting for its peer.
 static int default_max_ctas() {
@@ -148,16 +142,34 @@ static bool use_pair() {
   return on;
 }
 
-// 512 = 256 x 256 on a CTA pair (least operand traffic per FLOP), 256 = 128 x 256 on one CTA, 128 = 128 x 128.  A wider
-// tile wins unless a narrower one fills the SMs clearly better.
-static int pick_bn(int M, int N, int splits, int sms) {
-  if (N <= 128) return 128;
-  const double e128 = tile_efficiency(M, N, splits, 128, 128, sms), e256 = tile_efficiency(M, N, splits, 128, 256, sms);
-  if (use_pair() && M >= 256) {
-    const double pair = tile_efficiency(M, N, splits, 256, 256, sms / 2);
-    if (pair >= fmax(e128 * 0.8, e256 * 0.9)) return 512;
+// The kernels for many rows.  bn = 512: 256 x 256 on a CTA pair, 384: 256 x 128 on a pair, 256: 128 x 256 on one CTA, 128:
+// 128 x 128.  Times in ns per k-block of a tile, fitted to launches of 2128 to 16384 rows (N and K of GPT-2 small, large
+// and xl): what an SM needs to take in its operands (some 120 bytes per ns; 32 KB for 128 x 128 and for a CTA of the wide
+// pair, 24 KB for the narrow one, 48 KB for 128 x 256), the wide pair a little more where its arithmetic shows.
+struct TileKind { int bn, bm, width, ctas; double per_kb, epilogue, setup, per_kb_wgrad, setup_wgrad; };
+constexpr TileKind TILE_KINDS[] = {
+    {128, 128, 128, 1, 280.0, 1400.0, 3600.0, 280.0, 5000.0},
+    {256, 128, 256, 1, 390.0, 2600.0, 3600.0, 400.0, 6000.0},
+    {384, 256, 128, 2, 260.0, 1400.0, 4000.0, 260.0, 6500.0},
+    {512, 256, 256, 2, 340.0, 2600.0, 4000.0, 380.0, 7000.0},
+};
+static bool allowed(const TileKind& t, int M) { return t.ctas == 1 || (use_pair() && M >= 256); }
+
+// The one whose waves take least.  A tile's epilogue hides behind the next tile's main loop when that is the longer.
+static int pick_bn(int M, int N, int K, int splits, int mode, int sms, double* cost) {
+  const int kb = ((K + BK - 1) / BK + splits - 1) / splits;
+  const double heavy = mode == EPI_GELU || mode == EPI_MUL ? 2.0 : 1.0;
+  int best = 128;
+  double least = 1e30;
+  for (const TileKind& t : TILE_KINDS) {
+    if (!allowed(t, M) || (t.width > 128 && N <= 128)) continue;
+    const long long tiles = (long long)((M + t.bm - 1) / t.bm) * ((N + t.width - 1) / t.width) * splits;
+    const int units = sms / t.ctas;
+    const double c = t.setup + double((tiles + units - 1) / units) * fmax(kb * t.per_kb, heavy * t.epilogue) + heavy * t.epilogue;
+    if (c < least) { least = c; best = t.bn; }
   }
-  return e256 >= e128 * 0.93 ? 256 : 128;
+  *cost = least;
+  return best;
 }
 
 // Few rows: tile width and split of K for the cluster kernel (gemm_split.cuh), or 0 where the kernels for many rows are
@@ -165,10 +177,9 @@ static int pick_bn(int M, int N, int splits, int sms) {
 // into question while all its CTAs fit on the SMs at once.  Times in ns, fitted to launches of 24 to 2128 rows (N and K
 // of GPT-2 small, weights cold in L2): a k-block takes its share of the load latency, which falls with the stages in
 // flight; partial sums leave a CTA at 18 bytes per ns; a thread stores one row of the CTA's columns.
-static int pick_few_rows(int M, int N, int K, bool b_mn, int sms, int* split) {
+static int pick_few_rows(int M, int N, int K, bool b_mn, int sms, double many_rows, int* split) {
   const int tm = (M + BM - 1) / BM, kb = (K + BK - 1) / BK;
-  const int waves = (tm * ((N + 127) / 128) + sms - 1) / sms;          // of the 128 x 128 kernel
-  double best = 1500.0 + 280.0 * waves * kb;
+  double best = many_rows - 3400.0;             // what a launch takes besides the terms below
   int bn = 0;
   for (int w = b_mn ? 64 : 32; w <= 128; w *= 2)
     for (int s = 1; s <= 8 && s <= kb && w / s >= 8; s *= 2) {
@@ -180,22 +191,32 @@ static int pick_few_rows(int M, int N, int K, bool b_mn, int sms, int* split) {
   return bn;
 }
 
-// Split of K (tokens) for a weight gradient dW[M,N]: few output tiles, so K is split until the SMs are full.
-static int pick_wgrad_split(int M, int N, int K, int sms) {
-  const bool pair = use_pair() && M >= 256;
-  const int bm = pair ? 256 : 128, units = pair ? sms / 2 : sms;
-  const long long tiles = (long long)((M + bm - 1) / bm) * ((N + 255) / 256);
-  if (tiles >= 4 * units) return 1;
-  const int kb = (K + 63) / 64;
-  int best = 1;
-  double best_eff = 0.0;
-  for (int s = 1; s <= 16 && kb / s >= 4; ++s) {
-    const long long waves = (tiles * s + units - 1) / units;
-    const double eff = double(tiles * s) / double(waves * units) - 0.01 * (s - 1);      // small price per split (atomics)
-    if (eff > best_eff + 1e-9) { best = s; best_eff = eff; }
+// Tile and split of K (tokens) for a weight gradient dW[M,N], whose tiles are added into memory with fp32 reductions: few
+// tiles, so K is split, but every further split adds the whole matrix once more.  L2 takes reductions at some 4.3 TB/s,
+// of which about 0.4 shows beside the main loops; parts that meet on one address wait for one another.  Fitted to
+// 128 x 128 ... 6400 x 1600 with 128 to 16384 tokens (5120 x 1280, 2128 tokens: 4 splits by the earlier rule, which filled
+// the last wave at any price, 43.4 us; 2 splits 32.6 us).
+static int pick_wgrad(int M, int N, int K, int bn, int sms, int* split) {
+  const int kb = (K + BK - 1) / BK, fixed = *split;
+  const double mb = 4.0 * M * N;
+  double least = 1e30;
+  int best = 128, best_split = 1;
+  for (const TileKind& t : TILE_KINDS) {
+    if (bn ? t.bn != bn : !allowed(t, M) || (t.width > 128 && N <= 128)) continue;
+    const long long tiles = (long long)((M + t.bm - 1) / t.bm) * ((N + t.width - 1) / t.width);
+    const int units = sms / t.ctas;
+    for (int s : {1, 2, 3, 4, 5, 6, 8, 10, 12, 16, 24, 32, 48, 64}) {
+      if (fixed) s = fixed;
+      if (s > 1 && kb / s < 2 && !fixed) continue;
+      const double c = t.setup_wgrad + double((tiles * s + units - 1) / units) * ((kb + s - 1) / s) * t.per_kb_wgrad +
+                       0.4 * mb * s / 4300.0 + 30.0 * s;
+      if (c < least) { least = c; best = t.bn; best_split = s; }
+      if (fixed) break;
+    }
   }
-  const int per = (kb + best - 1) / best;
-  return (kb + per - 1) / per;                   // no empty split
+  const int per = (kb + best_split - 1) / best_split;
+  *split = (kb + per - 1) / per;                 // no empty split
+  return best;
 }
 
 }  // namespace dsw
@@ -209,7 +230,8 @@ extern "C" int dsw_gemm_set_trace(long long* buf) { g_gemm_trace = buf; return 0
 // A: [M,K] row-major (a_mn_major = 0) or [K,M] row-major (1); lda = row pitch in
 // elements.  B: [N,K] (b_mn_major = 0) or [K,N] (1).  All pitches and the
 // contiguous extents must be multiples of 8 elements; pointers 16-byte aligned.
-// bn = 128 or 256 selects the one-CTA tile width, 512 the CTA-pair kernel, 0 leaves it to the shape; max_ctas > 0 caps the
+// bn = 128 or 256 selects the one-CTA tile width, 384 or 512 the CTA-pair kernel (128 or 256 wide), 1032 / 1064 / 1128 the
+// cluster kernel for few rows (split_k = cluster size), 0 leaves it to the shape; max_ctas > 0 caps the
 // grid (to leave SMs to a concurrent kernel).  Returns 0 or a negative error code.
 extern "C" int dsw_gemm_bf16(const void* A, long long lda, int a_mn_major, const void* B, long long ldb,
                              int b_mn_major, int M, int N, int K, int mode, int split_k, void* out, long long ldo,
@@ -220,7 +242,7 @@ extern "C" int dsw_gemm_bf16(const void* A, long long lda, int a_mn_major, const
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(out)) & 15)
     return -11;
   bool few_rows = bn == 1032 || bn == 1064 || bn == 1128;      // the split-K cluster kernel, tile 32 / 64 / 128 wide
-  if (bn != 0 && bn != 128 && bn != 256 && bn != 512 && !few_rows) return -12;   // 512 = CTA-pair kernel (256 x 256 per cluster)
+  if (bn != 0 && bn != 128 && bn != 256 && bn != 384 && bn != 512 && !few_rows) return -12;
   if (mode < EPI_STORE || mode > EPI_STORE_F32) return -13;
   if ((mode == EPI_RESID && (resid == nullptr || ldr % 8)) || (mode == EPI_MUL && (aux_in == nullptr || ldaux % 8)) ||
       ((mode == EPI_GELU || mode == EPI_RESID) && (aux_out != nullptr || aux_in != nullptr) && ldaux % 8))
@@ -229,19 +251,26 @@ extern "C" int dsw_gemm_bf16(const void* A, long long lda, int a_mn_major, const
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -2;
   if (num_sms[dev] == 0) cudaDeviceGetAttribute(&num_sms[dev], cudaDevAttrMultiProcessorCount, dev);
-  if (split_k == 0) split_k = mode == EPI_ATOMIC_F32 ? pick_wgrad_split(M, N, K, num_sms[dev]) : 1;
-  if (bn == 0 && split_k == 1 && mode <= EPI_MUL && !a_mn_major && max_ctas == 0 && default_max_ctas() == 0) {
-    bn = pick_few_rows(M, N, K, b_mn_major != 0, num_sms[dev], &split_k);
-    if (bn) { bn += 1000; few_rows = true; }
+  if (mode == EPI_ATOMIC_F32 && (split_k == 0 || bn == 0) && !few_rows) {
+    const int picked = pick_wgrad(M, N, K, bn, num_sms[dev], &split_k);
+    if (bn == 0) bn = picked;
   }
-  if (bn == 0) bn = pick_bn(M, N, split_k, num_sms[dev]);
+  if (split_k == 0) split_k = 1;
+  if (bn == 0) {
+    double cost;
+    bn = pick_bn(M, N, K, split_k, mode, num_sms[dev], &cost);
+    if (split_k == 1 && mode <= EPI_MUL && !a_mn_major && max_ctas == 0 && default_max_ctas() == 0) {
+      const int width = pick_few_rows(M, N, K, b_mn_major != 0, num_sms[dev], cost, &split_k);
+      if (width) { bn = 1000 + width; few_rows = true; }
+    }
+  }
   if (max_ctas == 0) max_ctas = default_max_ctas();
   CUtensorMap ta, tb;
   int rc;
   if (!a_mn_major) rc = cached_tmap(&ta, TMAP_BF16_2D, A, K, 1, M, lda, BK, BM);
   else             rc = cached_tmap(&ta, TMAP_BF16_2D, A, M, 1, K, lda, 64, BK);
   if (rc) return rc;
-  if (!b_mn_major) rc = cached_tmap(&tb, TMAP_BF16_2D, B, K, 1, N, ldb, BK, bn == 512 ? 128 : bn % 1000);
+  if (!b_mn_major) rc = cached_tmap(&tb, TMAP_BF16_2D, B, K, 1, N, ldb, BK, bn == 512 ? 128 : bn == 384 ? 64 : bn % 1000);
   else             rc = cached_tmap(&tb, TMAP_BF16_2D, B, N, 1, K, ldb, 64, BK);
   if (rc) return rc;
   GemmArgs g;
@@ -256,7 +285,7 @@ extern "C" int dsw_gemm_bf16(const void* A, long long lda, int a_mn_major, const
   g.b_static = tl_launch.static_b;
   g.trace = g_gemm_trace;
   if (few_rows) return launch_split(bn - 1000, ta, tb, g, stream);
-  if (bn == 512) return launch_pair(ta, tb, g, num_sms[dev], max_ctas, stream);
+  if (bn == 512 || bn == 384) return launch_pair(bn == 512 ? 256 : 128, ta, tb, g, num_sms[dev], max_ctas, stream);
   return launch_one_cta(bn, ta, tb, g, num_sms[dev], max_ctas, stream);
 }
 

@@ -117,6 +117,14 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   }
 }
 
+// The same wait by a whole warp: true on every lane or on none.  Roles that issue TMA or tensor-core instructions run as
+// whole warps on warp-uniform values and elect a lane around the instruction itself: descriptors, addresses and barriers
+// then live in uniform registers.  Issued from a branch that only lane 0 had entered, each of them was first moved there
+// value by value, about 50 ns for a tcgen05.mma however small it was.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status));
+}
+
 // ---------------------------------------------------------------- programmatic dependent launch (launch.h)
 // Returns when the kernel before this one in the stream has completed; at once where the launch was a plain one.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

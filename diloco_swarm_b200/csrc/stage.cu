@@ -305,15 +305,16 @@ struct Run {
     }
     slot->used = ++s.tick;
     if (slot->failed) return body();
+    // what earlier passes left on the side stream comes first; after that their events are free to be recorded again
+    TRY(join());
+    if (s.head_used) MAIN_WAIT(s.head_done);
+    s.side_used[0] = s.side_used[1] = s.head_used = false;
     if (!slot->exec) {
       TRY(capture(*slot, body));
       if (slot->failed) return body();
     }
-    TRY(join());                      // work that earlier passes left on the side stream
-    if (s.head_used) TRY_CUDA(cudaStreamWaitEvent(st, s.head_done, 0));
     TRY_CUDA(cudaGraphLaunch(slot->exec, st));
     TRY_CUDA(cudaEventRecord(slot->launched, st));
-    s.side_used[0] = s.side_used[1] = s.head_used = false;
     dsw::tl_launch.pdl = false;
     g_launches.fetch_add(slot->launches, std::memory_order_relaxed);
     return 0;
@@ -334,12 +335,10 @@ struct Run {
   template <class F>
   int capture(GraphSlot& slot, F&& body) {
     const cudaStream_t on = st;
-    const bool used[3] = {s.side_used[0], s.side_used[1], s.head_used};
     const int before = g_launches.load(std::memory_order_relaxed);
     slot.failed = true;
     if (cudaStreamBeginCapture(s.cap, cudaStreamCaptureModeThreadLocal) != cudaSuccess) { cudaGetLastError(); return 0; }
     st = s.cap;
-    s.side_used[0] = s.side_used[1] = s.head_used = false;
     dsw::tl_launch.pdl = false;
     int rc = body();
     if (rc == 0) rc = join();
@@ -348,7 +347,7 @@ struct Run {
     const bool ended = cudaStreamEndCapture(s.cap, &graph) == cudaSuccess && graph != nullptr;
     st = on;
     dsw::tl_launch.pdl = false;
-    s.side_used[0] = used[0]; s.side_used[1] = used[1]; s.head_used = used[2];
+    s.side_used[0] = s.side_used[1] = s.head_used = false;      // the capture joined the side stream
     slot.launches = g_launches.load(std::memory_order_relaxed) - before;
     g_launches.fetch_sub(slot.launches, std::memory_order_relaxed);
     if (rc == 0 && ended && cudaEventCreateWithFlags(&slot.launched, cudaEventDisableTiming) == cudaSuccess) {
@@ -369,7 +368,19 @@ struct Run {
       TRY_CUDA(cudaEventRecord(s.head_done, s.side));
       s.head_used = true;
     }
-    LAUNCH(gemm(c.logits, s.head_w, false, s.d, s.V, c.dln + size_t(r0) * s.d, DSW_EPI_STORE, nullptr, nullptr, nullptr, nullptr, m));
+    bf16* dln = c.dln + size_t(r0) * s.d;
+    // m x d output tiles and a K of the whole vocabulary: few of them leave most SMs idle for hundreds of k-blocks (2128
+    // rows of GPT-2 small: 27 CTA pairs, 238 us), so K is split as in a weight gradient, with the fp32 sums in the
+    // scratch that the attention backward uses later.  Not with deterministic gradients: the sums meet in atomics.
+    if (!deterministic && ((m + 255) / 256) * ((s.d + 255) / 256) < 74) {
+      TRY_CUDA(cudaMemsetAsync(c.dq_acc, 0, size_t(m) * s.d * sizeof(float), st));
+      dsw::tl_launch.pdl = false;
+      LAUNCH(dsw_gemm_bf16(c.logits, s.V, 0, s.head_w, s.d, 1, m, s.d, s.V, DSW_EPI_ATOMIC_F32, 0, c.dq_acc, s.d, nullptr, nullptr, 0,
+                           nullptr, nullptr, 0, 0, 0, s.status, st));
+      LAUNCH(dsw_cast_f32_bf16(c.dq_acc, dln, (long long)m * s.d, st));
+      return 0;
+    }
+    LAUNCH(gemm(c.logits, s.head_w, false, s.d, s.V, dln, DSW_EPI_STORE, nullptr, nullptr, nullptr, nullptr, m));
     return 0;
   }
 

@@ -52,6 +52,28 @@ def test_interleaved_microbatches_of_different_sizes(layers):
             assert torch.allclose(a[k], b[k], rtol=1e-3, atol=1e-5 * a[k].abs().max().item() + 1e-9), k
 
 
+def test_a_middle_stage_replays_its_passes():
+    """forward and backward of a stage without ends, queued, captured and replayed: the same gradients every time."""
+    cfg = make_config(model={"n_layer": 3}, swarm={"num_stages": 3})
+    mid = _stages(cfg)[1]
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x, dy = (torch.randn(3, 50, 128, device="cuda", generator=g).to(torch.bfloat16) for _ in range(2))
+    seen = []
+    for _ in range(4):
+        mid.grad.zero_()
+        y = mid.forward(0, None, x)
+        dx = mid.backward(0, dy)
+        mid._join()
+        seen.append((y.clone(), dx.clone(), mid.grad.clone()))
+    torch.cuda.synchronize()
+    mid.check_status()
+    for y, dx, grad in seen[1:]:
+        assert torch.equal(y, seen[0][0])
+        # dQ is summed by fp32 reductions in any order, then rounded to bf16: an element may round the other way
+        assert torch.allclose(dx.float(), seen[0][1].float(), rtol=2 ** -7, atol=2 ** -8 * seen[0][1].abs().max().item())
+        assert torch.allclose(grad, seen[0][2], rtol=1e-2, atol=1e-3 * seen[0][2].abs().max().item())
+
+
 def test_inference_logits_match_the_loss_path():
     """forward_infer's fp32 logits against autograd's, at a length below one tile."""
     cfg, eb, et = _engines()
