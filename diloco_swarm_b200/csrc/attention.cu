@@ -163,94 +163,103 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, __nv_bfloat16
   if (warp >= 6) {
     // nothing to do: these warps exist so that the register hand-over works on whole warpgroups
   } else if (warp == 5) {
-    // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      tma_prefetch_desc(&tmap_qkv);
-      pdl_wait();
-      uint32_t g = 0, w = 0;
-      bool ok = true;
-      for (int r = 0; r < rounds && ok; ++r) {
-        int idx;
-        if (!att_item(r, cta, G, total, idx)) continue;
-        const int qi = nq - 1 - idx / n_bh, bh = idx % n_bh;
-        const int b = bh / nh, h = bh - b * nh;
-        if (w > 0 && !mbar_wait(q_empty, (w - 1) & 1, abort_flag, status)) break;
+    // ------------------------------------------------------------ TMA producer (the whole warp, one lane issues)
+    if (elect_one()) tma_prefetch_desc(&tmap_qkv);
+    pdl_wait();
+    uint32_t g = 0, w = 0;
+    bool ok = true;
+    for (int r = 0; r < rounds && ok; ++r) {
+      int idx;
+      if (!att_item(r, cta, G, total, idx)) continue;
+      const int qi = nq - 1 - idx / n_bh, bh = idx % n_bh;
+      const int b = bh / nh, h = bh - b * nh;
+      if (w > 0 && !mbar_wait_warp(q_empty, (w - 1) & 1, abort_flag, status)) break;
+      if (elect_one()) {
         mbar_expect_tx(q_full, ATT_TILE_BYTES);
         att_load_tile(smem + AttSmem::Q_OFF, &tmap_qkv, q_full, hs, h, b * T + qi * ATT_BQ);
-        for (int j = 0; j <= qi; ++j, ++g) {
-          const int s = g & 1;
-          if (!mbar_wait(&kv_empty[s], ((g >> 1) & 1) ^ 1, abort_flag, status)) { ok = false; break; }
+      }
+      __syncwarp();
+      for (int j = 0; j <= qi; ++j, ++g) {
+        const int s = g & 1;
+        if (!mbar_wait_warp(&kv_empty[s], ((g >> 1) & 1) ^ 1, abort_flag, status)) { ok = false; break; }
+        const int kvrow = b * T + j * ATT_BK;
+        if (elect_one()) {
           mbar_expect_tx(&kv_full[s], 2 * ATT_TILE_BYTES);
-          const int kvrow = b * T + j * ATT_BK;
           att_load_tile(smem + AttSmem::K_OFF + s * ATT_TILE_BYTES, &tmap_qkv, &kv_full[s], hs, nh + h, kvrow);
           att_load_tile(smem + AttSmem::V_OFF + s * ATT_TILE_BYTES, &tmap_qkv, &kv_full[s], hs, 2 * nh + h, kvrow);
         }
-        ++w;
+        __syncwarp();
       }
-      pdl_launch();
+      ++w;
     }
+    pdl_launch();
   } else if (warp == 4) {
-    // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      const uint32_t idesc_s = make_idesc_bf16(128, 128, 0, 0);
-      const uint32_t idesc_o = make_idesc_bf16(128, 64, 0, 1);
-      const uint32_t desc_hi = smem_desc_hi(1024);
-      const uint32_t q_lo = smem_desc_lo(smem_u32(smem + AttSmem::Q_OFF), 16);
-      const uint32_t p_lo = smem_desc_lo(smem_u32(smem + AttSmem::P_OFF), 16);
-      // S of global tile gt = Q K^T into the (single) score buffer; `first` / `last`: position in its item wi
-      auto issue_s = [&](uint32_t gt, uint32_t wi, bool first, bool last) -> bool {
-        if (first && !mbar_wait(q_full, wi & 1, abort_flag, status)) return false;
-        const int st = gt & 1;
-        if (!mbar_wait(&kv_full[st], (gt >> 1) & 1, abort_flag, status)) return false;
-        const uint32_t k_lo = smem_desc_lo(smem_u32(smem + AttSmem::K_OFF + st * ATT_TILE_BYTES), 16);
+    // ------------------------------------------------------------ MMA issuer (the whole warp, one lane issues)
+    if (lane != 0) tr = nullptr;
+    const uint32_t idesc_s = make_idesc_bf16(128, 128, 0, 0);
+    const uint32_t idesc_o = make_idesc_bf16(128, 64, 0, 1);
+    const uint32_t desc_hi = smem_desc_hi(1024);
+    const uint32_t q_lo = smem_desc_lo(smem_u32(smem + AttSmem::Q_OFF), 16);
+    const uint32_t p_lo = smem_desc_lo(smem_u32(smem + AttSmem::P_OFF), 16);
+    // S of global tile gt = Q K^T into the (single) score buffer; `first` / `last`: position in its item wi
+    auto issue_s = [&](uint32_t gt, uint32_t wi, bool first, bool last) -> bool {
+      if (first && !mbar_wait_warp(q_full, wi & 1, abort_flag, status)) return false;
+      const int st = gt & 1;
+      if (!mbar_wait_warp(&kv_full[st], (gt >> 1) & 1, abort_flag, status)) return false;
+      const uint32_t k_lo = smem_desc_lo(smem_u32(smem + AttSmem::K_OFF + st * ATT_TILE_BYTES), 16);
+      if (elect_one()) {
 #pragma unroll
         for (int k = 0; k < ATT_HS / 16; ++k)
           umma_bf16_lohi(tmem_s, q_lo + k * 2, k_lo + k * 2, desc_hi, idesc_s, k > 0);
         umma_commit(s_full);
         if (last) umma_commit(q_empty);
-        ATT_TRACE(tr, 256, tslot);          // S issued
-        return true;
-      };
-      uint32_t g = 0, w = 0;
-      bool ok = true;
-      for (int r = 0; r < rounds && ok; ++r) {
-        int idx;
-        if (!att_item(r, cta, G, total, idx)) continue;
-        const int n_kv = nq - idx / n_bh;
-        // the item after this one (its first score tile is issued during this item's last tile)
-        int next_n_kv = 0;
-        for (int r2 = r + 1, idx2; r2 < rounds; ++r2)
-          if (att_item(r2, cta, G, total, idx2)) { next_n_kv = nq - idx2 / n_bh; break; }
-        if (g == 0) ok = issue_s(0, 0, true, n_kv == 1);
-        for (int j = 0; j < n_kv && ok; ++j, ++g) {
-          const int s = g & 1;
-          const uint32_t v_lo = smem_desc_lo(smem_u32(smem + AttSmem::V_OFF + s * ATT_TILE_BYTES), ATT_TILE_BYTES);
-          // The next score tile goes first, as soon as the softmax warps have read this one for the last
-          // time (they are still turning its last columns into P): they need the next S next, while the
-          // P V product is only folded in after their first pass over it.
-          const bool more = j + 1 < n_kv;
-          if (more || next_n_kv > 0) {
-            if (!mbar_wait(s_free, g & 1, abort_flag, status)) { ok = false; break; }
-            tc_fence_after();
-            const bool okk = more ? issue_s(g + 1, w, false, j + 2 == n_kv) : issue_s(g + 1, w + 1, true, next_n_kv == 1);
-            if (!okk) { ok = false; break; }
-          }
-          // P of this tile is in shared memory (and the output rows are rescaled if they had to be)
-          if (!mbar_wait(p_full, g & 1, abort_flag, status)) { ok = false; break; }
-          ATT_TRACE(tr, 256, tslot);          // P ready
-          // a new item starts its output from zero: the previous item's must have been read out
-          if (j == 0 && w > 0 && !mbar_wait(o_free, (w - 1) & 1, abort_flag, status)) { ok = false; break; }
+      }
+      __syncwarp();
+      ATT_TRACE(tr, 256, tslot);          // S issued
+      return true;
+    };
+    uint32_t g = 0, w = 0;
+    bool ok = true;
+    for (int r = 0; r < rounds && ok; ++r) {
+      int idx;
+      if (!att_item(r, cta, G, total, idx)) continue;
+      const int n_kv = nq - idx / n_bh;
+      // the item after this one (its first score tile is issued during this item's last tile)
+      int next_n_kv = 0;
+      for (int r2 = r + 1, idx2; r2 < rounds; ++r2)
+        if (att_item(r2, cta, G, total, idx2)) { next_n_kv = nq - idx2 / n_bh; break; }
+      if (g == 0) ok = issue_s(0, 0, true, n_kv == 1);
+      for (int j = 0; j < n_kv && ok; ++j, ++g) {
+        const int s = g & 1;
+        const uint32_t v_lo = smem_desc_lo(smem_u32(smem + AttSmem::V_OFF + s * ATT_TILE_BYTES), ATT_TILE_BYTES);
+        // The next score tile goes first, as soon as the softmax warps have read this one for the last
+        // time (they are still turning its last columns into P): they need the next S next, while the
+        // P V product is only folded in after their first pass over it.
+        const bool more = j + 1 < n_kv;
+        if (more || next_n_kv > 0) {
+          if (!mbar_wait_warp(s_free, g & 1, abort_flag, status)) { ok = false; break; }
           tc_fence_after();
+          const bool okk = more ? issue_s(g + 1, w, false, j + 2 == n_kv) : issue_s(g + 1, w + 1, true, next_n_kv == 1);
+          if (!okk) { ok = false; break; }
+        }
+        // P of this tile is in shared memory (and the output rows are rescaled if they had to be)
+        if (!mbar_wait_warp(p_full, g & 1, abort_flag, status)) { ok = false; break; }
+        ATT_TRACE(tr, 256, tslot);          // P ready
+        // a new item starts its output from zero: the previous item's must have been read out
+        if (j == 0 && w > 0 && !mbar_wait_warp(o_free, (w - 1) & 1, abort_flag, status)) { ok = false; break; }
+        tc_fence_after();
+        if (elect_one()) {
 #pragma unroll
           for (int k = 0; k < ATT_BK / 16; ++k)          // P: 32 bytes along the row per step, second k-block after 4
             umma_bf16_lohi(tmem_o, p_lo + (k >> 2) * (ATT_TILE_BYTES >> 4) + (k & 3) * 2, v_lo + k * (2048 >> 4), desc_hi,
                            idesc_o, (j > 0 || k > 0));
           umma_commit(o_full);
           umma_commit(&kv_empty[s]);
-          ATT_TRACE(tr, 256, tslot);          // PV issued
         }
-        ++w;
+        __syncwarp();
+        ATT_TRACE(tr, 256, tslot);          // PV issued
       }
+      ++w;
     }
   } else {
     // ------------------------------------------------------------ softmax + output (thread = query row)
@@ -587,32 +596,37 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
                  tm_dq = tmem_base + 384;
 
   if (warp == TMA_WARP) {
-    // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    // ------------------------------------------------------------ TMA producer (the whole warp, one lane issues)
+    if (elect_one()) {
       tma_prefetch_desc(&tmap_qkv);
       tma_prefetch_desc(&tmap_do);
-      pdl_wait();
-      uint32_t g = 0, w = 0;
-      bool ok = true;
-      for (int r = 0; r < rounds && ok; ++r) {
-        int idx;
-        if (!att_item(r, cta, G, total, idx)) continue;
-        const int j = idx / n_bh, bh = idx % n_bh;
-        const int b = bh / nh, h = bh - b * nh;
-        const int steps = nq - j;
-        // K and V of the item go into the buffer of its parity, free since the item two back finished: they
-        // are on their way while the item before still runs
-        const int kb = w & 1;
-        if (!mbar_wait(&kv_empty[kb], ((w >> 1) & 1) ^ 1, abort_flag, status)) break;
-        const int kvrow = b * T + j * ATT_BK;
+    }
+    pdl_wait();
+    uint32_t g = 0, w = 0;
+    bool ok = true;
+    for (int r = 0; r < rounds && ok; ++r) {
+      int idx;
+      if (!att_item(r, cta, G, total, idx)) continue;
+      const int j = idx / n_bh, bh = idx % n_bh;
+      const int b = bh / nh, h = bh - b * nh;
+      const int steps = nq - j;
+      // K and V of the item go into the buffer of its parity, free since the item two back finished: they
+      // are on their way while the item before still runs
+      const int kb = w & 1;
+      if (!mbar_wait_warp(&kv_empty[kb], ((w >> 1) & 1) ^ 1, abort_flag, status)) break;
+      const int kvrow = b * T + j * ATT_BK;
+      if (elect_one()) {
         mbar_expect_tx(&kv_full[kb], 2 * ATT_TILE_BYTES);
         att_load_tile(smem + L::K_OFF + kb * L::KV_BYTES, &tmap_qkv, &kv_full[kb], hs, nh + h, kvrow);
         att_load_tile(smem + L::V_OFF + kb * L::KV_BYTES, &tmap_qkv, &kv_full[kb], hs, 2 * nh + h, kvrow);
-        for (int it = 0; it < steps; ++it, ++g) {
-          const int s = g % L::QSTAGES;
-          if (!mbar_wait(&q_empty[s], ((g / L::QSTAGES) & 1) ^ 1, abort_flag, status)) { ok = false; break; }
+      }
+      __syncwarp();
+      for (int it = 0; it < steps; ++it, ++g) {
+        const int s = g % L::QSTAGES;
+        if (!mbar_wait_warp(&q_empty[s], ((g / L::QSTAGES) & 1) ^ 1, abort_flag, status)) { ok = false; break; }
+        const int qrow = b * T + (j + it) * ATT_BQ;
+        if (elect_one()) {
           mbar_expect_tx(&q_full[s], 2 * ATT_TILE_BYTES);
-          const int qrow = b * T + (j + it) * ATT_BQ;
           att_load_tile(smem + L::Q_OFF + s * ATT_TILE_BYTES, &tmap_qkv, &q_full[s], hs, h, qrow);
           att_load_tile(smem + L::DO_OFF + s * ATT_TILE_BYTES, &tmap_do, &q_full[s], hs, h, qrow);
           // The pair two steps on is asked into L2 now: its load can only start when its stage is released, and
@@ -622,79 +636,84 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
             tma_prefetch_l2_2d(&tmap_do, h * 64, qrow + 2 * ATT_BQ);
           }
         }
-        ++w;
+        __syncwarp();
       }
-      pdl_launch();
+      ++w;
     }
+    pdl_launch();
   } else if (warp == MMA_WARP) {
-    // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      const uint32_t id_s = make_idesc_bf16(128, 128, 0, 0);      // Q K^T and dO V^T
-      const uint32_t id_t = make_idesc_bf16(128, 64, 1, 1);       // P^T dO and dS^T Q : A M-major, B N-major
-      const uint32_t id_q = make_idesc_bf16(128, 64, 0, 1);       // dS K : A K-major, B N-major
-      // Descriptor low words: K-major operands (leading offset 16) step 32 bytes per MMA, M/N-major ones
-      // (leading offset = one tile) step 16 rows of 128 bytes; the high word is the same for all.
-      constexpr uint32_t KSTEP = 32 >> 4, MNSTEP = 2048 >> 4, TILE16 = ATT_TILE_BYTES >> 4;
-      const uint32_t desc_hi = smem_desc_hi(1024);
-      // K and V descriptors of buffer 0; buffer 1 lies KVBUF16 further
-      const uint32_t k_km0 = smem_desc_lo(smem_u32(smem + L::K_OFF), 16), v_km0 = smem_desc_lo(smem_u32(smem + L::V_OFF), 16);
-      const uint32_t k_mn0 = smem_desc_lo(smem_u32(smem + L::K_OFF), ATT_TILE_BYTES);
-      constexpr uint32_t KVBUF16 = L::KV_BYTES >> 4;
-      const uint32_t p_mn = smem_desc_lo(smem_u32(smem + L::P_OFF), ATT_TILE_BYTES);
-      const uint32_t ds_mn = smem_desc_lo(smem_u32(smem + L::DS_OFF), ATT_TILE_BYTES);
-      const uint32_t ds_km = smem_desc_lo(smem_u32(smem + L::DS_OFF), 16);
-      uint32_t g = 0, w = 0;
-      bool ok = true;
-      // S = Q K^T and dP = dO V^T of global step gs, which belongs to item wi (operands: Q/dO stage
-      // gs % QSTAGES, K/V buffer wi & 1).  The row threads must have read the pair of the step before out of
-      // TMEM; the first step of an item also waits for its K and V.
-      auto issue_sdp = [&](uint32_t gs, uint32_t wi, bool first_of_item) -> bool {
-        const int st = gs % L::QSTAGES, kb = wi & 1;
-        if (gs > 0 && !mbar_wait(sdp_read, (gs - 1) & 1, abort_flag, status)) return false;
-        if (first_of_item && !mbar_wait(&kv_full[kb], (wi >> 1) & 1, abort_flag, status)) return false;
-        if (!mbar_wait(&q_full[st], (gs / L::QSTAGES) & 1, abort_flag, status)) return false;
-        tc_fence_after();
-        const uint32_t q_km = smem_desc_lo(smem_u32(smem + L::Q_OFF + st * ATT_TILE_BYTES), 16);
-        const uint32_t do_km = smem_desc_lo(smem_u32(smem + L::DO_OFF + st * ATT_TILE_BYTES), 16);
-        const uint32_t k_km = k_km0 + kb * KVBUF16, v_km = v_km0 + kb * KVBUF16;
+    // ------------------------------------------------------------ MMA issuer (the whole warp, one lane issues)
+    if (lane != 0) tr = nullptr;
+    const uint32_t id_s = make_idesc_bf16(128, 128, 0, 0);      // Q K^T and dO V^T
+    const uint32_t id_t = make_idesc_bf16(128, 64, 1, 1);       // P^T dO and dS^T Q : A M-major, B N-major
+    const uint32_t id_q = make_idesc_bf16(128, 64, 0, 1);       // dS K : A K-major, B N-major
+    // Descriptor low words: K-major operands (leading offset 16) step 32 bytes per MMA, M/N-major ones
+    // (leading offset = one tile) step 16 rows of 128 bytes; the high word is the same for all.
+    constexpr uint32_t KSTEP = 32 >> 4, MNSTEP = 2048 >> 4, TILE16 = ATT_TILE_BYTES >> 4;
+    const uint32_t desc_hi = smem_desc_hi(1024);
+    // K and V descriptors of buffer 0; buffer 1 lies KVBUF16 further
+    const uint32_t k_km0 = smem_desc_lo(smem_u32(smem + L::K_OFF), 16), v_km0 = smem_desc_lo(smem_u32(smem + L::V_OFF), 16);
+    const uint32_t k_mn0 = smem_desc_lo(smem_u32(smem + L::K_OFF), ATT_TILE_BYTES);
+    constexpr uint32_t KVBUF16 = L::KV_BYTES >> 4;
+    const uint32_t p_mn = smem_desc_lo(smem_u32(smem + L::P_OFF), ATT_TILE_BYTES);
+    const uint32_t ds_mn = smem_desc_lo(smem_u32(smem + L::DS_OFF), ATT_TILE_BYTES);
+    const uint32_t ds_km = smem_desc_lo(smem_u32(smem + L::DS_OFF), 16);
+    uint32_t g = 0, w = 0;
+    bool ok = true;
+    // S = Q K^T and dP = dO V^T of global step gs, which belongs to item wi (operands: Q/dO stage
+    // gs % QSTAGES, K/V buffer wi & 1).  The row threads must have read the pair of the step before out of
+    // TMEM; the first step of an item also waits for its K and V.
+    auto issue_sdp = [&](uint32_t gs, uint32_t wi, bool first_of_item) -> bool {
+      const int st = gs % L::QSTAGES, kb = wi & 1;
+      if (gs > 0 && !mbar_wait_warp(sdp_read, (gs - 1) & 1, abort_flag, status)) return false;
+      if (first_of_item && !mbar_wait_warp(&kv_full[kb], (wi >> 1) & 1, abort_flag, status)) return false;
+      if (!mbar_wait_warp(&q_full[st], (gs / L::QSTAGES) & 1, abort_flag, status)) return false;
+      tc_fence_after();
+      const uint32_t q_km = smem_desc_lo(smem_u32(smem + L::Q_OFF + st * ATT_TILE_BYTES), 16);
+      const uint32_t do_km = smem_desc_lo(smem_u32(smem + L::DO_OFF + st * ATT_TILE_BYTES), 16);
+      const uint32_t k_km = k_km0 + kb * KVBUF16, v_km = v_km0 + kb * KVBUF16;
+      if (elect_one()) {
 #pragma unroll
         for (int k = 0; k < 4; ++k) umma_bf16_lohi(tm_s, q_km + k * KSTEP, k_km + k * KSTEP, desc_hi, id_s, k > 0);
 #pragma unroll
         for (int k = 0; k < 4; ++k) umma_bf16_lohi(tm_dp, do_km + k * KSTEP, v_km + k * KSTEP, desc_hi, id_s, k > 0);
         umma_commit(sdp_full);
-        ATT_TRACE(tr, 256, tslot);          // S, dP issued
-        return true;
-      };
-      for (int r = 0; r < rounds && ok; ++r) {
-        int idx;
-        if (!att_item(r, cta, G, total, idx)) continue;
-        const int steps = nq - idx / n_bh;
-        bool more = false;                  // does this CTA have another item after this one?
-        for (int r2 = r + 1; r2 < rounds && !more; ++r2) {
-          int idx2;
-          more = att_item(r2, cta, G, total, idx2);
+      }
+      __syncwarp();
+      ATT_TRACE(tr, 256, tslot);          // S, dP issued
+      return true;
+    };
+    for (int r = 0; r < rounds && ok; ++r) {
+      int idx;
+      if (!att_item(r, cta, G, total, idx)) continue;
+      const int steps = nq - idx / n_bh;
+      bool more = false;                  // does this CTA have another item after this one?
+      for (int r2 = r + 1; r2 < rounds && !more; ++r2) {
+        int idx2;
+        more = att_item(r2, cta, G, total, idx2);
+      }
+      const int kb = w & 1;
+      const uint32_t k_mn = k_mn0 + kb * KVBUF16;
+      if (w == 0) ok = issue_sdp(0, 0, true);
+      for (int it = 0; it < steps && ok; ++it, ++g) {
+        const int s = g % L::QSTAGES;
+        const uint32_t sq = smem_u32(smem + L::Q_OFF + s * ATT_TILE_BYTES);
+        const uint32_t sdo = smem_u32(smem + L::DO_OFF + s * ATT_TILE_BYTES);
+        const uint32_t q_mn = smem_desc_lo(sq, ATT_TILE_BYTES), do_mn = smem_desc_lo(sdo, ATT_TILE_BYTES);
+        // The next step's pair goes as soon as the row threads have S and dP of this one in registers, while
+        // they are still writing P / dS: they find it finished when they come back for it.  Across items
+        // too: the next item's K and V sit in the other buffer.
+        if (it + 1 < steps) {
+          if (!issue_sdp(g + 1, w, false)) { ok = false; break; }
+        } else if (more) {
+          if (!issue_sdp(g + 1, w + 1, true)) { ok = false; break; }
         }
-        const int kb = w & 1;
-        const uint32_t k_mn = k_mn0 + kb * KVBUF16;
-        if (w == 0) ok = issue_sdp(0, 0, true);
-        for (int it = 0; it < steps && ok; ++it, ++g) {
-          const int s = g % L::QSTAGES;
-          const uint32_t sq = smem_u32(smem + L::Q_OFF + s * ATT_TILE_BYTES);
-          const uint32_t sdo = smem_u32(smem + L::DO_OFF + s * ATT_TILE_BYTES);
-          const uint32_t q_mn = smem_desc_lo(sq, ATT_TILE_BYTES), do_mn = smem_desc_lo(sdo, ATT_TILE_BYTES);
-          // The next step's pair goes as soon as the row threads have S and dP of this one in registers, while
-          // they are still writing P / dS: they find it finished when they come back for it.  Across items
-          // too: the next item's K and V sit in the other buffer.
-          if (it + 1 < steps) {
-            if (!issue_sdp(g + 1, w, false)) { ok = false; break; }
-          } else if (more) {
-            if (!issue_sdp(g + 1, w + 1, true)) { ok = false; break; }
-          }
-          if (!mbar_wait(pds_full, g & 1, abort_flag, status)) { ok = false; break; }
-          ATT_TRACE(tr, 256, tslot);          // P, dS ready
-          // a new item starts its dV / dK sums from zero: the previous item's must have been read out
-          if (it == 0 && w > 0 && !mbar_wait(dkv_free, (w - 1) & 1, abort_flag, status)) { ok = false; break; }
-          tc_fence_after();
+        if (!mbar_wait_warp(pds_full, g & 1, abort_flag, status)) { ok = false; break; }
+        ATT_TRACE(tr, 256, tslot);          // P, dS ready
+        // a new item starts its dV / dK sums from zero: the previous item's must have been read out
+        if (it == 0 && w > 0 && !mbar_wait_warp(dkv_free, (w - 1) & 1, abort_flag, status)) { ok = false; break; }
+        tc_fence_after();
+        if (elect_one()) {
 #pragma unroll
           for (int k = 0; k < 8; ++k)       // dV += P^T dO_i   (K = query rows, 16 per step)
             umma_bf16_lohi(tm_dv, p_mn + k * MNSTEP, do_mn + k * MNSTEP, desc_hi, id_t, (it > 0 || k > 0));
@@ -702,18 +721,22 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
           for (int k = 0; k < 8; ++k)       // dK += dS^T Q_i
             umma_bf16_lohi(tm_dk, ds_mn + k * MNSTEP, q_mn + k * MNSTEP, desc_hi, id_t, (it > 0 || k > 0));
           umma_commit(&q_empty[s]);         // Q_i and dO_i have their last readers queued: the stage reloads early
-          // the previous step's dQ has been read out of TMEM (the row threads do that right after their hand-over)
-          if (g > 0 && !mbar_wait(dq_free, (g - 1) & 1, abort_flag, status)) { ok = false; break; }
-          tc_fence_after();
+        }
+        __syncwarp();
+        // the previous step's dQ has been read out of TMEM (the row threads do that right after their hand-over)
+        if (g > 0 && !mbar_wait_warp(dq_free, (g - 1) & 1, abort_flag, status)) { ok = false; break; }
+        tc_fence_after();
+        if (elect_one()) {
 #pragma unroll
           for (int k = 0; k < 8; ++k)       // dQ_i = dS K_j     (K = kv rows)
             umma_bf16_lohi(tm_dq, ds_km + (k >> 2) * TILE16 + (k & 3) * KSTEP, k_mn + k * MNSTEP, desc_hi, id_q, k > 0);
           umma_commit(dq_full);
           if (it + 1 == steps) umma_commit(&kv_empty[kb]);
-          ATT_TRACE(tr, 256, tslot);          // dV, dK, dQ issued
         }
-        ++w;
+        __syncwarp();
+        ATT_TRACE(tr, 256, tslot);          // dV, dK, dQ issued
       }
+      ++w;
     }
   } else if (warp == RED_WARP) {
     // ------------------------------------------------------------ dQ reducer

@@ -49,6 +49,7 @@ struct GemmArgs {
   const __nv_bfloat16* resid; long long ldr;
   __nv_bfloat16* aux_out; const __nv_bfloat16* aux_in; long long ldaux;
   int* status;
+  int group;            // row tiles per group of the tile order
   int b_static;         // B is older than the kernel before in the stream (weights): it may be loaded before pdl_wait()
   long long* trace;     // optional: CTA 0's MMA thread stores %globaltimer stamps per k-block (tuning aid)
 };
@@ -264,6 +265,14 @@ __device__ __forceinline__ void drain_tile(const GemmArgs& g, uint32_t t_addr, i
   epilogue_warp<MODE, NCOLS>(g, t_addr, row_base, lane, col_base, stage, release);
 }
 
+// Tile `rem` of a slice of K: groups of g.group row tiles, all column tiles of a group before the next group.
+__device__ __forceinline__ void tile_at(const GemmArgs& g, int rem, int tiles_m, int tiles_n, int& mt, int& nt) {
+  const int per = g.group * tiles_n, grp = rem / per, r = rem - grp * per;
+  const int first = grp * g.group, rows = min(g.group, tiles_m - first);
+  nt = r / rows;
+  mt = first + r - nt * rows;
+}
+
 template <int BN, int NSTAGE>
 struct SmemLayout {
   static constexpr int A_BYTES = BM * BK * 2;
@@ -325,8 +334,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
       const int ks = tile / (tiles_m * tiles_n);
       const int rem = tile - ks * tiles_m * tiles_n;
-      const int m0 = (rem % tiles_m) * BM;
-      const int n0 = (rem / tiles_m) * BN;
+      int mt, nt;
+      tile_at(g, rem, tiles_m, tiles_n, mt, nt);
+      const int m0 = mt * BM, n0 = nt * BN;
       const int kb0 = ks * kb_per_split;
       const int kb1 = min(kb_total, kb0 + kb_per_split);
       for (int kb = kb0; kb < kb1; ++kb, ++it) {
@@ -418,15 +428,18 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     auto prefetch_tile = [&](int tile) {
       if (tile >= num_tiles) return;
       const int rem = tile % (tiles_m * tiles_n);
-      prefetch_extra<MODE, BN / 4>(g, (rem % tiles_m) * BM + q * 32, lane, (rem / tiles_m) * BN + part * (BN / 4));
+      int mt, nt;
+      tile_at(g, rem, tiles_m, tiles_n, mt, nt);
+      prefetch_extra<MODE, BN / 4>(g, mt * BM + q * 32, lane, nt * BN + part * (BN / 4));
     };
     pdl_wait();
     prefetch_tile(blockIdx.x);
     for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++tcount) {
       const int ks = tile / (tiles_m * tiles_n);
       const int rem = tile - ks * tiles_m * tiles_n;
-      const int m0 = (rem % tiles_m) * BM;
-      const int n0 = (rem / tiles_m) * BN;
+      int mt, nt;
+      tile_at(g, rem, tiles_m, tiles_n, mt, nt);
+      const int m0 = mt * BM, n0 = nt * BN;
       const int ab = tcount & 1;
       const uint32_t aph = (tcount >> 1) & 1;
       const bool has_k = ks * kb_per_split < kb_total;
@@ -540,8 +553,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
       const int ks = tile / (tiles_m * tiles_n);
       const int rem = tile - ks * tiles_m * tiles_n;
-      const int m0 = (rem % tiles_m) * 256 + int(rank) * 128;     // this CTA's rows of A
-      const int n0 = (rem / tiles_m) * BN + int(rank) * (BN / 2);      // this CTA's columns of B
+      int mt, nt;
+      tile_at(g, rem, tiles_m, tiles_n, mt, nt);
+      const int m0 = mt * 256 + int(rank) * 128;         // this CTA's rows of A
+      const int n0 = nt * BN + int(rank) * (BN / 2);     // this CTA's columns of B
       const int kb0 = ks * kb_per_split;
       const int kb1 = min(kb_total, kb0 + kb_per_split);
       for (int kb = kb0; kb < kb1; kb += KSUB, ++it) {
@@ -643,16 +658,18 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     auto prefetch_tile = [&](int tile) {
       if (tile >= num_tiles) return;
       const int rem = tile % (tiles_m * tiles_n);
-      prefetch_extra<MODE, BN / 4>(g, (rem % tiles_m) * 256 + int(rank) * 128 + q * 32, lane,
-                                   (rem / tiles_m) * BN + part * (BN / 4));
+      int mt, nt;
+      tile_at(g, rem, tiles_m, tiles_n, mt, nt);
+      prefetch_extra<MODE, BN / 4>(g, mt * 256 + int(rank) * 128 + q * 32, lane, nt * BN + part * (BN / 4));
     };
     pdl_wait();
     prefetch_tile(pair);
     for (int tile = pair; tile < num_tiles && ok; tile += num_pairs, ++tcount) {
       const int ks = tile / (tiles_m * tiles_n);
       const int rem = tile - ks * tiles_m * tiles_n;
-      const int m0 = (rem % tiles_m) * 256 + int(rank) * 128;
-      const int n0 = (rem / tiles_m) * BN;
+      int mt, nt;
+      tile_at(g, rem, tiles_m, tiles_n, mt, nt);
+      const int m0 = mt * 256 + int(rank) * 128, n0 = nt * BN;
       const int ab = tcount & 1;
       const uint32_t aph = (tcount >> 1) & 1;
       const bool has_k = ks * kb_per_split < kb_total;

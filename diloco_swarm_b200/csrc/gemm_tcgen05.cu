@@ -282,6 +282,10 @@ extern "C" int dsw_gemm_bf16(const void* A, long long lda, int a_mn_major, const
   g.aux_out = reinterpret_cast<__nv_bfloat16*>(aux_out);
   g.aux_in = reinterpret_cast<const __nv_bfloat16*>(aux_in); g.ldaux = ldaux;
   g.status = status;
+  // CTAs that run at the same time then share rows and columns: with all row tiles of a column first, 74 pairs read 75
+  // operand tiles at a time instead of some 20, and L2 gave out at 11 TB/s (16384 x 768 from K 3072: 65.7 -> 58.4 us,
+  // 16384 x 768 from 50304: 992 -> 864; neutral where one wave does, no difference between 4 and 24)
+  g.group = 8;
   g.b_static = tl_launch.static_b;
   g.trace = g_gemm_trace;
   if (few_rows) return launch_split(bn - 1000, ta, tb, g, stream);
