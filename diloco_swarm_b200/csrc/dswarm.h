@@ -45,6 +45,16 @@ int dsw_gemm_bf16(const void* A, long long lda, int a_mn_major, const void* B, l
                   int M, int N, int K, int mode, int split_k, void* out, long long ldo, const float* bias,
                   const void* resid, long long ldr, void* aux_out, const void* aux_in, long long ldaux, int bn,
                   int max_ctas, int* status, cudaStream_t stream);
+// Masked cross-entropy of logits = A [M,K] W[N,K]^T in pieces that never hold the logits: dsw_head_lse writes partial
+// log-sum-exps (fp32 [ceil(N / 64)][M]) and the target's logit (fp32 [M]), dsw_head_rows (elementwise.cu) joins them into
+// the loss and one 16-byte record per row, dsw_head_dlogits computes the logits again and stores scale / count *
+// (softmax - onehot), zeros in masked rows.
+int dsw_head_lse(const void* A, const void* W, const long long* targets, float* parts, float* tlogit, int M, int N, int K,
+                 int* status, cudaStream_t stream);
+int dsw_head_rows(const float* parts, const float* tlogit, const long long* targets, const long long* mask, const float* count,
+                  float scale, float* loss_acc, void* rows, int M, int N, int* status, cudaStream_t stream);
+int dsw_head_dlogits(const void* A, const void* W, const void* rows, void* out, int M, int N, int K, int* status,
+                     cudaStream_t stream);
 // Tracing build of the library only (-DDSWARM_TRACE): device buffer of 512 int64 that receives the timeline
 // stamps of CTA 0's MMA thread and first epilogue warp (null switches it off).  A no-op in the shipped build.
 int dsw_gemm_set_trace(long long* buf);

@@ -640,6 +640,60 @@ cross_entropy_kernel(__nv_bfloat16* __restrict__ logits, long long ld, const lon
   }
 }
 
+// Joins the partial log-sum-exps of 32 rows per block (lane = row, so every load is one 128-byte line; the warps share
+// out the groups), adds the kept rows' losses and leaves {lse2, scale / count or 0, target} per row when there is a
+// gradient to follow.  32768 rows of 786 groups are 103 MB: about 25 us, against 3.3 GB for the logits themselves.
+__global__ void __launch_bounds__(1024)
+head_rows_kernel(const float* __restrict__ parts, const float* __restrict__ tlogit, const long long* __restrict__ targets,
+                 const long long* __restrict__ mask, const float* __restrict__ count, float scale,
+                 float* __restrict__ loss_acc, float4* __restrict__ rows, int M, int V, int groups, int* status) {
+  __shared__ float shm[32][33], shs[32][33];
+  pdl_wait();
+  pdl_launch();
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int row = blockIdx.x * 32 + lane;
+  float m = -INFINITY, s = 0.f;
+  if (row < M) {
+    constexpr int U = 8;
+    for (int g0 = w; g0 < groups; g0 += U * nw) {
+      float v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) v[u] = g0 + u * nw < groups ? parts[(long long)(g0 + u * nw) * M + row] : -INFINITY;
+      float nm = m;
+#pragma unroll
+      for (int u = 0; u < U; ++u) nm = fmaxf(nm, v[u]);
+      const float ref = nm == -INFINITY ? 0.f : nm;
+      s *= ex2_approx(m - ref);
+#pragma unroll
+      for (int u = 0; u < U; ++u) s += ex2_approx(v[u] - ref);
+      m = nm;
+    }
+  }
+  shm[w][lane] = m;
+  shs[w][lane] = s;
+  __syncthreads();
+  if (w != 0) return;
+  float bm = -INFINITY, bs = 0.f;
+  for (int i = 0; i < nw; ++i) bm = fmaxf(bm, shm[i][lane]);
+  const float ref = bm == -INFINITY ? 0.f : bm;
+  for (int i = 0; i < nw; ++i) bs += shs[i][lane] * ex2_approx(shm[i][lane] - ref);
+  float loss = 0.f;
+  if (row < M) {
+    const bool keep = mask == nullptr || mask[row] != 0;
+    const float k = scale / (count ? fmaxf(count[0], 1.f) : 1.f);
+    const float lse2 = ref + log2f(bs);
+    long long t = targets[row];
+    if (t < 0 || t >= V) {
+      if (keep && status) atomicCAS(status, 0, ST_BAD_ARG);
+      t = 0;
+    }
+    if (keep) loss = k * (lse2 * 0.6931471805599453f - tlogit[row]);
+    if (rows) rows[row] = make_float4(lse2, keep ? k : 0.f, __int_as_float(int(t)), 0.f);
+  }
+  loss = warp_sum(loss);
+  if (lane == 0) atomicAdd(loss_acc, loss);
+}
+
 // ------------------------------------------------------------------ casts
 __global__ void cast_f32_bf16_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, long long n) {
   pdl_wait();
@@ -786,6 +840,17 @@ extern "C" int dsw_cross_entropy(void* logits, long long ld, const long long* ta
                 write_grad, status) == cudaSuccess ? 0 : -3;
 }
 
+extern "C" int dsw_head_rows(const float* parts, const float* tlogit, const long long* targets, const long long* mask,
+                             const float* count, float scale, float* loss_acc, void* rows, int M, int N, int* status,
+                             cudaStream_t st) {
+  if (M <= 0) return 0;
+  if (reinterpret_cast<uintptr_t>(rows) & 15) return -11;
+  const int groups = (N + 63) / 64;
+  const int warps = groups >= 256 ? 32 : groups >= 64 ? 8 : 2;
+  return launch(head_rows_kernel, (M + 31) / 32, 32 * warps, 0, st, 1, parts, tlogit, targets, mask, count, scale, loss_acc,
+                (float4*)rows, M, N, groups, status) == cudaSuccess ? 0 : -3;
+}
+
 extern "C" int dsw_cast_f32_bf16(const float* src, void* dst, long long n, cudaStream_t st) {
   return launch(cast_f32_bf16_kernel, grid_for(n / 8 + 1, 256), 256, 0, st, 1, src, (bf16*)dst, n) == cudaSuccess ? 0 : -3;
 }
@@ -841,7 +906,7 @@ extern "C" int dsw_load_elementwise() {
   L(layernorm_bwd_kernel<5>); L(layernorm_bwd_kernel<6>); L(layernorm_bwd_kernel<7>); L(layernorm_bwd_kernel<8>);
   L(layernorm_bwd_finish_kernel); L(colsum_kernel); L(embedding_fwd_kernel); L(embedding_bwd_kernel);
   L(embedding_bwd_sorted_kernel); L(embedding_bwd_pos_kernel);
-  L(mask_count_kernel); L(loss_begin_kernel); L(cross_entropy_kernel); L(cast_f32_bf16_kernel); L(cast_bf16_f32_kernel);
+  L(mask_count_kernel); L(loss_begin_kernel); L(cross_entropy_kernel); L(head_rows_kernel); L(cast_f32_bf16_kernel); L(cast_bf16_f32_kernel);
 #undef L
   return bad ? -1 : 0;
 }

@@ -37,7 +37,15 @@ enum EpiMode : int {
   EPI_MUL = 3,          // out = acc * aux_in  (aux_in = the gelu' saved by EPI_GELU: the GELU backward)
   EPI_ATOMIC_F32 = 4,   // out_f32 += acc   (split-K safe)
   EPI_STORE_F32 = 5,    // out_f32 = acc
+  // LM head without stored logits (dsw_head_lse / dsw_head_dlogits); acc = the logits of row and column
+  EPI_LSE = 6,          // parts[column / 64][row] = log2 of the sum of 2^(acc log2 e) over 64 columns; tlogit[row] = acc at the target
+  EPI_DLOGITS = 7,      // out = coef (softmax(acc) - onehot), lse2, target and coef from rows[row]
 };
+
+// What the second pass over the logits needs to know of a row: {log2-sum-exp2, factor (0: the row is masked), target as
+// int bits, unused}.
+typedef float4 HeadRow;
+constexpr int LSE_COLS = 64;            // columns per partial log-sum-exp: what one epilogue warp drains of a 256-wide tile
 
 struct GemmArgs {
   int M, N, K;
@@ -49,6 +57,8 @@ struct GemmArgs {
   const __nv_bfloat16* resid; long long ldr;
   __nv_bfloat16* aux_out; const __nv_bfloat16* aux_in; long long ldaux;
   int* status;
+  const long long* targets; float* parts; float* tlogit;      // EPI_LSE
+  const HeadRow* rows;                                         // EPI_DLOGITS
   int group;            // row tiles per group of the tile order
   int b_static;         // B is older than the kernel before in the stream (weights): it may be loaded before pdl_wait()
   long long* trace;     // optional: CTA 0's MMA thread stores %globaltimer stamps per k-block (tuning aid)
@@ -93,12 +103,87 @@ __device__ __forceinline__ void unstage_rows64(const uint8_t* stage, int lane, F
   }
 }
 
+// What a thread of the LM-head epilogues keeps of its row, asked for before the wait for the accumulator.
+template <int MODE>
+struct RowInfo {
+  __device__ __forceinline__ void load(const GemmArgs&, int) {}
+};
+template <>
+struct RowInfo<EPI_LSE> {
+  int target;
+  __device__ __forceinline__ void load(const GemmArgs& g, int row) {
+    const long long t = row < g.M ? g.targets[row] : 0;
+    target = t < 0 || t >= g.N ? 0 : int(t);          // reported by head_rows_kernel where the row counts
+  }
+};
+template <>
+struct RowInfo<EPI_DLOGITS> {
+  float lse2, coef;
+  int target;
+  __device__ __forceinline__ void load(const GemmArgs& g, int row) {
+    const HeadRow r = row < g.M ? g.rows[row] : make_float4(0.f, 0.f, 0.f, 0.f);
+    lse2 = r.x; coef = r.y; target = __float_as_int(r.z);
+  }
+};
+constexpr float LOG2E = 1.4426950408889634f;
+
 // NCOLS accumulator columns (a multiple of 32) starting at TMEM address t_addr, rows row_base..+31
 // (one per lane), output columns col_base..+NCOLS-1.  `release` is called once, right after the last
 // TMEM load has landed, so the MMA thread can refill the accumulator while the last chunk is written.
 template <int MODE, int NCOLS, class Release>
 __device__ __forceinline__ void epilogue_warp(const GemmArgs& g, uint32_t t_addr, int row_base, int lane, int col_base,
-                                              uint8_t* stage, Release&& release) {
+                                              uint8_t* stage, const RowInfo<MODE>& info, Release&& release) {
+  if constexpr (MODE == EPI_LSE) {
+    // Thread = row: maximum and sum of 2^(x - maximum) over the warp's 64 columns, straight from the fp32 accumulators.
+    // Per column one special-function operation and two packed halves; nothing but 4 bytes per 64 columns leaves the SM.
+    static_assert(NCOLS == LSE_COLS, "one partial result per warp and tile");
+    constexpr int NCH = NCOLS / 32;
+    uint32_t r[32];
+    tmem_ld_32x32(t_addr, r);
+    float m = -INFINITY, s = 0.f;
+#pragma unroll
+    for (int c = 0; c < NCH; ++c) {
+      const int cb = col_base + c * 32;
+      tmem_ld_wait();
+      float v[32];
+#pragma unroll
+      for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
+      if (c + 1 < NCH) tmem_ld_32x32(t_addr + (c + 1) * 32, r);
+      else release();
+      if (cb >= g.N) continue;
+      if (cb + 32 > g.N) {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v[i] = cb + i < g.N ? v[i] : -INFINITY;
+      }
+      if (unsigned(info.target - cb) < 32u && row_base + lane < g.M) {
+        float t = 0.f;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) t = cb + i == info.target ? v[i] : t;
+        g.tlogit[row_base + lane] = t;
+      }
+      float mx[4] = {v[0], v[1], v[2], v[3]};
+#pragma unroll
+      for (int i = 4; i < 32; ++i) mx[i & 3] = fmaxf(mx[i & 3], v[i]);
+      const float nm = fmaxf(m, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * LOG2E);
+      const float ref = nm == -INFINITY ? 0.f : nm;          // nothing but -inf so far: a sum of zeros
+      s *= ex2_approx(m - ref);
+      m = nm;
+      f2 acc[2] = {f2_bcast(0.f), f2_bcast(0.f)};
+      const f2 l2 = f2_bcast(LOG2E), neg = f2_bcast(-ref);
+#pragma unroll
+      for (int i = 0; i < 32; i += 2) {
+        float x0, x1;
+        f2_split(f2_fma(f2_make(v[i], v[i + 1]), l2, neg), x0, x1);
+        acc[(i >> 1) & 1] = f2_add(acc[(i >> 1) & 1], f2_make(ex2_approx(x0), ex2_approx(x1)));
+      }
+      float a0, a1;
+      f2_split(f2_add(acc[0], acc[1]), a0, a1);
+      s += a0 + a1;
+    }
+    if (col_base < g.N && row_base + lane < g.M)
+      g.parts[(long long)(col_base / LSE_COLS) * g.M + row_base + lane] = (m == -INFINITY ? 0.f : m) + log2f(s);
+    return;
+  } else
   if constexpr (MODE == EPI_ATOMIC_F32) {     // both fp32 outputs: accumulate (split-K safe) or plain store
     constexpr int NCH = NCOLS / 16;
     uint32_t r[16];
@@ -157,7 +242,32 @@ __device__ __forceinline__ void epilogue_warp(const GemmArgs& g, uint32_t t_addr
       // one evaluation of the fp32 sum; the derivative waits in registers until the activation chunk is out
       uint32_t w[16];
       uint32_t post[MODE == EPI_GELU ? 16 : 1];
-      if (chunk_ok) {
+      if constexpr (MODE == EPI_DLOGITS) {
+        if (chunk_ok) {
+          const f2 l2 = f2_bcast(LOG2E), neg = f2_bcast(-info.lse2), k2 = f2_bcast(info.coef);
+          auto pair = [&](int i) {
+            float x0, x1;
+            f2_split(f2_fma(f2_make(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), l2, neg), x0, x1);
+            return f2_mul(f2_make(ex2_approx(x0), ex2_approx(x1)), k2);
+          };
+#pragma unroll
+          for (int i = 0; i < 16; ++i) w[i] = pack_bf16_f2(pair(i));
+          if (unsigned(info.target - cb) < 32u) {            // one chunk of a row's 1572
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+              if (cb + 2 * i == (info.target & ~1)) {
+                float p0, p1;
+                f2_split(pair(i), p0, p1);
+                if (info.target & 1) p1 -= info.coef; else p0 -= info.coef;
+                w[i] = pack_bf16(p0, p1);
+              }
+          }
+          if (info.coef == 0.f) {                              // a masked row: zeros, whatever its logits are
+#pragma unroll
+            for (int i = 0; i < 16; ++i) w[i] = 0;
+          }
+        }
+      } else if (chunk_ok) {
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           const float4 bb = (g.bias != nullptr && cb + 4 * i < g.N) ? __ldg(reinterpret_cast<const float4*>(g.bias + cb) + i)
@@ -260,9 +370,9 @@ __device__ __forceinline__ void prefetch_extra(const GemmArgs& g, int row_base, 
 // that switched on the mode at run time carried the registers of every epilogue at once and spilled.
 template <int MODE, int NCOLS, class Release>
 __device__ __forceinline__ void drain_tile(const GemmArgs& g, uint32_t t_addr, int row_base, int lane, int col_base,
-                                           bool has_k, uint8_t* stage, Release&& release) {
+                                           bool has_k, uint8_t* stage, const RowInfo<MODE>& info, Release&& release) {
   if (!has_k) { release(); return; }
-  epilogue_warp<MODE, NCOLS>(g, t_addr, row_base, lane, col_base, stage, release);
+  epilogue_warp<MODE, NCOLS>(g, t_addr, row_base, lane, col_base, stage, info, release);
 }
 
 // Tile `rem` of a slice of K: groups of g.group row tiles, all column tiles of a group before the next group.
@@ -444,11 +554,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       const uint32_t aph = (tcount >> 1) & 1;
       const bool has_k = ks * kb_per_split < kb_total;
       prefetch_tile(tile + gridDim.x);
+      RowInfo<MODE> info;
+      info.load(g, m0 + q * 32 + lane);
       if (!mbar_wait(&acc_full[ab], aph, abort_flag, g.status)) { ok = false; break; }
       tc_fence_after();
       const uint32_t t_addr = tmem_base + ab * BN + part * (BN / 4) + (uint32_t(q * 32) << 16);
       drain_tile<MODE, BN / 4>(g, t_addr, m0 + q * 32, lane, n0 + part * (BN / 4), has_k,
-                         smem + L::EPI_OFFSET + (warp - EPI_WARP0) * EPI_STAGE_BYTES, [&] {
+                         smem + L::EPI_OFFSET + (warp - EPI_WARP0) * EPI_STAGE_BYTES, info, [&] {
         tmem_ld_wait();
         tc_fence_before();
         __syncwarp();
@@ -674,13 +786,15 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       const uint32_t aph = (tcount >> 1) & 1;
       const bool has_k = ks * kb_per_split < kb_total;
       prefetch_tile(tile + num_pairs);
+      RowInfo<MODE> info;
+      info.load(g, m0 + q * 32 + lane);
       GEMM_TRACE2(etr, eslot);
       if (!mbar_wait(&acc_full[ab], aph, abort_flag, g.status)) { ok = false; break; }
       GEMM_TRACE2(etr, eslot);
       tc_fence_after();
       const uint32_t t_addr = tmem_base + ab * BN + part * (BN / 4) + (uint32_t(q * 32) << 16);
       drain_tile<MODE, BN / 4>(g, t_addr, m0 + q * 32, lane, n0 + part * (BN / 4), has_k,
-                         smem + L::EPI_OFFSET + (warp - EPI_WARP0) * EPI_STAGE_BYTES, [&] {
+                         smem + L::EPI_OFFSET + (warp - EPI_WARP0) * EPI_STAGE_BYTES, info, [&] {
         tmem_ld_wait();
         tc_fence_before();
         __syncwarp();

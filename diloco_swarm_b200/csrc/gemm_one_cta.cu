@@ -37,8 +37,13 @@ int launch_bn(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& g, i
     case EPI_MUL: return launch_one<BN, NSTAGE, EPI_MUL>(ta, tb, g, num_sms, max_ctas, st);
     case EPI_ATOMIC_F32: return launch_one<BN, NSTAGE, EPI_ATOMIC_F32>(ta, tb, g, num_sms, max_ctas, st);
     case EPI_STORE: return launch_one<BN, NSTAGE, EPI_STORE>(ta, tb, g, num_sms, max_ctas, st);
-    default: return -13;
+    default: break;
   }
+  if constexpr (BN == 256) {          // the LM head's epilogues
+    if (g.mode == EPI_LSE) return launch_one<BN, NSTAGE, EPI_LSE>(ta, tb, g, num_sms, max_ctas, st);
+    if (g.mode == EPI_DLOGITS) return launch_one<BN, NSTAGE, EPI_DLOGITS>(ta, tb, g, num_sms, max_ctas, st);
+  }
+  return -13;
 }
 
 template <int BN, int NSTAGE>
@@ -50,6 +55,10 @@ int load_bn() {
   bad |= cudaFuncGetAttributes(&a, gemm_kernel<BN, NSTAGE, EPI_RESID>) != cudaSuccess;
   bad |= cudaFuncGetAttributes(&a, gemm_kernel<BN, NSTAGE, EPI_MUL>) != cudaSuccess;
   bad |= cudaFuncGetAttributes(&a, gemm_kernel<BN, NSTAGE, EPI_ATOMIC_F32>) != cudaSuccess;
+  if constexpr (BN == 256) {
+    bad |= cudaFuncGetAttributes(&a, gemm_kernel<BN, NSTAGE, EPI_LSE>) != cudaSuccess;
+    bad |= cudaFuncGetAttributes(&a, gemm_kernel<BN, NSTAGE, EPI_DLOGITS>) != cudaSuccess;
+  }
   return bad;
 }
 }  // namespace

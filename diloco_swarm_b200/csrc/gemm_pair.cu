@@ -36,8 +36,13 @@ int launch_bn(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& g, i
     case EPI_MUL: return launch_pair_mode<BN, EPI_MUL>(ta, tb, g, num_sms, max_ctas, st);
     case EPI_ATOMIC_F32: return launch_pair_mode<BN, EPI_ATOMIC_F32>(ta, tb, g, num_sms, max_ctas, st);
     case EPI_STORE: return launch_pair_mode<BN, EPI_STORE>(ta, tb, g, num_sms, max_ctas, st);
-    default: return -13;
+    default: break;
   }
+  if constexpr (BN == 256) {          // the LM head's epilogues
+    if (g.mode == EPI_LSE) return launch_pair_mode<BN, EPI_LSE>(ta, tb, g, num_sms, max_ctas, st);
+    if (g.mode == EPI_DLOGITS) return launch_pair_mode<BN, EPI_DLOGITS>(ta, tb, g, num_sms, max_ctas, st);
+  }
+  return -13;
 }
 
 template <int BN>
@@ -49,6 +54,10 @@ int load_bn() {
   bad |= cudaFuncGetAttributes(&a, gemm_pair_kernel<BN, EPI_RESID>) != cudaSuccess;
   bad |= cudaFuncGetAttributes(&a, gemm_pair_kernel<BN, EPI_MUL>) != cudaSuccess;
   bad |= cudaFuncGetAttributes(&a, gemm_pair_kernel<BN, EPI_ATOMIC_F32>) != cudaSuccess;
+  if constexpr (BN == 256) {
+    bad |= cudaFuncGetAttributes(&a, gemm_pair_kernel<BN, EPI_LSE>) != cudaSuccess;
+    bad |= cudaFuncGetAttributes(&a, gemm_pair_kernel<BN, EPI_DLOGITS>) != cudaSuccess;
+  }
   return bad;
 }
 }  // namespace

@@ -273,7 +273,7 @@ extern "C" int dsw_gemm_bf16(const void* A, long long lda, int a_mn_major, const
   if (!b_mn_major) rc = cached_tmap(&tb, TMAP_BF16_2D, B, K, 1, N, ldb, BK, bn == 512 ? 128 : bn == 384 ? 64 : bn % 1000);
   else             rc = cached_tmap(&tb, TMAP_BF16_2D, B, N, 1, K, ldb, 64, BK);
   if (rc) return rc;
-  GemmArgs g;
+  GemmArgs g = {};
   g.M = M; g.N = N; g.K = K;
   g.a_mn_major = a_mn_major; g.b_mn_major = b_mn_major;
   g.mode = mode; g.split_k = split_k;
@@ -291,6 +291,43 @@ extern "C" int dsw_gemm_bf16(const void* A, long long lda, int a_mn_major, const
   if (few_rows) return launch_split(bn - 1000, ta, tb, g, stream);
   if (bn == 512 || bn == 384) return launch_pair(bn == 512 ? 256 : 128, ta, tb, g, num_sms[dev], max_ctas, stream);
   return launch_one_cta(bn, ta, tb, g, num_sms[dev], max_ctas, stream);
+}
+
+// Logits = A [M,K] W[N,K]^T (both row-major bf16) that are not stored: one of the LM head's two epilogues on 256-wide tiles.
+static int head_gemm(const void* A, const void* W, int M, int N, int K, int mode, void* out, const long long* targets, float* parts,
+                     float* tlogit, const HeadRow* rows, int* status, cudaStream_t stream) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if (K % 8 || N % 8) return -10;
+  if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(out) |
+       reinterpret_cast<uintptr_t>(rows)) & 15)
+    return -11;
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return -2;
+  const bool pair = use_pair() && M >= 256;
+  CUtensorMap ta, tb;
+  int rc = cached_tmap(&ta, TMAP_BF16_2D, A, K, 1, M, K, BK, BM);
+  if (rc == 0) rc = cached_tmap(&tb, TMAP_BF16_2D, W, K, 1, N, K, BK, pair ? 128 : 256);
+  if (rc) return rc;
+  GemmArgs g = {};
+  g.M = M; g.N = N; g.K = K;
+  g.mode = mode; g.split_k = 1;
+  g.out = out; g.ldo = N;
+  g.targets = targets; g.parts = parts; g.tlogit = tlogit; g.rows = rows;
+  g.status = status;
+  g.group = 8;
+  const int cap = default_max_ctas();
+  return pair ? launch_pair(256, ta, tb, g, sms, cap, stream) : launch_one_cta(256, ta, tb, g, sms, cap, stream);
+}
+
+// parts [ceil(N / 64)][M], tlogit [M]: see EPI_LSE; a target outside [0, N) counts as 0 here and is reported by dsw_head_rows.
+extern "C" int dsw_head_lse(const void* A, const void* W, const long long* targets, float* parts, float* tlogit, int M, int N, int K,
+                            int* status, cudaStream_t stream) {
+  return head_gemm(A, W, M, N, K, EPI_LSE, nullptr, targets, parts, tlogit, nullptr, status, stream);
+}
+// out [M,N] bf16 = gradient of the loss by the logits, rows [M] as dsw_head_rows wrote them.
+extern "C" int dsw_head_dlogits(const void* A, const void* W, const void* rows, void* out, int M, int N, int K, int* status,
+                                cudaStream_t stream) {
+  return head_gemm(A, W, M, N, K, EPI_DLOGITS, out, nullptr, nullptr, nullptr, static_cast<const HeadRow*>(rows), status, stream);
 }
 
 // Force the modules that hold the GEMM kernels to load now (see dsw_load_all).

@@ -159,14 +159,35 @@ SavedAll take_saved(Area& a, const Stage& s, size_t M, bool keep) {
 
 struct Scratch {
   bf16 *dh[2], *dx[3], *dx1[2], *dqkv[2], *dln, *datt, *logits;
+  float *parts, *tlogit;         // see dsw_head_lse
+  float4* rows;                  // see dsw_head_rows
   float *dq_acc, *dvec, *ln;
 };
+
+// Whether the cross-entropy of a pass goes without stored logits (dsw_head_lse and its companions; tiles are 256 columns
+// wide).  Without a gradient always: no logits are written and read again (width 768, 32768 rows: 3007 -> 1749 us, 128
+// rows: 37 -> 32).  With one they have to be computed a second time, which narrow models do faster than they read and
+// write them once more, given enough rows for the third launch (us, stored / unstored, 50304 columns; width 128: 512 rows
+// 49 / 51, 2048 145 / 120, 32768 2018 / 1750; width 384: 512 rows 68 / 78, 2048 219 / 182, 32768 2820 / 2083; width 768:
+// 2048 rows 267 / 287, 32768 3512 / 3823).
+constexpr int HEAD_TWICE_WIDTH = 384, HEAD_TWICE_ROWS = 1024;
+bool unstored_logits(const Stage& s, bool grad, size_t rows) {
+  return s.V > 128 && (!grad || (s.d <= HEAD_TWICE_WIDTH && rows >= size_t(HEAD_TWICE_ROWS)));
+}
 
 // logit_rows: rows of the logits that exist at a time (0: the caller keeps them elsewhere)
 Scratch take_scratch(Area& a, const Stage& s, size_t M, bool grad, size_t logit_rows) {
   const size_t d = s.d;
   Scratch v = {};
-  v.logits = s.head_w && logit_rows ? a.take<bf16>(logit_rows * s.V) : nullptr;
+  if (s.head_w && logit_rows) {
+    const bool unstored = unstored_logits(s, grad, logit_rows);
+    if (grad || !unstored) v.logits = a.take<bf16>(logit_rows * s.V);
+    if (unstored) {
+      v.parts = a.take<float>((size_t(s.V) + 63) / 64 * logit_rows);
+      v.tlogit = a.take<float>(logit_rows);
+      v.rows = a.take<float4>(logit_rows);
+    }
+  }
   if (!grad) return v;
   for (int p = 0; p < 2; ++p) {
     v.dh[p] = a.take<bf16>(M * 4 * d);
@@ -513,25 +534,38 @@ extern "C" int dsw_stage_head(void* stage, void* saved, void* scratch, const lon
   if (s.head_used) MAIN_WAIT(s.head_done);
   LAUNCH(dsw_loss_begin(mask, M, s.count, loss, st));
   const int flags = (keep ? 1 : 0) | (deterministic ? 2 : 0) | chunks << 2;
+  const bool unstored = unstored_logits(s, grad != 0, rows);
+  const auto dlogits = [&](const bf16* ln, int m) {
+    return dsw_head_dlogits(ln, s.head_w, c.rows, c.logits, m, V, d, s.status, r.st);
+  };
   TRY(r.replayed(GraphKey{1, B, T, flags, {saved, scratch, nullptr, nullptr, nullptr, nullptr}}, [&]() -> int {
     LAUNCH(dsw_layernorm_fwd(x, s.lnf_w, s.lnf_b, v.lnf, v.muf, v.rsf, M, d, 1e-5f, r.st));
-    if (rows == M) LAUNCH(r.gemm(v.lnf, s.head_w, true, V, d, c.logits, DSW_EPI_STORE, nullptr, nullptr, nullptr, nullptr, M));
+    if (rows == M && !unstored) LAUNCH(r.gemm(v.lnf, s.head_w, true, V, d, c.logits, DSW_EPI_STORE, nullptr, nullptr, nullptr, nullptr, M));
     return 0;
   }));
   for (int r0 = 0; r0 < M; r0 += rows) {
     const int m = M - r0 < rows ? M - r0 : rows;
     const bf16* ln = v.lnf + size_t(r0) * d;
-    if (rows < M) {
-      if (s.head_used) MAIN_WAIT(s.head_done);      // the slice before is still read
-      LAUNCH(r.gemm(ln, s.head_w, true, V, d, c.logits, DSW_EPI_STORE, nullptr, nullptr, nullptr, nullptr, m));
+    const long long* mk = mask ? mask + r0 : nullptr;
+    if (unstored) {
+      LAUNCH(dsw_head_lse(ln, s.head_w, targets + r0, c.parts, c.tlogit, m, V, d, s.status, st));
+      LAUNCH(dsw_head_rows(c.parts, c.tlogit, targets + r0, mk, s.count, scale, loss, grad ? c.rows : nullptr, m, V, s.status, st));
     }
-    LAUNCH(dsw_cross_entropy(c.logits, V, targets + r0, mask ? mask + r0 : nullptr, s.count, scale, loss, m, V, grad, s.status, st));
+    if (rows < M && grad && s.head_used) MAIN_WAIT(s.head_done);      // the slice before is still read
+    if (!unstored) {
+      if (rows < M) LAUNCH(r.gemm(ln, s.head_w, true, V, d, c.logits, DSW_EPI_STORE, nullptr, nullptr, nullptr, nullptr, m));
+      LAUNCH(dsw_cross_entropy(c.logits, V, targets + r0, mk, s.count, scale, loss, m, V, grad, s.status, st));
+    }
     if (!grad || rows == M) continue;
+    if (unstored) LAUNCH(dlogits(ln, m));
     TRY(r.head_grads(c, ln, r0, m));
   }
   if (!grad) return 0;
   TRY(r.replayed(GraphKey{2, B, T, flags, {saved, scratch, nullptr, nullptr, nullptr, nullptr}}, [&]() -> int {
-    if (rows == M) TRY(r.head_grads(c, v.lnf, 0, M));
+    if (rows == M) {
+      if (unstored) LAUNCH(dlogits(v.lnf, M));
+      TRY(r.head_grads(c, v.lnf, 0, M));
+    }
     LAUNCH(dsw_layernorm_bwd(c.dln, x, s.lnf_w, v.muf, v.rsf, nullptr, c.dx[s.n % 3], s.dlnf_w, s.dlnf_b, nullptr, c.ln, M, d, r.st));
     return 0;
   }));

@@ -36,6 +36,10 @@ _SIGS = {
     "dsw_loss_begin": [c_void_p, c_int, c_void_p, c_void_p, c_void_p],
     "dsw_cross_entropy": [c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_int, c_int, c_int,
                           c_void_p, c_void_p],
+    "dsw_head_lse": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p],
+    "dsw_head_rows": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_void_p, c_int, c_int, c_void_p,
+                      c_void_p],
+    "dsw_head_dlogits": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p],
     "dsw_cast_f32_bf16": [c_void_p, c_void_p, c_ll, c_void_p],
     "dsw_cast_bf16_f32": [c_void_p, c_void_p, c_ll, c_void_p],
     "dsw_sumsq": [c_void_p, c_ll, c_void_p, c_void_p],
