@@ -55,6 +55,11 @@ int dsw_head_rows(const float* parts, const float* tlogit, const long long* targ
                   float scale, float* loss_acc, void* rows, int M, int N, int* status, cudaStream_t stream);
 int dsw_head_dlogits(const void* A, const void* W, const void* rows, void* out, int M, int N, int K, int* status,
                      cudaStream_t stream);
+// partials[s] (fp32 [M,N] each, *splits <= most of them) = A [M,K] B [K,N] over slice s of K.
+int dsw_gemm_partials(const void* A, const void* B, int M, int N, int K, float* partials, int most, int* splits, int* status,
+                      cudaStream_t stream);
+// out (bf16) = the sum of `splits` arrays of n fp32 values, in order; n a multiple of 8
+int dsw_sum_partials_bf16(const float* partials, int splits, void* out, long long n, cudaStream_t st);
 // Tracing build of the library only (-DDSWARM_TRACE): device buffer of 512 int64 that receives the timeline
 // stamps of CTA 0's MMA thread and first epilogue warp (null switches it off).  A no-op in the shipped build.
 int dsw_gemm_set_trace(long long* buf);

@@ -36,7 +36,7 @@ enum EpiMode : int {
   EPI_RESID = 2,        // out = acc + bias + resid (+ aux_in); aux_out (optional) = what rounding out to bf16 left over
   EPI_MUL = 3,          // out = acc * aux_in  (aux_in = the gelu' saved by EPI_GELU: the GELU backward)
   EPI_ATOMIC_F32 = 4,   // out_f32 += acc   (split-K safe)
-  EPI_STORE_F32 = 5,    // out_f32 = acc
+  EPI_STORE_F32 = 5,    // out_f32 = acc; split of K number s stores split_stride * s elements further on
   // LM head without stored logits (dsw_head_lse / dsw_head_dlogits); acc = the logits of row and column
   EPI_LSE = 6,          // parts[column / 64][row] = log2 of the sum of 2^(acc log2 e) over 64 columns; tlogit[row] = acc at the target
   EPI_DLOGITS = 7,      // out = coef (softmax(acc) - onehot), lse2, target and coef from rows[row]
@@ -59,6 +59,7 @@ struct GemmArgs {
   int* status;
   const long long* targets; float* parts; float* tlogit;      // EPI_LSE
   const HeadRow* rows;                                         // EPI_DLOGITS
+  long long split_stride;                                      // EPI_STORE_F32
   int group;            // row tiles per group of the tile order
   int b_static;         // B is older than the kernel before in the stream (weights): it may be loaded before pdl_wait()
   long long* trace;     // optional: CTA 0's MMA thread stores %globaltimer stamps per k-block (tuning aid)
@@ -103,15 +104,20 @@ __device__ __forceinline__ void unstage_rows64(const uint8_t* stage, int lane, F
   }
 }
 
-// What a thread of the LM-head epilogues keeps of its row, asked for before the wait for the accumulator.
+// What an epilogue keeps of its row and tile; loads are asked for before the wait for the accumulator.
 template <int MODE>
 struct RowInfo {
-  __device__ __forceinline__ void load(const GemmArgs&, int) {}
+  __device__ __forceinline__ void load(const GemmArgs&, int, int) {}
+};
+template <>
+struct RowInfo<EPI_ATOMIC_F32> {
+  float* out;
+  __device__ __forceinline__ void load(const GemmArgs& g, int, int ks) { out = reinterpret_cast<float*>(g.out) + ks * g.split_stride; }
 };
 template <>
 struct RowInfo<EPI_LSE> {
   int target;
-  __device__ __forceinline__ void load(const GemmArgs& g, int row) {
+  __device__ __forceinline__ void load(const GemmArgs& g, int row, int) {
     const long long t = row < g.M ? g.targets[row] : 0;
     target = t < 0 || t >= g.N ? 0 : int(t);          // reported by head_rows_kernel where the row counts
   }
@@ -120,7 +126,7 @@ template <>
 struct RowInfo<EPI_DLOGITS> {
   float lse2, coef;
   int target;
-  __device__ __forceinline__ void load(const GemmArgs& g, int row) {
+  __device__ __forceinline__ void load(const GemmArgs& g, int row, int) {
     const HeadRow r = row < g.M ? g.rows[row] : make_float4(0.f, 0.f, 0.f, 0.f);
     lse2 = r.x; coef = r.y; target = __float_as_int(r.z);
   }
@@ -204,7 +210,7 @@ __device__ __forceinline__ void epilogue_warp(const GemmArgs& g, uint32_t t_addr
       unstage_rows64(stage, lane, [&](int, int rl, int ch, const uint4& d) {
         const int row = row_base + rl, col = cb + ch * 4;
         if (row < g.M && col < g.N) {
-          float* o = reinterpret_cast<float*>(g.out) + (long long)row * g.ldo + col;
+          float* o = info.out + (long long)row * g.ldo + col;
           if (g.mode == EPI_ATOMIC_F32)
             asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(o), "f"(__uint_as_float(d.x)),
                          "f"(__uint_as_float(d.y)), "f"(__uint_as_float(d.z)), "f"(__uint_as_float(d.w))
@@ -555,7 +561,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       const bool has_k = ks * kb_per_split < kb_total;
       prefetch_tile(tile + gridDim.x);
       RowInfo<MODE> info;
-      info.load(g, m0 + q * 32 + lane);
+      info.load(g, m0 + q * 32 + lane, ks);
       if (!mbar_wait(&acc_full[ab], aph, abort_flag, g.status)) { ok = false; break; }
       tc_fence_after();
       const uint32_t t_addr = tmem_base + ab * BN + part * (BN / 4) + (uint32_t(q * 32) << 16);
@@ -787,7 +793,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       const bool has_k = ks * kb_per_split < kb_total;
       prefetch_tile(tile + num_pairs);
       RowInfo<MODE> info;
-      info.load(g, m0 + q * 32 + lane);
+      info.load(g, m0 + q * 32 + lane, ks);
       GEMM_TRACE2(etr, eslot);
       if (!mbar_wait(&acc_full[ab], aph, abort_flag, g.status)) { ok = false; break; }
       GEMM_TRACE2(etr, eslot);

@@ -196,7 +196,7 @@ static int pick_few_rows(int M, int N, int K, bool b_mn, int sms, double many_ro
 // of which about 0.4 shows beside the main loops; parts that meet on one address wait for one another.  Fitted to
 // 128 x 128 ... 6400 x 1600 with 128 to 16384 tokens (5120 x 1280, 2128 tokens: 4 splits by the earlier rule, which filled
 // the last wave at any price, 43.4 us; 2 splits 32.6 us).
-static int pick_wgrad(int M, int N, int K, int bn, int sms, int* split) {
+static int pick_wgrad(int M, int N, int K, int bn, int sms, int* split, int most = 64) {
   const int kb = (K + BK - 1) / BK, fixed = *split;
   const double mb = 4.0 * M * N;
   double least = 1e30;
@@ -207,7 +207,7 @@ static int pick_wgrad(int M, int N, int K, int bn, int sms, int* split) {
     const int units = sms / t.ctas;
     for (int s : {1, 2, 3, 4, 5, 6, 8, 10, 12, 16, 24, 32, 48, 64}) {
       if (fixed) s = fixed;
-      if (s > 1 && kb / s < 2 && !fixed) continue;
+      if (s > 1 && (kb / s < 2 || s > most) && !fixed) continue;
       const double c = t.setup_wgrad + double((tiles * s + units - 1) / units) * ((kb + s - 1) / s) * t.per_kb_wgrad +
                        0.4 * mb * s / 4300.0 + 30.0 * s;
       if (c < least) { least = c; best = t.bn; best_split = s; }
@@ -328,6 +328,36 @@ extern "C" int dsw_head_lse(const void* A, const void* W, const long long* targe
 extern "C" int dsw_head_dlogits(const void* A, const void* W, const void* rows, void* out, int M, int N, int K, int* status,
                                 cudaStream_t stream) {
   return head_gemm(A, W, M, N, K, EPI_DLOGITS, out, nullptr, nullptr, nullptr, static_cast<const HeadRow*>(rows), status, stream);
+}
+
+// Partial products of A [M,K] (row-major) and B [K,N] (row-major) over slices of K, for outputs of too few tiles to fill the
+// SMs: slice s goes to partials + s * M * N (fp32, at most `most` slices, their number to *splits), and
+// dsw_sum_partials_bf16 adds them in order.  Sums that meet in atomics would do too, but their order, and with it the last
+// bit of what rounds to bf16 from here on, would change from run to run.
+extern "C" int dsw_gemm_partials(const void* A, const void* B, int M, int N, int K, float* partials, int most, int* splits,
+                                 int* status, cudaStream_t stream) {
+  *splits = 0;
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if (K % 8 || N % 8) return -10;
+  if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(partials)) & 15) return -11;
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return -2;
+  int split = 0;
+  const int bn = pick_wgrad(M, N, K, 0, sms, &split, most);
+  CUtensorMap ta, tb;
+  int rc = cached_tmap(&ta, TMAP_BF16_2D, A, K, 1, M, K, BK, BM);
+  if (rc == 0) rc = cached_tmap(&tb, TMAP_BF16_2D, B, N, 1, K, N, 64, BK);
+  if (rc) return rc;
+  GemmArgs g = {};
+  g.M = M; g.N = N; g.K = K;
+  g.b_mn_major = 1;
+  g.mode = EPI_STORE_F32; g.split_k = split; g.split_stride = (long long)M * N;
+  g.out = partials; g.ldo = N;
+  g.status = status;
+  g.group = 8;
+  *splits = split;
+  const int cap = default_max_ctas();
+  return bn >= 384 ? launch_pair(bn == 512 ? 256 : 128, ta, tb, g, sms, cap, stream) : launch_one_cta(bn, ta, tb, g, sms, cap, stream);
 }
 
 // Force the modules that hold the GEMM kernels to load now (see dsw_load_all).

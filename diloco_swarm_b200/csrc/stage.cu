@@ -391,14 +391,13 @@ struct Run {
     }
     bf16* dln = c.dln + size_t(r0) * s.d;
     // m x d output tiles and a K of the whole vocabulary: few of them leave most SMs idle for hundreds of k-blocks (2128
-    // rows of GPT-2 small: 27 CTA pairs, 238 us), so K is split as in a weight gradient, with the fp32 sums in the
-    // scratch that the attention backward uses later.  Not with deterministic gradients: the sums meet in atomics.
-    if (!deterministic && ((m + 255) / 256) * ((s.d + 255) / 256) < 74) {
-      TRY_CUDA(cudaMemsetAsync(c.dq_acc, 0, size_t(m) * s.d * sizeof(float), st));
-      dsw::tl_launch.pdl = false;
-      LAUNCH(dsw_gemm_bf16(c.logits, s.V, 0, s.head_w, s.d, 1, m, s.d, s.V, DSW_EPI_ATOMIC_F32, 0, c.dq_acc, s.d, nullptr, nullptr, 0,
-                           nullptr, nullptr, 0, 0, 0, s.status, st));
-      LAUNCH(dsw_cast_f32_bf16(c.dq_acc, dln, (long long)m * s.d, st));
+    // rows of GPT-2 small: 27 CTA pairs, 238 us), so K is split, with the partial sums in the buffers of the blocks'
+    // backward, which have not begun: dh, dx1 and dqkv of both parities lie side by side and hold 8 m x d fp32 arrays.
+    if (((m + 255) / 256) * ((s.d + 255) / 256) < 74) {
+      float* partials = reinterpret_cast<float*>(c.dh[0]);
+      int splits = 0;
+      LAUNCH(dsw_gemm_partials(c.logits, s.head_w, m, s.d, s.V, partials, 8, &splits, s.status, st));
+      LAUNCH(dsw_sum_partials_bf16(partials, splits, dln, (long long)m * s.d, st));
       return 0;
     }
     LAUNCH(gemm(c.logits, s.head_w, false, s.d, s.V, dln, DSW_EPI_STORE, nullptr, nullptr, nullptr, nullptr, m));
