@@ -18,6 +18,13 @@ __device__ __forceinline__ float warp_sum(float v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
+// The same over each group of LANES neighbouring lanes.
+template <int LANES>
+__device__ __forceinline__ float group_sum(float v) {
+#pragma unroll
+  for (int o = LANES / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
 __device__ __forceinline__ float warp_max(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
@@ -66,20 +73,25 @@ __device__ __forceinline__ void ln_load_row(uint4 (&o)[NCH], const __nv_bfloat16
 #pragma unroll
   for (int c = 0; c < NCH; ++c) {
     const int col = c * 256 + lane * 8;
-    o[c] = (col < d && DSW_OK(row >= 0 && row < M && col + 8 <= d)) ? *reinterpret_cast<const uint4*>(xr + col)
+    o[c] = (col < d && row < M && DSW_OK(row >= 0 && col + 8 <= d)) ? *reinterpret_cast<const uint4*>(xr + col)
                                                                    : make_uint4(0, 0, 0, 0);
   }
 }
 
 // LO: the row is the sum of two bf16 arrays (a residual stream kept with the bits that rounding to bf16 leaves over).
-template <int NCH, bool LO>
+// LPR: lanes per row.  A row of up to 128 columns takes half a warp, two rows per warp and step: with a whole warp per row
+// half of the lanes had nothing to load, and a warp's chain of rows (load, two reductions, store) set the time.
+template <int NCH, bool LO, int LPR>
 __global__ void __launch_bounds__(256)
 layernorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ x_lo, const float* __restrict__ gamma,
                      const float* __restrict__ beta, __nv_bfloat16* __restrict__ y, float* __restrict__ mean_out,
                      float* __restrict__ rstd_out, int M, int d, float eps) {
-  const int lane = threadIdx.x & 31;
-  const int stride = gridDim.x * (blockDim.x >> 5);
-  int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  static_assert(LPR == 32 || NCH == 1, "rows that share a warp are one chunk long");
+  const int lane = threadIdx.x & (LPR - 1);
+  const int stride = gridDim.x * (blockDim.x / LPR);
+  // the warp's first row; its other group of lanes may find itself past the last one and only takes part in the shuffles
+  int first = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * (32 / LPR);
+  int row = first + (threadIdx.x & 31) / LPR;
   float g[NCH][8], b[NCH][8];
 #pragma unroll
   for (int c = 0; c < NCH; ++c) {
@@ -92,13 +104,13 @@ layernorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* _
     }
   }
   const float inv_d = 1.f / d;
-  if (row >= M) return;
+  if (first >= M) return;
   pdl_wait();          // gamma and beta above are older than the kernel before
   pdl_launch();
   uint4 cur[NCH], nxt[NCH];
   ln_load_row<NCH>(cur, x, row, d, lane, M);
-  for (; row < M; row += stride) {
-    const bool more = row + stride < M;
+  for (; first < M; first += stride, row += stride) {
+    const bool more = first + stride < M;
     if (more) ln_load_row<NCH>(nxt, x, row + stride, d, lane, M);
     uint4 low[LO ? NCH : 1];
     if constexpr (LO) ln_load_row<NCH>(low, x_lo, row, d, lane, M);
@@ -119,7 +131,7 @@ layernorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* _
 #pragma unroll
       for (int j = 0; j < 8; ++j) s += v[j];
     }
-    const float mean = warp_sum(s) * inv_d;
+    const float mean = group_sum<LPR>(s) * inv_d;
     float q = 0.f;
 #pragma unroll
     for (int c = 0; c < NCH; ++c) {
@@ -130,13 +142,13 @@ layernorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* _
         for (int j = 0; j < 8; ++j) { const float t = v[j] - mean; q += t * t; }
       }
     }
-    const float rstd = rsqrtf(warp_sum(q) * inv_d + eps);
-    if (lane == 0) { mean_out[row] = mean; rstd_out[row] = rstd; }
+    const float rstd = rsqrtf(group_sum<LPR>(q) * inv_d + eps);
+    if (lane == 0 && row < M) { mean_out[row] = mean; rstd_out[row] = rstd; }
     __nv_bfloat16* yr = y + (long long)row * d;
 #pragma unroll
     for (int c = 0; c < NCH; ++c) {
       const int col = c * 256 + lane * 8;
-      if (col < d && DSW_OK(row < M && col + 8 <= d)) {
+      if (col < d && row < M && DSW_OK(col + 8 <= d)) {
         float v[8], o[8];
         value(c, v);
 #pragma unroll
@@ -172,36 +184,38 @@ template <int NCH>
 __device__ __forceinline__ void ln_bwd_load(LnBwdRow<NCH>& o, const __nv_bfloat16* __restrict__ dy,
                                             const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dres,
                                             const float* __restrict__ mean_in, const float* __restrict__ rstd_in,
-                                            int row, int d, int nch, int lane) {
+                                            int row, int M, int d, int nch, int lane) {
   const long long off = (long long)row * d;
 #pragma unroll
   for (int c = 0; c < NCH; ++c) {
     const int col = c * 256 + lane * 8;
-    if (c < nch && col < d && DSW_OK(row >= 0 && col + 8 <= d)) {
+    if (c < nch && col < d && row < M && DSW_OK(row >= 0 && col + 8 <= d)) {
       o.x[c] = *reinterpret_cast<const uint4*>(x + off + col);
       o.dy[c] = *reinterpret_cast<const uint4*>(dy + off + col);
       if (dres) o.r[c] = *reinterpret_cast<const uint4*>(dres + off + col);
     }
   }
-  o.mean = mean_in[row];
-  o.rstd = rstd_in[row];
+  o.mean = row < M ? mean_in[row] : 0.f;
+  o.rstd = row < M ? rstd_in[row] : 0.f;
 }
 
-// Blocks per SM: rows up to 768 columns keep the column sums, gamma and two rows (the current one and the
-// prefetched next one) in registers, about 200 per thread, so one block; wider rows use the strips, two blocks.
-constexpr int ln_bwd_blocks_per_sm(int nch) { return nch <= 3 ? 1 : 2; }
+// Blocks per SM: rows of 264 to 768 columns keep the column sums, gamma and two rows (the current one and the
+// prefetched next one) in registers, about 200 per thread, so one block; wider rows use the strips,
+// narrower ones need few, two blocks.
+constexpr int ln_bwd_blocks_per_sm(int nch) { return nch == 2 || nch == 3 ? 1 : 2; }
 
-template <int LN_MAX_CHUNKS>
+template <int LN_MAX_CHUNKS, int LPR>          // LPR: lanes per row, as in the forward
 __global__ void __launch_bounds__(32 * LN_BWD_WARPS, ln_bwd_blocks_per_sm(LN_MAX_CHUNKS))
 layernorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                      const float* __restrict__ gamma, const float* __restrict__ mean_in,
                      const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ dres,
                      __nv_bfloat16* __restrict__ dx, float* __restrict__ partial, int M, int d) {
   extern __shared__ float sh[];                 // [LN_BWD_WARPS][3][d]
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  static_assert(LPR == 32 || LN_MAX_CHUNKS == 1, "rows that share a warp are one chunk long");
+  const int lane = threadIdx.x & (LPR - 1), warp = threadIdx.x >> 5;
   const int nch = (d + 255) / 256;
   float* mine = sh + (long long)warp * 3 * d;
-  for (int i = lane; i < 3 * d; i += 32) mine[i] = 0.f;
+  for (int i = threadIdx.x & 31; i < 3 * d; i += 32) mine[i] = 0.f;
   __syncwarp();
   // Rows stay in the bf16 form they were loaded in and are unpacked in both passes (cheaper in registers
   // than a row of fp32).  Up to 768 columns the column sums live in registers (72 per thread) and reach the
@@ -221,15 +235,21 @@ layernorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
   }
   pdl_wait();
   pdl_launch();
-  const int stride = gridDim.x * LN_BWD_WARPS;
-  int row = blockIdx.x * LN_BWD_WARPS + warp;
+  const int stride = gridDim.x * LN_BWD_WARPS * (32 / LPR);
+  int first = (blockIdx.x * LN_BWD_WARPS + warp) * (32 / LPR);          // the warp's first row
+  int row = first + (threadIdx.x & 31) / LPR;
   LnBwdRow<LN_MAX_CHUNKS> cur, nxt;
-  if (PREFETCH && row < M) ln_bwd_load(cur, dy, x, dres, mean_in, rstd_in, row, d, nch, lane);
-  for (; row < M; row += stride) {
+  if (LPR < 32) {          // a row past the last one adds zeros
+    cur.x[0] = cur.dy[0] = cur.r[0] = make_uint4(0, 0, 0, 0);
+    nxt = cur;
+  }
+  if (PREFETCH && first < M) ln_bwd_load(cur, dy, x, dres, mean_in, rstd_in, row, M, d, nch, lane);
+  for (; first < M; first += stride, row += stride) {
     if (PREFETCH) {
-      if (row + stride < M) ln_bwd_load(nxt, dy, x, dres, mean_in, rstd_in, row + stride, d, nch, lane);
+      if (LPR < 32) nxt.x[0] = nxt.dy[0] = nxt.r[0] = make_uint4(0, 0, 0, 0);
+      if (first + stride < M) ln_bwd_load(nxt, dy, x, dres, mean_in, rstd_in, row + stride, M, d, nch, lane);
     } else {
-      ln_bwd_load(cur, dy, x, dres, mean_in, rstd_in, row, d, nch, lane);
+      ln_bwd_load(cur, dy, x, dres, mean_in, rstd_in, row, M, d, nch, lane);
     }
     const long long off = (long long)row * d;
     const float mean = cur.mean, rstd = cur.rstd;
@@ -270,8 +290,8 @@ layernorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
         }
       }
     }
-    s1 = warp_sum(s1) / d;
-    s2 = warp_sum(s2) / d;
+    s1 = group_sum<LPR>(s1) / d;
+    s2 = group_sum<LPR>(s2) / d;
 #pragma unroll
     for (int c = 0; c < LN_MAX_CHUNKS; ++c) {
       const int col = c * 256 + lane * 8;
@@ -301,10 +321,18 @@ layernorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
 #pragma unroll
         for (int j = 0; j < 8; ++j)
           o[j] = rstd * (dv[j] * g[j] - s1 - (xh[j] - mean) * rstd * s2) + (dres ? r[j] : 0.f);
-        if (DSW_OK(row < M && col + 8 <= d)) store8(dx + off + col, o);
+        if (row < M && DSW_OK(col + 8 <= d)) store8(dx + off + col, o);
       }
     }
     if (PREFETCH) cur = nxt;
+  }
+  if constexpr (LPR < 32) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      acc_g[0][j] += __shfl_xor_sync(0xffffffffu, acc_g[0][j], LPR);
+      acc_b[0][j] += __shfl_xor_sync(0xffffffffu, acc_b[0][j], LPR);
+      acc_r[0][j] += __shfl_xor_sync(0xffffffffu, acc_r[0][j], LPR);
+    }
   }
   if constexpr (REG_ACC) {
 #pragma unroll
@@ -313,6 +341,7 @@ layernorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
       if (c < nch && col < d) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
+          if (LPR < 32 && (threadIdx.x & LPR)) continue;          // folded into the lower lanes above
           mine[col + j] = acc_g[c][j];
           mine[d + col + j] = acc_b[c][j];
           mine[2 * d + col + j] = acc_r[c][j];
@@ -748,16 +777,21 @@ extern "C" int dsw_layernorm_fwd_lo(const void* x, const void* x_lo, const float
                                  float* rstd, int M, int d, float eps, cudaStream_t st) {
   if (d % 8 || d > 256 * LN_MAX_CHUNKS_ALL) return -10;
   // two blocks per SM, several rows per warp when there are enough rows: gamma and beta are paid once per warp
-  const int grid = grid_for(M, 16, 148 * 2);
+  const bool two_rows = d <= 128;
+  const int grid = two_rows ? grid_for(M, 32, 148 * 4) : grid_for(M, 16, 148 * 2);
   cudaError_t rc;
-#define LN_FWD(NCH)                                                                                                  \
-  rc = x_lo ? launch(layernorm_fwd_kernel<NCH, true>, grid, 256, 0, st, 1, (const bf16*)x, (const bf16*)x_lo, gamma, beta, \
+#define LN_FWD(NCH, LPR)                                                                                             \
+  rc = x_lo ? launch(layernorm_fwd_kernel<NCH, true, LPR>, grid, 256, 0, st, 1, (const bf16*)x, (const bf16*)x_lo, gamma, beta, \
                      (bf16*)y, mean, rstd, M, d, eps)                                                                \
-            : launch(layernorm_fwd_kernel<NCH, false>, grid, 256, 0, st, 1, (const bf16*)x, (const bf16*)x_lo, gamma, beta, \
+            : launch(layernorm_fwd_kernel<NCH, false, LPR>, grid, 256, 0, st, 1, (const bf16*)x, (const bf16*)x_lo, gamma, beta, \
                      (bf16*)y, mean, rstd, M, d, eps)
   switch ((d + 255) / 256) {
-    case 1: LN_FWD(1); break; case 2: LN_FWD(2); break; case 3: LN_FWD(3); break; case 4: LN_FWD(4); break;
-    case 5: LN_FWD(5); break; case 6: LN_FWD(6); break; case 7: LN_FWD(7); break; default: LN_FWD(8); break;
+    case 1:
+      if (two_rows) LN_FWD(1, 16);
+      else          LN_FWD(1, 32);
+      break;
+    case 2: LN_FWD(2, 32); break; case 3: LN_FWD(3, 32); break; case 4: LN_FWD(4, 32); break; case 5: LN_FWD(5, 32); break;
+    case 6: LN_FWD(6, 32); break; case 7: LN_FWD(7, 32); break; default: LN_FWD(8, 32); break;
   }
 #undef LN_FWD
   return rc == cudaSuccess ? 0 : -3;
@@ -776,27 +810,33 @@ extern "C" int dsw_layernorm_bwd(const void* dy, const void* x, const float* gam
                                  float* dres_sum, float* scratch, int M, int d, cudaStream_t st) {
   if (d % 8 || d > 256 * LN_MAX_CHUNKS_ALL) return -10;
   int grid = dsw_layernorm_bwd_blocks(M);
-  if ((d + 255) / 256 <= 3 && grid > 148) grid = 148;          // the register-resident variant runs one block per SM
+  const bool two_rows = d <= 128;
+  // the register-resident variant runs one block per SM, except for rows of one chunk
+  if (d > 256 && d <= 768 && grid > 148) grid = 148;
   const int want = dres_sum != nullptr && dres != nullptr;
   const size_t shmem = sizeof(float) * LN_BWD_WARPS * 3 * d;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -2;
   cudaError_t rc;
-#define LN_BWD(NCH)                                                                                              \
+#define LN_BWD(NCH, LPR)                                                                                          \
   do {                                                                                                           \
     static bool attr[64] = {false};          /* the attribute is per device */                                 \
     if (!attr[dev]) {                                                                                            \
-      if (cudaFuncSetAttribute(layernorm_bwd_kernel<NCH>, cudaFuncAttributeMaxDynamicSharedMemorySize,           \
+      if (cudaFuncSetAttribute(layernorm_bwd_kernel<NCH, LPR>, cudaFuncAttributeMaxDynamicSharedMemorySize,           \
                                8 * 3 * 256 * NCH * 4) != cudaSuccess)                                            \
         return -2;                                                                                               \
       attr[dev] = true;                                                                                          \
     }                                                                                                            \
-    rc = launch(layernorm_bwd_kernel<NCH>, grid, 32 * LN_BWD_WARPS, shmem, st, 1, (const bf16*)dy, (const bf16*)x, gamma, \
+    rc = launch(layernorm_bwd_kernel<NCH, LPR>, grid, 32 * LN_BWD_WARPS, shmem, st, 1, (const bf16*)dy, (const bf16*)x, gamma, \
                 mean, rstd, (const bf16*)dres, (bf16*)dx, scratch, M, d);                                        \
   } while (0)
   switch ((d + 255) / 256) {
-    case 1: LN_BWD(1); break; case 2: LN_BWD(2); break; case 3: LN_BWD(3); break; case 4: LN_BWD(4); break;
-    case 5: LN_BWD(5); break; case 6: LN_BWD(6); break; case 7: LN_BWD(7); break; default: LN_BWD(8); break;
+    case 1:
+      if (two_rows) LN_BWD(1, 16);
+      else          LN_BWD(1, 32);
+      break;
+    case 2: LN_BWD(2, 32); break; case 3: LN_BWD(3, 32); break; case 4: LN_BWD(4, 32); break; case 5: LN_BWD(5, 32); break;
+    case 6: LN_BWD(6, 32); break; case 7: LN_BWD(7, 32); break; default: LN_BWD(8, 32); break;
   }
 #undef LN_BWD
   if (rc != cudaSuccess) return -3;
@@ -921,10 +961,10 @@ extern "C" int dsw_load_elementwise() {
   cudaFuncAttributes a;
   int bad = 0;
 #define L(f) bad |= cudaFuncGetAttributes(&a, f) != cudaSuccess
-  L((layernorm_fwd_kernel<1, false>)); L((layernorm_fwd_kernel<1, true>)); L((layernorm_fwd_kernel<2, false>)); L((layernorm_fwd_kernel<2, true>)); L((layernorm_fwd_kernel<3, false>)); L((layernorm_fwd_kernel<3, true>)); L((layernorm_fwd_kernel<4, false>)); L((layernorm_fwd_kernel<4, true>));
-  L((layernorm_fwd_kernel<5, false>)); L((layernorm_fwd_kernel<5, true>)); L((layernorm_fwd_kernel<6, false>)); L((layernorm_fwd_kernel<6, true>)); L((layernorm_fwd_kernel<7, false>)); L((layernorm_fwd_kernel<7, true>)); L((layernorm_fwd_kernel<8, false>)); L((layernorm_fwd_kernel<8, true>));
-  L(layernorm_bwd_kernel<1>); L(layernorm_bwd_kernel<2>); L(layernorm_bwd_kernel<3>); L(layernorm_bwd_kernel<4>);
-  L(layernorm_bwd_kernel<5>); L(layernorm_bwd_kernel<6>); L(layernorm_bwd_kernel<7>); L(layernorm_bwd_kernel<8>);
+  L((layernorm_fwd_kernel<1, false, 16>)); L((layernorm_fwd_kernel<1, true, 16>)); L((layernorm_fwd_kernel<1, false, 32>)); L((layernorm_fwd_kernel<1, true, 32>)); L((layernorm_fwd_kernel<2, false, 32>)); L((layernorm_fwd_kernel<2, true, 32>)); L((layernorm_fwd_kernel<3, false, 32>)); L((layernorm_fwd_kernel<3, true, 32>)); L((layernorm_fwd_kernel<4, false, 32>)); L((layernorm_fwd_kernel<4, true, 32>));
+  L((layernorm_fwd_kernel<5, false, 32>)); L((layernorm_fwd_kernel<5, true, 32>)); L((layernorm_fwd_kernel<6, false, 32>)); L((layernorm_fwd_kernel<6, true, 32>)); L((layernorm_fwd_kernel<7, false, 32>)); L((layernorm_fwd_kernel<7, true, 32>)); L((layernorm_fwd_kernel<8, false, 32>)); L((layernorm_fwd_kernel<8, true, 32>));
+  L((layernorm_bwd_kernel<1, 16>)); L((layernorm_bwd_kernel<1, 32>)); L((layernorm_bwd_kernel<2, 32>)); L((layernorm_bwd_kernel<3, 32>)); L((layernorm_bwd_kernel<4, 32>));
+  L((layernorm_bwd_kernel<5, 32>)); L((layernorm_bwd_kernel<6, 32>)); L((layernorm_bwd_kernel<7, 32>)); L((layernorm_bwd_kernel<8, 32>));
   L(layernorm_bwd_finish_kernel); L(colsum_kernel); L(embedding_fwd_kernel); L(embedding_bwd_kernel);
   L(embedding_bwd_sorted_kernel); L(embedding_bwd_pos_kernel);
   L(mask_count_kernel); L(loss_begin_kernel); L(cross_entropy_kernel); L(head_rows_kernel); L(sum_partials_kernel); L(cast_f32_bf16_kernel); L(cast_bf16_f32_kernel);
