@@ -171,8 +171,9 @@ struct Scratch {
 // 49 / 51, 2048 145 / 120, 32768 2018 / 1750; width 384: 512 rows 68 / 78, 2048 219 / 182, 32768 2820 / 2083; width 768:
 // 2048 rows 267 / 287, 32768 3512 / 3823).
 constexpr int HEAD_TWICE_WIDTH = 384, HEAD_TWICE_ROWS = 1024;
-bool unstored_logits(const Stage& s, bool grad, size_t rows) {
-  return s.V > 128 && (!grad || (s.d <= HEAD_TWICE_WIDTH && rows >= size_t(HEAD_TWICE_ROWS)));
+// The rows are those of the microbatch, so that slicing the head does not change its arithmetic.
+bool unstored_logits(const Stage& s, bool grad, size_t M) {
+  return s.V > 128 && (!grad || (s.d <= HEAD_TWICE_WIDTH && M >= size_t(HEAD_TWICE_ROWS)));
 }
 
 // logit_rows: rows of the logits that exist at a time (0: the caller keeps them elsewhere)
@@ -180,7 +181,7 @@ Scratch take_scratch(Area& a, const Stage& s, size_t M, bool grad, size_t logit_
   const size_t d = s.d;
   Scratch v = {};
   if (s.head_w && logit_rows) {
-    const bool unstored = unstored_logits(s, grad, logit_rows);
+    const bool unstored = unstored_logits(s, grad, M);
     if (grad || !unstored) v.logits = a.take<bf16>(logit_rows * s.V);
     if (unstored) {
       v.parts = a.take<float>((size_t(s.V) + 63) / 64 * logit_rows);
@@ -533,7 +534,7 @@ extern "C" int dsw_stage_head(void* stage, void* saved, void* scratch, const lon
   if (s.head_used) MAIN_WAIT(s.head_done);
   LAUNCH(dsw_loss_begin(mask, M, s.count, loss, st));
   const int flags = (keep ? 1 : 0) | (deterministic ? 2 : 0) | chunks << 2;
-  const bool unstored = unstored_logits(s, grad != 0, rows);
+  const bool unstored = unstored_logits(s, grad != 0, size_t(M));
   const auto dlogits = [&](const bf16* ln, int m) {
     return dsw_head_dlogits(ln, s.head_w, c.rows, c.logits, m, V, d, s.status, r.st);
   };
