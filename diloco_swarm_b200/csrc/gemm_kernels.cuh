@@ -307,27 +307,28 @@ __device__ __forceinline__ void epilogue_warp(const GemmArgs& g, uint32_t t_addr
         if constexpr (EXTRA) {
           uint32_t du[4] = {d.x, d.y, d.z, d.w};
           const uint32_t xu[4] = {x[i].x, x[i].y, x[i].z, x[i].w};
-          uint32_t lo[4] = {0, 0, 0, 0};
-          if constexpr (MODE == EPI_RESID) {
+          // Both operands are bf16 by now, so one packed bf16 instruction does what unpacking, an fp32 product or sum and
+          // packing did in seven, with the same single rounding (a product of two bf16 values is exact in fp32).
+          if constexpr (MODE == EPI_MUL) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) du[q] = mul_bf16x2(du[q], xu[q]);
+          } else if (g.aux_in == nullptr && g.aux_out == nullptr) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) du[q] = add_bf16x2(du[q], xu[q]);
+          } else {          // with the residual stream's low halves
+            uint32_t lo[4] = {0, 0, 0, 0};
             if (g.aux_in != nullptr) {
               const uint4 t = *reinterpret_cast<const uint4*>(g.aux_in + (long long)row * g.ldaux + col);
               lo[0] = t.x; lo[1] = t.y; lo[2] = t.z; lo[3] = t.w;
             }
-          }
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const float2 a = unpack_bf16(du[q]), e = unpack_bf16(xu[q]);
-            if constexpr (MODE == EPI_RESID) {
-              const float2 t = unpack_bf16(lo[q]);
+            for (int q = 0; q < 4; ++q) {
+              const float2 a = unpack_bf16(du[q]), e = unpack_bf16(xu[q]), t = unpack_bf16(lo[q]);
               const float s0 = a.x + (e.x + t.x), s1 = a.y + (e.y + t.y);
               du[q] = pack_bf16(s0, s1);
               const float2 h = unpack_bf16(du[q]);
               lo[q] = pack_bf16(s0 - h.x, s1 - h.y);
-            } else {
-              du[q] = pack_bf16(a.x * e.x, a.y * e.y);
             }
-          }
-          if constexpr (MODE == EPI_RESID) {
             if (g.aux_out != nullptr)
               *reinterpret_cast<uint4*>(g.aux_out + (long long)row * g.ldaux + col) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
           }

@@ -158,7 +158,7 @@ static bool allowed(const TileKind& t, int M) { return t.ctas == 1 || (use_pair(
 // The one whose waves take least.  A tile's epilogue hides behind the next tile's main loop when that is the longer.
 static int pick_bn(int M, int N, int K, int splits, int mode, int sms, double* cost) {
   const int kb = ((K + BK - 1) / BK + splits - 1) / splits;
-  const double heavy = mode == EPI_GELU || mode == EPI_MUL ? 2.0 : 1.0;
+  const double heavy = mode == EPI_GELU ? 2.0 : 1.0;
   int best = 128;
   double least = 1e30;
   for (const TileKind& t : TILE_KINDS) {
