@@ -17,10 +17,13 @@
 // two up, which is long done.  A block's outgoing gradient is read by the side work of the block below it, so those
 // buffers form a ring of three.
 //
-// Graphs.  A launch still costs the host 3.3 us, more than many kernels of a short pass take.  So a run of launches whose
-// pointers come back (the work areas do; what the caller brings or takes away stays outside: token ids, targets, mask,
-// loss, logits of forward_infer) is captured into a CUDA graph when it is asked for a second time and replayed from then
-// on, side work and dependent launches included.  A handful of graphs per stage is kept, the one used longest ago goes.
+// Graphs.  A launch still costs the host 3.3 us, more than many kernels of a short pass take.  So a run of launches that
+// touches the work areas only is captured into a CUDA graph when it is asked for a second time in the same areas and
+// replayed from then on, side work and dependent launches included.  What the caller brings or takes away stays outside:
+// token ids, targets, mask, loss, logits of forward_infer; hidden states and their gradients are copied into or out of the
+// areas (some 4 us each at GRAPH_COPY elements; larger ones are not copied and their passes not replayed), so
+// it makes no difference whether they come in the same buffers again.  A handful of graphs per stage is kept, the one
+// used longest ago goes.
 // Only for passes of up to GRAPH_TOKENS tokens: longer ones keep the device busy for longer than the host needs anyway,
 // and there a replay, which ends with the side stream's work, would cost the overlap with the next pass.
 #include <cuda_bf16.h>
@@ -50,14 +53,12 @@ struct Block {
   float *dw[4], *db[4];
 };
 
-// What a captured run of launches depends on: every pointer and number that its kernels were given.
+// What a captured run of launches depends on: the work areas and every number that its kernels were given.
 struct GraphKey {
   int what, B, T, flags;
-  const void* p[6];
+  const void *saved, *scratch;
   bool operator==(const GraphKey& o) const {
-    for (int i = 0; i < 6; ++i)
-      if (p[i] != o.p[i]) return false;
-    return what == o.what && B == o.B && T == o.T && flags == o.flags;
+    return what == o.what && B == o.B && T == o.T && flags == o.flags && saved == o.saved && scratch == o.scratch;
   }
 };
 struct GraphSlot {
@@ -69,6 +70,7 @@ struct GraphSlot {
   unsigned long long used;
 };
 constexpr int GRAPH_TOKENS = 8192, GRAPH_SLOTS = 32;
+constexpr long long GRAPH_COPY = 6 << 20;
 
 struct Stage {
   int n, d, nh, V;
@@ -132,9 +134,12 @@ Saved take_block(Area& a, const Stage& s, size_t M, bool keep) {
   return v;
 }
 
+// whether a pass copies what the caller brings and takes away, so that it can be replayed
+bool copied(size_t M, int d) { return M <= size_t(GRAPH_TOKENS) && M * d <= size_t(GRAPH_COPY); }
+
 // saved area of a microbatch: input embedding (first stage), blocks, final LayerNorm
 struct SavedAll {
-  bf16* x0;
+  bf16* x0;                      // first stage: the embedding; others: the caller's hidden state, where passes are replayed
   std::vector<Saved> blk;
   bf16* lnf;
   float *muf, *rsf;
@@ -142,7 +147,7 @@ struct SavedAll {
 
 SavedAll take_saved(Area& a, const Stage& s, size_t M, bool keep) {
   SavedAll v;
-  v.x0 = s.wte ? a.take<bf16>(M * s.d) : nullptr;
+  v.x0 = s.wte || copied(M, s.d) ? a.take<bf16>(M * s.d) : nullptr;
   v.blk.resize(s.n);
   if (keep) {
     for (int l = 0; l < s.n; ++l) v.blk[l] = take_block(a, s, M, true);
@@ -307,10 +312,17 @@ struct Run {
     return 0;
   }
 
-  // Queues `body` on the stage's stream, as a graph once the same run has been asked for before.
+  int copy(void* to, const void* from) const {          // a hidden state
+    TRY_CUDA(cudaMemcpyAsync(to, from, size_t(M) * s.d * sizeof(bf16), cudaMemcpyDeviceToDevice, st));
+    dsw::tl_launch.pdl = false;
+    return 0;
+  }
+
+  // Queues `body` on the stage's stream, as a graph once the same run has been asked for before (if it only touches the
+  // work areas).
   template <class F>
-  int replayed(const GraphKey& key, F&& body) {
-    if (M > GRAPH_TOKENS || !graphs_on()) return body();
+  int replayed(const GraphKey& key, bool own_memory, F&& body) {
+    if (!own_memory || M > GRAPH_TOKENS || !graphs_on()) return body();
     GraphSlot* slot = nullptr;
     for (GraphSlot& g : s.graphs)
       if (g.key == key) { slot = &g; break; }
@@ -480,7 +492,7 @@ extern "C" int dsw_stage_sizes(void* stage, int B, int T, int keep, int grad, in
 extern "C" int dsw_stage_forward(void* stage, const long long* ids, const void* x, void* saved, void* y,
                                  float* infer_logits, int B, int T, int keep, cudaStream_t st) {
   Stage& s = *static_cast<Stage*>(stage);
-  if (B <= 0 || T <= 0 || (s.wte ? ids == nullptr : x == nullptr)) return -10;
+  if (B <= 0 || T <= 0 || s.n < 1 || (s.wte ? ids == nullptr : x == nullptr)) return -10;
   std::lock_guard<std::mutex> lock(s.mu);
   const Dependent mode;
   Run r{s, B, T, B * T, 0, st};
@@ -491,14 +503,20 @@ extern "C" int dsw_stage_forward(void* stage, const long long* ids, const void* 
     LAUNCH(dsw_embedding_fwd(ids, s.wte, s.wpe, v.x0, B, T, s.d, s.V, s.status, st));
     in = v.x0;
   }
+  const bool copies = copied(size_t(r.M), s.d);
+  if (!s.wte && copies) {
+    TRY(r.copy(v.x0, x));
+    in = v.x0;
+  }
+  bf16* last = y && !copies ? static_cast<bf16*>(y) : v.blk[s.n - 1].out;
   // Sampling: the residual stream, whose rounding at every addition is most of what bf16 costs the logits, keeps its low
   // half in a second bf16 array (GPT-2 small, 5 x 24 tokens: error of the logits 9.2e-3 without, see the test)
   const bool precise = infer_logits != nullptr && !keep;
-  const GraphKey key{0, B, T, (keep ? 1 : 0) | (precise ? 2 : 0), {saved, x, y, nullptr, nullptr, nullptr}};
-  TRY(r.replayed(key, [&]() -> int {
+  const GraphKey key{0, B, T, (keep ? 1 : 0) | (precise ? 2 : 0), saved, nullptr};
+  TRY(r.replayed(key, copies || (s.wte && !y), [&]() -> int {
     const bf16 *cur = in, *cur_lo = nullptr;
     for (int l = 0; l < s.n; ++l) {
-      bf16* out = l + 1 == s.n && y ? static_cast<bf16*>(y) : v.blk[l].out;
+      bf16* out = l + 1 == s.n ? last : v.blk[l].out;
       TRY(r.block_fwd(s.blocks[l], cur, cur_lo, precise, v.blk[l], out));
       cur = out;
       cur_lo = precise ? v.blk[l].out_lo : nullptr;
@@ -507,6 +525,7 @@ extern "C" int dsw_stage_forward(void* stage, const long long* ids, const void* 
       LAUNCH(dsw_layernorm_fwd_lo(cur, cur_lo, s.lnf_w, s.lnf_b, v.lnf, v.muf, v.rsf, r.M, s.d, 1e-5f, r.st));
     return 0;
   }));
+  if (y && copies) TRY(r.copy(y, last));
   if (infer_logits)
     LAUNCH(dsw_gemm_bf16(v.lnf, s.d, 0, s.head_w, s.d, 0, r.M, s.V, s.d, DSW_EPI_STORE_F32, 1, infer_logits, s.V, nullptr,
                          nullptr, 0, nullptr, nullptr, 0, 0, 0, s.status, st));
@@ -538,7 +557,7 @@ extern "C" int dsw_stage_head(void* stage, void* saved, void* scratch, const lon
   const auto dlogits = [&](const bf16* ln, int m) {
     return dsw_head_dlogits(ln, s.head_w, c.rows, c.logits, m, V, d, s.status, r.st);
   };
-  TRY(r.replayed(GraphKey{1, B, T, flags, {saved, scratch, nullptr, nullptr, nullptr, nullptr}}, [&]() -> int {
+  TRY(r.replayed(GraphKey{1, B, T, flags, saved, scratch}, true, [&]() -> int {
     LAUNCH(dsw_layernorm_fwd(x, s.lnf_w, s.lnf_b, v.lnf, v.muf, v.rsf, M, d, 1e-5f, r.st));
     if (rows == M && !unstored) LAUNCH(r.gemm(v.lnf, s.head_w, true, V, d, c.logits, DSW_EPI_STORE, nullptr, nullptr, nullptr, nullptr, M));
     return 0;
@@ -561,7 +580,7 @@ extern "C" int dsw_stage_head(void* stage, void* saved, void* scratch, const lon
     TRY(r.head_grads(c, ln, r0, m));
   }
   if (!grad) return 0;
-  TRY(r.replayed(GraphKey{2, B, T, flags, {saved, scratch, nullptr, nullptr, nullptr, nullptr}}, [&]() -> int {
+  TRY(r.replayed(GraphKey{2, B, T, flags, saved, scratch}, true, [&]() -> int {
     if (rows == M) {
       if (unstored) LAUNCH(dlogits(v.lnf, M));
       TRY(r.head_grads(c, v.lnf, 0, M));
@@ -588,12 +607,15 @@ extern "C" int dsw_stage_backward(void* stage, int hi, int lo, const void* dy, c
   const SavedAll v = take_saved(a, s, size_t(r.M), true);
   const Scratch c = take_scratch(ca, s, size_t(r.M), true, chunks > 0 ? head_rows(size_t(r.M), chunks) : 0);
   if (hi == s.n && dy) TRY(r.join());
-  const bf16* g = dy ? static_cast<const bf16*>(dy) : c.dx[hi % 3];
+  const bool copies = copied(size_t(r.M), s.d);
+  if (dy && copies) TRY(r.copy(c.dx[hi % 3], dy));
+  const bf16* g = dy && !copies ? static_cast<const bf16*>(dy) : c.dx[hi % 3];
+  bf16* first = dx0 && !copies ? static_cast<bf16*>(dx0) : c.dx[0];
   const auto blocks = [&]() -> int {
     const bf16* dx = g;
     for (int l = hi - 1; l >= lo; --l) {
-      const bf16* in = l > 0 ? v.blk[l - 1].out : (s.wte ? v.x0 : static_cast<const bf16*>(x));
-      bf16* out = l == 0 && dx0 ? static_cast<bf16*>(dx0) : c.dx[l % 3];
+      const bf16* in = l > 0 ? v.blk[l - 1].out : (v.x0 ? v.x0 : static_cast<const bf16*>(x));
+      bf16* out = l == 0 ? first : c.dx[l % 3];
       TRY(r.block_bwd(l, s.blocks[l], in, v.blk[l], c, dx, out));
       dx = out;
     }
@@ -601,11 +623,13 @@ extern "C" int dsw_stage_backward(void* stage, int hi, int lo, const void* dy, c
   };
   // in one piece it can be replayed; block by block (gradient buckets sent in between) it is queued as it is
   if (hi == s.n && lo == 0) {
-    TRY(r.replayed(GraphKey{3, B, T, (deterministic ? 2 : 0) | chunks << 2, {saved, scratch, dy, x, dx0, nullptr}}, blocks));
+    const bool own_memory = copies || (s.wte && !dx0 && !dy);
+    TRY(r.replayed(GraphKey{3, B, T, (deterministic ? 2 : 0) | chunks << 2, saved, scratch}, own_memory, blocks));
   } else {
     TRY(blocks());
   }
-  if (hi > lo) g = lo == 0 && dx0 ? static_cast<bf16*>(dx0) : c.dx[lo % 3];
+  if (hi > lo) g = lo == 0 ? first : c.dx[lo % 3];
+  if (hi > lo && lo == 0 && dx0 && copies) TRY(r.copy(dx0, first));
   if (lo == 0 && ids) LAUNCH(dsw_embedding_bwd(ids, g, s.dwte, s.dwpe, B, T, s.d, s.V, st));
   return 0;
 }
