@@ -1,6 +1,6 @@
 // Device side of the tcgen05 GEMMs: epilogue, the one-CTA kernel and the CTA-pair kernel, as templates.
 // Each kernel is a template on its epilogue class; gemm_one_cta.cu and gemm_pair.cu instantiate them
-// (two translation units, so the fifteen kernels compile side by side) and gemm_tcgen05.cu holds the
+// (two translation units, so the kernels compile side by side) and gemm_tcgen05.cu holds the
 // host entry point.
 #pragma once
 #include <cuda.h>
