@@ -393,11 +393,14 @@ class B200Engine:
 
     # ------------------------------------------------------------------ the same passes through the native executor
     def _input(self, input_ids, hidden):
-        """(ids, hidden state, B, T) as the kernels read them."""
+        """(ids, hidden state, B, T) as the kernels read them.  The executor takes addresses, so what does not have the
+        stage's type or size is refused here: it would be read past its end."""
         if self.is_first:
             B, T = input_ids.shape
+            assert input_ids.dtype == torch.long, f"token ids are int64, not {input_ids.dtype}"
             return input_ids.contiguous(), None, B, T
         B, T = hidden.shape[0], hidden.shape[1]
+        assert hidden.numel() == B * T * self.exec.d, f"hidden state {tuple(hidden.shape)} of a stage {self.exec.d} wide"
         x = hidden if hidden.dtype == BF16 else hidden.to(BF16)
         return None, x.contiguous(), B, T
 
@@ -460,6 +463,7 @@ class B200Engine:
         if dx.dtype != BF16:
             dx = dx.to(BF16)
         if "area" in s:
+            assert dx.numel() == B * T * self.exec.d, f"gradient {tuple(grad_out.shape)} of an output of {B} x {T} x {self.exec.d}"
             dx = dx.contiguous()
             if self.side is not None:
                 dx.record_stream(self.side)           # the last block's weight gradient reads it there
