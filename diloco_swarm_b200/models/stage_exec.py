@@ -21,11 +21,17 @@ MAX_STREAMS = 4                  # scratch areas kept (one per calling stream)
 
 
 class SavedArea:
-    """``saved`` area of one microbatch, with the point on the streams after which it may be written again."""
-    __slots__ = ("buf", "free", "stream")
+    """``saved`` area of one microbatch, with the point on the streams after which it may be written again.
+    ``home``: the stream that it was allocated on."""
+    __slots__ = ("buf", "free", "stream", "home")
 
-    def __init__(self, buf: torch.Tensor):
-        self.buf, self.free, self.stream = buf, None, None
+    def __init__(self, buf: torch.Tensor, home: torch.cuda.Stream):
+        self.buf, self.free, self.stream, self.home = buf, None, None, home
+
+    def used_on(self, stream: torch.cuda.Stream) -> None:
+        """Once dropped, the memory goes back to ``home``'s pool: the allocator has to know of everybody else."""
+        if stream != self.home:
+            self.buf.record_stream(stream)
 
 
 class StageExec:
@@ -87,9 +93,10 @@ class StageExec:
                 stream.wait_event(a.free)
                 if a.stream != stream:
                     stream.wait_stream(a.stream)
+                a.used_on(stream)
                 return a
         self._idle.clear()                        # another microbatch size: the old areas go back to the allocator
-        return SavedArea(self._alloc(nbytes))
+        return SavedArea(self._alloc(nbytes), stream)
 
     def give(self, area: SavedArea, stream: torch.cuda.Stream) -> None:
         """The backward that read ``area`` has been queued on ``stream`` (and the side stream)."""
@@ -97,6 +104,7 @@ class StageExec:
             area.free = torch.cuda.Event()
         area.free.record(self.side if self.side is not None else stream)
         area.stream = stream
+        area.used_on(stream)
         most = 2 if area.buf.numel() <= KEEP_AREA_BYTES else 1
         if len(self._idle) < most:
             self._idle.append(area)

@@ -1,0 +1,61 @@
+"""Work areas of the stage executor and the streams that use them, with stand-ins for buffers, events and streams."""
+import pytest
+import torch
+
+from diloco_swarm_b200.models.stage_exec import SavedArea, StageExec
+
+
+class Stream:
+    def __init__(self):
+        self.waited = []
+
+    def wait_event(self, event):
+        self.waited.append(event)
+
+    def wait_stream(self, other):
+        self.waited.append(other)
+
+
+class Event:
+    def record(self, stream):
+        self.on = stream
+
+
+class Buffer:
+    def __init__(self, nbytes):
+        self.nbytes, self.recorded = nbytes, []
+
+    def numel(self):
+        return self.nbytes
+
+    def record_stream(self, stream):
+        self.recorded.append(stream)
+
+
+@pytest.fixture
+def executor(monkeypatch):
+    monkeypatch.setattr(torch.cuda, "Event", Event)
+    ex = StageExec.__new__(StageExec)
+    ex.side, ex._idle, ex._alloc = Stream(), [], Buffer
+    return ex
+
+
+def test_an_area_is_recorded_on_every_stream_but_its_own(executor):
+    """Taken by a pass on another stream than the one it was allocated on, an area is dropped when a pass of another
+    size comes: the allocator must not hand it out again on the first stream before the second is done with it."""
+    a, b = Stream(), Stream()
+    area = executor.take(100, a)
+    executor.give(area, a)
+    assert executor.take(100, a) is area and area.buf.recorded == []
+    executor.give(area, a)
+    assert executor.take(100, b) is area and a in b.waited and b in area.buf.recorded
+    executor.give(area, b)
+    other = executor.take(200, a)                      # another size: the area is dropped, b still runs
+    assert other is not area and executor._idle == [] and set(area.buf.recorded) == {b}
+
+
+def test_a_backward_on_another_stream_is_recorded(executor):
+    a, b = Stream(), Stream()
+    area = executor.take(100, a)
+    executor.give(area, b)
+    assert area.buf.recorded == [b] and isinstance(area, SavedArea)
