@@ -170,7 +170,9 @@ int dsw_grad_allreduce_nvls(void* const* bufs, void* mc, void* const* flags, flo
 // ---------------------------------------------------------------- stage executor (stage.cu)
 // A pipeline stage's forward and backward as sequences of the launches above, one call each.  desc: int64 array of
 // sizes and device pointers (layout at dsw_stage_create); saved / scratch: work areas of the sizes that
-// dsw_stage_sizes gives for the same B, T, keep, grad and chunks.  Several threads may call; a pass is queued whole.
+// dsw_stage_sizes gives for the same B, T, keep, grad and chunks.  Several threads may call, each call is queued whole.
+// The calls of a pass (forward, head, backward) share its work areas: a caller whose threads use the same areas keeps
+// others out from the first to the last of them.
 int dsw_stage_create(const long long* desc, int len, void** out);
 int dsw_stage_destroy(void* stage);
 int dsw_stage_launches();

@@ -442,15 +442,16 @@ class B200Engine:
     # ------------------------------------------------------------------ engine API
     def forward(self, key: int, input_ids, hidden, keep: bool = True) -> torch.Tensor:
         if self._native():
-            ex, st = self.exec, torch.cuda.current_stream()
-            ids, x, B, T = self._input(input_ids, hidden)
-            nbytes = ex.sizes(B, T, keep, False, 0)[0]
-            area = ex.take(nbytes, st) if keep else None
-            y = torch.empty(B, T, ex.d, dtype=BF16, device=self.device)
-            ex.forward(ids, x, area.buf if keep else ex.area("saved", nbytes, st), y, None, B, T, keep, st)
-            if keep:
-                self.stash[key] = {"area": area, "ids": ids, "x": x, "B": B, "T": T}
-            return y
+            with self.exec.lock:
+                ex, st = self.exec, torch.cuda.current_stream()
+                ids, x, B, T = self._input(input_ids, hidden)
+                nbytes = ex.sizes(B, T, keep, False, 0)[0]
+                area = ex.take(nbytes, st) if keep else None
+                y = torch.empty(B, T, ex.d, dtype=BF16, device=self.device)
+                ex.forward(ids, x, area.buf if keep else ex.area("saved", nbytes, st), y, None, B, T, keep, st)
+                if keep:
+                    self.stash[key] = {"area": area, "ids": ids, "x": x, "B": B, "T": T}
+                return y
         x, saved, B, T = self._body_fwd(input_ids, hidden, keep)
         if keep:
             self.stash[key] = {"saved": saved, "ids": input_ids, "B": B, "T": T}
@@ -467,8 +468,9 @@ class B200Engine:
             dx = dx.contiguous()
             if self.side is not None:
                 dx.record_stream(self.side)           # the last block's weight gradient reads it there
-            return self._exec_backward(s["area"], dx, s["ids"], s["x"], B, T, self._want_overlap(sync), 0,
-                                       torch.cuda.current_stream())
+            with self.exec.lock:
+                return self._exec_backward(s["area"], dx, s["ids"], s["x"], B, T, self._want_overlap(sync), 0,
+                                           torch.cuda.current_stream())
         return self._body_bwd(s["saved"], dx.contiguous(), s["ids"], B, T, sync=self._want_overlap(sync))
 
     def _want_overlap(self, sync: bool) -> bool:
@@ -512,14 +514,15 @@ class B200Engine:
 
     def forward_backward(self, key: int, input_ids, hidden, targets, mask, scale: float, sync: bool = False):
         if self._native():
-            ex, st, chunks = self.exec, torch.cuda.current_stream(), self.head_chunks
-            ids, x, B, T = self._input(input_ids, hidden)
-            saved_bytes, scratch_bytes = ex.sizes(B, T, True, True, chunks)
-            area = ex.take(saved_bytes, st)
-            loss = torch.empty((), dtype=F32, device=self.device)
-            ex.forward(ids, x, area.buf, None, None, B, T, True, st)
-            self._exec_head(area.buf, ex.area("scratch", scratch_bytes, st), targets, mask, scale, loss, B, T, True, st)
-            return loss, self._exec_backward(area, None, ids, x, B, T, self._want_overlap(sync), chunks, st)
+            with self.exec.lock:
+                ex, st, chunks = self.exec, torch.cuda.current_stream(), self.head_chunks
+                ids, x, B, T = self._input(input_ids, hidden)
+                saved_bytes, scratch_bytes = ex.sizes(B, T, True, True, chunks)
+                area = ex.take(saved_bytes, st)
+                loss = torch.empty((), dtype=F32, device=self.device)
+                ex.forward(ids, x, area.buf, None, None, B, T, True, st)
+                self._exec_head(area.buf, ex.area("scratch", scratch_bytes, st), targets, mask, scale, loss, B, T, True, st)
+                return loss, self._exec_backward(area, None, ids, x, B, T, self._want_overlap(sync), chunks, st)
         x, saved, B, T = self._body_fwd(input_ids, hidden, True)
         if self.head_chunks > 1:
             loss, lnf, mu, rs, dlnf = self._head_chunked(x, targets, mask, scale, grad=True)
@@ -537,14 +540,15 @@ class B200Engine:
     @torch.no_grad()
     def forward_loss(self, input_ids, hidden, targets, mask, scale: float) -> torch.Tensor:
         if self._native():
-            ex, st = self.exec, torch.cuda.current_stream()
-            ids, x, B, T = self._input(input_ids, hidden)
-            saved_bytes, scratch_bytes = ex.sizes(B, T, False, False, self.head_chunks)
-            saved = ex.area("saved", saved_bytes, st)
-            loss = torch.empty((), dtype=F32, device=self.device)
-            ex.forward(ids, x, saved, None, None, B, T, False, st)
-            self._exec_head(saved, ex.area("scratch", scratch_bytes, st), targets, mask, scale, loss, B, T, False, st)
-            return loss
+            with self.exec.lock:
+                ex, st = self.exec, torch.cuda.current_stream()
+                ids, x, B, T = self._input(input_ids, hidden)
+                saved_bytes, scratch_bytes = ex.sizes(B, T, False, False, self.head_chunks)
+                saved = ex.area("saved", saved_bytes, st)
+                loss = torch.empty((), dtype=F32, device=self.device)
+                ex.forward(ids, x, saved, None, None, B, T, False, st)
+                self._exec_head(saved, ex.area("scratch", scratch_bytes, st), targets, mask, scale, loss, B, T, False, st)
+                return loss
         x, _, _, _ = self._body_fwd(input_ids, hidden, False)
         if self.head_chunks > 1:
             return self._head_chunked(x, targets, mask, scale, grad=False)[0]
@@ -554,16 +558,17 @@ class B200Engine:
     @torch.no_grad()
     def forward_infer(self, input_ids, hidden) -> torch.Tensor:
         if self._native():
-            ex, st = self.exec, torch.cuda.current_stream()
-            ids, x, B, T = self._input(input_ids, hidden)
-            saved = ex.area("saved", ex.sizes(B, T, False, False, 0)[0], st)
-            if self.is_last:          # the LM head's fp32 accumulators are the result
-                logits = torch.empty(B, T, self.cfg.vocab_size, dtype=F32, device=self.device)
-                ex.forward(ids, x, saved, None, logits, B, T, False, st)
-                return logits
-            y = torch.empty(B, T, ex.d, dtype=BF16, device=self.device)
-            ex.forward(ids, x, saved, y, None, B, T, False, st)
-            return y.float()
+            with self.exec.lock:
+                ex, st = self.exec, torch.cuda.current_stream()
+                ids, x, B, T = self._input(input_ids, hidden)
+                saved = ex.area("saved", ex.sizes(B, T, False, False, 0)[0], st)
+                if self.is_last:          # the LM head's fp32 accumulators are the result
+                    logits = torch.empty(B, T, self.cfg.vocab_size, dtype=F32, device=self.device)
+                    ex.forward(ids, x, saved, None, logits, B, T, False, st)
+                    return logits
+                y = torch.empty(B, T, ex.d, dtype=BF16, device=self.device)
+                ex.forward(ids, x, saved, y, None, B, T, False, st)
+                return y.float()
         x, _, B, T = self._body_fwd(input_ids, hidden, False)
         if self.is_last:
             lnf, _, _ = K.layernorm_fwd(x, self.lnf_w, self.lnf_b)

@@ -7,6 +7,7 @@ never has to wait for the side stream before it can give a block out again.
 from __future__ import annotations
 
 import ctypes
+import threading
 import weakref
 from collections import OrderedDict
 from typing import Dict, List, Optional, Tuple
@@ -51,6 +52,9 @@ class StageExec:
         self.handle, self.lib, self.side, self.device, self.d = h.value, lib, side, device, d
         self._keep = (status, ends, blocks)
         weakref.finalize(self, lib.dsw_stage_destroy, self.handle)
+        # A pass is several calls of the library on work areas that the passes of a stream share, so a thread holds this
+        # from the first to the last of them.
+        self.lock = threading.RLock()
         self._sizes: Dict[tuple, Tuple[int, int]] = {}
         self._scratch: "OrderedDict[Tuple[str, int], torch.Tensor]" = OrderedDict()
         self._idle: List[SavedArea] = []
