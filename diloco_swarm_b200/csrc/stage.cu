@@ -72,6 +72,34 @@ struct GraphSlot {
 constexpr int GRAPH_TOKENS = 8192, GRAPH_SLOTS = 32;
 constexpr long long GRAPH_COPY = 6 << 20;
 
+// A point on the side stream that streams wait for.
+struct SideMark {
+  cudaEvent_t ev;
+  bool used;                     // recorded so far
+  unsigned long long seen;       // the stream that waited for it last: need not again
+};
+constexpr unsigned long long NOBODY = ~0ull;
+
+// The side stream's marks.  Those of a capture mean nothing outside of it, and one stream's wait is not another's.
+struct SideMarks {
+  cudaEvent_t fork;              // main -> side
+  SideMark done[2];              // side work of the last block of each parity
+  SideMark head;                 // side work on the logits
+  SideMark* all[3] = {&done[0], &done[1], &head};
+  bool create() {
+    bool ok = cudaEventCreateWithFlags(&fork, cudaEventDisableTiming) == cudaSuccess;
+    for (SideMark* m : all) ok = ok && cudaEventCreateWithFlags(&m->ev, cudaEventDisableTiming) == cudaSuccess;
+    return ok;
+  }
+  void destroy() {
+    cudaEventDestroy(fork);
+    for (SideMark* m : all) cudaEventDestroy(m->ev);
+  }
+  void forget() {
+    for (SideMark* m : all) m->used = false;
+  }
+};
+
 struct Stage {
   int n, d, nh, V;
   int* status;
@@ -83,10 +111,7 @@ struct Stage {
   const bf16* head_w;
   float *dhead_w, *count;
   std::vector<Block> blocks;
-  cudaEvent_t fork;              // main -> side
-  cudaEvent_t side_done[2];      // side work of the last block of each parity
-  cudaEvent_t head_done;         // side work on the logits
-  bool side_used[2], head_used;
+  SideMarks live, captured;      // of passes queued on the callers' streams; of a graph while it is captured
   cudaStream_t cap;              // graphs are captured here
   std::vector<GraphSlot> graphs;
   unsigned long long tick;
@@ -242,6 +267,13 @@ struct Run {
   Stage& s;
   int B, T, M, deterministic;
   cudaStream_t st;               // the caller's, or the capturing one
+  SideMarks* marks = &s.live;
+  unsigned long long sid = stream_id(st);
+
+  static unsigned long long stream_id(cudaStream_t st) {
+    unsigned long long id;
+    return cudaStreamGetId(st, &id) == cudaSuccess ? id : NOBODY;
+  }
 
   int gemm(const void* A, const void* W, bool w_t, int N, int K, void* out, int mode, const float* bias, const void* resid,
            void* aux_out, const void* aux_in, int rows) const {
@@ -258,15 +290,27 @@ struct Run {
   // the side stream may use everything queued on the main stream so far
   int fork() const {
     if (!s.side) return 0;
-    TRY_CUDA(cudaEventRecord(s.fork, st));
-    TRY_CUDA(cudaStreamWaitEvent(s.side, s.fork, 0));
+    TRY_CUDA(cudaEventRecord(marks->fork, st));
+    TRY_CUDA(cudaStreamWaitEvent(s.side, marks->fork, 0));
     return 0;
   }
-
-  // everything queued on the side stream by earlier calls is done before what follows on the main stream
+  // what the side stream has been given so far is behind the mark
+  int mark(SideMark& m) const {
+    if (!s.side) return 0;
+    TRY_CUDA(cudaEventRecord(m.ev, s.side));
+    m.used = true;
+    m.seen = NOBODY;
+    return 0;
+  }
+  // what lies behind the mark is done before what follows on the main stream
+  int wait(SideMark& m) const {
+    if (!m.used || (m.seen == sid && sid != NOBODY)) return 0;
+    MAIN_WAIT(m.ev);
+    m.seen = sid;
+    return 0;
+  }
   int join() const {
-    for (int p = 0; p < 2; ++p)
-      if (s.side_used[p]) MAIN_WAIT(s.side_done[p]);
+    for (SideMark* m : marks->all) TRY(wait(*m));
     return 0;
   }
 
@@ -287,7 +331,7 @@ struct Run {
 
   int block_bwd(int l, const Block& b, const bf16* x, const Saved& v, const Scratch& c, const bf16* dx2, bf16* dx0) const {
     const int d = s.d, p = l & 1;
-    if (s.side_used[p]) MAIN_WAIT(s.side_done[p]);
+    TRY(wait(marks->done[p]));
     LAUNCH(gemm(dx2, b.w[W_PR], false, 4 * d, d, c.dh[p], DSW_EPI_MUL, nullptr, nullptr, nullptr, v.h, M));
     TRY(fork());
     SIDE(wgrad(dx2, v.g, d, 4 * d, b.dw[W_PR], M, side()));
@@ -303,10 +347,7 @@ struct Run {
     TRY(fork());
     SIDE(dsw_colsum_accum(c.dqkv[p], 3 * d, b.db[W_QKV], M, 3 * d, side()));
     SIDE(wgrad(c.dqkv[p], v.ln1, 3 * d, d, b.dw[W_QKV], M, side()));
-    if (s.side) {
-      TRY_CUDA(cudaEventRecord(s.side_done[p], s.side));
-      s.side_used[p] = true;
-    }
+    TRY(mark(marks->done[p]));
     LAUNCH(gemm(c.dqkv[p], b.w[W_QKV], false, d, 3 * d, c.dln, DSW_EPI_STORE, nullptr, nullptr, nullptr, nullptr, M));
     LAUNCH(dsw_layernorm_bwd(c.dln, x, b.ln1_w, v.mu1, v.rs1, c.dx1[p], dx0, b.dln1_w, b.dln1_b, b.db[W_O], c.ln, M, d, st));
     return 0;
@@ -339,10 +380,6 @@ struct Run {
     }
     slot->used = ++s.tick;
     if (slot->failed) return body();
-    // what earlier passes left on the side stream comes first; after that their events are free to be recorded again
-    TRY(join());
-    if (s.head_used) MAIN_WAIT(s.head_done);
-    s.side_used[0] = s.side_used[1] = s.head_used = false;
     if (!slot->exec) {
       TRY(capture(*slot, body));
       if (slot->failed) return body();
@@ -373,15 +410,16 @@ struct Run {
     slot.failed = true;
     if (cudaStreamBeginCapture(s.cap, cudaStreamCaptureModeThreadLocal) != cudaSuccess) { cudaGetLastError(); return 0; }
     st = s.cap;
+    marks = &s.captured;
+    marks->forget();
     dsw::tl_launch.pdl = false;
     int rc = body();
     if (rc == 0) rc = join();
-    if (rc == 0 && s.head_used) rc = cudaStreamWaitEvent(st, s.head_done, 0) == cudaSuccess ? 0 : -3;
     cudaGraph_t graph = nullptr;
     const bool ended = cudaStreamEndCapture(s.cap, &graph) == cudaSuccess && graph != nullptr;
     st = on;
+    marks = &s.live;
     dsw::tl_launch.pdl = false;
-    s.side_used[0] = s.side_used[1] = s.head_used = false;      // the capture joined the side stream
     slot.launches = g_launches.load(std::memory_order_relaxed) - before;
     g_launches.fetch_sub(slot.launches, std::memory_order_relaxed);
     if (rc == 0 && ended && cudaEventCreateWithFlags(&slot.launched, cudaEventDisableTiming) == cudaSuccess) {
@@ -398,10 +436,7 @@ struct Run {
   int head_grads(const Scratch& c, const bf16* ln, int r0, int m) const {
     TRY(fork());
     SIDE(wgrad(c.logits, ln, s.V, s.d, s.dhead_w, m, side()));
-    if (s.side) {
-      TRY_CUDA(cudaEventRecord(s.head_done, s.side));
-      s.head_used = true;
-    }
+    TRY(mark(marks->head));
     bf16* dln = c.dln + size_t(r0) * s.d;
     // m x d output tiles and a K of the whole vocabulary: few of them leave most SMs idle for hundreds of k-blocks (2128
     // rows of GPT-2 small: 27 CTA pairs, 238 us), so K is split, with the partial sums in the buffers of the blocks'
@@ -449,11 +484,7 @@ extern "C" int dsw_stage_create(const long long* desc, int len, void** out) {
     }
     s->blocks.push_back(b);
   }
-  bool ok = cudaEventCreateWithFlags(&s->fork, cudaEventDisableTiming) == cudaSuccess &&
-            cudaEventCreateWithFlags(&s->head_done, cudaEventDisableTiming) == cudaSuccess;
-  ok = ok && cudaStreamCreateWithFlags(&s->cap, cudaStreamNonBlocking) == cudaSuccess;
-  for (int i = 0; i < 2; ++i) ok = ok && cudaEventCreateWithFlags(&s->side_done[i], cudaEventDisableTiming) == cudaSuccess;
-  if (!ok) { delete s; return -2; }
+  if (!s->live.create() || !s->captured.create() || cudaStreamCreateWithFlags(&s->cap, cudaStreamNonBlocking) != cudaSuccess) { delete s; return -2; }
   *out = s;
   return 0;
 }
@@ -463,9 +494,8 @@ extern "C" int dsw_stage_destroy(void* stage) {
   if (!s) return 0;
   for (GraphSlot& g : s->graphs) Run::drop(g);
   cudaStreamDestroy(s->cap);
-  cudaEventDestroy(s->fork);
-  cudaEventDestroy(s->head_done);
-  for (int i = 0; i < 2; ++i) cudaEventDestroy(s->side_done[i]);
+  s->live.destroy();
+  s->captured.destroy();
   delete s;
   return 0;
 }
@@ -550,7 +580,6 @@ extern "C" int dsw_stage_head(void* stage, void* saved, void* scratch, const lon
   const Scratch c = take_scratch(ca, s, M, grad != 0, rows);
   const bf16* x = v.blk[s.n - 1].out;
   TRY(r.join());           // an earlier call may have laid the scratch out differently
-  if (s.head_used) MAIN_WAIT(s.head_done);
   LAUNCH(dsw_loss_begin(mask, M, s.count, loss, st));
   const int flags = (keep ? 1 : 0) | (deterministic ? 2 : 0) | chunks << 2;
   const bool unstored = unstored_logits(s, grad != 0, size_t(M));
@@ -570,7 +599,7 @@ extern "C" int dsw_stage_head(void* stage, void* saved, void* scratch, const lon
       LAUNCH(dsw_head_lse(ln, s.head_w, targets + r0, c.parts, c.tlogit, m, V, d, s.status, st));
       LAUNCH(dsw_head_rows(c.parts, c.tlogit, targets + r0, mk, s.count, scale, loss, grad ? c.rows : nullptr, m, V, s.status, st));
     }
-    if (rows < M && grad && s.head_used) MAIN_WAIT(s.head_done);      // the slice before is still read
+    if (rows < M && grad) TRY(r.wait(r.marks->head));      // the slice before is still read
     if (!unstored) {
       if (rows < M) LAUNCH(r.gemm(ln, s.head_w, true, V, d, c.logits, DSW_EPI_STORE, nullptr, nullptr, nullptr, nullptr, m));
       LAUNCH(dsw_cross_entropy(c.logits, V, targets + r0, mk, s.count, scale, loss, m, V, grad, s.status, st));

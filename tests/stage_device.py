@@ -1,0 +1,215 @@
+"""The stage executor's host code (csrc/stage.cu) compiled against stand-ins (stage_fakes.cpp), and a device that runs what
+it queues: streams, events, graph captures and replays with their ordering rules, and every kernel as the ranges that it
+reads and writes.  Two accesses of one range, one of them a write, that nothing orders are a race."""
+import ctypes
+import os
+import shutil
+import subprocess
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "diloco_swarm_b200", "csrc")
+ERROR = 999
+HOOK = ctypes.CFUNCTYPE(ctypes.c_longlong, ctypes.c_char_p)
+
+
+def build(folder):
+    """The executor as a shared library for the CPU (None without a compiler and CUDA's headers)."""
+    cxx, inc = shutil.which("g++"), "/usr/local/cuda/include"
+    if cxx is None or not os.path.exists(os.path.join(inc, "cuda_runtime.h")):
+        return None
+    out = os.path.join(str(folder), "libstage_fake.so")
+    here = os.path.dirname(os.path.abspath(__file__))
+    subprocess.check_call([cxx, "-O1", "-std=c++17", "-shared", "-fPIC", "-Wl,-Bsymbolic", "-x", "c++", "-I", inc, "-I", CSRC,
+                           os.path.join(here, "stage_fakes.cpp"), os.path.join(CSRC, "stage.cu"), "-o", out])
+    return out
+
+
+class Device:
+    def __init__(self, lib):
+        self.lib, self.error = lib, None
+        self._hook = HOOK(self._call)
+        lib.fake_set_hook(self._hook)
+        self.clocks, self.events, self.captures, self.graphs = {}, {}, {}, {}
+        self.accesses, self.races, self.names = [], [], []
+        self.counts, self.busy, self.next = {}, set(), 50000
+
+    # ------------------------------------------------------------------ ordering
+    def clock(self, s):
+        return self.clocks.setdefault(s, {s: 0})
+
+    def join(self, s, other):
+        c = self.clock(s)
+        for k, v in other.items():
+            c[k] = max(c.get(k, 0), v)
+
+    def launch(self, s, name, ranges):
+        c = self.clock(s)
+        c[s] += 1
+        self.names.append(name)
+        for how, at, n in ranges:
+            for how2, at2, n2, s2, when, name2 in self.accesses:
+                if (how, how2) != ("r", "r") and at < at2 + n2 and at2 < at + n and c.get(s2, 0) < when:
+                    self.races.append((name2, how2, name, how))
+            self.accesses.append((how, at, n, s, c[s], name))
+
+    # ------------------------------------------------------------------ what the executor calls
+    def _call(self, line):
+        try:
+            return self.handle(line.decode().split())
+        except Exception as e:                            # an exception must not cross the C frames
+            self.error = self.error or e
+            return ERROR
+
+    def handle(self, w):
+        kind = w[0]
+        args = [int(x) for x in w[1:] if x.lstrip("-").isdigit()] if kind != "launch" else []
+        self.counts[kind] = self.counts.get(kind, 0) + 1
+        if kind == "launch":
+            s, rest = int(w[2]), w[3:]
+            what = (w[1], [(rest[i], int(rest[i + 1]), int(rest[i + 2])) for i in range(0, len(rest), 3)])
+            cap = self.capturing(s)
+            if cap:
+                cap["ops"].append(("launch", s) + what)
+                cap["last"][s] = cap["last"].get(s, 0) + 1
+                self.see(cap, s)[s] = cap["last"][s]
+            else:
+                self.launch(s, *what)
+            return 0
+        return getattr(self, "do_" + kind)(*args)
+
+    def capturing(self, s):
+        for cap in self.captures.values():
+            if s in cap["streams"]:
+                return cap
+        return None
+
+    @staticmethod
+    def see(cap, s):
+        return cap["seen"].setdefault(s, {})
+
+    def do_status(self, s):
+        cap = self.capturing(s)
+        return cap["id"] if cap else 0
+
+    def do_begin(self, s):
+        self.next += 1
+        self.captures[self.next] = {"id": self.next, "origin": s, "streams": {s}, "ops": [], "seen": {}, "last": {}, "bad": False}
+        return 0
+
+    def do_end(self, s):
+        cap = self.capturing(s)
+        assert cap and cap["origin"] == s
+        del self.captures[cap["id"]]
+        joined = all(self.see(cap, s).get(o, 0) >= n for o, n in cap["last"].items())
+        if cap["bad"] or not joined:
+            return 0
+        self.graphs[cap["id"]] = cap["ops"]
+        return cap["id"]
+
+    def do_instantiate(self, g):
+        return 0
+
+    def do_destroy(self, g):
+        assert g not in self.busy, "a graph was destroyed while it may still run"
+        self.graphs.pop(g)
+        return 0
+
+    def do_record(self, e, s):
+        cap = self.capturing(s)
+        if cap:
+            cap["ops"].append(("record", s, e))
+            self.events[e] = (cap["id"], dict(self.see(cap, s)))
+        else:
+            self.events[e] = (0, dict(self.clock(s)))
+        return 0
+
+    def do_wait(self, s, e):
+        if e not in self.events:
+            return 0
+        of, when = self.events[e]
+        cap = self.capturing(s)
+        if cap is None and of in self.captures:
+            cap = self.captures[of]                       # the stream joins the capture
+            cap["streams"].add(s)
+        if cap is None:
+            if of:
+                return ERROR                              # recorded under a capture that is over
+            self.join(s, when)
+            return 0
+        if of != cap["id"]:
+            cap["bad"] = True                             # a dependency on work outside of the capture
+            return ERROR
+        cap["ops"].append(("wait", s, e))
+        seen = self.see(cap, s)
+        for k, v in when.items():
+            seen[k] = max(seen.get(k, 0), v)
+        return 0
+
+    def do_replay(self, g, s):
+        cap = self.capturing(s)
+        if cap:
+            cap["ops"] += self.graphs[g]
+            return 0
+        self.busy.add(g)
+        self.next += 1
+        tag, start, events, mine = self.next, dict(self.clock(s)), {}, {}
+        for op in self.graphs[g]:
+            p = mine.setdefault(op[1], (tag, op[1]))
+            if p not in self.clocks:
+                self.clocks[p] = {**start, p: 0}
+            if op[0] == "launch":
+                self.launch(p, op[2], op[3])
+            elif op[0] == "record":
+                events[op[2]] = dict(self.clocks[p])
+            else:
+                self.join(p, events[op[2]])
+        for p in mine.values():
+            self.join(s, self.clocks[p])
+        return 0
+
+    def do_sync(self, e):
+        assert not self.events.get(e, (0,))[0], "waited for an event of a capture"
+        self.busy.clear()
+        return 0
+
+    def do_query(self, e):
+        assert not self.events.get(e, (0,))[0], "asked for an event of a capture"
+        return 600 if self.busy else 0                    # not ready
+
+
+class FakeStage:
+    """A stage of ``n`` blocks in areas at made-up addresses."""
+
+    def __init__(self, lib, n=2, d=64, heads=1, vocab=512, first=True, last=True, side=7):
+        self.lib, self.n, self.d, self.vocab, self.first, self.last = lib, n, d, vocab, first, last
+        p = iter(range(1 << 50, 1 << 51, 1 << 20))
+        ends = [next(p) if have else 0 for have in [first] * 4 + [last] * 7]
+        desc = [n, d, heads, vocab, 0, side] + ends[:4] + ends[4:8] + ends[8:11] + [next(p) for _ in range(24 * n)]
+        h = ctypes.c_void_p()
+        rc = lib.dsw_stage_create((ctypes.c_longlong * len(desc))(*desc), len(desc), ctypes.byref(h))
+        assert rc == 0
+        self.h = h
+
+    def sizes(self, B, T, keep, grad, chunks):
+        a, b = ctypes.c_size_t(), ctypes.c_size_t()
+        assert self.lib.dsw_stage_sizes(self.h, B, T, keep, grad, chunks, ctypes.byref(a), ctypes.byref(b)) == 0
+        return a.value, b.value
+
+    def _p(self, x):
+        return ctypes.c_void_p(x) if x else None
+
+    def forward(self, saved, B, T, st, keep=1, x=None, y=None, logits=None):
+        ids = self._p(1 << 44) if self.first else None
+        return self.lib.dsw_stage_forward(self.h, ids, self._p(x), self._p(saved), self._p(y), self._p(logits), B, T, keep, self._p(st))
+
+    def head(self, saved, scratch, B, T, st, keep=1, grad=1, chunks=1, det=0):
+        return self.lib.dsw_stage_head(self.h, self._p(saved), self._p(scratch), self._p((1 << 44) + 4096), None, ctypes.c_float(1.0),
+                                       self._p((1 << 44) + 8192), B, T, keep, grad, chunks, det, self._p(st))
+
+    def backward(self, saved, scratch, B, T, st, hi=None, lo=0, dy=None, x=None, dx0=None, chunks=1, det=0):
+        ids = self._p(1 << 44) if self.first else None
+        return self.lib.dsw_stage_backward(self.h, self.n if hi is None else hi, lo, self._p(dy), self._p(x), ids, self._p(saved),
+                                           self._p(scratch), self._p(dx0), B, T, chunks, det, self._p(st))
+
+    def train(self, saved, scratch, B, T, st, **kw):
+        """One microbatch of a stage that owns both ends."""
+        return (self.forward(saved, B, T, st), self.head(saved, scratch, B, T, st, **kw), self.backward(saved, scratch, B, T, st, **kw))

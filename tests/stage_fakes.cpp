@@ -1,0 +1,142 @@
+// Stand-ins for what the stage executor (csrc/stage.cu) calls: the CUDA runtime's streams, events and graphs and the
+// library's own launchers.  Each hands one line of text to the test, which emulates the device and gives the return code:
+//   launch <name> <stream> [r <address> <bytes> | w <address> <bytes>]...
+//   record <event> <stream> | wait <stream> <event> | begin <stream> | end <stream> | instantiate <graph> |
+//   replay <graph> <stream> | sync <event> | query <event> | destroy <graph> | status <stream> | id <stream>
+// Gradients that kernels add to (commutative, any order) are left out; nothing is ever dereferenced.
+#include <cuda_runtime.h>
+#include <cstdio>
+#include <initializer_list>
+#include <string>
+#include "dswarm.h"
+#include "launch.h"
+
+namespace dsw {
+thread_local LaunchMode tl_launch;
+}
+
+static long long (*g_hook)(const char*) = nullptr;
+static long long g_handles = 1000;
+extern "C" void fake_set_hook(long long (*hook)(const char*)) { g_hook = hook; }
+
+static long long tell(const std::string& line) { return g_hook(line.c_str()); }
+static std::string num(const void* p) { return " " + std::to_string(reinterpret_cast<long long>(p)); }
+static std::string num(long long v) { return " " + std::to_string(v); }
+
+struct Range { char how; const void* at; long long bytes; };
+static int op(const char* name, cudaStream_t st, std::initializer_list<Range> ranges) {
+  std::string line = std::string("launch ") + name + num(st);
+  for (const Range& r : ranges)
+    if (r.at && r.bytes > 0) line += std::string(" ") + r.how + num(r.at) + num(r.bytes);
+  return int(tell(line));
+}
+
+// ---------------------------------------------------------------- runtime
+static cudaError_t err(long long rc) { return static_cast<cudaError_t>(rc); }
+template <class T> static cudaError_t made(T* out) { *out = reinterpret_cast<T>(++g_handles); return cudaSuccess; }
+extern "C" {
+cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }
+cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int) { *v = 148; return cudaSuccess; }
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { return made(e); }
+cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) { return made(s); }
+cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) { return err(tell("record" + num(e) + num(s))); }
+cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, unsigned) { return err(tell("wait" + num(s) + num(e))); }
+cudaError_t cudaEventSynchronize(cudaEvent_t e) { return err(tell("sync" + num(e))); }
+cudaError_t cudaEventQuery(cudaEvent_t e) { return err(tell("query" + num(e))); }
+cudaError_t cudaStreamBeginCapture(cudaStream_t s, cudaStreamCaptureMode) { return err(tell("begin" + num(s))); }
+cudaError_t cudaStreamEndCapture(cudaStream_t s, cudaGraph_t* g) {
+  const long long id = tell("end" + num(s));
+  *g = reinterpret_cast<cudaGraph_t>(id);
+  return id ? cudaSuccess : cudaErrorStreamCaptureInvalidated;
+}
+cudaError_t cudaGraphInstantiate(cudaGraphExec_t* x, cudaGraph_t g, unsigned long long) {
+  *x = reinterpret_cast<cudaGraphExec_t>(g);
+  return err(tell("instantiate" + num(g)));
+}
+cudaError_t cudaGraphDestroy(cudaGraph_t) { return cudaSuccess; }
+cudaError_t cudaGraphExecDestroy(cudaGraphExec_t x) { return err(tell("destroy" + num(x))); }
+cudaError_t cudaGraphLaunch(cudaGraphExec_t x, cudaStream_t s) { return err(tell("replay" + num(x) + num(s))); }
+cudaError_t cudaStreamGetCaptureInfo(cudaStream_t s, cudaStreamCaptureStatus* st, unsigned long long* id, cudaGraph_t*,
+                                     const cudaGraphNode_t**, size_t*) {
+  const long long c = tell("status" + num(s));                // 0, or a number of the capture that the stream is part of
+  *st = c ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone;
+  if (id) *id = (unsigned long long)c;
+  return cudaSuccess;
+}
+cudaError_t cudaStreamGetId(cudaStream_t s, unsigned long long* id) {
+  *id = reinterpret_cast<unsigned long long>(s);
+  return cudaSuccess;
+}
+cudaError_t cudaMemcpyAsync(void* to, const void* from, size_t n, cudaMemcpyKind, cudaStream_t st) {
+  return err(op("copy", st, {{'r', from, (long long)n}, {'w', to, (long long)n}}));
+}
+
+// ---------------------------------------------------------------- launchers
+int dsw_gemm_bf16(const void* A, long long lda, int a_mn, const void* B, long long ldb, int b_mn, int M, int N, int K, int mode, int,
+                  void* out, long long ldo, const float*, const void* resid, long long, void* aux_out, const void* aux_in, long long,
+                  int, int, int*, cudaStream_t st) {
+  const long long mn = 2LL * M * N;
+  return op("gemm", st, {{'r', A, 2LL * M * K}, {'r', B, 2LL * N * K}, {'r', resid, mn}, {'r', aux_in, mn}, {'w', aux_out, mn},
+                         {'w', mode == DSW_EPI_ATOMIC_F32 ? nullptr : out, mode >= DSW_EPI_ATOMIC_F32 ? 2 * mn : mn}});
+}
+int dsw_head_lse(const void* A, const void*, const long long*, float* parts, float* tlogit, int M, int N, int K, int*, cudaStream_t st) {
+  return op("head_lse", st, {{'r', A, 2LL * M * K}, {'w', parts, (N + 63) / 64 * 4LL * M}, {'w', tlogit, 4LL * M}});
+}
+int dsw_head_rows(const float* parts, const float* tlogit, const long long*, const long long*, const float*, float, float*, void* rows,
+                  int M, int N, int*, cudaStream_t st) {
+  return op("head_rows", st, {{'r', parts, (N + 63) / 64 * 4LL * M}, {'r', tlogit, 4LL * M}, {'w', rows, 16LL * M}});
+}
+int dsw_head_dlogits(const void* A, const void*, const void* rows, void* out, int M, int N, int K, int*, cudaStream_t st) {
+  return op("head_dlogits", st, {{'r', A, 2LL * M * K}, {'r', rows, 16LL * M}, {'w', out, 2LL * M * N}});
+}
+int dsw_gemm_partials(const void* A, const void*, int M, int N, int K, float* partials, int most, int* splits, int*, cudaStream_t st) {
+  *splits = most;
+  return op("gemm_partials", st, {{'r', A, 2LL * M * K}, {'w', partials, 4LL * most * M * N}});
+}
+int dsw_sum_partials_bf16(const float* partials, int splits, void* out, long long n, cudaStream_t st) {
+  return op("sum_partials", st, {{'r', partials, 4 * splits * n}, {'w', out, 2 * n}});
+}
+int dsw_attention_fwd(const void* qkv, void* out, float* lse, int B, int T, int nh, int hs, float, int*, cudaStream_t st) {
+  const long long n = 2LL * B * T * nh * hs;
+  return op("attention_fwd", st, {{'r', qkv, 3 * n}, {'w', out, n}, {'w', lse, 4LL * B * T * nh}});
+}
+int dsw_attention_bwd(const void* qkv, const void* out, const void* dout, const float* lse, void* dqkv, float* dq_acc, float* Dvec, int B,
+                      int T, int nh, int hs, float, int*, cudaStream_t st) {
+  const long long n = 2LL * B * T * nh * hs;
+  return op("attention_bwd", st, {{'r', qkv, 3 * n}, {'r', out, n}, {'r', dout, n}, {'r', lse, 4LL * B * T * nh}, {'w', dqkv, 3 * n},
+                                  {'w', dq_acc, 2 * n}, {'w', Dvec, 4LL * B * T * nh}});
+}
+int dsw_layernorm_fwd(const void* x, const float* g, const float* b, void* y, float* mean, float* rstd, int M, int d, float e,
+                      cudaStream_t st) {
+  return dsw_layernorm_fwd_lo(x, nullptr, g, b, y, mean, rstd, M, d, e, st);
+}
+int dsw_layernorm_fwd_lo(const void* x, const void* lo, const float*, const float*, void* y, float* mean, float* rstd, int M, int d, float,
+                         cudaStream_t st) {
+  const long long n = 2LL * M * d;
+  return op("layernorm_fwd", st, {{'r', x, n}, {'r', lo, n}, {'w', y, n}, {'w', mean, 4LL * M}, {'w', rstd, 4LL * M}});
+}
+int dsw_layernorm_bwd_blocks(int) { return 296; }
+int dsw_layernorm_bwd(const void* dy, const void* x, const float*, const float* mean, const float* rstd, const void* dres, void* dx, float*,
+                      float*, float*, float* scratch, int M, int d, cudaStream_t st) {
+  const long long n = 2LL * M * d;
+  return op("layernorm_bwd", st, {{'r', dy, n}, {'r', x, n}, {'r', mean, 4LL * M}, {'r', rstd, 4LL * M}, {'r', dres, n}, {'w', dx, n},
+                                  {'w', scratch, 296LL * 12 * d}});
+}
+int dsw_colsum_accum(const void* x, long long, float*, int M, int N, cudaStream_t st) {
+  return op("colsum", st, {{'r', x, 2LL * M * N}});
+}
+int dsw_embedding_fwd(const long long* ids, const float*, const float*, void* y, int B, int T, int d, int, int*, cudaStream_t st) {
+  return op("embedding_fwd", st, {{'r', ids, 8LL * B * T}, {'w', y, 2LL * B * T * d}});
+}
+int dsw_embedding_bwd(const long long* ids, const void* dx, float*, float*, int B, int T, int d, int, cudaStream_t st) {
+  return op("embedding_bwd", st, {{'r', ids, 8LL * B * T}, {'r', dx, 2LL * B * T * d}});
+}
+int dsw_loss_begin(const long long*, int, float*, float*, cudaStream_t st) { return op("loss_begin", st, {}); }
+int dsw_cross_entropy(void* logits, long long, const long long*, const long long*, const float*, float, float*, int M, int V, int grad, int*,
+                      cudaStream_t st) {
+  return op("cross_entropy", st, {{'r', logits, 2LL * M * V}, {'w', grad ? logits : nullptr, 2LL * M * V}});
+}
+}  // extern "C"

@@ -1,0 +1,63 @@
+"""Order of the stage executor's work on its streams: every two accesses of a work area that meet are ordered, launch by
+launch and replayed, on one calling stream and on two (stage_device.py)."""
+import ctypes
+
+import pytest
+
+from stage_device import Device, FakeStage, build
+
+AREA = 1 << 32                       # work areas lie this far apart
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    path = build(tmp_path_factory.mktemp("stage"))
+    if path is None:
+        pytest.skip("needs g++ and CUDA's headers")
+    return ctypes.CDLL(path)
+
+
+@pytest.fixture
+def device(lib):
+    dev = Device(lib)
+    yield dev
+    assert dev.error is None, dev.error
+
+
+def ordered(dev, *codes):
+    assert all(c == 0 for group in codes for c in (group if isinstance(group, tuple) else (group,))), codes
+    assert dev.races == [], dev.races[:5]
+
+
+@pytest.mark.parametrize("blocks", [1, 2, 3, 4])
+@pytest.mark.parametrize("vocab,chunks", [(512, 1), (512, 3), (4096, 1)])
+@pytest.mark.parametrize("B,T", [(2, 512), (16, 1024)])               # replayed from the third pass on, and never
+def test_microbatches_on_one_stream(device, blocks, vocab, chunks, B, T):
+    s = FakeStage(device.lib, n=blocks, vocab=vocab)
+    rcs = [s.train((2 + i % 2) * AREA, 5 * AREA, B, T, 1, chunks=chunks) for i in range(7)]
+    ordered(device, *rcs)
+    assert ("replay" in device.counts) == (B * T <= 8192)
+
+
+def test_a_detector_that_detects(device):
+    """Two streams that use one scratch without waiting for one another."""
+    s = FakeStage(device.lib)
+    s.train(2 * AREA, 5 * AREA, 2, 512, 1)
+    s.train(3 * AREA, 5 * AREA, 2, 512, 2)
+    assert device.races
+
+
+@pytest.mark.parametrize("blocks", [1, 3])
+@pytest.mark.parametrize("B,T", [(2, 512), (16, 1024)])
+def test_a_pass_on_another_stream_hides_no_side_work(device, blocks, B, T):
+    """Training on stream 1 leaves weight gradients on the side stream; passes of stream 2, replayed ones among them, in
+    areas of their own must not make stream 1 forget to wait for it."""
+    s = FakeStage(device.lib, n=blocks)
+    rcs = []
+    for i in range(8):
+        saved = 2 + i % 2                                # two areas in turn, each free once the side work of its pass is done
+        device.do_wait(1, saved)
+        rcs.append(s.train(saved * AREA, 5 * AREA, B, T, 1))
+        device.do_record(saved, 7)
+        rcs += [s.forward(8 * AREA, 1, 64, 2, keep=0), s.head(8 * AREA, 9 * AREA, 1, 64, 2, keep=0, grad=0)]
+    ordered(device, *rcs)
