@@ -542,7 +542,7 @@ extern "C" int dsw_stage_forward(void* stage, const long long* ids, const void* 
   // Sampling: the residual stream, whose rounding at every addition is most of what bf16 costs the logits, keeps its low
   // half in a second bf16 array (GPT-2 small, 5 x 24 tokens: error of the logits 9.2e-3 without, see the test)
   const bool precise = infer_logits != nullptr && !keep;
-  const GraphKey key{0, B, T, (keep ? 1 : 0) | (precise ? 2 : 0), saved, nullptr};
+  const GraphKey key{0, B, T, (keep ? 1 : 0) | (infer_logits ? 2 : 0), saved, nullptr};
   TRY(r.replayed(key, copies || (s.wte && !y), [&]() -> int {
     const bf16 *cur = in, *cur_lo = nullptr;
     for (int l = 0; l < s.n; ++l) {
@@ -581,7 +581,7 @@ extern "C" int dsw_stage_head(void* stage, void* saved, void* scratch, const lon
   const bf16* x = v.blk[s.n - 1].out;
   TRY(r.join());           // an earlier call may have laid the scratch out differently
   LAUNCH(dsw_loss_begin(mask, M, s.count, loss, st));
-  const int flags = (keep ? 1 : 0) | (deterministic ? 2 : 0) | chunks << 2;
+  const int flags = (keep ? 1 : 0) | (deterministic ? 2 : 0) | (grad ? 4 : 0) | chunks << 3;
   const bool unstored = unstored_logits(s, grad != 0, size_t(M));
   const auto dlogits = [&](const bf16* ln, int m) {
     return dsw_head_dlogits(ln, s.head_w, c.rows, c.logits, m, V, d, s.status, r.st);

@@ -61,3 +61,23 @@ def test_a_pass_on_another_stream_hides_no_side_work(device, blocks, B, T):
         device.do_record(saved, 7)
         rcs += [s.forward(8 * AREA, 1, 64, 2, keep=0), s.head(8 * AREA, 9 * AREA, 1, 64, 2, keep=0, grad=0)]
     ordered(device, *rcs)
+
+
+def test_a_graph_is_found_by_all_that_shaped_it(device):
+    """Calls that differ in one argument only are not served by the other's graph: with a gradient the logits of a wide
+    model are stored, without one they are not; a forward that is to end in logits has a LayerNorm more."""
+    def launched(calls, s):
+        out = []
+        for call in calls:
+            at = len(device.names)
+            assert call(s) == 0
+            out.append(device.names[at:])
+        return out
+
+    head = lambda grad: lambda s: s.head(2 * AREA, 5 * AREA, 2, 64, 1, keep=1, grad=grad)
+    fwd = lambda logits: lambda s: s.forward(2 * AREA, 2, 64, 1, keep=1, logits=logits)
+    for kind in ([head(0)] * 3 + [head(1)] * 3, [head(1)] * 3 + [head(0)] * 3, [fwd(None)] * 3 + [fwd(7 * AREA)] * 3,
+                 [fwd(7 * AREA)] * 3 + [fwd(None)] * 3):
+        got = launched(kind, FakeStage(device.lib, d=512, heads=8))
+        assert got[0] == got[1] == got[2] and got[3] == got[4] == got[5]
+        assert got[3] == launched(kind[3:4], FakeStage(device.lib, d=512, heads=8))[0] != got[0]
