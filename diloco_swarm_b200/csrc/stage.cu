@@ -112,6 +112,8 @@ struct Stage {
   float *dhead_w, *count;
   std::vector<Block> blocks;
   SideMarks live, captured;      // of passes queued on the callers' streams; of a graph while it is captured
+  SideMarks callers;             // of passes under a capture of the caller's
+  unsigned long long callers_id; // which one
   cudaStream_t cap;              // graphs are captured here
   std::vector<GraphSlot> graphs;
   unsigned long long tick;
@@ -269,6 +271,20 @@ struct Run {
   cudaStream_t st;               // the caller's, or the capturing one
   SideMarks* marks = &s.live;
   unsigned long long sid = stream_id(st);
+  bool callers = false;          // the caller captures its stream
+
+  Run(Stage& stage, int B_, int T_, int det, cudaStream_t stream) : s(stage), B(B_), T(T_), M(B_ * T_), deterministic(det), st(stream) {
+    // Under a capture of the caller's everything is queued launch by launch, and only what the same capture has put on
+    // the side stream can be waited for (nothing else uses the areas that it is given).
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    unsigned long long id = 0;
+    if (cudaStreamGetCaptureInfo(st, &status, &id) != cudaSuccess) { cudaGetLastError(); return; }
+    if (status != cudaStreamCaptureStatusActive) return;
+    if (s.callers_id != id) s.callers.forget();
+    s.callers_id = id;
+    marks = &s.callers;
+    callers = true;
+  }
 
   static unsigned long long stream_id(cudaStream_t st) {
     unsigned long long id;
@@ -363,7 +379,7 @@ struct Run {
   // work areas).
   template <class F>
   int replayed(const GraphKey& key, bool own_memory, F&& body) {
-    if (!own_memory || M > GRAPH_TOKENS || !graphs_on()) return body();
+    if (!own_memory || M > GRAPH_TOKENS || callers || !graphs_on()) return body();
     GraphSlot* slot = nullptr;
     for (GraphSlot& g : s.graphs)
       if (g.key == key) { slot = &g; break; }
@@ -484,7 +500,8 @@ extern "C" int dsw_stage_create(const long long* desc, int len, void** out) {
     }
     s->blocks.push_back(b);
   }
-  if (!s->live.create() || !s->captured.create() || cudaStreamCreateWithFlags(&s->cap, cudaStreamNonBlocking) != cudaSuccess) { delete s; return -2; }
+  if (!s->live.create() || !s->captured.create() || !s->callers.create() ||
+       cudaStreamCreateWithFlags(&s->cap, cudaStreamNonBlocking) != cudaSuccess) { delete s; return -2; }
   *out = s;
   return 0;
 }
@@ -496,6 +513,7 @@ extern "C" int dsw_stage_destroy(void* stage) {
   cudaStreamDestroy(s->cap);
   s->live.destroy();
   s->captured.destroy();
+  s->callers.destroy();
   delete s;
   return 0;
 }
@@ -525,7 +543,7 @@ extern "C" int dsw_stage_forward(void* stage, const long long* ids, const void* 
   if (B <= 0 || T <= 0 || s.n < 1 || (s.wte ? ids == nullptr : x == nullptr)) return -10;
   std::lock_guard<std::mutex> lock(s.mu);
   const Dependent mode;
-  Run r{s, B, T, B * T, 0, st};
+  Run r(s, B, T, 0, st);
   Area a(saved);
   const SavedAll v = take_saved(a, s, size_t(B) * T, keep != 0);
   const bf16* in = static_cast<const bf16*>(x);
@@ -573,7 +591,7 @@ extern "C" int dsw_stage_head(void* stage, void* saved, void* scratch, const lon
   std::lock_guard<std::mutex> lock(s.mu);
   const Dependent mode;
   const int M = B * T, d = s.d, V = s.V;
-  Run r{s, B, T, M, deterministic, st};
+  Run r(s, B, T, deterministic, st);
   Area a(saved), ca(scratch);
   const SavedAll v = take_saved(a, s, M, keep != 0);
   const int rows = int(head_rows(M, chunks));
@@ -631,7 +649,7 @@ extern "C" int dsw_stage_backward(void* stage, int hi, int lo, const void* dy, c
   if (B <= 0 || T <= 0 || hi > s.n || lo < 0) return -10;
   std::lock_guard<std::mutex> lock(s.mu);
   const Dependent mode;
-  Run r{s, B, T, B * T, deterministic, st};
+  Run r(s, B, T, deterministic, st);
   Area a(saved), ca(scratch);
   const SavedAll v = take_saved(a, s, size_t(r.M), true);
   const Scratch c = take_scratch(ca, s, size_t(r.M), true, chunks > 0 ? head_rows(size_t(r.M), chunks) : 0);

@@ -411,12 +411,11 @@ class B200Engine:
         assert mk is None or (mk.dtype == torch.long and mk.numel() == B * T)
         self.exec.head(saved, scratch, tg, mk, scale, loss, B, T, grad, grad, self.head_chunks, st)
 
-    def _exec_backward(self, area: SavedArea, dy, ids, x, B: int, T: int, sync: bool, chunks: int, st
+    def _exec_backward(self, area: SavedArea, scratch, dy, ids, x, B: int, T: int, sync: bool, chunks: int, st
                        ) -> Optional[torch.Tensor]:
-        """Backward of the blocks (and the embedding) behind ``dy``, or behind what the head left in the scratch;
+        """Backward of the blocks (and the embedding) behind ``dy``, or behind what the head left in ``scratch``;
         gradient buckets are sent as they are completed when ``sync``."""
         ex, n = self.exec, len(self.blocks)
-        scratch = ex.area("scratch", ex.sizes(B, T, True, True, chunks)[1], st)
         dx0 = None if self.is_first and not K.deterministic() else torch.empty(B, T, ex.d, dtype=BF16, device=self.device)
         emb = ids if dx0 is None else None
         if sync and self.is_last:
@@ -469,8 +468,9 @@ class B200Engine:
             if self.side is not None:
                 dx.record_stream(self.side)           # the last block's weight gradient reads it there
             with self.exec.lock:
-                return self._exec_backward(s["area"], dx, s["ids"], s["x"], B, T, self._want_overlap(sync), 0,
-                                           torch.cuda.current_stream())
+                ex, st = self.exec, torch.cuda.current_stream()
+                scratch = ex.area("scratch", ex.sizes(B, T, True, True, 0)[1], st)
+                return self._exec_backward(s["area"], scratch, dx, s["ids"], s["x"], B, T, self._want_overlap(sync), 0, st)
         return self._body_bwd(s["saved"], dx.contiguous(), s["ids"], B, T, sync=self._want_overlap(sync))
 
     def _want_overlap(self, sync: bool) -> bool:
@@ -521,8 +521,9 @@ class B200Engine:
                 area = ex.take(saved_bytes, st)
                 loss = torch.empty((), dtype=F32, device=self.device)
                 ex.forward(ids, x, area.buf, None, None, B, T, True, st)
-                self._exec_head(area.buf, ex.area("scratch", scratch_bytes, st), targets, mask, scale, loss, B, T, True, st)
-                return loss, self._exec_backward(area, None, ids, x, B, T, self._want_overlap(sync), chunks, st)
+                scratch = ex.area("scratch", scratch_bytes, st)
+                self._exec_head(area.buf, scratch, targets, mask, scale, loss, B, T, True, st)
+                return loss, self._exec_backward(area, scratch, None, ids, x, B, T, self._want_overlap(sync), chunks, st)
         x, saved, B, T = self._body_fwd(input_ids, hidden, True)
         if self.head_chunks > 1:
             loss, lnf, mu, rs, dlnf = self._head_chunked(x, targets, mask, scale, grad=True)

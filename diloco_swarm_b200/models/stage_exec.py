@@ -79,7 +79,11 @@ class StageExec:
         return buf
 
     def area(self, kind: str, nbytes: int, stream: torch.cuda.Stream) -> torch.Tensor:
-        """Scratch of this calling stream, at least ``nbytes``: its contents live within one pass."""
+        """Scratch of this calling stream, at least ``nbytes``: its contents live within one pass.  Under a capture of
+        the caller's it is the capture's own, and so are the areas of ``take``: replays must not meet other passes there,
+        and a capture cannot wait for work from outside of it."""
+        if torch.cuda.is_current_stream_capturing():
+            return self._alloc(nbytes)
         key = (kind, stream.cuda_stream)
         buf = self._scratch.get(key)
         if buf is None or buf.numel() < nbytes:
@@ -91,6 +95,8 @@ class StageExec:
         return buf
 
     def take(self, nbytes: int, stream: torch.cuda.Stream) -> SavedArea:
+        if torch.cuda.is_current_stream_capturing():
+            return SavedArea(self._alloc(nbytes), stream)
         for i, a in enumerate(self._idle):
             if a.buf.numel() == nbytes:
                 del self._idle[i]
@@ -104,6 +110,8 @@ class StageExec:
 
     def give(self, area: SavedArea, stream: torch.cuda.Stream) -> None:
         """The backward that read ``area`` has been queued on ``stream`` (and the side stream)."""
+        if torch.cuda.is_current_stream_capturing():
+            return
         if area.free is None:
             area.free = torch.cuda.Event()
         area.free.record(self.side if self.side is not None else stream)

@@ -35,6 +35,7 @@ class Buffer:
 @pytest.fixture
 def executor(monkeypatch):
     monkeypatch.setattr(torch.cuda, "Event", Event)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
     ex = StageExec.__new__(StageExec)
     ex.side, ex._idle, ex._alloc = Stream(), [], Buffer
     return ex
@@ -59,3 +60,17 @@ def test_a_backward_on_another_stream_is_recorded(executor):
     area = executor.take(100, a)
     executor.give(area, b)
     assert area.buf.recorded == [b] and isinstance(area, SavedArea)
+
+
+def test_a_capture_has_areas_of_its_own(executor, monkeypatch):
+    """Under a capture of the caller's no kept area is used, none is kept, and no event from outside is waited for."""
+    executor._scratch, a = {}, Stream()
+    a.cuda_stream = 1
+    area = executor.take(100, a)
+    executor.give(area, a)
+    scratch = executor.area("scratch", 100, a)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: True)
+    mine = executor.take(100, a)
+    assert mine is not area and executor.area("scratch", 100, a) is not scratch and a.waited == []
+    executor.give(mine, a)
+    assert executor._idle == [area] and list(executor._scratch.values()) == [scratch] and mine.free is None

@@ -81,3 +81,24 @@ def test_a_graph_is_found_by_all_that_shaped_it(device):
         got = launched(kind, FakeStage(device.lib, d=512, heads=8))
         assert got[0] == got[1] == got[2] and got[3] == got[4] == got[5]
         assert got[3] == launched(kind[3:4], FakeStage(device.lib, d=512, heads=8))[0] != got[0]
+
+
+@pytest.mark.parametrize("chunks", [1, 3])
+def test_a_capture_by_the_caller(device, chunks):
+    """After training, queued and replayed, the caller captures a whole microbatch and a forward in areas of their own: no
+    wait for work from outside breaks the capture, and once the caller has joined the side stream it ends well."""
+    s = FakeStage(device.lib, n=3)
+    rcs = [s.train(2 * AREA, 5 * AREA, 16, 1024, 1, chunks=chunks), s.train(3 * AREA, 6 * AREA, 2, 512, 1, chunks=chunks)]
+    device.do_record(3, 7)
+    for i in range(3):
+        device.do_begin(1)
+        rcs += [s.train(10 * AREA, 11 * AREA, 2, 512, 1, chunks=chunks), s.forward(12 * AREA, 2, 512, 1, keep=0, logits=13 * AREA)]
+        device.do_record(91, 7)
+        device.do_wait(1, 91)
+        graph = device.do_end(1)
+        assert graph
+        device.do_replay(graph, 1)
+        device.do_wait(1, 3)                             # the area is free again
+        rcs.append(s.train(3 * AREA, 6 * AREA, 2, 512, 1, chunks=chunks))
+        device.do_record(3, 7)
+    ordered(device, *rcs)
