@@ -21,10 +21,10 @@
 // 256 TMEM columns each), so one CTA's MMAs run under the other's softmax.
 // Only kv tiles up to the diagonal are visited; the diagonal tile is masked.
 //
-// Head size 32 (the 4-head, 128-wide test model) runs the same tiles: its tensor maps describe the matrix as
-// (32 columns, head, row) and the 64-column box reaches past the head, so TMA fills the right half of each
+// The tensor maps describe the matrices as (head's columns, head, row, sequence).  Head size 32 (the 4-head, 128-wide
+// test model) runs the same tiles: the 64-column box reaches past the head, so TMA fills the right half of each
 // operand tile with zeros.  Q K^T and dO V^T are unchanged by the zero columns, the output tiles get zero
-// right halves, and the epilogues write the first 32 columns only.
+// right halves, and only the first 32 columns are written.
 #include <cuda.h>
 #include "ptx.cuh"
 #include "launch.h"
@@ -33,10 +33,13 @@
 
 namespace dsw {
 
-// [128 x 64] operand tile of column block `cb` (= part * heads + head) at `row`.
-__device__ __forceinline__ void att_load_tile(void* dst, const CUtensorMap* tm, uint64_t* bar, int hs, int cb, int row) {
-  if (hs == 64) tma_load_2d(dst, tm, bar, cb * 64, row);
-  else          tma_load_3d(dst, tm, bar, 0, cb, row);
+// [128 x 64] operand tile of column block `cb` (= part * heads + head) at `row` of sequence b.  The sequence is a dimension
+// of the maps, so a tile that reaches past its sequence's end holds zeros there and never a row of the next one, whose
+// infinities or NaN would spoil this one's products (0 x Inf); stores and reductions end there as well.
+// Per call against maps over all rows at once: forward unchanged; backward of 32 x 1024 tokens, 12 heads of 64, 370 -> 336 us,
+// 16 x 133 29.9 -> 28.5, 64 x 1024, 4 heads of 32, whose dK and dV had left row by row, 205 -> 186.
+__device__ __forceinline__ void att_load_tile(void* dst, const CUtensorMap* tm, uint64_t* bar, int cb, int row, int b) {
+  tma_load_4d(dst, tm, bar, 0, cb, row, b);
 }
 
 // Optional in-kernel timeline for tuning: when a trace buffer is registered (dsw_attention_set_trace),
@@ -176,17 +179,17 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, __nv_bfloat16
       if (w > 0 && !mbar_wait_warp(q_empty, (w - 1) & 1, abort_flag, status)) break;
       if (elect_one()) {
         mbar_expect_tx(q_full, ATT_TILE_BYTES);
-        att_load_tile(smem + AttSmem::Q_OFF, &tmap_qkv, q_full, hs, h, b * T + qi * ATT_BQ);
+        att_load_tile(smem + AttSmem::Q_OFF, &tmap_qkv, q_full, h, qi * ATT_BQ, b);
       }
       __syncwarp();
       for (int j = 0; j <= qi; ++j, ++g) {
         const int s = g & 1;
         if (!mbar_wait_warp(&kv_empty[s], ((g >> 1) & 1) ^ 1, abort_flag, status)) { ok = false; break; }
-        const int kvrow = b * T + j * ATT_BK;
+        const int kvrow = j * ATT_BK;
         if (elect_one()) {
           mbar_expect_tx(&kv_full[s], 2 * ATT_TILE_BYTES);
-          att_load_tile(smem + AttSmem::K_OFF + s * ATT_TILE_BYTES, &tmap_qkv, &kv_full[s], hs, nh + h, kvrow);
-          att_load_tile(smem + AttSmem::V_OFF + s * ATT_TILE_BYTES, &tmap_qkv, &kv_full[s], hs, 2 * nh + h, kvrow);
+          att_load_tile(smem + AttSmem::K_OFF + s * ATT_TILE_BYTES, &tmap_qkv, &kv_full[s], nh + h, kvrow, b);
+          att_load_tile(smem + AttSmem::V_OFF + s * ATT_TILE_BYTES, &tmap_qkv, &kv_full[s], 2 * nh + h, kvrow, b);
         }
         __syncwarp();
       }
@@ -436,7 +439,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, __nv_bfloat16
 // then, on pds_full, dV, dK (releasing the Q / dO stage), dQ.  TMA warp (one thread): K / V
 // of the item into the buffer of its parity, Q / dO pairs into two stages.  Reducer warp (one
 // thread): one bulk reduce-add per staged dQ tile, two bulk stores per item for dK / dV
-// (staged by the row warps in the P buffer, head size 64; with 32 the row warps store them).
+// (staged by the row warps in the P buffer).
 // Every wait is bounded; a wait that runs out sets the CTA's abort flag and the status word.
 struct AttBwdSmem {
   static constexpr int KV_BYTES = 2 * ATT_TILE_BYTES;               // K_j then V_j
@@ -536,8 +539,7 @@ constexpr int ATT_BWD_THREADS = 32 * (ATT_BWD_ROW_WARPS + 3);    // + MMA issuer
 __global__ void __launch_bounds__(ATT_BWD_THREADS, 1)
 attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_constant__ CUtensorMap tmap_do,
                      const __grid_constant__ CUtensorMap tmap_dq, const __grid_constant__ CUtensorMap tmap_dkv,
-                     const float* __restrict__ lse, const float* __restrict__ Dvec, __nv_bfloat16* __restrict__ dqkv,
-                     int T, int nh, int n_bh, int hs,
+                     const float* __restrict__ lse, const float* __restrict__ Dvec, int T, int nh, int n_bh, int hs,
                      float scale, int* status, long long* trace) {
   using L = AttBwdSmem;
   extern __shared__ uint8_t smem_raw[];
@@ -616,26 +618,26 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
       // are on their way while the item before still runs
       const int kb = w & 1;
       if (!mbar_wait_warp(&kv_empty[kb], ((w >> 1) & 1) ^ 1, abort_flag, status)) break;
-      const int kvrow = b * T + j * ATT_BK;
+      const int kvrow = j * ATT_BK;
       if (elect_one()) {
         mbar_expect_tx(&kv_full[kb], 2 * ATT_TILE_BYTES);
-        att_load_tile(smem + L::K_OFF + kb * L::KV_BYTES, &tmap_qkv, &kv_full[kb], hs, nh + h, kvrow);
-        att_load_tile(smem + L::V_OFF + kb * L::KV_BYTES, &tmap_qkv, &kv_full[kb], hs, 2 * nh + h, kvrow);
+        att_load_tile(smem + L::K_OFF + kb * L::KV_BYTES, &tmap_qkv, &kv_full[kb], nh + h, kvrow, b);
+        att_load_tile(smem + L::V_OFF + kb * L::KV_BYTES, &tmap_qkv, &kv_full[kb], 2 * nh + h, kvrow, b);
       }
       __syncwarp();
       for (int it = 0; it < steps; ++it, ++g) {
         const int s = g % L::QSTAGES;
         if (!mbar_wait_warp(&q_empty[s], ((g / L::QSTAGES) & 1) ^ 1, abort_flag, status)) { ok = false; break; }
-        const int qrow = b * T + (j + it) * ATT_BQ;
+        const int qrow = (j + it) * ATT_BQ;
         if (elect_one()) {
           mbar_expect_tx(&q_full[s], 2 * ATT_TILE_BYTES);
-          att_load_tile(smem + L::Q_OFF + s * ATT_TILE_BYTES, &tmap_qkv, &q_full[s], hs, h, qrow);
-          att_load_tile(smem + L::DO_OFF + s * ATT_TILE_BYTES, &tmap_do, &q_full[s], hs, h, qrow);
+          att_load_tile(smem + L::Q_OFF + s * ATT_TILE_BYTES, &tmap_qkv, &q_full[s], h, qrow, b);
+          att_load_tile(smem + L::DO_OFF + s * ATT_TILE_BYTES, &tmap_do, &q_full[s], h, qrow, b);
           // The pair two steps on is asked into L2 now: its load can only start when its stage is released, and
           // the time from there to the data is on the issuing thread's path.
           if (hs == 64 && it + 2 < steps) {
-            tma_prefetch_l2_2d(&tmap_qkv, h * 64, qrow + 2 * ATT_BQ);
-            tma_prefetch_l2_2d(&tmap_do, h * 64, qrow + 2 * ATT_BQ);
+            tma_prefetch_l2_4d(&tmap_qkv, 0, h, qrow + 2 * ATT_BQ, b);
+            tma_prefetch_l2_4d(&tmap_do, 0, h, qrow + 2 * ATT_BQ, b);
           }
         }
         __syncwarp();
@@ -755,37 +757,26 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
         const int b = bh / nh, h = bh - b * nh;
         for (int i = j; i < nq; ++i, ++g) {
           if (!mbar_wait(dq_staged, g & 1, abort_flag, status)) { ok = false; break; }
-          const int row_g = b * T + i * ATT_BQ;
-          if (hs == 64) {
-#pragma unroll
-            for (int hh = 0; hh < 2; ++hh)
-              asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2}], [%3];"
-                           ::"l"(&tmap_dq), "r"(h * ATT_HS + hh * 32), "r"(row_g),
-                             "r"(smem_u32(smem + L::DQ_OFF + hh * ATT_TILE_BYTES))
-                           : "memory");
-          } else {          // 32 columns per head: the first staging half is the whole dQ tile
-            asm volatile("cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2, %3}], [%4];"
-                         ::"l"(&tmap_dq), "r"(0), "r"(h), "r"(row_g), "r"(smem_u32(smem + L::DQ_OFF))
+          for (int hh = 0; hh * 32 < hs; ++hh)          // 32 columns per head: the first staging half is the whole dQ tile
+            asm volatile("cp.reduce.async.bulk.tensor.4d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2, %3, %4}], [%5];"
+                         ::"l"(&tmap_dq), "r"(hh * 32), "r"(h), "r"(i * ATT_BQ), "r"(b),
+                           "r"(smem_u32(smem + L::DQ_OFF + hh * ATT_TILE_BYTES))
                          : "memory");
-          }
           asm volatile("cp.async.bulk.commit_group;" ::: "memory");
           asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
           mbar_arrive(dq_stage_free);
         }
-        if (ok && hs == 64) {
+        if (ok) {
           // dK and dV of the item: two [128 x 64] bf16 tiles staged in the P buffer, one bulk store each
           if (!mbar_wait(dkv_staged, w & 1, abort_flag, status)) break;
-          const int kvrow = b * T + j * ATT_BK;
-          if ((j + 1) * ATT_BK <= T) {
 #pragma unroll
-            for (int which = 0; which < 2; ++which)
-              asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];"
-                           ::"l"(&tmap_dkv), "r"(((which + 1) * nh + h) * ATT_HS), "r"(kvrow),
-                             "r"(smem_u32(smem + L::P_OFF + which * ATT_TILE_BYTES))
-                           : "memory");
-            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-          }
+          for (int which = 0; which < 2; ++which)
+            asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3, %4}], [%5];"
+                         ::"l"(&tmap_dkv), "r"(0), "r"((which + 1) * nh + h), "r"(j * ATT_BK), "r"(b),
+                           "r"(smem_u32(smem + L::P_OFF + which * ATT_TILE_BYTES))
+                         : "memory");
+          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+          asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
           mbar_arrive(dkv_stored);
         }
         ++w;
@@ -893,7 +884,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
         // the item before was waited for when its dQ was taken out)
         if (it > 0 && !mbar_wait(dq_full, (g - 1) & 1, abort_flag, status)) { ok = false; break; }
         // ... and the bulk stores of the item before with the dK / dV tiles staged in the P buffer
-        if (it == 0 && w > 0 && hs == 64 && !mbar_wait(dkv_stored, (w - 1) & 1, abort_flag, status)) { ok = false; break; }
+        if (it == 0 && w > 0 && !mbar_wait(dkv_stored, (w - 1) & 1, abort_flag, status)) { ok = false; break; }
 #pragma unroll
         for (int cc = 0; cc < 2; ++cc) {
 #pragma unroll
@@ -923,10 +914,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
       }
       // the last step's dQ; its barrier also says that every dV / dK product of the item is done
       if (!ok || !drain_dq(g - 1)) { ok = false; break; }
-      // dV and dK rows of this kv tile (TMEM lane = kv row).  A tile that ends behind its sequence cannot leave as
-      // a whole (the rows there belong to the next sequence): its rows are stored one by one.
-      const bool whole = (j + 1) * ATT_BK <= T;
-      __nv_bfloat16* row = dqkv + (long long)(b * T + j * ATT_BK + r) * 3 * d + h * hs;
+      // dV and dK rows of this kv tile (TMEM lane = kv row)
       uint32_t vk[32], vv[32];
       tmem_ld_32x32(tm_dk + lane_addr + half * 32, vk);
       tmem_ld_32x32(tm_dv + lane_addr + half * 32, vv);
@@ -934,42 +922,22 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(dkv_free);          // the next item's first products may overwrite the sums
-      if (hs == 64 && whole) {
-        // staged as two 128-byte-swizzled [128 x 64] bf16 tiles (dK, dV) in the P buffer, which nothing reads
-        // any more; the reducer warp stores them with one bulk copy each
+      // staged as two 128-byte-swizzled [128 x 64] bf16 tiles (dK, dV) in the P buffer, which nothing reads any more; the
+      // reducer warp stores them with one bulk copy each
 #pragma unroll
-        for (int which = 0; which < 2; ++which) {
-          const uint32_t* v = which == 0 ? vk : vv;
+      for (int which = 0; which < 2; ++which) {
+        const uint32_t* v = which == 0 ? vk : vv;
 #pragma unroll
-          for (int c = 0; c < 4; ++c)
-            *reinterpret_cast<uint4*>(sp + which * ATT_TILE_BYTES + r * 128 + (((half * 4 + c) ^ (r & 7)) << 4)) = make_uint4(
-                pack_bf16(__uint_as_float(v[8 * c]), __uint_as_float(v[8 * c + 1])),
-                pack_bf16(__uint_as_float(v[8 * c + 2]), __uint_as_float(v[8 * c + 3])),
-                pack_bf16(__uint_as_float(v[8 * c + 4]), __uint_as_float(v[8 * c + 5])),
-                pack_bf16(__uint_as_float(v[8 * c + 6]), __uint_as_float(v[8 * c + 7])));
-        }
-        fence_proxy_async();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(dkv_staged);
-      } else if (half * 32 < hs && j * ATT_BK + r < T) {
-#pragma unroll
-        for (int which = 0; which < 2; ++which) {
-          __nv_bfloat16* dst = row + (which == 0 ? d : 2 * d) + half * 32;
-#pragma unroll
-          for (int c = 0; c < 32; c += 8) {
-            const uint32_t* v = which == 0 ? vk : vv;
-            *reinterpret_cast<uint4*>(dst + c) = make_uint4(
-                pack_bf16(__uint_as_float(v[c]), __uint_as_float(v[c + 1])),
-                pack_bf16(__uint_as_float(v[c + 2]), __uint_as_float(v[c + 3])),
-                pack_bf16(__uint_as_float(v[c + 4]), __uint_as_float(v[c + 5])),
-                pack_bf16(__uint_as_float(v[c + 6]), __uint_as_float(v[c + 7])));
-          }
-        }
+        for (int c = 0; c < 4; ++c)
+          *reinterpret_cast<uint4*>(sp + which * ATT_TILE_BYTES + r * 128 + (((half * 4 + c) ^ (r & 7)) << 4)) = make_uint4(
+              pack_bf16(__uint_as_float(v[8 * c]), __uint_as_float(v[8 * c + 1])),
+              pack_bf16(__uint_as_float(v[8 * c + 2]), __uint_as_float(v[8 * c + 3])),
+              pack_bf16(__uint_as_float(v[8 * c + 4]), __uint_as_float(v[8 * c + 5])),
+              pack_bf16(__uint_as_float(v[8 * c + 6]), __uint_as_float(v[8 * c + 7])));
       }
-      if (hs == 64 && !whole) {                        // nothing staged: the reducer only passes the buffer on
-        __syncwarp();
-        if (lane == 0) mbar_arrive(dkv_staged);
-      }
+      fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(dkv_staged);
       ++w;
     }
   }
@@ -1002,14 +970,13 @@ static int att_num_sms() {
 extern "C" int dsw_attention_set_trace(long long* buf) { g_att_trace = buf; return 0; }
 
 // qkv: bf16 [B*T, 3*nh*hs]; out: bf16 [B*T, nh*hs]; lse: fp32 [B*nh*T].
-// Requires hs == 64 or 32.
+// Requires hs == 64 or 32; T is any length.
 extern "C" int dsw_attention_fwd(const void* qkv, void* out, float* lse, int B, int T, int nh, int hs, float scale,
                                  int* status, cudaStream_t st) {
   if ((hs != 64 && hs != 32) || T <= 0) return -10;
   const int d = nh * hs;
   CUtensorMap tm;
-  int rc = hs == 64 ? cached_tmap(&tm, TMAP_BF16_2D, qkv, 3LL * d, 1, (long long)B * T, 3LL * d, 64, 128)
-                    : cached_tmap(&tm, TMAP_BF16_3D, qkv, hs, 3LL * nh, (long long)B * T, 3LL * d, 64, 128);
+  const int rc = cached_tmap(&tm, TMAP_BF16_4D, qkv, hs, 3LL * nh, T, 3LL * d, 64, 128, B);
   if (rc) return rc;
   static bool attr_set = false;
   if (!attr_set) {
@@ -1034,18 +1001,10 @@ extern "C" int dsw_attention_bwd(const void* qkv, const void* out, const void* d
   const int d = nh * hs;
   const long long rows = (long long)B * T;
   CUtensorMap tq, tdo, tdq, tdkv;
-  int rc;
-  if (hs == 64) {
-    rc = cached_tmap(&tq, TMAP_BF16_2D, qkv, 3LL * d, 1, rows, 3LL * d, 64, 128);
-    if (!rc) rc = cached_tmap(&tdkv, TMAP_BF16_2D, dqkv, 3LL * d, 1, rows, 3LL * d, 64, 128);
-    if (!rc) rc = cached_tmap(&tdo, TMAP_BF16_2D, dout, d, 1, rows, d, 64, 128);
-    if (!rc) rc = cached_tmap(&tdq, TMAP_F32_2D, dq_acc, d, 1, rows, d, 32, 128);
-  } else {
-    rc = cached_tmap(&tq, TMAP_BF16_3D, qkv, hs, 3LL * nh, rows, 3LL * d, 64, 128);
-    tdkv = tq;            // not used with 32 columns per head: dK and dV are stored by the row threads
-    if (!rc) rc = cached_tmap(&tdo, TMAP_BF16_3D, dout, hs, nh, rows, d, 64, 128);
-    if (!rc) rc = cached_tmap(&tdq, TMAP_F32_3D, dq_acc, hs, nh, rows, d, 32, 128);
-  }
+  int rc = cached_tmap(&tq, TMAP_BF16_4D, qkv, hs, 3LL * nh, T, 3LL * d, 64, 128, B);
+  if (!rc) rc = cached_tmap(&tdkv, TMAP_BF16_4D, dqkv, hs, 3LL * nh, T, 3LL * d, 64, 128, B);
+  if (!rc) rc = cached_tmap(&tdo, TMAP_BF16_4D, dout, hs, nh, T, d, 64, 128, B);
+  if (!rc) rc = cached_tmap(&tdq, TMAP_F32_4D, dq_acc, hs, nh, T, d, 32, 128, B);
   if (rc) return rc;
   static bool attr_set = false;
   if (!attr_set) {
@@ -1066,7 +1025,7 @@ extern "C" int dsw_attention_bwd(const void* qkv, const void* out, const void* d
   const int total = ((T + ATT_BK - 1) / ATT_BK) * B * nh;
   const int G = total < att_num_sms() ? total : att_num_sms();
   if (launch(attention_bwd_kernel, G, ATT_BWD_THREADS, AttBwdSmem::TOTAL, st, 1, tq, tdo, tdq, tdkv, lse, Dvec,
-             (__nv_bfloat16*)dqkv, T, nh, B * nh, hs, scale, status, g_att_trace) != cudaSuccess)
+             T, nh, B * nh, hs, scale, status, g_att_trace) != cudaSuccess)
     return -3;
   return launch(attention_dq_convert_kernel, 148 * 4, 256, 0, st, 1, dq_acc, (__nv_bfloat16*)dqkv, (long long)B * T, d) ==
                  cudaSuccess

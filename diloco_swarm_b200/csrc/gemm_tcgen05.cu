@@ -49,7 +49,7 @@ static EncodeTiledFn get_encode() {
 }
 
 // 2-D bf16 tensor map: `inner` contiguous elements, `outer` rows of `ld` elements.
-int make_tmap_bf16_2d(CUtensorMap* tm, const void* ptr, long long inner, long long outer, long long ld,
+static int make_tmap_bf16_2d(CUtensorMap* tm, const void* ptr, long long inner, long long outer, long long ld,
                       int box_inner, int box_outer) {
   EncodeTiledFn enc = get_encode();
   if (!enc) return -1;
@@ -63,47 +63,33 @@ int make_tmap_bf16_2d(CUtensorMap* tm, const void* ptr, long long inner, long lo
   return r == CUDA_SUCCESS ? 0 : -(int)r - 100;
 }
 
-// 2-D fp32 tensor map, 128-byte swizzle (box_inner * 4 bytes must be 128).
-int make_tmap_f32_2d(CUtensorMap* tm, const void* ptr, long long inner, long long outer, long long ld, int box_inner,
-                     int box_outer) {
-  EncodeTiledFn enc = get_encode();
-  if (!enc) return -1;
-  cuuint64_t dims[2] = {(cuuint64_t)inner, (cuuint64_t)outer};
-  cuuint64_t strides[1] = {(cuuint64_t)ld * 4};
-  cuuint32_t box[2] = {(cuuint32_t)box_inner, (cuuint32_t)box_outer};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = enc(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(ptr), dims, strides, box, estr,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? 0 : -(int)r - 100;
-}
-
-// 3-D map over a [rows, ncol * inner] matrix seen as (inner, ncol, rows), 128-byte swizzle.  The box may be wider
-// than `inner`: the columns past it are out of bounds, so loads fill them with zeros and stores skip them.
-int make_tmap_3d(CUtensorMap* tm, int is_f32, const void* ptr, long long inner, long long ncol, long long rows,
-                 long long ld, int box_inner, int box_rows) {
+// 4-D map over a [batch, rows, ncol * inner] array seen as (inner, ncol, rows, batch), 128-byte swizzle.  The box may be
+// wider than `inner`, or reach past the last row: what lies out of bounds there is filled with zeros by loads and skipped
+// by stores and reductions, and belongs neither to the next column block nor to the next element of the batch.
+static int make_tmap_4d(CUtensorMap* tm, int is_f32, const void* ptr, long long inner, long long ncol, long long rows,
+                        long long batch, long long ld, int box_inner, int box_rows) {
   EncodeTiledFn enc = get_encode();
   if (!enc) return -1;
   const cuuint64_t es = is_f32 ? 4 : 2;
-  cuuint64_t dims[3] = {(cuuint64_t)inner, (cuuint64_t)ncol, (cuuint64_t)rows};
-  cuuint64_t strides[2] = {(cuuint64_t)inner * es, (cuuint64_t)ld * es};
-  cuuint32_t box[3] = {(cuuint32_t)box_inner, 1, (cuuint32_t)box_rows};
-  cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = enc(tm, is_f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3,
+  cuuint64_t dims[4] = {(cuuint64_t)inner, (cuuint64_t)ncol, (cuuint64_t)rows, (cuuint64_t)batch};
+  cuuint64_t strides[3] = {(cuuint64_t)inner * es, (cuuint64_t)ld * es, (cuuint64_t)(rows * ld) * es};
+  cuuint32_t box[4] = {(cuuint32_t)box_inner, 1, (cuuint32_t)box_rows, 1};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  CUresult r = enc(tm, is_f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4,
                    const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                   CU_TENSOR_MAP_SWIZZLE_128B, is_f32 ? CU_TENSOR_MAP_L2_PROMOTION_NONE : CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : -(int)r - 100;
 }
-
 
 // Encoded tensor maps of recent launches.  A training step calls the GEMMs and the attention kernels thousands of
 // times on a few dozen distinct (pointer, shape, pitch, box) combinations, because work areas and the caching
 // allocator's blocks come back microbatch after microbatch; encoding a map costs more host time than the rest of a
 // launch.  One small direct-mapped table per host thread, so no lock is taken.
 struct TmapKey {
-  const void* ptr; long long inner, ncol, outer, ld; int box_inner, box_outer, kind;
+  const void* ptr; long long inner, ncol, outer, ld, batch; int box_inner, box_outer, kind;
   bool operator==(const TmapKey& o) const {
-    return ptr == o.ptr && inner == o.inner && ncol == o.ncol && outer == o.outer && ld == o.ld &&
+    return ptr == o.ptr && inner == o.inner && ncol == o.ncol && outer == o.outer && ld == o.ld && batch == o.batch &&
            box_inner == o.box_inner && box_outer == o.box_outer && kind == o.kind;
   }
 };
@@ -111,20 +97,18 @@ struct TmapSlot { TmapKey key; CUtensorMap map; bool used; };
 constexpr int TMAP_SLOTS = 2048;
 
 int cached_tmap(CUtensorMap* tm, int kind, const void* ptr, long long inner, long long ncol, long long outer, long long ld,
-                int box_inner, int box_outer) {
+                int box_inner, int box_outer, long long batch) {
   static thread_local TmapSlot table[TMAP_SLOTS];
-  const TmapKey key{ptr, inner, ncol, outer, ld, box_inner, box_outer, kind};
+  const TmapKey key{ptr, inner, ncol, outer, ld, batch, box_inner, box_outer, kind};
   unsigned long long h = reinterpret_cast<unsigned long long>(ptr) >> 8;
   h ^= (unsigned long long)inner * 0x9E3779B97F4A7C15ull;
   h ^= ((unsigned long long)outer << 21) ^ ((unsigned long long)ld << 7) ^
-       (unsigned long long)(box_inner * 131 + box_outer + kind * 8191 + ncol * 524287);
+       (unsigned long long)(box_inner * 131 + box_outer + kind * 8191 + ncol * 524287 + batch * 131071);
   h ^= h >> 29;
   TmapSlot& s = table[h % TMAP_SLOTS];
   if (s.used && s.key == key) { *tm = s.map; return 0; }
-  int rc;
-  if (kind == TMAP_BF16_2D)     rc = make_tmap_bf16_2d(tm, ptr, inner, outer, ld, box_inner, box_outer);
-  else if (kind == TMAP_F32_2D) rc = make_tmap_f32_2d(tm, ptr, inner, outer, ld, box_inner, box_outer);
-  else                          rc = make_tmap_3d(tm, kind == TMAP_F32_3D, ptr, inner, ncol, outer, ld, box_inner, box_outer);
+  const int rc = kind == TMAP_BF16_2D ? make_tmap_bf16_2d(tm, ptr, inner, outer, ld, box_inner, box_outer)
+                                      : make_tmap_4d(tm, kind == TMAP_F32_4D, ptr, inner, ncol, outer, batch, ld, box_inner, box_outer);
   if (rc == 0) { s.key = key; s.map = *tm; s.used = true; }
   return rc;
 }
