@@ -270,7 +270,7 @@ struct Run {
   int B, T, M, deterministic;
   cudaStream_t st;               // the caller's, or the capturing one
   SideMarks* marks = &s.live;
-  unsigned long long sid = stream_id(st);
+  unsigned long long sid = NOBODY;
   bool callers = false;          // the caller captures its stream
 
   Run(Stage& stage, int B_, int T_, int det, cudaStream_t stream) : s(stage), B(B_), T(T_), M(B_ * T_), deterministic(det), st(stream) {
@@ -278,18 +278,17 @@ struct Run {
     // the side stream can be waited for (nothing else uses the areas that it is given).
     cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
     unsigned long long id = 0;
-    if (cudaStreamGetCaptureInfo(st, &status, &id) != cudaSuccess) { cudaGetLastError(); return; }
-    if (status != cudaStreamCaptureStatusActive) return;
+    if (cudaStreamGetCaptureInfo(st, &status, &id) != cudaSuccess) { cudaGetLastError(); status = cudaStreamCaptureStatusNone; }
+    if (status != cudaStreamCaptureStatusActive) {
+      if (cudaStreamGetId(st, &sid) != cudaSuccess) sid = NOBODY;      // not to be asked under a capture: it would end it
+      return;
+    }
     if (s.callers_id != id) s.callers.forget();
     s.callers_id = id;
     marks = &s.callers;
     callers = true;
   }
 
-  static unsigned long long stream_id(cudaStream_t st) {
-    unsigned long long id;
-    return cudaStreamGetId(st, &id) == cudaSuccess ? id : NOBODY;
-  }
 
   int gemm(const void* A, const void* W, bool w_t, int N, int K, void* out, int mode, const float* bias, const void* resid,
            void* aux_out, const void* aux_in, int rows) const {
