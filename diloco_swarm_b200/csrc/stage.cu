@@ -116,6 +116,8 @@ struct Stage {
   unsigned long long callers_id; // which one
   cudaStream_t cap;              // graphs are captured here
   std::vector<GraphSlot> graphs;
+  bool graphs_on;                // DSWARM_GRAPHS=0 at the stage's creation: every pass is queued launch by launch
+  int replays, failures;         // replayed runs; captures that came to nothing
   unsigned long long tick;
   std::mutex mu;                 // one pass is queued at a time: passes of one stage share its scratch
 };
@@ -378,7 +380,7 @@ struct Run {
   // work areas).
   template <class F>
   int replayed(const GraphKey& key, bool own_memory, F&& body) {
-    if (!own_memory || M > GRAPH_TOKENS || callers || !graphs_on()) return body();
+    if (!own_memory || M > GRAPH_TOKENS || callers || !s.graphs_on) return body();
     GraphSlot* slot = nullptr;
     for (GraphSlot& g : s.graphs)
       if (g.key == key) { slot = &g; break; }
@@ -397,18 +399,17 @@ struct Run {
     if (slot->failed) return body();
     if (!slot->exec) {
       TRY(capture(*slot, body));
-      if (slot->failed) return body();
+      if (slot->failed) {
+        ++s.failures;
+        return body();
+      }
     }
     TRY_CUDA(cudaGraphLaunch(slot->exec, st));
     TRY_CUDA(cudaEventRecord(slot->launched, st));
     dsw::tl_launch.pdl = false;
+    ++s.replays;
     g_launches.fetch_add(slot->launches, std::memory_order_relaxed);
     return 0;
-  }
-
-  static bool graphs_on() {
-    static const bool on = [] { const char* e = getenv("DSWARM_GRAPHS"); return !(e && e[0] == '0' && e[1] == 0); }();
-    return on;
   }
 
   static void drop(GraphSlot& g) {
@@ -480,6 +481,8 @@ extern "C" int dsw_stage_create(const long long* desc, int len, void** out) {
   if (len < HEAD || desc[0] < 0 || len != HEAD + PER_BLOCK * desc[0] || desc[1] % 8 || desc[1] > 2048 || desc[3] % 8) return -10;
   Stage* s = new (std::nothrow) Stage();
   if (!s) return -1;
+  const char* graphs = getenv("DSWARM_GRAPHS");
+  s->graphs_on = !(graphs && graphs[0] == '0' && graphs[1] == 0);
   const long long* p = desc;
   s->n = int(*p++); s->d = int(*p++); s->nh = int(*p++); s->V = int(*p++);
   s->status = reinterpret_cast<int*>(*p++);
@@ -514,6 +517,15 @@ extern "C" int dsw_stage_destroy(void* stage) {
   s->captured.destroy();
   s->callers.destroy();
   delete s;
+  return 0;
+}
+
+// Runs that this stage has replayed, and captures that failed.
+extern "C" int dsw_stage_graphs(void* stage, int* replays, int* failures) {
+  Stage& s = *static_cast<Stage*>(stage);
+  std::lock_guard<std::mutex> lock(s.mu);
+  *replays = s.replays;
+  *failures = s.failures;
   return 0;
 }
 

@@ -121,6 +121,12 @@ class StageExec:
         if len(self._idle) < most:
             self._idle.append(area)
 
+    def graphs(self) -> Tuple[int, int]:
+        """(runs replayed so far, captures that failed)"""
+        a, b = ctypes.c_int(), ctypes.c_int()
+        check(self.lib.dsw_stage_graphs(self.handle, ctypes.byref(a), ctypes.byref(b)), "dsw_stage_graphs")
+        return a.value, b.value
+
     # ------------------------------------------------------------------ passes
     def forward(self, ids, x, saved: torch.Tensor, y, logits, B: int, T: int, keep: bool, stream) -> None:
         check(self.lib.dsw_stage_forward(self.handle, ptr(ids), ptr(x), saved.data_ptr(), ptr(y), ptr(logits), B, T,

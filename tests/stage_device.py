@@ -90,6 +90,12 @@ class Device:
         cap = self.capturing(s)
         return cap["id"] if cap else 0
 
+    def do_id(self, s):
+        cap = self.capturing(s)
+        if cap:
+            cap["bad"] = True                             # not allowed under a capture
+        return ERROR if cap else 0
+
     def do_begin(self, s):
         self.next += 1
         self.captures[self.next] = {"id": self.next, "origin": s, "streams": {s}, "ops": [], "seen": {}, "last": {}, "bad": False}

@@ -68,7 +68,7 @@ cudaError_t cudaStreamGetCaptureInfo(cudaStream_t s, cudaStreamCaptureStatus* st
 }
 cudaError_t cudaStreamGetId(cudaStream_t s, unsigned long long* id) {
   *id = reinterpret_cast<unsigned long long>(s);
-  return cudaSuccess;
+  return err(tell("id" + num(s)));
 }
 cudaError_t cudaMemcpyAsync(void* to, const void* from, size_t n, cudaMemcpyKind, cudaStream_t st) {
   return err(op("copy", st, {{'r', from, (long long)n}, {'w', to, (long long)n}}));
