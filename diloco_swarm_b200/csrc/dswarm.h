@@ -176,6 +176,7 @@ int dsw_grad_allreduce_nvls(void* const* bufs, void* mc, void* const* flags, flo
 int dsw_stage_create(const long long* desc, int len, void** out);
 int dsw_stage_destroy(void* stage);
 int dsw_stage_graphs(void* stage, int* replays, int* failures);     // CUDA graph replays so far, captures that failed
+int dsw_stage_seal(void* stage);          // no further CUDA graphs are captured, those that exist stay in use
 int dsw_stage_launches();
 int dsw_stage_sizes(void* stage, int B, int T, int keep, int grad, int chunks, size_t* saved, size_t* scratch);
 int dsw_stage_forward(void* stage, const long long* ids, const void* x, void* saved, void* y, float* infer_logits,

@@ -23,7 +23,9 @@
 // token ids, targets, mask, loss, logits of forward_infer; hidden states and their gradients are copied into or out of the
 // areas (some 4 us each at GRAPH_COPY elements; larger ones are not copied and their passes not replayed), so
 // it makes no difference whether they come in the same buffers again.  A handful of graphs per stage is kept, the one
-// used longest ago goes.
+// used longest ago goes.  Capturing and instantiating may have to wait for an idle device, which never comes while a
+// pipeline receive waits there for a peer that waits for this rank: a stage with neighbours captures while it warms up
+// and is sealed then.
 // Only for passes of up to GRAPH_TOKENS tokens: longer ones keep the device busy for longer than the host needs anyway,
 // and there a replay, which ends with the side stream's work, would cost the overlap with the next pass.
 #include <cuda_bf16.h>
@@ -118,6 +120,8 @@ struct Stage {
   std::vector<GraphSlot> graphs;
   bool graphs_on;                // DSWARM_GRAPHS=0 at the stage's creation: every pass is queued launch by launch
   int replays, failures;         // replayed runs; captures that came to nothing
+  std::vector<GraphSlot> retired;      // no longer looked up; destroyed once their last replay is over
+  bool sealed;                   // no further graphs are captured
   unsigned long long tick;
   std::mutex mu;                 // one pass is queued at a time: passes of one stage share its scratch
 };
@@ -384,14 +388,9 @@ struct Run {
     GraphSlot* slot = nullptr;
     for (GraphSlot& g : s.graphs)
       if (g.key == key) { slot = &g; break; }
+    if (s.sealed && (!slot || !slot->exec)) return body();
     if (!slot) {
-      if (int(s.graphs.size()) >= GRAPH_SLOTS) {
-        size_t oldest = 0;
-        for (size_t i = 1; i < s.graphs.size(); ++i)
-          if (s.graphs[i].used < s.graphs[oldest].used) oldest = i;
-        drop(s.graphs[oldest]);
-        s.graphs.erase(s.graphs.begin() + oldest);
-      }
+      make_room();
       s.graphs.push_back(GraphSlot{key, nullptr, nullptr, false, 0, ++s.tick});
       return body();
     }
@@ -412,9 +411,35 @@ struct Run {
     return 0;
   }
 
-  static void drop(GraphSlot& g) {
-    if (!g.exec) return;
-    cudaEventSynchronize(g.launched);
+  // Runs that have been seen once go before captured ones (a series of odd sizes leaves the graphs of the training alone),
+  // then the one used longest ago.  The host does not wait for a graph that is still running.
+  void make_room() const {
+    for (size_t i = 0; i < s.retired.size();) {
+      if (idle(s.retired[i])) {
+        drop(s.retired[i]);
+        s.retired.erase(s.retired.begin() + i);
+      } else {
+        ++i;
+      }
+    }
+    if (int(s.graphs.size()) < GRAPH_SLOTS) return;
+    size_t out = 0;
+    for (size_t i = 1; i < s.graphs.size(); ++i) {
+      const GraphSlot &a = s.graphs[i], &b = s.graphs[out];
+      if (!a.exec != !b.exec ? !a.exec : a.used < b.used) out = i;
+    }
+    if (s.graphs[out].exec) s.retired.push_back(s.graphs[out]);
+    s.graphs.erase(s.graphs.begin() + out);
+  }
+  static bool idle(const GraphSlot& g) {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;       // other threads may be capturing
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    const bool over = cudaEventQuery(g.launched) == cudaSuccess;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    cudaGetLastError();
+    return over;
+  }
+  static void drop(const GraphSlot& g) {
     cudaGraphExecDestroy(g.exec);
     cudaEventDestroy(g.launched);
   }
@@ -511,7 +536,12 @@ extern "C" int dsw_stage_create(const long long* desc, int len, void** out) {
 extern "C" int dsw_stage_destroy(void* stage) {
   Stage* s = static_cast<Stage*>(stage);
   if (!s) return 0;
-  for (GraphSlot& g : s->graphs) Run::drop(g);
+  s->retired.insert(s->retired.end(), s->graphs.begin(), s->graphs.end());
+  for (const GraphSlot& g : s->retired)
+    if (g.exec) {
+      cudaEventSynchronize(g.launched);
+      Run::drop(g);
+    }
   cudaStreamDestroy(s->cap);
   s->live.destroy();
   s->captured.destroy();
@@ -526,6 +556,14 @@ extern "C" int dsw_stage_graphs(void* stage, int* replays, int* failures) {
   std::lock_guard<std::mutex> lock(s.mu);
   *replays = s.replays;
   *failures = s.failures;
+  return 0;
+}
+
+// From now on runs that have not been captured are queued launch by launch.
+extern "C" int dsw_stage_seal(void* stage) {
+  Stage& s = *static_cast<Stage*>(stage);
+  std::lock_guard<std::mutex> lock(s.mu);
+  s.sealed = true;
   return 0;
 }
 

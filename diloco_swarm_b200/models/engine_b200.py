@@ -217,25 +217,36 @@ class B200Engine:
                     out.append(b)
         return out
 
-    def warmup(self, B: int, T: int) -> None:
+    def warmup(self, B: int, T: int, in_flight: int = 1) -> None:
         """Run every code path of a step once on dummy data of the real shape, then
         put the state back.  Library kernels (attention, copies) are loaded on first
         use, and a first use that happens while a pipeline receive is spinning on the
-        device can wait forever; after this pass nothing is loaded inside a step."""
+        device can wait forever; after this pass nothing is loaded inside a step.
+        The executor's CUDA graphs are such a first use as well (a pass is captured
+        when it comes a second time in the same work areas), so a stage that has
+        neighbours goes on until the passes of up to ``in_flight`` microbatches at a
+        time are replayed, and captures nothing from then on."""
         dev, d = self.device, self.cfg.n_embd
         theta0 = self.theta.clone()
         ids = torch.zeros(B, T, dtype=torch.long, device=dev) if self.is_first else None
         hidden = torch.zeros(B, T, d, dtype=BF16, device=dev) if not self.is_first else None
         tg = torch.zeros(B, T, dtype=torch.long, device=dev)
         mask = torch.ones(B, T, dtype=torch.long, device=dev)
-        if self.is_last:
-            self.forward_backward(-1, ids, hidden, tg, mask, 1.0)
-            self.forward_loss(ids, hidden, tg, mask, 1.0)
-        else:
-            y = self.forward(-1, ids, hidden)
-            self.backward(-1, torch.zeros_like(y))
-            self.forward(-1, ids, hidden, keep=False)
-        self.forward_infer(ids, hidden)
+        seal = self.exec is not None and self.world.num_stages > 1
+        if seal and not self.is_last:
+            in_flight = min(in_flight, self.exec.keeps(self.exec.sizes(B, T, True, False, 0)[0]))
+        for _ in range(3 if seal else 1):            # queued, captured and replayed, replayed
+            if self.is_last:
+                self.forward_backward(-1, ids, hidden, tg, mask, 1.0)
+                self.forward_loss(ids, hidden, tg, mask, 1.0)
+            else:
+                y = [self.forward(-1 - k, ids, hidden) for k in range(in_flight if seal else 1)]
+                for k, t in enumerate(y):
+                    self.backward(-1 - k, torch.zeros_like(t))
+                self.forward(-1, ids, hidden, keep=False)
+            self.forward_infer(ids, hidden)
+        if seal:
+            self.exec.seal()
         self.optimizer_step(0.0, 1.0)
         torch.cuda.synchronize(dev)
         self.theta.copy_(theta0)

@@ -17,7 +17,7 @@ import torch
 from ..ops import kernels as K
 from ..ops._lib import check, cuda_lib, ptr
 
-KEEP_AREA_BYTES = 4 << 30        # finished `saved` areas of up to this size are kept two at a time, larger ones singly
+KEEP_AREA_BYTES = 8 << 30        # finished `saved` areas are kept up to this much in all, one of any size
 MAX_STREAMS = 4                  # scratch areas kept (one per calling stream)
 
 
@@ -117,8 +117,7 @@ class StageExec:
         area.free.record(self.side if self.side is not None else stream)
         area.stream = stream
         area.used_on(stream)
-        most = 2 if area.buf.numel() <= KEEP_AREA_BYTES else 1
-        if len(self._idle) < most:
+        if not self._idle or sum(a.buf.numel() for a in self._idle) + area.buf.numel() <= KEEP_AREA_BYTES:
             self._idle.append(area)
 
     def graphs(self) -> Tuple[int, int]:
@@ -126,6 +125,15 @@ class StageExec:
         a, b = ctypes.c_int(), ctypes.c_int()
         check(self.lib.dsw_stage_graphs(self.handle, ctypes.byref(a), ctypes.byref(b)), "dsw_stage_graphs")
         return a.value, b.value
+
+    @staticmethod
+    def keeps(nbytes: int) -> int:
+        """How many finished areas of a size wait for the next microbatches."""
+        return max(1, KEEP_AREA_BYTES // nbytes)
+
+    def seal(self) -> None:
+        """Passes that have no CUDA graph yet get none any more."""
+        check(self.lib.dsw_stage_seal(self.handle), "dsw_stage_seal")
 
     # ------------------------------------------------------------------ passes
     def forward(self, ids, x, saved: torch.Tensor, y, logits, B: int, T: int, keep: bool, stream) -> None:

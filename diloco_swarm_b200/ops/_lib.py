@@ -52,6 +52,7 @@ _SIGS = {
     "dsw_stage_create": [c_void_p, c_int, ctypes.POINTER(c_void_p)],
     "dsw_stage_destroy": [c_void_p],
     "dsw_stage_graphs": [c_void_p, ctypes.POINTER(c_int), ctypes.POINTER(c_int)],
+    "dsw_stage_seal": [c_void_p],
     "dsw_stage_launches": [],
     "dsw_stage_sizes": [c_void_p, c_int, c_int, c_int, c_int, c_int, ctypes.POINTER(c_size_t), ctypes.POINTER(c_size_t)],
     "dsw_stage_forward": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],

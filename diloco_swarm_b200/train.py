@@ -108,7 +108,7 @@ class Trainer:
             pool = torch.empty(int(tc.reserve_memory_gb * 2 ** 30), dtype=torch.uint8, device=self.device)
             del pool
         if hasattr(self.engine, "warmup"):
-            self.engine.warmup(self.mbs, self.seq)
+            self.engine.warmup(self.mbs, self.seq, in_flight=min(tc.max_micro_batches, self.num_micro))
         self.comm.warmup()
         self.alive: Optional[List[bool]] = None
         self._step_failed = False    # the last step was dropped by the common verdict

@@ -70,6 +70,7 @@ cudaError_t cudaStreamGetId(cudaStream_t s, unsigned long long* id) {
   *id = reinterpret_cast<unsigned long long>(s);
   return err(tell("id" + num(s)));
 }
+cudaError_t cudaThreadExchangeStreamCaptureMode(cudaStreamCaptureMode*) { return cudaSuccess; }
 cudaError_t cudaMemcpyAsync(void* to, const void* from, size_t n, cudaMemcpyKind, cudaStream_t st) {
   return err(op("copy", st, {{'r', from, (long long)n}, {'w', to, (long long)n}}));
 }

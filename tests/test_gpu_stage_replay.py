@@ -65,3 +65,35 @@ def test_a_middle_stage(monkeypatch):
     for mid in pair:
         mid.check_status()
     assert pair[0].exec.graphs() == (2 * 5, 0) and pair[1].exec.graphs() == (0, 0)
+
+
+@pytest.mark.parametrize("stage", [0, 1, 2])
+def test_a_stage_with_neighbours_captures_while_it_warms_up(stage):
+    """Behind warmup() the passes of up to four microbatches in flight are replayed at once and nothing is captured: in a
+    step the device may be held by a receive that waits for a peer."""
+    cfg = make_config(model={"n_layer": 3}, swarm={"num_stages": 3})
+    eng = _stages(cfg)[stage]
+    eng.warmup(2, 50, in_flight=4)
+    x = torch.randn(2, 50, 128, device="cuda").to(torch.bfloat16)
+    ids, tg, mask = _batch(cfg, B=2, T=50)
+
+    def step(T):
+        i, h, t, m = ids[:, :T], x[:, :T], tg[:, :T], mask[:, :T]
+        if stage == 2:
+            for k in range(4):
+                eng.forward_backward(k, None, h, t, m, 0.5)
+            return
+        for k in range(4):
+            eng.forward(k, i if stage == 0 else None, h if stage else None)
+        for k in range(4):
+            eng.backward(k, h)
+    before = eng.exec.graphs()[0]
+    step(50)
+    assert eng.exec.graphs() == (before + 4 * (4 if stage == 2 else 2), 0)
+    before = eng.exec.graphs()[0]
+    for _ in range(3):
+        step(40)                                         # a size that warmup has not seen
+    eng._join()
+    torch.cuda.synchronize()
+    eng.check_status()
+    assert eng.exec.graphs() == (before, 0)

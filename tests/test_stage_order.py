@@ -102,3 +102,44 @@ def test_a_capture_by_the_caller(device, chunks):
         rcs.append(s.train(3 * AREA, 6 * AREA, 2, 512, 1, chunks=chunks))
         device.do_record(3, 7)
     ordered(device, *rcs)
+
+
+def test_one_off_sizes_leave_the_graphs_alone(device):
+    """Forty lengths that come once, after a training pass has been captured: it is still replayed, and where captured
+    graphs do go (as many again that come twice) the host waits for none and destroys none that may be running."""
+    s = FakeStage(device.lib)
+    for _ in range(3):
+        assert s.train(2 * AREA, 5 * AREA, 2, 512, 1) == (0, 0, 0)
+    for t in range(40):
+        assert s.forward(8 * AREA, 1, 8 + t, 1, keep=0) == 0
+    replays = device.counts["replay"]
+    assert s.train(2 * AREA, 5 * AREA, 2, 512, 1) == (0, 0, 0)
+    assert device.counts["replay"] == replays + 4
+    for t in range(80):
+        assert s.forward(8 * AREA, 1, 100 + t, 1, keep=0) == 0 and s.forward(8 * AREA, 1, 100 + t, 1, keep=0) == 0
+    assert device.counts.get("sync", 0) == 0 and device.counts.get("destroy", 0) == 0
+    device.busy.clear()                                  # the device has caught up
+    assert s.forward(8 * AREA, 1, 300, 1, keep=0) == 0
+    assert device.counts["destroy"] > 40
+    device.busy.update(device.graphs)
+    assert device.lib.dsw_stage_destroy(s.h) == 0
+    assert device.graphs == {}
+
+
+def test_a_sealed_stage_captures_nothing_new(device):
+    s = FakeStage(device.lib, first=False)
+
+    def step(t):
+        device.do_wait(1, 2)                             # the area is free again
+        rcs = (s.forward(2 * AREA, 2, t, 1, x=7 * AREA), s.head(2 * AREA, 5 * AREA, 2, t, 1),
+               s.backward(2 * AREA, 5 * AREA, 2, t, 1, x=7 * AREA, dx0=8 * AREA))
+        device.do_record(2, 7)
+        return rcs
+    for _ in range(3):
+        assert step(64) == (0, 0, 0)
+    assert device.lib.dsw_stage_seal(s.h) == 0
+    captures, replays = device.counts["begin"], device.counts["replay"]
+    for t in (64, 96, 96, 96, 64):
+        assert step(t) == (0, 0, 0)
+    assert device.counts["begin"] == captures and device.counts["replay"] == replays + 8
+    ordered(device)
