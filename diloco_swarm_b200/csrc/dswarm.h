@@ -1,9 +1,10 @@
 // C ABI of libdswarm_cuda.so: every exported entry point, in one place.
 //
 // Conventions.  Every entry point takes raw device pointers and the stream to
-// launch on, returns 0 on success or a negative code, and never synchronises.
+// launch on, returns 0 on success or a negative code, and never synchronises
+// (dsw_stage_destroy waits for graphs that still run).
 // bf16 arrays are passed as void*, fp32 arrays as float*, token ids / targets /
-// masks as 64-bit integers.  Return codes: -3 a launch failed, -10 a shape the
+// masks as 64-bit integers.  Return codes: -1 no host memory, -3 a launch failed, -10 a shape the
 // kernel does not cover (sizes must be multiples of 8 elements unless noted),
 // -11 a pointer that is not 16-byte aligned, -12 an unknown tile width.
 // Kernels that can wait (mbarriers, peer flags) never spin without a limit: a

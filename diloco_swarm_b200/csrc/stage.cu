@@ -33,8 +33,8 @@
 #include <atomic>
 #include <cmath>
 #include <cstdlib>
+#include <memory>
 #include <mutex>
-#include <new>
 #include <vector>
 #include "dswarm.h"
 #include "launch.h"
@@ -94,8 +94,9 @@ struct SideMarks {
     return ok;
   }
   void destroy() {
-    cudaEventDestroy(fork);
-    for (SideMark* m : all) cudaEventDestroy(m->ev);
+    if (fork) cudaEventDestroy(fork);
+    for (SideMark* m : all)
+      if (m->ev) cudaEventDestroy(m->ev);
   }
   void forget() {
     for (SideMark* m : all) m->used = false;
@@ -124,6 +125,13 @@ struct Stage {
   bool sealed;                   // no further graphs are captured
   unsigned long long tick;
   std::mutex mu;                 // one pass is queued at a time: passes of one stage share its scratch
+
+  void destroy() {               // events and stream, as far as there are any
+    if (cap) cudaStreamDestroy(cap);
+    live.destroy();
+    captured.destroy();
+    callers.destroy();
+  }
 };
 
 // Layout of a work area: pieces are handed out 256 bytes apart.
@@ -454,8 +462,13 @@ struct Run {
     marks = &s.captured;
     marks->forget();
     dsw::tl_launch.pdl = false;
-    int rc = body();
-    if (rc == 0) rc = join();
+    int rc;
+    try {
+      rc = body();
+      if (rc == 0) rc = join();
+    } catch (...) {
+      rc = -1;
+    }
     cudaGraph_t graph = nullptr;
     const bool ended = cudaStreamEndCapture(s.cap, &graph) == cudaSuccess && graph != nullptr;
     st = on;
@@ -501,11 +514,10 @@ struct Run {
 // desc: n, d, heads, V, status, side stream, wte, wpe, dwte, dwpe, lnf_w, lnf_b, dlnf_w, dlnf_b, head_w, dhead_w,
 // count, then per block ln1_w, ln1_b, dln1_w, dln1_b, ln2_w, ln2_b, dln2_w, dln2_b and for each of qkv, out, fc,
 // proj: w (bf16), b, dw, db.  Device pointers as integers; those of a part that the stage does not have are 0.
-extern "C" int dsw_stage_create(const long long* desc, int len, void** out) {
+extern "C" int dsw_stage_create(const long long* desc, int len, void** out) try {
   constexpr int HEAD = 17, PER_BLOCK = 24;
   if (len < HEAD || desc[0] < 0 || len != HEAD + PER_BLOCK * desc[0] || desc[1] % 8 || desc[1] > 2048 || desc[3] % 8) return -10;
-  Stage* s = new (std::nothrow) Stage();
-  if (!s) return -1;
+  std::unique_ptr<Stage> s(new Stage());
   const char* graphs = getenv("DSWARM_GRAPHS");
   s->graphs_on = !(graphs && graphs[0] == '0' && graphs[1] == 0);
   const long long* p = desc;
@@ -528,25 +540,26 @@ extern "C" int dsw_stage_create(const long long* desc, int len, void** out) {
     s->blocks.push_back(b);
   }
   if (!s->live.create() || !s->captured.create() || !s->callers.create() ||
-       cudaStreamCreateWithFlags(&s->cap, cudaStreamNonBlocking) != cudaSuccess) { delete s; return -2; }
-  *out = s;
+      cudaStreamCreateWithFlags(&s->cap, cudaStreamNonBlocking) != cudaSuccess) {
+    s->destroy();
+    return -2;
+  }
+  *out = s.release();
   return 0;
+} catch (...) {      // out of host memory
+  return -1;
 }
 
 extern "C" int dsw_stage_destroy(void* stage) {
-  Stage* s = static_cast<Stage*>(stage);
+  std::unique_ptr<Stage> s(static_cast<Stage*>(stage));
   if (!s) return 0;
-  s->retired.insert(s->retired.end(), s->graphs.begin(), s->graphs.end());
-  for (const GraphSlot& g : s->retired)
-    if (g.exec) {
-      cudaEventSynchronize(g.launched);
-      Run::drop(g);
-    }
-  cudaStreamDestroy(s->cap);
-  s->live.destroy();
-  s->captured.destroy();
-  s->callers.destroy();
-  delete s;
+  for (const std::vector<GraphSlot>* list : {&s->graphs, &s->retired})
+    for (const GraphSlot& g : *list)
+      if (g.exec) {
+        cudaEventSynchronize(g.launched);
+        Run::drop(g);
+      }
+  s->destroy();
   return 0;
 }
 
@@ -572,7 +585,7 @@ extern "C" int dsw_stage_launches() { return g_launches.load(std::memory_order_r
 
 // Bytes of the two work areas of a microbatch of B sequences of T tokens.  keep: a backward will follow; grad: the
 // scratch serves a backward too; chunks: slices of the LM head (0: no logits in the scratch).
-extern "C" int dsw_stage_sizes(void* stage, int B, int T, int keep, int grad, int chunks, size_t* saved, size_t* scratch) {
+extern "C" int dsw_stage_sizes(void* stage, int B, int T, int keep, int grad, int chunks, size_t* saved, size_t* scratch) try {
   const Stage& s = *static_cast<Stage*>(stage);
   if (B <= 0 || T <= 0) return -10;
   const size_t M = size_t(B) * T;
@@ -582,12 +595,14 @@ extern "C" int dsw_stage_sizes(void* stage, int B, int T, int keep, int grad, in
   *saved = a.used;
   *scratch = c.used;
   return 0;
+} catch (...) {      // out of host memory
+  return -1;
 }
 
 // Embedding (ids) or a hidden state (x) through the stage's blocks; y (bf16 [B*T, d]) is the last block's output, by
 // default a place in `saved`.  infer_logits (fp32 [B*T, V]): also the final LayerNorm and the LM head.
 extern "C" int dsw_stage_forward(void* stage, const long long* ids, const void* x, void* saved, void* y,
-                                 float* infer_logits, int B, int T, int keep, cudaStream_t st) {
+                                 float* infer_logits, int B, int T, int keep, cudaStream_t st) try {
   Stage& s = *static_cast<Stage*>(stage);
   if (B <= 0 || T <= 0 || s.n < 1 || (s.wte ? ids == nullptr : x == nullptr)) return -10;
   std::lock_guard<std::mutex> lock(s.mu);
@@ -627,6 +642,8 @@ extern "C" int dsw_stage_forward(void* stage, const long long* ids, const void* 
     LAUNCH(dsw_gemm_bf16(v.lnf, s.d, 0, s.head_w, s.d, 0, r.M, s.V, s.d, DSW_EPI_STORE_F32, 1, infer_logits, s.V, nullptr,
                          nullptr, 0, nullptr, nullptr, 0, 0, 0, s.status, st));
   return 0;
+} catch (...) {      // out of host memory
+  return -1;
 }
 
 // Final LayerNorm, LM head and masked mean cross-entropy of what dsw_stage_forward left in `saved` (loss[0] is
@@ -634,7 +651,7 @@ extern "C" int dsw_stage_forward(void* stage, const long long* ids, const void* 
 // for dsw_stage_backward.  The logits exist one slice of rows at a time.
 extern "C" int dsw_stage_head(void* stage, void* saved, void* scratch, const long long* targets, const long long* mask,
                               float scale, float* loss, int B, int T, int keep, int grad, int chunks, int deterministic,
-                              cudaStream_t st) {
+                              cudaStream_t st) try {
   Stage& s = *static_cast<Stage*>(stage);
   if (B <= 0 || T <= 0 || !s.head_w || s.n < 1) return -10;
   std::lock_guard<std::mutex> lock(s.mu);
@@ -685,6 +702,8 @@ extern "C" int dsw_stage_head(void* stage, void* saved, void* scratch, const lon
     return 0;
   }));
   return 0;
+} catch (...) {      // out of host memory
+  return -1;
 }
 
 // Backward of the blocks hi-1 .. lo.  dy: gradient of block hi-1's output, or null for the one that dsw_stage_head or
@@ -693,7 +712,7 @@ extern "C" int dsw_stage_head(void* stage, void* saved, void* scratch, const lon
 // followed by the embedding's gradient.
 extern "C" int dsw_stage_backward(void* stage, int hi, int lo, const void* dy, const void* x, const long long* ids,
                                   void* saved, void* scratch, void* dx0, int B, int T, int chunks, int deterministic,
-                                  cudaStream_t st) {
+                                  cudaStream_t st) try {
   Stage& s = *static_cast<Stage*>(stage);
   if (B <= 0 || T <= 0 || hi > s.n || lo < 0) return -10;
   std::lock_guard<std::mutex> lock(s.mu);
@@ -728,4 +747,6 @@ extern "C" int dsw_stage_backward(void* stage, int hi, int lo, const void* dy, c
   if (hi > lo && lo == 0 && dx0 && copies) TRY(r.copy(dx0, first));
   if (lo == 0 && ids) LAUNCH(dsw_embedding_bwd(ids, g, s.dwte, s.dwpe, B, T, s.d, s.V, st));
   return 0;
+} catch (...) {      // out of host memory
+  return -1;
 }

@@ -5,8 +5,9 @@
 //   replay <graph> <stream> | sync <event> | query <event> | destroy <graph> | status <stream> | id <stream>
 // Gradients that kernels add to (commutative, any order) are left out; nothing is ever dereferenced.
 #include <cuda_runtime.h>
-#include <cstdio>
+#include <cstdlib>
 #include <initializer_list>
+#include <new>
 #include <string>
 #include "dswarm.h"
 #include "launch.h"
@@ -17,6 +18,19 @@ thread_local LaunchMode tl_launch;
 
 static long long (*g_hook)(const char*) = nullptr;
 static long long g_handles = 1000;
+// Allocation number n from now on fails (-1: none does).
+static long long g_failing = -1;
+extern "C" void fake_fail_allocation(long long n) { g_failing = n; }
+static void* allocate(size_t n) {
+  if (g_failing >= 0 && g_failing-- == 0) throw std::bad_alloc();
+  return malloc(n ? n : 1);
+}
+void* operator new(size_t n) { return allocate(n); }
+void* operator new[](size_t n) { return allocate(n); }
+void operator delete(void* p) noexcept { free(p); }
+void operator delete[](void* p) noexcept { free(p); }
+void operator delete(void* p, size_t) noexcept { free(p); }
+void operator delete[](void* p, size_t) noexcept { free(p); }
 extern "C" void fake_set_hook(long long (*hook)(const char*)) { g_hook = hook; }
 
 static long long tell(const std::string& line) { return g_hook(line.c_str()); }

@@ -1,6 +1,9 @@
 """Order of the stage executor's work on its streams: every two accesses of a work area that meet are ordered, launch by
 launch and replayed, on one calling stream and on two (stage_device.py)."""
 import ctypes
+import os
+import subprocess
+import sys
 
 import pytest
 
@@ -143,3 +146,39 @@ def test_a_sealed_stage_captures_nothing_new(device):
         assert step(t) == (0, 0, 0)
     assert device.counts["begin"] == captures and device.counts["replay"] == replays + 8
     ordered(device)
+
+
+OUT_OF_MEMORY = """
+import ctypes, sys
+sys.path.insert(0, {here!r})
+from stage_device import Device, FakeStage
+lib = ctypes.CDLL({path!r})
+lib.fake_fail_allocation.argtypes = [ctypes.c_longlong]
+dev = Device(lib)
+A = 1 << 32
+failed = 0
+for n in range(40):
+    s = FakeStage(lib)
+    for call in (lambda: s.sizes(2, 64, 1, 1, 1), lambda: s.forward(2 * A, 2, 64, 1), lambda: s.head(2 * A, 5 * A, 2, 64, 1),
+                 lambda: s.backward(2 * A, 5 * A, 2, 64, 1)):
+        lib.fake_fail_allocation(n)
+        try:
+            rc = call()
+        except AssertionError:
+            rc = -1
+        lib.fake_fail_allocation(-1)
+        failed += rc == -1
+        assert rc in (0, -1) or isinstance(rc, tuple), rc
+    assert lib.dsw_stage_destroy(s.h) == 0
+assert failed > 20, failed
+"""
+
+
+def test_no_exception_leaves_a_c_entry(tmp_path):
+    """Where the host has no memory left a call returns -1.  In a process of its own: an exception ends it."""
+    path = build(tmp_path)
+    if path is None:
+        pytest.skip("needs g++ and CUDA's headers")
+    code = OUT_OF_MEMORY.format(here=os.path.dirname(os.path.abspath(__file__)), path=path)
+    done = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True)
+    assert done.returncode == 0, done.stderr[-2000:]
