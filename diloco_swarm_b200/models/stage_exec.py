@@ -105,7 +105,8 @@ class StageExec:
                     stream.wait_stream(a.stream)
                 a.used_on(stream)
                 return a
-        self._idle.clear()                        # another microbatch size: the old areas go back to the allocator
+        while self._idle and self._idle_bytes() + nbytes > KEEP_AREA_BYTES:
+            self._idle.pop(0)                     # areas of another size go back to the allocator
         return SavedArea(self._alloc(nbytes), stream)
 
     def give(self, area: SavedArea, stream: torch.cuda.Stream) -> None:
@@ -117,8 +118,11 @@ class StageExec:
         area.free.record(self.side if self.side is not None else stream)
         area.stream = stream
         area.used_on(stream)
-        if not self._idle or sum(a.buf.numel() for a in self._idle) + area.buf.numel() <= KEEP_AREA_BYTES:
+        if not self._idle or self._idle_bytes() + area.buf.numel() <= KEEP_AREA_BYTES:
             self._idle.append(area)
+
+    def _idle_bytes(self) -> int:
+        return sum(a.buf.numel() for a in self._idle)
 
     def graphs(self) -> Tuple[int, int]:
         """(runs replayed so far, captures that failed)"""

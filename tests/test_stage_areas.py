@@ -2,7 +2,7 @@
 import pytest
 import torch
 
-from diloco_swarm_b200.models.stage_exec import SavedArea, StageExec
+from diloco_swarm_b200.models.stage_exec import KEEP_AREA_BYTES, SavedArea, StageExec
 
 
 class Stream:
@@ -45,13 +45,14 @@ def test_an_area_is_recorded_on_every_stream_but_its_own(executor):
     """Taken by a pass on another stream than the one it was allocated on, an area is dropped when a pass of another
     size comes: the allocator must not hand it out again on the first stream before the second is done with it."""
     a, b = Stream(), Stream()
-    area = executor.take(100, a)
+    size = KEEP_AREA_BYTES - 100
+    area = executor.take(size, a)
     executor.give(area, a)
-    assert executor.take(100, a) is area and area.buf.recorded == []
+    assert executor.take(size, a) is area and area.buf.recorded == []
     executor.give(area, a)
-    assert executor.take(100, b) is area and a in b.waited and b in area.buf.recorded
+    assert executor.take(size, b) is area and a in b.waited and b in area.buf.recorded
     executor.give(area, b)
-    other = executor.take(200, a)                      # another size: the area is dropped, b still runs
+    other = executor.take(200, a)                      # another size, no room for both: the area is dropped, b still runs
     assert other is not area and executor._idle == [] and set(area.buf.recorded) == {b}
 
 
@@ -74,3 +75,18 @@ def test_a_capture_has_areas_of_its_own(executor, monkeypatch):
     assert mine is not area and executor.area("scratch", 100, a) is not scratch and a.waited == []
     executor.give(mine, a)
     assert executor._idle == [area] and list(executor._scratch.values()) == [scratch] and mine.free is None
+
+
+def test_sizes_that_alternate_keep_their_areas(executor):
+    """As many as fit: the areas of one microbatch size are not given back because another one comes."""
+    a = Stream()
+    first = {}
+    for n in (100, 200, 100, 200):
+        area = executor.take(n, a)
+        assert area is first.setdefault(n, area)
+        executor.give(area, a)
+    large = executor.take(KEEP_AREA_BYTES, a)            # larger than all that may lie idle: the others go
+    executor.give(large, a)
+    assert executor._idle == [large]
+    executor.give(executor.take(100, a), a)              # and it goes when another size comes
+    assert [x.buf.numel() for x in executor._idle] == [100]
