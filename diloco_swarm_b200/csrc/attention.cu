@@ -459,7 +459,7 @@ struct AttBwdSmem {
 // D[bh, t] = sum_c dO[t, h*hs + c] * O[t, h*hs + c], and dq_acc[t, :] = 0.  One warp per token row: 16-byte
 // loads, one head's hs columns lie in hs/8 neighbouring lanes (hs = 64 or 32), which a few shuffles add up.
 __global__ void __launch_bounds__(256)
-attention_bwd_prep_kernel(const __nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ dout,
+attention_bwd_prep_kernel(const __nv_bfloat16* out, const __nv_bfloat16* dout,
                           float* __restrict__ D, float* __restrict__ dq_acc, int B, int T, int nh, int hs) {
   const int lane = threadIdx.x & 31;
   const int d = nh * hs, chunks = d >> 3, lanes_per_head = hs >> 3;
@@ -494,7 +494,7 @@ attention_bwd_prep_kernel(const __nv_bfloat16* __restrict__ out, const __nv_bflo
 
 // dqkv[:, 0:d] = bf16(dq_acc)
 __global__ void __launch_bounds__(256)
-attention_dq_convert_kernel(const float* __restrict__ dq_acc, __nv_bfloat16* __restrict__ dqkv, long long rows, int d) {
+attention_dq_convert_kernel(const float* dq_acc, __nv_bfloat16* __restrict__ dqkv, long long rows, int d) {
   pdl_wait();
   pdl_launch();
   const int per_row = d / 8;
@@ -539,7 +539,7 @@ constexpr int ATT_BWD_THREADS = 32 * (ATT_BWD_ROW_WARPS + 3);    // + MMA issuer
 __global__ void __launch_bounds__(ATT_BWD_THREADS, 1)
 attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_constant__ CUtensorMap tmap_do,
                      const __grid_constant__ CUtensorMap tmap_dq, const __grid_constant__ CUtensorMap tmap_dkv,
-                     const float* __restrict__ lse, const float* __restrict__ Dvec, int T, int nh, int n_bh, int hs,
+                     const float* lse, const float* Dvec, int T, int nh, int n_bh, int hs,
                      float scale, int* status, long long* trace) {
   using L = AttBwdSmem;
   extern __shared__ uint8_t smem_raw[];

@@ -67,7 +67,7 @@ __device__ __forceinline__ void unpack8(const uint4& u, float (&f)[8]) {
 }
 
 template <int NCH>
-__device__ __forceinline__ void ln_load_row(uint4 (&o)[NCH], const __nv_bfloat16* __restrict__ x, int row, int d, int lane,
+__device__ __forceinline__ void ln_load_row(uint4 (&o)[NCH], const __nv_bfloat16* x, int row, int d, int lane,
                                             int M) {
   const __nv_bfloat16* xr = x + (long long)row * d;
 #pragma unroll
@@ -83,7 +83,7 @@ __device__ __forceinline__ void ln_load_row(uint4 (&o)[NCH], const __nv_bfloat16
 // half of the lanes had nothing to load, and a warp's chain of rows (load, two reductions, store) set the time.
 template <int NCH, bool LO, int LPR>
 __global__ void __launch_bounds__(256)
-layernorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ x_lo, const float* __restrict__ gamma,
+layernorm_fwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* x_lo, const float* __restrict__ gamma,
                      const float* __restrict__ beta, __nv_bfloat16* __restrict__ y, float* __restrict__ mean_out,
                      float* __restrict__ rstd_out, int M, int d, float eps) {
   static_assert(LPR == 32 || NCH == 1, "rows that share a warp are one chunk long");
@@ -181,9 +181,8 @@ struct LnBwdRow {
 };
 
 template <int NCH>
-__device__ __forceinline__ void ln_bwd_load(LnBwdRow<NCH>& o, const __nv_bfloat16* __restrict__ dy,
-                                            const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dres,
-                                            const float* __restrict__ mean_in, const float* __restrict__ rstd_in,
+__device__ __forceinline__ void ln_bwd_load(LnBwdRow<NCH>& o, const __nv_bfloat16* dy, const __nv_bfloat16* x,
+                                            const __nv_bfloat16* dres, const float* mean_in, const float* rstd_in,
                                             int row, int M, int d, int nch, int lane) {
   const long long off = (long long)row * d;
 #pragma unroll
@@ -206,9 +205,8 @@ constexpr int ln_bwd_blocks_per_sm(int nch) { return nch == 2 || nch == 3 ? 1 : 
 
 template <int LN_MAX_CHUNKS, int LPR>          // LPR: lanes per row, as in the forward
 __global__ void __launch_bounds__(32 * LN_BWD_WARPS, ln_bwd_blocks_per_sm(LN_MAX_CHUNKS))
-layernorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
-                     const float* __restrict__ gamma, const float* __restrict__ mean_in,
-                     const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ dres,
+layernorm_bwd_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* x, const float* __restrict__ gamma, const float* mean_in,
+                     const float* rstd_in, const __nv_bfloat16* dres,
                      __nv_bfloat16* __restrict__ dx, float* __restrict__ partial, int M, int d) {
   extern __shared__ float sh[];                 // [LN_BWD_WARPS][3][d]
   static_assert(LPR == 32 || LN_MAX_CHUNKS == 1, "rows that share a warp are one chunk long");
@@ -363,7 +361,7 @@ layernorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
 // dres_sum[c] += sum_b partial[b][2][c] (when requested).  Block = 32 columns x 32 slices of the
 // partial blocks, so the few hundred partials per column are summed by 32 threads, not one.
 __global__ void __launch_bounds__(1024)
-layernorm_bwd_finish_kernel(const float* __restrict__ partial, int nblocks, int d, float* __restrict__ dgamma,
+layernorm_bwd_finish_kernel(const float* partial, int nblocks, int d, float* __restrict__ dgamma,
                             float* __restrict__ dbeta, float* __restrict__ dres_sum) {
   __shared__ float sh[32][33];
   pdl_wait();
@@ -387,7 +385,7 @@ layernorm_bwd_finish_kernel(const float* __restrict__ partial, int nblocks, int 
 // ------------------------------------------------------------------ column sum (bias gradients)
 // out[n] += sum_m x[m, n].  Block = 32 column groups of 8 x 8 row lanes.
 __global__ void __launch_bounds__(256)
-colsum_kernel(const __nv_bfloat16* __restrict__ x, long long ld, float* __restrict__ out, int M, int N) {
+colsum_kernel(const __nv_bfloat16* x, long long ld, float* __restrict__ out, int M, int N) {
   __shared__ float sh[8][256];
   pdl_wait();
   pdl_launch();
@@ -454,7 +452,7 @@ embedding_fwd_kernel(const long long* __restrict__ ids, const float* __restrict_
 }
 // dwte[ids[r], :] += dx[r, :] (fp32 atomics); dwpe[t, :] += sum_b dx[b, t, :].
 __global__ void __launch_bounds__(256)
-embedding_bwd_kernel(const long long* __restrict__ ids, const __nv_bfloat16* __restrict__ dx,
+embedding_bwd_kernel(const long long* __restrict__ ids, const __nv_bfloat16* dx,
                      float* __restrict__ dwte, float* __restrict__ dwpe, int B, int T, int d, int V) {
   pdl_wait();
   pdl_launch();
@@ -580,7 +578,7 @@ loss_begin_kernel(const long long* __restrict__ mask, int M, float* __restrict__
 // (zeros for masked rows).  Two passes over the row; the second hits L2.
 __global__ void __launch_bounds__(512)
 cross_entropy_kernel(__nv_bfloat16* __restrict__ logits, long long ld, const long long* __restrict__ targets,
-                     const long long* __restrict__ mask, const float* __restrict__ count, float scale,
+                     const long long* __restrict__ mask, const float* count, float scale,
                      float* __restrict__ loss_acc, int M, int V, int write_grad, int* status) {
   __shared__ float shm[16], shs[16];
   pdl_wait();
@@ -673,8 +671,8 @@ cross_entropy_kernel(__nv_bfloat16* __restrict__ logits, long long ld, const lon
 // out the groups), adds the kept rows' losses and leaves {lse2, scale / count or 0, target} per row when there is a
 // gradient to follow.  32768 rows of 786 groups are 103 MB: about 25 us, against 3.3 GB for the logits themselves.
 __global__ void __launch_bounds__(1024)
-head_rows_kernel(const float* __restrict__ parts, const float* __restrict__ tlogit, const long long* __restrict__ targets,
-                 const long long* __restrict__ mask, const float* __restrict__ count, float scale,
+head_rows_kernel(const float* parts, const float* tlogit, const long long* __restrict__ targets,
+                 const long long* __restrict__ mask, const float* count, float scale,
                  float* __restrict__ loss_acc, float4* __restrict__ rows, int M, int V, int groups, int* status) {
   __shared__ float shm[32][33], shs[32][33];
   pdl_wait();
@@ -724,7 +722,7 @@ head_rows_kernel(const float* __restrict__ parts, const float* __restrict__ tlog
 }
 
 // ------------------------------------------------------------------ casts
-__global__ void cast_f32_bf16_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, long long n) {
+__global__ void cast_f32_bf16_kernel(const float* src, __nv_bfloat16* __restrict__ dst, long long n) {
   pdl_wait();
   pdl_launch();
   const long long n8 = n / 8;
@@ -738,7 +736,7 @@ __global__ void cast_f32_bf16_kernel(const float* __restrict__ src, __nv_bfloat1
 }
 // 4 * splits + 2 bytes per element; at 2128 x 768 and 8 splits (56 MB, out of L2 where the partials just were) 13 us.
 __global__ void __launch_bounds__(256)
-sum_partials_kernel(const float* __restrict__ partials, int splits, __nv_bfloat16* __restrict__ out, long long n) {
+sum_partials_kernel(const float* partials, int splits, __nv_bfloat16* __restrict__ out, long long n) {
   pdl_wait();
   pdl_launch();
   for (long long i = (blockIdx.x * (long long)blockDim.x + threadIdx.x) * 8; i < n; i += (long long)gridDim.x * blockDim.x * 8) {

@@ -239,7 +239,7 @@ __device__ __forceinline__ void epilogue_warp(const GemmArgs& g, uint32_t t_addr
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const int row = row_base + i * 8 + my_r;
-          x[i] = (row < g.M && col < g.N) ? __ldg(reinterpret_cast<const uint4*>(src + (long long)row * ld + col))
+          x[i] = (row < g.M && col < g.N) ? *reinterpret_cast<const uint4*>(src + (long long)row * ld + col)
                                           : make_uint4(0, 0, 0, 0);
         }
       }

@@ -7,6 +7,10 @@
 // pdl_wait() before its first access to activations, so completion is transitive.  No kernel calls pdl_launch() before
 // its own pdl_wait(), so when a kernel starts, everything before its predecessor has completed: what was written two
 // launches back (weights, by an optimiser step of an earlier pass) may be read before pdl_wait().
+//
+// What a predecessor writes is read through plain pointers: const __restrict__ and __ldg allow non-coherent loads, which
+// are only defined for memory that nothing writes while the kernel lives, and here its life begins under the
+// predecessor's.  They are for what is older than the pass: weights, biases, token ids, targets, masks.
 #pragma once
 #include <cuda_runtime.h>
 
