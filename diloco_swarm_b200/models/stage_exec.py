@@ -48,7 +48,7 @@ class StageExec:
         h = ctypes.c_void_p()
         with torch.cuda.device(device):
             check(lib.dsw_stage_create((ctypes.c_longlong * len(desc))(*desc), len(desc), ctypes.byref(h)),
-                  "dsw_stage_create")
+                  "dsw_stage_create", 0)
         self.handle, self.lib, self.side, self.device, self.d = h.value, lib, side, device, d
         self._keep = (status, ends, blocks)
         weakref.finalize(self, lib.dsw_stage_destroy, self.handle)
@@ -66,7 +66,7 @@ class StageExec:
         if got is None:
             a, b = ctypes.c_size_t(), ctypes.c_size_t()
             check(self.lib.dsw_stage_sizes(self.handle, B, T, int(keep), int(grad), chunks, ctypes.byref(a),
-                                           ctypes.byref(b)), "dsw_stage_sizes")
+                                           ctypes.byref(b)), "dsw_stage_sizes", 0)
             if len(self._sizes) > 1024:
                 self._sizes.clear()
             got = self._sizes[key] = (a.value, b.value)
@@ -127,7 +127,7 @@ class StageExec:
     def graphs(self) -> Tuple[int, int]:
         """(runs replayed so far, captures that failed)"""
         a, b = ctypes.c_int(), ctypes.c_int()
-        check(self.lib.dsw_stage_graphs(self.handle, ctypes.byref(a), ctypes.byref(b)), "dsw_stage_graphs")
+        check(self.lib.dsw_stage_graphs(self.handle, ctypes.byref(a), ctypes.byref(b)), "dsw_stage_graphs", 0)
         return a.value, b.value
 
     @staticmethod
@@ -137,21 +137,21 @@ class StageExec:
 
     def seal(self) -> None:
         """Passes that have no CUDA graph yet get none any more."""
-        check(self.lib.dsw_stage_seal(self.handle), "dsw_stage_seal")
+        check(self.lib.dsw_stage_seal(self.handle), "dsw_stage_seal", 0)
 
     # ------------------------------------------------------------------ passes
     def forward(self, ids, x, saved: torch.Tensor, y, logits, B: int, T: int, keep: bool, stream) -> None:
         check(self.lib.dsw_stage_forward(self.handle, ptr(ids), ptr(x), saved.data_ptr(), ptr(y), ptr(logits), B, T,
-                                         int(keep), stream.cuda_stream), "dsw_stage_forward")
+                                         int(keep), stream.cuda_stream), "dsw_stage_forward", 0)
 
     def head(self, saved: torch.Tensor, scratch: torch.Tensor, targets, mask, scale: float, loss, B: int, T: int,
              keep: bool, grad: bool, chunks: int, stream) -> None:
         check(self.lib.dsw_stage_head(self.handle, saved.data_ptr(), scratch.data_ptr(), targets.data_ptr(), ptr(mask),
                                       scale, loss.data_ptr(), B, T, int(keep), int(grad), chunks,
-                                      int(K.deterministic()), stream.cuda_stream), "dsw_stage_head")
+                                      int(K.deterministic()), stream.cuda_stream), "dsw_stage_head", 0)
 
     def backward(self, hi: int, lo: int, dy, x, ids, saved: torch.Tensor, scratch: torch.Tensor, dx0, B: int, T: int,
                  chunks: int, stream) -> None:
         check(self.lib.dsw_stage_backward(self.handle, hi, lo, ptr(dy), ptr(x), ptr(ids), saved.data_ptr(),
                                           scratch.data_ptr(), ptr(dx0), B, T, chunks, int(K.deterministic()),
-                                          stream.cuda_stream), "dsw_stage_backward")
+                                          stream.cuda_stream), "dsw_stage_backward", 0)

@@ -135,11 +135,12 @@ def ptr(t: Optional[torch.Tensor]) -> Optional[int]:
 LAUNCHES = 0   # launcher calls so far (each launches at least one kernel of this library)
 
 
-def check(rc: int, what: str) -> None:
+def check(rc: int, what: str, launches: int = 1) -> None:
+    """``launches``: 0 for a call that launches nothing, or whose launches the library counts itself."""
     global LAUNCHES
     if rc != 0:
         raise RuntimeError(f"{what} failed with code {rc}")
-    LAUNCHES += 1
+    LAUNCHES += launches
 
 
 def launch_count() -> int:

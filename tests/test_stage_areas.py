@@ -90,3 +90,24 @@ def test_sizes_that_alternate_keep_their_areas(executor):
     assert executor._idle == [large]
     executor.give(executor.take(100, a), a)              # and it goes when another size comes
     assert [x.buf.numel() for x in executor._idle] == [100]
+
+
+def test_a_pass_is_not_counted_on_top_of_its_launches(executor, monkeypatch):
+    """The executor counts the kernels that it launches; the calls that queue them are no launches themselves."""
+    from diloco_swarm_b200.models import stage_exec
+    from diloco_swarm_b200.ops import _lib
+    monkeypatch.setattr(stage_exec, "ptr", lambda t: None)
+    executor.handle, executor.d, executor._sizes = 1, 64, {}
+
+    class Library:
+        def __getattr__(self, name):
+            return lambda *a: 0
+    executor.lib = Library()
+    stream, t = Stream(), torch.zeros(1, dtype=torch.long)
+    stream.cuda_stream = 1
+    before = _lib.LAUNCHES
+    executor.sizes(2, 3, True, True, 1)
+    executor.forward(t, None, t, None, None, 2, 3, True, stream)
+    executor.head(t, t, t, None, 1.0, t, 2, 3, True, True, 1, stream)
+    executor.backward(1, 0, None, None, t, t, t, None, 2, 3, 1, stream)
+    assert _lib.LAUNCHES == before
