@@ -40,6 +40,7 @@ enum EpiMode : int {
   // LM head without stored logits (dsw_head_lse / dsw_head_dlogits); acc = the logits of row and column
   EPI_LSE = 6,          // parts[column / 64][row] = log2 of the sum of 2^(acc log2 e) over 64 columns; tlogit[row] = acc at the target
   EPI_DLOGITS = 7,      // out = coef (softmax(acc) - onehot), lse2, target and coef from rows[row]
+  EPI_RESID_LO = 8,     // EPI_RESID with aux_in or aux_out, on the kernels for many rows
 };
 
 // What the second pass over the logits needs to know of a row: {log2-sum-exp2, factor (0: the row is masked), target as
@@ -220,6 +221,81 @@ __device__ __forceinline__ void epilogue_warp(const GemmArgs& g, uint32_t t_addr
         }
       });
     }
+  } else if constexpr (MODE == EPI_RESID_LO) {
+    // Residual stream of two bf16 arrays.  The accumulator passes the staging tile as fp32, 16 rows at a time, so that the
+    // sum is rounded once, at its end, and its remainder once more: staged as bf16 like the plain residual's it lost the
+    // bits that the low half is there to keep (sampling 8 x 777 tokens of GPT-2 small: error of the logits 4.4e-3 ->
+    // 3.6e-3; 16384 x 768 from 3072 72.2 -> 73.2 us, 6216 x 768 from 768 some 1 us more).  Loads and stores cover 8 rows
+    // of 64 bytes, as below; 16-column slices, whose 16 rows of 32 bytes cost the load/store unit twice the lines, took
+    // 76.  The low half is asked for when its rows are staged: sooner, its registers spilled.
+    constexpr int NCH = NCOLS / 32;
+    const int my_ch = lane & 3, my_r = lane >> 2;
+    uint32_t r[32];
+    tmem_ld_32x32(t_addr, r);
+#pragma unroll
+    for (int c = 0; c < NCH; ++c) {
+      const int cb = col_base + c * 32, col = cb + my_ch * 8;
+      uint4 x[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int row = row_base + i * 8 + my_r;
+        const bool in = row < g.M && col < g.N;
+        x[i] = in ? *reinterpret_cast<const uint4*>(g.resid + (long long)row * g.ldr + col) : make_uint4(0, 0, 0, 0);
+      }
+      tmem_ld_wait();
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {          // rows half * 16 .. + 15 as [16][128 bytes], chunks of 16 swizzled by row
+        uint4 t[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const int row = row_base + half * 16 + j * 8 + my_r;
+          t[j] = row < g.M && col < g.N && g.aux_in != nullptr ? *reinterpret_cast<const uint4*>(g.aux_in + (long long)row * g.ldaux + col)
+                                                               : make_uint4(0, 0, 0, 0);
+        }
+        __syncwarp();                                 // the rows before have been read out
+        if ((lane >> 4) == half) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const float4 bb = (g.bias != nullptr && cb + 4 * i < g.N) ? __ldg(reinterpret_cast<const float4*>(g.bias + cb) + i)
+                                                                     : make_float4(0.f, 0.f, 0.f, 0.f);
+            *reinterpret_cast<float4*>(stage + (lane & 15) * 128 + ((i ^ (lane & 7)) << 4)) =
+                make_float4(__uint_as_float(r[4 * i]) + bb.x, __uint_as_float(r[4 * i + 1]) + bb.y,
+                            __uint_as_float(r[4 * i + 2]) + bb.z, __uint_as_float(r[4 * i + 3]) + bb.w);
+          }
+        }
+        __syncwarp();
+        if (half == 1) {
+          if (c + 1 < NCH) tmem_ld_32x32(t_addr + (c + 1) * 32, r);
+          else release();
+        }
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const int i = half * 2 + j, rl = j * 8 + my_r, row = row_base + half * 16 + rl;
+          float a[8];
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const float4 f = *reinterpret_cast<const float4*>(stage + rl * 128 + (((my_ch * 2 + h) ^ (rl & 7)) << 4));
+            a[4 * h] = f.x; a[4 * h + 1] = f.y; a[4 * h + 2] = f.z; a[4 * h + 3] = f.w;
+          }
+          if (row >= g.M || col >= g.N) continue;
+          if (!DSW_OK(col + 8 <= g.N && col + 8 <= g.ldo && rl >= 0 && rl < 16)) continue;
+          const uint32_t xu[4] = {x[i].x, x[i].y, x[i].z, x[i].w}, tu[4] = {t[j].x, t[j].y, t[j].z, t[j].w};
+          uint32_t hi[4], lo[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const float2 e = unpack_bf16(xu[q]), f = unpack_bf16(tu[q]);
+            const float s0 = a[2 * q] + (e.x + f.x), s1 = a[2 * q + 1] + (e.y + f.y);
+            hi[q] = pack_bf16(s0, s1);
+            const float2 h = unpack_bf16(hi[q]);
+            lo[q] = pack_bf16(s0 - h.x, s1 - h.y);
+          }
+          *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(g.out) + (long long)row * g.ldo + col) =
+              make_uint4(hi[0], hi[1], hi[2], hi[3]);
+          if (g.aux_out != nullptr)
+            *reinterpret_cast<uint4*>(g.aux_out + (long long)row * g.ldaux + col) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        }
+      }
+    }
   } else {
     constexpr int NCH = NCOLS / 32;
     constexpr bool EXTRA = MODE == EPI_RESID || MODE == EPI_MUL;
@@ -312,25 +388,9 @@ __device__ __forceinline__ void epilogue_warp(const GemmArgs& g, uint32_t t_addr
           if constexpr (MODE == EPI_MUL) {
 #pragma unroll
             for (int q = 0; q < 4; ++q) du[q] = mul_bf16x2(du[q], xu[q]);
-          } else if (g.aux_in == nullptr && g.aux_out == nullptr) {
+          } else {
 #pragma unroll
             for (int q = 0; q < 4; ++q) du[q] = add_bf16x2(du[q], xu[q]);
-          } else {          // with the residual stream's low halves
-            uint32_t lo[4] = {0, 0, 0, 0};
-            if (g.aux_in != nullptr) {
-              const uint4 t = *reinterpret_cast<const uint4*>(g.aux_in + (long long)row * g.ldaux + col);
-              lo[0] = t.x; lo[1] = t.y; lo[2] = t.z; lo[3] = t.w;
-            }
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              const float2 a = unpack_bf16(du[q]), e = unpack_bf16(xu[q]), t = unpack_bf16(lo[q]);
-              const float s0 = a.x + (e.x + t.x), s1 = a.y + (e.y + t.y);
-              du[q] = pack_bf16(s0, s1);
-              const float2 h = unpack_bf16(du[q]);
-              lo[q] = pack_bf16(s0 - h.x, s1 - h.y);
-            }
-            if (g.aux_out != nullptr)
-              *reinterpret_cast<uint4*>(g.aux_out + (long long)row * g.ldaux + col) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
           }
           d = make_uint4(du[0], du[1], du[2], du[3]);
         }
@@ -356,9 +416,9 @@ __device__ __forceinline__ void epilogue_warp(const GemmArgs& g, uint32_t t_addr
 // Same lane-to-address map as the loads in epilogue_warp; one request per 32-byte sector.
 template <int MODE, int NCOLS>
 __device__ __forceinline__ void prefetch_extra(const GemmArgs& g, int row_base, int lane, int col_base) {
-  if constexpr (MODE == EPI_RESID || MODE == EPI_MUL) {
-    const __nv_bfloat16* src = MODE == EPI_RESID ? g.resid : g.aux_in;
-    const long long ld = MODE == EPI_RESID ? g.ldr : g.ldaux;
+  if constexpr (MODE == EPI_RESID || MODE == EPI_RESID_LO || MODE == EPI_MUL) {
+    const __nv_bfloat16* src = MODE == EPI_MUL ? g.aux_in : g.resid;
+    const long long ld = MODE == EPI_MUL ? g.ldaux : g.ldr;
     if (lane & 1) return;
 #pragma unroll
     for (int c = 0; c < NCOLS / 32; ++c) {
@@ -366,8 +426,11 @@ __device__ __forceinline__ void prefetch_extra(const GemmArgs& g, int row_base, 
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int row = row_base + i * 8 + (lane >> 2);
-        if (row < g.M && col < g.N)
+        if (row < g.M && col < g.N) {
           asm volatile("prefetch.global.L2 [%0];" ::"l"(src + (long long)row * ld + col));
+          if (MODE == EPI_RESID_LO && g.aux_in != nullptr)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(g.aux_in + (long long)row * g.ldaux + col));
+        }
       }
     }
   }
@@ -823,7 +886,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 
 
 // Epilogue classes the kernels are instantiated for; both fp32 outputs share one.
-__host__ __device__ constexpr int epi_class(int mode) { return mode == EPI_STORE_F32 ? EPI_ATOMIC_F32 : mode; }
+inline int epi_class(const GemmArgs& g) {
+  if (g.mode == EPI_STORE_F32) return EPI_ATOMIC_F32;
+  return g.mode == EPI_RESID && (g.aux_in != nullptr || g.aux_out != nullptr) ? EPI_RESID_LO : g.mode;
+}
 
 // Defined in gemm_one_cta.cu / gemm_pair.cu.  bn = 128 or 256 for the one-CTA kernel.
 int launch_one_cta(int bn, const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& g, int num_sms, int max_ctas,

@@ -31,9 +31,10 @@ int launch_one(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& g, 
 template <int BN, int NSTAGE>
 int launch_bn(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& g, int num_sms, int max_ctas,
               cudaStream_t st) {
-  switch (epi_class(g.mode)) {
+  switch (epi_class(g)) {
     case EPI_GELU: return launch_one<BN, NSTAGE, EPI_GELU>(ta, tb, g, num_sms, max_ctas, st);
     case EPI_RESID: return launch_one<BN, NSTAGE, EPI_RESID>(ta, tb, g, num_sms, max_ctas, st);
+    case EPI_RESID_LO: return launch_one<BN, NSTAGE, EPI_RESID_LO>(ta, tb, g, num_sms, max_ctas, st);
     case EPI_MUL: return launch_one<BN, NSTAGE, EPI_MUL>(ta, tb, g, num_sms, max_ctas, st);
     case EPI_ATOMIC_F32: return launch_one<BN, NSTAGE, EPI_ATOMIC_F32>(ta, tb, g, num_sms, max_ctas, st);
     case EPI_STORE: return launch_one<BN, NSTAGE, EPI_STORE>(ta, tb, g, num_sms, max_ctas, st);
@@ -53,6 +54,7 @@ int load_bn() {
   bad |= cudaFuncGetAttributes(&a, gemm_kernel<BN, NSTAGE, EPI_STORE>) != cudaSuccess;
   bad |= cudaFuncGetAttributes(&a, gemm_kernel<BN, NSTAGE, EPI_GELU>) != cudaSuccess;
   bad |= cudaFuncGetAttributes(&a, gemm_kernel<BN, NSTAGE, EPI_RESID>) != cudaSuccess;
+  bad |= cudaFuncGetAttributes(&a, gemm_kernel<BN, NSTAGE, EPI_RESID_LO>) != cudaSuccess;
   bad |= cudaFuncGetAttributes(&a, gemm_kernel<BN, NSTAGE, EPI_MUL>) != cudaSuccess;
   bad |= cudaFuncGetAttributes(&a, gemm_kernel<BN, NSTAGE, EPI_ATOMIC_F32>) != cudaSuccess;
   if constexpr (BN == 256) {
