@@ -622,7 +622,8 @@ extern "C" int dsw_stage_forward(void* stage, const long long* ids, const void* 
   }
   bf16* last = y && !copies ? static_cast<bf16*>(y) : v.blk[s.n - 1].out;
   // Sampling: the residual stream, whose rounding at every addition is most of what bf16 costs the logits, keeps its low
-  // half in a second bf16 array (GPT-2 small, 5 x 24 tokens: error of the logits 9.2e-3 without, see the test)
+  // half in a second bf16 array (GPT-2 small, 5 x 24
+  // tokens: error of the logits 9.5e-3 without, 4.2e-3 with it; tests/test_gpu_infer_precision.py)
   const bool precise = infer_logits != nullptr && !keep;
   const GraphKey key{0, B, T, (keep ? 1 : 0) | (infer_logits ? 2 : 0), saved, nullptr};
   TRY(r.replayed(key, copies || (s.wte && !y), [&]() -> int {
