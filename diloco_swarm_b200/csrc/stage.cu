@@ -105,6 +105,7 @@ struct SideMarks {
 
 struct Stage {
   int n, d, nh, V;
+  int sms;                       // of the device it was created on
   int* status;
   cudaStream_t side;
   const float *wte, *wpe;
@@ -495,7 +496,7 @@ struct Run {
     // m x d output tiles and a K of the whole vocabulary: few of them leave most SMs idle for hundreds of k-blocks (2128
     // rows of GPT-2 small: 27 CTA pairs, 238 us), so K is split, with the partial sums in the buffers of the blocks'
     // backward, which have not begun: dh, dx1 and dqkv of both parities lie side by side and hold 8 m x d fp32 arrays.
-    if (((m + 255) / 256) * ((s.d + 255) / 256) < 74) {
+    if (((m + 255) / 256) * ((s.d + 255) / 256) < s.sms / 2) {          // fewer tiles than CTA pairs
       float* partials = reinterpret_cast<float*>(c.dh[0]);
       int splits = 0;
       LAUNCH(dsw_gemm_partials(c.logits, s.head_w, m, s.d, s.V, partials, 8, &splits, s.status, st));
@@ -518,6 +519,10 @@ extern "C" int dsw_stage_create(const long long* desc, int len, void** out) try 
   constexpr int HEAD = 17, PER_BLOCK = 24;
   if (len < HEAD || desc[0] < 0 || len != HEAD + PER_BLOCK * desc[0] || desc[1] % 8 || desc[1] > 2048 || desc[3] % 8) return -10;
   std::unique_ptr<Stage> s(new Stage());
+  int device = 0;
+  if (cudaGetDevice(&device) != cudaSuccess ||
+      cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
+    return -2;
   const char* graphs = getenv("DSWARM_GRAPHS");
   s->graphs_on = !(graphs && graphs[0] == '0' && graphs[1] == 0);
   const long long* p = desc;
@@ -622,8 +627,8 @@ extern "C" int dsw_stage_forward(void* stage, const long long* ids, const void* 
   }
   bf16* last = y && !copies ? static_cast<bf16*>(y) : v.blk[s.n - 1].out;
   // Sampling: the residual stream, whose rounding at every addition is most of what bf16 costs the logits, keeps its low
-  // half in a second bf16 array (GPT-2 small, 5 x 24
-  // tokens: error of the logits 9.5e-3 without, 4.2e-3 with it; tests/test_gpu_infer_precision.py)
+  // half in a second bf16 array (GPT-2 small, 5 x 24 tokens: error of the logits 9.5e-3 without, 4.2e-3 with it;
+  // tests/test_gpu_infer_precision.py)
   const bool precise = infer_logits != nullptr && !keep;
   const GraphKey key{0, B, T, (keep ? 1 : 0) | (infer_logits ? 2 : 0), saved, nullptr};
   TRY(r.replayed(key, copies || (s.wte && !y), [&]() -> int {

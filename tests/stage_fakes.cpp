@@ -18,6 +18,8 @@ thread_local LaunchMode tl_launch;
 
 static long long (*g_hook)(const char*) = nullptr;
 static long long g_handles = 1000;
+static int g_sms = 148;
+extern "C" void fake_set_sms(int n) { g_sms = n; }
 // Allocation number n from now on fails (-1: none does).
 static long long g_failing = -1;
 extern "C" void fake_fail_allocation(long long n) { g_failing = n; }
@@ -51,7 +53,7 @@ template <class T> static cudaError_t made(T* out) { *out = reinterpret_cast<T>(
 extern "C" {
 cudaError_t cudaGetLastError() { return cudaSuccess; }
 cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }
-cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int) { *v = 148; return cudaSuccess; }
+cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int) { *v = g_sms; return cudaSuccess; }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { return made(e); }
 cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) { return made(s); }

@@ -182,3 +182,15 @@ def test_no_exception_leaves_a_c_entry(tmp_path):
     code = OUT_OF_MEMORY.format(here=os.path.dirname(os.path.abspath(__file__)), path=path)
     done = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True)
     assert done.returncode == 0, done.stderr[-2000:]
+
+
+@pytest.mark.parametrize("sms,split", [(148, True), (6, True), (4, False)])
+def test_the_head_is_split_where_pairs_would_idle(device, sms, split):
+    """Two tiles of the head's input gradient: K is split as long as the device has more CTA pairs than that."""
+    device.lib.fake_set_sms(sms)
+    try:
+        s = FakeStage(device.lib)
+    finally:
+        device.lib.fake_set_sms(148)
+    assert s.train(2 * AREA, 5 * AREA, 1, 512, 1) == (0, 0, 0)
+    assert ("gemm_partials" in device.names) == split
