@@ -433,12 +433,12 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, __nv_bfloat16
 // Eleven warps.  Row warps 0-7 (thread = query row, two threads per row, 64 columns each):
 // wait sdp_full, take S and dP out of TMEM in one load group, arrive sdp_read, compute P / dS
 // in registers, wait dq_full of the step before (its products read P / dS), write P / dS,
-// arrive pds_full, then stage the dQ of the step before for the reducer.  MMA warp (one
-// thread): issues the S / dP pair of step i+1 as soon as sdp_read of step i is complete (also
-// for the first step of the next work item: K and V are double-buffered by item parity),
-// then, on pds_full, dV, dK (releasing the Q / dO stage), dQ.  TMA warp (one thread): K / V
-// of the item into the buffer of its parity, Q / dO pairs into two stages.  Reducer warp (one
-// thread): one bulk reduce-add per staged dQ tile, two bulk stores per item for dK / dV
+// arrive pds_full, then stage the dQ of the step before for the reducer.  MMA warp (a whole
+// warp on uniform values, a lane elected around each instruction): issues the S / dP pair of
+// step i+1 as soon as sdp_read of step i is complete (also for the first step of the next work
+// item: K and V are double-buffered by item parity), then, on pds_full, dV, dK (releasing the
+// Q / dO stage), dQ.  TMA warp (likewise): K / V of the item into the buffer of its parity,
+// Q / dO pairs into two stages.  Reducer warp (one lane): one bulk reduce-add per staged dQ tile, two bulk stores per item for dK / dV
 // (staged by the row warps in the P buffer).
 // Every wait is bounded; a wait that runs out sets the CTA's abort flag and the status word.
 struct AttBwdSmem {
@@ -840,8 +840,8 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
         const int i = j + it;
         const int stat = bh * T + i * ATT_BQ + r;       // < 2^31: the launcher checks B * nh * T
         // row statistics: loaded for the CTA's first step, fetched one step ahead (across items too) after that
-        // Rows past the end of the sequence (last tile of a length that is no multiple of 128) have an infinite
-        // log-sum-exp: their P and dS come out as zeros, so whatever the tile holds there adds nothing.
+        // Rows past the end of the sequence (last tile of a length that is no multiple of 128), which the tiles hold
+        // as zeros, have an infinite log-sum-exp: their P and dS come out as zeros and add nothing.
         const bool in_seq = i * ATT_BQ + r < T;
         if (g == 0 && in_seq) { lse_next = lse[stat]; D_next = Dvec[stat]; }
         const float lse2 = in_seq ? lse_next * 1.4426950408889634f : INFINITY;

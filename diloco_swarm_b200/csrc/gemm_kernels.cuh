@@ -334,7 +334,7 @@ __device__ __forceinline__ void epilogue_warp(const GemmArgs& g, uint32_t t_addr
           };
 #pragma unroll
           for (int i = 0; i < 16; ++i) w[i] = pack_bf16_f2(pair(i));
-          if (unsigned(info.target - cb) < 32u) {            // one chunk of a row's 1572
+          if (unsigned(info.target - cb) < 32u) {            // one chunk of the row
 #pragma unroll
             for (int i = 0; i < 16; ++i)
               if (cb + 2 * i == (info.target & ~1)) {

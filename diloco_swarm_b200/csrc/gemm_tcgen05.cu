@@ -11,11 +11,12 @@
 //
 // Structure: persistent CTAs (one per SM), 640 threads.
 //   warp 0      TMA producer: fills a ring of NSTAGE {A,B} k-blocks
-//   warp 1      allocates TMEM, issues tcgen05.mma (one elected lane)
+//   warp 1      allocates TMEM, issues tcgen05.mma (a whole warp on uniform values, one elected lane)
 //   warps 4..19 epilogue: tcgen05.ld of the finished accumulator, math, stores
 //               (four warps per TMEM lane quarter, each takes a quarter of the columns)
 // Two accumulators (2 x BN columns of TMEM) let the epilogue of tile i overlap
-// the main loop of tile i+1.  No thread-block clusters and no multicast loads.
+// the main loop of tile i+1.  That is the one-CTA kernel; the others run 256-row tiles on clusters of two (CTA pairs)
+// and few rows on clusters of up to eight that share K.  No multicast loads anywhere.
 #include <cuda.h>
 #include <cmath>
 #include <cstdio>

@@ -3,13 +3,13 @@
 //
 // What it is for.  A microbatch is some twenty launches per block.  Queued one by one from Python (argument checks,
 // an allocation, a ctypes call, stream bookkeeping) a launch costs about 20 us of host time, which is what bounded
-// every pass of fewer than some eight thousand tokens: one position of the sampling loop on GPT-2 small spent
-// 730 us on the device and 2050 us on the host.  From here a launch costs the driver's own 2 us.
+// every pass of fewer than some eight thousand tokens: one position of the sampling loop on GPT-2 small took 1839 us
+// for 730 us of device work.  From here a launch costs some 3 us.
 //
 // Memory.  The caller hands in two work areas per call: `saved` holds what the backward of a microbatch needs (one
 // per microbatch in flight), `scratch` what lives within a call.  Their sizes come from dsw_stage_sizes.  Nothing is
 // allocated here, so no pass waits for the allocator, and memory that the side stream reads needs no bookkeeping
-// beyond the events below.
+// beyond the marks below.
 //
 // Streams.  Weight-gradient GEMMs and bias column sums feed nothing in the backward, so they go to the stage's side
 // stream (when it has one) and fill the SMs that the dgrad chain leaves idle.  The buffers they read (dh, dx1, dqkv)
@@ -17,13 +17,13 @@
 // two up, which is long done.  A block's outgoing gradient is read by the side work of the block below it, so those
 // buffers form a ring of three.
 //
-// Graphs.  A launch still costs the host 3.3 us, more than many kernels of a short pass take.  So a run of launches that
+// Graphs.  Some 3 us of host time per launch are still more than many kernels of a short pass take.  So a run of launches that
 // touches the work areas only is captured into a CUDA graph when it is asked for a second time in the same areas and
 // replayed from then on, side work and dependent launches included.  What the caller brings or takes away stays outside:
 // token ids, targets, mask, loss, logits of forward_infer; hidden states and their gradients are copied into or out of the
 // areas (some 4 us each at GRAPH_COPY elements; larger ones are not copied and their passes not replayed), so
 // it makes no difference whether they come in the same buffers again.  A handful of graphs per stage is kept, the one
-// used longest ago goes.  Capturing and instantiating may have to wait for an idle device, which never comes while a
+// used longest ago goes (make_room).  Capturing and instantiating may have to wait for an idle device, which never comes while a
 // pipeline receive waits there for a peer that waits for this rank: a stage with neighbours captures while it warms up
 // and is sealed then.
 // Only for passes of up to GRAPH_TOKENS tokens: longer ones keep the device busy for longer than the host needs anyway,
@@ -214,7 +214,8 @@ struct Scratch {
 // Whether the cross-entropy of a pass goes without stored logits (dsw_head_lse and its companions; tiles are 256 columns
 // wide).  Without a gradient always: no logits are written and read again (width 768, 32768 rows: 3007 -> 1749 us, 128
 // rows: 37 -> 32).  With one they have to be computed a second time, which narrow models do faster than they read and
-// write them once more, given enough rows for the third launch (us, stored / unstored, 50304 columns; width 128: 512 rows
+// write them once more, given enough rows for the third launch (us, stored / unstored, 50304 columns; no width between 384
+// and 768 was measured; width 128: 512 rows
 // 49 / 51, 2048 145 / 120, 32768 2018 / 1750; width 384: 512 rows 68 / 78, 2048 219 / 182, 32768 2820 / 2083; width 768:
 // 2048 rows 267 / 287, 32768 3512 / 3823).
 constexpr int HEAD_TWICE_WIDTH = 384, HEAD_TWICE_ROWS = 1024;
