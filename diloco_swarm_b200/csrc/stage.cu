@@ -286,7 +286,7 @@ struct Run {
   int B, T, M, deterministic;
   cudaStream_t st;               // the caller's, or the capturing one
   SideMarks* marks = &s.live;
-  unsigned long long sid = NOBODY;
+  unsigned long long sid = NOBODY;      // of the caller's stream, once asked for
   bool callers = false;          // the caller captures its stream
 
   Run(Stage& stage, int B_, int T_, int det, cudaStream_t stream) : s(stage), B(B_), T(T_), M(B_ * T_), deterministic(det), st(stream) {
@@ -295,10 +295,7 @@ struct Run {
     cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
     unsigned long long id = 0;
     if (cudaStreamGetCaptureInfo(st, &status, &id) != cudaSuccess) { cudaGetLastError(); status = cudaStreamCaptureStatusNone; }
-    if (status != cudaStreamCaptureStatusActive) {
-      if (cudaStreamGetId(st, &sid) != cudaSuccess) sid = NOBODY;      // not to be asked under a capture: it would end it
-      return;
-    }
+    if (status != cudaStreamCaptureStatusActive) return;
     if (s.callers_id != id) s.callers.forget();
     s.callers_id = id;
     marks = &s.callers;
@@ -334,13 +331,16 @@ struct Run {
     return 0;
   }
   // what lies behind the mark is done before what follows on the main stream
-  int wait(SideMark& m) const {
-    if (!m.used || (m.seen == sid && sid != NOBODY)) return 0;
+  int wait(SideMark& m) {
+    if (!m.used) return 0;
+    // not to be asked under a capture, which it would end
+    if (marks == &s.live && sid == NOBODY && cudaStreamGetId(st, &sid) != cudaSuccess) sid = NOBODY;
+    if (m.seen == sid && sid != NOBODY) return 0;
     MAIN_WAIT(m.ev);
     m.seen = sid;
     return 0;
   }
-  int join() const {
+  int join() {
     for (SideMark* m : marks->all) TRY(wait(*m));
     return 0;
   }
@@ -360,7 +360,7 @@ struct Run {
     return 0;
   }
 
-  int block_bwd(int l, const Block& b, const bf16* x, const Saved& v, const Scratch& c, const bf16* dx2, bf16* dx0) const {
+  int block_bwd(int l, const Block& b, const bf16* x, const Saved& v, const Scratch& c, const bf16* dx2, bf16* dx0) {
     const int d = s.d, p = l & 1;
     TRY(wait(marks->done[p]));
     LAUNCH(gemm(dx2, b.w[W_PR], false, 4 * d, d, c.dh[p], DSW_EPI_MUL, nullptr, nullptr, nullptr, v.h, M));

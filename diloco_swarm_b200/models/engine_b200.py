@@ -453,7 +453,7 @@ class B200Engine:
     def forward(self, key: int, input_ids, hidden, keep: bool = True) -> torch.Tensor:
         if self._native():
             with self.exec.lock:
-                ex, st = self.exec, torch.cuda.current_stream()
+                ex, st = self.exec, self.exec.enter()
                 ids, x, B, T = self._input(input_ids, hidden)
                 nbytes = ex.sizes(B, T, keep, False, 0)[0]
                 area = ex.take(nbytes, st) if keep else None
@@ -479,7 +479,7 @@ class B200Engine:
             if self.side is not None:
                 dx.record_stream(self.side)           # the last block's weight gradient reads it there
             with self.exec.lock:
-                ex, st = self.exec, torch.cuda.current_stream()
+                ex, st = self.exec, self.exec.enter()
                 scratch = ex.area("scratch", ex.sizes(B, T, True, True, 0)[1], st)
                 return self._exec_backward(s["area"], scratch, dx, s["ids"], s["x"], B, T, self._want_overlap(sync), 0, st)
         return self._body_bwd(s["saved"], dx.contiguous(), s["ids"], B, T, sync=self._want_overlap(sync))
@@ -526,7 +526,7 @@ class B200Engine:
     def forward_backward(self, key: int, input_ids, hidden, targets, mask, scale: float, sync: bool = False):
         if self._native():
             with self.exec.lock:
-                ex, st, chunks = self.exec, torch.cuda.current_stream(), self.head_chunks
+                ex, st, chunks = self.exec, self.exec.enter(), self.head_chunks
                 ids, x, B, T = self._input(input_ids, hidden)
                 saved_bytes, scratch_bytes = ex.sizes(B, T, True, True, chunks)
                 area = ex.take(saved_bytes, st)
@@ -553,7 +553,7 @@ class B200Engine:
     def forward_loss(self, input_ids, hidden, targets, mask, scale: float) -> torch.Tensor:
         if self._native():
             with self.exec.lock:
-                ex, st = self.exec, torch.cuda.current_stream()
+                ex, st = self.exec, self.exec.enter()
                 ids, x, B, T = self._input(input_ids, hidden)
                 saved_bytes, scratch_bytes = ex.sizes(B, T, False, False, self.head_chunks)
                 saved = ex.area("saved", saved_bytes, st)
@@ -571,7 +571,7 @@ class B200Engine:
     def forward_infer(self, input_ids, hidden) -> torch.Tensor:
         if self._native():
             with self.exec.lock:
-                ex, st = self.exec, torch.cuda.current_stream()
+                ex, st = self.exec, self.exec.enter()
                 ids, x, B, T = self._input(input_ids, hidden)
                 saved = ex.area("saved", ex.sizes(B, T, False, False, 0)[0], st)
                 if self.is_last:          # the LM head's fp32 accumulators are the result

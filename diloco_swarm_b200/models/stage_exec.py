@@ -55,9 +55,15 @@ class StageExec:
         # A pass is several calls of the library on work areas that the passes of a stream share, so a thread holds this
         # from the first to the last of them.
         self.lock = threading.RLock()
+        self.capturing = False
         self._sizes: Dict[tuple, Tuple[int, int]] = {}
         self._scratch: "OrderedDict[Tuple[str, int], torch.Tensor]" = OrderedDict()
         self._idle: List[SavedArea] = []
+
+    def enter(self) -> torch.cuda.Stream:
+        """The calling stream of a pass that begins (the lock is held), looked at for a capture by the caller."""
+        self.capturing = torch.cuda.is_current_stream_capturing()
+        return torch.cuda.current_stream()
 
     # ------------------------------------------------------------------ work areas
     def sizes(self, B: int, T: int, keep: bool, grad: bool, chunks: int) -> Tuple[int, int]:
@@ -82,7 +88,7 @@ class StageExec:
         """Scratch of this calling stream, at least ``nbytes``: its contents live within one pass.  Under a capture of
         the caller's it is the capture's own, and so are the areas of ``take``: replays must not meet other passes there,
         and a capture cannot wait for work from outside of it."""
-        if torch.cuda.is_current_stream_capturing():
+        if self.capturing:
             return self._alloc(nbytes)
         key = (kind, stream.cuda_stream)
         buf = self._scratch.get(key)
@@ -95,7 +101,7 @@ class StageExec:
         return buf
 
     def take(self, nbytes: int, stream: torch.cuda.Stream) -> SavedArea:
-        if torch.cuda.is_current_stream_capturing():
+        if self.capturing:
             return SavedArea(self._alloc(nbytes), stream)
         for i, a in enumerate(self._idle):
             if a.buf.numel() == nbytes:
@@ -111,7 +117,7 @@ class StageExec:
 
     def give(self, area: SavedArea, stream: torch.cuda.Stream) -> None:
         """The backward that read ``area`` has been queued on ``stream`` (and the side stream)."""
-        if torch.cuda.is_current_stream_capturing():
+        if self.capturing:
             return
         if area.free is None:
             area.free = torch.cuda.Event()

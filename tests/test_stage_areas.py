@@ -35,9 +35,8 @@ class Buffer:
 @pytest.fixture
 def executor(monkeypatch):
     monkeypatch.setattr(torch.cuda, "Event", Event)
-    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
     ex = StageExec.__new__(StageExec)
-    ex.side, ex._idle, ex._alloc = Stream(), [], Buffer
+    ex.side, ex._idle, ex._alloc, ex.capturing = Stream(), [], Buffer, False
     return ex
 
 
@@ -71,6 +70,8 @@ def test_a_capture_has_areas_of_its_own(executor, monkeypatch):
     executor.give(area, a)
     scratch = executor.area("scratch", 100, a)
     monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: True)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda: a)
+    assert executor.enter() is a
     mine = executor.take(100, a)
     assert mine is not area and executor.area("scratch", 100, a) is not scratch and a.waited == []
     executor.give(mine, a)
