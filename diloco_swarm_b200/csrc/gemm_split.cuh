@@ -2,7 +2,7 @@
 //
 // What bounds such a GEMM is neither arithmetic nor bandwidth but latency and how many bytes are in flight: 120 rows of
 // GPT-2 small through the MLP's second projection (N 768, K 3072) are six 128-wide tiles, so six SMs walked 48 k-blocks
-// one after the other (18.2 us with 4.7 MB of weights cold in L2, 8.2 here).  Here a tile is 32, 64 or 128 columns wide and its K range is
+// one after the other (17.3 us with 4.7 MB of weights cold in L2, 8.4 here).  Here a tile is 32, 64 or 128 columns wide and its K range is
 // divided over up to eight CTAs, enough of them to fill the SMs; every CTA has most of its share in flight at once.
 // The partial sums meet inside the cluster: a CTA owns BN / S of the tile's columns, receives the other CTAs' fp32
 // sums of those through distributed shared memory and runs the epilogue on them.  No atomics, no second launch, and a
