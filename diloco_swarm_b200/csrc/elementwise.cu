@@ -165,186 +165,223 @@ layernorm_fwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* x_lo, const fl
 
 // LayerNorm backward: dx = rstd * (g*dy - mean(g*dy) - xhat * mean(g*dy*xhat)) (+ dres), and the
 // column sums dgamma = sum_rows dy*xhat, dbeta = sum_rows dy and (optionally) sum_rows dres, which is
-// the bias gradient of the linear layer that fed the residual branch.
-// One warp per row, the row in registers.  The column sums would cost 72 registers per thread if
-// they lived there (d = 768), which caps the kernel at one block per SM; instead every warp adds its
-// row's terms into its own fp32 strip of shared memory (lane-private columns, so no conflicts and no
-// atomics).  At the end the block folds its warps' strips and writes partial[block][3][d]; a small
-// finish kernel adds the per-block partials into the fp32 gradients in a fixed order.
-constexpr int LN_BWD_WARPS = 8;
+// the bias gradient of the linear layer that fed the residual branch.  The sums of a block go to partial[block][3][d];
+// a small finish kernel adds the per-block partials into the fp32 gradients in a fixed order.
+//
+// A thread owns eight columns (16 bytes) of every row that its group of warps works on, so the column sums and
+// gamma are 32 registers at any width, and no sum leaves the thread before the end.  A group takes LN_BWD_ROWS rows at a
+// time, whose loads are all in flight together, and the two row sums of all of them cross the group in one exchange
+// (shuffles that halve the number of values at each step, then shared memory and one barrier of the group's own, so that
+// one group computes while another's loads are under way).
+#ifndef LR
+#define LR 2
+#define LW 16
+#endif
+constexpr int LN_BWD_ROWS = LR;
+constexpr int LN_BWD_MAX_WARPS = LW;
 
-// One row's operands as loaded (bf16, 8 per lane per 256-column chunk) plus its statistics.
-template <int NCH>
-struct LnBwdRow {
-  uint4 x[NCH], dy[NCH], r[NCH];
-  float mean, rstd;
-};
-
-template <int NCH>
-__device__ __forceinline__ void ln_bwd_load(LnBwdRow<NCH>& o, const __nv_bfloat16* dy, const __nv_bfloat16* x,
-                                            const __nv_bfloat16* dres, const float* mean_in, const float* rstd_in,
-                                            int row, int M, int d, int nch, int lane) {
-  const long long off = (long long)row * d;
+// Sums v[i] over the warp for N values, a power of two: lane l ends with the sum of value l / (32 / N).
+template <int N>
+__device__ __forceinline__ float warp_sums(float (&v)[N]) {
+  const int lane = threadIdx.x & 31;
+  int o = 16;
 #pragma unroll
-  for (int c = 0; c < NCH; ++c) {
-    const int col = c * 256 + lane * 8;
-    if (c < nch && col < d && row < M && DSW_OK(row >= 0 && col + 8 <= d)) {
-      o.x[c] = *reinterpret_cast<const uint4*>(x + off + col);
-      o.dy[c] = *reinterpret_cast<const uint4*>(dy + off + col);
-      if (dres) o.r[c] = *reinterpret_cast<const uint4*>(dres + off + col);
+  for (int n = N / 2; n >= 1; n >>= 1, o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int i = 0; i < n; ++i) {
+      const float keep = up ? v[i + n] : v[i], send = up ? v[i] : v[i + n];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
     }
   }
+  float s = v[0];
+#pragma unroll
+  for (; o >= 1; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
+
+// Hides from the compiler that a value is the one it has seen before.
+__device__ __forceinline__ void opaque(uint4& u) { asm volatile("" : "+r"(u.x), "+r"(u.y), "+r"(u.z), "+r"(u.w)); }
+
+// W: warps per group = ceil(d / 256), blockDim.x / (32 W) groups per block.
+template <int W>
+__global__ void __launch_bounds__(32 * LN_BWD_MAX_WARPS, 1)
+layernorm_bwd_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* x, const float* __restrict__ gamma, const float* mean_in,
+                     const float* rstd_in, const __nv_bfloat16* dres,
+                     __nv_bfloat16* __restrict__ dx, float* __restrict__ partial, int M, int d) {
+  constexpr int R = LN_BWD_ROWS;
+  extern __shared__ float sh[];                 // [2][groups][W][2 R] while rows are worked on, then [groups][3][d]
+  const int groups = blockDim.x / (32 * W), grp = threadIdx.x / (32 * W);
+  const int t = threadIdx.x - grp * 32 * W, lane = threadIdx.x & 31, col = t * 8;
+  const bool live = col < d;                    // the last warp of a group may reach past the row
+  float gm[8], acc_g[8], acc_b[8], acc_r[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) { gm[j] = 0.f; acc_g[j] = 0.f; acc_b[j] = 0.f; acc_r[j] = 0.f; }
+  if (live) load8f(gamma + col, gm);
+  const float inv_d = 1.f / d;
+  pdl_wait();
+  pdl_launch();
+  const int step = gridDim.x * groups * R;
+  int buf = 0;
+  for (int row0 = (blockIdx.x * groups + grp) * R; row0 < M; row0 += step, buf ^= 1) {
+    uint4 xv[R], dv[R], rv[R];
+    float mean[R], rstd[R];
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+      const int row = row0 + k;
+      const long long off = (long long)row * d + col;
+      const bool in = live && row < M && DSW_OK(row >= 0 && col + 8 <= d);
+      xv[k] = in ? *reinterpret_cast<const uint4*>(x + off) : make_uint4(0, 0, 0, 0);
+      dv[k] = in ? *reinterpret_cast<const uint4*>(dy + off) : make_uint4(0, 0, 0, 0);
+      rv[k] = in && dres ? *reinterpret_cast<const uint4*>(dres + off) : make_uint4(0, 0, 0, 0);
+      mean[k] = row < M ? mean_in[row] : 0.f;
+      rstd[k] = row < M ? rstd_in[row] : 0.f;
+    }
+    float s[2 * R];
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+      float xh[8], g[8];
+      unpack8(xv[k], xh);
+      unpack8(dv[k], g);
+      float s1 = 0.f, s2 = 0.f;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float xhat = (xh[j] - mean[k]) * rstd[k];
+        const float gy = g[j] * gm[j];
+        s1 += gy;
+        s2 += gy * xhat;
+        acc_g[j] += g[j] * xhat;
+        acc_b[j] += g[j];
+      }
+      s[2 * k] = s1;
+      s[2 * k + 1] = s2;
+      float r[8];
+      unpack8(rv[k], r);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc_r[j] += r[j];
+    }
+    const float mine = warp_sums(s);
+    float* part = sh + (buf * groups + grp) * W * 2 * R;
+    constexpr int LANES = 32 / (2 * R);         // that hold the same sum
+    if ((lane & (LANES - 1)) == 0) part[(t >> 5) * 2 * R + lane / LANES] = mine;
+    // the buffer is written again two rounds on, when every warp of the group has passed the next round's barrier
+    if constexpr (W == 1) __syncwarp();
+    else asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "n"(32 * W) : "memory");
+    // unpacked again below: the floats from above would not fit
+#pragma unroll
+    for (int k = 0; k < R; ++k) { opaque(xv[k]); opaque(dv[k]); opaque(rv[k]); }
+#pragma unroll
+    for (int i = 0; i < 2 * R; ++i) s[i] = 0.f;
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+#pragma unroll
+      for (int i = 0; i < 2 * R; i += 4) {
+        const float4 a = *reinterpret_cast<const float4*>(part + w * 2 * R + i);
+        s[i] += a.x; s[i + 1] += a.y; s[i + 2] += a.z; s[i + 3] += a.w;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+      const int row = row0 + k;
+      if (!live || row >= M || !DSW_OK(row >= 0 && col + 8 <= d)) continue;
+      const float m1 = s[2 * k] * inv_d, m2 = s[2 * k + 1] * inv_d;
+      float xh[8], g[8], r[8], o[8];
+      unpack8(xv[k], xh);
+      unpack8(dv[k], g);
+      unpack8(rv[k], r);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) o[j] = rstd[k] * (g[j] * gm[j] - m1 - (xh[j] - mean[k]) * rstd[k] * m2) + r[j];
+      store8(dx + (long long)row * d + col, o);
+    }
+  }
+  __syncthreads();                              // the exchange buffers become the block's sums
+  if (live) {
+    float* out = sh + (long long)grp * 3 * d + col;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) { out[j] = acc_g[j]; out[d + j] = acc_b[j]; out[2 * d + j] = acc_r[j]; }
+  }
+  __syncthreads();
+  float* out = partial + (long long)blockIdx.x * 3 * d;
+  for (int i = threadIdx.x; i < 3 * d; i += blockDim.x) {
+    float v = 0.f;
+    for (int k = 0; k < groups; ++k) v += sh[(long long)k * 3 * d + i];
+    out[i] = v;
+  }
+}
+
+// Rows of up to 128 columns: half a warp per row, as in the forward; the row and its successor in registers.
+constexpr int LN_BWD_WARPS = 8;
+
+// One row's operands as loaded (eight bf16 per lane) plus its statistics.
+struct LnBwdRow {
+  uint4 x, dy, r;
+  float mean, rstd;
+};
+__device__ __forceinline__ void ln_bwd_load(LnBwdRow& o, const __nv_bfloat16* dy, const __nv_bfloat16* x, const __nv_bfloat16* dres,
+                                            const float* mean_in, const float* rstd_in, int row, int M, int d, int lane) {
+  const long long off = (long long)row * d + lane * 8;
+  const bool in = lane * 8 < d && row < M && DSW_OK(row >= 0 && lane * 8 + 8 <= d);       // a row past the last one adds zeros
+  o.x = in ? *reinterpret_cast<const uint4*>(x + off) : make_uint4(0, 0, 0, 0);
+  o.dy = in ? *reinterpret_cast<const uint4*>(dy + off) : make_uint4(0, 0, 0, 0);
+  o.r = in && dres ? *reinterpret_cast<const uint4*>(dres + off) : make_uint4(0, 0, 0, 0);
   o.mean = row < M ? mean_in[row] : 0.f;
   o.rstd = row < M ? rstd_in[row] : 0.f;
 }
 
-// Blocks per SM: rows of 264 to 768 columns keep the column sums, gamma and two rows (the current one and the
-// prefetched next one) in registers, about 200 per thread, so one block; wider rows use the strips,
-// narrower ones need few, two blocks.
-constexpr int ln_bwd_blocks_per_sm(int nch) { return nch == 2 || nch == 3 ? 1 : 2; }
-
-template <int LN_MAX_CHUNKS, int LPR>          // LPR: lanes per row, as in the forward
-__global__ void __launch_bounds__(32 * LN_BWD_WARPS, ln_bwd_blocks_per_sm(LN_MAX_CHUNKS))
-layernorm_bwd_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* x, const float* __restrict__ gamma, const float* mean_in,
-                     const float* rstd_in, const __nv_bfloat16* dres,
-                     __nv_bfloat16* __restrict__ dx, float* __restrict__ partial, int M, int d) {
+__global__ void __launch_bounds__(32 * LN_BWD_WARPS, 2)
+layernorm_bwd_narrow_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* x, const float* __restrict__ gamma, const float* mean_in,
+                            const float* rstd_in, const __nv_bfloat16* dres,
+                            __nv_bfloat16* __restrict__ dx, float* __restrict__ partial, int M, int d) {
+  constexpr int LPR = 16;                       // lanes per row
   extern __shared__ float sh[];                 // [LN_BWD_WARPS][3][d]
-  static_assert(LPR == 32 || LN_MAX_CHUNKS == 1, "rows that share a warp are one chunk long");
-  const int lane = threadIdx.x & (LPR - 1), warp = threadIdx.x >> 5;
-  const int nch = (d + 255) / 256;
-  float* mine = sh + (long long)warp * 3 * d;
-  for (int i = threadIdx.x & 31; i < 3 * d; i += 32) mine[i] = 0.f;
-  __syncwarp();
-  // Rows stay in the bf16 form they were loaded in and are unpacked in both passes (cheaper in registers
-  // than a row of fp32).  Up to 768 columns the column sums live in registers (72 per thread) and reach the
-  // warp's shared strip once, at the end: a read-modify-write of the strips per row costs more shared-memory
-  // cycles than the whole row costs in DRAM time.  Wider rows add into the strips row by row; up to 1024
-  // columns the next row's loads are issued before the current row is worked on.
-  constexpr bool REG_ACC = LN_MAX_CHUNKS <= 3;
-  constexpr bool PREFETCH = LN_MAX_CHUNKS <= 4;
-  constexpr int NACC = REG_ACC ? LN_MAX_CHUNKS : 1;
-  float acc_g[NACC][8], acc_b[NACC][8], acc_r[NACC][8], gm[NACC][8];
+  const int lane = threadIdx.x & (LPR - 1), warp = threadIdx.x >> 5, col = lane * 8;
+  float acc_g[8], acc_b[8], acc_r[8], gm[8];
 #pragma unroll
-  for (int c = 0; c < NACC; ++c) {
-#pragma unroll
-    for (int j = 0; j < 8; ++j) { acc_g[c][j] = 0.f; acc_b[c][j] = 0.f; acc_r[c][j] = 0.f; gm[c][j] = 0.f; }
-    // gamma lives in registers next to the sums (read per row it was 12 of a 768-wide row's 24 memory instructions)
-    if (REG_ACC && c * 256 + lane * 8 < d) load8f(gamma + c * 256 + lane * 8, gm[c]);
-  }
+  for (int j = 0; j < 8; ++j) { acc_g[j] = 0.f; acc_b[j] = 0.f; acc_r[j] = 0.f; gm[j] = 0.f; }
+  if (col < d) load8f(gamma + col, gm);
   pdl_wait();
   pdl_launch();
   const int stride = gridDim.x * LN_BWD_WARPS * (32 / LPR);
   int first = (blockIdx.x * LN_BWD_WARPS + warp) * (32 / LPR);          // the warp's first row
   int row = first + (threadIdx.x & 31) / LPR;
-  LnBwdRow<LN_MAX_CHUNKS> cur, nxt;
-  if (LPR < 32) {          // a row past the last one adds zeros
-    cur.x[0] = cur.dy[0] = cur.r[0] = make_uint4(0, 0, 0, 0);
-    nxt = cur;
-  }
-  if (PREFETCH && first < M) ln_bwd_load(cur, dy, x, dres, mean_in, rstd_in, row, M, d, nch, lane);
+  LnBwdRow cur, nxt;
+  if (first < M) ln_bwd_load(cur, dy, x, dres, mean_in, rstd_in, row, M, d, lane);
   for (; first < M; first += stride, row += stride) {
-    if (PREFETCH) {
-      if (LPR < 32) nxt.x[0] = nxt.dy[0] = nxt.r[0] = make_uint4(0, 0, 0, 0);
-      if (first + stride < M) ln_bwd_load(nxt, dy, x, dres, mean_in, rstd_in, row + stride, M, d, nch, lane);
-    } else {
-      ln_bwd_load(cur, dy, x, dres, mean_in, rstd_in, row, M, d, nch, lane);
-    }
-    const long long off = (long long)row * d;
-    const float mean = cur.mean, rstd = cur.rstd;
-    float s1 = 0.f, s2 = 0.f;
+    if (first + stride < M) ln_bwd_load(nxt, dy, x, dres, mean_in, rstd_in, row + stride, M, d, lane);
+    float dv[8], xh[8], r[8], s1 = 0.f, s2 = 0.f;
+    unpack8(cur.x, xh);
+    unpack8(cur.dy, dv);
+    unpack8(cur.r, r);
 #pragma unroll
-    for (int c = 0; c < LN_MAX_CHUNKS; ++c) {
-      const int col = c * 256 + lane * 8;
-      if (c < nch && col < d) {
-        float g[8], dv[8], xh[8];
-        unpack8(cur.x[c], xh);
-        unpack8(cur.dy[c], dv);
-        if constexpr (!REG_ACC) load8f(gamma + col, g);
-        if constexpr (REG_ACC) {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const float xhat = (xh[j] - mean) * rstd;
-            const float gy = dv[j] * gm[c][j];
-            s1 += gy;
-            s2 += gy * xhat;
-            acc_g[c][j] += dv[j] * xhat;
-            acc_b[c][j] += dv[j];
-          }
-        } else {
-          float4* a0 = reinterpret_cast<float4*>(mine + col);
-          float4* b0 = reinterpret_cast<float4*>(mine + d + col);
-          float4 ag0 = a0[0], ag1 = a0[1], ab0 = b0[0], ab1 = b0[1];
-          float* ag = &ag0.x; float* agh = &ag1.x; float* ab = &ab0.x; float* abh = &ab1.x;
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const float xhat = (xh[j] - mean) * rstd;
-            const float gy = dv[j] * g[j];
-            s1 += gy;
-            s2 += gy * xhat;
-            if (j < 4) { ag[j] += dv[j] * xhat; ab[j] += dv[j]; }
-            else       { agh[j - 4] += dv[j] * xhat; abh[j - 4] += dv[j]; }
-          }
-          a0[0] = ag0; a0[1] = ag1; b0[0] = ab0; b0[1] = ab1;
-        }
-      }
+    for (int j = 0; j < 8; ++j) {
+      const float xhat = (xh[j] - cur.mean) * cur.rstd;
+      const float gy = dv[j] * gm[j];
+      s1 += gy;
+      s2 += gy * xhat;
+      acc_g[j] += dv[j] * xhat;
+      acc_b[j] += dv[j];
+      acc_r[j] += r[j];
     }
     s1 = group_sum<LPR>(s1) / d;
     s2 = group_sum<LPR>(s2) / d;
+    if (col < d && row < M && DSW_OK(col + 8 <= d)) {
+      float o[8];
 #pragma unroll
-    for (int c = 0; c < LN_MAX_CHUNKS; ++c) {
-      const int col = c * 256 + lane * 8;
-      if (c < nch && col < d) {
-        float g[8], dv[8], xh[8], o[8], r[8];
-        unpack8(cur.x[c], xh);
-        unpack8(cur.dy[c], dv);
-        if constexpr (REG_ACC) {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) g[j] = gm[c][j];
-        } else {
-          load8f(gamma + col, g);
-        }
-        if (dres) {
-          unpack8(cur.r[c], r);
-          if constexpr (REG_ACC) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) acc_r[c][j] += r[j];
-          } else {
-            float4* c0 = reinterpret_cast<float4*>(mine + 2 * d + col);
-            float4 r0 = c0[0], r1 = c0[1];
-            r0.x += r[0]; r0.y += r[1]; r0.z += r[2]; r0.w += r[3];
-            r1.x += r[4]; r1.y += r[5]; r1.z += r[6]; r1.w += r[7];
-            c0[0] = r0; c0[1] = r1;
-          }
-        }
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-          o[j] = rstd * (dv[j] * g[j] - s1 - (xh[j] - mean) * rstd * s2) + (dres ? r[j] : 0.f);
-        if (row < M && DSW_OK(col + 8 <= d)) store8(dx + off + col, o);
-      }
+      for (int j = 0; j < 8; ++j) o[j] = cur.rstd * (dv[j] * gm[j] - s1 - (xh[j] - cur.mean) * cur.rstd * s2) + r[j];
+      store8(dx + (long long)row * d + col, o);
     }
-    if (PREFETCH) cur = nxt;
+    cur = nxt;
   }
-  if constexpr (LPR < 32) {
+  float* mine = sh + (long long)warp * 3 * d;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      acc_g[0][j] += __shfl_xor_sync(0xffffffffu, acc_g[0][j], LPR);
-      acc_b[0][j] += __shfl_xor_sync(0xffffffffu, acc_b[0][j], LPR);
-      acc_r[0][j] += __shfl_xor_sync(0xffffffffu, acc_r[0][j], LPR);
-    }
-  }
-  if constexpr (REG_ACC) {
-#pragma unroll
-    for (int c = 0; c < LN_MAX_CHUNKS; ++c) {
-      const int col = c * 256 + lane * 8;
-      if (c < nch && col < d) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          if (LPR < 32 && (threadIdx.x & LPR)) continue;          // folded into the lower lanes above
-          mine[col + j] = acc_g[c][j];
-          mine[d + col + j] = acc_b[c][j];
-          mine[2 * d + col + j] = acc_r[c][j];
-        }
-      }
+  for (int j = 0; j < 8; ++j) {
+    acc_g[j] += __shfl_xor_sync(0xffffffffu, acc_g[j], LPR);
+    acc_b[j] += __shfl_xor_sync(0xffffffffu, acc_b[j], LPR);
+    acc_r[j] += __shfl_xor_sync(0xffffffffu, acc_r[j], LPR);
+    if (col < d && !(threadIdx.x & LPR)) {
+      mine[col + j] = acc_g[j];
+      mine[d + col + j] = acc_b[j];
+      mine[2 * d + col + j] = acc_r[j];
     }
   }
   __syncthreads();
@@ -795,9 +832,9 @@ extern "C" int dsw_layernorm_fwd_lo(const void* x, const void* x_lo, const float
   return rc == cudaSuccess ? 0 : -3;
 }
 
-// Number of blocks dsw_layernorm_bwd launches for M rows = rows of scratch it needs.
+// The most blocks dsw_layernorm_bwd launches for M rows = rows of scratch it needs.
 extern "C" int dsw_layernorm_bwd_blocks(int M) {
-  const int want = (M + LN_BWD_WARPS * 4 - 1) / (LN_BWD_WARPS * 4);      // about 4 rows per warp at least
+  const int want = (M + 2 * LN_BWD_ROWS - 1) / (2 * LN_BWD_ROWS);      // the widest rows: two groups to a block
   return want < 1 ? 1 : (want > 296 ? 296 : want);     // at most two blocks per SM
 }
 
@@ -807,36 +844,29 @@ extern "C" int dsw_layernorm_bwd(const void* dy, const void* x, const float* gam
                                  const float* rstd, const void* dres, void* dx, float* dgamma, float* dbeta,
                                  float* dres_sum, float* scratch, int M, int d, cudaStream_t st) {
   if (d % 8 || d > 256 * LN_MAX_CHUNKS_ALL) return -10;
-  int grid = dsw_layernorm_bwd_blocks(M);
-  const bool two_rows = d <= 128;
-  // the register-resident variant runs one block per SM, except for rows of one chunk
-  if (d > 256 && d <= 768 && grid > 148) grid = 148;
   const int want = dres_sum != nullptr && dres != nullptr;
-  const size_t shmem = sizeof(float) * LN_BWD_WARPS * 3 * d;
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -2;
   cudaError_t rc;
-#define LN_BWD(NCH, LPR)                                                                                          \
-  do {                                                                                                           \
-    static bool attr[64] = {false};          /* the attribute is per device */                                 \
-    if (!attr[dev]) {                                                                                            \
-      if (cudaFuncSetAttribute(layernorm_bwd_kernel<NCH, LPR>, cudaFuncAttributeMaxDynamicSharedMemorySize,           \
-                               8 * 3 * 256 * NCH * 4) != cudaSuccess)                                            \
-        return -2;                                                                                               \
-      attr[dev] = true;                                                                                          \
-    }                                                                                                            \
-    rc = launch(layernorm_bwd_kernel<NCH, LPR>, grid, 32 * LN_BWD_WARPS, shmem, st, 1, (const bf16*)dy, (const bf16*)x, gamma, \
-                mean, rstd, (const bf16*)dres, (bf16*)dx, scratch, M, d);                                        \
-  } while (0)
-  switch ((d + 255) / 256) {
-    case 1:
-      if (two_rows) LN_BWD(1, 16);
-      else          LN_BWD(1, 32);
-      break;
-    case 2: LN_BWD(2, 32); break; case 3: LN_BWD(3, 32); break; case 4: LN_BWD(4, 32); break; case 5: LN_BWD(5, 32); break;
-    case 6: LN_BWD(6, 32); break; case 7: LN_BWD(7, 32); break; default: LN_BWD(8, 32); break;
-  }
+  int grid;
+  if (d <= 128) {
+    grid = (M + 4 * LN_BWD_WARPS - 1) / (4 * LN_BWD_WARPS);      // two steps of two rows per warp at least
+    grid = grid < 1 ? 1 : grid > 296 ? 296 : grid;
+    rc = launch(layernorm_bwd_narrow_kernel, grid, 32 * LN_BWD_WARPS, sizeof(float) * LN_BWD_WARPS * 3 * d, st, 1, (const bf16*)dy,
+                (const bf16*)x, gamma, mean, rstd, (const bf16*)dres, (bf16*)dx, scratch, M, d);
+  } else {
+    const int W = (d + 255) / 256, groups = LN_BWD_MAX_WARPS / W, rows = groups * LN_BWD_ROWS;
+    grid = (M + rows - 1) / rows;
+    grid = grid < 1 ? 1 : grid > 148 ? 148 : grid;
+    // the block's sums, at most 48 KB; never less than the exchange buffers ([2][warps][2 rows] floats)
+    const size_t shmem = sizeof(float) * groups * 3 * d;
+#define LN_BWD(W_)                                                                                                           \
+  rc = launch(layernorm_bwd_kernel<W_>, grid, 32 * W_ * groups, shmem, st, 1, (const bf16*)dy, (const bf16*)x, gamma, mean, rstd, \
+              (const bf16*)dres, (bf16*)dx, scratch, M, d)
+    switch (W) {
+      case 1: LN_BWD(1); break; case 2: LN_BWD(2); break; case 3: LN_BWD(3); break; case 4: LN_BWD(4); break;
+      case 5: LN_BWD(5); break; case 6: LN_BWD(6); break; case 7: LN_BWD(7); break; default: LN_BWD(8); break;
+    }
 #undef LN_BWD
+  }
   if (rc != cudaSuccess) return -3;
   return launch(layernorm_bwd_finish_kernel, (3 * d + 31) / 32, dim3(32, 32), 0, st, 1, scratch, grid, d, dgamma, dbeta,
                 want ? dres_sum : nullptr) == cudaSuccess
@@ -961,8 +991,8 @@ extern "C" int dsw_load_elementwise() {
 #define L(f) bad |= cudaFuncGetAttributes(&a, f) != cudaSuccess
   L((layernorm_fwd_kernel<1, false, 16>)); L((layernorm_fwd_kernel<1, true, 16>)); L((layernorm_fwd_kernel<1, false, 32>)); L((layernorm_fwd_kernel<1, true, 32>)); L((layernorm_fwd_kernel<2, false, 32>)); L((layernorm_fwd_kernel<2, true, 32>)); L((layernorm_fwd_kernel<3, false, 32>)); L((layernorm_fwd_kernel<3, true, 32>)); L((layernorm_fwd_kernel<4, false, 32>)); L((layernorm_fwd_kernel<4, true, 32>));
   L((layernorm_fwd_kernel<5, false, 32>)); L((layernorm_fwd_kernel<5, true, 32>)); L((layernorm_fwd_kernel<6, false, 32>)); L((layernorm_fwd_kernel<6, true, 32>)); L((layernorm_fwd_kernel<7, false, 32>)); L((layernorm_fwd_kernel<7, true, 32>)); L((layernorm_fwd_kernel<8, false, 32>)); L((layernorm_fwd_kernel<8, true, 32>));
-  L((layernorm_bwd_kernel<1, 16>)); L((layernorm_bwd_kernel<1, 32>)); L((layernorm_bwd_kernel<2, 32>)); L((layernorm_bwd_kernel<3, 32>)); L((layernorm_bwd_kernel<4, 32>));
-  L((layernorm_bwd_kernel<5, 32>)); L((layernorm_bwd_kernel<6, 32>)); L((layernorm_bwd_kernel<7, 32>)); L((layernorm_bwd_kernel<8, 32>));
+  L(layernorm_bwd_kernel<1>); L(layernorm_bwd_kernel<2>); L(layernorm_bwd_kernel<3>); L(layernorm_bwd_kernel<4>);
+  L(layernorm_bwd_kernel<5>); L(layernorm_bwd_kernel<6>); L(layernorm_bwd_kernel<7>); L(layernorm_bwd_kernel<8>); L(layernorm_bwd_narrow_kernel);
   L(layernorm_bwd_finish_kernel); L(colsum_kernel); L(embedding_fwd_kernel); L(embedding_bwd_kernel);
   L(embedding_bwd_sorted_kernel); L(embedding_bwd_pos_kernel);
   L(mask_count_kernel); L(loss_begin_kernel); L(cross_entropy_kernel); L(head_rows_kernel); L(sum_partials_kernel); L(cast_f32_bf16_kernel); L(cast_bf16_f32_kernel);
