@@ -168,17 +168,20 @@ layernorm_fwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* x_lo, const fl
 // the bias gradient of the linear layer that fed the residual branch.  The sums of a block go to partial[block][3][d];
 // a small finish kernel adds the per-block partials into the fp32 gradients in a fixed order.
 //
-// A thread owns eight columns (16 bytes) of every row that its group of warps works on, so the column sums and
-// gamma are 32 registers at any width, and no sum leaves the thread before the end.  A group takes LN_BWD_ROWS rows at a
-// time, whose loads are all in flight together, and the two row sums of all of them cross the group in one exchange
-// (shuffles that halve the number of values at each step, then shared memory and one barrier of the group's own, so that
-// one group computes while another's loads are under way).
-#ifndef LR
-#define LR 2
-#define LW 16
-#endif
-constexpr int LN_BWD_ROWS = LR;
-constexpr int LN_BWD_MAX_WARPS = LW;
+// A thread owns eight columns (16 bytes) of every row that its group of ceil(d / 256) warps works on, so the column sums
+// and gamma are 32 registers at any width, and no sum leaves the thread before the end.  A group takes LN_BWD_ROWS rows at
+// a time, and their two row sums cross it in one exchange: shuffles that halve the number of values at each step, then
+// shared memory and one barrier of the group's own, so that one group computes while another waits.  The next rows are on
+// their way into shared memory meanwhile, by cp.async: a thread reads only what it copied itself, so nothing has to be
+// synchronised, and the second look at a row costs no registers.
+// Before, a warp took a whole row: its sums were 72 registers at 768 columns, which left eight warps to an SM, and had to be
+// added up in shared memory, row by row, above that.  Kernel alone, operands cold, us: 8192 x 1024 41.4 -> 14.8 (67 MB),
+// 4096 x 1280 20.4 -> 12.4, 2000 x 1600 25.8 -> 10.8, 4096 x 2048 40.1 -> 16.8, 2128 x 768 9.9 -> 6.1, 16384 x 768 24.3 ->
+// 22.0, 32768 x 768 42.8 -> 38.4 (201 MB).  Rows in registers instead of shared memory took 43.6 at the largest and 0.3 less
+// at the smallest; three stages 39.0; 24 warps 37.1 there, 1.2 more at 128 x 768.
+constexpr int LN_BWD_ROWS = 2;
+constexpr int LN_BWD_MAX_WARPS = 16;
+constexpr int LN_BWD_STAGES = 2;
 
 // Sums v[i] over the warp for N values, a power of two: lane l ends with the sum of value l / (32 / N).
 template <int N>
@@ -200,8 +203,10 @@ __device__ __forceinline__ float warp_sums(float (&v)[N]) {
   return s;
 }
 
-// Hides from the compiler that a value is the one it has seen before.
-__device__ __forceinline__ void opaque(uint4& u) { asm volatile("" : "+r"(u.x), "+r"(u.y), "+r"(u.z), "+r"(u.w)); }
+// 16 bytes global -> shared, zeros where !in.
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, bool in) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(in ? 16 : 0) : "memory");
+}
 
 // W: warps per group = ceil(d / 256), blockDim.x / (32 W) groups per block.
 template <int W>
@@ -210,10 +215,14 @@ layernorm_bwd_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* x, const floa
                      const float* rstd_in, const __nv_bfloat16* dres,
                      __nv_bfloat16* __restrict__ dx, float* __restrict__ partial, int M, int d) {
   constexpr int R = LN_BWD_ROWS;
-  extern __shared__ float sh[];                 // [2][groups][W][2 R] while rows are worked on, then [groups][3][d]
+  constexpr int S = LN_BWD_STAGES;
+  extern __shared__ __align__(16) uint8_t ln_smem[];
   const int groups = blockDim.x / (32 * W), grp = threadIdx.x / (32 * W);
   const int t = threadIdx.x - grp * 32 * W, lane = threadIdx.x & 31, col = t * 8;
   const bool live = col < d;                    // the last warp of a group may reach past the row
+  uint4* mine = reinterpret_cast<uint4*>(ln_smem) + threadIdx.x;              // [S][R][3][threads]: a thread reads what it copied
+  float* exch = reinterpret_cast<float*>(ln_smem + S * R * 3 * 16 * blockDim.x);         // [2][groups][W][2 R]
+  const auto slot = [&](int st, int k, int what) -> uint4& { return mine[((st * R + k) * 3 + what) * blockDim.x]; };
   float gm[8], acc_g[8], acc_b[8], acc_r[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) { gm[j] = 0.f; acc_g[j] = 0.f; acc_b[j] = 0.f; acc_r[j] = 0.f; }
@@ -222,27 +231,44 @@ layernorm_bwd_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* x, const floa
   pdl_wait();
   pdl_launch();
   const int step = gridDim.x * groups * R;
-  int buf = 0;
-  for (int row0 = (blockIdx.x * groups + grp) * R; row0 < M; row0 += step, buf ^= 1) {
-    uint4 xv[R], dv[R], rv[R];
-    float mean[R], rstd[R];
+  const auto fetch = [&](int st, int row0) {
 #pragma unroll
     for (int k = 0; k < R; ++k) {
       const int row = row0 + k;
-      const long long off = (long long)row * d + col;
       const bool in = live && row < M && DSW_OK(row >= 0 && col + 8 <= d);
-      xv[k] = in ? *reinterpret_cast<const uint4*>(x + off) : make_uint4(0, 0, 0, 0);
-      dv[k] = in ? *reinterpret_cast<const uint4*>(dy + off) : make_uint4(0, 0, 0, 0);
-      rv[k] = in && dres ? *reinterpret_cast<const uint4*>(dres + off) : make_uint4(0, 0, 0, 0);
-      mean[k] = row < M ? mean_in[row] : 0.f;
-      rstd[k] = row < M ? rstd_in[row] : 0.f;
+      const long long off = in ? (long long)row * d + col : 0;
+      cp_async16(&slot(st, k, 0), x + off, in);
+      cp_async16(&slot(st, k, 1), dy + off, in);
+      cp_async16(&slot(st, k, 2), dres ? dres + off : x, in && dres != nullptr);
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  const int first = (blockIdx.x * groups + grp) * R;
+  float mean[R], rstd[R], mean_n[R], rstd_n[R];
+  const auto stats = [&](int row0) {
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+      mean_n[k] = row0 + k < M ? mean_in[row0 + k] : 0.f;
+      rstd_n[k] = row0 + k < M ? rstd_in[row0 + k] : 0.f;
+    }
+  };
+#pragma unroll
+  for (int i = 0; i < S - 1; ++i) fetch(i, first + i * step);
+  stats(first);
+  int st = 0, buf = 0;
+  for (int row0 = first; row0 < M; row0 += step, buf ^= 1) {
+    // the stage that the round before has left
+    fetch(st == 0 ? S - 1 : st - 1, row0 + (S - 1) * step);
+#pragma unroll
+    for (int k = 0; k < R; ++k) { mean[k] = mean_n[k]; rstd[k] = rstd_n[k]; }
+    stats(row0 + step);
+    asm volatile("cp.async.wait_group %0;" ::"n"(S - 1) : "memory");
     float s[2 * R];
 #pragma unroll
     for (int k = 0; k < R; ++k) {
       float xh[8], g[8];
-      unpack8(xv[k], xh);
-      unpack8(dv[k], g);
+      unpack8(slot(st, k, 0), xh);
+      unpack8(slot(st, k, 1), g);
       float s1 = 0.f, s2 = 0.f;
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
@@ -255,21 +281,14 @@ layernorm_bwd_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* x, const floa
       }
       s[2 * k] = s1;
       s[2 * k + 1] = s2;
-      float r[8];
-      unpack8(rv[k], r);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) acc_r[j] += r[j];
     }
-    const float mine = warp_sums(s);
-    float* part = sh + (buf * groups + grp) * W * 2 * R;
+    const float sum = warp_sums(s);
+    float* part = exch + (buf * groups + grp) * W * 2 * R;
     constexpr int LANES = 32 / (2 * R);         // that hold the same sum
-    if ((lane & (LANES - 1)) == 0) part[(t >> 5) * 2 * R + lane / LANES] = mine;
+    if ((lane & (LANES - 1)) == 0) part[(t >> 5) * 2 * R + lane / LANES] = sum;
     // the buffer is written again two rounds on, when every warp of the group has passed the next round's barrier
     if constexpr (W == 1) __syncwarp();
     else asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "n"(32 * W) : "memory");
-    // unpacked again below: the floats from above would not fit
-#pragma unroll
-    for (int k = 0; k < R; ++k) { opaque(xv[k]); opaque(dv[k]); opaque(rv[k]); }
 #pragma unroll
     for (int i = 0; i < 2 * R; ++i) s[i] = 0.f;
 #pragma unroll
@@ -283,22 +302,32 @@ layernorm_bwd_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* x, const floa
 #pragma unroll
     for (int k = 0; k < R; ++k) {
       const int row = row0 + k;
-      if (!live || row >= M || !DSW_OK(row >= 0 && col + 8 <= d)) continue;
       const float m1 = s[2 * k] * inv_d, m2 = s[2 * k + 1] * inv_d;
       float xh[8], g[8], r[8], o[8];
-      unpack8(xv[k], xh);
-      unpack8(dv[k], g);
-      unpack8(rv[k], r);
+      unpack8(slot(st, k, 0), xh);          // read again: kept in registers from above they would not fit
+      unpack8(slot(st, k, 1), g);
+      unpack8(slot(st, k, 2), r);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) o[j] = rstd[k] * (g[j] * gm[j] - m1 - (xh[j] - mean[k]) * rstd[k] * m2) + r[j];
-      store8(dx + (long long)row * d + col, o);
+      for (int j = 0; j < 8; ++j) {
+        acc_r[j] += r[j];
+        o[j] = rstd[k] * (g[j] * gm[j] - m1 - (xh[j] - mean[k]) * rstd[k] * m2) + r[j];
+      }
+      if (live && row < M && DSW_OK(row >= 0 && col + 8 <= d)) store8(dx + (long long)row * d + col, o);
     }
+    st = st + 1 == S ? 0 : st + 1;
   }
-  __syncthreads();                              // the exchange buffers become the block's sums
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  float* sh = reinterpret_cast<float*>(ln_smem);               // [groups][3][d]
+  __syncthreads();                              // the stages become the block's sums
   if (live) {
-    float* out = sh + (long long)grp * 3 * d + col;
+    float4* out = reinterpret_cast<float4*>(sh + (long long)grp * 3 * d + col);
+    const int d4 = d / 4;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) { out[j] = acc_g[j]; out[d + j] = acc_b[j]; out[2 * d + j] = acc_r[j]; }
+    for (int h = 0; h < 2; ++h) {
+      out[h] = make_float4(acc_g[4 * h], acc_g[4 * h + 1], acc_g[4 * h + 2], acc_g[4 * h + 3]);
+      out[d4 + h] = make_float4(acc_b[4 * h], acc_b[4 * h + 1], acc_b[4 * h + 2], acc_b[4 * h + 3]);
+      out[2 * d4 + h] = make_float4(acc_r[4 * h], acc_r[4 * h + 1], acc_r[4 * h + 2], acc_r[4 * h + 3]);
+    }
   }
   __syncthreads();
   float* out = partial + (long long)blockIdx.x * 3 * d;
@@ -856,11 +885,24 @@ extern "C" int dsw_layernorm_bwd(const void* dy, const void* x, const float* gam
     const int W = (d + 255) / 256, groups = LN_BWD_MAX_WARPS / W, rows = groups * LN_BWD_ROWS;
     grid = (M + rows - 1) / rows;
     grid = grid < 1 ? 1 : grid > 148 ? 148 : grid;
-    // the block's sums, at most 48 KB; never less than the exchange buffers ([2][warps][2 rows] floats)
-    const size_t shmem = sizeof(float) * groups * 3 * d;
+    // stages (the block's sums, 12 bytes per column and group, fit in there afterwards) and exchange buffers
+    const auto shmem = [](int threads) {
+      return size_t(threads) * LN_BWD_STAGES * LN_BWD_ROWS * 48 + size_t(threads / 32) * 2 * 2 * LN_BWD_ROWS * sizeof(float);
+    };
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -2;
 #define LN_BWD(W_)                                                                                                           \
-  rc = launch(layernorm_bwd_kernel<W_>, grid, 32 * W_ * groups, shmem, st, 1, (const bf16*)dy, (const bf16*)x, gamma, mean, rstd, \
-              (const bf16*)dres, (bf16*)dx, scratch, M, d)
+  do {                                                                                                                       \
+    static bool attr[64] = {false};          /* the attribute is per device */                                               \
+    if (!attr[dev]) {                                                                                                        \
+      if (cudaFuncSetAttribute(layernorm_bwd_kernel<W_>, cudaFuncAttributeMaxDynamicSharedMemorySize,                        \
+                               int(shmem(32 * LN_BWD_MAX_WARPS))) != cudaSuccess)                                            \
+        return -2;                                                                                                           \
+      attr[dev] = true;                                                                                                      \
+    }                                                                                                                        \
+    rc = launch(layernorm_bwd_kernel<W_>, grid, 32 * W_ * groups, shmem(32 * W_ * groups), st, 1, (const bf16*)dy, (const bf16*)x, \
+                gamma, mean, rstd, (const bf16*)dres, (bf16*)dx, scratch, M, d);                                             \
+  } while (0)
     switch (W) {
       case 1: LN_BWD(1); break; case 2: LN_BWD(2); break; case 3: LN_BWD(3); break; case 4: LN_BWD(4); break;
       case 5: LN_BWD(5); break; case 6: LN_BWD(6); break; case 7: LN_BWD(7); break; default: LN_BWD(8); break;
