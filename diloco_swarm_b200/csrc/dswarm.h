@@ -83,11 +83,12 @@ int dsw_layernorm_fwd(const void* x, const float* gamma, const float* beta, void
 // The same of x + x_lo (x_lo: bf16 like x, or null).
 int dsw_layernorm_fwd_lo(const void* x, const void* x_lo, const float* gamma, const float* beta, void* y, float* mean,
                          float* rstd, int M, int d, float eps, cudaStream_t st);
-// Number of blocks dsw_layernorm_bwd launches for M rows = rows of scratch it needs.
+// The most blocks dsw_layernorm_bwd launches for M rows = rows of scratch it needs.
 int dsw_layernorm_bwd_blocks(int M);
 // dx = LayerNorm backward of dy (+ dres when given: the residual branch's gradient).  dgamma, dbeta and the
 // optional dres_sum (column sum of dres) are fp32 [d] and are accumulated (+=).
 // scratch: fp32 [dsw_layernorm_bwd_blocks(M)][3][d], contents irrelevant on entry.
+// In two calls with one scratch: dgamma null leaves the column sums there, dx null only joins them (on any stream).
 int dsw_layernorm_bwd(const void* dy, const void* x, const float* gamma, const float* mean, const float* rstd,
                       const void* dres, void* dx, float* dgamma, float* dbeta, float* dres_sum, float* scratch,
                       int M, int d, cudaStream_t st);

@@ -869,17 +869,20 @@ extern "C" int dsw_layernorm_bwd_blocks(int M) {
 
 // scratch: fp32 [dsw_layernorm_bwd_blocks(M)][3][d], contents irrelevant on entry.
 // dres_sum (optional): fp32 [d] += column sum of dres.
+// In two calls, so that the second can go to another stream: without dgamma only dx and the scratch are written, without
+// dx only the sums that are in the scratch (of the same M and d) are joined; dres_sum then asks for those of the first call's dres.
 extern "C" int dsw_layernorm_bwd(const void* dy, const void* x, const float* gamma, const float* mean,
                                  const float* rstd, const void* dres, void* dx, float* dgamma, float* dbeta,
                                  float* dres_sum, float* scratch, int M, int d, cudaStream_t st) {
-  if (d % 8 || d > 256 * LN_MAX_CHUNKS_ALL) return -10;
-  const int want = dres_sum != nullptr && dres != nullptr;
-  cudaError_t rc;
+  if (d % 8 || d > 256 * LN_MAX_CHUNKS_ALL || (dx == nullptr && dgamma == nullptr)) return -10;
+  const bool rows_part = dx != nullptr, sums_part = dgamma != nullptr;
+  float* const res_out = dres != nullptr || !rows_part ? dres_sum : nullptr;
+  cudaError_t rc = cudaSuccess;
   int grid;
   if (d <= 128) {
     grid = (M + 4 * LN_BWD_WARPS - 1) / (4 * LN_BWD_WARPS);      // two steps of two rows per warp at least
     grid = grid < 1 ? 1 : grid > 296 ? 296 : grid;
-    rc = launch(layernorm_bwd_narrow_kernel, grid, 32 * LN_BWD_WARPS, sizeof(float) * LN_BWD_WARPS * 3 * d, st, 1, (const bf16*)dy,
+    if (rows_part) rc = launch(layernorm_bwd_narrow_kernel, grid, 32 * LN_BWD_WARPS, sizeof(float) * LN_BWD_WARPS * 3 * d, st, 1, (const bf16*)dy,
                 (const bf16*)x, gamma, mean, rstd, (const bf16*)dres, (bf16*)dx, scratch, M, d);
   } else {
     const int W = (d + 255) / 256, groups = LN_BWD_MAX_WARPS / W, rows = groups * LN_BWD_ROWS;
@@ -903,15 +906,16 @@ extern "C" int dsw_layernorm_bwd(const void* dy, const void* x, const float* gam
     rc = launch(layernorm_bwd_kernel<W_>, grid, 32 * W_ * groups, shmem(32 * W_ * groups), st, 1, (const bf16*)dy, (const bf16*)x, \
                 gamma, mean, rstd, (const bf16*)dres, (bf16*)dx, scratch, M, d);                                             \
   } while (0)
-    switch (W) {
+    if (rows_part) switch (W) {
       case 1: LN_BWD(1); break; case 2: LN_BWD(2); break; case 3: LN_BWD(3); break; case 4: LN_BWD(4); break;
       case 5: LN_BWD(5); break; case 6: LN_BWD(6); break; case 7: LN_BWD(7); break; default: LN_BWD(8); break;
     }
 #undef LN_BWD
   }
   if (rc != cudaSuccess) return -3;
-  return launch(layernorm_bwd_finish_kernel, (3 * d + 31) / 32, dim3(32, 32), 0, st, 1, scratch, grid, d, dgamma, dbeta,
-                want ? dres_sum : nullptr) == cudaSuccess
+  if (!sums_part) return 0;
+  return launch(layernorm_bwd_finish_kernel, (3 * d + 31) / 32, dim3(32, 32), 0, st, 1, scratch, grid, d, dgamma, dbeta, res_out) ==
+                 cudaSuccess
              ? 0
              : -3;
 }
