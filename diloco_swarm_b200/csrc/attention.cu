@@ -384,9 +384,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, __nv_bfloat16
       if (!ok || !mbar_wait(o_full, (g - 1) & 1, abort_flag, status)) { ok = false; break; }
       tc_fence_after();
       const float inv = 1.f / l;
-      const int row0 = b * T + qi * ATT_BQ;                // first global row of this query tile
-      const bool in_seq = qi * ATT_BQ + r < T;             // a last tile may reach into the next sequence
-      __nv_bfloat16* dst = out + (long long)(row0 + r) * d + h * hs;
+      const bool in_seq = qi * ATT_BQ + r < T;             // a last tile may reach past the sequence's end
       uint32_t ov[2][32];
       tmem_ld_32x32(tmem_o + lane_addr, ov[0]);
       tmem_ld_32x32(tmem_o + lane_addr + 32, ov[1]);
@@ -394,16 +392,29 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, __nv_bfloat16
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(o_free);          // the next item's first product may overwrite the rows
+      // The warp's 32 rows pass through its own rows of the P tile, which no product reads any more, so that a store
+      // covers four whole rows of 128 bytes: a lane that stores its own row 16 bytes at a time touches 32 lines with
+      // every instruction (32 x 1024 tokens, 12 heads of 64: 135.6 -> 129.0 us; 16 x 1024: 72.9 -> 68.6).
+      uint8_t* so = sp + warp * 32 * 128;
 #pragma unroll
-      for (int i = 0; i < ATT_HS; i += 8)
-        if (i < hs && in_seq) {
-          const uint32_t* o = ov[i >> 5] + (i & 31);
-          *reinterpret_cast<uint4*>(dst + i) =
-              make_uint4(pack_bf16(__uint_as_float(o[0]) * inv, __uint_as_float(o[1]) * inv),
-                         pack_bf16(__uint_as_float(o[2]) * inv, __uint_as_float(o[3]) * inv),
-                         pack_bf16(__uint_as_float(o[4]) * inv, __uint_as_float(o[5]) * inv),
-                         pack_bf16(__uint_as_float(o[6]) * inv, __uint_as_float(o[7]) * inv));
-        }
+      for (int c = 0; c < 8; ++c) {
+        const uint32_t* o = ov[c >> 2] + (c & 3) * 8;
+        *reinterpret_cast<uint4*>(so + lane * 128 + ((c ^ (lane & 7)) << 4)) =
+            make_uint4(pack_bf16(__uint_as_float(o[0]) * inv, __uint_as_float(o[1]) * inv),
+                       pack_bf16(__uint_as_float(o[2]) * inv, __uint_as_float(o[3]) * inv),
+                       pack_bf16(__uint_as_float(o[4]) * inv, __uint_as_float(o[5]) * inv),
+                       pack_bf16(__uint_as_float(o[6]) * inv, __uint_as_float(o[7]) * inv));
+      }
+      __syncwarp();
+      const int ch = lane & 7, t0 = qi * ATT_BQ + warp * 32 + (lane >> 3);
+      __nv_bfloat16* dst = out + ((long long)b * T + t0) * d + h * hs + ch * 8;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int rl = i * 4 + (lane >> 3);
+        const uint4 w = *reinterpret_cast<const uint4*>(so + rl * 128 + ((ch ^ (rl & 7)) << 4));
+        if (t0 + i * 4 < T && ch * 8 < hs) *reinterpret_cast<uint4*>(dst + (long long)i * 4 * d) = w;
+      }
+      __syncwarp();                                // read out before the next item's P is written here
       // natural-log LSE of the scaled scores
       if (in_seq) lse_out[(long long)bh * T + qi * ATT_BQ + r] = (m + log2f(l)) * 0.6931471805599453f;
     }
