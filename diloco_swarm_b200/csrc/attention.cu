@@ -544,9 +544,47 @@ __device__ __forceinline__ void bwd_row_chunk(const uint32_t (&sv)[N], const uin
   }
 }
 
+// The two halves of bwd_row_chunk for a sequence of one tile, where a row's whole P and dP are at hand:
+// p[c] = P in place of S, the return value sum_c P dP, then dS with D = that sum over the whole row.
+template <int N>
+__device__ __forceinline__ float bwd_row_probs(uint32_t (&sv)[N], const uint32_t (&dpv)[N], int c0, int r, float scale_log2, float lse2) {
+  const f2 sc = f2_bcast(scale_log2), nl = f2_bcast(-lse2);
+  f2 sum = f2_bcast(0.f);
+#pragma unroll
+  for (int c = 0; c < N; c += 2) {
+    float x0, x1;
+    f2_split(f2_fma(f2_make(__uint_as_float(sv[c]), __uint_as_float(sv[c + 1])), sc, nl), x0, x1);
+    const float p0 = c0 + c <= r ? fast_exp2(x0) : 0.f, p1 = c0 + c + 1 <= r ? fast_exp2(x1) : 0.f;
+    sv[c] = __float_as_uint(p0);
+    sv[c + 1] = __float_as_uint(p1);
+    sum = f2_fma(f2_make(p0, p1), f2_make(c0 + c <= r ? __uint_as_float(dpv[c]) : 0.f, c0 + c + 1 <= r ? __uint_as_float(dpv[c + 1]) : 0.f),
+                 sum);
+  }
+  float a, b;
+  f2_split(sum, a, b);
+  return a + b;
+}
+template <int N>
+__device__ __forceinline__ void bwd_row_ds(const uint32_t (&p)[N], const uint32_t (&dpv)[N], uint32_t* pk_p, uint32_t* pk_ds, float Dr,
+                                           float scale) {
+  const f2 s2 = f2_bcast(scale), nd = f2_bcast(-Dr * scale);
+#pragma unroll
+  for (int c = 0; c < N; c += 2) {
+    const f2 pp = f2_make(__uint_as_float(p[c]), __uint_as_float(p[c + 1]));
+    const f2 u = f2_fma(f2_make(__uint_as_float(dpv[c]), __uint_as_float(dpv[c + 1])), s2, nd);
+    pk_p[c >> 1] = pack_bf16_f2(pp);
+    pk_ds[c >> 1] = pack_bf16_f2(f2_mul(pp, u));
+  }
+}
+
 constexpr int ATT_BWD_ROW_WARPS = 8;     // two per TMEM lane quarter: each thread takes half of its row's columns
 constexpr int ATT_BWD_THREADS = 32 * (ATT_BWD_ROW_WARPS + 3);    // + MMA issuer, TMA producer, dQ reducer
 
+// ONE: sequences of a single tile (T <= 128).  Every item is one step: D comes out of the row algebra, and dQ needs no
+// sum over kv tiles, so it leaves as bf16 with dK and dV.  No accumulator, and neither of the kernels around this one
+// (which clear it and compute D, and convert it): 64 x 128 tokens, 12 heads of 64, 51.5 -> 33.6 us; 16 x 128, 16 heads,
+// 27.1 -> 17.5; 1 x 128, 4 heads of 32, 20.6 -> 16.4.
+template <bool ONE>
 __global__ void __launch_bounds__(ATT_BWD_THREADS, 1)
 attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_constant__ CUtensorMap tmap_do,
                      const __grid_constant__ CUtensorMap tmap_dq, const __grid_constant__ CUtensorMap tmap_dkv,
@@ -768,6 +806,11 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
         const int b = bh / nh, h = bh - b * nh;
         for (int i = j; i < nq; ++i, ++g) {
           if (!mbar_wait(dq_staged, g & 1, abort_flag, status)) { ok = false; break; }
+          if constexpr (ONE) {
+            asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3, %4}], [%5];"
+                         ::"l"(&tmap_dkv), "r"(0), "r"(h), "r"(0), "r"(b), "r"(smem_u32(smem + L::DQ_OFF))
+                         : "memory");
+          } else
           for (int hh = 0; hh * 32 < hs; ++hh)          // 32 columns per head: the first staging half is the whole dQ tile
             asm volatile("cp.reduce.async.bulk.tensor.4d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2, %3, %4}], [%5];"
                          ::"l"(&tmap_dq), "r"(hh * 32), "r"(h), "r"(i * ATT_BQ), "r"(b),
@@ -822,9 +865,19 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
       // the previous reduction must have finished reading the staging tile
       if (gs > 0 && !mbar_wait(dq_stage_free, (gs - 1) & 1, abort_flag, status)) return false;
       ATT_TRACE(tr, 0, tslot);                // the previous reduction has let go of the staging tile
+      if constexpr (ONE) {          // one [128 x 64] bf16 tile
 #pragma unroll
-      for (int c = 0; c < 8; ++c)
-        *reinterpret_cast<uint4*>(sdq + r * 128 + ((c ^ (r & 7)) << 4)) = make_uint4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+        for (int c = 0; c < 4; ++c)
+          *reinterpret_cast<uint4*>(smem + L::DQ_OFF + r * 128 + (((half * 4 + c) ^ (r & 7)) << 4)) = make_uint4(
+              pack_bf16(__uint_as_float(v[8 * c]), __uint_as_float(v[8 * c + 1])),
+              pack_bf16(__uint_as_float(v[8 * c + 2]), __uint_as_float(v[8 * c + 3])),
+              pack_bf16(__uint_as_float(v[8 * c + 4]), __uint_as_float(v[8 * c + 5])),
+              pack_bf16(__uint_as_float(v[8 * c + 6]), __uint_as_float(v[8 * c + 7])));
+      } else {
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+          *reinterpret_cast<uint4*>(sdq + r * 128 + ((c ^ (r & 7)) << 4)) = make_uint4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+      }
       fence_proxy_async();
       __syncwarp();
       if (lane == 0) mbar_arrive(dq_staged);
@@ -854,7 +907,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
         // Rows past the end of the sequence (last tile of a length that is no multiple of 128), which the tiles hold
         // as zeros, have an infinite log-sum-exp: their P and dS come out as zeros and add nothing.
         const bool in_seq = i * ATT_BQ + r < T;
-        if (g == 0 && in_seq) { lse_next = lse[stat]; D_next = Dvec[stat]; }
+        if (g == 0 && in_seq) { lse_next = lse[stat]; D_next = ONE ? 0.f : Dvec[stat]; }
         const float lse2 = in_seq ? lse_next * 1.4426950408889634f : INFINITY;
         const float Dr = in_seq ? D_next : 0.f;
         ATT_TRACE(tr, 0, tslot);              // step start
@@ -862,7 +915,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
         tc_fence_after();
         {
           const int sn = it + 1 < steps ? ((i + 1) * ATT_BQ + r < T ? stat + ATT_BQ : -1) : stat_after;
-          if (sn >= 0) { lse_next = lse[sn]; D_next = Dvec[sn]; }
+          if (sn >= 0) { lse_next = lse[sn]; D_next = ONE ? 0.f : Dvec[sn]; }
         }
         ATT_TRACE(tr, 0, tslot);              // S, dP arrived
         // P and dS of this thread's 64 columns, in registers: the previous step's products may still be
@@ -878,6 +931,19 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
             tmem_ld_32x16(tm_dp + lane_addr + half * 64 + q * 16, raw[q][1]);
           }
           tmem_ld_wait();
+          if constexpr (ONE) {
+            // a row's other 64 columns are with the thread of the same lane four warps on
+            float* xch = reinterpret_cast<float*>(smem + L::DQ_OFF + ATT_TILE_BYTES);          // free: dQ is staged as bf16
+            float sum = 0.f;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) sum += bwd_row_probs(raw[q][0], raw[q][1], half * 64 + q * 16, r, scale_log2, lse2);
+            xch[half * 128 + r] = sum;
+            asm volatile("bar.sync %0, 64;" ::"r"(1 + q4) : "memory");
+            const float D = sum + xch[(half ^ 1) * 128 + r];
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+              bwd_row_ds(raw[q][0], raw[q][1], &pk_p[q >> 1][(q & 1) * 8], &pk_ds[q >> 1][(q & 1) * 8], D, scale);
+          } else
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
             const int c0 = half * 64 + q * 16;
@@ -1004,7 +1070,7 @@ extern "C" int dsw_attention_fwd(const void* qkv, void* out, float* lse, int B, 
 }
 
 // qkv, out, dout as in the forward; lse from the forward.  dqkv: bf16 [B*T, 3*d] (all of it is written).
-// dq_acc: fp32 scratch [B*T, d]; Dvec: fp32 scratch [B*nh*T].  Both are overwritten.
+// dq_acc: fp32 scratch [B*T, d]; Dvec: fp32 scratch [B*nh*T].  Both are overwritten where T > 128.
 extern "C" int dsw_attention_bwd(const void* qkv, const void* out, const void* dout, const float* lse, void* dqkv,
                                  float* dq_acc, float* Dvec, int B, int T, int nh, int hs, float scale, int* status,
                                  cudaStream_t st) {
@@ -1019,11 +1085,17 @@ extern "C" int dsw_attention_bwd(const void* qkv, const void* out, const void* d
   if (rc) return rc;
   static bool attr_set = false;
   if (!attr_set) {
-    if (cudaFuncSetAttribute(attention_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AttBwdSmem::TOTAL) !=
-        cudaSuccess)
+    if (cudaFuncSetAttribute(attention_bwd_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, AttBwdSmem::TOTAL) != cudaSuccess ||
+        cudaFuncSetAttribute(attention_bwd_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, AttBwdSmem::TOTAL) != cudaSuccess)
       return -2;
     attr_set = true;
   }
+  // persistent: one CTA per SM walks the work items
+  const int total = ((T + ATT_BK - 1) / ATT_BK) * B * nh;
+  const int G = total < att_num_sms() ? total : att_num_sms();
+  if (T <= ATT_BK)
+    return launch(attention_bwd_kernel<true>, G, ATT_BWD_THREADS, AttBwdSmem::TOTAL, st, 1, tq, tdo, tdq, tdkv, lse, Dvec, T, nh, B * nh,
+                  hs, scale, status, g_att_trace) == cudaSuccess ? 0 : -3;
   // D = rowsum(dO * O) per head, and the dQ accumulator zeroed in the same pass
   {
     const long long want = (rows * 32 + 255) / 256;
@@ -1032,10 +1104,7 @@ extern "C" int dsw_attention_bwd(const void* qkv, const void* out, const void* d
                (const __nv_bfloat16*)dout, Dvec, dq_acc, B, T, nh, hs) != cudaSuccess)
       return -3;
   }
-  // persistent: one CTA per SM walks the work items
-  const int total = ((T + ATT_BK - 1) / ATT_BK) * B * nh;
-  const int G = total < att_num_sms() ? total : att_num_sms();
-  if (launch(attention_bwd_kernel, G, ATT_BWD_THREADS, AttBwdSmem::TOTAL, st, 1, tq, tdo, tdq, tdkv, lse, Dvec,
+  if (launch(attention_bwd_kernel<false>, G, ATT_BWD_THREADS, AttBwdSmem::TOTAL, st, 1, tq, tdo, tdq, tdkv, lse, Dvec,
              T, nh, B * nh, hs, scale, status, g_att_trace) != cudaSuccess)
     return -3;
   return launch(attention_dq_convert_kernel, 148 * 4, 256, 0, st, 1, dq_acc, (__nv_bfloat16*)dqkv, (long long)B * T, d) ==
@@ -1048,7 +1117,8 @@ extern "C" int dsw_load_attention() {
   cudaFuncAttributes a;
   int bad = 0;
   bad |= cudaFuncGetAttributes(&a, attention_fwd_kernel) != cudaSuccess;
-  bad |= cudaFuncGetAttributes(&a, attention_bwd_kernel) != cudaSuccess;
+  bad |= cudaFuncGetAttributes(&a, attention_bwd_kernel<false>) != cudaSuccess;
+  bad |= cudaFuncGetAttributes(&a, attention_bwd_kernel<true>) != cudaSuccess;
   bad |= cudaFuncGetAttributes(&a, attention_bwd_prep_kernel) != cudaSuccess;
   bad |= cudaFuncGetAttributes(&a, attention_dq_convert_kernel) != cudaSuccess;
   return bad ? -1 : 0;

@@ -70,7 +70,7 @@ int dsw_gemm_set_trace(long long* buf);
 // h*hs of each).  out: bf16 [B*T, nh*hs]; lse: fp32 [B*nh*T].  hs is 64 or 32.
 int dsw_attention_fwd(const void* qkv, void* out, float* lse, int B, int T, int nh, int hs, float scale,
                       int* status, cudaStream_t st);
-// dqkv: bf16 like qkv.  dq_acc: fp32 [B*T, nh*hs] and Dvec: fp32 [B*nh*T] are work arrays, contents irrelevant.
+// dqkv: bf16 like qkv.  dq_acc: fp32 [B*T, nh*hs] and Dvec: fp32 [B*nh*T] are work arrays, contents irrelevant (not touched up to T = 128).
 int dsw_attention_bwd(const void* qkv, const void* out, const void* dout, const float* lse, void* dqkv,
                       float* dq_acc, float* Dvec, int B, int T, int nh, int hs, float scale, int* status,
                       cudaStream_t st);

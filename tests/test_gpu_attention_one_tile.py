@@ -1,0 +1,37 @@
+"""Attention backward of sequences of one tile (up to 128 tokens): one kernel, D from its own rows, dQ straight to bf16."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+# one token; one short of a warp's rows, of half a tile, of a tile; a whole tile; more items than SMs; both head sizes
+SHAPES = [(1, 1, 1, 64), (3, 31, 3, 64), (2, 63, 12, 64), (2, 127, 4, 32), (2, 128, 4, 32), (20, 128, 12, 64), (40, 65, 4, 32), (1, 129, 2, 64)]
+
+
+def _grads(qkv, dout, B, T, nh, hs):
+    x = qkv.double().view(B, T, 3, nh, hs).permute(2, 0, 3, 1, 4).detach().requires_grad_()
+    s = x[0] @ x[1].transpose(-1, -2) / hs ** 0.5
+    s = s.masked_fill(torch.ones(T, T, dtype=torch.bool, device=s.device).triu(1), float("-inf"))
+    o = s.softmax(-1) @ x[2]
+    o.backward(dout.double().view(B, T, nh, hs).transpose(1, 2))
+    return x.grad.permute(1, 3, 0, 2, 4).reshape(B * T, 3 * nh * hs)
+
+
+@pytest.mark.parametrize("B,T,nh,hs", SHAPES)
+def test_backward_against_64_bits(B, T, nh, hs):
+    from diloco_swarm_b200.ops._lib import Status
+    from diloco_swarm_b200.ops.attention import attention_bwd, attention_fwd
+    g = torch.Generator(device="cuda").manual_seed(T)
+    st, d = Status(torch.device("cuda")), nh * hs
+    qkv = torch.randn(B * T, 3 * d, device="cuda", generator=g).to(torch.bfloat16)
+    dout = torch.randn(B * T, d, device="cuda", generator=g).to(torch.bfloat16)
+    _, ctx = attention_fwd(qkv, B, T, nh, status=st)
+    got = attention_bwd(dout, ctx).double()
+    torch.cuda.synchronize()
+    st.raise_if_set()
+    want = _grads(qkv, dout, B, T, nh, hs)
+    for part in range(3):
+        a, b = got[:, part * d:(part + 1) * d], want[:, part * d:(part + 1) * d]
+        # P and dS are rounded to bf16 before the products, the results once more: each by at most 2^-9 of its value, in
+        # squares 2^-9 sqrt(2 / 3) of a result's norm and less; T = 1 has a zero gradient of q and k
+        assert (a - b).norm() <= 2 ** -8 * b.norm() + 1e-6 * (B * T * d) ** 0.5, "qkv"[part]
