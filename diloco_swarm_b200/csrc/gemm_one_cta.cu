@@ -33,6 +33,7 @@ int launch_bn(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& g, i
               cudaStream_t st) {
   switch (epi_class(g)) {
     case EPI_GELU: return launch_one<BN, NSTAGE, EPI_GELU>(ta, tb, g, num_sms, max_ctas, st);
+    case EPI_GELU_ONLY: return launch_one<BN, NSTAGE, EPI_GELU_ONLY>(ta, tb, g, num_sms, max_ctas, st);
     case EPI_RESID: return launch_one<BN, NSTAGE, EPI_RESID>(ta, tb, g, num_sms, max_ctas, st);
     case EPI_RESID_LO: return launch_one<BN, NSTAGE, EPI_RESID_LO>(ta, tb, g, num_sms, max_ctas, st);
     case EPI_MUL: return launch_one<BN, NSTAGE, EPI_MUL>(ta, tb, g, num_sms, max_ctas, st);
@@ -53,6 +54,7 @@ int load_bn() {
   int bad = 0;
   bad |= cudaFuncGetAttributes(&a, gemm_kernel<BN, NSTAGE, EPI_STORE>) != cudaSuccess;
   bad |= cudaFuncGetAttributes(&a, gemm_kernel<BN, NSTAGE, EPI_GELU>) != cudaSuccess;
+  bad |= cudaFuncGetAttributes(&a, gemm_kernel<BN, NSTAGE, EPI_GELU_ONLY>) != cudaSuccess;
   bad |= cudaFuncGetAttributes(&a, gemm_kernel<BN, NSTAGE, EPI_RESID>) != cudaSuccess;
   bad |= cudaFuncGetAttributes(&a, gemm_kernel<BN, NSTAGE, EPI_RESID_LO>) != cudaSuccess;
   bad |= cudaFuncGetAttributes(&a, gemm_kernel<BN, NSTAGE, EPI_MUL>) != cudaSuccess;

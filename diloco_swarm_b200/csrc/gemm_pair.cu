@@ -32,6 +32,7 @@ template <int BN>
 int launch_bn(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& g, int num_sms, int max_ctas, cudaStream_t st) {
   switch (epi_class(g)) {
     case EPI_GELU: return launch_pair_mode<BN, EPI_GELU>(ta, tb, g, num_sms, max_ctas, st);
+    case EPI_GELU_ONLY: return launch_pair_mode<BN, EPI_GELU_ONLY>(ta, tb, g, num_sms, max_ctas, st);
     case EPI_RESID: return launch_pair_mode<BN, EPI_RESID>(ta, tb, g, num_sms, max_ctas, st);
     case EPI_RESID_LO: return launch_pair_mode<BN, EPI_RESID_LO>(ta, tb, g, num_sms, max_ctas, st);
     case EPI_MUL: return launch_pair_mode<BN, EPI_MUL>(ta, tb, g, num_sms, max_ctas, st);
@@ -52,6 +53,7 @@ int load_bn() {
   int bad = 0;
   bad |= cudaFuncGetAttributes(&a, gemm_pair_kernel<BN, EPI_STORE>) != cudaSuccess;
   bad |= cudaFuncGetAttributes(&a, gemm_pair_kernel<BN, EPI_GELU>) != cudaSuccess;
+  bad |= cudaFuncGetAttributes(&a, gemm_pair_kernel<BN, EPI_GELU_ONLY>) != cudaSuccess;
   bad |= cudaFuncGetAttributes(&a, gemm_pair_kernel<BN, EPI_RESID>) != cudaSuccess;
   bad |= cudaFuncGetAttributes(&a, gemm_pair_kernel<BN, EPI_RESID_LO>) != cudaSuccess;
   bad |= cudaFuncGetAttributes(&a, gemm_pair_kernel<BN, EPI_MUL>) != cudaSuccess;
