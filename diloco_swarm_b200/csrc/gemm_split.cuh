@@ -16,7 +16,12 @@
 
 namespace dsw {
 
-constexpr int SPLIT_THREADS = 192;          // warps 0-3 epilogue (one TMEM lane quarter each), 4 TMA, 5 MMA
+// Warps 0-7 epilogue (two per TMEM lane quarter, each takes half of the tile's columns), 8 TMA, 9 MMA.  With one warp per
+// quarter, and the bias and the residual's low half asked for only when the sums were there, what followed the last
+// product was the longest part of a short launch: 120 x 3072 from 768 with GELU 8.3 -> 7.0 us, 120 x 2304 7.0 -> 6.3,
+// 120 x 512 from 128 4.9 -> 3.9, 120 x 768 from 3072 8.6 -> 8.0 (32 weight matrices in turn, one graph).
+constexpr int SPLIT_EPI_WARPS = 8, SPLIT_TMA_WARP = 8, SPLIT_MMA_WARP = 9;
+constexpr int SPLIT_THREADS = 32 * (SPLIT_EPI_WARPS + 2);
 
 template <int BN>
 struct SplitSmem {
@@ -25,7 +30,8 @@ struct SplitSmem {
   static constexpr int B_BYTES = BN * BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int RECV_OFFSET = NSTAGE * STAGE_BYTES;       // fp32 [source][BN / S / 4][128 rows][4]
-  static constexpr int BAR_OFFSET = RECV_OFFSET + BM * BN * 4;
+  static constexpr int BIAS_OFFSET = RECV_OFFSET + BM * BN * 4;  // per epilogue warp: the bias of its columns
+  static constexpr int BAR_OFFSET = BIAS_OFFSET + SPLIT_EPI_WARPS * (BN / 2) * 4;
   static constexpr int TOTAL = BAR_OFFSET + 128 + 1024;          // + alignment slack
 };
 
@@ -66,7 +72,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     mbar_fence_init();
     fence_proxy_async();
   }
-  if (warp == 5) {
+  if (warp == SPLIT_MMA_WARP) {
     tmem_alloc(tmem_holder, BN);
     tmem_relinquish();
   }
@@ -82,7 +88,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   const auto owner_of = [lgS](int u) { return (u << lgS) / U; };
   bool ok = true;
 
-  if (warp == 4) {
+  if (warp == SPLIT_TMA_WARP) {
     // ------------------------------------------------------------ producer (the whole warp, one lane issues)
     const auto load_b = [&](int i) {
       uint8_t* sb = smem + (i % NSTAGE) * L::STAGE_BYTES + L::A_BYTES;
@@ -124,7 +130,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       }
       __syncwarp();
     }
-  } else if (warp == 5) {
+  } else if (warp == SPLIT_MMA_WARP) {
     // ------------------------------------------------------------ MMA issuer (the whole warp, one lane issues)
     const uint32_t idesc = make_idesc_bf16(BM, BN, 0, g.b_mn_major);
     const uint32_t desc_hi = smem_desc_hi(1024);
@@ -146,26 +152,51 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     __syncwarp();
   }
 
-  if (warp < 4) {
-    // ------------------------------------------------------------ epilogue: thread = row
-    const int r = warp * 32 + lane, row = m0 + r;
+  if (warp < SPLIT_EPI_WARPS) {
+    // ------------------------------------------------------------ epilogue: thread = row and half of the columns
+    const int quarter = warp & 3, half = warp >> 2;
+    const int r = quarter * 32 + lane, row = m0 + r;
+    constexpr int UT = U / 2;           // units of this thread: u0 .. u0 + UT - 1
+    const int u0 = half * UT;
     constexpr bool EXTRA = MODE == EPI_RESID || MODE == EPI_MUL;
-    uint4 x[EXTRA ? U : 1];
+    uint4 x[EXTRA ? UT : 1], t[MODE == EPI_RESID ? UT : 1];
+    // Everything from global memory is asked for before the accumulator is waited for, the bias (older than the kernel
+    // before, like the weights) even before that kernel has ended.
+    float* bias = reinterpret_cast<float*>(smem + L::BIAS_OFFSET) + warp * (BN / 2);
+    const auto load_bias = [&] {
+#pragma unroll
+      for (int c = lane; c < BN / 2; c += 32) {
+        const int col = n0 + u0 * 8 + c;
+        bias[c] = g.bias != nullptr && col < g.N ? __ldg(g.bias + col) : 0.f;
+      }
+      __syncwarp();
+    };
+    if (g.b_static) load_bias();
     pdl_wait();
-    if constexpr (EXTRA) {              // on their way while the products run
+    if (!g.b_static) load_bias();
+    if constexpr (EXTRA) {
       const __nv_bfloat16* src = MODE == EPI_RESID ? g.resid : g.aux_in;
       const long long ld = MODE == EPI_RESID ? g.ldr : g.ldaux;
 #pragma unroll
-      for (int u = 0; u < U; ++u)
-        if (owner_of(u) == ks)
-          x[u] = row < g.M && n0 + u * 8 < g.N ? *reinterpret_cast<const uint4*>(src + (long long)row * ld + n0 + u * 8)
-                                               : make_uint4(0, 0, 0, 0);
+      for (int i = 0; i < UT; ++i) {
+        const int col = n0 + (u0 + i) * 8;
+        const bool in = owner_of(u0 + i) == ks && row < g.M && col < g.N;
+        x[i] = in ? *reinterpret_cast<const uint4*>(src + (long long)row * ld + col) : make_uint4(0, 0, 0, 0);
+        if constexpr (MODE == EPI_RESID)
+          t[i] = in && g.aux_in != nullptr ? *reinterpret_cast<const uint4*>(g.aux_in + (long long)row * g.ldaux + col)
+                                           : make_uint4(0, 0, 0, 0);
+      }
     }
     ok = mbar_wait(acc_full, 0, abort_flag, g.status);
     tc_fence_after();
-    uint32_t v[BN / 32][32];
-#pragma unroll
-    for (int c = 0; c < BN / 32; ++c) tmem_ld_32x32(tmem_base + (uint32_t(warp * 32) << 16) + c * 32, v[c]);
+    uint32_t v[UT * 8];
+    const uint32_t t_addr = tmem_base + (uint32_t(quarter * 32) << 16) + u0 * 8;
+    if constexpr (UT == 2) tmem_ld_32x16(t_addr, v);
+    else if constexpr (UT == 4) tmem_ld_32x32(t_addr, v);
+    else {
+      tmem_ld_32x32(t_addr, *reinterpret_cast<uint32_t(*)[32]>(v));
+      tmem_ld_32x32(t_addr + 32, *reinterpret_cast<uint32_t(*)[32]>(v + 32));
+    }
     tmem_ld_wait();
     uint8_t* recv = smem + L::RECV_OFFSET;
     if (S > 1) {
@@ -173,12 +204,12 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       const uint32_t recv_addr = smem_u32(recv);
       cluster_wait();
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int owner = owner_of(u);
+      for (int i = 0; i < UT; ++i) {
+        const int u = u0 + i, owner = owner_of(u);
         if (owner != ks) {
           const int slot = ks < owner ? ks : ks - 1;              // sources in rank order, the owner left out
           const uint32_t at = map_to_cta(recv_addr, owner) + ((slot * UW + (u - owner * UW)) * 2 * BM + r) * 16;
-          const uint32_t* q = &v[u / 4][(u & 3) * 8];
+          const uint32_t* q = &v[i * 8];
           st_cluster_v4(at, q[0], q[1], q[2], q[3]);
           st_cluster_v4(at + BM * 16, q[4], q[5], q[6], q[7]);
         }
@@ -187,10 +218,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       cluster_wait();
     }
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int col = n0 + u * 8;
+    for (int i = 0; i < UT; ++i) {
+      const int u = u0 + i, col = n0 + u * 8;
       if (owner_of(u) == ks && row < g.M && col < g.N && ok) {
-        const uint32_t* q = &v[u / 4][(u & 3) * 8];
+        const uint32_t* q = &v[i * 8];
         float f[8];
 #pragma unroll
         for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(q[e]);
@@ -200,8 +231,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           f[0] += lo.x; f[1] += lo.y; f[2] += lo.z; f[3] += lo.w;
           f[4] += hi.x; f[5] += hi.y; f[6] += hi.z; f[7] += hi.w;
         }
-        if (g.bias != nullptr) {
-          const float4 lo = __ldg(reinterpret_cast<const float4*>(g.bias + col)), hi = __ldg(reinterpret_cast<const float4*>(g.bias + col) + 1);
+        {
+          const float4 lo = *reinterpret_cast<const float4*>(bias + i * 8), hi = *reinterpret_cast<const float4*>(bias + i * 8 + 4);
           f[0] += lo.x; f[1] += lo.y; f[2] += lo.z; f[3] += lo.w;
           f[4] += hi.x; f[5] += hi.y; f[6] += hi.z; f[7] += hi.w;
         }
@@ -218,12 +249,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           if (g.aux_out != nullptr)
             *reinterpret_cast<uint4*>(g.aux_out + (long long)row * g.ldaux + col) = make_uint4(dw[0], dw[1], dw[2], dw[3]);
         } else {
-if constexpr (EXTRA) {
-            const uint32_t xu[4] = {x[u].x, x[u].y, x[u].z, x[u].w};
-            uint4 t = make_uint4(0, 0, 0, 0);
-            if (MODE == EPI_RESID && g.aux_in != nullptr)
-              t = *reinterpret_cast<const uint4*>(g.aux_in + (long long)row * g.ldaux + col);
-            const uint32_t tu[4] = {t.x, t.y, t.z, t.w};
+          if constexpr (EXTRA) {
+            const uint32_t xu[4] = {x[i].x, x[i].y, x[i].z, x[i].w};
+            uint32_t tu[4] = {0, 0, 0, 0};
+            if constexpr (MODE == EPI_RESID) { tu[0] = t[i].x; tu[1] = t[i].y; tu[2] = t[i].z; tu[3] = t[i].w; }
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
               const float2 b = unpack_bf16(xu[e]), c = unpack_bf16(tu[e]);
@@ -255,7 +284,7 @@ if constexpr (EXTRA) {
 
   tc_fence_before();
   __syncthreads();
-  if (warp == 5) {
+  if (warp == SPLIT_MMA_WARP) {
     tc_fence_after();
     tmem_dealloc(tmem_base, BN);
   }

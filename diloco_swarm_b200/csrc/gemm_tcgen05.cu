@@ -159,18 +159,20 @@ static int pick_bn(int M, int N, int K, int splits, int mode, bool derivative, i
 
 // Few rows: tile width and split of K for the cluster kernel (gemm_split.cuh), or 0 where the kernels for many rows are
 // the better ones.  The cluster kernel has one tile per CTA and no overlap of epilogue and main loop, so it only comes
-// into question while all its CTAs fit on the SMs at once.  Times in ns, fitted to launches of 24 to 2128 rows (N and K
-// of GPT-2 small, weights cold in L2): a k-block takes its share of the load latency, which falls with the stages in
-// flight; partial sums leave a CTA at 18 bytes per ns; a thread stores one row of the CTA's columns.
+// into question while all its CTAs fit on the SMs at once.  Times in ns, fitted to launches of 24 to 512 rows (N and K of
+// GPT-2 tiny, small and medium, weights cold in L2): a k-block takes its share of the load latency, which falls with the
+// stages in flight; the epilogue goes by the columns, and so does the exchange of partial sums, which takes another
+// barrier for every doubling of the cluster (768 x 3072: 64 wide, 8 splits 8.1 us, 32 wide, 4 splits 8.0; 1024 x 4096:
+// 10.4 and 9.3).
 static int pick_few_rows(int M, int N, int K, bool b_mn, int sms, double many_rows, int* split) {
   const int tm = (M + BM - 1) / BM, kb = (K + BK - 1) / BK;
-  double best = many_rows - 3400.0;             // what a launch takes besides the terms below
+  double best = many_rows - 2800.0;             // what a launch takes besides the terms below
   int bn = 0;
   for (int w = b_mn ? 64 : 32; w <= 128; w *= 2)
-    for (int s = 1; s <= 8 && s <= kb && w / s >= 8; s *= 2) {
+    for (int s = 1, lg = 0; s <= 8 && s <= kb && w / s >= 8; s *= 2, ++lg) {
       if ((long long)tm * ((N + w - 1) / w) * s > sms) continue;
-      const double per_kb = w == 32 ? 220.0 : w == 64 ? 280.0 : 300.0;
-      const double t = ((kb + s - 1) / s) * per_kb + (s > 1 ? 300.0 + 512.0 * w * (s - 1) / s / 18.0 : 0.0) + 25.0 * w / s;
+      const double per_kb = w == 32 ? 265.0 : w == 64 ? 350.0 : 330.0;
+      const double t = ((kb + s - 1) / s) * per_kb + 15.0 * w + (s > 1 ? 100.0 + 22.0 * w + 300.0 * lg : 0.0);
       if (t < best) { best = t; bn = w; *split = s; }
     }
   return bn;
