@@ -840,9 +840,10 @@ extern "C" int dsw_layernorm_fwd(const void* x, const float* gamma, const float*
 extern "C" int dsw_layernorm_fwd_lo(const void* x, const void* x_lo, const float* gamma, const float* beta, void* y, float* mean,
                                  float* rstd, int M, int d, float eps, cudaStream_t st) {
   if (d % 8 || d > 256 * LN_MAX_CHUNKS_ALL) return -10;
-  // two blocks per SM, several rows per warp when there are enough rows: gamma and beta are paid once per warp
+  // Two blocks per SM (narrow rows: four), each warp several rows when there are that many: gamma and beta are paid once
+  // per warp.  Fewer rows are spread out first: a second row per warp would only wait for the first one.
   const bool two_rows = d <= 128;
-  const int grid = two_rows ? grid_for(M, 32, 148 * 4) : grid_for(M, 16, 148 * 2);
+  const int grid = two_rows ? grid_for(M, 16, 148 * 4) : grid_for(M, 8, 148 * 2);
   cudaError_t rc;
 #define LN_FWD(NCH, LPR)                                                                                             \
   rc = x_lo ? launch(layernorm_fwd_kernel<NCH, true, LPR>, grid, 256, 0, st, 1, (const bf16*)x, (const bf16*)x_lo, gamma, beta, \
