@@ -463,7 +463,12 @@ struct AttBwdSmem {
   static constexpr int DS_OFF = P_OFF + 2 * ATT_TILE_BYTES;         // 2 k-blocks
   static constexpr int DQ_OFF = DS_OFF + 2 * ATT_TILE_BYTES;        // fp32 [2 halves][128 rows][32], 128-byte swizzled
   static constexpr int BAR_OFF = DQ_OFF + 2 * ATT_TILE_BYTES;
-  static constexpr int TOTAL = BAR_OFF + 256 + 1024;
+  static constexpr int SUM_OFF = BAR_OFF + 256;                     // column sums of dK and dV: fp32 [lane quarter][2][64]
+  // no room for alignment slack: the segment is declared 1024-aligned, and the kernel checks that it is
+  static constexpr int TOTAL = SUM_OFF + 4 * 2 * 64 * 4;
+  // sequences of one tile stage dQ in half of its buffer; behind that the exchange of row sums and dQ's column sums
+  static constexpr int ONE_XCH_OFF = DQ_OFF + ATT_TILE_BYTES;       // fp32 [2 halves][128 rows]
+  static constexpr int ONE_SUM_OFF = ONE_XCH_OFF + 1024;            // fp32 [lane quarter][64]
 };
 
 
@@ -503,20 +508,35 @@ attention_bwd_prep_kernel(const __nv_bfloat16* out, const __nv_bfloat16* dout,
   }
 }
 
-// dqkv[:, 0:d] = bf16(dq_acc)
-__global__ void __launch_bounds__(256)
-attention_dq_convert_kernel(const float* dq_acc, __nv_bfloat16* __restrict__ dqkv, long long rows, int d) {
+// dqkv[:, 0:d] = bf16(dq_acc); a thread keeps to eight columns, whose sums over all rows go to colsum (optional).
+// A block has `width` threads to a row, and a grid column for every 8 * width columns.
+__global__ void __launch_bounds__(512)
+attention_dq_convert_kernel(const float* dq_acc, __nv_bfloat16* __restrict__ dqkv, long long rows, int d, int width, float* colsum) {
+  extern __shared__ float cvt_sums[];                // [rows per step][8 * width], with colsum
   pdl_wait();
   pdl_launch();
-  const int per_row = d / 8;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < rows * per_row;
-       i += (long long)gridDim.x * blockDim.x) {
-    const long long row = i / per_row;
-    const int col = int(i - row * per_row) * 8;
+  const int per_step = blockDim.x / width, rl = threadIdx.x / width, cl = (threadIdx.x - rl * width) * 8;
+  const int col0 = blockIdx.y * width * 8, col = col0 + cl;
+  float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  const long long step = (long long)gridDim.x * per_step;
+#pragma unroll 4
+  for (long long row = (long long)blockIdx.x * per_step + rl; row < rows && col < d; row += step) {
     const float4 a = *reinterpret_cast<const float4*>(dq_acc + row * d + col);
     const float4 b = *reinterpret_cast<const float4*>(dq_acc + row * d + col + 4);
     *reinterpret_cast<uint4*>(dqkv + row * 3 * d + col) =
         make_uint4(pack_bf16(a.x, a.y), pack_bf16(a.z, a.w), pack_bf16(b.x, b.y), pack_bf16(b.z, b.w));
+    s[0] += a.x; s[1] += a.y; s[2] += a.z; s[3] += a.w;
+    s[4] += b.x; s[5] += b.y; s[6] += b.z; s[7] += b.w;
+  }
+  if (colsum == nullptr) return;
+  float4* mine = reinterpret_cast<float4*>(cvt_sums + rl * width * 8 + cl);
+  mine[0] = make_float4(s[0], s[1], s[2], s[3]);
+  mine[1] = make_float4(s[4], s[5], s[6], s[7]);
+  __syncthreads();
+  for (int c = threadIdx.x; c < width * 8 && col0 + c < d; c += blockDim.x) {
+    float v = 0.f;
+    for (int k = 0; k < per_step; ++k) v += cvt_sums[k * width * 8 + c];
+    atomicAdd(colsum + col0 + c, v);
   }
 }
 
@@ -580,6 +600,21 @@ __device__ __forceinline__ void bwd_row_ds(const uint32_t (&p)[N], const uint32_
 constexpr int ATT_BWD_ROW_WARPS = 8;     // two per TMEM lane quarter: each thread takes half of its row's columns
 constexpr int ATT_BWD_THREADS = 32 * (ATT_BWD_ROW_WARPS + 3);    // + MMA issuer, TMA producer, dQ reducer
 
+// Column sums of dqkv (a bias gradient) meet in global memory by bulk reductions that the reducer warp issues, 64 columns
+// of 32 rows each: a row thread that adds to global memory itself finds its next barrier waiting for that (32 x 1024
+// tokens: 328 -> 387 us; with a warp of its own that read the staged tiles 396, since the next item's P waits for it).
+__device__ __forceinline__ void bulk_add(float* to, const void* from, int bytes) {
+  asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(to), "r"(smem_u32(from)), "r"(bytes)
+               : "memory");
+}
+// The sums over the warp's 32 rows of a thread's 32 columns, a column per lane.
+__device__ __forceinline__ float column_sum(const uint32_t (&row)[32]) {
+  float v[32];
+#pragma unroll
+  for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(row[i]);
+  return warp_sums(v);
+}
+
 // ONE: sequences of a single tile (T <= 128).  Every item is one step: D comes out of the row algebra, and dQ needs no
 // sum over kv tiles, so it leaves as bf16 with dK and dV.  No accumulator, and neither of the kernels around this one
 // (which clear it and compute D, and convert it): 64 x 128 tokens, 12 heads of 64, 51.5 -> 33.6 us; 16 x 128, 16 heads,
@@ -589,10 +624,14 @@ __global__ void __launch_bounds__(ATT_BWD_THREADS, 1)
 attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_constant__ CUtensorMap tmap_do,
                      const __grid_constant__ CUtensorMap tmap_dq, const __grid_constant__ CUtensorMap tmap_dkv,
                      const float* lse, const float* Dvec, int T, int nh, int n_bh, int hs,
-                     float scale, int* status, long long* trace) {
+                     float scale, float* colsum, int* status, long long* trace) {
   using L = AttBwdSmem;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = smem_raw;
+  if (smem_u32(smem) & 1023) {
+    if (threadIdx.x == 0 && status) atomicCAS(status, 0, ST_BAD_ARG);
+    return;
+  }
   // Persistent: one CTA per SM walks work items (kv tile, batch*head).  The per-step barriers complete one
   // phase per step, kv_full / kv_empty / dkv_free one per item, counted over the life of the CTA
   // (g = steps done, w = items done).
@@ -810,6 +849,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
             asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3, %4}], [%5];"
                          ::"l"(&tmap_dkv), "r"(0), "r"(h), "r"(0), "r"(b), "r"(smem_u32(smem + L::DQ_OFF))
                          : "memory");
+            for (int q = 0; q < 4 && colsum != nullptr; ++q) bulk_add(colsum + h * hs, smem + L::ONE_SUM_OFF + q * 256, hs * 4);
           } else
           for (int hh = 0; hh * 32 < hs; ++hh)          // 32 columns per head: the first staging half is the whole dQ tile
             asm volatile("cp.reduce.async.bulk.tensor.4d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2, %3, %4}], [%5];"
@@ -829,6 +869,8 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
                          ::"l"(&tmap_dkv), "r"(0), "r"((which + 1) * nh + h), "r"(j * ATT_BK), "r"(b),
                            "r"(smem_u32(smem + L::P_OFF + which * ATT_TILE_BYTES))
                          : "memory");
+          for (int q = 0; q < 8 && colsum != nullptr; ++q)
+            bulk_add(colsum + ((q & 1) + 1) * d + h * hs, smem + L::SUM_OFF + q * 256, hs * 4);
           asm volatile("cp.async.bulk.commit_group;" ::: "memory");
           asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
           mbar_arrive(dkv_stored);
@@ -866,6 +908,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
       if (gs > 0 && !mbar_wait(dq_stage_free, (gs - 1) & 1, abort_flag, status)) return false;
       ATT_TRACE(tr, 0, tslot);                // the previous reduction has let go of the staging tile
       if constexpr (ONE) {          // one [128 x 64] bf16 tile
+        if (colsum != nullptr) reinterpret_cast<float*>(smem + L::ONE_SUM_OFF)[q4 * 64 + half * 32 + lane] = column_sum(v);
 #pragma unroll
         for (int c = 0; c < 4; ++c)
           *reinterpret_cast<uint4*>(smem + L::DQ_OFF + r * 128 + (((half * 4 + c) ^ (r & 7)) << 4)) = make_uint4(
@@ -933,7 +976,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
           tmem_ld_wait();
           if constexpr (ONE) {
             // a row's other 64 columns are with the thread of the same lane four warps on
-            float* xch = reinterpret_cast<float*>(smem + L::DQ_OFF + ATT_TILE_BYTES);          // free: dQ is staged as bf16
+            float* xch = reinterpret_cast<float*>(smem + L::ONE_XCH_OFF);
             float sum = 0.f;
 #pragma unroll
             for (int q = 0; q < 4; ++q) sum += bwd_row_probs(raw[q][0], raw[q][1], half * 64 + q * 16, r, scale_log2, lse2);
@@ -999,6 +1042,11 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(dkv_free);          // the next item's first products may overwrite the sums
+      if (colsum != nullptr) {          // rows past the sequence are zeros
+        float* sums = reinterpret_cast<float*>(smem + L::SUM_OFF) + q4 * 128 + half * 32 + lane;
+        sums[0] = column_sum(vk);
+        sums[64] = column_sum(vv);
+      }
       // staged as two 128-byte-swizzled [128 x 64] bf16 tiles (dK, dV) in the P buffer, which nothing reads any more; the
       // reducer warp stores them with one bulk copy each
 #pragma unroll
@@ -1093,9 +1141,11 @@ extern "C" int dsw_attention_bwd(const void* qkv, const void* out, const void* d
   // persistent: one CTA per SM walks the work items
   const int total = ((T + ATT_BK - 1) / ATT_BK) * B * nh;
   const int G = total < att_num_sms() ? total : att_num_sms();
+  float* const colsum = reinterpret_cast<uintptr_t>(tl_launch.colsum) & 15 ? nullptr : tl_launch.colsum;          // for bulk reductions
+  if (colsum != nullptr) tl_launch.colsum = nullptr;
   if (T <= ATT_BK)
     return launch(attention_bwd_kernel<true>, G, ATT_BWD_THREADS, AttBwdSmem::TOTAL, st, 1, tq, tdo, tdq, tdkv, lse, Dvec, T, nh, B * nh,
-                  hs, scale, status, g_att_trace) == cudaSuccess ? 0 : -3;
+                  hs, scale, colsum, status, g_att_trace) == cudaSuccess ? 0 : -3;
   // D = rowsum(dO * O) per head, and the dQ accumulator zeroed in the same pass
   {
     const long long want = (rows * 32 + 255) / 256;
@@ -1105,10 +1155,12 @@ extern "C" int dsw_attention_bwd(const void* qkv, const void* out, const void* d
       return -3;
   }
   if (launch(attention_bwd_kernel<false>, G, ATT_BWD_THREADS, AttBwdSmem::TOTAL, st, 1, tq, tdo, tdq, tdkv, lse, Dvec,
-             T, nh, B * nh, hs, scale, status, g_att_trace) != cudaSuccess)
+             T, nh, B * nh, hs, scale, colsum, status, g_att_trace) != cudaSuccess)
     return -3;
-  return launch(attention_dq_convert_kernel, 148 * 4, 256, 0, st, 1, dq_acc, (__nv_bfloat16*)dqkv, (long long)B * T, d) ==
-                 cudaSuccess
+  const int width = d / 8 < 512 ? d / 8 : 512, per_step = 512 / width;
+  const long long steps = (rows + per_step - 1) / per_step;
+  return launch(attention_dq_convert_kernel, dim3(unsigned(steps < 296 ? steps : 296), (d + 8 * width - 1) / (8 * width)), width * per_step,
+                colsum ? sizeof(float) * per_step * width * 8 : 0, st, 1, dq_acc, (__nv_bfloat16*)dqkv, rows, d, width, colsum) == cudaSuccess
              ? 0
              : -3;
 }

@@ -183,26 +183,6 @@ constexpr int LN_BWD_ROWS = 2;
 constexpr int LN_BWD_MAX_WARPS = 16;
 constexpr int LN_BWD_STAGES = 2;
 
-// Sums v[i] over the warp for N values, a power of two: lane l ends with the sum of value l / (32 / N).
-template <int N>
-__device__ __forceinline__ float warp_sums(float (&v)[N]) {
-  const int lane = threadIdx.x & 31;
-  int o = 16;
-#pragma unroll
-  for (int n = N / 2; n >= 1; n >>= 1, o >>= 1) {
-    const bool up = lane & o;
-#pragma unroll
-    for (int i = 0; i < n; ++i) {
-      const float keep = up ? v[i + n] : v[i], send = up ? v[i] : v[i + n];
-      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-    }
-  }
-  float s = v[0];
-#pragma unroll
-  for (; o >= 1; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  return s;
-}
-
 // 16 bytes global -> shared, zeros where !in.
 __device__ __forceinline__ void cp_async16(void* dst, const void* src, bool in) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(in ? 16 : 0) : "memory");

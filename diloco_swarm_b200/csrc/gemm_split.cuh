@@ -220,6 +220,11 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 #pragma unroll
     for (int i = 0; i < UT; ++i) {
       const int u = u0 + i, col = n0 + u * 8;
+      float out8[MODE == EPI_MUL ? 8 : 1];          // of a row that exists, else zeros
+      if constexpr (MODE == EPI_MUL) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) out8[e] = 0.f;
+      }
       if (owner_of(u) == ks && row < g.M && col < g.N && ok) {
         const uint32_t* q = &v[i * 8];
         float f[8];
@@ -262,6 +267,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           }
 #pragma unroll
           for (int e = 0; e < 4; ++e) w[e] = pack_bf16(f[2 * e], f[2 * e + 1]);
+          if constexpr (MODE == EPI_MUL) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) out8[e] = f[e];
+          }
           if (MODE == EPI_RESID && g.aux_out != nullptr) {
             uint32_t lo[4];
 #pragma unroll
@@ -274,6 +283,12 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         }
         *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(g.out) + (long long)row * g.ldo + col) =
             make_uint4(w[0], w[1], w[2], w[3]);
+      }
+      if constexpr (MODE == EPI_MUL) {
+        if (g.colsum != nullptr && owner_of(u) == ks && col < g.N) {          // the same for the whole warp
+          const float sum = warp_sums(out8);
+          if ((lane & 3) == 0) atomicAdd(g.colsum + col + (lane >> 2), sum);
+        }
       }
     }
   } else if (S > 1) {

@@ -274,6 +274,10 @@ extern "C" int dsw_gemm_bf16(const void* A, long long lda, int a_mn_major, const
   // 16384 x 768 from 50304: 992 -> 864; neutral where one wave does, no difference between 4 and 24)
   g.group = 8;
   g.b_static = tl_launch.static_b;
+  if (mode == EPI_MUL) {
+    g.colsum = tl_launch.colsum;
+    tl_launch.colsum = nullptr;
+  }
   g.trace = g_gemm_trace;
   if (few_rows) return launch_split(bn - 1000, ta, tb, g, stream);
   if (bn == 512 || bn == 384) return launch_pair(bn == 512 ? 256 : 128, ta, tb, g, num_sms[dev], max_ctas, stream);

@@ -20,6 +20,10 @@ namespace dsw {
 struct LaunchMode {
   bool pdl = false;           // the predecessor in the stream is a kernel of this library and nothing lies in between
   bool static_b = false;      // a GEMM's B operand (the weights) is older than the predecessor
+  // fp32, one per output column, to which the next launch adds the sums over all rows of what it writes (dsw_gemm_bf16 with
+  // the multiply epilogue: of its output; dsw_attention_bwd: of dqkv).  A launcher that does so sets it to null again; one
+  // that does not leaves it, and the caller has dsw_colsum_accum read the output once more.
+  float* colsum = nullptr;
 };
 extern thread_local LaunchMode tl_launch;
 

@@ -345,6 +345,16 @@ struct Run {
     return 0;
   }
 
+  // The next launch is asked to add its output's column sums (a bias gradient) to `to`: in its epilogue or beside its
+  // products, in place of a pass that reads dh or dqkv once more.  Its sums meet in atomics, which a deterministic
+  // backward does without.
+  void sum_columns(float* to) const { dsw::tl_launch.colsum = deterministic ? nullptr : to; }
+  bool columns_unsummed() const {
+    const bool left = deterministic || dsw::tl_launch.colsum != nullptr;
+    dsw::tl_launch.colsum = nullptr;
+    return left;
+  }
+
   // The rows' part of a LayerNorm backward on the main stream; its column sums, which nothing in the backward reads, are
   // joined on the side stream once it may go on (ln_sums after a fork): some 3 us less of the chain per LayerNorm.
   int ln_rows(const void* dy, const bf16* x, const float* w, const float* mu, const float* rs, const bf16* dres, bf16* dx,
@@ -373,10 +383,12 @@ struct Run {
   int block_bwd(int l, const Block& b, const bf16* x, const Saved& v, const Scratch& c, const bf16* dx2, bf16* dx0) {
     const int d = s.d, p = l & 1;
     TRY(wait(marks->done[p]));
+    sum_columns(b.db[W_FC]);
     LAUNCH(gemm(dx2, b.w[W_PR], false, 4 * d, d, c.dh[p], DSW_EPI_MUL, nullptr, nullptr, nullptr, v.h, M));
+    const bool sum_dh = columns_unsummed();
     TRY(fork());
     SIDE(wgrad(dx2, v.g, d, 4 * d, b.dw[W_PR], M, side()));
-    SIDE(dsw_colsum_accum(c.dh[p], 4 * d, b.db[W_FC], M, 4 * d, side()));
+    if (sum_dh) SIDE(dsw_colsum_accum(c.dh[p], 4 * d, b.db[W_FC], M, 4 * d, side()));
     SIDE(wgrad(c.dh[p], v.ln2, 4 * d, d, b.dw[W_FC], M, side()));
     LAUNCH(gemm(c.dh[p], b.w[W_FC], false, d, 4 * d, c.dln, DSW_EPI_STORE, nullptr, nullptr, nullptr, nullptr, M));
     // the column sum of dx2 (bias gradient of the MLP's second projection) comes out of the LayerNorm backward as well
@@ -385,9 +397,11 @@ struct Run {
     TRY(fork());
     SIDE(ln_sums(c.ln[2 * p], b.dln2_w, b.dln2_b, b.db[W_PR]));
     SIDE(wgrad(c.dx1[p], v.att, d, d, b.dw[W_O], M, side()));
+    sum_columns(b.db[W_QKV]);
     LAUNCH(dsw_attention_bwd(v.qkv, v.att, c.datt, v.lse, c.dqkv[p], c.dq_acc, c.dvec, B, T, s.nh, d / s.nh, scale(), s.status, st));
+    const bool sum_dqkv = columns_unsummed();
     TRY(fork());
-    SIDE(dsw_colsum_accum(c.dqkv[p], 3 * d, b.db[W_QKV], M, 3 * d, side()));
+    if (sum_dqkv) SIDE(dsw_colsum_accum(c.dqkv[p], 3 * d, b.db[W_QKV], M, 3 * d, side()));
     SIDE(wgrad(c.dqkv[p], v.ln1, 3 * d, d, b.dw[W_QKV], M, side()));
     LAUNCH(gemm(c.dqkv[p], b.w[W_QKV], false, d, 3 * d, c.dln, DSW_EPI_STORE, nullptr, nullptr, nullptr, nullptr, M));
     LAUNCH(ln_rows(c.dln, x, b.ln1_w, v.mu1, v.rs1, c.dx1[p], dx0, c.ln[2 * p + 1]));
