@@ -56,7 +56,11 @@ class B200Engine:
         self.layers = split_layers(cfg.n_layer, S, config.swarm.layer_split, cfg.n_embd, cfg.vocab_size)[world.stage]
         self.specs = stage_param_specs(cfg, self.layers, self.is_first, self.is_last)
         self.act_dtype = BF16
-        self.status = Status(device)
+        # What the host reads of a step, in one copy: sum of squares, norm and clip coefficient of the gradient, then the
+        # step's loss and the kernels' status word (an int32).
+        self.report = torch.zeros(8, dtype=F32, device=device)
+        self.stats, self.loss_slot = self.report[:4], self.report[4]
+        self.status = Status(device, self.report[5:6].view(torch.int32))
         d = cfg.n_embd
         assert d % 8 == 0 and cfg.vocab_size % 8 == 0, "n_embd and vocab_size must be multiples of 8"
         assert cfg.bias, "the b200 engine implements the reference's bias=True model"
@@ -83,7 +87,6 @@ class B200Engine:
         self.w16 = torch.zeros(self.n, dtype=BF16, device=device)
         self.m = torch.zeros(self.n, dtype=F32, device=device)
         self.v = torch.zeros(self.n, dtype=F32, device=device)
-        self.stats = torch.zeros(4, dtype=F32, device=device)        # sumsq, norm, clip coef
         self.count_buf = torch.zeros(1, dtype=F32, device=device)
         for key, gname, shape in self.specs:
             self.p32(key).copy_(init_tensor(gname, shape, config.train.seed, cfg.n_layer))
@@ -201,8 +204,14 @@ class B200Engine:
             n -= self.cfg.block_size * self.cfg.n_embd
         return n
 
-    def check_status(self) -> None:
-        self.status.raise_if_set()
+    def step_report(self) -> Tuple[float, float]:
+        """(what ``loss_slot`` holds, gradient norm) of a step whose work is over; raises what ``check_status`` raises."""
+        host = self.report.cpu()
+        self.check_status(int(host.view(torch.int32)[5]))
+        return float(host[4]), float(host[1])
+
+    def check_status(self, code: Optional[int] = None) -> None:
+        self.status.raise_if_set(code)
         if self._canary_every_step:
             for buf in self.symmetric_buffers():
                 buf.check_canaries()

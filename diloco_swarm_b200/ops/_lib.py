@@ -158,8 +158,9 @@ class Status:
     give up on a wait write a code here instead of hanging; ``raise_if_set``
     turns it into an exception at a point where the host synchronises anyway."""
 
-    def __init__(self, device: torch.device):
-        self.word = torch.zeros(1, dtype=torch.int32, device=device)
+    def __init__(self, device: torch.device, word: Optional[torch.Tensor] = None):
+        """``word``: one int32 on the device that holds zero, where the caller keeps the word among its own numbers."""
+        self.word = torch.zeros(1, dtype=torch.int32, device=device) if word is None else word
 
     @property
     def ptr(self) -> int:
@@ -168,8 +169,10 @@ class Status:
     def read(self) -> int:
         return int(self.word.item())
 
-    def raise_if_set(self) -> None:
-        code = self.read()
+    def raise_if_set(self, code: Optional[int] = None) -> None:
+        """``code``: the word's value where the host has read it already."""
+        if code is None:
+            code = self.read()
         if code != 0:
             self.word.zero_()
             raise RuntimeError(f"kernel status {code}: {_STATUS_TEXT.get(code, 'unknown')}")

@@ -350,7 +350,8 @@ class Trainer:
         _, ops = self._plan(step, 0, forward_only=False)
         dev = self._stage_batch(batch)
         tokens_per_mb = self.mbs * self.seq
-        loss_acc = torch.zeros((), dtype=torch.float32, device=self.device)
+        slot = getattr(eng, "loss_slot", None)          # where the engine reports a step in one read
+        loss_acc = torch.zeros((), dtype=torch.float32, device=self.device) if slot is None else slot.zero_()
         H = cfg.swarm.sync_every_n_steps
         do_sync = (H > 0 and step % H == 0) or step == self.num_train_steps
         # the static plan tells which backward is this rank's last one: when the step ends with a
@@ -394,10 +395,15 @@ class Trainer:
         self.last_enqueue_s = time.time() - start   # host time to queue the whole step
         if comm.device_async and w.world_size > 1 and not failed:
             self._watch_step_deadline(step, start + cfg.train.step_timeout)
-        loss_val = float(loss_acc.item())      # the step's one device-to-host read
+        if slot is None:
+            loss_val = float(loss_acc.item())
         if self.device.type == "cuda":
             torch.cuda.synchronize(self.device)
-        eng.check_status()
+        if slot is None:
+            eng.check_status()
+        else:
+            loss_val, dev_norm = eng.step_report()      # the step's one device-to-host read
+            norm = dev_norm if applied else norm
         self.last_phase_ms = self.timer.collect()
         if do_sync and applied:
             self.last_sync_phase_ms = dict(self.last_phase_ms)     # phases of the latest step that synchronised
