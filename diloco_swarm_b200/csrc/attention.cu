@@ -451,6 +451,8 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, __nv_bfloat16
 // Q / dO stage), dQ.  TMA warp (likewise): K / V of the item into the buffer of its parity,
 // Q / dO pairs into two stages.  Reducer warp (one lane): one bulk reduce-add per staged dQ tile, two bulk stores per item for dK / dV
 // (staged by the row warps in the P buffer).
+// Sequences of one tile have an instantiation of their own (ONE, below); where the caller asks for the column sums of dqkv
+// (LaunchMode::colsum), the row threads leave those of dK and dV in shared memory with the tiles.
 // Every wait is bounded; a wait that runs out sets the CTA's abort flag and the status word.
 struct AttBwdSmem {
   static constexpr int KV_BYTES = 2 * ATT_TILE_BYTES;               // K_j then V_j
