@@ -46,6 +46,9 @@ int dsw_gemm_bf16(const void* A, long long lda, int a_mn_major, const void* B, l
                   int M, int N, int K, int mode, int split_k, void* out, long long ldo, const float* bias,
                   const void* resid, long long ldr, void* aux_out, const void* aux_in, long long ldaux, int bn,
                   int max_ctas, int* status, cudaStream_t stream);
+// The kernel (bn) that dsw_gemm_bf16 takes for activations [M,K] times a weight matrix when bn is 0, and the split of K of
+// the cluster kernel; derivative: DSW_EPI_GELU with aux_out.  Host arithmetic only.
+int dsw_gemm_choice(int M, int N, int K, int mode, int b_mn_major, int derivative, int sms, int* split);
 // Masked cross-entropy of logits = A [M,K] W[N,K]^T in pieces that never hold the logits: dsw_head_lse writes partial
 // log-sum-exps (fp32 [ceil(N / 64)][M]) and the target's logit (fp32 [M]), dsw_head_rows (elementwise.cu) joins them into
 // the loss and one 16-byte record per row, dsw_head_dlogits computes the logits again and stores scale / count *

@@ -159,20 +159,22 @@ static int pick_bn(int M, int N, int K, int splits, int mode, bool derivative, i
 
 // Few rows: tile width and split of K for the cluster kernel (gemm_split.cuh), or 0 where the kernels for many rows are
 // the better ones.  The cluster kernel has one tile per CTA and no overlap of epilogue and main loop, so it only comes
-// into question while all its CTAs fit on the SMs at once.  Times in ns, fitted to launches of 24 to 512 rows (N and K of
-// GPT-2 tiny, small and medium, weights cold in L2): a k-block takes its share of the load latency, which falls with the
-// stages in flight; the epilogue goes by the columns, and so does the exchange of partial sums, which takes another
-// barrier for every doubling of the cluster (768 x 3072: 64 wide, 8 splits 8.1 us, 32 wide, 4 splits 8.0; 1024 x 4096:
-// 10.4 and 9.3).
+// into question while all its CTAs fit on the SMs at once.  Times in ns, fitted to launches of 24 to 2128 rows (N and K of
+// GPT-2 small): a k-block takes its share of the load latency, which falls with the stages in flight; partial sums leave
+// a CTA at 18 bytes per ns; a thread stores one row of the CTA's columns.  Checked on 585 calls, forward and backward of
+// widths 128 to 1600 with 24 to 2128 rows, weights cold in L2: 6735 us for all of them, 6522 with the best choice for each.
+// A fit to the smaller models alone (launches cheaper, exchange dearer) came to 6739 and left the cluster kernel where it
+// was the better one (24 x 3072 from 1024: 8.1 -> 9.5 us, 64 x 3840 from 1280: 8.7 -> 9.2), though it won others (128 x
+// 1024 from 4096: 10.8 -> 9.1).
 static int pick_few_rows(int M, int N, int K, bool b_mn, int sms, double many_rows, int* split) {
   const int tm = (M + BM - 1) / BM, kb = (K + BK - 1) / BK;
-  double best = many_rows - 2800.0;             // what a launch takes besides the terms below
+  double best = many_rows - 3400.0;             // what a launch takes besides the terms below
   int bn = 0;
   for (int w = b_mn ? 64 : 32; w <= 128; w *= 2)
-    for (int s = 1, lg = 0; s <= 8 && s <= kb && w / s >= 8; s *= 2, ++lg) {
+    for (int s = 1; s <= 8 && s <= kb && w / s >= 8; s *= 2) {
       if ((long long)tm * ((N + w - 1) / w) * s > sms) continue;
-      const double per_kb = w == 32 ? 265.0 : w == 64 ? 350.0 : 330.0;
-      const double t = ((kb + s - 1) / s) * per_kb + 15.0 * w + (s > 1 ? 100.0 + 22.0 * w + 300.0 * lg : 0.0);
+      const double per_kb = w == 32 ? 220.0 : w == 64 ? 280.0 : 300.0;
+      const double t = ((kb + s - 1) / s) * per_kb + (s > 1 ? 300.0 + 512.0 * w * (s - 1) / s / 18.0 : 0.0) + 25.0 * w / s;
       if (t < best) { best = t; bn = w; *split = s; }
     }
   return bn;
@@ -206,9 +208,25 @@ static int pick_wgrad(int M, int N, int K, int bn, int sms, int* split, int most
   return best;
 }
 
+// The kernel of a call that leaves it to the library, as dsw_gemm_bf16's bn.  few: the cluster kernel may be taken.
+static int pick_kernel(int M, int N, int K, int mode, bool b_mn, bool derivative, bool few, int sms, int* split) {
+  double cost;
+  const int bn = pick_bn(M, N, K, *split, mode, derivative, sms, &cost);
+  const int width = few ? pick_few_rows(M, N, K, b_mn, sms, cost, split) : 0;
+  return width ? 1000 + width : bn;
+}
+
 }  // namespace dsw
 
 using namespace dsw;
+
+// The kernel that dsw_gemm_bf16 takes on a GPU of that many SMs for an activation [M, K] times a weight matrix, and the
+// cluster kernel's split of K.  Host arithmetic only.
+extern "C" int dsw_gemm_choice(int M, int N, int K, int mode, int b_mn_major, int derivative, int sms, int* split) {
+  if (M <= 0 || N <= 0 || K <= 0 || mode < EPI_STORE || mode > EPI_MUL || sms <= 0) return -10;
+  *split = 1;
+  return pick_kernel(M, N, K, mode, b_mn_major != 0, derivative != 0, true, sms, split);
+}
 
 static long long* g_gemm_trace = nullptr;
 // Tracing build only: register (or clear) a device buffer of 512 int64 for the kernels' timeline stamps.
@@ -244,12 +262,9 @@ extern "C" int dsw_gemm_bf16(const void* A, long long lda, int a_mn_major, const
   }
   if (split_k == 0) split_k = 1;
   if (bn == 0) {
-    double cost;
-    bn = pick_bn(M, N, K, split_k, mode, aux_out != nullptr, num_sms[dev], &cost);
-    if (split_k == 1 && mode <= EPI_MUL && !a_mn_major && max_ctas == 0 && default_max_ctas() == 0) {
-      const int width = pick_few_rows(M, N, K, b_mn_major != 0, num_sms[dev], cost, &split_k);
-      if (width) { bn = 1000 + width; few_rows = true; }
-    }
+    const bool few = split_k == 1 && mode <= EPI_MUL && !a_mn_major && max_ctas == 0 && default_max_ctas() == 0;
+    bn = pick_kernel(M, N, K, mode, b_mn_major != 0, aux_out != nullptr, few, num_sms[dev], &split_k);
+    few_rows = bn > 1000;
   }
   if (max_ctas == 0) max_ctas = default_max_ctas();
   CUtensorMap ta, tb;

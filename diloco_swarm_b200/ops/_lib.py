@@ -40,6 +40,7 @@ _SIGS = {
     "dsw_head_rows": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_void_p, c_int, c_int, c_void_p,
                       c_void_p],
     "dsw_head_dlogits": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p],
+    "dsw_gemm_choice": [c_int, c_int, c_int, c_int, c_int, c_int, c_int, ctypes.POINTER(c_int)],
     "dsw_gemm_partials": [c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_int, ctypes.POINTER(c_int), c_void_p, c_void_p],
     "dsw_sum_partials_bf16": [c_void_p, c_int, c_void_p, c_ll, c_void_p],
     "dsw_cast_f32_bf16": [c_void_p, c_void_p, c_ll, c_void_p],
