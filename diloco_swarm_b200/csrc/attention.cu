@@ -468,11 +468,23 @@ struct AttBwdSmem {
   static constexpr int SUM_OFF = BAR_OFF + 256;                     // column sums of dK and dV: fp32 [lane quarter][2][64]
   // no room for alignment slack: the segment is declared 1024-aligned, and the kernel checks that it is
   static constexpr int TOTAL = SUM_OFF + 4 * 2 * 64 * 4;
-  // sequences of one tile stage dQ in half of its buffer; behind that the exchange of row sums and dQ's column sums
-  static constexpr int ONE_XCH_OFF = DQ_OFF + ATT_TILE_BYTES;       // fp32 [2 halves][128 rows]
-  static constexpr int ONE_SUM_OFF = ONE_XCH_OFF + 1024;            // fp32 [lane quarter][64]
+  // sequences of one tile stage dQ in half of its buffer; behind that dQ's column sums, D, and rows of O for the next D
+  static constexpr int ONE_SUM_OFF = DQ_OFF + ATT_TILE_BYTES;       // fp32 [lane quarter][64]
+  static constexpr int ONE_D_OFF = ONE_SUM_OFF + 1024;              // fp32 [2 item parities][128 rows]
+  static constexpr int ONE_O_OFF = ONE_D_OFF + 1024;                // [8 row warps][3 pieces][32 lanes] of 16 bytes
 };
 
+// Dot product of eight bf16 values, fp32 sums.
+__device__ __forceinline__ float dot8(const uint4& a, const uint4& g) {
+  const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, gw[4] = {g.x, g.y, g.z, g.w};
+  float v = 0.f;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const float2 x = unpack_bf16(aw[k]), y = unpack_bf16(gw[k]);
+    v += x.x * y.x + x.y * y.y;
+  }
+  return v;
+}
 
 // D[bh, t] = sum_c dO[t, h*hs + c] * O[t, h*hs + c], and dq_acc[t, :] = 0.  One warp per token row: 16-byte
 // loads, one head's hs columns lie in hs/8 neighbouring lanes (hs = 64 or 32), which a few shuffles add up.
@@ -494,13 +506,7 @@ attention_bwd_prep_kernel(const __nv_bfloat16* out, const __nv_bfloat16* dout,
       const int u = u0 + lane;
       float v = 0.f;
       if (u < chunks) {
-        const uint4 a = po[u], g = pg[u];
-        const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, gw[4] = {g.x, g.y, g.z, g.w};
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const float2 x = unpack_bf16(aw[k]), y = unpack_bf16(gw[k]);
-          v += x.x * y.x + x.y * y.y;
-        }
+        v = dot8(po[u], pg[u]);
         pz[2 * u] = make_float4(0.f, 0.f, 0.f, 0.f);
         pz[2 * u + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
       }
@@ -566,39 +572,6 @@ __device__ __forceinline__ void bwd_row_chunk(const uint32_t (&sv)[N], const uin
   }
 }
 
-// The two halves of bwd_row_chunk for a sequence of one tile, where a row's whole P and dP are at hand:
-// p[c] = P in place of S, the return value sum_c P dP, then dS with D = that sum over the whole row.
-template <int N>
-__device__ __forceinline__ float bwd_row_probs(uint32_t (&sv)[N], const uint32_t (&dpv)[N], int c0, int r, float scale_log2, float lse2) {
-  const f2 sc = f2_bcast(scale_log2), nl = f2_bcast(-lse2);
-  f2 sum = f2_bcast(0.f);
-#pragma unroll
-  for (int c = 0; c < N; c += 2) {
-    float x0, x1;
-    f2_split(f2_fma(f2_make(__uint_as_float(sv[c]), __uint_as_float(sv[c + 1])), sc, nl), x0, x1);
-    const float p0 = c0 + c <= r ? fast_exp2(x0) : 0.f, p1 = c0 + c + 1 <= r ? fast_exp2(x1) : 0.f;
-    sv[c] = __float_as_uint(p0);
-    sv[c + 1] = __float_as_uint(p1);
-    sum = f2_fma(f2_make(p0, p1), f2_make(c0 + c <= r ? __uint_as_float(dpv[c]) : 0.f, c0 + c + 1 <= r ? __uint_as_float(dpv[c + 1]) : 0.f),
-                 sum);
-  }
-  float a, b;
-  f2_split(sum, a, b);
-  return a + b;
-}
-template <int N>
-__device__ __forceinline__ void bwd_row_ds(const uint32_t (&p)[N], const uint32_t (&dpv)[N], uint32_t* pk_p, uint32_t* pk_ds, float Dr,
-                                           float scale) {
-  const f2 s2 = f2_bcast(scale), nd = f2_bcast(-Dr * scale);
-#pragma unroll
-  for (int c = 0; c < N; c += 2) {
-    const f2 pp = f2_make(__uint_as_float(p[c]), __uint_as_float(p[c + 1]));
-    const f2 u = f2_fma(f2_make(__uint_as_float(dpv[c]), __uint_as_float(dpv[c + 1])), s2, nd);
-    pk_p[c >> 1] = pack_bf16_f2(pp);
-    pk_ds[c >> 1] = pack_bf16_f2(f2_mul(pp, u));
-  }
-}
-
 constexpr int ATT_BWD_ROW_WARPS = 8;     // two per TMEM lane quarter: each thread takes half of its row's columns
 constexpr int ATT_BWD_THREADS = 32 * (ATT_BWD_ROW_WARPS + 3);    // + MMA issuer, TMA producer, dQ reducer
 
@@ -617,16 +590,76 @@ __device__ __forceinline__ float column_sum(const uint32_t (&row)[32]) {
   return warp_sums(v);
 }
 
-// ONE: sequences of a single tile (T <= 128).  Every item is one step: D comes out of the row algebra, and dQ needs no
-// sum over kv tiles, so it leaves as bf16 with dK and dV.  No accumulator, and neither of the kernels around this one
-// (which clear it and compute D, and convert it): 64 x 128 tokens, 12 heads of 64, 51.5 -> 33.6 us; 16 x 128, 16 heads,
-// 27.1 -> 17.5; 1 x 128, 4 heads of 32, 20.6 -> 16.4.
+// D = rowsum(dO O) of 16 rows of a sequence of one tile by a warp, LPR lanes (hs / 8) to a row, added up in the order of
+// attention_bwd_prep_kernel.  piece(i, r, o, g): a lane's eight values of O and dO in row r (of the 16), the i-th it has.
+template <int LPR, class F>
+__device__ __forceinline__ void row_dots16(float* to, int lane, F&& piece) {
+  constexpr int N = LPR / 2, RPI = 32 / LPR;          // pieces, rows per piece
+  float v[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    uint4 o, g;
+    piece(i, i * RPI + lane / LPR, o, g);
+    v[i] = dot8(o, g);
+  }
+  // over the lanes of a row, each step with half as many rows
+#pragma unroll
+  for (int n = N / 2, x = LPR / 2; n >= 1; n >>= 1, x >>= 1) {
+    const bool up = lane & x;
+#pragma unroll
+    for (int i = 0; i < n; ++i) {
+      const float keep = up ? v[i + n] : v[i], send = up ? v[i] : v[i + n];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, x);
+    }
+  }
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+  if (!(lane & 1)) to[((lane & (LPR - 1)) >> 1) * RPI + lane / LPR] = v[0];
+}
+
+// A row warp's 16 rows of D, item by item.  O of an item is asked for a whole item ahead: three of a lane's four pieces
+// into shared memory, where there is no room for four, and one into registers; dO is in its stage.  Loaded when they are
+// wanted, the pieces came from DRAM while the row warps waited (64 x 128 tokens, 12 heads of 64: 45 us a launch, this
+// way 37; by a warp of its own 38).
+template <int LPR>
+struct ItemDots {
+  static __device__ __forceinline__ uint4 load(const __nv_bfloat16* p, int r, int d, int rows, int lane) {
+    return r < rows ? *reinterpret_cast<const uint4*>(p + (long long)r * d + (lane & (LPR - 1)) * 8) : make_uint4(0, 0, 0, 0);
+  }
+  // o, g: the head's columns of the first of the 16 rows; `rows` of them lie within the sequence
+  static __device__ __forceinline__ void first(const __nv_bfloat16* o, const __nv_bfloat16* g, int d, int rows, float* to, int lane) {
+    row_dots16<LPR>(to, lane, [&](int, int r, uint4& ov, uint4& gv) { ov = load(o, r, d, rows, lane); gv = load(g, r, d, rows, lane); });
+  }
+  static __device__ __forceinline__ void fetch(const __nv_bfloat16* o, int d, int rows, uint4* mine, uint4& last, int lane) {
+#pragma unroll
+    for (int i = 0; i < LPR / 2; ++i) {
+      const int r = i * (32 / LPR) + lane / LPR;
+      if (i < 3) cp_async16(mine + i * 32, r < rows ? o + (long long)r * d + (lane & (LPR - 1)) * 8 : o, r < rows);
+      else       last = load(o, r, d, rows, lane);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  // tile: the 128 rows of dO, row0: the first of the 16
+  static __device__ __forceinline__ void finish(const uint8_t* tile, int row0, const uint4* mine, const uint4& last, float* to, int lane) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    row_dots16<LPR>(to, lane, [&](int i, int r, uint4& ov, uint4& gv) {
+      ov = i < 3 ? mine[i * 32] : last;
+      gv = *reinterpret_cast<const uint4*>(tile + (row0 + r) * 128 + (((lane & (LPR - 1)) ^ ((row0 + r) & 7)) << 4));
+    });
+  }
+};
+
+// ONE: sequences of a single tile (T <= 128).  Every item is one step, and dQ needs no sum over kv tiles, so it leaves as
+// bf16 with dK and dV.  D is computed by the row warps, 16 rows each, that of the next item under the products of this one.
+// No accumulator, and neither of the kernels around this one (which clear it and compute D, and convert it).  The results
+// are those of the three kernels, bit for bit: 64 x 128 tokens, 12 heads of 64, 45.7 -> 36.8 us; 16 x 128, 16 heads, 23.9 ->
+// 16.9; 200 x 64, 12 heads, 95.4 -> 84.0; 1 x 128, 4 heads of 32, 11.0 -> 7.6.  (With D as the row sum of P dP, which is
+// another rounding and has the two warps of a row wait for each other inside the row algebra: 33.1, 15.4, 77.0, 7.6.)
 template <bool ONE>
 __global__ void __launch_bounds__(ATT_BWD_THREADS, 1)
 attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_constant__ CUtensorMap tmap_do,
                      const __grid_constant__ CUtensorMap tmap_dq, const __grid_constant__ CUtensorMap tmap_dkv,
-                     const float* lse, const float* Dvec, int T, int nh, int n_bh, int hs,
-                     float scale, float* colsum, int* status, long long* trace) {
+                     const __nv_bfloat16* out, const __nv_bfloat16* dout, const float* lse, const float* Dvec, int T, int nh,
+                     int n_bh, int hs, float scale, float* colsum, int* status, long long* trace) {
   using L = AttBwdSmem;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw;
@@ -652,7 +685,8 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
   uint64_t* dq_stage_free = bars + 15; // the reduction of this step's dQ has read the staging tile
   uint64_t* dkv_staged = bars + 16;    // dK, dV of the item staged in the P buffer (8 warps arrive; hs = 64)
   uint64_t* dkv_stored = bars + 17;    // their bulk stores have read the P buffer
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 18);
+  uint64_t* dots_full = bars + 18;     // D of the item in shared memory (8 warps arrive; ONE)
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 19);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -673,6 +707,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
     mbar_init(sdp_read, ATT_BWD_ROW_WARPS);
     mbar_init(dq_staged, ATT_BWD_ROW_WARPS); mbar_init(dq_stage_free, 1);
     mbar_init(dkv_staged, ATT_BWD_ROW_WARPS); mbar_init(dkv_stored, 1);
+    mbar_init(dots_full, ATT_BWD_ROW_WARPS);
     *abort_flag = 0;
     mbar_fence_init();
     fence_proxy_async();
@@ -929,19 +964,52 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
       ATT_TRACE(tr, 0, tslot);                // staged
       return true;
     };
+    // this warp's 16 rows of D of an item (ONE)
+    const int dot_row = q4 * 32 + half * 16;
+    uint4* const o_mine = reinterpret_cast<uint4*>(smem + L::ONE_O_OFF) + warp * 96 + lane;
+    uint4 o_last = make_uint4(0, 0, 0, 0);
+    const auto dots_at = [&](int bh) {          // the first of the rows, or of the sequence where they lie behind it
+      return ((long long)(bh / nh) * T + (dot_row < T ? dot_row : 0)) * d + (bh % nh) * hs;
+    };
+    const auto dots_to = [&](uint32_t item) { return reinterpret_cast<float*>(smem + L::ONE_D_OFF) + (item & 1) * 128 + dot_row; };
+    const auto dots_done = [&] {
+      __syncwarp();
+      if (lane == 0) mbar_arrive(dots_full);
+    };
+    const auto dots_fetch = [&](int bh) {
+      if (hs == 64) ItemDots<8>::fetch(out + dots_at(bh), d, T - dot_row, o_mine, o_last, lane);
+      else          ItemDots<4>::fetch(out + dots_at(bh), d, T - dot_row, o_mine, o_last, lane);
+    };
+    const auto dots_finish = [&](uint32_t item) -> bool {
+      const int s = item % L::QSTAGES;
+      if (!mbar_wait(&q_full[s], (item / L::QSTAGES) & 1, abort_flag, status)) return false;
+      const uint8_t* tile = smem + L::DO_OFF + s * ATT_TILE_BYTES;
+      if (hs == 64) ItemDots<8>::finish(tile, dot_row, o_mine, o_last, dots_to(item), lane);
+      else          ItemDots<4>::finish(tile, dot_row, o_mine, o_last, dots_to(item), lane);
+      dots_done();
+      return true;
+    };
+    if (ONE) {                        // the CTA's first item, while its tiles are on their way
+      int idx;
+      att_item(0, cta, G, total, idx);          // there is one: G <= total
+      const long long at = dots_at(idx % n_bh);
+      if (hs == 64) ItemDots<8>::first(out + at, dout + at, d, T - dot_row, dots_to(0), lane);
+      else          ItemDots<4>::first(out + at, dout + at, d, T - dot_row, dots_to(0), lane);
+      dots_done();
+    }
     for (int rr = 0; rr < rounds && ok; ++rr) {
       int idx;
       if (!att_item(rr, cta, G, total, idx)) continue;
       const int j = idx / n_bh, bh = idx % n_bh;
-      const int b = bh / nh, h = bh - b * nh;
       const int steps = nq - j;
       // where the next item's first step finds its row statistics (-1: this is the CTA's last item)
-      int stat_after = -1;
+      int stat_after = -1, bh_after = -1;
       for (int r2 = rr + 1; r2 < rounds; ++r2) {
         int idx2;
         if (att_item(r2, cta, G, total, idx2)) {
           // a row past the end of the sequence: its statistics are never used
-          stat_after = (idx2 / n_bh) * ATT_BQ + r < T ? (idx2 % n_bh) * T + (idx2 / n_bh) * ATT_BQ + r : -1;
+          bh_after = idx2 % n_bh;
+          stat_after = (idx2 / n_bh) * ATT_BQ + r < T ? bh_after * T + (idx2 / n_bh) * ATT_BQ + r : -1;
           break;
         }
       }
@@ -952,15 +1020,20 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
         // Rows past the end of the sequence (last tile of a length that is no multiple of 128), which the tiles hold
         // as zeros, have an infinite log-sum-exp: their P and dS come out as zeros and add nothing.
         const bool in_seq = i * ATT_BQ + r < T;
-        if (g == 0 && in_seq) { lse_next = lse[stat]; D_next = ONE ? 0.f : Dvec[stat]; }
+        if (g == 0 && in_seq) { lse_next = lse[stat]; if (!ONE) D_next = Dvec[stat]; }
         const float lse2 = in_seq ? lse_next * 1.4426950408889634f : INFINITY;
-        const float Dr = in_seq ? D_next : 0.f;
+        float Dr = in_seq ? D_next : 0.f;
+        if (ONE && bh_after >= 0) dots_fetch(bh_after);
         ATT_TRACE(tr, 0, tslot);              // step start
         if (!mbar_wait(sdp_full, g & 1, abort_flag, status)) { ok = false; break; }
+        if constexpr (ONE) {          // a buffer is written again when every warp has handed over the item in between
+          if (!mbar_wait(dots_full, g & 1, abort_flag, status)) { ok = false; break; }
+          Dr = reinterpret_cast<const float*>(smem + L::ONE_D_OFF)[(g & 1) * 128 + r];
+        }
         tc_fence_after();
         {
           const int sn = it + 1 < steps ? ((i + 1) * ATT_BQ + r < T ? stat + ATT_BQ : -1) : stat_after;
-          if (sn >= 0) { lse_next = lse[sn]; D_next = ONE ? 0.f : Dvec[sn]; }
+          if (sn >= 0) { lse_next = lse[sn]; if (!ONE) D_next = Dvec[sn]; }
         }
         ATT_TRACE(tr, 0, tslot);              // S, dP arrived
         // P and dS of this thread's 64 columns, in registers: the previous step's products may still be
@@ -976,19 +1049,6 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
             tmem_ld_32x16(tm_dp + lane_addr + half * 64 + q * 16, raw[q][1]);
           }
           tmem_ld_wait();
-          if constexpr (ONE) {
-            // a row's other 64 columns are with the thread of the same lane four warps on
-            float* xch = reinterpret_cast<float*>(smem + L::ONE_XCH_OFF);
-            float sum = 0.f;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) sum += bwd_row_probs(raw[q][0], raw[q][1], half * 64 + q * 16, r, scale_log2, lse2);
-            xch[half * 128 + r] = sum;
-            asm volatile("bar.sync %0, 64;" ::"r"(1 + q4) : "memory");
-            const float D = sum + xch[(half ^ 1) * 128 + r];
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-              bwd_row_ds(raw[q][0], raw[q][1], &pk_p[q >> 1][(q & 1) * 8], &pk_ds[q >> 1][(q & 1) * 8], D, scale);
-          } else
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
             const int c0 = half * 64 + q * 16;
@@ -1030,6 +1090,8 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(pds_full);
+        // the next item's D, under the products of this one
+        if (ONE && bh_after >= 0 && !dots_finish(g + 1)) { ok = false; break; }
         // the previous step's dQ leaves after the hand-over, off the critical path (the next dQ product
         // waits for its read-out)
         if (it > 0 && !drain_dq(g - 1)) { ok = false; break; }
@@ -1146,8 +1208,8 @@ extern "C" int dsw_attention_bwd(const void* qkv, const void* out, const void* d
   float* const colsum = reinterpret_cast<uintptr_t>(tl_launch.colsum) & 15 ? nullptr : tl_launch.colsum;          // for bulk reductions
   if (colsum != nullptr) tl_launch.colsum = nullptr;
   if (T <= ATT_BK)
-    return launch(attention_bwd_kernel<true>, G, ATT_BWD_THREADS, AttBwdSmem::TOTAL, st, 1, tq, tdo, tdq, tdkv, lse, Dvec, T, nh, B * nh,
-                  hs, scale, colsum, status, g_att_trace) == cudaSuccess ? 0 : -3;
+    return launch(attention_bwd_kernel<true>, G, ATT_BWD_THREADS, AttBwdSmem::TOTAL, st, 1, tq, tdo, tdq, tdkv, (const __nv_bfloat16*)out,
+                  (const __nv_bfloat16*)dout, lse, Dvec, T, nh, B * nh, hs, scale, colsum, status, g_att_trace) == cudaSuccess ? 0 : -3;
   // D = rowsum(dO * O) per head, and the dQ accumulator zeroed in the same pass
   {
     const long long want = (rows * 32 + 255) / 256;
@@ -1156,8 +1218,8 @@ extern "C" int dsw_attention_bwd(const void* qkv, const void* out, const void* d
                (const __nv_bfloat16*)dout, Dvec, dq_acc, B, T, nh, hs) != cudaSuccess)
       return -3;
   }
-  if (launch(attention_bwd_kernel<false>, G, ATT_BWD_THREADS, AttBwdSmem::TOTAL, st, 1, tq, tdo, tdq, tdkv, lse, Dvec,
-             T, nh, B * nh, hs, scale, colsum, status, g_att_trace) != cudaSuccess)
+  if (launch(attention_bwd_kernel<false>, G, ATT_BWD_THREADS, AttBwdSmem::TOTAL, st, 1, tq, tdo, tdq, tdkv, (const __nv_bfloat16*)out,
+             (const __nv_bfloat16*)dout, lse, Dvec, T, nh, B * nh, hs, scale, colsum, status, g_att_trace) != cudaSuccess)
     return -3;
   const int width = d / 8 < 512 ? d / 8 : 512, per_step = 512 / width;
   const long long steps = (rows + per_step - 1) / per_step;

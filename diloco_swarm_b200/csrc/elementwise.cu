@@ -183,11 +183,6 @@ constexpr int LN_BWD_ROWS = 2;
 constexpr int LN_BWD_MAX_WARPS = 16;
 constexpr int LN_BWD_STAGES = 2;
 
-// 16 bytes global -> shared, zeros where !in.
-__device__ __forceinline__ void cp_async16(void* dst, const void* src, bool in) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(in ? 16 : 0) : "memory");
-}
-
 // W: warps per group = ceil(d / 256), blockDim.x / (32 W) groups per block.
 template <int W>
 __global__ void __launch_bounds__(32 * LN_BWD_MAX_WARPS, 1)

@@ -16,6 +16,12 @@ list of step counts: an item is one kv tile of one (batch, head), a step one que
   reducer   per step: wait dq_staged, bulk reduce-add out of the staging tile, arrive dq_stage_free; per
             item: wait dkv_staged, two bulk stores out of the P buffer, arrive dkv_stored
 
+The staged tiles of dQ and of dK / dV carry their column sums along (``sums``).  Sequences of one tile (``one``: every item
+is one step) are walked by two row roles, each with half of the rows and columns, as the eight row warps of the kernel:
+
+  rows      D of the first item at the start, that of the next item (reads its dO: q_full) after pds_full; arrive dots_full;
+            before an item's P / dS: wait dots_full, read D of all rows from the buffer of the item's parity
+
 ``drop`` names one wait or one ordering to leave out (a mutation): the tests use it to show that the checker
 sees the race or the deadlock that the wait prevents.
 """
@@ -28,20 +34,27 @@ from .protocol_sim import Barrier, Sim
 
 MUTATIONS = ("rows_wait_dq_full", "mma_wait_sdp_read", "mma_wait_dq_free", "producer_wait_q_empty",
              "producer_wait_kv_empty", "rows_wait_dq_stage_free", "rows_wait_dkv_stored", "q_empty_before_dk")
+ONE_MUTATIONS = ("rows_wait_dots_full", "rows_wait_q_full", "rows_wait_dkv_stored", "mma_wait_sdp_read", "one_dots_buffer")
+# The reducer takes the staged dQ of an item before its dK / dV, and the row threads wait for those (dkv_stored).
+ONE_IMPLIED = ("rows_wait_dq_stage_free",)
 # A wait of the kernel that the model shows to be implied by another: the issuer's wait for dkv_free before an
 # item's first dV / dK products.  Those products also wait for pds_full of that step, at which the row threads
 # arrive only after they have read the previous item's dK / dV (program order of the row threads).
 IMPLIED = ("mma_wait_dkv_free",)
 
 
-def run_attention_bwd(items: List[int], rng: random.Random, drop: Optional[str] = None) -> float:
+def run_attention_bwd(items: List[int], rng: random.Random, drop: Optional[str] = None, one: bool = False) -> float:
     """Simulates one CTA; returns the finishing time in ns.  Raises ``Hazard`` or ``Deadlock``."""
-    assert drop is None or drop in MUTATIONS + IMPLIED
+    assert drop is None or drop in (ONE_MUTATIONS + ONE_IMPLIED if one else MUTATIONS + IMPLIED)
+    assert not one or all(n == 1 for n in items)
     sim = Sim()
+    parts = range(2 if one else 1)                # row roles
     B: Dict[str, Barrier] = {n: Barrier(n, 1) for n in (
         "kv_full0", "kv_full1", "kv_empty0", "kv_empty1", "q_full0", "q_full1", "q_empty0", "q_empty1",
-        "sdp_full", "pds_full", "dq_full", "dq_free", "dkv_free", "sdp_read", "dq_staged", "dq_stage_free",
-        "dkv_staged", "dkv_stored")}
+        "sdp_full", "dq_full", "dq_stage_free", "dkv_stored")}
+    B.update({n: Barrier(n, len(parts)) for n in ("pds_full", "dq_free", "dkv_free", "sdp_read", "dq_staged", "dkv_staged",
+                                                  "dots_full")})
+    each = lambda name, version: [(f"{name}.{k}", version) for k in parts]
 
     def lat(lo: float, hi: float) -> float:
         return rng.uniform(lo, hi)
@@ -90,23 +103,23 @@ def run_attention_bwd(items: List[int], rng: random.Random, drop: Optional[str] 
                 yield ("wait", B["pds_full"], g & 1)
                 if it == 0 and w > 0 and drop != "mma_wait_dkv_free":
                     yield ("wait", B["dkv_free"], (w - 1) & 1)
-                yield ("mma", [("P", g), (f"QDO{s}", g)], ["DKV"], 8 * t_mma)            # dV
+                yield ("mma", each("P", g) + [(f"QDO{s}", g)], ["DKV"], 8 * t_mma)            # dV
                 if drop == "q_empty_before_dk":
                     yield ("commit", B[f"q_empty{s}"])
-                yield ("mma", [("DS", g), (f"QDO{s}", g)], [("DKV", (w, it))], 8 * t_mma)   # dK
+                yield ("mma", each("DS", g) + [(f"QDO{s}", g)], [("DKV", (w, it))], 8 * t_mma)   # dK
                 if drop != "q_empty_before_dk":
                     yield ("commit", B[f"q_empty{s}"])
                 yield ("delay", 16 * t_issue)
                 if g > 0 and drop != "mma_wait_dq_free":
                     yield ("wait", B["dq_free"], (g - 1) & 1)
-                yield ("mma", [("DS", g), (f"KV{kb}", w)], [("DQT", g)], 8 * t_mma)       # dQ
+                yield ("mma", each("DS", g) + [(f"KV{kb}", w)], [("DQT", g)], 8 * t_mma)       # dQ
                 yield ("commit", B["dq_full"])
                 if it + 1 == steps:
                     yield ("commit", B[f"kv_empty{kb}"])
                 yield ("delay", 8 * t_issue)
                 g += 1
 
-    def drain_dq(gs: int):
+    def drain_dq(gs: int, k: int):
         yield ("delay", lat(0, 1500))                  # the row warps are not in step with the issuing thread
         yield ("wait", B["dq_full"], gs & 1)
         yield ("read", ("DQT", gs))
@@ -114,14 +127,35 @@ def run_attention_bwd(items: List[int], rng: random.Random, drop: Optional[str] 
         yield ("arrive", B["dq_free"])
         if gs > 0 and drop != "rows_wait_dq_stage_free":
             yield ("wait", B["dq_stage_free"], (gs - 1) & 1)
-        yield ("write", ("STG", gs))
+        yield ("write", (f"STG.{k}", gs))
+        yield ("write", (f"DQSUM.{k}", gs))
         yield ("delay", lat(50, 300))
         yield ("arrive", B["dq_staged"])
 
-    def rows():
+    def dots(item: int, k: int):
+        if item > 0:
+            if drop != "rows_wait_q_full":
+                yield ("wait", B[f"q_full{item % 2}"], (item // 2) & 1)
+            yield ("read", (f"QDO{item % 2}", item))
+        yield ("delay", lat(100, 1500))
+        yield ("write", (dots_buffer(item, k), item))
+        yield ("arrive", B["dots_full"])
+
+    def dots_buffer(item: int, k: int) -> str:
+        return f"D{0 if drop == 'one_dots_buffer' else item & 1}.{k}"
+
+    def rows(k: int):
         g = 0
+        if one:
+            yield from dots(0, k)
         for w, steps in enumerate(items):
             for it in range(steps):
+                if one:
+                    if drop != "rows_wait_dots_full":
+                        yield ("wait", B["dots_full"], g & 1)
+                    yield ("delay", lat(0, 3000))          # the row warps are not in step with one another
+                    for other in parts:
+                        yield ("read", (dots_buffer(g, other), g))
                 yield ("wait", B["sdp_full"], g & 1)
                 yield ("read", ("S", g))
                 yield ("delay", lat(100, 500))
@@ -131,18 +165,21 @@ def run_attention_bwd(items: List[int], rng: random.Random, drop: Optional[str] 
                     yield ("wait", B["dq_full"], (g - 1) & 1)
                 if it == 0 and w > 0 and drop != "rows_wait_dkv_stored":
                     yield ("wait", B["dkv_stored"], (w - 1) & 1)
-                yield ("write", ("DS", g))
-                yield ("write", ("P", g))
+                yield ("write", (f"DS.{k}", g))
+                yield ("write", (f"P.{k}", g))
                 yield ("delay", lat(100, 700))
                 yield ("arrive", B["pds_full"])
+                if one and w + 1 < n_items:
+                    yield from dots(g + 1, k)
                 if it > 0:
-                    yield from drain_dq(g - 1)
+                    yield from drain_dq(g - 1, k)
                 g += 1
-            yield from drain_dq(g - 1)
+            yield from drain_dq(g - 1, k)
             yield ("read", ("DKV", (w, steps - 1)))
             yield ("delay", lat(50, 300))
             yield ("arrive", B["dkv_free"])
-            yield ("write", ("P", ("dkv", w)))         # dK / dV staged in the P buffer
+            yield ("write", (f"DKVSUM.{k}", w))
+            yield ("write", (f"P.{k}", ("dkv", w)))    # dK / dV staged in the P buffer
             yield ("delay", lat(50, 300))
             yield ("arrive", B["dkv_staged"])
 
@@ -152,19 +189,20 @@ def run_attention_bwd(items: List[int], rng: random.Random, drop: Optional[str] 
             for _ in range(steps):
                 yield ("wait", B["dq_staged"], g & 1)
                 done = Barrier(f"reduce{g}", 1)
-                yield ("copy", [("STG", g)], [], lat(100, 1500), done, None)
+                yield ("copy", each("STG", g) + each("DQSUM", g), [], lat(100, 1500), done, None)
                 yield ("wait", done, 0)               # cp.async.bulk.wait_group.read
                 yield ("arrive", B["dq_stage_free"])
                 g += 1
             yield ("wait", B["dkv_staged"], w & 1)
             done = Barrier(f"store{w}", 1)
-            yield ("copy", [("P", ("dkv", w))], [], lat(100, 1500), done, None)
+            yield ("copy", each("P", ("dkv", w)) + each("DKVSUM", w), [], lat(100, 1500), done, None)
             yield ("wait", done, 0)
             yield ("arrive", B["dkv_stored"])
 
     sim.add_role("producer", producer())
     sim.add_role("mma", mma())
-    sim.add_role("rows", rows())
+    for k in parts:
+        sim.add_role(f"rows{k}", rows(k))
     sim.add_role("reducer", reducer())
     return sim.run()
 

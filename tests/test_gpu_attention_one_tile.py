@@ -35,3 +35,20 @@ def test_backward_against_64_bits(B, T, nh, hs):
         # P and dS are rounded to bf16 before the products, the results once more: each by at most 2^-9 of its value, in
         # squares 2^-9 sqrt(2 / 3) of a result's norm and less; T = 1 has a zero gradient of q and k
         assert (a - b).norm() <= 2 ** -8 * b.norm() + 1e-6 * (B * T * d) ** 0.5, "qkv"[part]
+
+
+@pytest.mark.parametrize("B,T,nh,hs", [(1, 1, 1, 64), (1, 128, 4, 32), (3, 31, 3, 64), (2, 100, 4, 32), (20, 127, 12, 64), (16, 128, 16, 64)])
+def test_backward_is_that_of_longer_sequences(B, T, nh, hs):
+    """The same tokens with a tail behind them whose output has no gradient: the tail adds zeros, so the kernels for several
+    tiles have to give the same bits."""
+    from diloco_swarm_b200.ops.attention import attention_bwd, attention_fwd
+    g = torch.Generator(device="cuda").manual_seed(T)
+    d, longer = nh * hs, T + 129
+    qkv = torch.randn(B, longer, 3 * d, device="cuda", generator=g).to(torch.bfloat16)
+    dout = torch.randn(B, longer, d, device="cuda", generator=g).to(torch.bfloat16)
+    dout[:, T:] = 0
+    grads = []
+    for n in (T, longer):
+        _, ctx = attention_fwd(qkv[:, :n].reshape(B * n, 3 * d).contiguous(), B, n, nh)
+        grads.append(attention_bwd(dout[:, :n].reshape(B * n, d).contiguous(), ctx).view(B, n, 3 * d)[:, :T])
+    assert torch.equal(*grads)

@@ -6,7 +6,7 @@ import random
 
 import pytest
 
-from diloco_swarm_b200.utils.attention_protocol import IMPLIED, MUTATIONS, run_attention_bwd
+from diloco_swarm_b200.utils.attention_protocol import IMPLIED, MUTATIONS, ONE_IMPLIED, ONE_MUTATIONS, run_attention_bwd
 from diloco_swarm_b200.utils.protocol_sim import Barrier, Deadlock, Hazard, Sim
 
 
@@ -52,6 +52,31 @@ def test_an_implied_wait_can_go_without_harm(drop):
     for seed in range(200):
         rng = random.Random(seed)
         run_attention_bwd(_items(rng), rng, drop=drop)
+
+
+def test_sequences_of_one_tile_are_deadlock_and_hazard_free():
+    for seed in range(300):
+        rng = random.Random(3000 + seed)
+        run_attention_bwd([1] * rng.randint(1, 12), rng, one=True)
+
+
+@pytest.mark.parametrize("drop", ONE_MUTATIONS)
+def test_sequences_of_one_tile_a_missing_wait_is_noticed(drop):
+    seen = 0
+    for seed in range(200):
+        rng = random.Random(seed)
+        try:
+            run_attention_bwd([1] * rng.randint(3, 12), rng, drop=drop, one=True)
+        except (Hazard, Deadlock, AssertionError):
+            seen += 1
+    assert seen > 0, f"leaving out {drop} went unnoticed in 200 random runs"
+
+
+@pytest.mark.parametrize("drop", ONE_IMPLIED)
+def test_sequences_of_one_tile_an_implied_wait_can_go_without_harm(drop):
+    for seed in range(200):
+        rng = random.Random(seed)
+        run_attention_bwd([1] * rng.randint(1, 12), rng, drop=drop, one=True)
 
 
 def test_sim_reports_a_deadlock():
@@ -126,3 +151,20 @@ def test_step_time_model_of_the_attention_backward():
     assert step_time(items, {**MEASURED, "tma": 600.0}) < 0.93 * base
     assert step_time(items, {**MEASURED, "t_issue": 26.0, "t_mma": 30.0}) < 0.9 * base
     assert step_time(items, {**MEASURED, "compute": 600.0}) > 0.95 * base
+
+
+def test_no_warp_waits_for_another_without_a_limit():
+    """In kernels whose waits are bounded (mbar_wait) a warp whose wait has run out leaves its loop.  A named barrier, which
+    waits for good, would hold the warps that count on it."""
+    import glob
+    import os
+    import re
+    csrc = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "diloco_swarm_b200", "csrc")
+    seen = 0
+    for path in glob.glob(os.path.join(csrc, "*.cu*")):
+        text = re.sub(r"//[^\n]*", "", open(path).read())
+        for kernel in text.split("__global__")[1:]:
+            if "mbar_wait" in kernel:
+                seen += 1
+                assert not re.search(r"\bbar(rier)?\.(cta\.)?(sync|red)|__barrier_sync|__syncthreads_(and|or|count)", kernel), os.path.basename(path)
+    assert seen >= 5
