@@ -898,7 +898,7 @@ extern "C" int dsw_layernorm_bwd(const void* dy, const void* x, const float* gam
 
 extern "C" int dsw_colsum_accum(const void* x, long long ld, float* out, int M, int N, cudaStream_t st) {
   if (N % 8 || ld % 8) return -10;
-  dim3 grid((N + 255) / 256, M >= 4096 ? 128 : (M >= 256 ? 16 : 1));
+  dim3 grid((N + 255) / 256, M >= 4096 ? 128 : (M >= COLSUM_ORDERED_ROWS ? 16 : 1));
   return launch(colsum_kernel, grid, 256, 0, st, 1, (const bf16*)x, ld, out, M, N) == cudaSuccess ? 0 : -3;
 }
 

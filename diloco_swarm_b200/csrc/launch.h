@@ -27,6 +27,9 @@ struct LaunchMode {
 };
 extern thread_local LaunchMode tl_launch;
 
+// Up to here (exclusive) dsw_colsum_accum adds the rows of a column in one block and in a fixed order.
+constexpr int COLSUM_ORDERED_ROWS = 256;
+
 template <class... P, class... A>
 inline cudaError_t launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, int cluster, A... args) {
   cudaLaunchConfig_t cfg = {};

@@ -347,11 +347,12 @@ struct Run {
 
   // The next launch is asked to add its output's column sums (a bias gradient) to `to`: in its epilogue or beside its
   // products, in place of a pass that reads dh or dqkv once more (a microbatch of GPT-2 small, 32 x 1024: 33.07 -> 32.38 ms,
-  // 16 x 133: 2786 -> 2762 us; six blocks of medium, 8 x 1024: 4788 -> 4667 us).  Its sums meet in atomics, which a
-  // deterministic backward does without.
-  void sum_columns(float* to) const { dsw::tl_launch.colsum = deterministic ? nullptr : to; }
+  // 16 x 133: 2786 -> 2762 us; six blocks of medium, 8 x 1024: 4788 -> 4667 us).  Its sums meet in atomics, as those of the
+  // pass do from COLSUM_ORDERED_ROWS rows on; fewer rows, whose gradients repeat themselves bit for bit, keep the pass.
+  bool columns_asked() const { return !deterministic && M >= dsw::COLSUM_ORDERED_ROWS; }
+  void sum_columns(float* to) const { dsw::tl_launch.colsum = columns_asked() ? to : nullptr; }
   bool columns_unsummed() const {
-    const bool left = deterministic || dsw::tl_launch.colsum != nullptr;
+    const bool left = !columns_asked() || dsw::tl_launch.colsum != nullptr;
     dsw::tl_launch.colsum = nullptr;
     return left;
   }

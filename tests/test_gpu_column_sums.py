@@ -40,3 +40,27 @@ def test_sums_are_those_of_a_pass_of_their_own(B, T, heads, width):
         assert (a - b).norm() <= 2 ** -8 * a.norm() * max(1.0, (B * T) ** 0.5 / 8) + 1e-9, k
         seen += "c_fc" in k or "c_attn" in k
     assert seen == 4
+
+
+@pytest.mark.parametrize("B,T", [(1, 24), (1, 128), (2, 100), (1, 255)])
+@pytest.mark.parametrize("heads,width", [(4, 128), (12, 768)])
+def test_few_rows_repeat_themselves(B, T, heads, width):
+    """Up to 255 rows every sum of a bias gradient is added up in one order, so the same pass gives the same bits."""
+    from diloco_swarm_b200.models.engine_b200 import B200Engine
+    from diloco_swarm_b200.models.gpt2 import GPT2Config
+    cfg = make_config(model={"n_layer": 2, "n_head": heads, "n_embd": width, "vocab_size": 512, "block_size": 256})
+    eng = B200Engine(GPT2Config(block_size=256, vocab_size=512, n_layer=2, n_head=heads, n_embd=width), single_world(), cfg,
+                     torch.device("cuda", 0))
+    gen = torch.Generator(device="cuda").manual_seed(11)
+    ids = torch.randint(0, 512, (B, T + 1), device="cuda", generator=gen)
+    mask = torch.ones(B, T, dtype=torch.long, device="cuda")
+    first = None
+    for _ in range(12):
+        eng.grad.zero_()
+        eng.forward_backward(0, ids[:, :-1].contiguous(), None, ids[:, 1:].contiguous(), mask, 1.0)
+        torch.cuda.synchronize()
+        got = {k: eng.g32(k).clone() for k, _, _ in eng.specs if k.endswith("bias")}
+        first = first or got
+        for k in got:
+            assert torch.equal(got[k], first[k]), k
+    eng.check_status()
