@@ -97,6 +97,8 @@ int dsw_layernorm_bwd(const void* dy, const void* x, const float* gamma, const f
                       int M, int d, cudaStream_t st);
 // out[N] (fp32) += column sums of x: bf16 [M, N] with row pitch ld.
 int dsw_colsum_accum(const void* x, long long ld, float* out, int M, int N, cudaStream_t st);
+// The same with a fixed order of additions.
+int dsw_colsum_ordered(const void* x, long long ld, float* out, int M, int N, cudaStream_t st);
 // y[b,t,:] = bf16(wte[ids[b,t]] + wpe[t]); an id outside [0, V) sets status 3 and reads row 0.
 int dsw_embedding_fwd(const long long* ids, const float* wte, const float* wpe, void* y, int B, int T, int d, int V,
                       int* status, cudaStream_t st);

@@ -356,6 +356,9 @@ struct Run {
     dsw::tl_launch.colsum = nullptr;
     return left;
   }
+  int colsum(const bf16* x, int n, float* to) const {
+    return (deterministic ? dsw_colsum_ordered : dsw_colsum_accum)(x, n, to, M, n, side());
+  }
 
   // The rows' part of a LayerNorm backward on the main stream; its column sums, which nothing in the backward reads, are
   // joined on the side stream once it may go on (ln_sums after a fork): some 3 us less of the chain per LayerNorm.
@@ -390,7 +393,7 @@ struct Run {
     const bool sum_dh = columns_unsummed();
     TRY(fork());
     SIDE(wgrad(dx2, v.g, d, 4 * d, b.dw[W_PR], M, side()));
-    if (sum_dh) SIDE(dsw_colsum_accum(c.dh[p], 4 * d, b.db[W_FC], M, 4 * d, side()));
+    if (sum_dh) SIDE(colsum(c.dh[p], 4 * d, b.db[W_FC]));
     SIDE(wgrad(c.dh[p], v.ln2, 4 * d, d, b.dw[W_FC], M, side()));
     LAUNCH(gemm(c.dh[p], b.w[W_FC], false, d, 4 * d, c.dln, DSW_EPI_STORE, nullptr, nullptr, nullptr, nullptr, M));
     // the column sum of dx2 (bias gradient of the MLP's second projection) comes out of the LayerNorm backward as well
@@ -403,7 +406,7 @@ struct Run {
     LAUNCH(dsw_attention_bwd(v.qkv, v.att, c.datt, v.lse, c.dqkv[p], c.dq_acc, c.dvec, B, T, s.nh, d / s.nh, scale(), s.status, st));
     const bool sum_dqkv = columns_unsummed();
     TRY(fork());
-    if (sum_dqkv) SIDE(dsw_colsum_accum(c.dqkv[p], 3 * d, b.db[W_QKV], M, 3 * d, side()));
+    if (sum_dqkv) SIDE(colsum(c.dqkv[p], 3 * d, b.db[W_QKV]));
     SIDE(wgrad(c.dqkv[p], v.ln1, 3 * d, d, b.dw[W_QKV], M, side()));
     LAUNCH(gemm(c.dqkv[p], b.w[W_QKV], false, d, 3 * d, c.dln, DSW_EPI_STORE, nullptr, nullptr, nullptr, nullptr, M));
     LAUNCH(ln_rows(c.dln, x, b.ln1_w, v.mu1, v.rs1, c.dx1[p], dx0, c.ln[2 * p + 1]));

@@ -77,9 +77,10 @@ _DETERMINISTIC = False
 def set_deterministic(on: bool) -> None:
     """Fixed order of floating-point additions in the gradient kernels that
     otherwise use atomics: the token-embedding scatter goes through a stable
-    sort with one writer per row, and weight gradients are not split along K
-    (each output tile then has one writer per launch, and launches are ordered
-    by the stream).  Slower; meant for debugging and regression runs."""
+    sort with one writer per row, weight gradients are not split along K (each
+    output tile then has one writer per launch, and launches are ordered by the
+    stream), and bias gradients have a pass of their own with one writer per
+    column.  Slower; meant for debugging and regression runs."""
     global _DETERMINISTIC
     _DETERMINISTIC = bool(on)
 
@@ -138,7 +139,8 @@ def colsum_accum(x: torch.Tensor, out: torch.Tensor) -> None:
     """out[n] += sum_m x[m,n] (bias gradients)."""
     M, N = x.shape
     assert x.dtype == BF16 and x.stride(1) == 1 and out.dtype == F32 and out.numel() == N
-    check(cuda_lib().dsw_colsum_accum(x.data_ptr(), x.stride(0), out.data_ptr(), M, N, stream_ptr()), "dsw_colsum_accum")
+    colsum = cuda_lib().dsw_colsum_ordered if _DETERMINISTIC else cuda_lib().dsw_colsum_accum
+    check(colsum(x.data_ptr(), x.stride(0), out.data_ptr(), M, N, stream_ptr()), "dsw_colsum")
 
 
 def embedding_fwd(ids: torch.Tensor, wte: torch.Tensor, wpe: torch.Tensor, status: Optional[Status] = None

@@ -145,6 +145,9 @@ int dsw_layernorm_bwd(const void* dy, const void* x, const float*, const float* 
 int dsw_colsum_accum(const void* x, long long, float*, int M, int N, cudaStream_t st) {
   return op("colsum", st, {{'r', x, 2LL * M * N}});
 }
+int dsw_colsum_ordered(const void* x, long long, float*, int M, int N, cudaStream_t st) {
+  return op("colsum_ordered", st, {{'r', x, 2LL * M * N}});
+}
 int dsw_embedding_fwd(const long long* ids, const float*, const float*, void* y, int B, int T, int d, int, int*, cudaStream_t st) {
   return op("embedding_fwd", st, {{'r', ids, 8LL * B * T}, {'w', y, 2LL * B * T * d}});
 }
