@@ -141,7 +141,8 @@ class TrainConfig(BaseConfig):
     seed: int = 42
     max_norm: float = 1.0
     step_timeout: float = 60
-    deterministic: bool = False  # (added) fixed order of additions in the gradient kernels (sorted embedding scatter, no split-K)
+    deterministic: bool = False  # (added) fixed order of additions in the gradient kernels (sorted embedding scatter, no split-K, one writer
+    # per bias gradient, dQ tile by tile); the loss value and the gradient's norm are still summed in any order
     # (added) the LM head, the cross-entropy and the head's two gradient GEMMs run over this many slices of a
     # microbatch's token rows, one after the other, so that only a slice of the [tokens, vocabulary] logits
     # exists at a time (GPT-2 small, 16 x 1024 tokens: 1.65 GB for one slice, 0.41 GB for four); b200 engine

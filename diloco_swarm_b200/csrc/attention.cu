@@ -659,7 +659,7 @@ __global__ void __launch_bounds__(ATT_BWD_THREADS, 1)
 attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_constant__ CUtensorMap tmap_do,
                      const __grid_constant__ CUtensorMap tmap_dq, const __grid_constant__ CUtensorMap tmap_dkv,
                      const __nv_bfloat16* out, const __nv_bfloat16* dout, const float* lse, const float* Dvec, int T, int nh,
-                     int n_bh, int hs, float scale, float* colsum, int* status, long long* trace) {
+                     int n_bh, int hs, int item0, int total, float scale, float* colsum, int* status, long long* trace) {
   using L = AttBwdSmem;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw;
@@ -691,9 +691,13 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nq = (T + ATT_BQ - 1) / ATT_BQ;
-  const int total = nq * n_bh;                   // items, heaviest first: kv tile 0 meets every query tile
-  const int G = gridDim.x, cta = blockIdx.x;
-  const int rounds = (total + G - 1) / G;
+  // items item0 .. item0 + total - 1, heaviest first: kv tile 0 meets every query tile
+  const auto next_item = [=](int r, int& idx) {
+    const bool is = att_item(r, int(blockIdx.x), int(gridDim.x), total, idx);
+    idx += item0;
+    return is;
+  };
+  const int rounds = (total + int(gridDim.x) - 1) / int(gridDim.x);
   const int d = nh * hs;
   const float scale_log2 = scale * 1.4426950408889634f;
   long long* tr = blockIdx.x == 0 ? trace : nullptr;
@@ -735,7 +739,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
     bool ok = true;
     for (int r = 0; r < rounds && ok; ++r) {
       int idx;
-      if (!att_item(r, cta, G, total, idx)) continue;
+      if (!next_item(r, idx)) continue;
       const int j = idx / n_bh, bh = idx % n_bh;
       const int b = bh / nh, h = bh - b * nh;
       const int steps = nq - j;
@@ -814,12 +818,12 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
     };
     for (int r = 0; r < rounds && ok; ++r) {
       int idx;
-      if (!att_item(r, cta, G, total, idx)) continue;
+      if (!next_item(r, idx)) continue;
       const int steps = nq - idx / n_bh;
       bool more = false;                  // does this CTA have another item after this one?
       for (int r2 = r + 1; r2 < rounds && !more; ++r2) {
         int idx2;
-        more = att_item(r2, cta, G, total, idx2);
+        more = next_item(r2, idx2);
       }
       const int kb = w & 1;
       const uint32_t k_mn = k_mn0 + kb * KVBUF16;
@@ -877,7 +881,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
       bool ok = true;
       for (int rr = 0; rr < rounds && ok; ++rr) {
         int idx;
-        if (!att_item(rr, cta, G, total, idx)) continue;
+        if (!next_item(rr, idx)) continue;
         const int j = idx / n_bh, bh = idx % n_bh;
         const int b = bh / nh, h = bh - b * nh;
         for (int i = j; i < nq; ++i, ++g) {
@@ -991,7 +995,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
     };
     if (ONE) {                        // the CTA's first item, while its tiles are on their way
       int idx;
-      att_item(0, cta, G, total, idx);          // there is one: G <= total
+      next_item(0, idx);          // there is one: G <= total
       const long long at = dots_at(idx % n_bh);
       if (hs == 64) ItemDots<8>::first(out + at, dout + at, d, T - dot_row, dots_to(0), lane);
       else          ItemDots<4>::first(out + at, dout + at, d, T - dot_row, dots_to(0), lane);
@@ -999,14 +1003,14 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
     }
     for (int rr = 0; rr < rounds && ok; ++rr) {
       int idx;
-      if (!att_item(rr, cta, G, total, idx)) continue;
+      if (!next_item(rr, idx)) continue;
       const int j = idx / n_bh, bh = idx % n_bh;
       const int steps = nq - j;
       // where the next item's first step finds its row statistics (-1: this is the CTA's last item)
       int stat_after = -1, bh_after = -1;
       for (int r2 = rr + 1; r2 < rounds; ++r2) {
         int idx2;
-        if (att_item(r2, cta, G, total, idx2)) {
+        if (next_item(r2, idx2)) {
           // a row past the end of the sequence: its statistics are never used
           bh_after = idx2 % n_bh;
           stat_after = (idx2 / n_bh) * ATT_BQ + r < T ? bh_after * T + (idx2 / n_bh) * ATT_BQ + r : -1;
@@ -1183,9 +1187,10 @@ extern "C" int dsw_attention_fwd(const void* qkv, void* out, float* lse, int B, 
 
 // qkv, out, dout as in the forward; lse from the forward.  dqkv: bf16 [B*T, 3*d] (all of it is written).
 // dq_acc: fp32 scratch [B*T, d]; Dvec: fp32 scratch [B*nh*T].  Both are overwritten where T > 128.
-extern "C" int dsw_attention_bwd(const void* qkv, const void* out, const void* dout, const float* lse, void* dqkv,
-                                 float* dq_acc, float* Dvec, int B, int T, int nh, int hs, float scale, int* status,
-                                 cudaStream_t st) {
+// ordered: the kv tiles' contributions to dQ, which otherwise meet in whatever order their CTAs get there, are added tile
+// by tile, one launch each.
+static int attention_bwd(const void* qkv, const void* out, const void* dout, const float* lse, void* dqkv, float* dq_acc, float* Dvec,
+                         int B, int T, int nh, int hs, float scale, bool ordered, int* status, cudaStream_t st) {
   if ((hs != 64 && hs != 32) || T <= 0 || (long long)B * nh * T >= (1LL << 31)) return -10;
   const int d = nh * hs;
   const long long rows = (long long)B * T;
@@ -1203,13 +1208,14 @@ extern "C" int dsw_attention_bwd(const void* qkv, const void* out, const void* d
     attr_set = true;
   }
   // persistent: one CTA per SM walks the work items
-  const int total = ((T + ATT_BK - 1) / ATT_BK) * B * nh;
-  const int G = total < att_num_sms() ? total : att_num_sms();
+  const int tiles = (T + ATT_BK - 1) / ATT_BK, n_bh = B * nh;
+  const auto grid = [](int items) { return items < att_num_sms() ? items : att_num_sms(); };
   float* const colsum = reinterpret_cast<uintptr_t>(tl_launch.colsum) & 15 ? nullptr : tl_launch.colsum;          // for bulk reductions
   if (colsum != nullptr) tl_launch.colsum = nullptr;
   if (T <= ATT_BK)
-    return launch(attention_bwd_kernel<true>, G, ATT_BWD_THREADS, AttBwdSmem::TOTAL, st, 1, tq, tdo, tdq, tdkv, (const __nv_bfloat16*)out,
-                  (const __nv_bfloat16*)dout, lse, Dvec, T, nh, B * nh, hs, scale, colsum, status, g_att_trace) == cudaSuccess ? 0 : -3;
+    return launch(attention_bwd_kernel<true>, grid(n_bh), ATT_BWD_THREADS, AttBwdSmem::TOTAL, st, 1, tq, tdo, tdq, tdkv,
+                  (const __nv_bfloat16*)out, (const __nv_bfloat16*)dout, lse, Dvec, T, nh, n_bh, hs, 0, n_bh, scale, colsum, status,
+                  g_att_trace) == cudaSuccess ? 0 : -3;
   // D = rowsum(dO * O) per head, and the dQ accumulator zeroed in the same pass
   {
     const long long want = (rows * 32 + 255) / 256;
@@ -1218,15 +1224,29 @@ extern "C" int dsw_attention_bwd(const void* qkv, const void* out, const void* d
                (const __nv_bfloat16*)dout, Dvec, dq_acc, B, T, nh, hs) != cudaSuccess)
       return -3;
   }
-  if (launch(attention_bwd_kernel<false>, G, ATT_BWD_THREADS, AttBwdSmem::TOTAL, st, 1, tq, tdo, tdq, tdkv, (const __nv_bfloat16*)out,
-             (const __nv_bfloat16*)dout, lse, Dvec, T, nh, B * nh, hs, scale, colsum, status, g_att_trace) != cudaSuccess)
-    return -3;
+  const int per_launch = ordered ? n_bh : tiles * n_bh;
+  for (int item0 = 0; item0 < tiles * n_bh; item0 += per_launch)
+    if (launch(attention_bwd_kernel<false>, grid(per_launch), ATT_BWD_THREADS, AttBwdSmem::TOTAL, st, 1, tq, tdo, tdq, tdkv,
+               (const __nv_bfloat16*)out, (const __nv_bfloat16*)dout, lse, Dvec, T, nh, n_bh, hs, item0, per_launch, scale, colsum, status,
+               g_att_trace) != cudaSuccess)
+      return -3;
   const int width = d / 8 < 512 ? d / 8 : 512, per_step = 512 / width;
   const long long steps = (rows + per_step - 1) / per_step;
   return launch(attention_dq_convert_kernel, dim3(unsigned(steps < 296 ? steps : 296), (d + 8 * width - 1) / (8 * width)), width * per_step,
                 colsum ? sizeof(float) * per_step * width * 8 : 0, st, 1, dq_acc, (__nv_bfloat16*)dqkv, rows, d, width, colsum) == cudaSuccess
              ? 0
              : -3;
+}
+
+extern "C" int dsw_attention_bwd(const void* qkv, const void* out, const void* dout, const float* lse, void* dqkv,
+                                 float* dq_acc, float* Dvec, int B, int T, int nh, int hs, float scale, int* status,
+                                 cudaStream_t st) {
+  return attention_bwd(qkv, out, dout, lse, dqkv, dq_acc, Dvec, B, T, nh, hs, scale, false, status, st);
+}
+extern "C" int dsw_attention_bwd_ordered(const void* qkv, const void* out, const void* dout, const float* lse, void* dqkv,
+                                         float* dq_acc, float* Dvec, int B, int T, int nh, int hs, float scale, int* status,
+                                         cudaStream_t st) {
+  return attention_bwd(qkv, out, dout, lse, dqkv, dq_acc, Dvec, B, T, nh, hs, scale, true, status, st);
 }
 
 extern "C" int dsw_load_attention() {

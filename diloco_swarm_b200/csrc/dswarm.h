@@ -77,6 +77,10 @@ int dsw_attention_fwd(const void* qkv, void* out, float* lse, int B, int T, int 
 int dsw_attention_bwd(const void* qkv, const void* out, const void* dout, const float* lse, void* dqkv,
                       float* dq_acc, float* Dvec, int B, int T, int nh, int hs, float scale, int* status,
                       cudaStream_t st);
+// The same with a fixed order of additions to dQ: one launch per 128 tokens of a sequence.
+int dsw_attention_bwd_ordered(const void* qkv, const void* out, const void* dout, const float* lse, void* dqkv,
+                      float* dq_acc, float* Dvec, int B, int T, int nh, int hs, float scale, int* status,
+                      cudaStream_t st);
 int dsw_attention_set_trace(long long* buf);
 
 // ---------------------------------------------------------------- LayerNorm, embedding, loss, casts (elementwise.cu)

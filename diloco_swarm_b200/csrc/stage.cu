@@ -403,7 +403,8 @@ struct Run {
     SIDE(ln_sums(c.ln[2 * p], b.dln2_w, b.dln2_b, b.db[W_PR]));
     SIDE(wgrad(c.dx1[p], v.att, d, d, b.dw[W_O], M, side()));
     sum_columns(b.db[W_QKV]);
-    LAUNCH(dsw_attention_bwd(v.qkv, v.att, c.datt, v.lse, c.dqkv[p], c.dq_acc, c.dvec, B, T, s.nh, d / s.nh, scale(), s.status, st));
+    LAUNCH((deterministic ? dsw_attention_bwd_ordered : dsw_attention_bwd)(v.qkv, v.att, c.datt, v.lse, c.dqkv[p], c.dq_acc, c.dvec, B, T,
+                                                                           s.nh, d / s.nh, scale(), s.status, st));
     const bool sum_dqkv = columns_unsummed();
     TRY(fork());
     if (sum_dqkv) SIDE(colsum(c.dqkv[p], 3 * d, b.db[W_QKV]));

@@ -82,6 +82,8 @@ _SIGS = {
     "dsw_attention_fwd": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_void_p, c_void_p],
     "dsw_attention_bwd": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                           c_int, c_float, c_void_p, c_void_p],
+    "dsw_attention_bwd_ordered": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
+                          c_int, c_float, c_void_p, c_void_p],
 }
 
 

@@ -21,6 +21,7 @@ import torch
 import torch.nn.functional as F
 
 from ._lib import Status, check, cuda_lib, stream_ptr
+from .kernels import deterministic
 
 BF16 = torch.bfloat16
 
@@ -78,10 +79,10 @@ def attention_bwd(dout: torch.Tensor, ctx: AttnCtx) -> torch.Tensor:
         dq_acc = torch.empty(B * T, d, dtype=torch.float32, device=dout.device)     # fp32 accumulator of dQ
         dvec = torch.empty(B * nh * T, dtype=torch.float32, device=dout.device)     # rowsum(dO * O)
         dout = dout.contiguous()
-        check(cuda_lib().dsw_attention_bwd(ctx.qkv.data_ptr(), ctx.out.data_ptr(), dout.data_ptr(), ctx.lse.data_ptr(),
-                                           dqkv.data_ptr(), dq_acc.data_ptr(), dvec.data_ptr(), B, T, nh, hs,
-                                           1.0 / math.sqrt(hs), ctx.status.ptr if ctx.status is not None else None,
-                                           stream_ptr()), "dsw_attention_bwd")
+        bwd = cuda_lib().dsw_attention_bwd_ordered if deterministic() else cuda_lib().dsw_attention_bwd
+        check(bwd(ctx.qkv.data_ptr(), ctx.out.data_ptr(), dout.data_ptr(), ctx.lse.data_ptr(),
+                  dqkv.data_ptr(), dq_acc.data_ptr(), dvec.data_ptr(), B, T, nh, hs, 1.0 / math.sqrt(hs),
+                  ctx.status.ptr if ctx.status is not None else None, stream_ptr()), "dsw_attention_bwd")
         return dqkv
     q, k, v, o = ctx.q, ctx.k, ctx.v, ctx.o
     B, nh, T, hs = q.shape

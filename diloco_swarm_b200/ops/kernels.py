@@ -79,8 +79,10 @@ def set_deterministic(on: bool) -> None:
     otherwise use atomics: the token-embedding scatter goes through a stable
     sort with one writer per row, weight gradients are not split along K (each
     output tile then has one writer per launch, and launches are ordered by the
-    stream), and bias gradients have a pass of their own with one writer per
-    column.  Slower; meant for debugging and regression runs."""
+    stream), bias gradients have a pass of their own with one writer per column,
+    and the attention backward adds to dQ one kv tile per launch.  The loss value
+    and the gradient's norm, which scales it where it is clipped, are still
+    summed in any order.  Slower; meant for debugging and regression runs."""
     global _DETERMINISTIC
     _DETERMINISTIC = bool(on)
 

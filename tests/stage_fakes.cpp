@@ -126,6 +126,10 @@ int dsw_attention_bwd(const void* qkv, const void* out, const void* dout, const 
   return op("attention_bwd", st, {{'r', qkv, 3 * n}, {'r', out, n}, {'r', dout, n}, {'r', lse, 4LL * B * T * nh}, {'w', dqkv, 3 * n},
                                   {'w', dq_acc, 2 * n}, {'w', Dvec, 4LL * B * T * nh}});
 }
+int dsw_attention_bwd_ordered(const void* qkv, const void* out, const void* dout, const float* lse, void* dqkv, float* dq_acc, float* Dvec,
+                              int B, int T, int nh, int hs, float scale, int* status, cudaStream_t st) {
+  return dsw_attention_bwd(qkv, out, dout, lse, dqkv, dq_acc, Dvec, B, T, nh, hs, scale, status, st);
+}
 int dsw_layernorm_fwd(const void* x, const float* g, const float* b, void* y, float* mean, float* rstd, int M, int d, float e,
                       cudaStream_t st) {
   return dsw_layernorm_fwd_lo(x, nullptr, g, b, y, mean, rstd, M, d, e, st);

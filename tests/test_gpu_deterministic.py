@@ -25,7 +25,7 @@ def test_ordered_column_sums(M, N):
 
 
 @pytest.mark.parametrize("heads,width", [(4, 128), (12, 768)])
-@pytest.mark.parametrize("B,T", [(1, 100), (20, 100), (40, 128)])
+@pytest.mark.parametrize("B,T", [(1, 100), (20, 100), (40, 128), (3, 300), (2, 640), (1, 1000)])
 def test_the_same_pass_gives_the_same_gradients(B, T, heads, width):
     from diloco_swarm_b200.models.engine_b200 import B200Engine
     from diloco_swarm_b200.models.gpt2 import GPT2Config
@@ -50,3 +50,25 @@ def test_the_same_pass_gives_the_same_gradients(B, T, heads, width):
         eng.check_status()
     finally:
         K.set_deterministic(False)
+
+
+@pytest.mark.parametrize("B,T,nh,hs", [(1, 129, 1, 64), (2, 384, 4, 32), (3, 1000, 12, 64)])
+def test_ordered_attention_backward(B, T, nh, hs):
+    """One launch per kv tile: the same dK and dV, and a dQ whose fp32 sums differ in their order only."""
+    from diloco_swarm_b200.ops import kernels as K
+    from diloco_swarm_b200.ops._lib import Status
+    from diloco_swarm_b200.ops.attention import attention_bwd, attention_fwd
+    st, d = Status(torch.device("cuda")), nh * hs
+    qkv, dout = torch.randn(B * T, 3 * d, device="cuda").to(torch.bfloat16), torch.randn(B * T, d, device="cuda").to(torch.bfloat16)
+    _, ctx = attention_fwd(qkv, B, T, nh, status=st)
+    any_order = attention_bwd(dout, ctx)
+    K.set_deterministic(True)
+    try:
+        got = [attention_bwd(dout, ctx) for _ in range(6)]
+    finally:
+        K.set_deterministic(False)
+    torch.cuda.synchronize()
+    st.raise_if_set()
+    assert all(torch.equal(g, got[0]) for g in got) and torch.equal(got[0][:, d:], any_order[:, d:])
+    # both rounded to bf16 (2^-9 of a value each) after fp32 sums of at most eight terms
+    assert (got[0][:, :d].double() - any_order[:, :d].double()).norm() <= 2 ** -8 * any_order[:, :d].double().norm()
