@@ -92,10 +92,11 @@ int dsw_layernorm_fwd_lo(const void* x, const void* x_lo, const float* gamma, co
                          float* rstd, int M, int d, float eps, cudaStream_t st);
 // The most blocks dsw_layernorm_bwd launches for M rows = rows of scratch it needs.
 int dsw_layernorm_bwd_blocks(int M);
-// dx = LayerNorm backward of dy (+ dres when given: the residual branch's gradient).  dgamma, dbeta and the
-// optional dres_sum (column sum of dres) are fp32 [d] and are accumulated (+=).
+// dx = LayerNorm backward of dy (+ dres when given: the residual branch's gradient).  dgamma, dbeta and
+// dres_sum (column sum of dres), each optional, are fp32 [d] and are accumulated (+=).
 // scratch: fp32 [dsw_layernorm_bwd_blocks(M)][3][d], contents irrelevant on entry.
-// In two calls with one scratch: dgamma null leaves the column sums there, dx null only joins them (on any stream).
+// In two calls with one scratch: without any of the three the column sums stay there, without dx (null) they are only
+// joined (on any stream).  Neither: refused.
 int dsw_layernorm_bwd(const void* dy, const void* x, const float* gamma, const float* mean, const float* rstd,
                       const void* dres, void* dx, float* dgamma, float* dbeta, float* dres_sum, float* scratch,
                       int M, int d, cudaStream_t st);

@@ -32,7 +32,10 @@
 // Arguments and results are those of dsw_layernorm_bwd without `scratch`:
 //   dy, x, dres (optional), dx : bf16 [M, d] row-major, 16-byte aligned
 //   gamma, mean, rstd          : fp32 [d], [M], [M]
-//   dgamma, dbeta (optional), dres_sum (optional) : fp32 [d], accumulated (+=)
+//   dgamma, dbeta, dres_sum (each optional) : fp32 [d], accumulated (+=)
+// One call is the whole computation: a null dx, with which dsw_layernorm_bwd joins
+// the sums that an earlier call has left in its scratch, is refused
+// (DSW_NOALLOC_BAD_SHAPE).
 // Returns 0, one of the codes below, or the negative code of dsw_layernorm_bwd.
 #pragma once
 #include <cuda_runtime.h>

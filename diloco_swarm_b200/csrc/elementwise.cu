@@ -873,13 +873,14 @@ extern "C" int dsw_layernorm_bwd_blocks(int M) {
 
 // scratch: fp32 [dsw_layernorm_bwd_blocks(M)][3][d], contents irrelevant on entry.
 // dres_sum (optional): fp32 [d] += column sum of dres.
-// In two calls, so that the second can go to another stream: without dgamma only dx and the scratch are written, without
-// dx only the sums that are in the scratch (of the same M and d) are joined; dres_sum then asks for those of the first call's dres.
+// dgamma, dbeta and dres_sum are each optional.  In two calls, so that the second can go to another stream: without any of
+// the three only dx and the scratch are written, without dx only the sums that are in the scratch (of the same M and d) are
+// joined; dres_sum then asks for those of the first call's dres.
 extern "C" int dsw_layernorm_bwd(const void* dy, const void* x, const float* gamma, const float* mean,
                                  const float* rstd, const void* dres, void* dx, float* dgamma, float* dbeta,
                                  float* dres_sum, float* scratch, int M, int d, cudaStream_t st) {
-  if (d % 8 || d > 256 * LN_MAX_CHUNKS_ALL || (dx == nullptr && dgamma == nullptr)) return -10;
-  const bool rows_part = dx != nullptr, sums_part = dgamma != nullptr;
+  const bool rows_part = dx != nullptr, sums_part = dgamma != nullptr || dbeta != nullptr || dres_sum != nullptr;
+  if (d % 8 || d > 256 * LN_MAX_CHUNKS_ALL || !(rows_part || sums_part)) return -10;
   float* const res_out = dres != nullptr || !rows_part ? dres_sum : nullptr;
   cudaError_t rc = cudaSuccess;
   int grid;
@@ -1078,6 +1079,10 @@ extern "C" int dsw_layernorm_bwd_noalloc(const void* dy, const void* x, const fl
                                          float* dbeta, float* dres_sum, int M, int d, cudaStream_t st) {
   if (M <= 0 || d <= 0 || d % 8) {
     fprintf(stderr, "dsw_layernorm_bwd_noalloc: M=%d d=%d: d must be a positive multiple of 8\n", M, d);
+    return DSW_NOALLOC_BAD_SHAPE;
+  }
+  if (dx == nullptr) {          // the sums of an earlier call are nobody's to ask for: the array is shared
+    fprintf(stderr, "dsw_layernorm_bwd_noalloc: dx is null\n");
     return DSW_NOALLOC_BAD_SHAPE;
   }
   const int rb = dsw_layernorm_bwd_blocks(M);
