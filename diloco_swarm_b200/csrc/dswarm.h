@@ -90,11 +90,12 @@ int dsw_layernorm_fwd(const void* x, const float* gamma, const float* beta, void
 // The same of x + x_lo (x_lo: bf16 like x, or null).
 int dsw_layernorm_fwd_lo(const void* x, const void* x_lo, const float* gamma, const float* beta, void* y, float* mean,
                          float* rstd, int M, int d, float eps, cudaStream_t st);
-// The most blocks dsw_layernorm_bwd launches for M rows = rows of scratch it needs.
+// The most blocks dsw_layernorm_bwd launches for M rows of any width; floats of scratch that M rows of d columns need.
 int dsw_layernorm_bwd_blocks(int M);
+int dsw_layernorm_bwd_scratch(int M, int d);
 // dx = LayerNorm backward of dy (+ dres when given: the residual branch's gradient).  dgamma, dbeta and
 // dres_sum (column sum of dres), each optional, are fp32 [d] and are accumulated (+=).
-// scratch: fp32 [dsw_layernorm_bwd_blocks(M)][3][d], contents irrelevant on entry.
+// scratch: fp32, dsw_layernorm_bwd_scratch(M, d) or dsw_layernorm_bwd_blocks(M) * 3 * d of them, contents irrelevant on entry.
 // In two calls with one scratch: without any of the three the column sums stay there, without dx (null) they are only
 // joined (on any stream).  Neither: refused.
 int dsw_layernorm_bwd(const void* dy, const void* x, const float* gamma, const float* mean, const float* rstd,

@@ -865,13 +865,23 @@ extern "C" int dsw_layernorm_fwd_lo(const void* x, const void* x_lo, const float
   return rc == cudaSuccess ? 0 : -3;
 }
 
-// The most blocks dsw_layernorm_bwd launches for M rows = rows of scratch it needs.
-extern "C" int dsw_layernorm_bwd_blocks(int M) {
-  const int want = (M + 2 * LN_BWD_ROWS - 1) / (2 * LN_BWD_ROWS);      // the widest rows: two groups to a block
-  return want < 1 ? 1 : (want > 296 ? 296 : want);     // at most two blocks per SM
+// Blocks of dsw_layernorm_bwd.  Narrow rows: two steps of two rows per warp at least, at most two blocks per SM.  Wide ones:
+// groups of ceil(d / 256) warps, each LN_BWD_ROWS rows at least, at most one block per SM.
+static int ln_bwd_grid(int M, int d) {
+  const int rows = d <= 128 ? 4 * LN_BWD_WARPS : LN_BWD_MAX_WARPS / ((d + 255) / 256) * LN_BWD_ROWS;
+  const int want = M / rows + (M % rows != 0), most = d <= 128 ? 296 : 148;
+  return want < 1 ? 1 : want > most ? most : want;
 }
 
-// scratch: fp32 [dsw_layernorm_bwd_blocks(M)][3][d], contents irrelevant on entry.
+// The most blocks that rows of any width take = rows of scratch that serve all of them.
+extern "C" int dsw_layernorm_bwd_blocks(int M) {
+  const int narrow = ln_bwd_grid(M, 128), widest = ln_bwd_grid(M, 256 * LN_MAX_CHUNKS_ALL);
+  return narrow > widest ? narrow : widest;
+}
+// Floats of scratch that rows of d columns need.
+extern "C" int dsw_layernorm_bwd_scratch(int M, int d) { return ln_bwd_grid(M, d) * 3 * d; }
+
+// scratch: fp32, dsw_layernorm_bwd_scratch(M, d) of them, contents irrelevant on entry.
 // dres_sum (optional): fp32 [d] += column sum of dres.
 // dgamma, dbeta and dres_sum are each optional.  In two calls, so that the second can go to another stream: without any of
 // the three only dx and the scratch are written, without dx only the sums that are in the scratch (of the same M and d) are
@@ -883,16 +893,12 @@ extern "C" int dsw_layernorm_bwd(const void* dy, const void* x, const float* gam
   if (d % 8 || d > 256 * LN_MAX_CHUNKS_ALL || !(rows_part || sums_part)) return -10;
   float* const res_out = dres != nullptr || !rows_part ? dres_sum : nullptr;
   cudaError_t rc = cudaSuccess;
-  int grid;
+  const int grid = ln_bwd_grid(M, d);
   if (d <= 128) {
-    grid = (M + 4 * LN_BWD_WARPS - 1) / (4 * LN_BWD_WARPS);      // two steps of two rows per warp at least
-    grid = grid < 1 ? 1 : grid > 296 ? 296 : grid;
     if (rows_part) rc = launch(layernorm_bwd_narrow_kernel, grid, 32 * LN_BWD_WARPS, sizeof(float) * LN_BWD_WARPS * 3 * d, st, 1, (const bf16*)dy,
                 (const bf16*)x, gamma, mean, rstd, (const bf16*)dres, (bf16*)dx, scratch, M, d);
   } else {
-    const int W = (d + 255) / 256, groups = LN_BWD_MAX_WARPS / W, rows = groups * LN_BWD_ROWS;
-    grid = (M + rows - 1) / rows;
-    grid = grid < 1 ? 1 : grid > 148 ? 148 : grid;
+    const int W = (d + 255) / 256, groups = LN_BWD_MAX_WARPS / W;
     // stages (the block's sums, 12 bytes per column and group, fit in there afterwards) and exchange buffers
     const auto shmem = [](int threads) {
       return size_t(threads) * LN_BWD_STAGES * LN_BWD_ROWS * 48 + size_t(threads / 32) * 2 * 2 * LN_BWD_ROWS * sizeof(float);

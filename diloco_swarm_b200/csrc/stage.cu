@@ -248,7 +248,7 @@ Scratch take_scratch(Area& a, const Stage& s, size_t M, bool grad, size_t logit_
   v.datt = a.take<bf16>(M * d);
   v.dq_acc = a.take<float>(M * d);
   v.dvec = a.take<float>(M * s.nh);
-  for (float*& p : v.ln) p = a.take<float>(size_t(dsw_layernorm_bwd_blocks(int(M))) * 3 * d);
+  for (float*& p : v.ln) p = a.take<float>(dsw_layernorm_bwd_scratch(int(M), int(d)));
   return v;
 }
 

@@ -124,12 +124,12 @@ def layernorm_bwd(dy: torch.Tensor, x: torch.Tensor, gamma: torch.Tensor, mean: 
     assert dy.shape == x.shape and dy.is_contiguous() and x.is_contiguous()
     dx = torch.empty_like(x)
     lib = cuda_lib()
-    nblk = lib.dsw_layernorm_bwd_blocks(M)
-    key = (x.device.index, nblk, d)
+    floats = lib.dsw_layernorm_bwd_scratch(M, d)
+    key = (x.device.index, floats, d)
     scratch = _ln_scratch.get(key)
     if scratch is None:
         # per-block partial column sums; reused by every call of this shape (same stream order)
-        scratch = torch.empty(nblk * 3 * d, dtype=F32, device=x.device)
+        scratch = torch.empty(floats, dtype=F32, device=x.device)
         _ln_scratch[key] = scratch
     check(lib.dsw_layernorm_bwd(dy.data_ptr(), x.data_ptr(), gamma.data_ptr(), mean.data_ptr(), rstd.data_ptr(),
                                 ptr(dres), dx.data_ptr(), dgamma.data_ptr(), ptr(dbeta), ptr(dres_sum),

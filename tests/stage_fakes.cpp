@@ -139,12 +139,12 @@ int dsw_layernorm_fwd_lo(const void* x, const void* lo, const float*, const floa
   const long long n = 2LL * M * d;
   return op("layernorm_fwd", st, {{'r', x, n}, {'r', lo, n}, {'w', y, n}, {'w', mean, 4LL * M}, {'w', rstd, 4LL * M}});
 }
-int dsw_layernorm_bwd_blocks(int) { return 296; }
+int dsw_layernorm_bwd_scratch(int, int d) { return 148 * 3 * d; }
 int dsw_layernorm_bwd(const void* dy, const void* x, const float*, const float* mean, const float* rstd, const void* dres, void* dx, float*,
                       float*, float*, float* scratch, int M, int d, cudaStream_t st) {
   const long long n = 2LL * M * d;
   return op("layernorm_bwd", st, {{'r', dy, n}, {'r', x, n}, {'r', mean, 4LL * M}, {'r', rstd, 4LL * M}, {'r', dres, n}, {'w', dx, n},
-                                  {'w', scratch, 296LL * 12 * d}});
+                                  {'w', scratch, 4LL * dsw_layernorm_bwd_scratch(M, d)}});
 }
 int dsw_colsum_accum(const void* x, long long, float*, int M, int N, cudaStream_t st) {
   return op("colsum", st, {{'r', x, 2LL * M * N}});

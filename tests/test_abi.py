@@ -92,6 +92,18 @@ def test_built_libraries_export_the_declared_symbols():
     assert cuda.dsw_max_peers() == 8 and cuda.dsw_layernorm_bwd_blocks(16384) <= 296
 
 
+def test_layernorm_scratch_is_what_the_blocks_write():
+    """One row of three sums per block: one block per SM from 136 columns on (narrow rows: two), one per four rows of the
+    widest and per 32 of the narrow ones; dsw_layernorm_bwd_blocks serves every width."""
+    lib = _lib.cuda_lib()
+    for M in (1, 5, 31, 33, 300, 591, 593, 4737, 9473, 32768, 2 ** 31 - 1):
+        for d in (8, 128, 136, 256, 264, 768, 1024, 1600, 2048):
+            floats = lib.dsw_layernorm_bwd_scratch(M, d)
+            per_block = 32 if d <= 128 else 16 // -(-d // 256) * 2
+            assert floats == 3 * d * min(-(-M // per_block), 296 if d <= 128 else 148)
+            assert floats <= lib.dsw_layernorm_bwd_blocks(M) * 3 * d
+
+
 def test_wrappers_run_against_a_stub_of_the_header():
     """benchmarks/host_overhead.py: a no-op twin of the library generated from dswarm.h takes every call
     the wrappers make (argument counts and kinds fit), and the loader is put back afterwards."""
