@@ -131,12 +131,15 @@ static bool use_pair() {
 // 128 x 128.  Times in ns per k-block of a tile, fitted to launches of 2128 to 16384 rows (N and K of GPT-2 small, large
 // and xl): what an SM needs to take in its operands (some 120 bytes per ns; 32 KB for 128 x 128 and for a CTA of the wide
 // pair, 24 KB for the narrow one, 48 KB for 128 x 256), the wide pair a little more where its arithmetic shows.
-struct TileKind { int bn, bm, width, ctas; double per_kb, epilogue, setup, per_kb_wgrad, setup_wgrad; };
+// setup_gelu: what a launch with GELU without its derivative takes besides, fitted to 384 to 32768 rows of widths 128 to 1600;
+// without it the lighter epilogue drew the widest tiles where few waves do not pay for their set-up (2560 x 3072 from 768:
+// 20.7 us on 512, 18.6 on 256; 1024 x 5120 from 1280: 22.4 on 512, 19.9 on 384; 32768 x 3072 from 768 takes 512 either way).
+struct TileKind { int bn, bm, width, ctas; double per_kb, epilogue, setup, per_kb_wgrad, setup_wgrad, setup_gelu; };
 constexpr TileKind TILE_KINDS[] = {
-    {128, 128, 128, 1, 280.0, 1400.0, 3600.0, 280.0, 5000.0},
-    {256, 128, 256, 1, 390.0, 2600.0, 3600.0, 400.0, 6000.0},
-    {384, 256, 128, 2, 260.0, 1400.0, 4000.0, 260.0, 6500.0},
-    {512, 256, 256, 2, 340.0, 2600.0, 4000.0, 380.0, 7000.0},
+    {128, 128, 128, 1, 280.0, 1400.0, 3600.0, 280.0, 5000.0, 0.0},
+    {256, 128, 256, 1, 390.0, 2600.0, 3600.0, 400.0, 6000.0, 1500.0},
+    {384, 256, 128, 2, 260.0, 1400.0, 4000.0, 260.0, 6500.0, 0.0},
+    {512, 256, 256, 2, 340.0, 2600.0, 4000.0, 380.0, 7000.0, 2500.0},
 };
 static bool allowed(const TileKind& t, int M) { return t.ctas == 1 || (use_pair() && M >= 256); }
 
@@ -144,13 +147,14 @@ static bool allowed(const TileKind& t, int M) { return t.ctas == 1 || (use_pair(
 static int pick_bn(int M, int N, int K, int splits, int mode, bool derivative, int sms, double* cost) {
   const int kb = ((K + BK - 1) / BK + splits - 1) / splits;
   const double heavy = mode == EPI_GELU ? (derivative ? 2.0 : 1.4) : 1.0;      // 183, 140 and 118 us at 32768 x 3072 from 768
+  const bool gelu_only = mode == EPI_GELU && !derivative;
   int best = 128;
   double least = 1e30;
   for (const TileKind& t : TILE_KINDS) {
     if (!allowed(t, M) || (t.width > 128 && N <= 128)) continue;
     const long long tiles = (long long)((M + t.bm - 1) / t.bm) * ((N + t.width - 1) / t.width) * splits;
     const int units = sms / t.ctas;
-    const double c = t.setup + double((tiles + units - 1) / units) * fmax(kb * t.per_kb, heavy * t.epilogue) + heavy * t.epilogue;
+    const double c = t.setup + (gelu_only ? t.setup_gelu : 0.0) + double((tiles + units - 1) / units) * fmax(kb * t.per_kb, heavy * t.epilogue) + heavy * t.epilogue;
     if (c < least) { least = c; best = t.bn; }
   }
   *cost = least;

@@ -25,6 +25,18 @@ FEW_ROWS = [
     ((384, 4096, 1024, GELU, 0, 1), {"128/1": 11.84, "1128/1": 12.97, "384/1": 11.59}),
     ((256, 6400, 1600, GELU, 0, 1), {"384/1": 13.93, "1128/1": 15.73}),
 ]
+# GELU without its derivative (evaluation): "kernel / split of K" as before
+GELU_ONLY = [
+    ((1024, 3072, 768, GELU, 0, 0), {"384/1": 12.16, "512/1": 13.21}),
+    ((1536, 3072, 768, GELU, 0, 0), {"384/1": 12.6, "512/1": 13.57}),
+    ((2560, 3072, 768, GELU, 0, 0), {"256/1": 18.62, "512/1": 20.65}),
+    ((3072, 3072, 768, GELU, 0, 0), {"256/1": 18.88, "512/1": 20.67}),
+    ((8192, 3072, 768, GELU, 0, 0), {"256/1": 40.57, "512/1": 39.55}),
+    ((32768, 3072, 768, GELU, 0, 0), {"256/1": 139.9, "512/1": 132.2}),
+    ((768, 4096, 1024, GELU, 0, 0), {"384/1": 13.69, "512/1": 14.59}),
+    ((1024, 5120, 1280, GELU, 0, 0), {"384/1": 19.87, "512/1": 22.37}),
+    ((1024, 6400, 1600, GELU, 0, 0), {"384/1": 23.95, "512/1": 26.62}),
+]
 
 
 def _choice(call):
@@ -38,6 +50,12 @@ def _choice(call):
 def test_few_rows_take_a_kernel_that_is_near_the_best(call, us):
     got = _choice(call)
     assert got in us and us[got] <= 1.035 * min(us.values()), (got, us)
+
+
+@pytest.mark.parametrize("call,us", GELU_ONLY)
+def test_gelu_without_derivative_takes_a_tile_that_is_near_the_best(call, us):
+    got = _choice(call)
+    assert got in us and us[got] <= 1.02 * min(us.values()), (got, us)
 
 
 def test_the_split_of_a_call_is_that_of_its_recorded_outputs():
