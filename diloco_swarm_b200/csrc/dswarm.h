@@ -90,6 +90,8 @@ int dsw_layernorm_fwd(const void* x, const float* gamma, const float* beta, void
 // The same of x + x_lo (x_lo: bf16 like x, or null).
 int dsw_layernorm_fwd_lo(const void* x, const void* x_lo, const float* gamma, const float* beta, void* y, float* mean,
                          float* rstd, int M, int d, float eps, cudaStream_t st);
+// Blocks that dsw_layernorm_fwd launches for M rows of d columns.
+int dsw_layernorm_fwd_blocks(int M, int d);
 // The most blocks dsw_layernorm_bwd launches for M rows of any width; floats of scratch that M rows of d columns need.
 int dsw_layernorm_bwd_blocks(int M);
 int dsw_layernorm_bwd_scratch(int M, int d);

@@ -840,13 +840,22 @@ extern "C" int dsw_layernorm_fwd(const void* x, const float* gamma, const float*
   return dsw_layernorm_fwd_lo(x, nullptr, gamma, beta, y, mean, rstd, M, d, eps, st);
 }
 
+// Blocks of dsw_layernorm_fwd for rows of d columns, each warp several rows when there are that many: gamma and beta are paid
+// once per warp.  Fewer rows are spread out first: a second row per warp would only wait for the first one.  Above 768 columns
+// the registers leave room for one block per SM, and a second wave costs more than another row per warp does: 2128 x 1600 on
+// 266 blocks 8.0 us, on 133 6.1; 4736 x 1600 on 296 blocks 11.6, on 148 9.8; 32768 x 1024 33.5 and 32.8.
+extern "C" int dsw_layernorm_fwd_blocks(int M, int d) {
+  if (d <= 128) return grid_for(M, 16, 148 * 4);
+  if (d <= 768) return grid_for(M, 8, 148 * 2);
+  const int rows = M / (148 * 8) + (M % (148 * 8) > 0);          // per warp
+  return grid_for(M, 8 * (rows < 1 ? 1 : rows));
+}
+
 extern "C" int dsw_layernorm_fwd_lo(const void* x, const void* x_lo, const float* gamma, const float* beta, void* y, float* mean,
                                  float* rstd, int M, int d, float eps, cudaStream_t st) {
   if (d % 8 || d > 256 * LN_MAX_CHUNKS_ALL) return -10;
-  // Two blocks per SM (narrow rows: four), each warp several rows when there are that many: gamma and beta are paid once
-  // per warp.  Fewer rows are spread out first: a second row per warp would only wait for the first one.
   const bool two_rows = d <= 128;
-  const int grid = two_rows ? grid_for(M, 16, 148 * 4) : grid_for(M, 8, 148 * 2);
+  const int grid = dsw_layernorm_fwd_blocks(M, d);
   cudaError_t rc;
 #define LN_FWD(NCH, LPR)                                                                                             \
   rc = x_lo ? launch(layernorm_fwd_kernel<NCH, true, LPR>, grid, 256, 0, st, 1, (const bf16*)x, (const bf16*)x_lo, gamma, beta, \

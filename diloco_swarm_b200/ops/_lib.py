@@ -27,6 +27,7 @@ _SIGS = {
                              c_void_p],
     "dsw_layernorm_bwd": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                           c_void_p, c_void_p, c_int, c_int, c_void_p],
+    "dsw_layernorm_fwd_blocks": [c_int, c_int],
     "dsw_layernorm_bwd_blocks": [c_int],
     "dsw_layernorm_bwd_scratch": [c_int, c_int],
     "dsw_colsum_accum": [c_void_p, c_ll, c_void_p, c_int, c_int, c_void_p],

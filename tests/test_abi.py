@@ -112,3 +112,15 @@ def test_wrappers_run_against_a_stub_of_the_header():
     res = H.measure(iters=20, M=512, d=256)
     assert _lib._cuda is before
     assert set(res) >= {"gemm forward (bias)", "adamw step"} and all(0 < v < 1e5 for v in res.values())
+
+
+def test_layernorm_forward_is_one_wave_of_wide_rows():
+    """Above 768 columns one block fits on an SM: no more than 148 of them, and no warp with a row more than it takes."""
+    lib = _lib.cuda_lib()
+    for d in (776, 1024, 1600, 2048):
+        for M in (1, 8, 9, 600, 1184, 1185, 2128, 4737, 32768):
+            per_warp = -(-M // (148 * 8))
+            assert lib.dsw_layernorm_fwd_blocks(M, d) == -(-M // (8 * per_warp)) <= 148
+    for d, per_block, most in ((64, 16, 592), (128, 16, 592), (136, 8, 296), (768, 8, 296)):
+        for M in (1, 24, 1200, 2128, 32768):
+            assert lib.dsw_layernorm_fwd_blocks(M, d) == min(-(-M // per_block), most)
