@@ -102,6 +102,11 @@ __device__ __forceinline__ bool att_item(int r, int c, int G, int total, int& id
   return idx < total;
 }
 
+// SOLO: no more items than SMs.  A row then goes straight from its thread, 16 bytes at a time: staged through shared memory as
+// the rows of more items are, it leaves some 0.4 us later (1 x 24 tokens, 4 heads of 32: 6.4 -> 6.0 us a launch; 5 x 24, 12
+// heads of 64: 6.5 -> 6.1).  With two CTAs on an SM the stores of a row per lane get in each other's way: 16 x 128, 12 heads,
+// 192 items, 9.1 us staged, 10.0 not.
+template <bool SOLO>
 __global__ void __launch_bounds__(ATT_THREADS, 2)
 attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, __nv_bfloat16* __restrict__ out,
                      float* __restrict__ lse_out, int T, int nh, int n_bh, int hs, float scale_log2, int* status,
@@ -392,29 +397,42 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, __nv_bfloat16
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(o_free);          // the next item's first product may overwrite the rows
-      // The warp's 32 rows pass through its own rows of the P tile, which no product reads any more, so that a store
-      // covers four whole rows of 128 bytes: a lane that stores its own row 16 bytes at a time touches 32 lines with
-      // every instruction (32 x 1024 tokens, 12 heads of 64: 135.6 -> 129.0 us; 16 x 1024: 72.9 -> 68.6).
-      uint8_t* so = sp + warp * 32 * 128;
+      if constexpr (SOLO) {
+        __nv_bfloat16* dst = out + ((long long)b * T + qi * ATT_BQ + r) * d + h * hs;
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        const uint32_t* o = ov[c >> 2] + (c & 3) * 8;
-        *reinterpret_cast<uint4*>(so + lane * 128 + ((c ^ (lane & 7)) << 4)) =
-            make_uint4(pack_bf16(__uint_as_float(o[0]) * inv, __uint_as_float(o[1]) * inv),
-                       pack_bf16(__uint_as_float(o[2]) * inv, __uint_as_float(o[3]) * inv),
-                       pack_bf16(__uint_as_float(o[4]) * inv, __uint_as_float(o[5]) * inv),
-                       pack_bf16(__uint_as_float(o[6]) * inv, __uint_as_float(o[7]) * inv));
-      }
-      __syncwarp();
-      const int ch = lane & 7, t0 = qi * ATT_BQ + warp * 32 + (lane >> 3);
-      __nv_bfloat16* dst = out + ((long long)b * T + t0) * d + h * hs + ch * 8;
+        for (int c = 0; c < 8; ++c)
+          if (c * 8 < hs && in_seq) {
+            const uint32_t* o = ov[c >> 2] + (c & 3) * 8;
+            *reinterpret_cast<uint4*>(dst + c * 8) = make_uint4(pack_bf16(__uint_as_float(o[0]) * inv, __uint_as_float(o[1]) * inv),
+                                                                pack_bf16(__uint_as_float(o[2]) * inv, __uint_as_float(o[3]) * inv),
+                                                                pack_bf16(__uint_as_float(o[4]) * inv, __uint_as_float(o[5]) * inv),
+                                                                pack_bf16(__uint_as_float(o[6]) * inv, __uint_as_float(o[7]) * inv));
+          }
+      } else {
+        // The warp's 32 rows pass through its own rows of the P tile, which no product reads any more, so that a store
+        // covers four whole rows of 128 bytes: a lane that stores its own row 16 bytes at a time touches 32 lines with
+        // every instruction (32 x 1024 tokens, 12 heads of 64: 135.6 -> 129.0 us; 16 x 1024: 72.9 -> 68.6).
+        uint8_t* so = sp + warp * 32 * 128;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int rl = i * 4 + (lane >> 3);
-        const uint4 w = *reinterpret_cast<const uint4*>(so + rl * 128 + ((ch ^ (rl & 7)) << 4));
-        if (t0 + i * 4 < T && ch * 8 < hs) *reinterpret_cast<uint4*>(dst + (long long)i * 4 * d) = w;
+        for (int c = 0; c < 8; ++c) {
+          const uint32_t* o = ov[c >> 2] + (c & 3) * 8;
+          *reinterpret_cast<uint4*>(so + lane * 128 + ((c ^ (lane & 7)) << 4)) =
+              make_uint4(pack_bf16(__uint_as_float(o[0]) * inv, __uint_as_float(o[1]) * inv),
+                         pack_bf16(__uint_as_float(o[2]) * inv, __uint_as_float(o[3]) * inv),
+                         pack_bf16(__uint_as_float(o[4]) * inv, __uint_as_float(o[5]) * inv),
+                         pack_bf16(__uint_as_float(o[6]) * inv, __uint_as_float(o[7]) * inv));
+        }
+        __syncwarp();
+        const int ch = lane & 7, t0 = qi * ATT_BQ + warp * 32 + (lane >> 3);
+        __nv_bfloat16* dst = out + ((long long)b * T + t0) * d + h * hs + ch * 8;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int rl = i * 4 + (lane >> 3);
+          const uint4 w = *reinterpret_cast<const uint4*>(so + rl * 128 + ((ch ^ (rl & 7)) << 4));
+          if (t0 + i * 4 < T && ch * 8 < hs) *reinterpret_cast<uint4*>(dst + (long long)i * 4 * d) = w;
+        }
+        __syncwarp();                                // read out before the next item's P is written here
       }
-      __syncwarp();                                // read out before the next item's P is written here
       // natural-log LSE of the scaled scores
       if (in_seq) lse_out[(long long)bh * T + qi * ATT_BQ + r] = (m + log2f(l)) * 0.6931471805599453f;
     }
@@ -1173,16 +1191,16 @@ extern "C" int dsw_attention_fwd(const void* qkv, void* out, float* lse, int B, 
   if (rc) return rc;
   static bool attr_set = false;
   if (!attr_set) {
-    if (cudaFuncSetAttribute(attention_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AttSmem::TOTAL) !=
-        cudaSuccess)
+    if (cudaFuncSetAttribute(attention_fwd_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, AttSmem::TOTAL) != cudaSuccess ||
+        cudaFuncSetAttribute(attention_fwd_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, AttSmem::TOTAL) != cudaSuccess)
       return -2;
     attr_set = true;
   }
   // persistent: two CTAs per SM walk the work items
   const int total = ((T + ATT_BQ - 1) / ATT_BQ) * B * nh;
   const int G = total < 2 * att_num_sms() ? total : 2 * att_num_sms();
-  return launch(attention_fwd_kernel, G, ATT_THREADS, AttSmem::TOTAL, st, 1, tm, (__nv_bfloat16*)out, lse, T, nh, B * nh, hs,
-                scale * 1.4426950408889634f, status, g_att_trace) == cudaSuccess ? 0 : -3;
+  return launch(total <= att_num_sms() ? attention_fwd_kernel<true> : attention_fwd_kernel<false>, G, ATT_THREADS, AttSmem::TOTAL, st, 1,
+                tm, (__nv_bfloat16*)out, lse, T, nh, B * nh, hs, scale * 1.4426950408889634f, status, g_att_trace) == cudaSuccess ? 0 : -3;
 }
 
 // qkv, out, dout as in the forward; lse from the forward.  dqkv: bf16 [B*T, 3*d] (all of it is written).
@@ -1252,7 +1270,8 @@ extern "C" int dsw_attention_bwd_ordered(const void* qkv, const void* out, const
 extern "C" int dsw_load_attention() {
   cudaFuncAttributes a;
   int bad = 0;
-  bad |= cudaFuncGetAttributes(&a, attention_fwd_kernel) != cudaSuccess;
+  bad |= cudaFuncGetAttributes(&a, attention_fwd_kernel<true>) != cudaSuccess;
+  bad |= cudaFuncGetAttributes(&a, attention_fwd_kernel<false>) != cudaSuccess;
   bad |= cudaFuncGetAttributes(&a, attention_bwd_kernel<false>) != cudaSuccess;
   bad |= cudaFuncGetAttributes(&a, attention_bwd_kernel<true>) != cudaSuccess;
   bad |= cudaFuncGetAttributes(&a, attention_bwd_prep_kernel) != cudaSuccess;
