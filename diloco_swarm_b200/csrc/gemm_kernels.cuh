@@ -44,6 +44,7 @@ enum EpiMode : int {
   // EPI_GELU without aux_out, on the kernels for many rows: evaluation and sampling drop the derivative, whose arithmetic
   // and registers the class with aux_out carries all the same (32768 x 3072 from 768, CTA pairs: 144.8 -> 136.7 us)
   EPI_GELU_ONLY = 9,
+  EPI_MUL_SUM = 10,     // EPI_MUL with colsum, whose code and registers a product without it does not carry
 };
 
 // What the second pass over the logits needs to know of a row: {log2-sum-exp2, factor (0: the row is masked), target as
@@ -316,7 +317,8 @@ __device__ __forceinline__ void epilogue_warp(const GemmArgs& g, uint32_t t_addr
     }
   } else {
     constexpr int NCH = NCOLS / 32;
-    constexpr bool EXTRA = MODE == EPI_RESID || MODE == EPI_MUL;
+    constexpr bool MUL = MODE == EPI_MUL || MODE == EPI_MUL_SUM;
+    constexpr bool EXTRA = MODE == EPI_RESID || MUL;
     const int my_ch = lane & 3, my_r = lane >> 2;
     uint32_t r[32];
     tmem_ld_32x32(t_addr, r);
@@ -396,9 +398,9 @@ __device__ __forceinline__ void epilogue_warp(const GemmArgs& g, uint32_t t_addr
       __syncwarp();                                   // the previous chunk has been read out
       stage_row64(stage, lane, w);
       __syncwarp();
-      // sums of the output's columns (EPI_MUL with colsum): of this lane's rows, then over the warp's 32
-      float cs[MODE == EPI_MUL ? 8 : 1];
-      if constexpr (MODE == EPI_MUL) {
+      // sums of the output's columns (EPI_MUL_SUM): of this lane's rows, then over the warp's 32
+      float cs[MODE == EPI_MUL_SUM ? 8 : 1];
+      if constexpr (MODE == EPI_MUL_SUM) {
 #pragma unroll
         for (int e = 0; e < 8; ++e) cs[e] = 0.f;
       }
@@ -411,10 +413,10 @@ __device__ __forceinline__ void epilogue_warp(const GemmArgs& g, uint32_t t_addr
           const uint32_t xu[4] = {x[i].x, x[i].y, x[i].z, x[i].w};
           // Both operands are bf16 by now, so one packed bf16 instruction does what unpacking, an fp32 product or sum and
           // packing did in seven, with the same single rounding (a product of two bf16 values is exact in fp32).
-          if constexpr (MODE == EPI_MUL) {
+          if constexpr (MUL) {
 #pragma unroll
             for (int q = 0; q < 4; ++q) du[q] = mul_bf16x2(du[q], xu[q]);
-            if (g.colsum != nullptr) {
+            if constexpr (MODE == EPI_MUL_SUM) {
 #pragma unroll
               for (int q = 0; q < 4; ++q) {
                 const float2 e = unpack_bf16(du[q]);
@@ -430,13 +432,11 @@ __device__ __forceinline__ void epilogue_warp(const GemmArgs& g, uint32_t t_addr
         }
         *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(g.out) + (long long)row * g.ldo + col) = d;
       });
-      if constexpr (MODE == EPI_MUL) {
+      if constexpr (MODE == EPI_MUL_SUM) {
         // In place of a pass that reads the output once more (32768 x 3072: 40 us); here 150 -> 168 us with K = 768.
-        if (g.colsum != nullptr) {
-          // over the eight lanes that hold the same columns: lane ends with column e of its eight
-          const int e = sum_rows_of_8(cs, lane), col = cb + my_ch * 8 + e;
-          if (col < g.N) atomicAdd(g.colsum + col, cs[0]);
-        }
+        // Over the eight lanes that hold the same columns: lane ends with column e of its eight.
+        const int e = sum_rows_of_8(cs, lane), col = cb + my_ch * 8 + e;
+        if (col < g.N) atomicAdd(g.colsum + col, cs[0]);
       }
       if constexpr (MODE == EPI_GELU) {
         __syncwarp();
@@ -456,9 +456,10 @@ __device__ __forceinline__ void epilogue_warp(const GemmArgs& g, uint32_t t_addr
 // Same lane-to-address map as the loads in epilogue_warp; one request per 32-byte sector.
 template <int MODE, int NCOLS>
 __device__ __forceinline__ void prefetch_extra(const GemmArgs& g, int row_base, int lane, int col_base) {
-  if constexpr (MODE == EPI_RESID || MODE == EPI_RESID_LO || MODE == EPI_MUL) {
-    const __nv_bfloat16* src = MODE == EPI_MUL ? g.aux_in : g.resid;
-    const long long ld = MODE == EPI_MUL ? g.ldaux : g.ldr;
+  if constexpr (MODE == EPI_RESID || MODE == EPI_RESID_LO || MODE == EPI_MUL || MODE == EPI_MUL_SUM) {
+    constexpr bool MUL = MODE == EPI_MUL || MODE == EPI_MUL_SUM;
+    const __nv_bfloat16* src = MUL ? g.aux_in : g.resid;
+    const long long ld = MUL ? g.ldaux : g.ldr;
     if (lane & 1) return;
 #pragma unroll
     for (int c = 0; c < NCOLS / 32; ++c) {
@@ -929,6 +930,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 inline int epi_class(const GemmArgs& g) {
   if (g.mode == EPI_STORE_F32) return EPI_ATOMIC_F32;
   if (g.mode == EPI_GELU && g.aux_out == nullptr) return EPI_GELU_ONLY;
+  if (g.mode == EPI_MUL && g.colsum != nullptr) return EPI_MUL_SUM;
   return g.mode == EPI_RESID && (g.aux_in != nullptr || g.aux_out != nullptr) ? EPI_RESID_LO : g.mode;
 }
 

@@ -36,6 +36,7 @@ int launch_bn(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& g, i
     case EPI_RESID: return launch_pair_mode<BN, EPI_RESID>(ta, tb, g, num_sms, max_ctas, st);
     case EPI_RESID_LO: return launch_pair_mode<BN, EPI_RESID_LO>(ta, tb, g, num_sms, max_ctas, st);
     case EPI_MUL: return launch_pair_mode<BN, EPI_MUL>(ta, tb, g, num_sms, max_ctas, st);
+    case EPI_MUL_SUM: return launch_pair_mode<BN, EPI_MUL_SUM>(ta, tb, g, num_sms, max_ctas, st);
     case EPI_ATOMIC_F32: return launch_pair_mode<BN, EPI_ATOMIC_F32>(ta, tb, g, num_sms, max_ctas, st);
     case EPI_STORE: return launch_pair_mode<BN, EPI_STORE>(ta, tb, g, num_sms, max_ctas, st);
     default: break;
@@ -57,6 +58,7 @@ int load_bn() {
   bad |= cudaFuncGetAttributes(&a, gemm_pair_kernel<BN, EPI_RESID>) != cudaSuccess;
   bad |= cudaFuncGetAttributes(&a, gemm_pair_kernel<BN, EPI_RESID_LO>) != cudaSuccess;
   bad |= cudaFuncGetAttributes(&a, gemm_pair_kernel<BN, EPI_MUL>) != cudaSuccess;
+  bad |= cudaFuncGetAttributes(&a, gemm_pair_kernel<BN, EPI_MUL_SUM>) != cudaSuccess;
   bad |= cudaFuncGetAttributes(&a, gemm_pair_kernel<BN, EPI_ATOMIC_F32>) != cudaSuccess;
   if constexpr (BN == 256) {
     bad |= cudaFuncGetAttributes(&a, gemm_pair_kernel<BN, EPI_LSE>) != cudaSuccess;

@@ -32,7 +32,7 @@ int launch_bn(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& g, c
     case EPI_STORE: return launch_one<BN, EPI_STORE>(ta, tb, g, st);
     case EPI_GELU: return launch_one<BN, EPI_GELU>(ta, tb, g, st);
     case EPI_RESID: return launch_one<BN, EPI_RESID>(ta, tb, g, st);
-    case EPI_MUL: return launch_one<BN, EPI_MUL>(ta, tb, g, st);
+    case EPI_MUL: return g.colsum ? launch_one<BN, EPI_MUL_SUM>(ta, tb, g, st) : launch_one<BN, EPI_MUL>(ta, tb, g, st);
     default: return -13;
   }
 }
@@ -45,6 +45,7 @@ int load_bn() {
   bad |= cudaFuncGetAttributes(&a, gemm_split_kernel<BN, EPI_GELU>) != cudaSuccess;
   bad |= cudaFuncGetAttributes(&a, gemm_split_kernel<BN, EPI_RESID>) != cudaSuccess;
   bad |= cudaFuncGetAttributes(&a, gemm_split_kernel<BN, EPI_MUL>) != cudaSuccess;
+  bad |= cudaFuncGetAttributes(&a, gemm_split_kernel<BN, EPI_MUL_SUM>) != cudaSuccess;
   return bad;
 }
 }  // namespace

@@ -156,7 +156,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     const int r = quarter * 32 + lane, row = m0 + r;
     constexpr int UT = U / 2;           // units of this thread: u0 .. u0 + UT - 1
     const int u0 = half * UT;
-    constexpr bool EXTRA = MODE == EPI_RESID || MODE == EPI_MUL;
+    constexpr bool EXTRA = MODE == EPI_RESID || MODE == EPI_MUL || MODE == EPI_MUL_SUM;
     uint4 x[EXTRA ? UT : 1], t[MODE == EPI_RESID ? UT : 1];
     // Everything from global memory is asked for before the accumulator is waited for, the bias (older than the kernel
     // before, like the weights) even before that kernel has ended.
@@ -218,8 +218,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 #pragma unroll
     for (int i = 0; i < UT; ++i) {
       const int u = u0 + i, col = n0 + u * 8;
-      float out8[MODE == EPI_MUL ? 8 : 1];          // of a row that exists, else zeros
-      if constexpr (MODE == EPI_MUL) {
+      float out8[MODE == EPI_MUL_SUM ? 8 : 1];          // of a row that exists, else zeros
+      if constexpr (MODE == EPI_MUL_SUM) {
 #pragma unroll
         for (int e = 0; e < 8; ++e) out8[e] = 0.f;
       }
@@ -265,7 +265,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           }
 #pragma unroll
           for (int e = 0; e < 4; ++e) w[e] = pack_bf16(f[2 * e], f[2 * e + 1]);
-          if constexpr (MODE == EPI_MUL) {
+          if constexpr (MODE == EPI_MUL_SUM) {
 #pragma unroll
             for (int e = 0; e < 8; ++e) out8[e] = f[e];
           }
@@ -282,8 +282,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(g.out) + (long long)row * g.ldo + col) =
             make_uint4(w[0], w[1], w[2], w[3]);
       }
-      if constexpr (MODE == EPI_MUL) {
-        if (g.colsum != nullptr && owner_of(u) == ks && col < g.N) {          // the same for the whole warp
+      if constexpr (MODE == EPI_MUL_SUM) {
+        if (owner_of(u) == ks && col < g.N) {          // the same for the whole warp
           const float sum = warp_sums(out8);
           if ((lane & 3) == 0) atomicAdd(g.colsum + col + (lane >> 2), sum);
         }
