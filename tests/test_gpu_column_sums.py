@@ -7,50 +7,80 @@ from helpers import make_config, single_world
 pytestmark = pytest.mark.gpu
 
 
-# few rows (cluster kernel), several tiles (many rows), one and two tiles per sequence, rows that end inside a tile;
-# head sizes 32 and 64
-@pytest.mark.parametrize("B,T", [(1, 1), (3, 50), (1, 128), (2, 129), (9, 128), (20, 100), (6, 256)])
-@pytest.mark.parametrize("heads,width", [(4, 128), (4, 256), (12, 768)])
-def test_sums_are_those_of_a_pass_of_their_own(B, T, heads, width):
+def _engine(heads, width):
     from diloco_swarm_b200.models.engine_b200 import B200Engine
     from diloco_swarm_b200.models.gpt2 import GPT2Config
-    from diloco_swarm_b200.ops import kernels as K
     cfg = make_config(model={"n_layer": 2, "n_head": heads, "n_embd": width, "vocab_size": 512, "block_size": 256})
-    eng = B200Engine(GPT2Config(block_size=256, vocab_size=512, n_layer=2, n_head=heads, n_embd=width), single_world(), cfg,
-                     torch.device("cuda", 0))
+    return B200Engine(GPT2Config(block_size=256, vocab_size=512, n_layer=2, n_head=heads, n_embd=width), single_world(), cfg,
+                      torch.device("cuda", 0))
+
+
+# few rows, whose sums stay a pass of their own; the cluster kernel and the kernels for many rows; one and two tiles per
+# sequence, rows that end inside a tile, several items per CTA; head sizes 32 and 64
+@pytest.mark.parametrize("B,T", [(1, 1), (3, 50), (1, 128), (2, 129), (9, 128), (20, 100), (6, 256), (40, 128)])
+@pytest.mark.parametrize("heads,width", [(4, 128), (4, 256), (12, 768)])
+def test_sums_are_those_of_the_terms(B, T, heads, width, monkeypatch):
+    from diloco_swarm_b200.models import engine_b200
+    from diloco_swarm_b200.ops import kernels as K
+    from diloco_swarm_b200.ops._lib import cuda_lib
+    eng = _engine(heads, width)
     gen = torch.Generator(device="cuda").manual_seed(7)
     ids = torch.randint(0, 512, (B, T + 1), device="cuda", generator=gen)
     mask = torch.ones(B, T, dtype=torch.long, device="cuda")
-    got = []
-    for apart in (True, False):
+
+    def backward():
         eng.grad.zero_()
-        K.set_deterministic(apart)          # sums in atomics are not for a deterministic backward
-        try:
-            eng.forward_backward(0, ids[:, :-1].contiguous(), None, ids[:, 1:].contiguous(), mask, 1.0)
-        finally:
-            K.set_deterministic(False)
+        eng.forward_backward(0, ids[:, :-1].contiguous(), None, ids[:, 1:].contiguous(), mask, 1.0)
         torch.cuda.synchronize()
         eng.check_status()
-        got.append({k: eng.g32(k).double().clone() for k, _, _ in eng.specs if k.endswith("bias")})
+
+    def launches(deterministic):
+        K.set_deterministic(deterministic)
+        before = cuda_lib().dsw_stage_launches()
+        try:
+            backward()
+        finally:
+            K.set_deterministic(False)
+        return cuda_lib().dsw_stage_launches() - before
+
+    # a deterministic backward has two passes per block more, and queues the embedding's gradient elsewhere
+    ordered = launches(True)
+    want = {k: eng.g32(k).double().clone() for k, _, _ in eng.specs}
+    assert ordered + 1 - launches(False) == (4 if B * T >= 256 else 0)
+    got = {k: eng.g32(k).double().clone() for k, _, _ in eng.specs}
+    # the same backward launch by launch, where dh and dqkv are at hand: the size of the terms
+    size, summed = {}, K.colsum_accum
+
+    def record(x, out):
+        size[out.data_ptr()] = x.double().square().sum(0).sqrt()
+        summed(x, out)
+    monkeypatch.setattr(engine_b200.K, "colsum_accum", record)
+    eng.exec = None
+    backward()
     seen = 0
-    for k, a in got[0].items():
-        b = got[1][k]
-        # terms rounded to bf16 (2^-9 of each) on one side, fp32 on the other; rows are independent, so the sums differ by less
-        # than one rounding of the terms' norm, which the sum's norm over the columns is not below by more than sqrt(rows)
-        assert (a - b).norm() <= 2 ** -8 * a.norm() * max(1.0, (B * T) ** 0.5 / 8) + 1e-9, k
-        seen += "c_fc" in k or "c_attn" in k
-    assert seen == 4
+    for k in got:
+        t = size.get(eng.g32(k).data_ptr())
+        if t is None:
+            continue
+        # q, k and v by themselves: the sum of v's terms is the largest, that of k's is zero but for their rounding
+        for part in range(3 if "c_attn" in k else 1):
+            n = t.numel() // (3 if "c_attn" in k else 1)
+            off, whole, terms = (v[part * n:(part + 1) * n].norm() for v in (got[k] - want[k], want[k], t))
+            # the terms are the same, rounded to bf16 on one side: each by at most 2^-9 of itself, one independent of the other.
+            # The fp32 sums are good to 2^-20 of the whole.
+            bound = 2 ** -9 * terms + 2 ** -20 * whole + 1e-12
+            assert off <= bound, (k, part, float(off / bound))
+            # and a sum that is missing would be noticed; one token has no gradient of q and k
+            assert whole > 8 * bound or ("c_attn" in k and (part == 1 or (part == 0 and T == 1))), (k, part, float(whole / bound))
+            seen += 1
+    assert seen == 8
 
 
 @pytest.mark.parametrize("B,T", [(1, 24), (1, 128), (2, 100), (1, 255)])
 @pytest.mark.parametrize("heads,width", [(4, 128), (12, 768)])
 def test_few_rows_repeat_themselves(B, T, heads, width):
     """Up to 255 rows every sum of a bias gradient is added up in one order, so the same pass gives the same bits."""
-    from diloco_swarm_b200.models.engine_b200 import B200Engine
-    from diloco_swarm_b200.models.gpt2 import GPT2Config
-    cfg = make_config(model={"n_layer": 2, "n_head": heads, "n_embd": width, "vocab_size": 512, "block_size": 256})
-    eng = B200Engine(GPT2Config(block_size=256, vocab_size=512, n_layer=2, n_head=heads, n_embd=width), single_world(), cfg,
-                     torch.device("cuda", 0))
+    eng = _engine(heads, width)
     gen = torch.Generator(device="cuda").manual_seed(11)
     ids = torch.randint(0, 512, (B, T + 1), device="cuda", generator=gen)
     mask = torch.ones(B, T, dtype=torch.long, device="cuda")
