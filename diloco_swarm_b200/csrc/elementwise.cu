@@ -419,7 +419,9 @@ layernorm_bwd_finish_kernel(const float* partial, int nblocks, int d, float* __r
     for (int y = 0; y < 32; ++y) t += sh[y][threadIdx.x];
     const int which = i / d, c = i - which * d;
     float* dst = which == 0 ? dgamma : (which == 1 ? dbeta : dres_sum);
-    if (dst) dst[c] += t;
+    // one addition per launch, but another pass's may come at the same time: this one runs beside the main stream, and a graph
+    // that the caller has captured starts without waiting for what passes outside of it have put there
+    if (dst) atomicAdd(dst + c, t);
   }
 }
 
@@ -474,7 +476,7 @@ colsum_kernel(const __nv_bfloat16* x, long long ld, float* __restrict__ out, int
 }
 
 // The same with one order of additions at any number of rows: the eight blocks of a cluster share 256 columns, their sums
-// meet in the first one's shared memory, and it is the only writer.  For deterministic gradients: eight blocks per
+// meet in the first one's shared memory, and it adds them up.  For deterministic gradients: eight blocks per
 // 256 columns do not fill the GPU (32768 x 3072: 135 us, with atomics 33).
 constexpr int COLSUM_CLUSTER = 8;
 __global__ void __launch_bounds__(256)
@@ -493,7 +495,7 @@ colsum_ordered_kernel(const __nv_bfloat16* x, long long ld, float* __restrict__ 
   float t = 0.f;
 #pragma unroll
   for (int k = 0; k < COLSUM_CLUSTER; ++k) t += parts[k][threadIdx.x];
-  out[col0 + threadIdx.x] += t;
+  atomicAdd(out + col0 + threadIdx.x, t);          // as every gradient that the side stream adds to (layernorm_bwd_finish_kernel)
 }
 
 // ------------------------------------------------------------------ embedding

@@ -1,6 +1,6 @@
 """The stage executor's host code (csrc/stage.cu) compiled against stand-ins (stage_fakes.cpp), and a device that runs what
 it queues: streams, events, graph captures and replays with their ordering rules, and every kernel as the ranges that it
-reads and writes.  Two accesses of one range, one of them a write, that nothing orders are a race."""
+reads, writes and adds to.  Two accesses of one range that nothing orders are a race, unless both read or both add."""
 import ctypes
 import os
 import shutil
@@ -47,7 +47,7 @@ class Device:
         self.names.append(name)
         for how, at, n in ranges:
             for how2, at2, n2, s2, when, name2 in self.accesses:
-                if (how, how2) != ("r", "r") and at < at2 + n2 and at2 < at + n and c.get(s2, 0) < when:
+                if (how != how2 or how == "w") and at < at2 + n2 and at2 < at + n and c.get(s2, 0) < when:
                     self.races.append((name2, how2, name, how))
             self.accesses.append((how, at, n, s, c[s], name))
 
@@ -187,7 +187,7 @@ class FakeStage:
 
     def __init__(self, lib, n=2, d=64, heads=1, vocab=512, first=True, last=True, side=7):
         self.lib, self.n, self.d, self.vocab, self.first, self.last = lib, n, d, vocab, first, last
-        p = iter(range(1 << 50, 1 << 51, 1 << 20))
+        p = iter(range(1 << 50, 1 << 51, 1 << 24))
         ends = [next(p) if have else 0 for have in [first] * 4 + [last] * 7]
         desc = [n, d, heads, vocab, 0, side] + ends[:4] + ends[4:8] + ends[8:11] + [next(p) for _ in range(24 * n)]
         h = ctypes.c_void_p()

@@ -1,9 +1,10 @@
 // Stand-ins for what the stage executor (csrc/stage.cu) calls: the CUDA runtime's streams, events and graphs and the
 // library's own launchers.  Each hands one line of text to the test, which emulates the device and gives the return code:
-//   launch <name> <stream> [r <address> <bytes> | w <address> <bytes>]...
+//   launch <name> <stream> [r <address> <bytes> | w <address> <bytes> | a <address> <bytes>]...
+//   (reads, writes, and atomic additions, which are in nobody's way but a read's or a write's)
 //   record <event> <stream> | wait <stream> <event> | begin <stream> | end <stream> | instantiate <graph> |
 //   replay <graph> <stream> | sync <event> | query <event> | destroy <graph> | status <stream> | id <stream>
-// Gradients that kernels add to (commutative, any order) are left out; nothing is ever dereferenced.
+// Nothing is ever dereferenced.
 #include <cuda_runtime.h>
 #include <cstdlib>
 #include <initializer_list>
@@ -20,6 +21,14 @@ static long long (*g_hook)(const char*) = nullptr;
 static long long g_handles = 1000;
 static int g_sms = 148;
 extern "C" void fake_set_sms(int n) { g_sms = n; }
+// Whether the launchers take the column sums that they are asked for (LaunchMode::colsum).
+static bool g_take_columns = true;
+extern "C" void fake_take_columns(int on) { g_take_columns = on; }
+static float* take_columns() {
+  float* const to = g_take_columns ? dsw::tl_launch.colsum : nullptr;
+  if (to) dsw::tl_launch.colsum = nullptr;
+  return to;
+}
 // Allocation number n from now on fails (-1: none does).
 static long long g_failing = -1;
 extern "C" void fake_fail_allocation(long long n) { g_failing = n; }
@@ -96,8 +105,9 @@ int dsw_gemm_bf16(const void* A, long long lda, int a_mn, const void* B, long lo
                   void* out, long long ldo, const float*, const void* resid, long long, void* aux_out, const void* aux_in, long long,
                   int, int, int*, cudaStream_t st) {
   const long long mn = 2LL * M * N;
+  float* const columns = mode == DSW_EPI_MUL ? take_columns() : nullptr;
   return op("gemm", st, {{'r', A, 2LL * M * K}, {'r', B, 2LL * N * K}, {'r', resid, mn}, {'r', aux_in, mn}, {'w', aux_out, mn},
-                         {'w', mode == DSW_EPI_ATOMIC_F32 ? nullptr : out, mode >= DSW_EPI_ATOMIC_F32 ? 2 * mn : mn}});
+                         {mode == DSW_EPI_ATOMIC_F32 ? 'a' : 'w', out, mode >= DSW_EPI_ATOMIC_F32 ? 2 * mn : mn}, {'a', columns, 4LL * N}});
 }
 int dsw_head_lse(const void* A, const void*, const long long*, float* parts, float* tlogit, int M, int N, int K, int*, cudaStream_t st) {
   return op("head_lse", st, {{'r', A, 2LL * M * K}, {'w', parts, (N + 63) / 64 * 4LL * M}, {'w', tlogit, 4LL * M}});
@@ -123,8 +133,9 @@ int dsw_attention_fwd(const void* qkv, void* out, float* lse, int B, int T, int 
 int dsw_attention_bwd(const void* qkv, const void* out, const void* dout, const float* lse, void* dqkv, float* dq_acc, float* Dvec, int B,
                       int T, int nh, int hs, float, int*, cudaStream_t st) {
   const long long n = 2LL * B * T * nh * hs;
+  float* const columns = take_columns();
   return op("attention_bwd", st, {{'r', qkv, 3 * n}, {'r', out, n}, {'r', dout, n}, {'r', lse, 4LL * B * T * nh}, {'w', dqkv, 3 * n},
-                                  {'w', dq_acc, 2 * n}, {'w', Dvec, 4LL * B * T * nh}});
+                                  {'w', dq_acc, 2 * n}, {'w', Dvec, 4LL * B * T * nh}, {'a', columns, 12LL * nh * hs}});
 }
 int dsw_attention_bwd_ordered(const void* qkv, const void* out, const void* dout, const float* lse, void* dqkv, float* dq_acc, float* Dvec,
                               int B, int T, int nh, int hs, float scale, int* status, cudaStream_t st) {
@@ -140,23 +151,27 @@ int dsw_layernorm_fwd_lo(const void* x, const void* lo, const float*, const floa
   return op("layernorm_fwd", st, {{'r', x, n}, {'r', lo, n}, {'w', y, n}, {'w', mean, 4LL * M}, {'w', rstd, 4LL * M}});
 }
 int dsw_layernorm_bwd_scratch(int, int d) { return 148 * 3 * d; }
-int dsw_layernorm_bwd(const void* dy, const void* x, const float*, const float* mean, const float* rstd, const void* dres, void* dx, float*,
-                      float*, float*, float* scratch, int M, int d, cudaStream_t st) {
-  const long long n = 2LL * M * d;
-  return op("layernorm_bwd", st, {{'r', dy, n}, {'r', x, n}, {'r', mean, 4LL * M}, {'r', rstd, 4LL * M}, {'r', dres, n}, {'w', dx, n},
-                                  {'w', scratch, 4LL * dsw_layernorm_bwd_scratch(M, d)}});
+int dsw_layernorm_bwd(const void* dy, const void* x, const float*, const float* mean, const float* rstd, const void* dres, void* dx,
+                      float* dgamma, float* dbeta, float* dres_sum, float* scratch, int M, int d, cudaStream_t st) {
+  const long long n = 2LL * M * d, sums = 4LL * dsw_layernorm_bwd_scratch(M, d);
+  if (dx) {
+    const int rc = op("layernorm_bwd", st, {{'r', dy, n}, {'r', x, n}, {'r', mean, 4LL * M}, {'r', rstd, 4LL * M}, {'r', dres, n},
+                                            {'w', dx, n}, {'w', scratch, sums}});
+    if (rc || !(dgamma || dbeta || dres_sum)) return rc;
+  }
+  return op("layernorm_sums", st, {{'r', scratch, sums}, {'a', dgamma, 4LL * d}, {'a', dbeta, 4LL * d}, {'a', dres_sum, 4LL * d}});
 }
-int dsw_colsum_accum(const void* x, long long, float*, int M, int N, cudaStream_t st) {
-  return op("colsum", st, {{'r', x, 2LL * M * N}});
+int dsw_colsum_accum(const void* x, long long, float* out, int M, int N, cudaStream_t st) {
+  return op("colsum", st, {{'r', x, 2LL * M * N}, {'a', out, 4LL * N}});
 }
-int dsw_colsum_ordered(const void* x, long long, float*, int M, int N, cudaStream_t st) {
-  return op("colsum_ordered", st, {{'r', x, 2LL * M * N}});
+int dsw_colsum_ordered(const void* x, long long, float* out, int M, int N, cudaStream_t st) {
+  return op("colsum_ordered", st, {{'r', x, 2LL * M * N}, {'a', out, 4LL * N}});
 }
 int dsw_embedding_fwd(const long long* ids, const float*, const float*, void* y, int B, int T, int d, int, int*, cudaStream_t st) {
   return op("embedding_fwd", st, {{'r', ids, 8LL * B * T}, {'w', y, 2LL * B * T * d}});
 }
-int dsw_embedding_bwd(const long long* ids, const void* dx, float*, float*, int B, int T, int d, int, cudaStream_t st) {
-  return op("embedding_bwd", st, {{'r', ids, 8LL * B * T}, {'r', dx, 2LL * B * T * d}});
+int dsw_embedding_bwd(const long long* ids, const void* dx, float* dwte, float* dwpe, int B, int T, int d, int V, cudaStream_t st) {
+  return op("embedding_bwd", st, {{'r', ids, 8LL * B * T}, {'r', dx, 2LL * B * T * d}, {'a', dwte, 4LL * V * d}, {'w', dwpe, 4LL * T * d}});
 }
 int dsw_loss_begin(const long long*, int, float*, float*, cudaStream_t st) { return op("loss_begin", st, {}); }
 int dsw_cross_entropy(void* logits, long long, const long long*, const long long*, const float*, float, float*, int M, int V, int grad, int*,

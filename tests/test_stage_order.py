@@ -42,6 +42,35 @@ def test_microbatches_on_one_stream(device, blocks, vocab, chunks, B, T):
     assert ("replay" in device.counts) == (B * T <= 8192)
 
 
+@pytest.mark.parametrize("how,passes", [("asked", (0, 0)), ("refused", (4, 0)), ("few rows", (4, 0)), ("deterministic", (0, 4))])
+@pytest.mark.parametrize("side", [7, 0])
+@pytest.mark.parametrize("blocks", [2, 3])
+def test_bias_gradients_and_their_order(device, how, passes, side, blocks):
+    """The sums of dh and dqkv come out of the kernels that write them (asked), out of a pass over each where a launcher
+    leaves them (refused) or the rows are few, and out of an ordered pass in a deterministic backward: queued, captured and
+    replayed, every access of a bias gradient, a LayerNorm's sums and the work areas is ordered."""
+    device.lib.fake_take_columns(how != "refused")
+    try:
+        s = FakeStage(device.lib, n=blocks, side=side)
+        B, T = (3, 85) if how == "few rows" else (2, 512)
+        for i in range(5):
+            at = len(device.names)
+            ordered(device, s.train((2 + i % 2) * AREA, 5 * AREA, B, T, 1, det=int(how == "deterministic")))
+            names = device.names[at:]
+            assert (2 * names.count("colsum"), 2 * names.count("colsum_ordered")) == (passes[0] * blocks, passes[1] * blocks)
+            assert names.count("layernorm_sums") == names.count("layernorm_bwd") == 2 * blocks + 1
+        assert "replay" in device.counts
+    finally:
+        device.lib.fake_take_columns(1)
+
+
+def test_few_rows_between_many(device):
+    """Passes whose bias gradients are added on the side stream between passes that add them on the main stream."""
+    s = FakeStage(device.lib, n=3)
+    rcs = [s.train((2 + i % 2) * AREA, 5 * AREA, *((1, 100) if i % 3 == 1 else (2, 512)), 1) for i in range(9)]
+    ordered(device, *rcs)
+
+
 def test_a_detector_that_detects(device):
     """Two streams that use one scratch without waiting for one another."""
     s = FakeStage(device.lib)
