@@ -394,6 +394,11 @@ class B200Engine:
             saved.append(s)
         return x, saved, B, T
 
+    def _embedding_bwd(self, ids: torch.Tensor, dx: torch.Tensor) -> None:
+        if K.deterministic():
+            self._join()          # its rows have one writer each: a tied head's weight gradient on the side stream comes first
+        K.embedding_bwd(ids, dx, self.dwte, self.dwpe)
+
     def _body_bwd(self, saved, dx: torch.Tensor, input_ids, B: int, T: int, sync: bool = False
                   ) -> Optional[torch.Tensor]:
         """``sync``: this is the step's last backward on this rank and the step ends with a gradient
@@ -405,7 +410,7 @@ class B200Engine:
             if sync:
                 self._send_bucket()
         if self.is_first:
-            K.embedding_bwd(input_ids.contiguous(), dx, self.dwte, self.dwpe)
+            self._embedding_bwd(input_ids.contiguous(), dx)
             if sync:
                 self._send_bucket()
             return None
@@ -451,7 +456,7 @@ class B200Engine:
         if sync and emb is not None:
             ex.backward(0, 0, None, x, emb, area.buf, scratch, None, B, T, chunks, st)
         elif self.is_first and emb is None:
-            K.embedding_bwd(ids, dx0.view(B * T, -1), self.dwte, self.dwpe)
+            self._embedding_bwd(ids, dx0.view(B * T, -1))
             dx0 = None
         if sync and self.is_first:
             self._send_bucket()

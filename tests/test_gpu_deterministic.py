@@ -52,6 +52,37 @@ def test_the_same_pass_gives_the_same_gradients(B, T, heads, width):
         K.set_deterministic(False)
 
 
+@pytest.mark.parametrize("executor", [True, False])
+def test_a_tied_head_and_its_embedding_add_in_one_order(executor):
+    """One block between a head of 50304 rows, whose weight gradient takes longer than the rest of the backward, and the
+    embedding that it shares its weights with; two microbatches."""
+    from diloco_swarm_b200.models.engine_b200 import B200Engine
+    from diloco_swarm_b200.models.gpt2 import GPT2Config
+    from diloco_swarm_b200.ops import kernels as K
+    shape = {"n_layer": 1, "n_head": 4, "n_embd": 128, "vocab_size": 50304, "block_size": 256, "parameter_sharing": True}
+    cfg = make_config(model=shape)
+    cfg.train.deterministic = True
+    try:
+        eng = B200Engine(GPT2Config(**shape), single_world(), cfg, torch.device("cuda", 0))
+        if not executor:
+            eng.exec = None
+        gen = torch.Generator(device="cuda").manual_seed(5)
+        ids = torch.randint(0, 600, (2, 8, 257), device="cuda", generator=gen)
+        mask = torch.ones(8, 256, dtype=torch.long, device="cuda")
+        first = None
+        for _ in range(6):
+            eng.grad.zero_()
+            for m in ids:
+                eng.forward_backward(0, m[:, :-1].contiguous(), None, m[:, 1:].contiguous(), mask, 1.0)
+            eng._join()
+            torch.cuda.synchronize()
+            first = eng.grad.clone() if first is None else first
+            assert torch.equal(eng.grad, first)
+        eng.check_status()
+    finally:
+        K.set_deterministic(False)
+
+
 @pytest.mark.parametrize("B,T,nh,hs", [(1, 129, 1, 64), (2, 384, 4, 32), (3, 1000, 12, 64)])
 def test_ordered_attention_backward(B, T, nh, hs):
     """One launch per kv tile: the same dK and dV, and a dQ whose fp32 sums differ in their order only."""
