@@ -110,20 +110,6 @@ __device__ __forceinline__ void unstage_rows64(const uint8_t* stage, int lane, F
   }
 }
 
-// Sums of eight values over the lanes that differ in bits 2 to 4; v[0] becomes the sum of value e, which is returned.
-__device__ __forceinline__ int sum_rows_of_8(float (&v)[8], int lane) {
-#pragma unroll
-  for (int n = 4, o = 16; n >= 1; n >>= 1, o >>= 1) {
-    const bool up = lane & o;
-#pragma unroll
-    for (int i = 0; i < n; ++i) {
-      const float keep = up ? v[i + n] : v[i], send = up ? v[i] : v[i + n];
-      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-    }
-  }
-  return lane >> 2;
-}
-
 // What an epilogue keeps of its row and tile; loads are asked for before the wait for the accumulator.
 template <int MODE>
 struct RowInfo {
@@ -434,9 +420,10 @@ __device__ __forceinline__ void epilogue_warp(const GemmArgs& g, uint32_t t_addr
       });
       if constexpr (MODE == EPI_MUL_SUM) {
         // In place of a pass that reads the output once more (32768 x 3072: 40 us); here 150 -> 168 us with K = 768.
-        // Over the eight lanes that hold the same columns: lane ends with column e of its eight.
-        const int e = sum_rows_of_8(cs, lane), col = cb + my_ch * 8 + e;
-        if (col < g.N) atomicAdd(g.colsum + col, cs[0]);
+        // Over the eight lanes that hold the same columns: a lane ends with column lane / 4 of its eight.
+        const float sum = fold_sums(cs);
+        const int col = cb + my_ch * 8 + (lane >> 2);
+        if (col < g.N) atomicAdd(g.colsum + col, sum);
       }
       if constexpr (MODE == EPI_GELU) {
         // Always so in this class, and asked all the same: ptxas makes a slower epilogue of the code without the branch (2128 x 4096

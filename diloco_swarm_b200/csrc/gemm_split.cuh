@@ -2,7 +2,7 @@
 //
 // What bounds such a GEMM is neither arithmetic nor bandwidth but latency and how many bytes are in flight: 120 rows of
 // GPT-2 small through the MLP's second projection (N 768, K 3072) are six 128-wide tiles, so six SMs walked 48 k-blocks
-// one after the other (17.3 us with 4.7 MB of weights cold in L2, 8.4 here).  Here a tile is 32, 64 or 128 columns wide and its K range is
+// one after the other (17.2 us with 4.7 MB of weights cold in L2, 7.9 here).  Here a tile is 32, 64 or 128 columns wide and its K range is
 // divided over up to eight CTAs, enough of them to fill the SMs; every CTA has most of its share in flight at once.
 // The partial sums meet inside the cluster: a CTA owns BN / S of the tile's columns, receives the other CTAs' fp32
 // sums of those through distributed shared memory and runs the epilogue on them.  No atomics, no second launch, and a
@@ -19,7 +19,7 @@ namespace dsw {
 // Warps 0-7 epilogue (two per TMEM lane quarter, each takes half of the tile's columns), 8 TMA, 9 MMA.  With one warp per
 // quarter, and the bias and the residual's low half asked for only when the sums were there, what followed the last
 // product was the longest part of a short launch: 120 x 3072 from 768 with GELU 8.3 -> 7.0 us, 120 x 2304 7.0 -> 6.3,
-// 120 x 512 from 128 4.9 -> 3.9, 120 x 768 from 3072 8.6 -> 8.0 (32 weight matrices in turn, one graph).
+// 120 x 512 from 128 4.9 -> 3.9, 120 x 768 from 3072 8.6 -> 7.9 (32 weight matrices in turn, one graph).
 constexpr int SPLIT_EPI_WARPS = 8, SPLIT_TMA_WARP = 8, SPLIT_MMA_WARP = 9;
 constexpr int SPLIT_THREADS = 32 * (SPLIT_EPI_WARPS + 2);
 

@@ -448,13 +448,13 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
   __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<uint32_t*>(&v);
 }
-// Sums v[i] over the warp for N values, a power of two: lane l ends with the sum of value l / (32 / N).
+// Sums v[i] for N values, a power of two, over the lanes that have the same number modulo 32 / N: lane l ends with that of
+// value l / (32 / N).
 template <int N>
-__device__ __forceinline__ float warp_sums(float (&v)[N]) {
+__device__ __forceinline__ float fold_sums(float (&v)[N]) {
   const int lane = threadIdx.x & 31;
-  int o = 16;
 #pragma unroll
-  for (int n = N / 2; n >= 1; n >>= 1, o >>= 1) {
+  for (int n = N / 2, o = 16; n >= 1; n >>= 1, o >>= 1) {
     const bool up = lane & o;
 #pragma unroll
     for (int i = 0; i < n; ++i) {
@@ -462,9 +462,14 @@ __device__ __forceinline__ float warp_sums(float (&v)[N]) {
       v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
     }
   }
-  float s = v[0];
+  return v[0];
+}
+// The same over the whole warp.
+template <int N>
+__device__ __forceinline__ float warp_sums(float (&v)[N]) {
+  float s = fold_sums(v);
 #pragma unroll
-  for (; o >= 1; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  for (int o = 16 / N; o >= 1; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   return s;
 }
 

@@ -11,11 +11,12 @@
 // allocated here, so no pass waits for the allocator, and memory that the side stream reads needs no bookkeeping
 // beyond the marks below.
 //
-// Streams.  Weight-gradient GEMMs and bias column sums feed nothing in the backward, so they go to the stage's side
-// stream (when it has one) and fill the SMs that the dgrad chain leaves idle.  The buffers they read (dh, dx1, dqkv)
-// are doubled by block parity: before a block overwrites a set the main stream waits for the side work of the block
-// two up, which is long done.  A block's outgoing gradient is read by the side work of the block below it, so those
-// buffers form a ring of three.
+// Streams.  Weight-gradient GEMMs, the joining of LayerNorm's column sums and those bias column sums that do not come out of
+// the kernels which write dh and dqkv (few rows, deterministic gradients) feed nothing in the backward, so they go to the
+// stage's side stream (when it has one) and fill the SMs that the dgrad chain leaves idle.  The buffers they read (dh, dx1,
+// dqkv, LayerNorm's sums) are doubled by block parity: before a block overwrites a set the main stream waits for the side
+// work of the block two up, which is long done.  A block's outgoing gradient is read by the side work of the block below it,
+// so those buffers form a ring of three.  What both streams, or two passes, add to is added to atomically.
 //
 // Graphs.  Some 3 us of host time per launch are still more than many kernels of a short pass take.  So a run of launches that
 // touches the work areas only is captured into a CUDA graph when it is asked for a second time in the same areas and
@@ -346,8 +347,9 @@ struct Run {
   }
 
   // The next launch is asked to add its output's column sums (a bias gradient) to `to`: in its epilogue or beside its
-  // products, in place of a pass that reads dh or dqkv once more (a microbatch of GPT-2 small, 32 x 1024: 33.07 -> 32.38 ms,
-  // 16 x 133: 2786 -> 2762 us; six blocks of medium, 8 x 1024: 4788 -> 4667 us).  Its sums meet in atomics, as those of the
+  // products, in place of a pass that reads dh or dqkv once more (timed in turn: six blocks of medium, 8 x 1024, 4950 -> 4819 us;
+  // four of large, 4 x 1024, 2654 -> 2592; a microbatch of GPT-2 small, 16 x 133, 2856 -> 2820; 32 x 1024 33.4 -> 32.7 ms, runs of
+  // which differ by 1.9 %).  Its sums meet in atomics, as those of the
   // pass do from COLSUM_ORDERED_ROWS rows on; fewer rows, whose gradients repeat themselves bit for bit, keep the pass.
   bool columns_asked() const { return !deterministic && M >= dsw::COLSUM_ORDERED_ROWS; }
   void sum_columns(float* to) const { dsw::tl_launch.colsum = columns_asked() ? to : nullptr; }

@@ -6,7 +6,8 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("M", [1, 3, 37, 1487, 5003])     # 1487: more than one round of 148 blocks only for the widest rows
+# one round of 148 blocks is 4736 rows up to 256 columns, 2368 up to 512, 1480 up to 768, 1184 up to 1024 and fewer above
+@pytest.mark.parametrize("M", [1, 3, 37, 1487, 5003])
 @pytest.mark.parametrize("d", [136, 256, 264, 768, 776, 1024, 1288, 1600, 1800, 2048])
 @pytest.mark.parametrize("dres", [False, True])
 def test_backward_against_64_bits(M, d, dres):
