@@ -59,6 +59,18 @@ int dsw_head_rows(const float* parts, const float* tlogit, const long long* targ
                   float scale, float* loss_acc, void* rows, int M, int N, int* status, cudaStream_t stream);
 int dsw_head_dlogits(const void* A, const void* W, const void* rows, void* out, int M, int N, int K, int* status,
                      cudaStream_t stream);
+// The same for widths K <= 128, with both gradients and without storing logits or their gradient (head_flash.cu).  x [M,K], W
+// [V,K] bf16.  dsw_head_softmax: over each of `slices` (dsw_head_slices) slices of the vocabulary parts (fp32
+// [slices][M][128]) and ml (fp32 pairs [slices][4][M]); dsw_head_join: += the loss, dx (bf16 [M,K]; zeros in masked rows) and, for
+// the rows up to the next multiple of 128, nlse (fp32) and target (int32), and coef (one fp32) = scale / count;
+// dsw_head_wgrad: dW (fp32 [V,K]) += the weights' gradient, deterministic: in a fixed order.
+int dsw_head_slices(int M, int V, int K, int sms);          // 0: not for this width
+int dsw_head_softmax(const void* x, const void* W, float* parts, void* ml, int M, int V, int K, int slices, int* status, cudaStream_t st);
+int dsw_head_join(const float* parts, const void* ml, const void* x, const void* W, const long long* targets, const long long* mask,
+                  const float* count, float scale, float* loss_acc, void* dx, float* nlse, int* target, float* coef, int M, int V, int K,
+                  int slices, int* status, cudaStream_t st);
+int dsw_head_wgrad(const void* x, const void* W, const float* nlse, const int* target, const float* coef, float* dW, int M, int V, int K,
+                   int deterministic, int* status, cudaStream_t st);
 // partials[s] (fp32 [M,N] each, *splits <= most of them) = A [M,K] B [K,N] over slice s of K.
 int dsw_gemm_partials(const void* A, const void* B, int M, int N, int K, float* partials, int most, int* splits, int* status,
                       cudaStream_t stream);
@@ -204,7 +216,7 @@ int dsw_stage_backward(void* stage, int hi, int lo, const void* dy, const void* 
 
 // ---------------------------------------------------------------- bounds-checking build (-DDSWARM_BOUNDS)
 // First failed bounds check since the last call: 0 = none, else 100000 * unit + source line (units: 1
-// elementwise.cu, 2 optim.cu, 3 collectives.cu, 4 gemm_one_cta.cu, 5 gemm_pair.cu).  The shipped build has no
+// elementwise.cu, 2 optim.cu, 3 collectives.cu, 4 gemm_one_cta.cu, 5 gemm_pair.cu, 6 head_flash.cu).  The shipped build has no
 // checks and returns 0.  The per-unit readers return that unit's line.
 int dsw_bounds_status();
 int dsw_bounds_elementwise();
@@ -212,6 +224,7 @@ int dsw_bounds_optim();
 int dsw_bounds_collectives();
 int dsw_bounds_gemm_one_cta();
 int dsw_bounds_gemm_pair();
+int dsw_bounds_head_flash();
 // Bounds build: one check fails on purpose, without touching memory, so that the report path can be tested
 // (returns 1); shipped build: nothing happens (returns 0).
 int dsw_bounds_selftest(cudaStream_t st);
@@ -220,6 +233,7 @@ int dsw_bounds_selftest(cudaStream_t st);
 // Load every kernel of a source file on the current device now, so that no first launch has to wait for
 // the device to go idle while a pipeline receive is spinning on it.
 int dsw_load_gemm();
+int dsw_load_head_flash();
 int dsw_load_attention();
 int dsw_load_elementwise();
 int dsw_load_optim();

@@ -1029,13 +1029,13 @@ extern "C" int dsw_cast_bf16_f32(const void* src, float* dst, long long n, cudaS
 DSW_BOUNDS_TU(dsw_bounds_elementwise)
 
 // First failed bounds check since the last call: 0 = none, else 100000 * unit + source line (unit 1 =
-// elementwise.cu, 2 = optim.cu, 3 = collectives.cu, 4 = gemm_one_cta.cu, 5 = gemm_pair.cu); -1 if a word
+// elementwise.cu, 2 = optim.cu, 3 = collectives.cu, 4 = gemm_one_cta.cu, 5 = gemm_pair.cu, 6 = head_flash.cu); -1 if a word
 // could not be read.  Always 0 in the shipped build; synchronises the device in the bounds build.
 extern "C" int dsw_bounds_status() {
   int (*units[])() = {dsw_bounds_elementwise, dsw_bounds_optim, dsw_bounds_collectives, dsw_bounds_gemm_one_cta,
-                      dsw_bounds_gemm_pair};
+                      dsw_bounds_gemm_pair, dsw_bounds_head_flash};
   int first = 0;
-  for (int u = 0; u < 5; ++u) {
+  for (int u = 0; u < 6; ++u) {
     const int v = units[u]();
     if (v < 0) return -1;
     if (v > 0 && first == 0) first = 100000 * (u + 1) + v;

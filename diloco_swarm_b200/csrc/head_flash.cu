@@ -1,0 +1,614 @@
+// LM head and cross-entropy of narrow models (width up to 128) as a flash kernel: neither the logits nor their gradient
+// ever leave the SM.
+//
+// The gradient of the loss by the head's input is the softmax-weighted mean of the rows of W, less the target's row: the
+// same thing as attention whose queries are the activations and whose keys and values are both W.  So one pass over the
+// vocabulary gives log-sum-exp and input gradient together (dsw_head_softmax, online softmax; dsw_head_join puts the
+// slices of the vocabulary together), and a second one, with the roles of the activations and W exchanged, the weights'
+// gradient (dsw_head_wgrad): S^T = W x^T, P^T = 2^(S^T - lse) - onehot, dW += P^T x.
+//
+// One kernel does both.  A unit of work is 128 rows of the resident operand R and a run of 128-row tiles of the streamed
+// operand T:
+//   S_j = R T_j^T         [128 x 128] -> TMEM, one of three buffers      A, B: shared memory, K-major
+//   P_j = f(S_j)          bf16, thread = row and half of the columns, written over S_j in TMEM
+//   O += P_j T_j          [128 x 128] in TMEM      A: TMEM, B: the same tile, N-major
+// Sixteen row warps in two groups that take turns at the tiles, so that S and P of three tiles are under way: with two
+// blocks of rows in place of the third buffer a tile's chain (S, P, O, next S, some 3600 clocks) showed.  P in TMEM
+// instead of shared memory because S alone reads 128 bytes of it per clock, all that an SM has.
+//
+// P is computed against a reference that the slice's first tile gives, its maximum, and not against a running maximum:
+// fp32 and bf16 carry 2^100 and more above it with the same relative precision, no maximum is sought after the first tile
+// and O is never rescaled.  Rows that exceed it all the same are done over by dsw_head_join, one by one.
+//
+// What bounds it: per 128 x 128 tile 1024 clocks of tensor core and 1024 of exponentials (16 a clock and SM).  Before, the
+// head of 65536 tokens at width 128 and 50304 columns was four kernels: log-sum-exp 1462 us, the logits' gradient 1730
+// (6.6 GB written), and the two products that read it from DRAM, 1150 and 1232.  Here 1225, 100 and 1225 (some 1700 clocks a
+// tile); 8192 tokens 178, 14 and 183; 128 tokens 13, 10 and 17, where logits that are stored took 9.5, cross-entropy 11, and
+// the products 34 and 11.  What keeps a tile above 1024 clocks: eight dependent products with P from TMEM take 1025 by
+// themselves, eight of S (N = 128) 733 where 512 would do, and the chain S, P, O of a tile is only three tiles deep.  Without
+// the exponentials it was 11 % less, and a quarter to a half of them on the FMA pipe (a polynomial) gained nothing.
+#include <cuda.h>
+#include "gemm_kernels.cuh"
+#include "launch.h"
+#include "tmap.h"
+#include "dswarm.h"
+
+namespace dsw {
+
+constexpr int HF_W = 128;                        // widest model; also rows of a tile
+constexpr int HF_SLAB = 128 * 64 * 2;            // 128 rows x 64 columns
+constexpr int HF_TILE = 2 * HF_SLAB;
+constexpr int HF_STAGES = 4;
+constexpr int HF_BUFS = 3;                       // of S and P
+constexpr int HF_ROW_WARPS = 16;
+constexpr int HF_MMA_WARP = HF_ROW_WARPS, HF_TMA_WARP = HF_ROW_WARPS + 1;
+constexpr int HF_THREADS = 32 * (HF_ROW_WARPS + 4);
+
+struct HeadSmem {
+  static constexpr int R_OFF = 0;
+  static constexpr int T_OFF = R_OFF + HF_TILE;
+  static constexpr int STAT_OFF = T_OFF + HF_STAGES * HF_TILE;      // per stage: -lse2 fp32 [128], targets int32 [128]
+  static constexpr int EPI_OFF = STAT_OFF + HF_STAGES * 1024;       // a staging tile per softmax warp
+  static constexpr int MAX_OFF = EPI_OFF + HF_ROW_WARPS * EPI_STAGE_BYTES;      // row maxima of a first tile, fp32 [half][128]
+  static constexpr int BAR_OFF = MAX_OFF + 2 * 128 * 4;
+  static constexpr int TOTAL = BAR_OFF + 256;                       // declared 1024-aligned, and checked
+};
+
+struct HeadArgs {
+  int rows, cols;                // of the resident and the streamed operand
+  int width, slices;             // model width; slices of the streamed rows
+  float* out;                    // softmax: O [slices][rows][128]; gradient: dW [rows, width], added to
+  float2* ml;                    // softmax: {reference in base 2, sum of 2^(s - reference)} [slices][2 groups x 2 halves][rows]
+  const float* nlse; const int* target;          // gradient: per streamed row
+  const float* coef;             // gradient: what it is multiplied by
+  int* status;
+};
+
+// P from tensor memory (bf16 pairs, 8 columns per 16 values of K) times B from shared memory
+__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t hi, uint32_t idesc,
+                                             uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
+      "mov.b64 db, {%2, %3};\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, int bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+
+// GRAD: the weights' gradient (R = W, T = activations), else softmax and input gradient (R = activations, T = W).
+template <bool GRAD>
+__global__ void __launch_bounds__(HF_THREADS, 1)
+head_flash_kernel(const __grid_constant__ CUtensorMap tmap_r, const __grid_constant__ CUtensorMap tmap_t, HeadArgs g) {
+  using L = HeadSmem;
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = smem_raw;
+  if (smem_u32(smem) & 1023) {
+    if (threadIdx.x == 0 && g.status) atomicCAS(g.status, 0, ST_BAD_ARG);
+    return;
+  }
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);
+  uint64_t* r_full = bars;             // per unit: R loaded
+  uint64_t* r_empty = bars + 1;        // per unit: its last S product done
+  uint64_t* o_full = bars + 2;         // per unit: O complete
+  uint64_t* o_free = bars + 3;         // per unit: O read out (16 warps arrive)
+  uint64_t* m_full = bars + 4;         // per unit: maxima of the first tile written (8 warps arrive; softmax)
+  uint64_t* s_full = bars + 5;         // [bufs] per tile: S in TMEM
+  uint64_t* p_full = s_full + HF_BUFS; // [bufs] per tile: P in TMEM (8 warps arrive)
+  uint64_t* t_full = p_full + HF_BUFS; // [stages]
+  uint64_t* t_empty = t_full + HF_STAGES;
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(t_empty + HF_STAGES);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int row_units = (g.rows + 127) / 128, tiles = (g.cols + 127) / 128;
+  const int total = row_units * g.slices;
+  struct Unit { int r0, t0, n, slice; };
+  const auto unit_at = [&](int u) {
+    Unit x;
+    x.slice = u / row_units;
+    x.r0 = (u - x.slice * row_units) * 128;
+    x.t0 = int((long long)tiles * x.slice / g.slices);
+    x.n = int((long long)tiles * (x.slice + 1) / g.slices) - x.t0;
+    return x;
+  };
+
+  if (threadIdx.x == 0) {
+    mbar_init(r_full, 1); mbar_init(r_empty, 1); mbar_init(o_full, 1); mbar_init(o_free, HF_ROW_WARPS); mbar_init(m_full, 8);
+    for (int i = 0; i < HF_BUFS; ++i) { mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 8); }
+    for (int i = 0; i < HF_STAGES; ++i) { mbar_init(&t_full[i], 1); mbar_init(&t_empty[i], 1); }
+    *abort_flag = 0;
+    mbar_fence_init();
+    fence_proxy_async();
+  }
+  if (warp == HF_MMA_WARP) {
+    tmem_alloc(tmem_holder, 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_holder;
+  const auto tmem_s = [=](uint32_t buf) { return tmem_base + 128 + buf * 128; };          // P: columns 0-31 and 64-95 of it
+  const uint32_t tmem_o = tmem_base;
+
+  if (warp >= HF_ROW_WARPS) asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+  if (warp == HF_TMA_WARP) {
+    // ------------------------------------------------------------ TMA producer (the whole warp, one lane issues)
+    if (elect_one()) {
+      tma_prefetch_desc(&tmap_r);
+      tma_prefetch_desc(&tmap_t);
+    }
+    pdl_wait();
+    uint32_t it = 0, w = 0;
+    bool ok = true;
+    for (int u = blockIdx.x; u < total && ok; u += gridDim.x, ++w) {
+      const Unit x = unit_at(u);
+      if (w > 0 && !mbar_wait_warp(r_empty, (w - 1) & 1, abort_flag, g.status)) { ok = false; break; }
+      if (elect_one()) {
+        mbar_expect_tx(r_full, HF_TILE);
+#pragma unroll
+        for (int c = 0; c < 2; ++c) tma_load_2d(smem + L::R_OFF + c * HF_SLAB, &tmap_r, r_full, c * 64, x.r0);
+      }
+      __syncwarp();
+      for (int j = 0; j < x.n; ++j, ++it) {
+        const int s = it % HF_STAGES, row = (x.t0 + j) * 128;
+        if (!mbar_wait_warp(&t_empty[s], ((it / HF_STAGES) & 1) ^ 1, abort_flag, g.status)) { ok = false; break; }
+        if (elect_one()) {
+          mbar_expect_tx(&t_full[s], HF_TILE + (GRAD ? 1024 : 0));
+#pragma unroll
+          for (int c = 0; c < 2; ++c) tma_load_2d(smem + L::T_OFF + s * HF_TILE + c * HF_SLAB, &tmap_t, &t_full[s], c * 64, row);
+          if constexpr (GRAD) {
+            bulk_load(smem + L::STAT_OFF + s * 1024, g.nlse + row, 512, &t_full[s]);
+            bulk_load(smem + L::STAT_OFF + s * 1024 + 512, g.target + row, 512, &t_full[s]);
+          }
+        }
+        __syncwarp();
+      }
+    }
+    pdl_launch();
+    if (!ok) {
+      // give loads that are still in flight a bounded chance to land before the CTA exits
+      for (int s = 0; s < HF_STAGES + 1; ++s)
+        for (int spin = 0; spin < 100000; ++spin)
+          if (mbar_try_wait(s < HF_STAGES ? &t_full[s] : r_full, 0) || mbar_try_wait(s < HF_STAGES ? &t_full[s] : r_full, 1)) break;
+    }
+  } else if (warp == HF_MMA_WARP) {
+    // ------------------------------------------------------------ MMA issuer (the whole warp, one lane issues)
+    const uint32_t idesc_s = make_idesc_bf16(128, 128, 0, 0), idesc_o = make_idesc_bf16(128, 128, 0, 1);
+    const uint32_t desc_hi = smem_desc_hi(1024);
+    const uint32_t r_lo = smem_desc_lo(smem_u32(smem + L::R_OFF), 16);
+    uint32_t it = 0, w = 0;
+    bool ok = true;
+    // S of tile i into its buffer: over P of tile i - 3, right behind the product that reads it.  Eight products of each kind
+    // in a row take 1706 clocks that way, 1166 where S goes elsewhere; issued a product later, or after a wait for the one
+    // that reads P, the next tile's chain took as long as that saved (1222 and 1389 us for 65536 rows, this way 1212).
+    const auto issue_s = [&](uint32_t i) -> bool {
+      const int s = i % HF_STAGES, buf = i % HF_BUFS;
+      if (!mbar_wait_warp(&t_full[s], (i / HF_STAGES) & 1, abort_flag, g.status)) return false;
+      const uint32_t t_lo = smem_desc_lo(smem_u32(smem + L::T_OFF + s * HF_TILE), 16);
+      if (elect_one()) {
+#pragma unroll
+        for (int k = 0; k < HF_W / UMMA_K; ++k) {
+          const uint32_t step = (k >> 2) * (HF_SLAB >> 4) + (k & 3) * 2;
+          umma_bf16_lohi(tmem_s(buf), r_lo + step, t_lo + step, desc_hi, idesc_s, k > 0);
+        }
+        umma_commit(&s_full[buf]);
+      }
+      __syncwarp();
+      return true;
+    };
+    for (int u = blockIdx.x; u < total && ok; u += gridDim.x, ++w) {
+      const int n = unit_at(u).n, ahead = n < HF_BUFS ? n : HF_BUFS;
+      if (!mbar_wait_warp(r_full, w & 1, abort_flag, g.status)) break;
+      for (int j = 0; j < ahead && ok; ++j) ok = issue_s(it + j);
+      if (ok && n <= HF_BUFS && elect_one()) umma_commit(r_empty);
+      __syncwarp();
+      for (int j = 0; j < n && ok; ++j, ++it) {
+        const int s = it % HF_STAGES, buf = it % HF_BUFS;
+        const uint32_t t_lo = smem_desc_lo(smem_u32(smem + L::T_OFF + s * HF_TILE), HF_SLAB);
+        if (!mbar_wait_warp(&p_full[buf], (it / HF_BUFS) & 1, abort_flag, g.status)) { ok = false; break; }
+        // the unit before has been read out of O
+        if (j == 0 && w > 0 && !mbar_wait_warp(o_free, (w - 1) & 1, abort_flag, g.status)) { ok = false; break; }
+        tc_fence_after();
+        if (elect_one()) {
+#pragma unroll
+          for (int k = 0; k < 128 / UMMA_K; ++k)
+            umma_bf16_ts(tmem_o, tmem_s(buf) + (k >> 2) * 64 + (k & 3) * 8, t_lo + k * (2048 >> 4), desc_hi, idesc_o, j > 0 || k > 0);
+          umma_commit(&t_empty[s]);
+          if (j + 1 == n) umma_commit(o_full);
+        }
+        __syncwarp();
+        if (j + HF_BUFS < n) {
+          if (!issue_s(it + HF_BUFS)) { ok = false; break; }
+          if (j + HF_BUFS + 1 == n && elect_one()) umma_commit(r_empty);
+          __syncwarp();
+        }
+      }
+    }
+  } else if (warp < HF_ROW_WARPS) {
+    // ------------------------------------------------------------ softmax (thread = row and half of the columns)
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
+    const int grp = warp >> 3, half = (warp >> 2) & 1, q = warp & 3;
+    const uint32_t quarter = uint32_t(q * 32) << 16;
+    const uint32_t to = tmem_o + quarter + (grp * 2 + half) * 32;          // the columns of O that this warp reads out
+    uint8_t* stage = smem + L::EPI_OFF + warp * EPI_STAGE_BYTES;
+    float* xm = reinterpret_cast<float*>(smem + L::MAX_OFF) + q * 32 + lane;
+    uint32_t it = 0, w = 0;
+    bool ok = true;
+    pdl_wait();
+    const float coef = GRAD ? *g.coef : 1.f;
+    for (int u = blockIdx.x; u < total && ok; u += gridDim.x, ++w) {
+      const Unit x = unit_at(u);
+      const int row0 = x.r0 + q * 32;          // the warp's first row
+      float m = -1e30f, l = 0.f;
+      for (int j = 0; j < x.n; ++j, ++it) {
+        if (int(it & 1) != grp) continue;
+        const int s = it % HF_STAGES, buf = it % HF_BUFS;
+        const uint32_t ts = tmem_s(buf) + quarter + half * 64;
+        // its statistics lie in the stage: seen by waiting for the loads oneself
+        if (GRAD && !mbar_wait(&t_full[s], (it / HF_STAGES) & 1, abort_flag, g.status)) { ok = false; break; }
+        if (!mbar_wait(&s_full[buf], (it / HF_BUFS) & 1, abort_flag, g.status)) { ok = false; break; }
+        tc_fence_after();
+        uint32_t v[2][32];
+#pragma unroll
+        for (int c = 0; c < 2; ++c) tmem_ld_32x32(ts + c * 32, v[c]);
+        tmem_ld_wait();
+        if constexpr (!GRAD) {
+          const int left = g.cols - (x.t0 + j) * 128 - half * 64;          // of these 64 columns, those that exist
+          if (left < 64) {
+#pragma unroll
+            for (int c = 0; c < 2; ++c)
+#pragma unroll
+              for (int i = 0; i < 32; ++i) v[c][i] = c * 32 + i < left ? v[c][i] : 0xff800000u;          // -inf
+          }
+          if (j == 0) {
+            float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+            for (int c = 0; c < 2; ++c)
+#pragma unroll
+              for (int i = 0; i < 32; i += 2)
+                mx4[(i >> 1) & 3] = max3(mx4[(i >> 1) & 3], __uint_as_float(v[c][i]), __uint_as_float(v[c][i + 1]));
+            // read by all before P of the unit's last tile, written again behind it
+            xm[half * 128] = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+            __syncwarp();
+            if (lane == 0) mbar_arrive(m_full);
+          }
+          if (j < 2) {          // the first tile that this group has of the unit
+            if (!mbar_wait(m_full, w & 1, abort_flag, g.status)) { ok = false; break; }
+            m = max3(xm[0], xm[128], -1e30f) * LOG2E;          // finite, so that a row of nothing but -inf sums to zero
+          }
+          f2 sum2[2] = {f2_bcast(0.f), f2_bcast(0.f)};
+          const f2 sc2 = f2_bcast(LOG2E), nm2 = f2_bcast(-m);
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            uint32_t pk[16];
+#pragma unroll
+            for (int i = 0; i < 32; i += 2) {
+              float x0, x1;
+              f2_split(f2_fma(f2_make(__uint_as_float(v[c][i]), __uint_as_float(v[c][i + 1])), sc2, nm2), x0, x1);
+              const f2 p = f2_make(ex2_approx(x0), ex2_approx(x1));
+              sum2[(i >> 1) & 1] = f2_add(sum2[(i >> 1) & 1], p);
+              pk[i >> 1] = pack_bf16_f2(p);
+            }
+            tmem_st_32x16(ts + c * 16, pk);
+          }
+          float a0, a1;
+          f2_split(f2_add(sum2[0], sum2[1]), a0, a1);
+          l += a0 + a1;
+        } else {
+          const float* nl = reinterpret_cast<const float*>(smem + L::STAT_OFF + s * 1024) + half * 64;
+          const int* tg = reinterpret_cast<const int*>(nl + 128);
+          const f2 sc2 = f2_bcast(LOG2E);
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            const int t = tg[c * 32 + lane] - row0;          // the target of streamed row c * 32 + lane, if it is the warp's
+            const unsigned hit = __ballot_sync(0xffffffffu, unsigned(t) < 32u);
+            const unsigned dead = __ballot_sync(0xffffffffu, nl[c * 32 + lane] == -INFINITY);
+#pragma unroll
+            for (int i = 0; i < 32; i += 4) {
+              const ulonglong2 n4 = *reinterpret_cast<const ulonglong2*>(nl + c * 32 + i);
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {
+                const f2 n = {h ? n4.y : n4.x};
+                float x0, x1;
+                f2_split(f2_fma(f2_make(__uint_as_float(v[c][i + 2 * h]), __uint_as_float(v[c][i + 2 * h + 1])), sc2, n), x0, x1);
+                v[c][i + 2 * h] = __float_as_uint(ex2_approx(x0));
+                v[c][i + 2 * h + 1] = __float_as_uint(ex2_approx(x1));
+              }
+            }
+            if (hit | dead) {          // the same for the whole warp
+#pragma unroll
+              for (int i = 0; i < 32; ++i) {
+                float p = __uint_as_float(v[c][i]);
+                if (dead >> i & 1) p = 0.f;          // a masked row: whatever its logits are
+                if (lane == __shfl_sync(0xffffffffu, t, i)) p -= 1.f;
+                v[c][i] = __float_as_uint(p);
+              }
+            }
+            uint32_t pk[16];
+#pragma unroll
+            for (int i = 0; i < 32; i += 2) pk[i >> 1] = pack_bf16(__uint_as_float(v[c][i]), __uint_as_float(v[c][i + 1]));
+            tmem_st_32x16(ts + c * 16, pk);
+          }
+        }
+        tmem_st_wait();
+        tc_fence_before();          // orders P before the product behind the arrive
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&p_full[buf]);
+      }
+      if (!ok || !mbar_wait(o_full, w & 1, abort_flag, g.status)) { ok = false; break; }
+      tc_fence_after();
+      if (!GRAD && row0 + lane < g.rows) g.ml[((long long)x.slice * 4 + grp * 2 + half) * g.rows + row0 + lane] = make_float2(m, l);
+      uint32_t o[16];
+      tmem_ld_32x16(to, o);
+#pragma unroll 1
+      for (int c = 0; c < 32; c += 16) {
+        tmem_ld_wait();
+        uint32_t w[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) w[i] = GRAD ? __float_as_uint(__uint_as_float(o[i]) * coef) : o[i];
+        if (c + 16 < 32) {
+          tmem_ld_32x16(to + c + 16, o);
+        } else {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(o_free);
+        }
+        __syncwarp();                                   // the previous chunk has been read out
+        stage_row64(stage, lane, w);
+        __syncwarp();
+        unstage_rows64(stage, lane, [&](int, int rl, int ch, const uint4& d) {
+          const int row = row0 + rl, col = (grp * 2 + half) * 32 + c + ch * 4;
+          if (row >= g.rows) return;
+          if constexpr (GRAD) {
+            if (col < g.width && DSW_OK(col + 4 <= g.width))
+              asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(g.out + (long long)row * g.width + col),
+                           "f"(__uint_as_float(d.x)), "f"(__uint_as_float(d.y)), "f"(__uint_as_float(d.z)),
+                           "f"(__uint_as_float(d.w))
+                           : "memory");
+          } else if (DSW_OK(col + 4 <= HF_W && x.slice < g.slices)) {
+            *reinterpret_cast<uint4*>(g.out + ((long long)x.slice * g.rows + row) * HF_W + col) = d;
+          }
+        });
+      }
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (warp == HF_MMA_WARP) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, 512);
+  }
+}
+
+// Log-sum-exp (base 2) and softmax-weighted sum of the rows of W for one row by one warp: a row whose logits exceed those
+// of the first tile by more than its arithmetic carries.
+__device__ __noinline__ void row_alone(const __nv_bfloat16* x, const __nv_bfloat16* W, int row, int V, int width, int lane, float& m, float& l,
+                                       float4& o) {
+  const int col = lane * 4;
+  const bool in = col < width;
+  const uint2 xv = in ? *reinterpret_cast<const uint2*>(x + (long long)row * width + col) : make_uint2(0, 0);
+  const float2 x01 = unpack_bf16(xv.x), x23 = unpack_bf16(xv.y);
+  m = -1e30f;
+  l = 0.f;
+  o = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int v = 0; v < V; ++v) {
+    const uint2 wv = in ? *reinterpret_cast<const uint2*>(W + (long long)v * width + col) : make_uint2(0, 0);
+    const float2 w01 = unpack_bf16(wv.x), w23 = unpack_bf16(wv.y);
+    float s = fmaf(w01.x, x01.x, fmaf(w01.y, x01.y, fmaf(w23.x, x23.x, w23.y * x23.y)));
+#pragma unroll
+    for (int i = 16; i > 0; i >>= 1) s += __shfl_xor_sync(0xffffffffu, s, i);
+    s *= LOG2E;
+    const float nm = fmaxf(m, s), f = ex2_approx(m - nm), p = ex2_approx(s - nm);
+    m = nm;
+    l = fmaf(l, f, p);
+    o = make_float4(fmaf(o.x, f, p * w01.x), fmaf(o.y, f, p * w01.y), fmaf(o.z, f, p * w23.x), fmaf(o.w, f, p * w23.y));
+  }
+}
+
+// Slices of the vocabulary -> loss, input gradient, and what the weights' gradient wants to know of a row.  WPR warps share
+// a row's slices; a lane has four columns.  Rows past M (up to a multiple of 128) are marked as masked.
+template <int WPR>
+__global__ void __launch_bounds__(256)
+head_join_kernel(const float* parts, const float2* ml, const __nv_bfloat16* x, const __nv_bfloat16* W,
+                 const long long* __restrict__ targets, const long long* __restrict__ mask, const float* count, float scale,
+                 float* __restrict__ loss_acc, __nv_bfloat16* __restrict__ dx, float* __restrict__ nlse, int* __restrict__ target,
+                 float* __restrict__ coef, int M, int V, int width, int slices, int* status) {
+  constexpr int RPB = 8 / WPR;                 // rows per block and step
+  __shared__ float4 sho[8][32];
+  __shared__ float2 shs[8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, rb = warp / WPR, part = warp - rb * WPR;
+  const int padded = (M + 127) / 128 * 128, col = lane * 4;
+  pdl_wait();
+  pdl_launch();
+  const float k = scale / fmaxf(count[0], 1.f);
+  if (blockIdx.x == 0 && threadIdx.x == 0) *coef = k;
+  float loss = 0.f;
+  for (int row0 = blockIdx.x * RPB; row0 < padded; row0 += gridDim.x * RPB) {
+    const int row = row0 + rb;
+    const bool in = row < M, keep = in && (mask == nullptr || mask[row] != 0);
+    // what does not depend on the slices is asked for ahead of them
+    const bool first = part == 0 && in;
+    const long long wanted = first ? targets[row] : 0;
+    const long long t = wanted < 0 || wanted >= V ? 0 : wanted;
+    uint2 wv = make_uint2(0, 0), xv = wv;
+    if (first && col < width && DSW_OK(t >= 0 && t < V)) {
+      wv = *reinterpret_cast<const uint2*>(W + t * width + col);
+      xv = *reinterpret_cast<const uint2*>(x + (long long)row * width + col);
+    }
+    float mx = -INFINITY, l = 0.f;
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+    bool over = false;
+    // the reference of a slice: a group without a tile in it has none, and says -1e30
+    const auto ref_of = [&](int s) { return fmaxf(ml[4LL * s * M + row].x, ml[(4LL * s + 2) * M + row].x); };
+    if (keep) {
+      for (int s = lane; s < slices; s += 32) mx = fmaxf(mx, ref_of(s));
+#pragma unroll
+      for (int i = 16; i > 0; i >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, i));
+#pragma unroll 4
+      for (int s = part; s < slices; s += WPR) {
+        const float2* t = ml + 4LL * s * M + row;
+        const float sum = (t[0].y + t[M].y) + (t[2LL * M].y + t[3LL * M].y);
+        const float4 p = *reinterpret_cast<const float4*>(parts + ((long long)s * M + row) * HF_W + col);
+        const float f = ex2_approx(ref_of(s) - mx);
+        over |= sum > 0x1p100f;
+        l = fmaf(sum, f, l);
+        o.x = fmaf(p.x, f, o.x); o.y = fmaf(p.y, f, o.y); o.z = fmaf(p.z, f, o.z); o.w = fmaf(p.w, f, o.w);
+      }
+    }
+    if constexpr (WPR > 1) {
+      __syncthreads();                          // the round before has been read
+      sho[warp][lane] = o;
+      if (lane == 0) shs[warp] = make_float2(l, over ? 1.f : 0.f);
+      __syncthreads();
+      if (part == 0)
+        for (int i = 1; i < WPR; ++i) {
+          const float4 p = sho[warp + i][lane];
+          l += shs[warp + i].x;
+          over |= shs[warp + i].y != 0.f;
+          o.x += p.x; o.y += p.y; o.z += p.z; o.w += p.w;
+        }
+    }
+    if (part != 0 || row >= padded) continue;
+    float nl = -INFINITY;
+    int tgt = -1;
+    float4 dv = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (keep) {
+      if (t != wanted && status && lane == 0) atomicCAS(status, 0, ST_BAD_ARG);
+      tgt = int(t);
+      const float2 w01 = unpack_bf16(wv.x), w23 = unpack_bf16(wv.y), x01 = unpack_bf16(xv.x), x23 = unpack_bf16(xv.y);
+      float logit = fmaf(w01.x, x01.x, fmaf(w01.y, x01.y, fmaf(w23.x, x23.x, w23.y * x23.y)));
+#pragma unroll
+      for (int i = 16; i > 0; i >>= 1) logit += __shfl_xor_sync(0xffffffffu, logit, i);
+      if (over) row_alone(x, W, row, V, width, lane, mx, l, o);
+      const float lse2 = mx + log2f(l);
+      nl = -lse2;
+      if (lane == 0) loss += k * (lse2 * 0.6931471805599453f - logit);
+      const float inv = 1.f / l;
+      dv = make_float4(k * (o.x * inv - w01.x), k * (o.y * inv - w01.y), k * (o.z * inv - w23.x), k * (o.w * inv - w23.y));
+    }
+    if (lane == 0) { nlse[row] = nl; target[row] = tgt; }
+    if (in && col < width) *reinterpret_cast<uint2*>(dx + (long long)row * width + col) = make_uint2(pack_bf16(dv.x, dv.y), pack_bf16(dv.z, dv.w));
+  }
+  // one addition per block: the address takes one every 2 ns (8192 rows: 19 us with one per warp)
+  __shared__ float losses[8];
+  if (lane == 0) losses[warp] = loss;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int i = 1; i < 8; ++i) loss += losses[i];
+    atomicAdd(loss_acc, loss);
+  }
+}
+
+// Slices of the streamed rows: whole rounds of units over the SMs, each as long as its tiles (some 0.7 us each)
+// and what a unit takes besides; per_slice: what a further slice costs elsewhere, in us.
+static int pick_slices(int rows, int cols, int sms, double per_slice) {
+  const int units = (rows + 127) / 128, tiles = (cols + 127) / 128;
+  double least = 1e30;
+  int best = 1;
+  for (int s = 1; s <= tiles && s <= 128; ++s) {
+    const double c = double(((long long)units * s + sms - 1) / sms) * (((tiles + s - 1) / s) * 0.7 + 3.0) + per_slice * s;
+    if (c < least) { least = c; best = s; }
+  }
+  return best;
+}
+
+template <bool GRAD>
+static int launch_flash(const void* r, const void* t, const HeadArgs& g, int sms, cudaStream_t st) {
+  static bool attr_set[64] = {false};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -2;
+  if (!attr_set[dev]) {
+    if (cudaFuncSetAttribute(head_flash_kernel<GRAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, HeadSmem::TOTAL) != cudaSuccess) return -2;
+    attr_set[dev] = true;
+  }
+  CUtensorMap tr, tt;
+  int rc = cached_tmap(&tr, TMAP_BF16_2D, r, g.width, 1, g.rows, g.width, 64, 128);
+  if (rc == 0) rc = cached_tmap(&tt, TMAP_BF16_2D, t, g.width, 1, g.cols, g.width, 64, 128);
+  if (rc) return rc;
+  const int total = (g.rows + 127) / 128 * g.slices;
+  return launch(head_flash_kernel<GRAD>, total < sms ? total : sms, HF_THREADS, HeadSmem::TOTAL, st, 1, tr, tt, g) == cudaSuccess ? 0 : -3;
+}
+static int sm_count(int* sms) {
+  int dev = 0;
+  return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess ? 0 : -2;
+}
+static bool misaligned(const void* a, const void* b, const void* c = nullptr, const void* d = nullptr) {
+  return (reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c) | reinterpret_cast<uintptr_t>(d)) & 15;
+}
+
+}  // namespace dsw
+
+using namespace dsw;
+
+// Slices of the vocabulary that dsw_head_softmax is to be given for M rows, 0 for a width that it does not take.  Host
+// arithmetic only.
+extern "C" int dsw_head_slices(int M, int V, int K, int sms) {
+  if (M <= 0 || V <= 0 || K <= 0 || K > HF_W || K % 8 || sms <= 0) return 0;
+  // a slice's sums are written and read once (512 bytes a row at some 3 TB/s), one after the other where rows are few
+  return pick_slices(M, V, sms, 0.03 + M * 1024.0 / 3e6);
+}
+
+extern "C" int dsw_head_softmax(const void* x, const void* W, float* parts, void* ml, int M, int V, int K, int slices, int* status,
+                                cudaStream_t st) {
+  if (M <= 0 || V <= 0 || K <= 0) return 0;
+  if (K % 8 || K > HF_W || slices < 1 || slices > (V + 127) / 128) return -10;
+  if (misaligned(x, W, parts, ml)) return -11;
+  int sms = 0;
+  if (sm_count(&sms)) return -2;
+  HeadArgs g = {};
+  g.rows = M; g.cols = V; g.width = K; g.slices = slices;
+  g.out = parts; g.ml = static_cast<float2*>(ml); g.status = status;
+  return launch_flash<false>(x, W, g, sms, st);
+}
+
+extern "C" int dsw_head_join(const float* parts, const void* ml, const void* x, const void* W, const long long* targets,
+                             const long long* mask, const float* count, float scale, float* loss_acc, void* dx, float* nlse,
+                             int* target, float* coef, int M, int V, int K, int slices, int* status, cudaStream_t st) {
+  if (M <= 0) return 0;
+  if (K % 8 || K <= 0 || K > HF_W || V <= 0 || slices < 1) return -10;
+  if (misaligned(parts, x, W, dx)) return -11;
+  const int padded = (M + 127) / 128 * 128;
+  const auto go = [&](auto kernel, int rows_per_block) {
+    const int blocks = (padded + rows_per_block - 1) / rows_per_block;
+    return launch(kernel, blocks < 1184 ? blocks : 1184, 256, 0, st, 1, parts, static_cast<const float2*>(ml),
+                  static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(W), targets, mask, count, scale, loss_acc,
+                  static_cast<__nv_bfloat16*>(dx), nlse, target, coef, M, V, K, slices, status) == cudaSuccess ? 0 : -3;
+  };
+  return slices >= 16 ? go(head_join_kernel<8>, 1) : go(head_join_kernel<1>, 8);
+}
+
+extern "C" int dsw_head_wgrad(const void* x, const void* W, const float* nlse, const int* target, const float* coef, float* dW,
+                              int M, int V, int K, int deterministic, int* status, cudaStream_t st) {
+  if (M <= 0 || V <= 0 || K <= 0) return 0;
+  if (K % 8 || K > HF_W) return -10;
+  if (misaligned(x, W, nlse, target) || misaligned(dW, nullptr)) return -11;
+  int sms = 0;
+  if (sm_count(&sms)) return -2;
+  HeadArgs g = {};
+  g.rows = V; g.cols = M; g.width = K;
+  // a slice adds the whole matrix to memory once more; one slice adds to every element once, in any order of the units
+  g.slices = deterministic ? 1 : pick_slices(V, M, sms, 4.0 * V * K / 4e6);
+  g.out = dW; g.nlse = nlse; g.target = target; g.coef = coef; g.status = status;
+  return launch_flash<true>(W, x, g, sms, st);
+}
+
+extern "C" int dsw_load_head_flash() {
+  cudaFuncAttributes a;
+  const bool bad = cudaFuncGetAttributes(&a, head_flash_kernel<true>) != cudaSuccess || cudaFuncGetAttributes(&a, head_flash_kernel<false>) != cudaSuccess ||
+                   cudaFuncGetAttributes(&a, head_join_kernel<1>) != cudaSuccess || cudaFuncGetAttributes(&a, head_join_kernel<8>) != cudaSuccess;
+  return bad ? -1 : 0;
+}
+
+DSW_BOUNDS_TU(dsw_bounds_head_flash)

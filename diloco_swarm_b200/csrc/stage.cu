@@ -209,12 +209,15 @@ struct Scratch {
   bf16 *dh[2], *dx[3], *dx1[2], *dqkv[2], *dln, *datt, *logits;
   float *parts, *tlogit;         // see dsw_head_lse
   float4* rows;                  // see dsw_head_rows
+  float2* ml;                    // see dsw_head_softmax and its companions, as parts
+  float *nlse, *coef;
+  int* target;
   float *dq_acc, *dvec, *ln[5];  // LayerNorm backward's sums per block of threads: of ln_2 and ln_1 by block parity, of the final one
 };
 
 // Whether the cross-entropy of a pass goes without stored logits (dsw_head_lse and its companions; tiles are 256 columns
 // wide).  Without a gradient always: no logits are written and read again (width 768, 32768 rows: 3007 -> 1749 us, 128
-// rows: 37 -> 32).  With one they have to be computed a second time, which narrow models do faster than they read and
+// rows: 37 -> 32).  With one they have to be computed a second time, which narrow models (those of more than 128 columns) do faster than they read and
 // write them once more, given enough rows for the third launch (us, stored / unstored, 50304 columns; no width between 384
 // and 768 was measured; width 128: 512 rows
 // 49 / 51, 2048 145 / 120, 32768 2018 / 1750; width 384: 512 rows 68 / 78, 2048 219 / 182, 32768 2820 / 2083; width 768:
@@ -225,11 +228,25 @@ bool unstored_logits(const Stage& s, bool grad, size_t M) {
   return s.V > 128 && (!grad || (s.d <= HEAD_TWICE_WIDTH && M >= size_t(HEAD_TWICE_ROWS)));
 }
 
+// Whether loss and gradients of the head are computed without logits and without their gradient (head_flash.cu): where the
+// model is narrow enough for head_flash.cu's tiles, at any number of rows (whole head, us, width 128 and 50304 columns, the path
+// before / this one: 128 rows 66 / 40, 65536 5650 / 2550).
+// Slices of the vocabulary, by the rows of the microbatch as well; 0: the model is too wide, or there is no gradient.
+int vocabulary_slices(const Stage& s, size_t M, bool grad) { return grad ? dsw_head_slices(int(M), s.V, s.d, s.sms) : 0; }
+
 // logit_rows: rows of the logits that exist at a time (0: the caller keeps them elsewhere)
 Scratch take_scratch(Area& a, const Stage& s, size_t M, bool grad, size_t logit_rows) {
   const size_t d = s.d;
   Scratch v = {};
-  if (s.head_w && logit_rows) {
+  const int slices = vocabulary_slices(s, M, grad);
+  if (s.head_w && logit_rows && slices) {
+    const size_t n = logit_rows * slices, padded = (logit_rows + 127) / 128 * 128;
+    v.parts = a.take<float>(n * 128);
+    v.ml = a.take<float2>(4 * n);
+    v.nlse = a.take<float>(padded);
+    v.target = a.take<int>(padded);
+    v.coef = a.take<float>(1);
+  } else if (s.head_w && logit_rows) {
     const bool unstored = unstored_logits(s, grad, M);
     if (grad || !unstored) v.logits = a.take<bf16>(logit_rows * s.V);
     if (unstored) {
@@ -543,6 +560,13 @@ struct Run {
     return 0;
   }
 
+  // the head's weights' gradient by head_flash.cu, on the side stream
+  int flash_wgrad(const Scratch& c, const bf16* ln, int m) const {
+    TRY(fork());
+    SIDE(dsw_head_wgrad(ln, s.head_w, c.nlse, c.target, c.coef, s.dhead_w, m, s.V, s.d, deterministic, s.status, side()));
+    return mark(marks->head);
+  }
+
   float scale() const { return 1.f / sqrtf(float(s.d / s.nh)); }
 };
 
@@ -708,19 +732,34 @@ extern "C" int dsw_stage_head(void* stage, void* saved, void* scratch, const lon
   TRY(r.join());           // an earlier call may have laid the scratch out differently
   LAUNCH(dsw_loss_begin(mask, M, s.count, loss, st));
   const int flags = (keep ? 1 : 0) | (deterministic ? 2 : 0) | (grad ? 4 : 0) | chunks << 3;
-  const bool unstored = unstored_logits(s, grad != 0, size_t(M));
+  const int slices = vocabulary_slices(s, size_t(M), grad != 0);
+  const bool flash = slices > 0, unstored = !flash && unstored_logits(s, grad != 0, size_t(M));
   const auto dlogits = [&](const bf16* ln, int m) {
     return dsw_head_dlogits(ln, s.head_w, c.rows, c.logits, m, V, d, s.status, r.st);
   };
+  const auto softmax = [&](const bf16* ln, int m) {
+    return dsw_head_softmax(ln, s.head_w, c.parts, c.ml, m, V, d, slices, s.status, r.st);
+  };
   TRY(r.replayed(GraphKey{1, B, T, flags, saved, scratch}, true, [&]() -> int {
     LAUNCH(dsw_layernorm_fwd(x, s.lnf_w, s.lnf_b, v.lnf, v.muf, v.rsf, M, d, 1e-5f, r.st));
-    if (rows == M && !unstored) LAUNCH(r.gemm(v.lnf, s.head_w, true, V, d, c.logits, DSW_EPI_STORE, nullptr, nullptr, nullptr, nullptr, M));
+    if (rows == M && flash) LAUNCH(softmax(v.lnf, M));
+    else if (rows == M && !unstored) LAUNCH(r.gemm(v.lnf, s.head_w, true, V, d, c.logits, DSW_EPI_STORE, nullptr, nullptr, nullptr, nullptr, M));
     return 0;
   }));
   for (int r0 = 0; r0 < M; r0 += rows) {
     const int m = M - r0 < rows ? M - r0 : rows;
     const bf16* ln = v.lnf + size_t(r0) * d;
     const long long* mk = mask ? mask + r0 : nullptr;
+    if (flash) {
+      if (rows < M) {
+        TRY(r.wait(r.marks->head));      // the rows' numbers of the slice before are still read
+        LAUNCH(softmax(ln, m));
+      }
+      LAUNCH(dsw_head_join(c.parts, c.ml, ln, s.head_w, targets + r0, mk, s.count, scale, loss, c.dln + size_t(r0) * d, c.nlse, c.target,
+                           c.coef, m, V, d, slices, s.status, st));
+      if (rows < M) TRY(r.flash_wgrad(c, ln, m));
+      continue;
+    }
     if (unstored) {
       LAUNCH(dsw_head_lse(ln, s.head_w, targets + r0, c.parts, c.tlogit, m, V, d, s.status, st));
       LAUNCH(dsw_head_rows(c.parts, c.tlogit, targets + r0, mk, s.count, scale, loss, grad ? c.rows : nullptr, m, V, s.status, st));
@@ -736,7 +775,9 @@ extern "C" int dsw_stage_head(void* stage, void* saved, void* scratch, const lon
   }
   if (!grad) return 0;
   TRY(r.replayed(GraphKey{2, B, T, flags, saved, scratch}, true, [&]() -> int {
-    if (rows == M) {
+    if (rows == M && flash) {
+      TRY(r.flash_wgrad(c, v.lnf, M));
+    } else if (rows == M) {
       if (unstored) LAUNCH(dlogits(v.lnf, M));
       TRY(r.head_grads(c, v.lnf, 0, M));
     }

@@ -43,6 +43,11 @@ _SIGS = {
     "dsw_head_rows": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_void_p, c_int, c_int, c_void_p,
                       c_void_p],
     "dsw_head_dlogits": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p],
+    "dsw_head_slices": [c_int, c_int, c_int, c_int],
+    "dsw_head_softmax": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
+    "dsw_head_join": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_void_p, c_void_p,
+                      c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
+    "dsw_head_wgrad": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     "dsw_gemm_choice": [c_int, c_int, c_int, c_int, c_int, c_int, c_int, ctypes.POINTER(c_int)],
     "dsw_gemm_partials": [c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_int, ctypes.POINTER(c_int), c_void_p, c_void_p],
     "dsw_sum_partials_bf16": [c_void_p, c_int, c_void_p, c_ll, c_void_p],
@@ -120,6 +125,7 @@ def load_all_kernels() -> None:
         return
     lib = cuda_lib()
     for name in ("dsw_load_gemm", "dsw_load_elementwise", "dsw_load_optim", "dsw_load_collectives",
+                 "dsw_load_head_flash",
                  "dsw_load_attention"):
         fn = getattr(lib, name, None)
         if fn is not None:

@@ -119,6 +119,23 @@ int dsw_head_rows(const float* parts, const float* tlogit, const long long*, con
 int dsw_head_dlogits(const void* A, const void*, const void* rows, void* out, int M, int N, int K, int*, cudaStream_t st) {
   return op("head_dlogits", st, {{'r', A, 2LL * M * K}, {'r', rows, 16LL * M}, {'w', out, 2LL * M * N}});
 }
+static int g_slices = 0;
+void fake_set_slices(int n) { g_slices = n; }
+int dsw_head_slices(int, int, int, int) { return g_slices; }
+int dsw_head_softmax(const void* x, const void*, float* parts, void* ml, int M, int, int K, int slices, int*, cudaStream_t st) {
+  return op("head_softmax", st, {{'r', x, 2LL * M * K}, {'w', parts, 512LL * slices * M}, {'w', ml, 32LL * slices * M}});
+}
+int dsw_head_join(const float* parts, const void* ml, const void* x, const void*, const long long*, const long long*, const float*, float,
+                  float*, void* dx, float* nlse, int* target, float* coef, int M, int, int K, int slices, int*, cudaStream_t st) {
+  const long long padded = (M + 127) / 128 * 128;
+  return op("head_join", st, {{'r', parts, 512LL * slices * M}, {'r', ml, 32LL * slices * M}, {'r', x, 2LL * M * K}, {'w', dx, 2LL * M * K},
+                              {'w', nlse, 4 * padded}, {'w', target, 4 * padded}, {'w', coef, 4}});
+}
+int dsw_head_wgrad(const void* x, const void*, const float* nlse, const int* target, const float* coef, float* dW, int M, int V, int K, int,
+                   int*, cudaStream_t st) {
+  const long long padded = (M + 127) / 128 * 128;
+  return op("head_wgrad", st, {{'r', x, 2LL * M * K}, {'r', nlse, 4 * padded}, {'r', target, 4 * padded}, {'r', coef, 4}, {'a', dW, 4LL * V * K}});
+}
 int dsw_gemm_partials(const void* A, const void*, int M, int N, int K, float* partials, int most, int* splits, int*, cudaStream_t st) {
   *splits = most;
   return op("gemm_partials", st, {{'r', A, 2LL * M * K}, {'w', partials, 4LL * most * M * N}});

@@ -1,0 +1,97 @@
+"""Head of narrow models without logits (csrc/head_flash.cu): loss and both gradients."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(M, V, K, masked=False, scale=0.5, deterministic=0, slices=0, gain=1.0, seed=3, edit=None):
+    from diloco_swarm_b200.ops._lib import Status, check, cuda_lib, ptr, stream_ptr
+    lib, status = cuda_lib(), Status(torch.device("cuda", 0))
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    x = (torch.randn(M, K, device="cuda", generator=g) * gain).to(torch.bfloat16)
+    w = (torch.randn(V, K, device="cuda", generator=g) * 3 / K ** 0.5).to(torch.bfloat16)
+    tg = torch.randint(0, V, (M,), device="cuda", generator=g)
+    tg[::3] = torch.randint(0, min(V, 40), (len(tg[::3]),), device="cuda", generator=g)      # many rows with the same few targets
+    mask = (torch.rand(M, device="cuda", generator=g) < 0.7).long() if masked else None
+    if masked:
+        mask[0] = 1
+        tg[mask == 0] = -100                      # never looked at
+    if edit:
+        edit(x, tg, mask)
+    slices = slices or lib.dsw_head_slices(M, V, K, torch.cuda.get_device_properties(0).multi_processor_count)
+    padded = (M + 127) // 128 * 128
+    f = lambda *n: torch.full(n, 7.0, device="cuda")
+    parts, ml, nlse, coef, loss = f(slices, M, 128), f(slices, 4, M, 2), f(padded), f(1), torch.zeros((), device="cuda")
+    target = torch.full((padded,), 5, dtype=torch.int32, device="cuda")
+    dx, dw = f(M, K).to(torch.bfloat16), torch.ones(V, K, device="cuda")
+    count = torch.tensor([float(mask.sum()) if masked else float(M)], device="cuda")
+    check(lib.dsw_head_softmax(ptr(x), ptr(w), ptr(parts), ptr(ml), M, V, K, slices, status.ptr, stream_ptr()), "softmax")
+    check(lib.dsw_head_join(ptr(parts), ptr(ml), ptr(x), ptr(w), ptr(tg), ptr(mask), ptr(count), scale, ptr(loss), ptr(dx), ptr(nlse),
+                            ptr(target), ptr(coef), M, V, K, slices, status.ptr, stream_ptr()), "join")
+    check(lib.dsw_head_wgrad(ptr(x), ptr(w), ptr(nlse), ptr(target), ptr(coef), ptr(dw), M, V, K, deterministic, status.ptr,
+                             stream_ptr()), "wgrad")
+    torch.cuda.synchronize()
+    return x, w, tg, mask, loss, dx, dw - 1.0, status
+
+
+# tiles of 128 rows on either side: one, a remainder, several; widths with and without a second 64-column half; units with one,
+# two and more tiles (groups without a tile, fewer tiles than buffers)
+@pytest.mark.parametrize("M,V,K,slices", [(8, 136, 64, 2), (1, 8, 8, 1), (130, 264, 128, 1), (255, 512, 128, 4), (257, 1000, 72, 0),
+                                          (300, 50304, 128, 0), (700, 5000, 128, 16), (129, 904, 120, 1)])
+@pytest.mark.parametrize("masked", [False, True])
+def test_against_fp64(M, V, K, slices, masked):
+    scale = 0.5
+    x, w, tg, mask, loss, dx, dw, status = _run(M, V, K, masked, scale, slices=slices)
+    status.raise_if_set()
+    xd, wd = x.double().requires_grad_(), w.double().requires_grad_()
+    keep = mask.bool() if masked else torch.ones(M, dtype=torch.bool, device="cuda")
+    want = torch.nn.functional.cross_entropy((xd @ wd.t())[keep], tg[keep]) * scale
+    want.backward()
+    # fp32 sums over V columns in base 2: a few 1e-6 of a loss of the order of ten
+    assert abs(loss.item() - want.item()) <= 1e-5 * max(1.0, abs(want.item()))
+    # P is rounded to bf16 before its products (2^-9 of each term) and dx once more (2^-9): norm errors below 2^-8 and 2^-9
+    assert (dx.double() - xd.grad).norm() <= 2 ** -8 * xd.grad.norm()
+    # dw was added to ones in fp32: 2^-24 of them each
+    assert (dw.double() - wd.grad).norm() <= 2 ** -9 * wd.grad.norm() + 2 ** -24 * (V * K) ** 0.5
+    if masked:
+        assert torch.all(dx[~keep] == 0)
+
+
+def test_rows_far_above_their_first_tile():
+    """Logits that exceed the slice's reference by more than 2^100 are done over row by row: the same results."""
+    x, w, tg, mask, loss, dx, dw, status = _run(200, 3000, 128, True, gain=30.0, slices=12)
+    status.raise_if_set()
+    xd, wd = x.double().requires_grad_(), w.double().requires_grad_()
+    keep = mask.bool()
+    logits = xd @ wd.t()
+    first = logits.detach()[keep].view(int(keep.sum()), -1)[:, :128].max(1).values
+    assert (logits.detach()[keep].max(1).values - first > 100 * 0.6931).any()          # the case is met
+    want = torch.nn.functional.cross_entropy(logits[keep], tg[keep]) * 0.5
+    want.backward()
+    assert abs(loss.item() - want.item()) <= 1e-5 * want.item()
+    assert (dx.double() - xd.grad).norm() <= 2 ** -8 * xd.grad.norm()
+    # exponents of the order of 150: an fp32 logit is good to 2^-24 of that, some 1e-5 of a probability
+    assert (dw.double() - wd.grad).norm() <= 2 ** -8 * wd.grad.norm()
+
+
+def test_masked_rows_and_bad_targets():
+    """Infinities in a masked row reach neither the loss nor the other rows' gradient; a target outside the vocabulary in a kept
+    row sets the status word."""
+    def masked_inf(x, tg, mask):
+        x[3] = float("inf")
+        mask[3] = 0
+    *_, loss, dx, dw, status = _run(140, 264, 64, True, edit=masked_inf)
+    status.raise_if_set()
+    assert torch.isfinite(loss) and torch.all(dx[3] == 0) and torch.isfinite(dx.float()).all()
+
+    def bad(x, tg, mask):
+        tg[5] = 264
+    *_, status = _run(140, 264, 64, edit=bad)
+    with pytest.raises(RuntimeError):
+        status.raise_if_set()
+
+
+def test_deterministic_gradients_repeat():
+    a, b = (_run(1500, 1000, 128, True, deterministic=1) for _ in range(2))
+    assert torch.equal(a[6], b[6]) and torch.equal(a[5], b[5])

@@ -1,0 +1,22 @@
+"""The executor's narrow head (no stored logits, both gradients from head_flash.cu) on the emulated device: the order of all
+accesses, in one piece and in slices, queued, replayed and by turns with passes of other sizes."""
+import pytest
+
+from stage_device import FakeStage
+from test_stage_order import AREA, device, lib, ordered  # noqa: F401
+
+
+@pytest.mark.parametrize("chunks", [1, 3])
+@pytest.mark.parametrize("slices", [1, 5])
+def test_order_of_a_narrow_head(device, chunks, slices):  # noqa: F811
+    device.lib.fake_set_slices(slices)
+    try:
+        s = FakeStage(device.lib, n=3)
+        rcs = [s.train((2 + i % 2) * AREA, 5 * AREA, *((1, 100), (2, 512))[i % 3 == 1], 1, chunks=chunks) for i in range(9)]
+        ordered(device, *rcs)
+        for name in ("head_softmax", "head_join", "head_wgrad"):
+            assert device.names.count(name) == (9 if chunks == 1 else 12)          # slices are whole tiles: 100 rows are one, 1024 two
+        assert not any(name in device.names for name in ("head_lse", "cross_entropy", "gemm_partials"))
+        assert "replay" in device.counts
+    finally:
+        device.lib.fake_set_slices(0)
