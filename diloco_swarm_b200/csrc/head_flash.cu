@@ -22,11 +22,11 @@
 //
 // What bounds it: per 128 x 128 tile 1024 clocks of tensor core and 1024 of exponentials (16 a clock and SM).  Before, the
 // head of 65536 tokens at width 128 and 50304 columns was four kernels: log-sum-exp 1462 us, the logits' gradient 1730
-// (6.6 GB written), and the two products that read it from DRAM, 1150 and 1232.  Here 1225, 100 and 1225 (some 1700 clocks a
-// tile); 8192 tokens 178, 14 and 183; 128 tokens 13, 10 and 17, where logits that are stored took 9.5, cross-entropy 11, and
-// the products 34 and 11.  What keeps a tile above 1024 clocks: eight dependent products with P from TMEM take 1025 by
-// themselves, eight of S (N = 128) 733 where 512 would do, and the chain S, P, O of a tile is only three tiles deep.  Without
-// the exponentials it was 11 % less, and a quarter to a half of them on the FMA pipe (a polynomial) gained nothing.
+// (6.6 GB written), and the two products that read it from DRAM, 1150 and 1232.  Here 1125, 100 and 1155 (some 1500 clocks a
+// tile); 8192 tokens 155, 14 and 175; 128 tokens 13, 10 and 19, where logits that are stored took 9.5, cross-entropy 11, and
+// the products 34 and 11.  What keeps a tile above 1024 clocks is its chain S, P, O, which is three tiles deep: a barrier
+// passed, even a complete one, costs some 230 clocks, and P of a tile some 1500 for its two warps per scheduler.  With a
+// quarter to a half of the exponentials on the FMA pipe (a polynomial) nothing was gained, nor with five stages.
 #include <cuda.h>
 #include "gemm_kernels.cuh"
 #include "launch.h"
@@ -41,7 +41,7 @@ constexpr int HF_TILE = 2 * HF_SLAB;
 constexpr int HF_STAGES = 4;
 constexpr int HF_BUFS = 3;                       // of S and P
 constexpr int HF_ROW_WARPS = 16;
-constexpr int HF_MMA_WARP = HF_ROW_WARPS, HF_TMA_WARP = HF_ROW_WARPS + 1;
+constexpr int HF_S_WARP = HF_ROW_WARPS, HF_TMA_WARP = HF_ROW_WARPS + 1, HF_O_WARP = HF_ROW_WARPS + 2;
 constexpr int HF_THREADS = 32 * (HF_ROW_WARPS + 4);
 
 struct HeadSmem {
@@ -104,7 +104,8 @@ head_flash_kernel(const __grid_constant__ CUtensorMap tmap_r, const __grid_const
   uint64_t* m_full = bars + 4;         // per unit: maxima of the first tile written (8 warps arrive; softmax)
   uint64_t* s_full = bars + 5;         // [bufs] per tile: S in TMEM
   uint64_t* p_full = s_full + HF_BUFS; // [bufs] per tile: P in TMEM (8 warps arrive)
-  uint64_t* t_full = p_full + HF_BUFS; // [stages]
+  uint64_t* b_free = p_full + HF_BUFS; // [bufs] per tile: its P T product done
+  uint64_t* t_full = b_free + HF_BUFS; // [stages]
   uint64_t* t_empty = t_full + HF_STAGES;
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(t_empty + HF_STAGES);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
@@ -124,22 +125,22 @@ head_flash_kernel(const __grid_constant__ CUtensorMap tmap_r, const __grid_const
 
   if (threadIdx.x == 0) {
     mbar_init(r_full, 1); mbar_init(r_empty, 1); mbar_init(o_full, 1); mbar_init(o_free, HF_ROW_WARPS); mbar_init(m_full, 8);
-    for (int i = 0; i < HF_BUFS; ++i) { mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 8); }
+    for (int i = 0; i < HF_BUFS; ++i) { mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 8); mbar_init(&b_free[i], 1); }
     for (int i = 0; i < HF_STAGES; ++i) { mbar_init(&t_full[i], 1); mbar_init(&t_empty[i], 1); }
     *abort_flag = 0;
     mbar_fence_init();
     fence_proxy_async();
   }
-  if (warp == HF_MMA_WARP) {
+  if (warp == HF_S_WARP) {
     tmem_alloc(tmem_holder, 512);
     tmem_relinquish();
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  // all 512 columns, so from 0: O, then the three buffers of S (P: columns 0-31 and 64-95 of one)
   const uint32_t tmem_base = *tmem_holder;
-  const auto tmem_s = [=](uint32_t buf) { return tmem_base + 128 + buf * 128; };          // P: columns 0-31 and 64-95 of it
-  const uint32_t tmem_o = tmem_base;
+  if (tmem_base != 0 && threadIdx.x == 0 && g.status) atomicCAS(g.status, 0, ST_BAD_ARG);
 
   if (warp >= HF_ROW_WARPS) asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
   if (warp == HF_TMA_WARP) {
@@ -182,57 +183,62 @@ head_flash_kernel(const __grid_constant__ CUtensorMap tmap_r, const __grid_const
         for (int spin = 0; spin < 100000; ++spin)
           if (mbar_try_wait(s < HF_STAGES ? &t_full[s] : r_full, 0) || mbar_try_wait(s < HF_STAGES ? &t_full[s] : r_full, 1)) break;
     }
-  } else if (warp == HF_MMA_WARP) {
-    // ------------------------------------------------------------ MMA issuer (the whole warp, one lane issues)
-    const uint32_t idesc_s = make_idesc_bf16(128, 128, 0, 0), idesc_o = make_idesc_bf16(128, 128, 0, 1);
-    const uint32_t desc_hi = smem_desc_hi(1024);
-    const uint32_t r_lo = smem_desc_lo(smem_u32(smem + L::R_OFF), 16);
+  } else if (warp == HF_S_WARP) {
+    // ------------------------------------------------------------ issuer of S (a whole warp, one lane issues)
+    // Two warps issue, one the products S and one P T: passing a barrier, even one that is complete, takes some 230 clocks, two
+    // of them a tile, and the tensor core has few products queued to live on meanwhile (by one warp: 1700 clocks a tile).
+    constexpr uint32_t idesc = make_idesc_bf16(128, 128, 0, 0), desc_hi = smem_desc_hi(1024);
+    const uint32_t r_lo = smem_desc_lo(smem_u32(smem + L::R_OFF), 16), t_k = smem_desc_lo(smem_u32(smem + L::T_OFF), 16);
     uint32_t it = 0, w = 0;
     bool ok = true;
-    // S of tile i into its buffer: over P of tile i - 3, right behind the product that reads it.  Eight products of each kind
-    // in a row take 1706 clocks that way, 1166 where S goes elsewhere; issued a product later, or after a wait for the one
-    // that reads P, the next tile's chain took as long as that saved (1222 and 1389 us for 65536 rows, this way 1212).
-    const auto issue_s = [&](uint32_t i) -> bool {
-      const int s = i % HF_STAGES, buf = i % HF_BUFS;
-      if (!mbar_wait_warp(&t_full[s], (i / HF_STAGES) & 1, abort_flag, g.status)) return false;
-      const uint32_t t_lo = smem_desc_lo(smem_u32(smem + L::T_OFF + s * HF_TILE), 16);
-      if (elect_one()) {
-#pragma unroll
-        for (int k = 0; k < HF_W / UMMA_K; ++k) {
-          const uint32_t step = (k >> 2) * (HF_SLAB >> 4) + (k & 3) * 2;
-          umma_bf16_lohi(tmem_s(buf), r_lo + step, t_lo + step, desc_hi, idesc_s, k > 0);
-        }
-        umma_commit(&s_full[buf]);
-      }
-      __syncwarp();
-      return true;
-    };
     for (int u = blockIdx.x; u < total && ok; u += gridDim.x, ++w) {
-      const int n = unit_at(u).n, ahead = n < HF_BUFS ? n : HF_BUFS;
+      const int n = unit_at(u).n;
       if (!mbar_wait_warp(r_full, w & 1, abort_flag, g.status)) break;
-      for (int j = 0; j < ahead && ok; ++j) ok = issue_s(it + j);
-      if (ok && n <= HF_BUFS && elect_one()) umma_commit(r_empty);
-      __syncwarp();
-      for (int j = 0; j < n && ok; ++j, ++it) {
-        const int s = it % HF_STAGES, buf = it % HF_BUFS;
-        const uint32_t t_lo = smem_desc_lo(smem_u32(smem + L::T_OFF + s * HF_TILE), HF_SLAB);
+      for (int j = 0; j < n; ++j, ++it) {
+        const uint32_t s = it % HF_STAGES, buf = it % HF_BUFS;
+        if (!mbar_wait_warp(&t_full[s], (it / HF_STAGES) & 1, abort_flag, g.status)) { ok = false; break; }
+        // over P of the tile three before
+        if (!mbar_wait_warp(&b_free[buf], ((it / HF_BUFS) & 1) ^ 1, abort_flag, g.status)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t t_lo = t_k + s * (HF_TILE >> 4), to = 128 + buf * 128;
+        if (elect_one()) {
+#pragma unroll
+          for (int k = 0; k < HF_W / UMMA_K; ++k) {
+            const uint32_t step = (k >> 2) * (HF_SLAB >> 4) + (k & 3) * 2;
+            umma_bf16_lohi(to, r_lo + step, t_lo + step, desc_hi, idesc, k > 0);
+          }
+          umma_commit(&s_full[buf]);
+          if (j + 1 == n) umma_commit(r_empty);
+        }
+        __syncwarp();
+      }
+    }
+  } else if (warp == HF_O_WARP) {
+    // ------------------------------------------------------------ issuer of P T
+    constexpr uint32_t idesc = make_idesc_bf16(128, 128, 0, 1), desc_hi = smem_desc_hi(1024);
+    const uint32_t t_mn = smem_desc_lo(smem_u32(smem + L::T_OFF), HF_SLAB);
+    uint32_t it = 0, w = 0;
+    bool ok = true;
+    for (int u = blockIdx.x; u < total && ok; u += gridDim.x, ++w) {
+      const int n = unit_at(u).n;
+      for (int j = 0; j < n; ++j, ++it) {
+        const uint32_t s = it % HF_STAGES, buf = it % HF_BUFS;
+        // T is read here too: seen by waiting for the loads oneself
+        if (!mbar_wait_warp(&t_full[s], (it / HF_STAGES) & 1, abort_flag, g.status)) { ok = false; break; }
         if (!mbar_wait_warp(&p_full[buf], (it / HF_BUFS) & 1, abort_flag, g.status)) { ok = false; break; }
         // the unit before has been read out of O
         if (j == 0 && w > 0 && !mbar_wait_warp(o_free, (w - 1) & 1, abort_flag, g.status)) { ok = false; break; }
         tc_fence_after();
+        const uint32_t t_lo = t_mn + s * (HF_TILE >> 4), from = 128 + buf * 128;
         if (elect_one()) {
 #pragma unroll
           for (int k = 0; k < 128 / UMMA_K; ++k)
-            umma_bf16_ts(tmem_o, tmem_s(buf) + (k >> 2) * 64 + (k & 3) * 8, t_lo + k * (2048 >> 4), desc_hi, idesc_o, j > 0 || k > 0);
+            umma_bf16_ts(0, from + (k >> 2) * 64 + (k & 3) * 8, t_lo + k * (2048 >> 4), desc_hi, idesc, j > 0 || k > 0);
+          umma_commit(&b_free[buf]);
           umma_commit(&t_empty[s]);
           if (j + 1 == n) umma_commit(o_full);
         }
         __syncwarp();
-        if (j + HF_BUFS < n) {
-          if (!issue_s(it + HF_BUFS)) { ok = false; break; }
-          if (j + HF_BUFS + 1 == n && elect_one()) umma_commit(r_empty);
-          __syncwarp();
-        }
       }
     }
   } else if (warp < HF_ROW_WARPS) {
@@ -240,7 +246,7 @@ head_flash_kernel(const __grid_constant__ CUtensorMap tmap_r, const __grid_const
     asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
     const int grp = warp >> 3, half = (warp >> 2) & 1, q = warp & 3;
     const uint32_t quarter = uint32_t(q * 32) << 16;
-    const uint32_t to = tmem_o + quarter + (grp * 2 + half) * 32;          // the columns of O that this warp reads out
+    const uint32_t to = quarter + (grp * 2 + half) * 32;          // the columns of O that this warp reads out
     uint8_t* stage = smem + L::EPI_OFF + warp * EPI_STAGE_BYTES;
     float* xm = reinterpret_cast<float*>(smem + L::MAX_OFF) + q * 32 + lane;
     uint32_t it = 0, w = 0;
@@ -254,7 +260,7 @@ head_flash_kernel(const __grid_constant__ CUtensorMap tmap_r, const __grid_const
       for (int j = 0; j < x.n; ++j, ++it) {
         if (int(it & 1) != grp) continue;
         const int s = it % HF_STAGES, buf = it % HF_BUFS;
-        const uint32_t ts = tmem_s(buf) + quarter + half * 64;
+        const uint32_t ts = 128 + buf * 128 + quarter + half * 64;
         // its statistics lie in the stage: seen by waiting for the loads oneself
         if (GRAD && !mbar_wait(&t_full[s], (it / HF_STAGES) & 1, abort_flag, g.status)) { ok = false; break; }
         if (!mbar_wait(&s_full[buf], (it / HF_BUFS) & 1, abort_flag, g.status)) { ok = false; break; }
@@ -386,7 +392,7 @@ head_flash_kernel(const __grid_constant__ CUtensorMap tmap_r, const __grid_const
 
   tc_fence_before();
   __syncthreads();
-  if (warp == HF_MMA_WARP) {
+  if (warp == HF_S_WARP) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
   }
