@@ -29,6 +29,7 @@
 #include "ptx.cuh"
 #include "launch.h"
 #include "tmap.h"
+#include "attention_short.cuh"
 #include "dswarm.h"
 
 namespace dsw {
@@ -103,8 +104,8 @@ __device__ __forceinline__ bool att_item(int r, int c, int G, int total, int& id
 }
 
 // SOLO: no more items than SMs.  A row then goes straight from its thread, 16 bytes at a time: staged through shared memory as
-// the rows of more items are, it leaves some 0.4 us later (1 x 24 tokens, 4 heads of 32: 6.4 -> 6.0 us a launch; 5 x 24, 12
-// heads of 64: 6.5 -> 6.1).  With two CTAs on an SM the stores of a row per lane get in each other's way: 16 x 128, 12 heads,
+// the rows of more items are, it leaves some 0.4 us later (1 x 24 tokens, 4 heads of 32, before sequences of one tile had a
+// kernel of their own: 6.4 -> 6.0 us a launch; 5 x 24, 12 heads of 64: 6.5 -> 6.1).  With two CTAs on an SM the stores of a row per lane get in each other's way: 16 x 128, 12 heads,
 // 192 items, 9.1 us staged, 10.0 not.
 template <bool SOLO>
 __global__ void __launch_bounds__(ATT_THREADS, 2)
@@ -1177,6 +1178,14 @@ static int att_num_sms() {
   }
   return n;
 }
+// Which forward kernel a call takes; the bits are the same.  us a launch, tcgen05 / short (attention_short.cuh), n heads of all
+// sequences together.  Heads of 64: T = 24, n 4 to 296 5.8-7.0 / 2.7-2.9, 3000 41.5 / 10.6; T = 64, 4 5.9 / 3.5, 3000 41.7 /
+// 23.1; T = 96, 4 5.9 / 4.4, 296 7.7 / 5.5, 1000 18.4 / 17.3; T = 128, 4 6.1 / 5.1, 296 7.8 / 6.8, 400 11.2 / 11.8, 1000 19.5 /
+// 21.8 (296: one wave of two blocks per SM).  Heads of 32 at T = 128: 4 6.0 / 4.2, 296 7.8 / 5.2, 1000 19.4 / 15.6.
+static bool attention_is_short(int T, int hs, int n_bh) {
+  if (T > SHORT_MAX_T) return false;
+  return hs == 32 || T <= 64 || n_bh <= 2 * att_num_sms() || (T <= 96 && n_bh <= 6 * att_num_sms());
+}
 // Register (or clear, with nullptr) a device buffer of 512 int64 for the in-kernel timeline.
 extern "C" int dsw_attention_set_trace(long long* buf) { g_att_trace = buf; return 0; }
 
@@ -1186,6 +1195,11 @@ extern "C" int dsw_attention_fwd(const void* qkv, void* out, float* lse, int B, 
                                  int* status, cudaStream_t st) {
   if ((hs != 64 && hs != 32) || T <= 0) return -10;
   const int d = nh * hs;
+  if (attention_is_short(T, hs, B * nh)) {
+    const float s2 = scale * 1.4426950408889634f;
+    return hs == 64 ? attention_short<64>((const __nv_bfloat16*)qkv, (__nv_bfloat16*)out, lse, T, nh, B * nh, s2, st)
+                    : attention_short<32>((const __nv_bfloat16*)qkv, (__nv_bfloat16*)out, lse, T, nh, B * nh, s2, st);
+  }
   CUtensorMap tm;
   const int rc = cached_tmap(&tm, TMAP_BF16_4D, qkv, hs, 3LL * nh, T, 3LL * d, 64, 128, B);
   if (rc) return rc;
@@ -1271,6 +1285,7 @@ extern "C" int dsw_load_attention() {
   cudaFuncAttributes a;
   int bad = 0;
   bad |= cudaFuncGetAttributes(&a, attention_fwd_kernel<true>) != cudaSuccess;
+  bad |= load_attention_short();
   bad |= cudaFuncGetAttributes(&a, attention_fwd_kernel<false>) != cudaSuccess;
   bad |= cudaFuncGetAttributes(&a, attention_bwd_kernel<false>) != cudaSuccess;
   bad |= cudaFuncGetAttributes(&a, attention_bwd_kernel<true>) != cudaSuccess;

@@ -1,0 +1,42 @@
+"""Attention forward of short sequences on mma.sync (csrc/attention_short.cuh): the bits of the tcgen05 kernel, and 64 bits."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+# one row, remainders of a warp's 16 rows on either side of the block counts (32, 64, 128 rows), whole ones; both head sizes; one
+# head and more heads than SMs
+@pytest.mark.parametrize("T", [1, 15, 16, 17, 24, 31, 32, 33, 48, 64, 65, 96, 97, 127, 128])
+@pytest.mark.parametrize("B,nh,hs", [(1, 1, 64), (3, 4, 32), (13, 12, 64)])
+def test_short_sequences(T, B, nh, hs):
+    from diloco_swarm_b200.ops._lib import Status
+    from diloco_swarm_b200.ops.attention import attention_fwd
+    st, d, longer = Status(torch.device("cuda")), nh * hs, T + 129          # longer: the tcgen05 kernel's first rows
+    g = torch.Generator(device="cuda").manual_seed(T)
+    qkv = (torch.randn(B, longer, 3 * d, device="cuda", generator=g) * 2).to(torch.bfloat16)
+    out, ctx = attention_fwd(qkv[:, :T].reshape(B * T, 3 * d).contiguous(), B, T, nh, status=st)
+    all_rows, all_ctx = attention_fwd(qkv.view(B * longer, 3 * d), B, longer, nh, status=st)
+    torch.cuda.synchronize()
+    st.raise_if_set()
+    assert torch.equal(out.view(B, T, d), all_rows.view(B, longer, d)[:, :T])
+    assert torch.equal(ctx.lse.view(B * nh, T), all_ctx.lse.view(B * nh, longer)[:, :T])
+    q, k, v = qkv[:, :T].double().view(B, T, 3, nh, hs).permute(2, 0, 3, 1, 4)
+    s = (q @ k.transpose(-1, -2) / hs ** 0.5).masked_fill(torch.ones(T, T, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
+    want = (s.softmax(-1) @ v).transpose(1, 2).reshape(B * T, d)
+    # P is rounded to bf16 before its product and the result once more: 2^-9 of each
+    assert (out.double() - want).norm() <= 2 ** -8 * want.norm()
+    # an fp32 exponent of the order of 30, good to 2^-23 of that
+    assert (ctx.lse.view(B, nh, T).double() - s.logsumexp(-1)).abs().max() < 1e-4
+
+
+@pytest.mark.parametrize("T", [17, 64, 100])
+def test_what_lies_behind_a_sequence_stays_out(T):
+    """Infinities in the next sequence's rows, where a block's last rows would reach."""
+    from diloco_swarm_b200.ops.attention import attention_fwd
+    g = torch.Generator(device="cuda").manual_seed(T)
+    qkv = torch.randn(2 * T, 3 * 128, device="cuda", generator=g).to(torch.bfloat16)
+    alone, _ = attention_fwd(qkv[:T].contiguous(), 1, T, 4)
+    qkv[T:] = float("inf")
+    both, _ = attention_fwd(qkv, 2, T, 4)
+    assert torch.equal(both[:T], alone)
