@@ -49,6 +49,13 @@ int dsw_gemm_bf16(const void* A, long long lda, int a_mn_major, const void* B, l
 // The kernel (bn) that dsw_gemm_bf16 takes for activations [M,K] times a weight matrix when bn is 0, and the split of K of
 // the cluster kernel; derivative: DSW_EPI_GELU with aux_out.  Host arithmetic only.
 int dsw_gemm_choice(int M, int N, int K, int mode, int b_mn_major, int derivative, int sms, int* split);
+// out [M,N] = LayerNorm(x + x_lo) W^T + bias (W [N,K]) in one launch, DSW_EPI_STORE or DSW_EPI_GELU (aux_out as there), for rows and
+// widths that dsw_layernorm_gemm_fits answers 1 for (derivative: DSW_EPI_GELU with aux_out; host arithmetic only): the bits of
+// dsw_layernorm_fwd_lo and dsw_gemm_bf16.  x_lo, beta, bias optional; ln_out (bf16 [M,K]) with mean and rstd (fp32 [M]): kept, or all null.
+int dsw_layernorm_gemm_fits(int M, int N, int K, int mode, int derivative, int sms);
+int dsw_layernorm_gemm(const void* x, const void* x_lo, const float* gamma, const float* beta, void* ln_out, float* mean, float* rstd,
+                       float eps, const void* W, const float* bias, void* out, int mode, void* aux_out, int M, int N, int K, int* status,
+                       cudaStream_t stream);
 // Masked cross-entropy of logits = A [M,K] W[N,K]^T in pieces that never hold the logits: dsw_head_lse writes partial
 // log-sum-exps (fp32 [ceil(N / 64)][M]) and the target's logit (fp32 [M]), dsw_head_rows (elementwise.cu) joins them into
 // the loss and one 16-byte record per row, dsw_head_dlogits computes the logits again and stores scale / count *

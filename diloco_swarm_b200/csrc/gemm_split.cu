@@ -1,5 +1,5 @@
 // Instantiations and launcher of the split-K cluster GEMM kernel for few rows (gemm_split.cuh).
-#include "gemm_split.cuh"
+#include "gemm_narrow.cuh"
 #include "dswarm.h"
 #include "launch.h"
 
@@ -58,6 +58,48 @@ int launch_split(int bn, const CUtensorMap& ta, const CUtensorMap& tb, const Gem
   return launch_bn<128>(ta, tb, g, st);
 }
 
-int load_split_kernels() { return (load_bn<32>() | load_bn<64>() | load_bn<128>()) ? -1 : 0; }
+namespace {
+template <int MODE, bool MN, bool LN>
+int launch_narrow_one(const GemmArgs& g, const NarrowArgs& n, cudaStream_t st) {
+  static bool attr_set[kMaxDevices] = {false};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return -2;
+  if (!attr_set[dev]) {
+    if (cudaFuncSetAttribute(gemm_narrow_kernel<MODE, MN, LN>, cudaFuncAttributeMaxDynamicSharedMemorySize, narrow_smem_bytes(NARROW_MAX_K, 8)) !=
+        cudaSuccess)
+      return -2;
+    attr_set[dev] = true;
+  }
+  const dim3 grid((g.M + NARROW_ROWS - 1) / NARROW_ROWS, (g.N + NARROW_COLS - 1) / NARROW_COLS);
+  return launch(gemm_narrow_kernel<MODE, MN, LN>, grid, NARROW_THREADS, narrow_smem_bytes(g.K, g.split_k), st, 1, g, n) == cudaSuccess ? 0 : -3;
+}
+template <bool MN>
+int launch_narrow_mn(const GemmArgs& g, const NarrowArgs& n, cudaStream_t st) {
+  switch (g.mode) {
+    case EPI_STORE: return launch_narrow_one<EPI_STORE, MN, false>(g, n, st);
+    case EPI_GELU: return launch_narrow_one<EPI_GELU, MN, false>(g, n, st);
+    case EPI_RESID: return launch_narrow_one<EPI_RESID, MN, false>(g, n, st);
+    case EPI_MUL: return launch_narrow_one<EPI_MUL, MN, false>(g, n, st);
+    default: return -13;
+  }
+}
+template <bool MN>
+int load_narrow() {
+  cudaFuncAttributes a;
+  return cudaFuncGetAttributes(&a, gemm_narrow_kernel<EPI_STORE, MN, false>) != cudaSuccess ||
+         cudaFuncGetAttributes(&a, gemm_narrow_kernel<EPI_GELU, MN, false>) != cudaSuccess ||
+         cudaFuncGetAttributes(&a, gemm_narrow_kernel<EPI_RESID, MN, false>) != cudaSuccess ||
+         cudaFuncGetAttributes(&a, gemm_narrow_kernel<EPI_MUL, MN, false>) != cudaSuccess ||
+         cudaFuncGetAttributes(&a, gemm_narrow_kernel<EPI_STORE, false, true>) != cudaSuccess ||
+         cudaFuncGetAttributes(&a, gemm_narrow_kernel<EPI_GELU, false, true>) != cudaSuccess;
+}
+}  // namespace
+
+int launch_narrow(const GemmArgs& g, const NarrowArgs& n, bool layernorm, cudaStream_t st) {
+  if (layernorm) return g.mode == EPI_GELU ? launch_narrow_one<EPI_GELU, false, true>(g, n, st) : launch_narrow_one<EPI_STORE, false, true>(g, n, st);
+  return g.b_mn_major ? launch_narrow_mn<true>(g, n, st) : launch_narrow_mn<false>(g, n, st);
+}
+
+int load_split_kernels() { return load_narrow<false>() || load_narrow<true>() ? -1 : (load_bn<32>() | load_bn<64>() | load_bn<128>()) ? -1 : 0; }
 
 }  // namespace dsw

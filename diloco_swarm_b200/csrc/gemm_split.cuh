@@ -39,6 +39,49 @@ __device__ __forceinline__ void st_cluster_v4(uint32_t addr, uint32_t a, uint32_
   asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
 
+// Eight columns of a row, f: the finished sum with bias, x: residual or factor, t: the residual's low half.  f is left as what
+// was rounded.
+template <int MODE>
+__device__ __forceinline__ void finish_unit(const GemmArgs& g, int row, int col, float (&f)[8], const uint4& x, const uint4& t) {
+  uint32_t w[4];
+  if constexpr (MODE == EPI_GELU) {
+    uint32_t dw[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      f2 ga, da;
+      gelu_pair(f[2 * e], f[2 * e + 1], ga, da);
+      w[e] = pack_bf16_f2(ga);
+      dw[e] = pack_bf16_f2(da);
+    }
+    if (g.aux_out != nullptr)
+      *reinterpret_cast<uint4*>(g.aux_out + (long long)row * g.ldaux + col) = make_uint4(dw[0], dw[1], dw[2], dw[3]);
+  } else {
+    if constexpr (MODE == EPI_RESID || MODE == EPI_MUL || MODE == EPI_MUL_SUM) {
+      const uint32_t xu[4] = {x.x, x.y, x.z, x.w};
+      uint32_t tu[4] = {0, 0, 0, 0};
+      if constexpr (MODE == EPI_RESID) { tu[0] = t.x; tu[1] = t.y; tu[2] = t.z; tu[3] = t.w; }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 b = unpack_bf16(xu[e]), c = unpack_bf16(tu[e]);
+        f[2 * e] = MODE == EPI_RESID ? f[2 * e] + (b.x + c.x) : f[2 * e] * b.x;
+        f[2 * e + 1] = MODE == EPI_RESID ? f[2 * e + 1] + (b.y + c.y) : f[2 * e + 1] * b.y;
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) w[e] = pack_bf16(f[2 * e], f[2 * e + 1]);
+    if (MODE == EPI_RESID && g.aux_out != nullptr) {
+      uint32_t lo[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 h = unpack_bf16(w[e]);
+        lo[e] = pack_bf16(f[2 * e] - h.x, f[2 * e + 1] - h.y);
+      }
+      *reinterpret_cast<uint4*>(g.aux_out + (long long)row * g.ldaux + col) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    }
+  }
+  *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(g.out) + (long long)row * g.ldo + col) = make_uint4(w[0], w[1], w[2], w[3]);
+}
+
 // Cluster size (splits) is a launch attribute: 1, 2, 4 or 8, with BN / splits >= 8.
 template <int BN, int MODE>
 __global__ void __launch_bounds__(SPLIT_THREADS, BN <= 64 ? 2 : 1)
@@ -239,48 +282,12 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           f[0] += lo.x; f[1] += lo.y; f[2] += lo.z; f[3] += lo.w;
           f[4] += hi.x; f[5] += hi.y; f[6] += hi.z; f[7] += hi.w;
         }
-        uint32_t w[4];
-        if constexpr (MODE == EPI_GELU) {
-          uint32_t dw[4];
+        if constexpr (EXTRA) finish_unit<MODE>(g, row, col, f, x[i], t[MODE == EPI_RESID ? i : 0]);
+        else finish_unit<MODE>(g, row, col, f, make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0));
+        if constexpr (MODE == EPI_MUL_SUM) {
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            f2 ga, da;
-            gelu_pair(f[2 * e], f[2 * e + 1], ga, da);
-            w[e] = pack_bf16_f2(ga);
-            dw[e] = pack_bf16_f2(da);
-          }
-          if (g.aux_out != nullptr)
-            *reinterpret_cast<uint4*>(g.aux_out + (long long)row * g.ldaux + col) = make_uint4(dw[0], dw[1], dw[2], dw[3]);
-        } else {
-          if constexpr (EXTRA) {
-            const uint32_t xu[4] = {x[i].x, x[i].y, x[i].z, x[i].w};
-            uint32_t tu[4] = {0, 0, 0, 0};
-            if constexpr (MODE == EPI_RESID) { tu[0] = t[i].x; tu[1] = t[i].y; tu[2] = t[i].z; tu[3] = t[i].w; }
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const float2 b = unpack_bf16(xu[e]), c = unpack_bf16(tu[e]);
-              f[2 * e] = MODE == EPI_RESID ? f[2 * e] + (b.x + c.x) : f[2 * e] * b.x;
-              f[2 * e + 1] = MODE == EPI_RESID ? f[2 * e + 1] + (b.y + c.y) : f[2 * e + 1] * b.y;
-            }
-          }
-#pragma unroll
-          for (int e = 0; e < 4; ++e) w[e] = pack_bf16(f[2 * e], f[2 * e + 1]);
-          if constexpr (MODE == EPI_MUL_SUM) {
-#pragma unroll
-            for (int e = 0; e < 8; ++e) out8[e] = f[e];
-          }
-          if (MODE == EPI_RESID && g.aux_out != nullptr) {
-            uint32_t lo[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const float2 h = unpack_bf16(w[e]);
-              lo[e] = pack_bf16(f[2 * e] - h.x, f[2 * e + 1] - h.y);
-            }
-            *reinterpret_cast<uint4*>(g.aux_out + (long long)row * g.ldaux + col) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-          }
+          for (int e = 0; e < 8; ++e) out8[e] = f[e];
         }
-        *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(g.out) + (long long)row * g.ldo + col) =
-            make_uint4(w[0], w[1], w[2], w[3]);
       }
       if constexpr (MODE == EPI_MUL_SUM) {
         if (owner_of(u) == ks && col < g.N) {          // the same for the whole warp

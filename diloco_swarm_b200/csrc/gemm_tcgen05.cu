@@ -23,7 +23,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
-#include "gemm_split.cuh"
+#include "gemm_narrow.cuh"
 #include "launch.h"
 #include "tmap.h"
 #include "dswarm.h"
@@ -212,6 +212,20 @@ static int pick_wgrad(int M, int N, int K, int bn, int sms, int* split, int most
   return best;
 }
 
+// Whether what the cluster kernel would take goes to gemm_narrow.cuh instead (the bits are the same): while all its blocks are
+// resident at once and what they copy, with a launch's worth of work each besides, stays below a line.  us a launch, cluster /
+// narrow (one graph of launches; blocks and K): 128 x 384 from 128 3.9 / 2.5 (48), 1536 x 384 from 128 4.2 / 3.6 (576), 2048 x 512
+// from 128 4.9 / 5.5 (1024), 120 x 128 from 512 4.6 / 3.7 (16), 768 x 512 from 512 5.95 / 5.8 (384), 1024 x 512 6.0 / 7.4 (512),
+// 512 x 768 from 256 4.5 / 3.9 (384), 1024 x 768 5.2 / 5.9 (768); weights cold in L2: 120 x 768 from 768 5.0 / 4.3 (96), 64 x 3072
+// 7.2 / 5.9 (192), 120 x 3072 7.4 / 10.0 (384), 128 x 1024 from 1024 5.4 / 4.9 (128), 192 x 1024, of whose blocks an SM takes one,
+// 6.2 / 7.9 (192).
+static bool narrow_fits(int M, int N, int K, int splits, int sms) {
+  if (K > NARROW_MAX_K || K % BK) return false;
+  const long long blocks = (long long)((M + NARROW_ROWS - 1) / NARROW_ROWS) * ((N + NARROW_COLS - 1) / NARROW_COLS);
+  const int resident = (227 << 10) / (narrow_smem_bytes(K, splits) + 1024);
+  return blocks <= (long long)(resident < 8 ? resident : 8) * sms && blocks * (K + 256) <= 2000LL * sms;
+}
+
 // The kernel of a call that leaves it to the library, as dsw_gemm_bf16's bn.  few: the cluster kernel may be taken.
 static int pick_kernel(int M, int N, int K, int mode, bool b_mn, bool derivative, bool few, int sms, int* split) {
   double cost;
@@ -269,6 +283,22 @@ extern "C" int dsw_gemm_bf16(const void* A, long long lda, int a_mn_major, const
     const bool few = split_k == 1 && mode <= EPI_MUL && !a_mn_major && max_ctas == 0 && default_max_ctas() == 0;
     bn = pick_kernel(M, N, K, mode, b_mn_major != 0, aux_out != nullptr, few, num_sms[dev], &split_k);
     few_rows = bn > 1000;
+    if (few_rows && narrow_fits(M, N, K, split_k, num_sms[dev]) && (mode != EPI_MUL || tl_launch.colsum == nullptr) && !(reinterpret_cast<uintptr_t>(bias) & 15)) {
+      GemmArgs g = {};
+      g.M = M; g.N = N; g.K = K;
+      g.b_mn_major = b_mn_major; g.mode = mode; g.split_k = split_k;
+      g.out = out; g.ldo = ldo; g.bias = bias;
+      g.resid = reinterpret_cast<const __nv_bfloat16*>(resid); g.ldr = ldr;
+      g.aux_out = reinterpret_cast<__nv_bfloat16*>(aux_out);
+      g.aux_in = reinterpret_cast<const __nv_bfloat16*>(aux_in); g.ldaux = ldaux;
+      g.status = status;
+      g.b_static = tl_launch.static_b;
+      NarrowArgs n = {};
+      n.a = static_cast<const __nv_bfloat16*>(A); n.lda = lda;
+      n.w = static_cast<const __nv_bfloat16*>(B); n.ldw = ldb;
+      n.ref_width = bn - 1000;
+      return launch_narrow(g, n, false, stream);
+    }
   }
   if (max_ctas == 0) max_ctas = default_max_ctas();
   CUtensorMap ta, tb;
@@ -301,6 +331,40 @@ extern "C" int dsw_gemm_bf16(const void* A, long long lda, int a_mn_major, const
   if (few_rows) return launch_split(bn - 1000, ta, tb, g, stream);
   if (bn == 512 || bn == 384) return launch_pair(bn == 512 ? 256 : 128, ta, tb, g, num_sms[dev], max_ctas, stream);
   return launch_one_cta(bn, ta, tb, g, num_sms[dev], max_ctas, stream);
+}
+
+// Whether dsw_layernorm_gemm takes a call: the product would go to gemm_narrow.cuh, unsplit, and a row is one of a narrow model.
+extern "C" int dsw_layernorm_gemm_fits(int M, int N, int K, int mode, int derivative, int sms) {
+  if (M <= 0 || N <= 0 || K <= 0 || N % 8 || K > 128 || sms <= 0 || (mode != EPI_STORE && mode != EPI_GELU) || default_max_ctas() != 0) return 0;
+  int split = 1;
+  return pick_kernel(M, N, K, mode, false, derivative != 0, true, sms, &split) > 1000 && split == 1 && narrow_fits(M, N, K, 1, sms);
+}
+
+extern "C" int dsw_layernorm_gemm(const void* x, const void* x_lo, const float* gamma, const float* beta, void* ln_out, float* mean,
+                                  float* rstd, float eps, const void* W, const float* bias, void* out, int mode, void* aux_out, int M,
+                                  int N, int K, int* status, cudaStream_t stream) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if (K % BK || K > 128 || N % 8) return -10;
+  if (mode != EPI_STORE && mode != EPI_GELU) return -13;
+  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(x_lo) | reinterpret_cast<uintptr_t>(ln_out) |
+       reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(aux_out) |
+       reinterpret_cast<uintptr_t>(gamma) | reinterpret_cast<uintptr_t>(beta) | reinterpret_cast<uintptr_t>(bias)) & 15)
+    return -11;
+  GemmArgs g = {};
+  g.M = M; g.N = N; g.K = K;
+  g.mode = mode; g.split_k = 1;
+  g.out = out; g.ldo = N; g.bias = bias;
+  g.aux_out = static_cast<__nv_bfloat16*>(aux_out); g.ldaux = N;
+  g.status = status;
+  g.b_static = tl_launch.static_b;
+  NarrowArgs n = {};
+  n.a = static_cast<const __nv_bfloat16*>(x); n.lda = K;
+  n.a_lo = static_cast<const __nv_bfloat16*>(x_lo);
+  n.w = static_cast<const __nv_bfloat16*>(W); n.ldw = K;
+  n.ref_width = 32;
+  n.gamma = gamma; n.beta = beta; n.eps = eps;
+  n.ln_out = static_cast<__nv_bfloat16*>(ln_out); n.mean_out = mean; n.rstd_out = rstd;
+  return launch_narrow(g, n, true, stream);
 }
 
 // Logits = A [M,K] W[N,K]^T (both row-major bf16) that are not stored: one of the LM head's two epilogues on 256-wide tiles.

@@ -389,17 +389,33 @@ struct Run {
     return dsw_layernorm_bwd(nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, dw, db, dres_sum, sums, M, s.d, side());
   }
 
+  // LayerNorm and the product behind it in one launch (few rows of a narrow model); its rows are written where a backward follows
+  int normed(const bf16* x, const bf16* x_lo, const float* gamma, const float* beta, bf16* ln, float* mu, float* rs, bool keep,
+             const Block& b, int which, int n_out, bf16* out, int mode, bf16* aux_out) const {
+    return dsw_layernorm_gemm(x, x_lo, gamma, beta, keep ? ln : nullptr, keep ? mu : nullptr, keep ? rs : nullptr, 1e-5f, b.w[which],
+                              b.b[which], out, mode, aux_out, M, n_out, s.d, s.status, st);
+  }
+
   // x_lo: the low part of x (or null); precise: keep the low parts of the residual stream
   int block_fwd(const Block& b, const bf16* x, const bf16* x_lo, bool precise, const Saved& v, bf16* out) const {
     const int d = s.d;
+    const bool keep = v.h != nullptr;          // for a backward
     bf16* x1_lo = precise ? v.x1_lo : nullptr;
-    LAUNCH(dsw_layernorm_fwd_lo(x, x_lo, b.ln1_w, b.ln1_b, v.ln1, v.mu1, v.rs1, M, d, 1e-5f, st));
-    LAUNCH(gemm(v.ln1, b.w[W_QKV], true, 3 * d, d, v.qkv, DSW_EPI_STORE, b.b[W_QKV], nullptr, nullptr, nullptr, M));
+    if (dsw_layernorm_gemm_fits(M, 3 * d, d, DSW_EPI_STORE, 0, s.sms)) {
+      LAUNCH(normed(x, x_lo, b.ln1_w, b.ln1_b, v.ln1, v.mu1, v.rs1, keep, b, W_QKV, 3 * d, v.qkv, DSW_EPI_STORE, nullptr));
+    } else {
+      LAUNCH(dsw_layernorm_fwd_lo(x, x_lo, b.ln1_w, b.ln1_b, v.ln1, v.mu1, v.rs1, M, d, 1e-5f, st));
+      LAUNCH(gemm(v.ln1, b.w[W_QKV], true, 3 * d, d, v.qkv, DSW_EPI_STORE, b.b[W_QKV], nullptr, nullptr, nullptr, M));
+    }
     LAUNCH(dsw_attention_fwd(v.qkv, v.att, v.lse, B, T, s.nh, d / s.nh, scale(), s.status, st));
     LAUNCH(gemm(v.att, b.w[W_O], true, d, d, v.x1, DSW_EPI_RESID, b.b[W_O], x, x1_lo, x_lo, M));
-    LAUNCH(dsw_layernorm_fwd_lo(v.x1, x1_lo, b.ln2_w, b.ln2_b, v.ln2, v.mu2, v.rs2, M, d, 1e-5f, st));
     // the GELU epilogue also emits gelu'(pre-activation) when there is a backward, which then only multiplies by it
-    LAUNCH(gemm(v.ln2, b.w[W_FC], true, 4 * d, d, v.g, DSW_EPI_GELU, b.b[W_FC], nullptr, v.h, nullptr, M));
+    if (dsw_layernorm_gemm_fits(M, 4 * d, d, DSW_EPI_GELU, v.h != nullptr, s.sms)) {
+      LAUNCH(normed(v.x1, x1_lo, b.ln2_w, b.ln2_b, v.ln2, v.mu2, v.rs2, keep, b, W_FC, 4 * d, v.g, DSW_EPI_GELU, v.h));
+    } else {
+      LAUNCH(dsw_layernorm_fwd_lo(v.x1, x1_lo, b.ln2_w, b.ln2_b, v.ln2, v.mu2, v.rs2, M, d, 1e-5f, st));
+      LAUNCH(gemm(v.ln2, b.w[W_FC], true, 4 * d, d, v.g, DSW_EPI_GELU, b.b[W_FC], nullptr, v.h, nullptr, M));
+    }
     LAUNCH(gemm(v.g, b.w[W_PR], true, d, 4 * d, out, DSW_EPI_RESID, b.b[W_PR], v.x1, precise ? v.out_lo : nullptr, x1_lo, M));
     return 0;
   }

@@ -43,6 +43,9 @@ _SIGS = {
     "dsw_head_rows": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_void_p, c_int, c_int, c_void_p,
                       c_void_p],
     "dsw_head_dlogits": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p],
+    "dsw_layernorm_gemm_fits": [c_int, c_int, c_int, c_int, c_int, c_int],
+    "dsw_layernorm_gemm": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_void_p, c_void_p,
+                           c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p],
     "dsw_head_slices": [c_int, c_int, c_int, c_int],
     "dsw_head_softmax": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     "dsw_head_join": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_void_p, c_void_p,

@@ -119,6 +119,14 @@ int dsw_head_rows(const float* parts, const float* tlogit, const long long*, con
 int dsw_head_dlogits(const void* A, const void*, const void* rows, void* out, int M, int N, int K, int*, cudaStream_t st) {
   return op("head_dlogits", st, {{'r', A, 2LL * M * K}, {'r', rows, 16LL * M}, {'w', out, 2LL * M * N}});
 }
+static int g_normed = 0;
+void fake_set_normed(int on) { g_normed = on; }
+int dsw_layernorm_gemm_fits(int, int, int, int, int, int) { return g_normed; }
+int dsw_layernorm_gemm(const void* x, const void* lo, const float*, const float*, void* ln, float* mean, float* rstd, float, const void* W,
+                       const float*, void* out, int, void* aux_out, int M, int N, int K, int*, cudaStream_t st) {
+  return op("layernorm_gemm", st, {{'r', x, 2LL * M * K}, {'r', lo, 2LL * M * K}, {'r', W, 2LL * N * K}, {'w', ln, 2LL * M * K}, {'w', mean, 4LL * M},
+                                   {'w', rstd, 4LL * M}, {'w', out, 2LL * M * N}, {'w', aux_out, 2LL * M * N}});
+}
 static int g_slices = 0;
 void fake_set_slices(int n) { g_slices = n; }
 int dsw_head_slices(int, int, int, int) { return g_slices; }

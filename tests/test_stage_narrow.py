@@ -1,5 +1,5 @@
-"""The executor's narrow head (no stored logits, both gradients from head_flash.cu) on the emulated device: the order of all
-accesses, in one piece and in slices, queued, replayed and by turns with passes of other sizes."""
+"""Routes of narrow models through the executor, on the emulated device: the head without logits (head_flash.cu), in one piece and
+in slices, and LayerNorm in one launch with the product behind it; queued, replayed and by turns with passes of other sizes."""
 import pytest
 
 from stage_device import FakeStage
@@ -20,3 +20,16 @@ def test_order_of_a_narrow_head(device, chunks, slices):  # noqa: F811
         assert "replay" in device.counts
     finally:
         device.lib.fake_set_slices(0)
+
+
+def test_order_with_layernorm_in_the_products(device):  # noqa: F811
+    device.lib.fake_set_normed(1)
+    try:
+        s = FakeStage(device.lib, n=3)
+        rcs = [s.train((2 + i % 2) * AREA, 5 * AREA, *((1, 100), (2, 50))[i % 3 == 1], 1) for i in range(7)]
+        rcs += [s.forward(8 * AREA, 5, 24, 1, keep=0, logits=9 * AREA) for _ in range(3)]
+        ordered(device, *rcs)
+        assert device.names.count("layernorm_gemm") == 10 * 2 * 3          # two a block
+        assert device.names.count("layernorm_fwd") == 10                    # the final one
+    finally:
+        device.lib.fake_set_normed(0)
