@@ -1,0 +1,125 @@
+// Weight gradients of a transformer block for few tokens, all four in one launch: dW [n_out, n_in] += dy^T x, 64 x 64 tiles on
+// mma.sync, both operands of a tile (every token) in shared memory at once.
+//
+// With a hundred tokens such a product is a few microseconds of launch, tensor memory and TMA latency for some 30 ns of
+// arithmetic, and a block has four of them, two bias sums and the joining of two LayerNorms' sums: eight launches one after
+// the other on the side stream took longer (34 us at width 128) than the chain that they run beside (27).  The sums are the
+// other launch (dsw_block_sums, elementwise.cu).  The four products of a block, us: width 128, 128 tokens 22.8 -> 3.3; width 768
+// 26.8 -> 15.1 (28 MB of gradients read and written: 9); where the line lies stands beside few_tokens in stage.cu.
+#include "attention_short.cuh"
+#include "dswarm.h"
+
+namespace dsw {
+
+constexpr int BG_TILE = 64, BG_THREADS = 128, BG_MAX_PARTS = 4;
+constexpr int BG_MAX_TOKENS = 256;
+
+struct BlockGradArgs {
+  const __nv_bfloat16 *dy[BG_MAX_PARTS], *x[BG_MAX_PARTS];
+  float* dw[BG_MAX_PARTS];
+  int n_out[BG_MAX_PARTS], n_in[BG_MAX_PARTS], first[BG_MAX_PARTS + 1];          // first tile of each
+  int tokens;
+};
+
+__global__ void __launch_bounds__(BG_THREADS)
+block_wgrad_kernel(BlockGradArgs g) {
+  extern __shared__ __align__(128) uint8_t bg_smem[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int part = 0;
+#pragma unroll
+  for (int i = 1; i < BG_MAX_PARTS; ++i) part += int(blockIdx.x) >= g.first[i];
+  const int tile = blockIdx.x - g.first[part], n_out = g.n_out[part], n_in = g.n_in[part], tiles_in = (n_in + BG_TILE - 1) / BG_TILE;
+  const int to = tile / tiles_in, o0 = to * BG_TILE, i0 = (tile - to * tiles_in) * BG_TILE;
+  const int steps = (g.tokens + 15) >> 4, rows = steps * 16;          // rows past the last token are zeros
+  uint8_t *sy = bg_smem, *sx = bg_smem + rows * 128;
+  const auto offset = [](int row, int chunk) { return row * 128 + ((chunk ^ (row & 7)) << 4); };
+  pdl_wait();
+  pdl_launch();
+  {
+    const int ch = threadIdx.x & 7;
+    const bool in_o = o0 + ch * 8 < n_out, in_i = i0 + ch * 8 < n_in;
+    const __nv_bfloat16 *py = g.dy[part] + (in_o ? o0 + ch * 8 : 0), *px = g.x[part] + (in_i ? i0 + ch * 8 : 0);
+    for (int r = threadIdx.x >> 3; r < rows; r += BG_THREADS / 8) {
+      const bool in = r < g.tokens;
+      cp_async16(sy + offset(r, ch), py + (in ? (long long)r * n_out : 0), in && in_o);
+      cp_async16(sx + offset(r, ch), px + (in ? (long long)r * n_in : 0), in && in_i);
+    }
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+  // warp = 32 x 32 of the tile
+  const int wo = (warp & 1) * 32, wi = (warp >> 1) * 32;
+  const uint32_t ay = smem_u32(sy), ax = smem_u32(sx);
+  float c[2][4][4];
+#pragma unroll
+  for (int m = 0; m < 2; ++m)
+#pragma unroll
+    for (int n = 0; n < 4; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) c[m][n][e] = 0.f;
+#pragma unroll 2
+  for (int k = 0; k < steps; ++k) {
+    uint32_t a[2][4], b[2][4];
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+      ldmatrix4_trans(a[m], ay + offset(k * 16 + (lane & 7) + ((lane >> 4) << 3), (wo >> 3) + m * 2 + ((lane >> 3) & 1)));
+#pragma unroll
+    for (int n = 0; n < 2; ++n) ldmatrix4_trans(b[n], ax + offset(k * 16 + (lane & 15), (wi >> 3) + n * 2 + (lane >> 4)));
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+      for (int n = 0; n < 4; ++n) mma_bf16(c[m][n], a[m], b[n >> 1][(n & 1) * 2], b[n >> 1][(n & 1) * 2 + 1]);
+  }
+  // one addition to every element: their order is nobody's
+  float* dw = g.dw[part];
+#pragma unroll
+  for (int m = 0; m < 2; ++m)
+#pragma unroll
+    for (int n = 0; n < 4; ++n)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int o = o0 + wo + m * 16 + (lane >> 2) + h * 8, i = i0 + wi + n * 8 + (lane & 3) * 2;
+        if (o < n_out && i < n_in)
+          asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(dw + (long long)o * n_in + i), "f"(c[m][n][2 * h]), "f"(c[m][n][2 * h + 1])
+                       : "memory");
+      }
+}
+
+}  // namespace dsw
+
+using namespace dsw;
+
+extern "C" int dsw_block_wgrads(const void* const* dy, const void* const* x, float* const* dw, const int* n_out, const int* n_in, int count,
+                                int M, cudaStream_t st) {
+  if (M <= 0 || count <= 0) return 0;
+  if (M > BG_MAX_TOKENS || count > BG_MAX_PARTS) return -10;
+  BlockGradArgs g = {};
+  int tiles = 0;
+  for (int i = 0; i < BG_MAX_PARTS; ++i) {
+    g.first[i] = tiles;
+    if (i >= count) continue;
+    if (n_out[i] <= 0 || n_in[i] <= 0 || n_out[i] % 8 || n_in[i] % 8) return -10;
+    if ((reinterpret_cast<uintptr_t>(dy[i]) | reinterpret_cast<uintptr_t>(x[i]) | reinterpret_cast<uintptr_t>(dw[i])) & 15) return -11;
+    g.dy[i] = static_cast<const __nv_bfloat16*>(dy[i]);
+    g.x[i] = static_cast<const __nv_bfloat16*>(x[i]);
+    g.dw[i] = dw[i];
+    g.n_out[i] = n_out[i];
+    g.n_in[i] = n_in[i];
+    tiles += ((n_out[i] + BG_TILE - 1) / BG_TILE) * ((n_in[i] + BG_TILE - 1) / BG_TILE);
+  }
+  g.first[BG_MAX_PARTS] = tiles;
+  g.tokens = M;
+  static bool attr_set[64] = {false};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -2;
+  if (!attr_set[dev]) {
+    if (cudaFuncSetAttribute(block_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BG_MAX_TOKENS * 256) != cudaSuccess) return -2;
+    attr_set[dev] = true;
+  }
+  return launch(block_wgrad_kernel, tiles, BG_THREADS, (M + 15) / 16 * 16 * 256, st, 1, g) == cudaSuccess ? 0 : -3;
+}
+
+extern "C" int dsw_load_block_grads() {
+  cudaFuncAttributes a;
+  return cudaFuncGetAttributes(&a, block_wgrad_kernel) != cudaSuccess ? -1 : 0;
+}

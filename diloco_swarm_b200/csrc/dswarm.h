@@ -56,6 +56,15 @@ int dsw_layernorm_gemm_fits(int M, int N, int K, int mode, int derivative, int s
 int dsw_layernorm_gemm(const void* x, const void* x_lo, const float* gamma, const float* beta, void* ln_out, float* mean, float* rstd,
                        float eps, const void* W, const float* bias, void* out, int mode, void* aux_out, int M, int N, int K, int* status,
                        cudaStream_t stream);
+// Few tokens (M <= 256): up to four weight gradients dw[i] (fp32 [n_out[i], n_in[i]]) += dy[i]^T x[i] (bf16 [M, n_out[i]], [M, n_in[i]])
+// in one launch, one addition to every element (block_grads.cu); and, with the results of the calls by themselves (elementwise.cu),
+// the column sums of two arrays (dsw_colsum_accum, M < 256) and the joining of two LayerNorm backwards' sums (dsw_layernorm_bwd
+// without dx) in another.
+int dsw_block_wgrads(const void* const* dy, const void* const* x, float* const* dw, const int* n_out, const int* n_in, int count, int M,
+                     cudaStream_t st);
+int dsw_block_sums(const void* a, int na, float* sum_a, const void* b, int nb, float* sum_b, const float* ln_a, float* dgamma_a,
+                   float* dbeta_a, float* dres_a, const float* ln_b, float* dgamma_b, float* dbeta_b, float* dres_b, int M, int d,
+                   cudaStream_t st);
 // Masked cross-entropy of logits = A [M,K] W[N,K]^T in pieces that never hold the logits: dsw_head_lse writes partial
 // log-sum-exps (fp32 [ceil(N / 64)][M]) and the target's logit (fp32 [M]), dsw_head_rows (elementwise.cu) joins them into
 // the loss and one 16-byte record per row, dsw_head_dlogits computes the logits again and stores scale / count *
@@ -240,6 +249,7 @@ int dsw_bounds_selftest(cudaStream_t st);
 // Load every kernel of a source file on the current device now, so that no first launch has to wait for
 // the device to go idle while a pipeline receive is spinning on it.
 int dsw_load_gemm();
+int dsw_load_block_grads();
 int dsw_load_head_flash();
 int dsw_load_attention();
 int dsw_load_elementwise();

@@ -475,6 +475,48 @@ colsum_kernel(const __nv_bfloat16* x, long long ld, float* __restrict__ out, int
   if (c < N) atomicAdd(&out[c], s);
 }
 
+// Few rows: what dsw_colsum_accum adds for two arrays and layernorm_bwd_finish_kernel for two LayerNorms, in one launch.  The
+// same orders of addition: a block to 256 columns; a thread to a column of a LayerNorm's sums, which adds up its partial sums as
+// those 32 threads and the one that joins them would.  Four launches of 2 to 3 us each before, on a stream where they followed
+// one another.
+struct BlockSums {
+  const __nv_bfloat16* x[2];
+  int n[2];
+  float* sum[2];
+  const float* ln[2];
+  float* out[6];
+  int M, d, ln_blocks;
+};
+__global__ void __launch_bounds__(256)
+block_sums_kernel(BlockSums g) {
+  pdl_wait();
+  pdl_launch();
+  int blk = blockIdx.x;
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int blocks = (g.n[i] + 255) / 256;
+    if (blk >= 0 && blk < blocks) {
+      const float s = colsum_block(g.x[i], g.n[i], g.M, g.n[i], blk * 256, 0, 1);
+      const int c = blk * 256 + threadIdx.x;
+      if (c < g.n[i]) atomicAdd(&g.sum[i][c], s);
+    }
+    blk -= blocks;
+  }
+  if (blk < 0) return;
+  const int per = (3 * g.d + 255) / 256, which_ln = blk >= per, i = (blk - which_ln * per) * 256 + threadIdx.x;
+  if (i >= 3 * g.d) return;
+  const float* p = g.ln[which_ln] + i;
+  float t = 0.f;
+  for (int y = 0; y < 32 && y < g.ln_blocks; ++y) {
+    float s = 0.f;
+    for (int b = y; b < g.ln_blocks; b += 32) s += p[(long long)b * 3 * g.d];
+    t += s;
+  }
+  const int which = i / g.d, c = i - which * g.d;
+  float* dst = g.out[which_ln * 3 + which];
+  if (dst) atomicAdd(dst + c, t);
+}
+
 // The same with one order of additions at any number of rows: the eight blocks of a cluster share 256 columns, their sums
 // meet in the first one's shared memory, and it adds them up.  For deterministic gradients: eight blocks per
 // 256 columns do not fill the GPU (32768 x 3072: 135 us, with atomics 33).
@@ -942,6 +984,23 @@ extern "C" int dsw_layernorm_bwd(const void* dy, const void* x, const float* gam
              : -3;
 }
 
+extern "C" int dsw_block_sums(const void* a, int na, float* sum_a, const void* b, int nb, float* sum_b, const float* ln_a, float* dgamma_a,
+                              float* dbeta_a, float* dres_a, const float* ln_b, float* dgamma_b, float* dbeta_b, float* dres_b, int M, int d,
+                              cudaStream_t st) {
+  if (M <= 0) return 0;
+  if (M >= COLSUM_ORDERED_ROWS || na <= 0 || nb <= 0 || na % 8 || nb % 8 || d <= 0 || d % 8 || d > 256 * LN_MAX_CHUNKS_ALL) return -10;
+  BlockSums g = {};
+  g.x[0] = (const bf16*)a; g.x[1] = (const bf16*)b;
+  g.n[0] = na; g.n[1] = nb;
+  g.sum[0] = sum_a; g.sum[1] = sum_b;
+  g.ln[0] = ln_a; g.ln[1] = ln_b;
+  float* const out[6] = {dgamma_a, dbeta_a, dres_a, dgamma_b, dbeta_b, dres_b};
+  for (int i = 0; i < 6; ++i) g.out[i] = out[i];
+  g.M = M; g.d = d; g.ln_blocks = ln_bwd_grid(M, d);
+  const int cols = (na + 255) / 256 + (nb + 255) / 256;
+  return launch(block_sums_kernel, cols + 2 * ((3 * d + 255) / 256), 256, 0, st, 1, g) == cudaSuccess ? 0 : -3;
+}
+
 extern "C" int dsw_colsum_accum(const void* x, long long ld, float* out, int M, int N, cudaStream_t st) {
   if (N % 8 || ld % 8) return -10;
   dim3 grid((N + 255) / 256, M >= 4096 ? 128 : (M >= COLSUM_ORDERED_ROWS ? 16 : 1));
@@ -1071,7 +1130,7 @@ extern "C" int dsw_load_elementwise() {
   L((layernorm_fwd_kernel<5, false, 32>)); L((layernorm_fwd_kernel<5, true, 32>)); L((layernorm_fwd_kernel<6, false, 32>)); L((layernorm_fwd_kernel<6, true, 32>)); L((layernorm_fwd_kernel<7, false, 32>)); L((layernorm_fwd_kernel<7, true, 32>)); L((layernorm_fwd_kernel<8, false, 32>)); L((layernorm_fwd_kernel<8, true, 32>));
   L(layernorm_bwd_kernel<1>); L(layernorm_bwd_kernel<2>); L(layernorm_bwd_kernel<3>); L(layernorm_bwd_kernel<4>);
   L(layernorm_bwd_kernel<5>); L(layernorm_bwd_kernel<6>); L(layernorm_bwd_kernel<7>); L(layernorm_bwd_kernel<8>); L(layernorm_bwd_narrow_kernel);
-  L(layernorm_bwd_finish_kernel); L(colsum_kernel); L(colsum_ordered_kernel); L(embedding_fwd_kernel); L(embedding_bwd_kernel);
+  L(layernorm_bwd_finish_kernel); L(block_sums_kernel); L(colsum_kernel); L(colsum_ordered_kernel); L(embedding_fwd_kernel); L(embedding_bwd_kernel);
   L(embedding_bwd_sorted_kernel); L(embedding_bwd_pos_kernel);
   L(mask_count_kernel); L(loss_begin_kernel); L(cross_entropy_kernel); L(head_rows_kernel); L(sum_partials_kernel); L(cast_f32_bf16_kernel); L(cast_bf16_f32_kernel);
 #undef L

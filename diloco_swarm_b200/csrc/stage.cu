@@ -13,7 +13,8 @@
 //
 // Streams.  Weight-gradient GEMMs, the joining of LayerNorm's column sums and those bias column sums that do not come out of
 // the kernels which write dh and dqkv (few rows, deterministic gradients) feed nothing in the backward, so they go to the
-// stage's side stream (when it has one) and fill the SMs that the dgrad chain leaves idle.  The buffers they read (dh, dx1,
+// stage's side stream (when it has one) and fill the SMs that the dgrad chain leaves idle; with few tokens (few_tokens) those of
+// a block together, at its end.  The buffers they read (dh, dx1,
 // dqkv, LayerNorm's sums) are doubled by block parity: before a block overwrites a set the main stream waits for the side
 // work of the block two up, which is long done.  A block's outgoing gradient is read by the side work of the block below it,
 // so those buffers form a ring of three.  What both streams, or two passes, add to is added to atomically.
@@ -270,6 +271,12 @@ Scratch take_scratch(Area& a, const Stage& s, size_t M, bool grad, size_t logit_
   return v;
 }
 
+// Whether a block's weight gradients, bias sums and LayerNorm sums are two launches (dsw_block_wgrads, dsw_block_sums) instead of
+// eight.  us for all of them one after the other, eight / two: width 128, 16 tokens 28.4 / 4.8, 128 31.8 / 6.6, 255 35.3 / 8.5; width
+// 768, 16 33.3 / 16.8, 128 36.1 / 21.0, 255 41.3 / 31.2; width 1024, 255 47.0 / 44.0; width 1600, 128 72.3 / 60.3, 200 82.8 / 80.3,
+// 255 85.3 / 98.7.
+bool few_tokens(int M, int d) { return M < dsw::COLSUM_ORDERED_ROWS && (d <= 1024 || M <= 128); }
+
 size_t head_rows(size_t M, int chunks) {
   if (chunks <= 1) return M;
   size_t rows = (M + chunks - 1) / chunks;
@@ -423,31 +430,48 @@ struct Run {
   int block_bwd(int l, const Block& b, const bf16* x, const Saved& v, const Scratch& c, const bf16* dx2, bf16* dx0) {
     const int d = s.d, p = l & 1;
     TRY(wait(marks->done[p]));
+    const bool few = few_tokens(M, d);          // then all side work of the block is two launches at its end
     sum_columns(b.db[W_FC]);
     LAUNCH(gemm(dx2, b.w[W_PR], false, 4 * d, d, c.dh[p], DSW_EPI_MUL, nullptr, nullptr, nullptr, v.h, M));
     const bool sum_dh = columns_unsummed();
-    TRY(fork());
-    SIDE(wgrad(dx2, v.g, d, 4 * d, b.dw[W_PR], M, side()));
-    if (sum_dh) SIDE(colsum(c.dh[p], 4 * d, b.db[W_FC]));
-    SIDE(wgrad(c.dh[p], v.ln2, 4 * d, d, b.dw[W_FC], M, side()));
+    if (!few) {
+      TRY(fork());
+      SIDE(wgrad(dx2, v.g, d, 4 * d, b.dw[W_PR], M, side()));
+      if (sum_dh) SIDE(colsum(c.dh[p], 4 * d, b.db[W_FC]));
+      SIDE(wgrad(c.dh[p], v.ln2, 4 * d, d, b.dw[W_FC], M, side()));
+    }
     LAUNCH(gemm(c.dh[p], b.w[W_FC], false, d, 4 * d, c.dln, DSW_EPI_STORE, nullptr, nullptr, nullptr, nullptr, M));
     // the column sum of dx2 (bias gradient of the MLP's second projection) comes out of the LayerNorm backward as well
     LAUNCH(ln_rows(c.dln, v.x1, b.ln2_w, v.mu2, v.rs2, dx2, c.dx1[p], c.ln[2 * p]));
     LAUNCH(gemm(c.dx1[p], b.w[W_O], false, d, d, c.datt, DSW_EPI_STORE, nullptr, nullptr, nullptr, nullptr, M));
-    TRY(fork());
-    SIDE(ln_sums(c.ln[2 * p], b.dln2_w, b.dln2_b, b.db[W_PR]));
-    SIDE(wgrad(c.dx1[p], v.att, d, d, b.dw[W_O], M, side()));
+    if (!few) {
+      TRY(fork());
+      SIDE(ln_sums(c.ln[2 * p], b.dln2_w, b.dln2_b, b.db[W_PR]));
+      SIDE(wgrad(c.dx1[p], v.att, d, d, b.dw[W_O], M, side()));
+    }
     sum_columns(b.db[W_QKV]);
     LAUNCH((deterministic ? dsw_attention_bwd_ordered : dsw_attention_bwd)(v.qkv, v.att, c.datt, v.lse, c.dqkv[p], c.dq_acc, c.dvec, B, T,
                                                                            s.nh, d / s.nh, scale(), s.status, st));
     const bool sum_dqkv = columns_unsummed();
-    TRY(fork());
-    if (sum_dqkv) SIDE(colsum(c.dqkv[p], 3 * d, b.db[W_QKV]));
-    SIDE(wgrad(c.dqkv[p], v.ln1, 3 * d, d, b.dw[W_QKV], M, side()));
+    if (!few) {
+      TRY(fork());
+      if (sum_dqkv) SIDE(colsum(c.dqkv[p], 3 * d, b.db[W_QKV]));
+      SIDE(wgrad(c.dqkv[p], v.ln1, 3 * d, d, b.dw[W_QKV], M, side()));
+    }
     LAUNCH(gemm(c.dqkv[p], b.w[W_QKV], false, d, 3 * d, c.dln, DSW_EPI_STORE, nullptr, nullptr, nullptr, nullptr, M));
     LAUNCH(ln_rows(c.dln, x, b.ln1_w, v.mu1, v.rs1, c.dx1[p], dx0, c.ln[2 * p + 1]));
     TRY(fork());
-    SIDE(ln_sums(c.ln[2 * p + 1], b.dln1_w, b.dln1_b, b.db[W_O]));
+    if (few) {
+      const void* dy[4] = {dx2, c.dh[p], c.dx1[p], c.dqkv[p]};
+      const void* x4[4] = {v.g, v.ln2, v.att, v.ln1};
+      float* dw[4] = {b.dw[W_PR], b.dw[W_FC], b.dw[W_O], b.dw[W_QKV]};
+      const int n_out[4] = {d, 4 * d, d, 3 * d}, n_in[4] = {4 * d, d, d, d};
+      SIDE(dsw_block_wgrads(dy, x4, dw, n_out, n_in, 4, M, side()));
+      SIDE(dsw_block_sums(c.dh[p], 4 * d, b.db[W_FC], c.dqkv[p], 3 * d, b.db[W_QKV], c.ln[2 * p], b.dln2_w, b.dln2_b, b.db[W_PR],
+                          c.ln[2 * p + 1], b.dln1_w, b.dln1_b, b.db[W_O], M, d, side()));
+    } else {
+      SIDE(ln_sums(c.ln[2 * p + 1], b.dln1_w, b.dln1_b, b.db[W_O]));
+    }
     TRY(mark(marks->done[p]));
     return 0;
   }

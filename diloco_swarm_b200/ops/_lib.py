@@ -46,6 +46,9 @@ _SIGS = {
     "dsw_layernorm_gemm_fits": [c_int, c_int, c_int, c_int, c_int, c_int],
     "dsw_layernorm_gemm": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_void_p, c_void_p,
                            c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p],
+    "dsw_block_wgrads": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p],
+    "dsw_block_sums": [c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+                       c_void_p, c_void_p, c_int, c_int, c_void_p],
     "dsw_head_slices": [c_int, c_int, c_int, c_int],
     "dsw_head_softmax": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     "dsw_head_join": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_void_p, c_void_p,
@@ -128,7 +131,7 @@ def load_all_kernels() -> None:
         return
     lib = cuda_lib()
     for name in ("dsw_load_gemm", "dsw_load_elementwise", "dsw_load_optim", "dsw_load_collectives",
-                 "dsw_load_head_flash",
+                 "dsw_load_head_flash", "dsw_load_block_grads",
                  "dsw_load_attention"):
         fn = getattr(lib, name, None)
         if fn is not None:

@@ -192,6 +192,23 @@ int dsw_colsum_accum(const void* x, long long, float* out, int M, int N, cudaStr
 int dsw_colsum_ordered(const void* x, long long, float* out, int M, int N, cudaStream_t st) {
   return op("colsum_ordered", st, {{'r', x, 2LL * M * N}, {'a', out, 4LL * N}});
 }
+int dsw_block_wgrads(const void* const* dy, const void* const* x, float* const* dw, const int* n_out, const int* n_in, int count, int M,
+                     cudaStream_t st) {
+  for (int i = 0; i < count; ++i) {
+    const int rc = op("block_wgrad", st, {{'r', dy[i], 2LL * M * n_out[i]}, {'r', x[i], 2LL * M * n_in[i]}, {'a', dw[i], 4LL * n_out[i] * n_in[i]}});
+    if (rc) return rc;
+  }
+  return 0;
+}
+// one launch, told as the calls that it stands for
+int dsw_block_sums(const void* a, int na, float* sum_a, const void* b, int nb, float* sum_b, const float* ln_a, float* ga, float* ba,
+                   float* ra, const float* ln_b, float* gb, float* bb, float* rb, int M, int d, cudaStream_t st) {
+  int rc = dsw_colsum_accum(a, na, sum_a, M, na, st);
+  if (!rc) rc = dsw_colsum_accum(b, nb, sum_b, M, nb, st);
+  if (!rc) rc = dsw_layernorm_bwd(nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, ga, ba, ra, const_cast<float*>(ln_a), M, d, st);
+  if (!rc) rc = dsw_layernorm_bwd(nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, gb, bb, rb, const_cast<float*>(ln_b), M, d, st);
+  return rc;
+}
 int dsw_embedding_fwd(const long long* ids, const float*, const float*, void* y, int B, int T, int d, int, int*, cudaStream_t st) {
   return op("embedding_fwd", st, {{'r', ids, 8LL * B * T}, {'w', y, 2LL * B * T * d}});
 }
