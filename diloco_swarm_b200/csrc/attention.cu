@@ -8,16 +8,19 @@
 //
 // A work item is (128 query rows, batch, head); persistent CTAs walk the items.
 // Warps 0-3 own one query row per thread: they read the score row from tensor
-// memory once, do the online softmax on it in registers and write P to shared
+// memory once, do the online softmax on it in registers and write P to tensor
 // memory.  The output row stays in tensor memory: every P V product accumulates
 // onto it, and the row threads rescale it in place only when the running maximum
 // has grown by more than 2^8 since the last rescale (until then P is computed
 // against the older maximum, which is exact algebra and safe in bf16/fp32 range).
 // Warp 4 issues the MMAs, warp 5 the TMA loads.
 //   S = Q K_j^T          A = Q  [128 x 64]  K-major,  B = K_j [128 x 64] K-major   -> TMEM, 128 columns
-//   O_j = P V_j          A = P  [128 x 128] K-major (written by the softmax warps
-//                        in the 128-byte-swizzled layout),  B = V_j [128 x 64] N-major -> TMEM, 64 columns
-// K/V tiles are double buffered; two CTAs fit on an SM (112 KB shared memory,
+//   O_j = P V_j          A = P  [128 x 128] in TMEM, 64 columns of bf16 pairs,  B = V_j [128 x 64] N-major -> TMEM, 64 columns
+// P by way of shared memory cost 64 KB of its bandwidth per tile, written and read by the product, of the 144 KB that a tile took
+// (128 bytes per clock; us, before / now: 32 x 1024 tokens, 12 heads of 64, 121.7 / 115.4; 8 x 1024, 16 heads 44.6 / 42.3; 16 x 133,
+// 12 heads 12.6 / 12.1; 64 x 1024, 4 heads of 32, 80.6 / 76.5).  A quarter to a half of the exponentials on the FMA pipe instead: slower
+// by 6 to 20 %, here as in the backward.
+// K/V tiles are double buffered; two CTAs fit on an SM (97 KB shared memory,
 // 256 TMEM columns each), so one CTA's MMAs run under the other's softmax.
 // Only kv tiles up to the diagonal are visited; the diagonal tile is masked.
 //
@@ -67,8 +70,8 @@ struct AttSmem {
   static constexpr int Q_OFF = 0;
   static constexpr int K_OFF = Q_OFF + ATT_TILE_BYTES;            // 2 stages
   static constexpr int V_OFF = K_OFF + 2 * ATT_TILE_BYTES;        // 2 stages
-  static constexpr int P_OFF = V_OFF + 2 * ATT_TILE_BYTES;        // [2 k-blocks][128 rows][64]
-  static constexpr int BAR_OFF = P_OFF + 2 * ATT_TILE_BYTES;
+  static constexpr int O_OFF = V_OFF + 2 * ATT_TILE_BYTES;        // output rows on their way out, [128 rows][64]
+  static constexpr int BAR_OFF = O_OFF + ATT_TILE_BYTES;
   // Two CTAs share an SM only if each stays under (227 KB - 2 KB) / 2 = 115200 bytes, so
   // there is no room for alignment slack: the dynamic segment is declared 1024-aligned
   // and the kernel checks that it really is.
@@ -125,7 +128,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, __nv_bfloat16
   uint64_t* kv_full = bars + 1;       // 2 stages
   uint64_t* kv_empty = bars + 3;      // 2 stages
   uint64_t* s_full = bars + 5;        // S ready in TMEM
-  uint64_t* p_full = bars + 6;        // P written to smem (4 warps arrive)
+  uint64_t* p_full = bars + 6;        // P written to TMEM (4 warps arrive)
   uint64_t* o_full = bars + 7;        // P V accumulated in TMEM
   uint64_t* o_free = bars + 8;        // per item: the output rows have been read out of TMEM (4 warps arrive)
   uint64_t* s_free = bars + 9;        // S read out of TMEM (4 warps arrive)
@@ -165,6 +168,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, __nv_bfloat16
   const uint32_t tmem_base = *tmem_holder;
   const uint32_t tmem_s = tmem_base;            // 128 columns
   const uint32_t tmem_o = tmem_base + 128;      // 64 columns
+  const uint32_t tmem_p = tmem_base + 192;      // 64 columns: P, two bf16 values to a column
 
   if (warp >= 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");          // the whole warpgroup, one instruction
@@ -209,7 +213,6 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, __nv_bfloat16
     const uint32_t idesc_o = make_idesc_bf16(128, 64, 0, 1);
     const uint32_t desc_hi = smem_desc_hi(1024);
     const uint32_t q_lo = smem_desc_lo(smem_u32(smem + AttSmem::Q_OFF), 16);
-    const uint32_t p_lo = smem_desc_lo(smem_u32(smem + AttSmem::P_OFF), 16);
     // S of global tile gt = Q K^T into the (single) score buffer; `first` / `last`: position in its item wi
     auto issue_s = [&](uint32_t gt, uint32_t wi, bool first, bool last) -> bool {
       if (first && !mbar_wait_warp(q_full, wi & 1, abort_flag, status)) return false;
@@ -251,7 +254,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, __nv_bfloat16
           const bool okk = more ? issue_s(g + 1, w, false, j + 2 == n_kv) : issue_s(g + 1, w + 1, true, next_n_kv == 1);
           if (!okk) { ok = false; break; }
         }
-        // P of this tile is in shared memory (and the output rows are rescaled if they had to be)
+        // P of this tile is in tensor memory (and the output rows are rescaled if they had to be)
         if (!mbar_wait_warp(p_full, g & 1, abort_flag, status)) { ok = false; break; }
         ATT_TRACE(tr, 256, tslot);          // P ready
         // a new item starts its output from zero: the previous item's must have been read out
@@ -259,9 +262,8 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, __nv_bfloat16
         tc_fence_after();
         if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < ATT_BK / 16; ++k)          // P: 32 bytes along the row per step, second k-block after 4
-            umma_bf16_lohi(tmem_o, p_lo + (k >> 2) * (ATT_TILE_BYTES >> 4) + (k & 3) * 2, v_lo + k * (2048 >> 4), desc_hi,
-                           idesc_o, (j > 0 || k > 0));
+          for (int k = 0; k < ATT_BK / 16; ++k)
+            umma_bf16_ts(tmem_o, tmem_p + k * 8, v_lo + k * (2048 >> 4), desc_hi, idesc_o, (j > 0 || k > 0));
           umma_commit(o_full);
           umma_commit(&kv_empty[s]);
         }
@@ -275,7 +277,6 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, __nv_bfloat16
     asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
     const int r = warp * 32 + lane;                      // row within the tile = TMEM lane
     const uint32_t lane_addr = uint32_t(warp * 32) << 16;
-    uint8_t* sp = smem + AttSmem::P_OFF;
     if (threadIdx.x != 0) tr = nullptr;
     uint32_t g = 0;
     bool ok = true;
@@ -327,7 +328,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, __nv_bfloat16
         if (j == 0) {
           m = mx;
         } else {
-          // the previous product must be done: it reads the P tile that is about to be overwritten, and it
+          // the previous product must be done: it reads the P that is about to be overwritten, and it
           // accumulates onto the output rows that may be rescaled here
           if (!mbar_wait(o_full, (g - 1) & 1, abort_flag, status)) { ok = false; break; }
           const bool grow = mx > m + 8.f;
@@ -348,7 +349,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, __nv_bfloat16
           }
         }
         ATT_TRACE(tr, 0, tslot);              // output rows ready for the next product
-        // probabilities -> shared memory (bf16, swizzled K-major), row sum
+        // probabilities -> tensor memory (bf16), row sum
         f2 sum2[2] = {f2_bcast(0.f), f2_bcast(0.f)};      // packed pairs (two columns per instruction)
         const f2 sc2 = f2_bcast(scale_log2), nm2 = f2_bcast(-m);
 #pragma unroll
@@ -372,9 +373,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, __nv_bfloat16
 #pragma unroll
             for (int i = 0; i < 16; ++i) pk[i] = 0;
           }
-#pragma unroll
-          for (int i = 0; i < 16; i += 4)
-            *reinterpret_cast<uint4*>(sp + p_offset(r, c * 32 + 2 * i)) = make_uint4(pk[i], pk[i + 1], pk[i + 2], pk[i + 3]);
+          tmem_st_32x16(tmem_p + lane_addr + c * 16, pk);
         }
         {
           float a0, a1;
@@ -382,8 +381,8 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, __nv_bfloat16
           l += a0 + a1;
         }
         ATT_TRACE(tr, 0, tslot);              // P written
-        fence_proxy_async();          // make the generic-proxy writes of P visible to the tensor core
-        tc_fence_before();            // orders the rescaled output rows before the product that follows the arrive
+        tmem_st_wait();
+        tc_fence_before();            // orders P and the rescaled output rows before the product that follows the arrive
         __syncwarp();
         if (lane == 0) mbar_arrive(p_full);
       }
@@ -410,10 +409,10 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, __nv_bfloat16
                                                                 pack_bf16(__uint_as_float(o[6]) * inv, __uint_as_float(o[7]) * inv));
           }
       } else {
-        // The warp's 32 rows pass through its own rows of the P tile, which no product reads any more, so that a store
+        // The warp's 32 rows pass through shared memory, so that a store
         // covers four whole rows of 128 bytes: a lane that stores its own row 16 bytes at a time touches 32 lines with
         // every instruction (32 x 1024 tokens, 12 heads of 64: 135.6 -> 129.0 us; 16 x 1024: 72.9 -> 68.6).
-        uint8_t* so = sp + warp * 32 * 128;
+        uint8_t* so = smem + AttSmem::O_OFF + warp * 32 * 128;
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
           const uint32_t* o = ov[c >> 2] + (c & 3) * 8;
@@ -432,7 +431,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, __nv_bfloat16
           const uint4 w = *reinterpret_cast<const uint4*>(so + rl * 128 + ((ch ^ (rl & 7)) << 4));
           if (t0 + i * 4 < T && ch * 8 < hs) *reinterpret_cast<uint4*>(dst + (long long)i * 4 * d) = w;
         }
-        __syncwarp();                                // read out before the next item's P is written here
+        __syncwarp();                                // read out before the next item's rows are written here
       }
       // natural-log LSE of the scaled scores
       if (in_seq) lse_out[(long long)bh * T + qi * ATT_BQ + r] = (m + log2f(l)) * 0.6931471805599453f;
