@@ -1195,6 +1195,7 @@ extern "C" int dsw_attention_fwd(const void* qkv, void* out, float* lse, int B, 
   if ((hs != 64 && hs != 32) || T <= 0) return -10;
   const int d = nh * hs;
   if (attention_is_short(T, hs, B * nh)) {
+    if (reinterpret_cast<uintptr_t>(qkv) & 15) return -10;          // 16-byte copies; a tensor map refuses it as well
     const float s2 = scale * 1.4426950408889634f;
     return hs == 64 ? attention_short<64>((const __nv_bfloat16*)qkv, (__nv_bfloat16*)out, lse, T, nh, B * nh, s2, st)
                     : attention_short<32>((const __nv_bfloat16*)qkv, (__nv_bfloat16*)out, lse, T, nh, B * nh, s2, st);

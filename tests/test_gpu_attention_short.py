@@ -40,3 +40,12 @@ def test_what_lies_behind_a_sequence_stays_out(T):
     qkv[T:] = float("inf")
     both, _ = attention_fwd(qkv, 2, T, 4)
     assert torch.equal(both[:T], alone)
+
+
+@pytest.mark.parametrize("T", [24, 128, 300])
+def test_an_unaligned_qkv_is_refused(T):
+    """On either side of the rule: its rows are copied 16 bytes at a time."""
+    from diloco_swarm_b200.ops.attention import attention_fwd
+    qkv = torch.zeros(T * 192 + 4, device="cuda", dtype=torch.bfloat16)[4:].view(T, 192)
+    with pytest.raises(RuntimeError):
+        attention_fwd(qkv, 1, T, 1)
