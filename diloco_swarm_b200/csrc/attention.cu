@@ -32,7 +32,7 @@
 #include "ptx.cuh"
 #include "launch.h"
 #include "tmap.h"
-#include "attention_short.cuh"
+#include "attention_short_bwd.cuh"
 #include "dswarm.h"
 
 namespace dsw {
@@ -491,18 +491,6 @@ struct AttBwdSmem {
   static constexpr int ONE_D_OFF = ONE_SUM_OFF + 1024;              // fp32 [2 item parities][128 rows]
   static constexpr int ONE_O_OFF = ONE_D_OFF + 1024;                // [8 row warps][3 pieces][32 lanes] of 16 bytes
 };
-
-// Dot product of eight bf16 values, fp32 sums.
-__device__ __forceinline__ float dot8(const uint4& a, const uint4& g) {
-  const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, gw[4] = {g.x, g.y, g.z, g.w};
-  float v = 0.f;
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const float2 x = unpack_bf16(aw[k]), y = unpack_bf16(gw[k]);
-    v += x.x * y.x + x.y * y.y;
-  }
-  return v;
-}
 
 // D[bh, t] = sum_c dO[t, h*hs + c] * O[t, h*hs + c], and dq_acc[t, :] = 0.  One warp per token row: 16-byte
 // loads, one head's hs columns lie in hs/8 neighbouring lanes (hs = 64 or 32), which a few shuffles add up.
@@ -1185,6 +1173,14 @@ static bool attention_is_short(int T, int hs, int n_bh) {
   if (T > SHORT_MAX_T) return false;
   return hs == 32 || T <= 64 || n_bh <= 2 * att_num_sms() || (T <= 96 && n_bh <= 6 * att_num_sms());
 }
+// Which kernel a backward of up to 128 tokens takes; the bits are the same.  us a launch, tcgen05 / short, n heads of all sequences
+// together.  Heads of 64: T = 16, n 60 7.5 / 2.9, 2400 82.6 / 15.4; T = 64, 60 7.8 / 5.8, 2400 84.2 / 65.2; T = 96, 60 8.0 / 6.7, 148
+// 8.8 / 7.9, 192 13.5 / 14.2, 2400 85.6 / 148; T = 128, 60 8.3 / 8.5, 148 9.1 / 10.0, 600 26.8 / 44.6.  Heads of 32, half the products:
+// T = 128, 4 7.8 / 5.1, 800 32.9 / 22.7.
+static bool attention_bwd_is_short(int T, int hs, int n_bh) {
+  if (T > SHORT_MAX_T) return false;
+  return hs == 32 || T <= 64 || (T <= 96 && n_bh <= att_num_sms());
+}
 // Register (or clear, with nullptr) a device buffer of 512 int64 for the in-kernel timeline.
 extern "C" int dsw_attention_set_trace(long long* buf) { g_att_trace = buf; return 0; }
 
@@ -1226,6 +1222,18 @@ static int attention_bwd(const void* qkv, const void* out, const void* dout, con
   if ((hs != 64 && hs != 32) || T <= 0 || (long long)B * nh * T >= (1LL << 31)) return -10;
   const int d = nh * hs;
   const long long rows = (long long)B * T;
+  if (attention_bwd_is_short(T, hs, B * nh)) {
+    // 16-byte copies, and what the tensor maps of the other kernel refuse
+    if ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(dout) |
+         reinterpret_cast<uintptr_t>(dqkv) | reinterpret_cast<uintptr_t>(dq_acc)) & 15)
+      return -10;
+    const ShortBwdArgs a = {(const __nv_bfloat16*)qkv, (const __nv_bfloat16*)out, (const __nv_bfloat16*)dout, lse, (__nv_bfloat16*)dqkv,
+                            tl_launch.colsum, T, nh, scale};
+    tl_launch.colsum = nullptr;
+    // where an SM is left over for them, dQ has blocks of its own
+    const int parts = B * nh < att_num_sms() ? 2 : 1;
+    return hs == 64 ? attention_short_bwd<64>(a, B * nh, parts, st) : attention_short_bwd<32>(a, B * nh, parts, st);
+  }
   CUtensorMap tq, tdo, tdq, tdkv;
   int rc = cached_tmap(&tq, TMAP_BF16_4D, qkv, hs, 3LL * nh, T, 3LL * d, 64, 128, B);
   if (!rc) rc = cached_tmap(&tdkv, TMAP_BF16_4D, dqkv, hs, 3LL * nh, T, 3LL * d, 64, 128, B);
@@ -1286,6 +1294,7 @@ extern "C" int dsw_load_attention() {
   int bad = 0;
   bad |= cudaFuncGetAttributes(&a, attention_fwd_kernel<true>) != cudaSuccess;
   bad |= load_attention_short();
+  bad |= load_attention_short_bwd();
   bad |= cudaFuncGetAttributes(&a, attention_fwd_kernel<false>) != cudaSuccess;
   bad |= cudaFuncGetAttributes(&a, attention_bwd_kernel<false>) != cudaSuccess;
   bad |= cudaFuncGetAttributes(&a, attention_bwd_kernel<true>) != cudaSuccess;

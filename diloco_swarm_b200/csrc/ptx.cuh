@@ -505,4 +505,16 @@ __device__ __forceinline__ float2 unpack_bf16(uint32_t u) {
   return __bfloat1622float2(v);
 }
 
+// Dot product of eight bf16 values, fp32 sums.
+__device__ __forceinline__ float dot8(const uint4& a, const uint4& g) {
+  const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, gw[4] = {g.x, g.y, g.z, g.w};
+  float v = 0.f;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const float2 x = unpack_bf16(aw[k]), y = unpack_bf16(gw[k]);
+    v += x.x * y.x + x.y * y.y;
+  }
+  return v;
+}
+
 }  // namespace dsw

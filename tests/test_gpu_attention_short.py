@@ -1,6 +1,9 @@
-"""Attention forward of short sequences on mma.sync (csrc/attention_short.cuh): the bits of the tcgen05 kernel, and 64 bits."""
+"""Attention of short sequences on mma.sync (csrc/attention_short.cuh, attention_short_bwd.cuh): the bits of the tcgen05 kernels, and 64 bits."""
 import pytest
 import torch
+
+import test_gpu_attention_one_tile as one_tile
+import test_gpu_column_sums as column_sums
 
 pytestmark = pytest.mark.gpu
 
@@ -49,3 +52,43 @@ def test_an_unaligned_qkv_is_refused(T):
     qkv = torch.zeros(T * 192 + 4, device="cuda", dtype=torch.bfloat16)[4:].view(T, 192)
     with pytest.raises(RuntimeError):
         attention_fwd(qkv, 1, T, 1)
+
+
+# as above, both sides of the rule (T of 64 and 96 for heads of 64); dQ in blocks of its own (fewer heads than SMs) and not
+BACKWARD = [(T, *shape) for T in (1, 15, 16, 17, 31, 32, 33, 64, 65, 96, 97, 127, 128) for shape in ((1, 1, 64), (2, 4, 32), (13, 12, 64), (40, 4, 32))]
+
+
+@pytest.mark.parametrize("T,B,nh,hs", BACKWARD)
+def test_backward_has_the_bits_of_longer_sequences(T, B, nh, hs):
+    one_tile.test_backward_is_that_of_longer_sequences(B, T, nh, hs)
+
+
+@pytest.mark.parametrize("T,B,nh,hs", [(1, 3, 2, 64), (17, 13, 12, 64), (33, 2, 4, 32), (64, 1, 12, 64), (96, 12, 12, 64), (128, 40, 4, 32)])
+def test_backward_against_64_bits(T, B, nh, hs):
+    one_tile.test_backward_against_64_bits(B, T, nh, hs)
+
+
+@pytest.mark.parametrize("B,T", [(300, 1), (16, 16), (9, 31), (30, 17), (6, 64), (3, 96)])
+def test_bias_gradient_of_the_qkv_projection(B, T, monkeypatch):
+    column_sums.test_sums_are_those_of_the_terms(B, T, 12, 768, monkeypatch)
+
+
+@pytest.mark.parametrize("T", [17, 64])
+def test_backward_leaves_out_what_lies_behind_a_sequence(T):
+    from diloco_swarm_b200.ops.attention import attention_bwd, attention_fwd
+    g = torch.Generator(device="cuda").manual_seed(T)
+    qkv = torch.randn(2 * T, 3 * 128, device="cuda", generator=g).to(torch.bfloat16)
+    dout = torch.randn(2 * T, 128, device="cuda", generator=g).to(torch.bfloat16)
+    _, ctx = attention_fwd(qkv[:T].contiguous(), 1, T, 4)
+    alone = attention_bwd(dout[:T].contiguous(), ctx)
+    qkv[T:], dout[T:] = float("inf"), float("nan")
+    _, ctx = attention_fwd(qkv, 2, T, 4)
+    assert torch.equal(attention_bwd(dout, ctx)[:T], alone)
+
+
+@pytest.mark.parametrize("T", [24, 128])
+def test_an_unaligned_gradient_is_refused(T):
+    from diloco_swarm_b200.ops.attention import attention_bwd, attention_fwd
+    _, ctx = attention_fwd(torch.zeros(T, 192, device="cuda", dtype=torch.bfloat16), 1, T, 1)
+    with pytest.raises(RuntimeError):
+        attention_bwd(torch.zeros(T * 64 + 4, device="cuda", dtype=torch.bfloat16)[4:].view(T, 64), ctx)
