@@ -654,12 +654,12 @@ struct ItemDots {
   }
 };
 
-// ONE: sequences of a single tile (T <= 128).  Every item is one step, and dQ needs no sum over kv tiles, so it leaves as
-// bf16 with dK and dV.  D is computed by the row warps, 16 rows each, that of the next item under the products of this one.
-// No accumulator, and neither of the kernels around this one (which clear it and compute D, and convert it).  The results
-// are those of the three kernels, bit for bit: 64 x 128 tokens, 12 heads of 64, 45.7 -> 36.8 us; 16 x 128, 16 heads, 23.9 ->
-// 16.9; 200 x 64, 12 heads, 95.4 -> 84.0; 1 x 128, 4 heads of 32, 11.0 -> 7.6.  (With D as the row sum of P dP, which is
-// another rounding and has the two warps of a row wait for each other inside the row algebra: 33.1, 15.4, 77.0, 7.6.)
+// ONE: sequences of a single tile (T <= 128), heads of 64 (of 32: attention_short_bwd.cuh).  Every item is one step, and dQ
+// needs no sum over kv tiles, so it leaves as bf16 with dK and dV.  D is computed by the row warps, 16 rows each, that of the
+// next item under the products of this one.  No accumulator, and neither of the kernels around this one (which clear it and
+// compute D, and convert it).  The results are those of the three kernels, bit for bit: 64 x 128 tokens, 12 heads of 64,
+// 45.7 -> 36.8 us; 16 x 128, 16 heads, 23.9 -> 16.9; 200 x 64, 12 heads, 95.4 -> 84.0.  (With D as the row sum of P dP, which is
+// another rounding and has the two warps of a row wait for each other inside the row algebra: 33.1, 15.4, 77.0.)
 template <bool ONE>
 __global__ void __launch_bounds__(ATT_BWD_THREADS, 1)
 attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_constant__ CUtensorMap tmap_do,
@@ -987,15 +987,13 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
       if (lane == 0) mbar_arrive(dots_full);
     };
     const auto dots_fetch = [&](int bh) {
-      if (hs == 64) ItemDots<8>::fetch(out + dots_at(bh), d, T - dot_row, o_mine, o_last, lane);
-      else          ItemDots<4>::fetch(out + dots_at(bh), d, T - dot_row, o_mine, o_last, lane);
+      ItemDots<8>::fetch(out + dots_at(bh), d, T - dot_row, o_mine, o_last, lane);
     };
     const auto dots_finish = [&](uint32_t item) -> bool {
       const int s = item % L::QSTAGES;
       if (!mbar_wait(&q_full[s], (item / L::QSTAGES) & 1, abort_flag, status)) return false;
       const uint8_t* tile = smem + L::DO_OFF + s * ATT_TILE_BYTES;
-      if (hs == 64) ItemDots<8>::finish(tile, dot_row, o_mine, o_last, dots_to(item), lane);
-      else          ItemDots<4>::finish(tile, dot_row, o_mine, o_last, dots_to(item), lane);
+      ItemDots<8>::finish(tile, dot_row, o_mine, o_last, dots_to(item), lane);
       dots_done();
       return true;
     };
@@ -1003,8 +1001,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
       int idx;
       next_item(0, idx);          // there is one: G <= total
       const long long at = dots_at(idx % n_bh);
-      if (hs == 64) ItemDots<8>::first(out + at, dout + at, d, T - dot_row, dots_to(0), lane);
-      else          ItemDots<4>::first(out + at, dout + at, d, T - dot_row, dots_to(0), lane);
+      ItemDots<8>::first(out + at, dout + at, d, T - dot_row, dots_to(0), lane);
       dots_done();
     }
     for (int rr = 0; rr < rounds && ok; ++rr) {
@@ -1173,13 +1170,21 @@ static bool attention_is_short(int T, int hs, int n_bh) {
   if (T > SHORT_MAX_T) return false;
   return hs == 32 || T <= 64 || n_bh <= 2 * att_num_sms() || (T <= 96 && n_bh <= 6 * att_num_sms());
 }
-// Which kernel a backward of up to 128 tokens takes; the bits are the same.  us a launch, tcgen05 / short, n heads of all sequences
-// together.  Heads of 64: T = 16, n 60 7.5 / 2.9, 2400 82.6 / 15.4; T = 64, 60 7.8 / 5.8, 2400 84.2 / 65.2; T = 96, 60 8.0 / 6.7, 148
-// 8.8 / 7.9, 192 13.5 / 14.2, 2400 85.6 / 148; T = 128, 60 8.3 / 8.5, 148 9.1 / 10.0, 600 26.8 / 44.6.  Heads of 32, half the products:
-// T = 128, 4 7.8 / 5.1, 800 32.9 / 22.7.
-static bool attention_bwd_is_short(int T, int hs, int n_bh) {
-  if (T > SHORT_MAX_T) return false;
-  return hs == 32 || T <= 64 || (T <= 96 && n_bh <= att_num_sms());
+// Which kernel a backward takes, and on how many blocks and warps if it is the one for short sequences; the bits are the same.
+// us a launch, tcgen05 / short, n heads of all sequences together.  Heads of 64: T = 16, n 60 7.8 / 3.7, 768 32.8 / 6.0; T = 64, 60 8.0 /
+// 5.3, 192 13.4 / 9.2, 768 33.0 / 21.3; T = 96, 192 13.5 / 13.1, 768 33.3 / 38.6; T = 128, 60 8.5 / 7.6, 148 9.2 / 9.6.  Where the two are
+// close the rest of a pass decides, with weight gradients on the SMs beside it: forward and backward of 12 blocks, 1 x 128 tokens
+// 1193 / 1203, 4 x 100 1464 / 1486, 12 x 192 2780 / 2842 (kernel alone, its three kernels against one, 20.3 / 17.8), 64 x 50 3681 / 3560,
+// 64 x 16 2320 / 1996.  Heads of 32, half the products: T = 128, n 4 8.0 / 4.8, 800 32.8 / 24.7; T = 192, 4 12.6 / 6.7, 800 74.6 / 48.3; three
+// blocks, 1 x 160 257 / 235, 64 x 190 1071 / 1026, 8 x 256 432 / 445.
+// A second block for a head where it finds an SM of its own: T = 128, n 4 5.4 -> 4.8.
+static ShortBwdPlan attention_bwd_plan(int T, int hs, int n_bh) {
+  const int sms = att_num_sms(), blocks = (T + 15) / 16;
+  if (T > (hs == 32 ? SHORT_BWD_MAX_T : 64)) return {0, 0, false};
+  if (T > 128) return n_bh <= sms ? ShortBwdPlan{2, blocks, true} : ShortBwdPlan{1, (blocks + 1) / 2, true};
+  if (n_bh > sms) return {1, T <= 32 ? 2 * blocks : blocks, true};
+  if (T <= 64) return {1, 2 * blocks, false};
+  return {2 * n_bh <= sms ? 2 : 1, blocks, false};
 }
 // Register (or clear, with nullptr) a device buffer of 512 int64 for the in-kernel timeline.
 extern "C" int dsw_attention_set_trace(long long* buf) { g_att_trace = buf; return 0; }
@@ -1214,7 +1219,7 @@ extern "C" int dsw_attention_fwd(const void* qkv, void* out, float* lse, int B, 
 }
 
 // qkv, out, dout as in the forward; lse from the forward.  dqkv: bf16 [B*T, 3*d] (all of it is written).
-// dq_acc: fp32 scratch [B*T, d]; Dvec: fp32 scratch [B*nh*T].  Both are overwritten where T > 128.
+// dq_acc: fp32 scratch [B*T, d]; Dvec: fp32 scratch [B*nh*T].  Both may be overwritten.
 // ordered: the kv tiles' contributions to dQ, which otherwise meet in whatever order their CTAs get there, are added tile
 // by tile, one launch each.
 static int attention_bwd(const void* qkv, const void* out, const void* dout, const float* lse, void* dqkv, float* dq_acc, float* Dvec,
@@ -1222,7 +1227,7 @@ static int attention_bwd(const void* qkv, const void* out, const void* dout, con
   if ((hs != 64 && hs != 32) || T <= 0 || (long long)B * nh * T >= (1LL << 31)) return -10;
   const int d = nh * hs;
   const long long rows = (long long)B * T;
-  if (attention_bwd_is_short(T, hs, B * nh)) {
+  if (const ShortBwdPlan plan = attention_bwd_plan(T, hs, B * nh); plan.warps) {
     // 16-byte copies, and what the tensor maps of the other kernel refuse
     if ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(dout) |
          reinterpret_cast<uintptr_t>(dqkv) | reinterpret_cast<uintptr_t>(dq_acc)) & 15)
@@ -1230,9 +1235,7 @@ static int attention_bwd(const void* qkv, const void* out, const void* dout, con
     const ShortBwdArgs a = {(const __nv_bfloat16*)qkv, (const __nv_bfloat16*)out, (const __nv_bfloat16*)dout, lse, (__nv_bfloat16*)dqkv,
                             tl_launch.colsum, T, nh, scale};
     tl_launch.colsum = nullptr;
-    // where an SM is left over for them, dQ has blocks of its own
-    const int parts = B * nh < att_num_sms() ? 2 : 1;
-    return hs == 64 ? attention_short_bwd<64>(a, B * nh, parts, st) : attention_short_bwd<32>(a, B * nh, parts, st);
+    return hs == 64 ? attention_short_bwd<64>(a, plan, B * nh, st) : attention_short_bwd<32>(a, plan, B * nh, st);
   }
   CUtensorMap tq, tdo, tdq, tdkv;
   int rc = cached_tmap(&tq, TMAP_BF16_4D, qkv, hs, 3LL * nh, T, 3LL * d, 64, 128, B);

@@ -54,8 +54,9 @@ def test_an_unaligned_qkv_is_refused(T):
         attention_fwd(qkv, 1, T, 1)
 
 
-# as above, both sides of the rule (T of 64 and 96 for heads of 64); dQ in blocks of its own (fewer heads than SMs) and not
-BACKWARD = [(T, *shape) for T in (1, 15, 16, 17, 31, 32, 33, 64, 65, 96, 97, 127, 128) for shape in ((1, 1, 64), (2, 4, 32), (13, 12, 64), (40, 4, 32))]
+# as above, both sides of the rule (64 tokens for heads of 64, 192 for heads of 32); a head on two blocks (fewer heads than SMs) and on
+# one, with operands kept and loaded again; dQ of two tiles of keys
+BACKWARD = [(T, *shape) for T in (1, 15, 16, 17, 31, 32, 33, 64, 65, 96, 97, 127, 128, 129, 145, 191, 192, 193) for shape in ((1, 1, 64), (2, 4, 32), (13, 12, 64), (40, 4, 32))]
 
 
 @pytest.mark.parametrize("T,B,nh,hs", BACKWARD)
@@ -63,14 +64,15 @@ def test_backward_has_the_bits_of_longer_sequences(T, B, nh, hs):
     one_tile.test_backward_is_that_of_longer_sequences(B, T, nh, hs)
 
 
-@pytest.mark.parametrize("T,B,nh,hs", [(1, 3, 2, 64), (17, 13, 12, 64), (33, 2, 4, 32), (64, 1, 12, 64), (96, 12, 12, 64), (128, 40, 4, 32)])
+@pytest.mark.parametrize("T,B,nh,hs", [(1, 3, 2, 64), (17, 13, 12, 64), (33, 2, 4, 32), (64, 1, 12, 64), (50, 20, 12, 64), (128, 40, 4, 32), (160, 3, 4, 32), (192, 40, 4, 32)])
 def test_backward_against_64_bits(T, B, nh, hs):
     one_tile.test_backward_against_64_bits(B, T, nh, hs)
 
 
-@pytest.mark.parametrize("B,T", [(300, 1), (16, 16), (9, 31), (30, 17), (6, 64), (3, 96)])
-def test_bias_gradient_of_the_qkv_projection(B, T, monkeypatch):
-    column_sums.test_sums_are_those_of_the_terms(B, T, 12, 768, monkeypatch)
+@pytest.mark.parametrize("B,T,heads,width", [(300, 1, 12, 768), (16, 16, 12, 768), (9, 31, 12, 768), (30, 17, 12, 768), (6, 64, 12, 768),
+                                             (2, 129, 4, 128), (40, 160, 4, 128), (3, 192, 4, 128)])
+def test_bias_gradient_of_the_qkv_projection(B, T, heads, width, monkeypatch):
+    column_sums.test_sums_are_those_of_the_terms(B, T, heads, width, monkeypatch)
 
 
 @pytest.mark.parametrize("T", [17, 64])
