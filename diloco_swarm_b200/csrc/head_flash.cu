@@ -414,8 +414,10 @@ __device__ __noinline__ void row_alone(const __nv_bfloat16* x, const __nv_bfloat
 
 // Slices of the vocabulary -> loss, input gradient, and what the weights' gradient wants to know of a row.  WPR warps share
 // a row's slices; a lane has four columns.  Rows past M (up to a multiple of 128) are marked as masked.
+// A row is a chain of loads (mask, references, sums; target, its row of W), so what counts is the number of warps: with the 128
+// registers the compiler would take, of 65536 rows, two slices, 186 us, with 64 and less unrolled 56 (in a pass 93, 57); 512 rows, 36 slices 12.6, 9.9.
 template <int WPR>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 4)
 head_join_kernel(const float* parts, const float2* ml, const __nv_bfloat16* x, const __nv_bfloat16* W,
                  const long long* __restrict__ targets, const long long* __restrict__ mask, const float* count, float scale,
                  float* __restrict__ loss_acc, __nv_bfloat16* __restrict__ dx, float* __restrict__ nlse, int* __restrict__ target,
@@ -451,7 +453,7 @@ head_join_kernel(const float* parts, const float2* ml, const __nv_bfloat16* x, c
       for (int s = lane; s < slices; s += 32) mx = fmaxf(mx, ref_of(s));
 #pragma unroll
       for (int i = 16; i > 0; i >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, i));
-#pragma unroll 4
+#pragma unroll 2
       for (int s = part; s < slices; s += WPR) {
         const float2* t = ml + 4LL * s * M + row;
         const float sum = (t[0].y + t[M].y) + (t[2LL * M].y + t[3LL * M].y);
