@@ -1,0 +1,36 @@
+"""Embedding backward: rows of one token are added up in a block before they go to memory (csrc/elementwise.cu)."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+# one row; rows on either side of a block's (16 to 256); blocks of columns that are whole, ragged and 8 wide; many sequences
+@pytest.mark.parametrize("B,T,d", [(1, 1, 8), (1, 15, 64), (3, 17, 136), (1, 257, 128), (9, 31, 768), (2, 1000, 1600), (65, 257, 128), (300, 3, 128)])
+@pytest.mark.parametrize("tokens", ["one", "few", "all different", "text"])
+def test_rows_of_a_token(B, T, d, tokens):
+    from diloco_swarm_b200.ops import kernels as K
+    V = 50304
+    g = torch.Generator(device="cuda").manual_seed(T)
+    u = torch.rand(B * T, generator=g, device="cuda", dtype=torch.float64)
+    ids = {"one": torch.full_like(u, V - 1), "few": (u * 5).floor() * 512, "all different": torch.arange(B * T, device="cuda") * 2 % V,
+           "text": ((V + 1.0) ** u).floor() - 1}[tokens].long().clamp_(0, V - 1).view(B, T)
+    dx = torch.randn(B * T, d, device="cuda", generator=g).to(torch.bfloat16)
+    dwte, dwpe = torch.ones(V, d, device="cuda"), torch.ones(T + 1, d, device="cuda")
+    K.embedding_bwd(ids, dx, dwte, dwpe)
+    x = dx.double()
+    for got, index, n in ((dwte, ids.view(-1), V), (dwpe, torch.arange(T, device="cuda").repeat(B), T + 1)):
+        want = torch.ones(n, d, device="cuda", dtype=torch.float64).index_add_(0, index, x)
+        terms = torch.ones(n, d, device="cuda", dtype=torch.float64).index_add_(0, index, x.abs())
+        count = torch.zeros(n, 1, device="cuda", dtype=torch.float64).index_add_(0, index, torch.ones(B * T, 1, device="cuda", dtype=torch.float64))
+        # every addition rounds a partial sum, at most the sum of the terms, by 2^-24 of it
+        assert ((got.double() - want).abs() <= count * 2 ** -24 * terms).all()
+
+
+def test_tokens_out_of_range_fall_on_the_first():
+    from diloco_swarm_b200.ops import kernels as K
+    ids = torch.tensor([[-1, 7, 1 << 40, 0, 10, -(1 << 40), 9]], device="cuda")
+    dx = torch.arange(1, 8, device="cuda").view(7, 1).expand(7, 16).contiguous().to(torch.bfloat16)
+    dwte, dwpe = torch.zeros(10, 16, device="cuda"), torch.zeros(7, 16, device="cuda")
+    K.embedding_bwd(ids, dx, dwte, dwpe)
+    assert dwte[:, 0].tolist() == [1 + 3 + 4 + 5 + 6, 0, 0, 0, 0, 0, 0, 2, 0, 7] and torch.equal(dwpe, dx.float())
